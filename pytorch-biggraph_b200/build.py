@@ -9,6 +9,7 @@ import glob
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -30,7 +31,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJ, exist_ok=True)
     headers = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(HERE, "..", "include", "*.h"))
     newest_header = max(os.path.getmtime(h) for h in headers)
-    objs, rebuilt = [], False
+    objs, commands = [], []
     for src in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
         obj = os.path.join(OBJ, os.path.basename(src)[:-3] + ".o")
         objs.append(obj)
@@ -39,9 +40,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
             cmd = [_nvcc()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-c", src, "-o", obj]
             if verbose:
                 print(" ".join(cmd), flush=True)
-            subprocess.check_call(cmd)
-            rebuilt = True
-    if rebuilt or not os.path.exists(OUT):
+            commands.append(cmd)
+    with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+        list(pool.map(subprocess.check_call, commands))
+    if commands or not os.path.exists(OUT):
         cmd = [_nvcc(), "-shared", "-o", OUT] + objs + ["-lcudart"]
         subprocess.check_call(cmd)
     return OUT

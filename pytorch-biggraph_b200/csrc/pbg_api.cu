@@ -21,8 +21,11 @@ struct pbg_context {
   char *ws = nullptr;
   size_t ws_bytes = 0;
   WaveBufs bufs;           // workspace pointers (table pointers filled per call)
-  SortPlan sort[2];        // double-buffered: wave w+1 is sorted on `side` while wave w trains
-  cudaStream_t side = nullptr;      // key build + sort of the next wave
+  SortPlan sort[2];        // double-buffered scratch of the three-launch sort: wave w+1 is sorted on `side` while wave w trains
+  // sorted lists of two groups of waves: the next group is sorted on `side` while this one trains
+  unsigned long long *wkeys[2][PBG_SORT_WAVES];
+  unsigned int *wvals[2][PBG_SORT_WAVES];
+  cudaStream_t side = nullptr;      // sorts of the waves to come
   cudaStream_t part2 = nullptr;     // second half of a wave's gather / score / loss / gradient kernels
   cudaEvent_t ev_wave = nullptr, ev_part2 = nullptr, ev_joined = nullptr, ev_stats = nullptr;
   cudaEvent_t ev_sorted[2] = {nullptr, nullptr}, ev_updated[2] = {nullptr, nullptr}, ev_inputs = nullptr;
@@ -53,11 +56,7 @@ struct pbg_context {
   long long *etab_dev = nullptr;      // per-relation tables of a sub_bucket call + its counts
   long long etab_cap = 0;
   char *allnegs_mem = nullptr;        // scratch of pbg_eval_batch_all_negs, allocated at its first call
-  SortPlan csort = {{nullptr, nullptr}, {nullptr, nullptr}, nullptr, 0, 0};   // call-wide sort of all waves' slots
-  char *csort_mem = nullptr;
   int split_min_k = 2;                // waves of at least this many batches run as two halves on two streams (PBG_SPLIT_MIN_K)
-  int group_sort_mode = -1;           // PBG_CALL_SORT: 1 = always sort waves in groups, 0 = never, unset = where it pays
-  std::vector<cudaEvent_t> ev_group;  // one per group of waves sorted together
   // optional event timing per kernel class
   const float *edge_w = nullptr;   // per-edge weights for the next train / eval call (pbg_set_edge_weights)
   bool profiling = false;
@@ -218,8 +217,6 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
     c->fused_halves = envh && envh[0] == '1';
     const char *envk = getenv("PBG_SPLIT_MIN_K");
     if (envk && atoi(envk) >= 2) c->split_min_k = atoi(envk);
-    const char *envs = getenv("PBG_CALL_SORT");
-    if (envs && (envs[0] == '0' || envs[0] == '1')) c->group_sort_mode = envs[0] - '0';
   }
   if (planes) {
     oXB[0] = take(nN * npl * Dpb * 2); oXB[1] = take(nN * npl * Dpb * 2);
@@ -245,6 +242,9 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
     oV[s][0] = take((size_t)nocc * 4); oV[s][1] = take((size_t)nocc * 4);
     oH[s] = take(pbg_sort_hist_entries((int)nocc) * 4);
   }
+  size_t oWK[2][PBG_SORT_WAVES], oWV[2][PBG_SORT_WAVES];
+  for (int s = 0; s < 2; ++s)
+    for (int i = 0; i < PBG_SORT_WAVES; ++i) { oWK[s][i] = take((size_t)nocc * 8); oWV[s][i] = take((size_t)nocc * 4); }
   size_t oSum = take(8 * sizeof(double)), oErr = take(256), oEval = take(8 * sizeof(double));
   size_t oPsum = take((size_t)nocc * c->Dp * 4), oHub = take(((size_t)nocc / 8 + 64) * 8), oHubCnt = take(256);
   size_t oBigTab = take(pbg_bigtab_bytes((long long)nocc));
@@ -297,6 +297,10 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
     c->sort[s].hist = (unsigned int *)(c->ws + oH[s]);
     c->sort[s].max_n = (int)nocc;
     c->sort[s].result = 0;
+    for (int i = 0; i < PBG_SORT_WAVES; ++i) {
+      c->wkeys[s][i] = (unsigned long long *)(c->ws + oWK[s][i]);
+      c->wvals[s][i] = (unsigned int *)(c->ws + oWV[s][i]);
+    }
     CU(c, cudaEventCreateWithFlags(&c->ev_sorted[s], cudaEventDisableTiming));
     CU(c, cudaEventCreateWithFlags(&c->ev_updated[s], cudaEventDisableTiming));
   }
@@ -347,8 +351,6 @@ extern "C" int pbg_destroy(pbg_context *c) {
   for (int i = 0; i < 2; ++i) if (c->uni_dev[i]) cudaFree(c->uni_dev[i]);
   if (c->esort_mem) cudaFree(c->esort_mem);
   if (c->allnegs_mem) cudaFree(c->allnegs_mem);
-  if (c->csort_mem) cudaFree(c->csort_mem);
-  for (auto e : c->ev_group) cudaEventDestroy(e);
   if (c->etab_dev) cudaFree(c->etab_dev);
   for (int s = 0; s < 2; ++s) {
     if (c->ev_sorted[s]) cudaEventDestroy(c->ev_sorted[s]);
@@ -386,24 +388,6 @@ extern "C" int pbg_neg_columns(const pbg_context *c, int32_t count, int32_t *chu
   if (chunks) *chunks = P > 0 ? (count + P - 1) / P : 0;
   if (lhs_neg_cols) *lhs_neg_cols = c->cfg.disable_lhs_negs ? 0 : cols;
   if (rhs_neg_cols) *rhs_neg_cols = c->cfg.disable_rhs_negs ? 0 : cols;
-  return PBG_OK;
-}
-
-#define PBG_CALL_SORT_MAX (1ll << 23)     // most slots of a call whose waves are sorted in groups (the buffers hold all of them: 24 bytes per slot)
-#define PBG_SORT_GROUP_SLOTS (1ll << 19)  // slots sorted at a time
-
-static int ensure_call_sort(pbg_context *c, long long n) {
-  if (n <= c->csort.max_n) return PBG_OK;
-  if (c->csort_mem) { cudaFree(c->csort_mem); c->csort_mem = nullptr; c->csort.max_n = 0; }
-  const long long cap = n + n / 8 + 1024;
-  const size_t kb = align_up((size_t)cap * 8, 256), vb = align_up((size_t)cap * 4, 256);
-  const size_t hb = align_up(pbg_sort_hist_entries((int)cap) * 4, 256);
-  CU(c, cudaMalloc(&c->csort_mem, 2 * kb + 2 * vb + hb));
-  char *p = c->csort_mem;
-  c->csort.keys[0] = (unsigned long long *)p; c->csort.keys[1] = (unsigned long long *)(p + kb);
-  c->csort.vals[0] = (unsigned int *)(p + 2 * kb); c->csort.vals[1] = (unsigned int *)(p + 2 * kb + vb);
-  c->csort.hist = (unsigned int *)(p + 2 * kb + 2 * vb);
-  c->csort.max_n = (int)cap;
   return PBG_OK;
 }
 
@@ -563,7 +547,6 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
   const int kbase = num_batches / nwaves, kextra = num_batches % nwaves;
   std::vector<WaveBatches> wbs((size_t)nwaves);
   std::vector<int> kks((size_t)nwaves);
-  std::vector<long long> slot0((size_t)nwaves + 1, 0);
   for (int wv = 0, b0 = 0; wv < nwaves; ++wv) {
     const int kk = kbase + (wv < kextra ? 1 : 0);
     WaveBatches &wb = wbs[wv];
@@ -576,73 +559,46 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
       wb.wrel[i] = bk->relation_weights ? bk->relation_weights[wi] : 1.0f;
     }
     kks[wv] = kk;
-    slot0[wv + 1] = slot0[wv] + (long long)kk * d.spb;
     b0 += kk;
   }
-  // Waves are sorted several at a time: the slots of a group of waves, keyed by (wave in the group, row), go through
-  // one radix sort of a few passes -- instead of a dozen launches of a few microseconds per wave, which on small
-  // dimensions (a wave of 56,000 slots of 100 floats) are a large part of the step.  The sorted list is the per-wave
-  // lists one after the other; the wave tags are masked off again.  Groups hold about PBG_SORT_GROUP_SLOTS slots, so
-  // that the first update of a call waits for a short sort only and the later groups are sorted beside the training
-  // of the earlier ones.  This pays where a wave's own sort needs three or more passes (keys above 22 bits: two
-  // partitions of millions of rows; measured +4.5 % on such a bucket at dimension 100); with two passes per wave the
-  // larger sort kernels of a group get in the way of the training kernels on the other stream more than the saved
-  // launches give back (-8 % on a 100,000-row graph), so those calls, and calls of a single wave, sort wave by wave.
-  // PBG_CALL_SORT=1 / 0 in the environment forces one or the other.
-  const long long wave_slots = (long long)c->kmax * d.spb;
-  int group = (int)((PBG_SORT_GROUP_SLOTS + wave_slots - 1) / wave_slots);
-  // the first update of a call waits for the first group's sort, which nothing hides: a call of few waves (a half
-  // sub-bucket of the several-GPU schedule is ten) is cut into at least four groups, of two waves or more
-  if (group > (nwaves + 3) / 4) group = (nwaves + 3) / 4;
-  if (group < 2) group = 2;
-  if (group > nwaves) group = nwaves;
-  if (group < 1) group = 1;
-  const int wave_bits = bit_length((unsigned long long)(group - 1));
-  const bool wanted = c->group_sort_mode == 1 || (c->group_sort_mode < 0 && bits > 22);
-  const bool call_sort = wanted && nwaves > 1 && group > 1 && slot0[nwaves] <= PBG_CALL_SORT_MAX && bits + wave_bits <= 44;
-  const int ngroups = call_sort ? (nwaves + group - 1) / group : 0;
-  SortPlan *csp = nullptr;
-  if (call_sort) {
-    int rcs = ensure_call_sort(c, slot0[nwaves]);
-    if (rcs) return rcs;
-    csp = &c->csort;
-    while ((int)c->ev_group.size() < ngroups) {
-      cudaEvent_t e;
-      CU(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-      c->ev_group.push_back(e);
+  // Waves are sorted PBG_SORT_WAVES at a time by one kernel, a cluster per wave, one group ahead of the group that
+  // trains: few launches, and the sort of the next group has a whole group's training to hide behind.  The call's
+  // first group is one wave, so that its update waits for the shortest sort there is.  Waves beyond what a cluster
+  // holds are sorted one by one, one wave ahead.
+  const bool cluster = pbg_cluster_sort_fits((long long)(kbase + (kextra ? 1 : 0)) * d.spb, bits);
+  const int gsize = cluster ? PBG_SORT_WAVES : 1;
+  auto group_of = [&](int wv) { return wv == 0 ? 0 : 1 + (wv - 1) / gsize; };
+  auto group_first = [&](int g) { return g == 0 ? 0 : 1 + (g - 1) * gsize; };
+  const int ngroups = group_of(nwaves - 1) + 1;
+  auto sort_group = [&](int g) -> int {                       // into buffer half g & 1
+    if (g >= ngroups) return PBG_OK;
+    if (g >= 2) CU(c, cudaStreamWaitEvent(c->side, c->ev_updated[g & 1], 0));   // group g - 2 has been applied
+    const int w0 = group_first(g), w1 = g + 1 < ngroups ? group_first(g + 1) : nwaves;
+    ClassTimer t(c, 0, c->side);
+    if (cluster) {
+      SortWaves sw;
+      sw.count = w1 - w0;
+      for (int i = 0; i < sw.count; ++i) { sw.w[i].wb = wbs[w0 + i]; sw.w[i].k = kks[w0 + i]; sw.w[i].keys = c->wkeys[g & 1][i]; sw.w[i].vals = c->wvals[g & 1][i]; }
+      t.done(launch_sort_waves(d, w, sw, bits, c->side));
+    } else {
+      WaveDims dw = d;
+      dw.k = kks[w0]; dw.nblk = dw.k * d.Cm; dw.nocc = dw.k * d.spb; dw.blk0 = 0;
+      SortPlan &sp = c->sort[g & 1];
+      int n = launch_build_keys(dw, wbs[w0], w, sp.keys[0], sp.vals[0], c->side);
+      t.done(n + pbg_sort(sp, dw.nocc, bits, c->side));
     }
-    for (int gi = 0; gi < ngroups; ++gi) {
-      const int w0 = gi * group, w1 = w0 + group < nwaves ? w0 + group : nwaves;
-      const long long off = slot0[w0], cnt = slot0[w1] - slot0[w0];
-      ClassTimer t(c, 0, c->side);
-      int n = 0;
-      for (int wv = w0; wv < w1; ++wv) {
-        WaveDims dw = d;
-        dw.k = kks[wv]; dw.nblk = kks[wv] * d.Cm; dw.nocc = kks[wv] * d.spb; dw.blk0 = 0;
-        n += launch_build_keys(dw, wbs[wv], w, csp->keys[0] + slot0[wv], csp->vals[0] + slot0[wv], c->side, (unsigned long long)(wv - w0) << bits);
-      }
-      SortPlan gsp = *csp;                                    // the group's part of the buffers; the counters are shared (one stream)
-      gsp.keys[0] += off; gsp.keys[1] += off; gsp.vals[0] += off; gsp.vals[1] += off;
-      n += pbg_sort(gsp, (int)cnt, bits + wave_bits, c->side);
-      csp->result = gsp.result;                               // the same number of passes for every group
-      n += launch_mask_keys(gsp.keys[gsp.result], cnt, (1ull << bits) - 1ull, c->side);
-      t.done(n);
-      CU(c, cudaEventRecord(c->ev_group[gi], c->side));
-    }
-  }
+    CU(c, cudaEventRecord(c->ev_sorted[g & 1], c->side));
+    return PBG_OK;
+  };
+  rc = sort_group(0);
+  if (rc) return rc;
   int wave = 0;
   for (int b0 = 0; b0 < num_batches; ++wave) {
     const int kk = kks[wave];
     const WaveBatches &wb = wbs[wave];
     d.k = kk; d.nblk = kk * d.Cm; d.nocc = kk * d.spb;
-    SortPlan &sp = c->sort[wave & 1];
-    if (!call_sort) {
-      if (wave >= 2) CU(c, cudaStreamWaitEvent(c->side, c->ev_updated[wave & 1], 0));   // buffers free again
-      ClassTimer t(c, 0, c->side);
-      int n = launch_build_keys(d, wb, w, sp.keys[0], sp.vals[0], c->side);
-      t.done(n + pbg_sort(sp, d.nocc, bits, c->side));
-      CU(c, cudaEventRecord(c->ev_sorted[wave & 1], c->side));
-    }
+    const int grp = group_of(wave), in_grp = wave - group_first(grp);
+    if (in_grp == 0) { rc = sort_group(grp + 1); if (rc) return rc; }
     // The batches of a wave all read the tables as the wave found them, so its forward / backward
     // kernels can run as two independent halves on two streams: the memory-bound kernels of one
     // half fill the SMs' idle issue slots while the other half's contractions run.
@@ -681,15 +637,16 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
       { ClassTimer t(c, 6, c->part2); t.done(launch_stats(d, wb, w, stats_out ? c->stats_dev : nullptr, c->sum_dev, c->part2)); }
       CU(c, cudaEventRecord(c->ev_stats, c->part2));
     }
-    CU(c, cudaStreamWaitEvent(c->stream, call_sort ? c->ev_group[wave / group] : c->ev_sorted[wave & 1], 0));
+    if (in_grp == 0) CU(c, cudaStreamWaitEvent(c->stream, c->ev_sorted[grp & 1], 0));
     {
       ClassTimer t(c, 5);
-      const unsigned long long *wkeys = call_sort ? csp->keys[csp->result] + slot0[wave] : sp.keys[sp.result];
-      const unsigned int *wvals = call_sort ? csp->vals[csp->result] + slot0[wave] : sp.vals[sp.result];
+      const SortPlan &sp = c->sort[grp & 1];
+      const unsigned long long *wkeys = cluster ? c->wkeys[grp & 1][in_grp] : sp.keys[sp.result];
+      const unsigned int *wvals = cluster ? c->wvals[grp & 1][in_grp] : sp.vals[sp.result];
       t.done(launch_update(d, wb, w, wkeys, wvals, c->cfg.lr, c->cfg.relation_lr, c->psum, c->hublist, c->hubcnt, c->bigtab, c->stream,
                            c->upd_side, c->ev_upd_fork, c->ev_upd_join));
     }
-    CU(c, cudaEventRecord(c->ev_updated[wave & 1], c->stream));
+    if (wave == nwaves - 1 || group_of(wave + 1) != grp) CU(c, cudaEventRecord(c->ev_updated[grp & 1], c->stream));
     if (stats_aside) CU(c, cudaStreamWaitEvent(c->stream, c->ev_stats, 0));   // the next wave rewrites the loss rows
     else { ClassTimer t(c, 6); t.done(launch_stats(d, wb, w, stats_out ? c->stats_dev : nullptr, c->sum_dev, c->stream)); }
     b0 += kk;
@@ -873,8 +830,14 @@ extern "C" int pbg_row_adagrad(pbg_context *c, float *emb, float *state, int64_t
   SortPlan &sp = c->sort[0];
   if (n > sp.max_n) return fail(c, PBG_ERR_TOO_LARGE, "%d gradient rows exceed this context's sort capacity %d", n, sp.max_n);
   CU(c, cudaSetDevice(c->device));
-  c->launches += launch_iota_keys((const long long *)rows, num_rows, n, sp.keys[0], sp.vals[0], c->errflag, c->stream);
-  c->launches += pbg_sort(sp, n, bit_length((unsigned long long)num_rows), c->stream);
+  const int bits = bit_length((unsigned long long)num_rows);
+  if (pbg_cluster_sort_fits(n, bits)) {
+    sp.result = 0;
+    c->launches += launch_sort_rows((const long long *)rows, num_rows, n, bits, sp.keys[0], sp.vals[0], c->errflag, c->stream);
+  } else {
+    c->launches += launch_iota_keys((const long long *)rows, num_rows, n, sp.keys[0], sp.vals[0], c->errflag, c->stream);
+    c->launches += pbg_sort(sp, n, bits, c->stream);
+  }
   c->launches += launch_row_adagrad_sorted(emb, state, c->cfg.dim, sp.keys[sp.result], sp.vals[sp.result],
                                            grads, n, lr, (unsigned long long)num_rows, c->stream);
   CU(c, pbg_take_launch_error());

@@ -183,6 +183,37 @@ __device__ __forceinline__ Occ occ_decode(const WaveDims &d, int o) {
   return q;
 }
 
+// Sort key of occurrence slot o: the table row its gradient belongs to.
+//   lhs-table rows            key = row
+//   rhs-table rows            key = row (+ lhs rows when the tables differ)
+//   operator-table rows       key = key_rel_base + table * num_rels + rel   (dynamic relations)
+//   slots without gradient    key = key_invalid (sorts to the end)
+__device__ __forceinline__ unsigned long long slot_key(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, int o) {
+  Occ q = occ_decode(d, o);
+  BlockInfo bi = block_info(d, wb, q.blk);
+  unsigned long long key = d.key_invalid;
+  unsigned long long rbase = d.shared_table ? 0ull : (unsigned long long)d.n_rows[0];
+  if (q.a == ARR_N0 || q.a == ARR_N1) {
+    int side = q.a == ARR_N0 ? 0 : 1;
+    long long row = slot_row(d, wb, w, bi, side, q.r);
+    if (row >= 0 && row < d.n_rows[side]) key = (side ? rbase : 0ull) + (unsigned long long)row;
+  } else if (q.r < bi.n) {
+    long long e = bi.e0 + q.r;
+    if (q.a == ARR_Q0) {
+      long long row = w.rhs[e];
+      if (row >= 0 && row < d.n_rows[1]) key = rbase + (unsigned long long)row;
+    } else if (q.a == ARR_Q1) {
+      long long row = w.lhs[e];
+      if (row >= 0 && row < d.n_rows[0]) key = (unsigned long long)row;
+    } else if (d.dynamic && d.op != PBG_OP_NONE) {
+      long long rl = w.rel[e];
+      int t = q.a == ARR_R0 ? 0 : 1;
+      if (rl >= 0 && rl < d.num_rels) key = d.key_rel_base + (unsigned long long)t * d.num_rels + (unsigned long long)rl;
+    }
+  }
+  return key;
+}
+
 // N3 regularizer pieces at elements [dd, dd + 4) of a row y: the term is sum m^3 with m = |y_d|, or for
 // complex_diagonal the modulus of the pair (y_d, y_{d +- D/2}) counted once per pair
 // (torchbiggraph/operators.py:42-43, 151-157).  n3_grad4: d(sum m^3)/dy = 3 m y.
@@ -299,6 +330,21 @@ inline cudaError_t pbg_opt_in_smem(const void *kernel, int bytes) {
   else pbg_note_launch(e);
   return e;
 }
+// Opt-in to clusters of sixteen CTAs (eight is the portable limit), per (kernel, device) like the above.
+inline cudaError_t pbg_opt_in_cluster16(const void *kernel) {
+  static std::mutex mu;
+  static std::map<std::pair<const void *, int>, bool> done;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) { pbg_note_launch(e); return e; }
+  std::lock_guard<std::mutex> lock(mu);
+  bool &d = done[{kernel, dev}];
+  if (d) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) d = true;
+  else pbg_note_launch(e);
+  return e;
+}
 inline int pbg_sm_count() {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 1;
@@ -318,9 +364,20 @@ size_t pbg_sort_hist_entries(int n);   // digit counters (unsigned int) a sort o
 // Stable LSD radix sort of n (key, value) pairs on `bits` low key bits; returns launches made.
 int pbg_sort(SortPlan &sp, int n, int bits, cudaStream_t st);
 
+// Stable sort in one kernel, a thread-block cluster per list: lists of at most PBG_CLUSTER_SORT_MAX pairs, keys below 2^32.
+#define PBG_CLUSTER_SORT_MAX (16 * 1024 * 16)
+inline bool pbg_cluster_sort_fits(long long n, int bits) { return n <= PBG_CLUSTER_SORT_MAX && bits <= 32; }
+#define PBG_SORT_WAVES 4            // most waves of one launch
+struct SortWave { WaveBatches wb; int k; unsigned long long *keys; unsigned int *vals; };
+struct SortWaves { SortWave w[PBG_SORT_WAVES]; int count; };
+// keys of the slots of `waves` (built on the fly) sorted into each wave's keys / vals
+int launch_sort_waves(const WaveDims &d, const WaveBufs &w, const SortWaves &waves, int bits, cudaStream_t st);
+// rows[i] -> (row, i) pairs sorted by row; rows outside [0, num_rows) are flagged and sort to the end as num_rows
+int launch_sort_rows(const long long *rows, long long num_rows, int n, int bits, unsigned long long *keys, unsigned int *vals,
+                     int *errflag, cudaStream_t st);
+
 int launch_build_keys(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w,
-                      unsigned long long *keys, unsigned int *vals, cudaStream_t st, unsigned long long tag = 0ull);
-int launch_mask_keys(unsigned long long *keys, long long n, unsigned long long mask, cudaStream_t st);
+                      unsigned long long *keys, unsigned int *vals, cudaStream_t st);
 int launch_gather(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st);
 void *pbg_tc_plan_create(const WaveDims &d, const WaveBufs &w, int nblk_max, int precision);
 void pbg_tc_plan_destroy(void *plan);

@@ -474,56 +474,18 @@ int launch_gather(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, c
   return 1;
 }
 
-// One thread per occurrence slot: the sort key is the table row the slot's gradient belongs to.
-//   lhs-table rows            key = row
-//   rhs-table rows            key = row (+ lhs rows when the tables differ)
-//   operator-table rows       key = key_rel_base + table * num_rels + rel   (dynamic relations)
-//   slots without gradient    key = key_invalid (sorts to the end)
-// `tag` is OR-ed into every key (the wave's number above the key bits when a whole call is sorted at once).
-__global__ void build_keys_kernel(WaveDims d, WaveBatches wb, WaveBufs w, unsigned long long *keys,
-                                  unsigned int *vals, unsigned long long tag) {
+// One thread per occurrence slot (waves too large for the one-kernel sort, which builds its keys itself).
+__global__ void build_keys_kernel(WaveDims d, WaveBatches wb, WaveBufs w, unsigned long long *keys, unsigned int *vals) {
   int o = blockIdx.x * blockDim.x + threadIdx.x;
   if (o >= d.nocc) return;
-  Occ q = occ_decode(d, o);
-  BlockInfo bi = block_info(d, wb, q.blk);
-  unsigned long long key = d.key_invalid;
-  unsigned long long rbase = d.shared_table ? 0ull : (unsigned long long)d.n_rows[0];
-  if (q.a == ARR_N0 || q.a == ARR_N1) {
-    int side = q.a == ARR_N0 ? 0 : 1;
-    long long row = slot_row(d, wb, w, bi, side, q.r);
-    if (row >= 0 && row < d.n_rows[side]) key = (side ? rbase : 0ull) + (unsigned long long)row;
-  } else if (q.r < bi.n) {
-    long long e = bi.e0 + q.r;
-    if (q.a == ARR_Q0) {
-      long long row = w.rhs[e];
-      if (row >= 0 && row < d.n_rows[1]) key = rbase + (unsigned long long)row;
-    } else if (q.a == ARR_Q1) {
-      long long row = w.lhs[e];
-      if (row >= 0 && row < d.n_rows[0]) key = (unsigned long long)row;
-    } else if (d.dynamic && d.op != PBG_OP_NONE) {
-      long long rl = w.rel[e];
-      int t = q.a == ARR_R0 ? 0 : 1;
-      if (rl >= 0 && rl < d.num_rels) key = d.key_rel_base + (unsigned long long)t * d.num_rels + (unsigned long long)rl;
-    }
-  }
-  keys[o] = key | tag;
+  keys[o] = slot_key(d, wb, w, o);
   vals[o] = (unsigned int)o;
 }
 
 int launch_build_keys(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w,
-                      unsigned long long *keys, unsigned int *vals, cudaStream_t st, unsigned long long tag) {
-  build_keys_kernel<<<(d.nocc + 255) / 256, 256, 0, st>>>(d, wb, w, keys, vals, tag);
+                      unsigned long long *keys, unsigned int *vals, cudaStream_t st) {
+  build_keys_kernel<<<(d.nocc + 255) / 256, 256, 0, st>>>(d, wb, w, keys, vals);
   return 1;
-}
-
-// keys[i] &= mask: drops the wave tags once the call-wide sort has grouped the slots by wave
-__global__ void mask_keys_kernel(unsigned long long *keys, long long n, unsigned long long mask) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) keys[i] &= mask;
-}
-int launch_mask_keys(unsigned long long *keys, long long n, unsigned long long mask, cudaStream_t st) {
-  if (n > 0) mask_keys_kernel<<<(int)((n + 255) / 256), 256, 0, st>>>(keys, n, mask);
-  return n > 0;
 }
 
 // ------------------------------------------------------------------------------------------------

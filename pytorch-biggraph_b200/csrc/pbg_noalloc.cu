@@ -65,11 +65,16 @@ extern "C" int pbg_row_adagrad_static(float *emb, float *state, int64_t num_rows
   int *errflag = (int *)(base + 2 * NA_KEYS_BYTES + 2 * NA_VALS_BYTES + NA_HIST_BYTES);
   // the array keeps whatever the previous call left: the error word has to start at zero
   if (cudaMemsetAsync(errflag, 0, sizeof(int), st) != cudaSuccess) return PBG_ERR_CUDA;
-  launch_iota_keys((const long long *)rows_dev, num_rows, n, sp.keys[0], sp.vals[0], errflag, st);
-  pbg_sort(sp, n, bit_len((unsigned long long)num_rows), st);
+  const int bits = bit_len((unsigned long long)num_rows);
+  if (pbg_cluster_sort_fits(n, bits)) {
+    launch_sort_rows((const long long *)rows_dev, num_rows, n, bits, sp.keys[0], sp.vals[0], errflag, st);
+  } else {
+    launch_iota_keys((const long long *)rows_dev, num_rows, n, sp.keys[0], sp.vals[0], errflag, st);
+    pbg_sort(sp, n, bits, st);
+  }
   launch_row_adagrad_sorted(emb, state, dim, sp.keys[sp.result], sp.vals[sp.result], grads_dev, n, lr,
                             (unsigned long long)num_rows, st);
-  if (cudaGetLastError() != cudaSuccess) return PBG_ERR_CUDA;
+  if (pbg_take_launch_error() != cudaSuccess) return PBG_ERR_CUDA;
   int flag = 0;
   if (cudaMemcpyAsync(&flag, errflag, sizeof flag, cudaMemcpyDeviceToHost, st) != cudaSuccess) return PBG_ERR_CUDA;
   if (cudaStreamSynchronize(st) != cudaSuccess) return PBG_ERR_CUDA;

@@ -13,7 +13,14 @@
 //                  every warp walks its run in order and writes each pair to
 //                  base[digit] + scanned[digit][warp] + (earlier pairs of the run with that digit)
 // Ranking inside a run uses __match_any_sync, so equal digits keep their input order (stable).
+//
+// That is the form for long lists.  A list that fits in the shared memory of one thread-block cluster -- every wave
+// up to 262,144 slots -- is sorted by ONE kernel (cluster_sort_kernel, at the end of this file).
+#include <cooperative_groups.h>
+
 #include "pbg_common.cuh"
+
+namespace cg = cooperative_groups;
 
 #define RUN_ITEMS 8                      // pairs per lane per run
 #define RUN (32 * RUN_ITEMS)             // pairs per warp
@@ -167,5 +174,179 @@ __global__ void iota_keys(const long long *__restrict__ rows, long long num_rows
 int launch_iota_keys(const long long *rows, long long num_rows, int n, unsigned long long *keys,
                      unsigned int *vals, int *errflag, cudaStream_t st) {
   iota_keys<<<(n + 255) / 256, 256, 0, st>>>(rows, num_rows, n, keys, vals, errflag);
+  return 1;
+}
+
+// ------------------------------------------------------------------------------------------------
+// One kernel, one cluster per list.  The three-launch passes above are latency: seven launches for the two passes of a
+// wave of 4,000 slots (keys included), each a few microseconds of which hardly any is work.  Here the list never leaves
+// the cluster: every thread holds IPT pairs in registers, a pass ranks them inside the warp (ballots), scans the warps'
+// digit counts inside the CTA, exchanges the CTAs' digit totals through distributed shared memory (one cluster
+// barrier) and writes every pair to its place in the shared memory of the CTA that owns it (a second barrier); the last
+// pass writes to global memory.  Digits of at most 8 bits: the warps' counters of a CTA are 32 KB, and the exchange of
+// 16 x 256 totals is one coalesced round.
+// ------------------------------------------------------------------------------------------------
+#define CS_THREADS 1024
+#define CS_WARPS 32
+#define CS_BINS 256
+
+struct SortRows { const long long *rows; long long num_rows; int n; unsigned long long *keys; unsigned int *vals; int *errflag; };
+
+template <int IPT>
+__device__ __forceinline__ void cluster_sort_body(uint2 (&item)[IPT], int n, int bits, unsigned long long *keys_out, unsigned int *vals_out,
+                                                  unsigned char *smem) {
+  uint2 *buf = (uint2 *)smem;                                           // [CS_THREADS * IPT] pairs of this CTA
+  unsigned int *cnt = (unsigned int *)(smem + (size_t)CS_THREADS * IPT * 8);   // [CS_WARPS][bins]
+  unsigned int *all = cnt + CS_WARPS * CS_BINS;                         // [CTAs][bins] digit totals of every CTA
+  unsigned int *base = all + 16 * CS_BINS;                              // [bins]
+  unsigned int *wsum = base + CS_BINS;                                  // [8]
+  cg::cluster_group cluster = cg::this_cluster();
+  const int nct = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int t = threadIdx.x, lane = t & 31, wl = t >> 5;
+  const int passes = (bits + 7) / 8, db = (bits + passes - 1) / passes, bins = 1 << db;
+  const unsigned int mask = (unsigned int)bins - 1u, lt = (1u << lane) - 1u;
+  unsigned int *wc = cnt + wl * bins;
+  unsigned int off[IPT];
+  for (int pass = 0, shift = 0; pass < passes; ++pass, shift += db) {
+    for (int i = lane; i < bins; i += 32) wc[i] = 0u;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < IPT; ++i) {
+      const unsigned int dg = (item[i].x >> shift) & mask;
+      unsigned int peers = 0xffffffffu;
+      for (int b = 0; b < db; ++b) {
+        const unsigned int m = __ballot_sync(0xffffffffu, (dg >> b) & 1u);
+        peers &= ((dg >> b) & 1u) ? m : ~m;
+      }
+      const unsigned int before = wc[dg];
+      __syncwarp();
+      if ((peers & lt) == 0u) wc[dg] = before + __popc(peers);
+      __syncwarp();
+      off[i] = before + __popc(peers & lt);
+    }
+    __syncthreads();
+    if (t < bins) {
+      unsigned int run = 0u;
+#pragma unroll 8
+      for (int w = 0; w < CS_WARPS; ++w) { const unsigned int c = cnt[w * bins + t]; cnt[w * bins + t] = run; run += c; }
+      for (int c = 0; c < nct; ++c) cluster.map_shared_rank(all, c)[rank * CS_BINS + t] = run;
+    }
+    cluster.sync();                                                     // totals are everywhere; every pair is in registers
+    unsigned int tot = 0u, lower = 0u;
+    if (t < bins) {
+      for (int c = 0; c < nct; ++c) { const unsigned int v = all[c * CS_BINS + t]; tot += v; if (c < rank) lower += v; }
+    }
+    if (t < CS_BINS) {
+      unsigned int incl = tot;
+      for (int o = 1; o < 32; o <<= 1) { const unsigned int v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
+      if (lane == 31) wsum[wl] = incl;
+      base[t] = incl - tot + lower;
+    }
+    __syncthreads();
+    if (t < CS_BINS && wl > 0) {
+      unsigned int before = 0u;
+      for (int w = 0; w < wl; ++w) before += wsum[w];
+      base[t] += before;
+    }
+    __syncthreads();
+    const bool last = pass == passes - 1;
+#pragma unroll
+    for (int i = 0; i < IPT; ++i) {
+      const unsigned int dg = (item[i].x >> shift) & mask;
+      const unsigned int pos = base[dg] + wc[dg] + off[i];
+      if (last) {
+        if (pos < (unsigned int)n) { keys_out[pos] = item[i].x; vals_out[pos] = item[i].y; }
+      } else {
+        cluster.map_shared_rank(buf, pos / (CS_THREADS * IPT))[pos % (CS_THREADS * IPT)] = item[i];
+      }
+    }
+    if (!last) {
+      cluster.sync();
+#pragma unroll
+      for (int i = 0; i < IPT; ++i) item[i] = buf[(wl * IPT + i) * 32 + lane];
+    }
+  }
+}
+
+template <int IPT>
+static size_t cluster_sort_smem() { return (size_t)CS_THREADS * IPT * 8 + (CS_WARPS * CS_BINS + 16 * CS_BINS + CS_BINS + 8) * 4; }
+
+// Pairs beyond the list's end carry the largest key; they come last in every pass and are not written out.
+template <int IPT>
+__global__ void __launch_bounds__(CS_THREADS, 1)
+sort_waves_kernel(WaveDims d, WaveBufs w, const __grid_constant__ SortWaves waves, int bits) {
+  extern __shared__ __align__(16) unsigned char cs_smem[];
+  const int nct = (int)cg::this_cluster().num_blocks(), rank = (int)cg::this_cluster().block_rank();
+  const SortWave &sw = waves.w[blockIdx.x / nct];
+  const int n = sw.k * d.spb;
+  const int first = rank * CS_THREADS * IPT + (threadIdx.x >> 5) * 32 * IPT + (threadIdx.x & 31);
+  uint2 item[IPT];
+#pragma unroll
+  for (int i = 0; i < IPT; ++i) {
+    const int o = first + i * 32;
+    item[i] = make_uint2(o < n ? (unsigned int)slot_key(d, sw.wb, w, o) : 0xffffffffu, (unsigned int)o);
+  }
+  cluster_sort_body<IPT>(item, n, bits, sw.keys, sw.vals, cs_smem);
+}
+
+template <int IPT>
+__global__ void __launch_bounds__(CS_THREADS, 1) sort_rows_kernel(SortRows a, int bits) {
+  extern __shared__ __align__(16) unsigned char cs_smem[];
+  const int first = (int)cg::this_cluster().block_rank() * CS_THREADS * IPT + (threadIdx.x >> 5) * 32 * IPT + (threadIdx.x & 31);
+  uint2 item[IPT];
+#pragma unroll
+  for (int i = 0; i < IPT; ++i) {
+    const int o = first + i * 32;
+    unsigned int key = 0xffffffffu;
+    if (o < a.n) {
+      const long long r = a.rows[o];
+      const bool bad = r < 0 || r >= a.num_rows;
+      if (bad) atomicOr(a.errflag, 1);
+      key = (unsigned int)(bad ? a.num_rows : r);
+    }
+    item[i] = make_uint2(key, (unsigned int)o);
+  }
+  cluster_sort_body<IPT>(item, a.n, bits, a.keys, a.vals, cs_smem);
+}
+
+// CTAs and pairs per thread for a list of n: four pairs per thread as long as the cluster can grow (a pass costs about
+// the same with one CTA as with sixteen, and more pairs per thread lengthen it), then 8 and 16 on sixteen CTAs.
+static void cluster_shape(int n, int &ctas, int &ipt) {
+  ipt = 4;
+  for (ctas = 1; ctas < 16 && ctas * CS_THREADS * 4 < n; ctas *= 2) {}
+  while (ctas * CS_THREADS * ipt < n) ipt *= 2;
+}
+
+template <class... Args>
+static void launch_cluster(void (*kernel)(Args...), int lists, int ctas, size_t smem, cudaStream_t st, Args... args) {
+  pbg_opt_in_smem((const void *)kernel, (int)smem);
+  if (ctas > 8) pbg_opt_in_cluster16((const void *)kernel);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(lists * ctas); cfg.blockDim = dim3(CS_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = ctas; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+  cfg.attrs = &at; cfg.numAttrs = 1;
+  pbg_note_launch(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+
+int launch_sort_waves(const WaveDims &d, const WaveBufs &w, const SortWaves &waves, int bits, cudaStream_t st) {
+  int most = 0, ctas, ipt;
+  for (int i = 0; i < waves.count; ++i) if (waves.w[i].k > most) most = waves.w[i].k;
+  cluster_shape(most * d.spb, ctas, ipt);
+  if (ipt == 4) launch_cluster(sort_waves_kernel<4>, waves.count, ctas, cluster_sort_smem<4>(), st, d, w, waves, bits);
+  else if (ipt == 8) launch_cluster(sort_waves_kernel<8>, waves.count, ctas, cluster_sort_smem<8>(), st, d, w, waves, bits);
+  else launch_cluster(sort_waves_kernel<16>, waves.count, ctas, cluster_sort_smem<16>(), st, d, w, waves, bits);
+  return 1;
+}
+
+int launch_sort_rows(const long long *rows, long long num_rows, int n, int bits, unsigned long long *keys, unsigned int *vals,
+                     int *errflag, cudaStream_t st) {
+  SortRows a{rows, num_rows, n, keys, vals, errflag};
+  int ctas, ipt;
+  cluster_shape(n, ctas, ipt);
+  if (ipt == 4) launch_cluster(sort_rows_kernel<4>, 1, ctas, cluster_sort_smem<4>(), st, a, bits);
+  else if (ipt == 8) launch_cluster(sort_rows_kernel<8>, 1, ctas, cluster_sort_smem<8>(), st, a, bits);
+  else launch_cluster(sort_rows_kernel<16>, 1, ctas, cluster_sort_smem<16>(), st, a, bits);
   return 1;
 }
