@@ -27,9 +27,14 @@ struct pbg_context {
   unsigned int *wvals[2][PBG_SORT_WAVES];
   cudaStream_t side = nullptr;      // sorts of the waves to come
   cudaStream_t part2 = nullptr;     // second half of a wave's gather / score / loss / gradient kernels
-  cudaEvent_t ev_wave = nullptr, ev_part2 = nullptr, ev_joined = nullptr, ev_stats = nullptr;
+  cudaEvent_t ev_wave = nullptr, ev_part2 = nullptr;
   cudaEvent_t ev_sorted[2] = {nullptr, nullptr}, ev_updated[2] = {nullptr, nullptr}, ev_inputs = nullptr;
-  pbg_batch_stats *stats_dev = nullptr;
+  // What a call reads back lies in pinned host memory that the kernels write themselves: the error word (written only
+  // when something is wrong), the evaluator's sums, a batch's Stats.  Reading it costs the call's one synchronisation
+  // and no copy (two pageable copies of a few bytes were 20 us of a 150 us call).
+  struct HostBox { int err; int pad[15]; double eval[8]; double sum[8]; };
+  HostBox *box = nullptr, *box_dev = nullptr;
+  pbg_batch_stats *stats_host = nullptr, *stats_dev = nullptr;
   int stats_cap = 0;
   double *sum_dev = nullptr;
   double *eval_dev = nullptr;
@@ -40,7 +45,8 @@ struct pbg_context {
   bool fused_halves = false;    // ... as two halves of the wave on two streams (PBG_HALVES=1; for comparisons)
   float *psum = nullptr;        // partial gradient rows of hub rows, indexed by slot position
   long long *hublist = nullptr;
-  int *hubcnt = nullptr;
+  int *hubcnt = nullptr;        // two sets of counters, used in turn
+  unsigned hub_turn = 0;
   long long *bigtab = nullptr;  // batch boundaries of the rows with 256 and more slots in a wave
   cudaStream_t upd_side = nullptr;                          // operator-row kernels that run beside the embedding rows' update
   cudaEvent_t ev_upd_fork = nullptr, ev_upd_join = nullptr;
@@ -169,9 +175,10 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= device || device < 0)
     return fail(c, PBG_ERR_NO_DEVICE, "CUDA device %d not available", device);
   CU(c, cudaSetDevice(device));
-  cudaDeviceProp prop;
-  CU(c, cudaGetDeviceProperties(&prop, device));
-  if (prop.major != 10) return fail(c, PBG_ERR_NO_DEVICE, "device %d is sm_%d%d; this library is built for sm_100a only", device, prop.major, prop.minor);
+  int major = 0, minor = 0;
+  CU(c, cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+  CU(c, cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
+  if (major != 10) return fail(c, PBG_ERR_NO_DEVICE, "device %d is sm_%d%d; this library is built for sm_100a only", device, major, minor);
 
   c->kmax = cfg->batches_in_flight;
   c->U = cfg->num_uniform_negs;
@@ -245,8 +252,8 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   size_t oWK[2][PBG_SORT_WAVES], oWV[2][PBG_SORT_WAVES];
   for (int s = 0; s < 2; ++s)
     for (int i = 0; i < PBG_SORT_WAVES; ++i) { oWK[s][i] = take((size_t)nocc * 8); oWV[s][i] = take((size_t)nocc * 4); }
-  size_t oSum = take(8 * sizeof(double)), oErr = take(256), oEval = take(8 * sizeof(double));
-  size_t oPsum = take((size_t)nocc * c->Dp * 4), oHub = take(((size_t)nocc / 8 + 64) * 8), oHubCnt = take(256);
+  size_t oSum = take(8 * sizeof(double)), oEval = take(8 * sizeof(double));
+  size_t oPsum = take((size_t)nocc * c->Dp * 4), oHub = take(((size_t)nocc / 8 + 64) * 8), oHubCnt = take(512);
   size_t oBigTab = take(pbg_bigtab_bytes((long long)nocc));
   // dynamic relations with a (vector) operator: the operator-row gradient of every edge, written by the pull-back pass
   size_t oGR[2] = {0, 0};
@@ -309,15 +316,16 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   CU(c, cudaStreamCreateWithFlags(&c->part2, cudaStreamNonBlocking));
   CU(c, cudaEventCreateWithFlags(&c->ev_wave, cudaEventDisableTiming));
   CU(c, cudaEventCreateWithFlags(&c->ev_part2, cudaEventDisableTiming));
-  CU(c, cudaEventCreateWithFlags(&c->ev_joined, cudaEventDisableTiming));
-  CU(c, cudaEventCreateWithFlags(&c->ev_stats, cudaEventDisableTiming));
+  CU(c, cudaHostAlloc((void **)&c->box, sizeof *c->box, cudaHostAllocMapped | cudaHostAllocPortable));
+  memset(c->box, 0, sizeof *c->box);
+  CU(c, cudaHostGetDevicePointer((void **)&c->box_dev, c->box, 0));
   if (!(getenv("PBG_REL_ASIDE") && getenv("PBG_REL_ASIDE")[0] == '0')) {        // PBG_REL_ASIDE=0: everything on one stream (for comparisons)
     CU(c, cudaStreamCreateWithFlags(&c->upd_side, cudaStreamNonBlocking));
     CU(c, cudaEventCreateWithFlags(&c->ev_upd_fork, cudaEventDisableTiming));
     CU(c, cudaEventCreateWithFlags(&c->ev_upd_join, cudaEventDisableTiming));
   }
   c->sum_dev = (double *)(c->ws + oSum);
-  c->errflag = (int *)(c->ws + oErr);
+  c->errflag = &c->box_dev->err;
   c->eval_dev = (double *)(c->ws + oEval);
   b.errflag = c->errflag;
   c->psum = (float *)(c->ws + oPsum);
@@ -346,7 +354,8 @@ extern "C" int pbg_destroy(pbg_context *c) {
   if (c->ws) cudaFree(c->ws);
   if (c->tcplan) pbg_tc_plan_destroy(c->tcplan);
   if (c->pairplan) pbg_pair_plan_destroy(c->pairplan);
-  if (c->stats_dev) cudaFree(c->stats_dev);
+  if (c->stats_host) cudaFreeHost(c->stats_host);
+  if (c->box) cudaFreeHost(c->box);
   for (int i = 0; i < 3; ++i) if (c->edge_dev[i]) cudaFree(c->edge_dev[i]);
   for (int i = 0; i < 2; ++i) if (c->uni_dev[i]) cudaFree(c->uni_dev[i]);
   if (c->esort_mem) cudaFree(c->esort_mem);
@@ -364,8 +373,6 @@ extern "C" int pbg_destroy(pbg_context *c) {
   if (c->ev_upd_join) cudaEventDestroy(c->ev_upd_join);
   if (c->ev_wave) cudaEventDestroy(c->ev_wave);
   if (c->ev_part2) cudaEventDestroy(c->ev_part2);
-  if (c->ev_joined) cudaEventDestroy(c->ev_joined);
-  if (c->ev_stats) cudaEventDestroy(c->ev_stats);
   for (auto &s : c->spans) { cudaEventDestroy(s.a); cudaEventDestroy(s.b); }
   for (auto e : c->event_pool) cudaEventDestroy(e);
   delete c;
@@ -433,12 +440,20 @@ static int bind_bucket(pbg_context *c, const pbg_bucket *bk, WaveDims &d, WaveBu
   return PBG_OK;
 }
 
+// Waits for the stream, then reads and clears the error word the kernels write in host memory.
+static int wait_for_flag(pbg_context *c, int &flag) {
+  CU(c, cudaStreamSynchronize(c->stream));
+  volatile int *err = &c->box->err;
+  flag = *err;
+  if (flag) *err = 0;
+  return PBG_OK;
+}
+
 static int check_errflag(pbg_context *c) {
   int flag = 0;
-  CU(c, cudaMemcpyAsync(&flag, c->errflag, sizeof flag, cudaMemcpyDeviceToHost, c->stream));
-  CU(c, cudaStreamSynchronize(c->stream));
+  int rc = wait_for_flag(c, flag);
+  if (rc) return rc;
   if (flag) {
-    cudaMemsetAsync(c->errflag, 0, sizeof(int), c->stream);
     if (flag & 2) return fail(c, PBG_ERR_TIMEOUT, "a bounded device-side wait ran out (flag %d)", flag);
     return fail(c, PBG_ERR_INDEX_RANGE, "an entity or relation id was outside its table; those rows were skipped");
   }
@@ -529,10 +544,12 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
   w.ew = c->edge_w; c->edge_w = nullptr;                    // per-edge weights apply to one call
   w.seed = seed ^ (c->batches_done * 0x9E3779B97F4A7C15ull);
   if (stats_out && num_batches > c->stats_cap) {
-    if (c->stats_dev) cudaFree(c->stats_dev);
-    c->stats_dev = nullptr;
+    CU(c, cudaStreamSynchronize(c->stream));                 // an earlier call may still write the old array
+    if (c->stats_host) cudaFreeHost(c->stats_host);
+    c->stats_host = nullptr; c->stats_cap = 0;
     int cap = num_batches + num_batches / 2 + 64;
-    CU(c, cudaMalloc(&c->stats_dev, (size_t)cap * sizeof(pbg_batch_stats)));
+    CU(c, cudaHostAlloc((void **)&c->stats_host, (size_t)cap * sizeof(pbg_batch_stats), cudaHostAllocMapped | cudaHostAllocPortable));
+    CU(c, cudaHostGetDevicePointer((void **)&c->stats_dev, c->stats_host, 0));
     c->stats_cap = cap;
   }
   const int bits = bit_length(d.key_invalid);
@@ -590,15 +607,14 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
     CU(c, cudaEventRecord(c->ev_sorted[g & 1], c->side));
     return PBG_OK;
   };
-  rc = sort_group(0);
-  if (rc) return rc;
+  UpdateScratch us{c->psum, c->hublist, c->hubcnt, &c->hub_turn, c->bigtab, c->upd_side, c->ev_upd_fork, c->ev_upd_join,
+                   stats_out ? c->stats_dev : nullptr, c->sum_dev};
   int wave = 0;
   for (int b0 = 0; b0 < num_batches; ++wave) {
     const int kk = kks[wave];
     const WaveBatches &wb = wbs[wave];
     d.k = kk; d.nblk = kk * d.Cm; d.nocc = kk * d.spb;
     const int grp = group_of(wave), in_grp = wave - group_first(grp);
-    if (in_grp == 0) { rc = sort_group(grp + 1); if (rc) return rc; }
     // The batches of a wave all read the tables as the wave found them, so its forward / backward
     // kernels can run as two independent halves on two streams: the memory-bound kernels of one
     // half fill the SMs' idle issue slots while the other half's contractions run.
@@ -628,35 +644,26 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
     } else {
       run_part(c, d, wb, w, c->stream);
     }
-    // The per-batch statistics need the loss rows of both halves and nothing of the update: they are
-    // summed on the second stream while the update runs on the first.
-    const bool stats_aside = kk >= c->split_min_k && !c->profile_serial;
-    if (stats_aside) {
-      CU(c, cudaEventRecord(c->ev_joined, c->stream));
-      CU(c, cudaStreamWaitEvent(c->part2, c->ev_joined, 0));
-      { ClassTimer t(c, 6, c->part2); t.done(launch_stats(d, wb, w, stats_out ? c->stats_dev : nullptr, c->sum_dev, c->part2)); }
-      CU(c, cudaEventRecord(c->ev_stats, c->part2));
-    }
+    // the sorts depend on ids only; their launches come after this wave's, which the GPU can start on meanwhile
+    if (wave == 0) { rc = sort_group(0); if (rc) return rc; }
+    if (in_grp == 0) { rc = sort_group(grp + 1); if (rc) return rc; }
     if (in_grp == 0) CU(c, cudaStreamWaitEvent(c->stream, c->ev_sorted[grp & 1], 0));
     {
       ClassTimer t(c, 5);
       const SortPlan &sp = c->sort[grp & 1];
       const unsigned long long *wkeys = cluster ? c->wkeys[grp & 1][in_grp] : sp.keys[sp.result];
       const unsigned int *wvals = cluster ? c->wvals[grp & 1][in_grp] : sp.vals[sp.result];
-      t.done(launch_update(d, wb, w, wkeys, wvals, c->cfg.lr, c->cfg.relation_lr, c->psum, c->hublist, c->hubcnt, c->bigtab, c->stream,
-                           c->upd_side, c->ev_upd_fork, c->ev_upd_join));
+      t.done(launch_update(d, wb, w, wkeys, wvals, c->cfg.lr, c->cfg.relation_lr, us, c->stream));
     }
     if (wave == nwaves - 1 || group_of(wave + 1) != grp) CU(c, cudaEventRecord(c->ev_updated[grp & 1], c->stream));
-    if (stats_aside) CU(c, cudaStreamWaitEvent(c->stream, c->ev_stats, 0));   // the next wave rewrites the loss rows
-    else { ClassTimer t(c, 6); t.done(launch_stats(d, wb, w, stats_out ? c->stats_dev : nullptr, c->sum_dev, c->stream)); }
     b0 += kk;
   }
   c->batches_done += (unsigned long long)num_batches;
   CU(c, pbg_take_launch_error());
   if (stats_out) {
-    CU(c, cudaMemcpyAsync(stats_out, c->stats_dev, (size_t)num_batches * sizeof(pbg_batch_stats),
-                          cudaMemcpyDeviceToHost, c->stream));
-    return check_errflag(c);
+    rc = check_errflag(c);
+    memcpy(stats_out, c->stats_host, (size_t)num_batches * sizeof(pbg_batch_stats));
+    return rc;
   }
   return PBG_OK;
 }
@@ -709,9 +716,9 @@ extern "C" int pbg_set_edge_weights(pbg_context *c, const float *weights_dev) {
 extern "C" int pbg_read_stats(pbg_context *c, pbg_batch_stats *out) {
   if (!c || !out) return PBG_ERR_BAD_ARGUMENT;
   CU(c, cudaSetDevice(c->device));
-  double s[5];
-  CU(c, cudaMemcpyAsync(s, c->sum_dev, sizeof s, cudaMemcpyDeviceToHost, c->stream));
-  CU(c, cudaMemsetAsync(c->sum_dev, 0, sizeof s, c->stream));
+  double *s = c->box->sum;
+  CU(c, cudaMemcpyAsync(s, c->sum_dev, 5 * sizeof *s, cudaMemcpyDeviceToHost, c->stream));
+  CU(c, cudaMemsetAsync(c->sum_dev, 0, 5 * sizeof *s, c->stream));
   int rc = check_errflag(c);
   out->loss = (float)s[0]; out->reg = (float)s[4];
   out->violators_lhs = (int64_t)(s[1] + 0.5); out->violators_rhs = (int64_t)(s[2] + 0.5); out->count = (int64_t)(s[3] + 0.5);
@@ -773,8 +780,8 @@ extern "C" int pbg_eval_batch(pbg_context *c, const pbg_bucket *bk, const int64_
   run_forward(c, d, wb, w, c->stream);
   c->launches += launch_eval(d, wb, w, c->eval_dev, c->stream);
   CU(c, pbg_take_launch_error());
-  double h[8];
-  CU(c, cudaMemcpyAsync(h, c->eval_dev, sizeof h, cudaMemcpyDeviceToHost, c->stream));
+  double *h = c->box->eval;
+  CU(c, cudaMemcpyAsync(h, c->eval_dev, sizeof c->box->eval, cudaMemcpyDeviceToHost, c->stream));
   rc = check_errflag(c);
   int sides = (d.neg_enabled[0] ? 1 : 0) + (d.neg_enabled[1] ? 1 : 0);
   double div = sides > 0 ? sides : 1;
@@ -810,8 +817,8 @@ extern "C" int pbg_eval_batch_all_negs(pbg_context *c, const pbg_bucket *bk, con
   const float wrel = bk->relation_weights ? bk->relation_weights[d.dynamic ? 0 : relidx] : 1.0f;
   c->launches += launch_allnegs_eval(d, w, c->allnegs_mem, count, PBG_ALLNEGS_SLAB, d.dynamic ? 0 : relidx, wrel, c->eval_dev, c->stream);
   CU(c, pbg_take_launch_error());
-  double h[8];
-  CU(c, cudaMemcpyAsync(h, c->eval_dev, sizeof h, cudaMemcpyDeviceToHost, c->stream));
+  double *h = c->box->eval;
+  CU(c, cudaMemcpyAsync(h, c->eval_dev, sizeof c->box->eval, cudaMemcpyDeviceToHost, c->stream));
   rc = check_errflag(c);
   int sides = (d.neg_enabled[0] ? 1 : 0) + (d.neg_enabled[1] ? 1 : 0);
   double div = sides > 0 ? sides : 1;
@@ -847,10 +854,9 @@ extern "C" int pbg_row_adagrad(pbg_context *c, float *emb, float *state, int64_t
 // ---- edge-list utilities (torchbiggraph/util.cpp) -------------------------------------------------
 static int check_errflag_edges(pbg_context *c, const char *what) {
   int flag = 0;
-  CU(c, cudaMemcpyAsync(&flag, c->errflag, sizeof flag, cudaMemcpyDeviceToHost, c->stream));
-  CU(c, cudaStreamSynchronize(c->stream));
+  int rc = wait_for_flag(c, flag);
+  if (rc) return rc;
   if (flag) {
-    cudaMemsetAsync(c->errflag, 0, sizeof(int), c->stream);
     if (flag & 4) return fail(c, PBG_ERR_INDEX_RANGE, "%s: rel > numRelations", what);
     return fail(c, PBG_ERR_INDEX_RANGE, "%s: a value lies outside its table; those elements were skipped", what);
   }

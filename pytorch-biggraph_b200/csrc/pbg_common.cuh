@@ -399,12 +399,17 @@ int launch_grad_simt(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w
 int launch_loss(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st);
 int launch_export_scores(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w,
                          float *lhs_pos, float *rhs_pos, float *lhs_neg, float *rhs_neg, cudaStream_t st);
-// side / fork / join: a second stream and two events for the parts of the update that can run beside the embedding
-// rows' kernels (null: everything on st)
-int launch_update(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w,
-                  const unsigned long long *keys, const unsigned int *vals, float lr, float rel_lr,
-                  float *psum, long long *hublist, int *hubcnt, long long *bigtab, cudaStream_t st,
-                  cudaStream_t side = nullptr, cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr);
+// What the optimizer kernels of a wave work with.  hubcnt: two sets of counters, 64 ints apart, used in turn (*turn):
+// while one set counts, the kernel behind it clears the other for the next user.  side / fork / join: a second stream and
+// two events for the parts of the update that can run beside the embedding rows' kernels (null: everything on the main
+// stream).  per_batch (may be null) / sum: where the Stats of the wave's batches go.
+struct UpdateScratch {
+  float *psum; long long *hublist; int *hubcnt; unsigned *turn; long long *bigtab;
+  cudaStream_t side; cudaEvent_t fork, join;
+  pbg_batch_stats *per_batch; double *sum;
+};
+int launch_update(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, const unsigned long long *keys, const unsigned int *vals,
+                  float lr, float rel_lr, const UpdateScratch &us, cudaStream_t st);
 // bigtab: (nocc / 256 + 2) rows of PBG_KMAX + 1 entries: where the batches of a row with 256 and more slots start, and its end
 inline size_t pbg_bigtab_bytes(long long nocc) { return (size_t)(nocc / 256 + 2) * (PBG_KMAX + 1) * sizeof(long long); }
 int launch_eval(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, double *out8_dev, cudaStream_t st);
@@ -412,8 +417,6 @@ size_t pbg_allnegs_bytes(int B, int Dp, int slab);
 int launch_allnegs_eval(const WaveDims &d, const WaveBufs &w, char *mem, int B, int slab, int rel_std, float wrel,
                         double *out8_dev, cudaStream_t st);
 int launch_reg_value(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st);
-int launch_stats(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w,
-                 pbg_batch_stats *per_batch_dev, double *sum_dev, cudaStream_t st);
 int launch_row_adagrad_sorted(float *emb, float *state, int dim, const unsigned long long *keys,
                               const unsigned int *vals, const float *grads, int n, float lr,
                               unsigned long long key_invalid, cudaStream_t st);

@@ -456,51 +456,6 @@ int launch_reg_value(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w
   return 1;
 }
 
-// Per-batch Stats (train_cpu.py:95-101): one CTA per batch of the wave sums its rows in a fixed
-// order; the running totals of the call live in sum_dev (loss, violators_lhs, violators_rhs, count).
-__global__ void __launch_bounds__(256) stats_kernel(WaveDims d, WaveBatches wb, WaveBufs w,
-                                                    pbg_batch_stats *per_batch, double *sum) {
-  __shared__ double sl[256], sr[256];
-  __shared__ long long sv0[256], sv1[256];
-  int b = blockIdx.x, t = threadIdx.x;
-  double l = 0.0, rg = 0.0;
-  long long v0 = 0, v1 = 0;
-  int rows = d.Cm * d.Pm;
-  for (int r = t; r < rows; r += 256) {
-    int c = r / d.Pm, i = r - c * d.Pm;
-    int blk = b * d.Cm + c;
-    BlockInfo bi = block_info(d, wb, blk);
-    if (i >= bi.n) continue;
-    size_t prow = (size_t)blk * d.Pm + i;
-    l += (double)w.lossrow[0][prow] + (double)w.lossrow[1][prow];
-    if (d.reg_coef != 0.f) rg += (double)w.regrow[prow];
-    v0 += w.violrow[0][prow];
-    v1 += w.violrow[1][prow];
-  }
-  sl[t] = l; sr[t] = rg; sv0[t] = v0; sv1[t] = v1;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (t < o) { sl[t] += sl[t + o]; sr[t] += sr[t + o]; sv0[t] += sv0[t + o]; sv1[t] += sv1[t + o]; }
-    __syncthreads();
-  }
-  if (t == 0) {
-    pbg_batch_stats s;
-    s.loss = (float)sl[0]; s.reg = (float)sr[0]; s.violators_lhs = sv0[0]; s.violators_rhs = sv1[0]; s.count = wb.n[b];
-    if (per_batch) per_batch[wb.gidx[b]] = s;
-    atomicAdd(&sum[0], sl[0]);
-    atomicAdd(&sum[1], (double)sv0[0]);
-    atomicAdd(&sum[2], (double)sv1[0]);
-    atomicAdd(&sum[3], (double)wb.n[b]);
-    atomicAdd(&sum[4], sr[0]);
-  }
-}
-
-int launch_stats(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w,
-                 pbg_batch_stats *per_batch_dev, double *sum_dev, cudaStream_t st) {
-  stats_kernel<<<d.k, 256, 0, st>>>(d, wb, w, per_batch_dev, sum_dev);
-  return 1;
-}
-
 // Scores as the reference returns them (model.py:842-844): [count] positives and
 // [count, Pl + U] negatives per side with ignored entries set to -1e9; single batch (wave of 1).
 __global__ void export_scores_kernel(WaveDims d, WaveBatches wb, WaveBufs w, float *lhs_pos, float *rhs_pos,

@@ -525,6 +525,47 @@ __device__ __forceinline__ long long warp_prefix_end(long long lo, long long hi,
   return hi;
 }
 
+// Per-batch Stats (train_cpu.py:95-101) of batch b of the wave, summed by one CTA in a fixed order; the running totals
+// live in `sum` (loss, violators_lhs, violators_rhs, count, reg).  The first k CTAs of the embedding rows'
+// hub_reduce_kernel do this: as a kernel of its own it was 5 to 29 us per wave of one CTA per batch, and a launch.
+__device__ __forceinline__ void batch_stats(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, int b, pbg_batch_stats *per_batch, double *sum) {
+  __shared__ double sl[UPD_WARPS], sr[UPD_WARPS];
+  __shared__ long long sv0[UPD_WARPS], sv1[UPD_WARPS];
+  const int t = threadIdx.x, lane = t & 31;
+  double l = 0.0, rg = 0.0;
+  long long v0 = 0, v1 = 0;
+  const int rows = d.Cm * d.Pm;
+  const int lim = d.batch_negs ? d.num_batch_negs : d.U, nb = wb.n[b], Pl = nb < lim ? nb : lim;
+#pragma unroll 4
+  for (int r = t; r < rows; r += blockDim.x) {
+    const int c = r / d.Pm, i = r - c * d.Pm;
+    if (i >= Pl || c * Pl + i >= nb) continue;
+    const size_t prow = (size_t)b * rows + r;
+    l += (double)w.lossrow[0][prow] + (double)w.lossrow[1][prow];
+    if (d.reg_coef != 0.f) rg += (double)w.regrow[prow];
+    v0 += w.violrow[0][prow];
+    v1 += w.violrow[1][prow];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    l += __shfl_xor_sync(0xffffffffu, l, o); rg += __shfl_xor_sync(0xffffffffu, rg, o);
+    v0 += __shfl_xor_sync(0xffffffffu, v0, o); v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+  }
+  if (lane == 0) { sl[t >> 5] = l; sr[t >> 5] = rg; sv0[t >> 5] = v0; sv1[t >> 5] = v1; }
+  __syncthreads();
+  if (t == 0) {
+    for (int u = 1; u < UPD_WARPS; ++u) { l += sl[u]; rg += sr[u]; v0 += sv0[u]; v1 += sv1[u]; }
+    pbg_batch_stats s;
+    s.loss = (float)l; s.reg = (float)rg; s.violators_lhs = v0; s.violators_rhs = v1; s.count = nb;
+    if (per_batch) per_batch[wb.gidx[b]] = s;
+    atomicAdd(&sum[0], l);
+    atomicAdd(&sum[1], (double)v0);
+    atomicAdd(&sum[2], (double)v1);
+    atomicAdd(&sum[3], (double)nb);
+    atomicAdd(&sum[4], rg);
+  }
+}
+
 // The few rows that collect hundreds of slots per wave (the top nodes of a power-law partition)
 // would keep one CTA of hub_update_kernel busy long after every other row is done.  One CTA per
 // (big row, batch) adds that batch's partial rows up first -- warp w takes runs w, w + 8, ..., the
@@ -532,15 +573,18 @@ __device__ __forceinline__ long long warp_prefix_end(long long lo, long long hi,
 // that hub_update_kernel reads one row per batch of a big row.
 template <int VEC>
 __global__ void __launch_bounds__(32 * UPD_WARPS)
-hub_reduce_kernel(WaveDims d, const unsigned long long *__restrict__ keys, const unsigned int *__restrict__ vals,
+hub_reduce_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys, const unsigned int *__restrict__ vals,
                   float *__restrict__ psum, const long long *__restrict__ hublist, const int *__restrict__ hubcnt,
-                  long long *__restrict__ bigtab) {
+                  int *__restrict__ hubcnt_next, long long *__restrict__ bigtab, int stats, pbg_batch_stats *per_batch, double *sum) {
   extern __shared__ __align__(16) float part[];              // [UPD_WARPS][VEC * 128]
+  if (blockIdx.x == 0 && threadIdx.x < 2) hubcnt_next[threadIdx.x] = 0;      // its last reader is behind us in the stream
+  if (stats && blockIdx.x < d.k) { batch_stats(d, wb, w, blockIdx.x, per_batch, sum); return; }
+  const int cta0 = stats ? d.k : 0;
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int D = d.D;
   const long long *biglist = hub_biglist(hublist, d.nocc);
   const long long items = (long long)hubcnt[1] * d.k;        // the tile kernel listed the big rows
-  for (long long item = blockIdx.x; item < items; item += gridDim.x) {
+  for (long long item = blockIdx.x - cta0; item < items; item += gridDim.x - cta0) {
     const int h = (int)(item / d.k), b = (int)(item % d.k);
     const long long head = biglist[h];
     const unsigned long long key = keys[head];
@@ -1110,8 +1154,6 @@ __global__ void __launch_bounds__(32 * UPD_WARPS, VEC <= 2 ? 4 : 2) dyn_pullback
   }
 }
 
-struct UpdateScratch { float *psum; long long *hublist; int *hubcnt; long long *bigtab; cudaStream_t side; cudaEvent_t fork, join; };
-
 template <int VEC>
 static int launch_update_vec(const WaveDims &d_in, const WaveBatches &wb, const WaveBufs &w,
                              const unsigned long long *keys, const unsigned int *vals, float lr, float rel_lr,
@@ -1181,34 +1223,36 @@ static int launch_update_vec(const WaveDims &d_in, const WaveBatches &wb, const 
     globgrad_kernel<VEC><<<d.nblk, 32 * UPD_WARPS, red_smem, st>>>(d, wb, w);
     ++launches;
   }
-  cudaMemsetAsync(us.hubcnt, 0, 2 * sizeof(int), st);
+  int *hubcnt = us.hubcnt + 64 * (*us.turn & 1), *hubcnt_next = us.hubcnt + 64 * ((*us.turn + 1) & 1);
+  ++*us.turn;
   // the gradient slot is the row's gradient as it stands: dot comparator, and no operator or a translation
   const bool plain = dyn_first || (d.cmp == PBG_CMP_DOT && !d.matrix_op && d.reg_coef == 0.f && (d.op == PBG_OP_NONE || d.op == PBG_OP_TRANSLATION));
-  if (plain) tile_update_kernel<VEC, RULE_EMB, 1><<<ctas_emb, 32 * TILE_WARPS_EMB, stage_smem, st>>>(d, wb, w, keys, vals, lr, us.psum, us.hublist, us.hubcnt);
+  if (plain) tile_update_kernel<VEC, RULE_EMB, 1><<<ctas_emb, 32 * TILE_WARPS_EMB, stage_smem, st>>>(d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt);
   else if (d.cmp == PBG_CMP_COS && !d.matrix_op && d.reg_coef == 0.f && (d.op == PBG_OP_NONE || d.op == PBG_OP_TRANSLATION))
-    tile_update_kernel<VEC, RULE_EMB, 2><<<ctas_emb, 32 * TILE_WARPS_EMB, stage_smem, st>>>(d, wb, w, keys, vals, lr, us.psum, us.hublist, us.hubcnt);
+    tile_update_kernel<VEC, RULE_EMB, 2><<<ctas_emb, 32 * TILE_WARPS_EMB, stage_smem, st>>>(d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt);
   else if (d.cmp == PBG_CMP_DOT && !d.matrix_op && d.reg_coef == 0.f)
-    tile_update_kernel<VEC, RULE_EMB, 3><<<ctas_emb, 32 * TILE_WARPS_EMB, stage_smem, st>>>(d, wb, w, keys, vals, lr, us.psum, us.hublist, us.hubcnt);
-  else tile_update_kernel<VEC, RULE_EMB, 0><<<ctas_emb, 32 * TILE_WARPS_EMB, stage_smem, st>>>(d, wb, w, keys, vals, lr, us.psum, us.hublist, us.hubcnt);
-  hub_reduce_kernel<VEC><<<2 * hub_ctas, 32 * UPD_WARPS, red_smem, st>>>(d, keys, vals, us.psum, us.hublist, us.hubcnt, us.bigtab);
-  hub_update_kernel<VEC, RULE_EMB><<<hub_ctas, 32 * UPD_WARPS, hub_smem, st>>>(d, wb, w, keys, vals, lr, us.psum, us.hublist, us.hubcnt, us.bigtab);
+    tile_update_kernel<VEC, RULE_EMB, 3><<<ctas_emb, 32 * TILE_WARPS_EMB, stage_smem, st>>>(d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt);
+  else tile_update_kernel<VEC, RULE_EMB, 0><<<ctas_emb, 32 * TILE_WARPS_EMB, stage_smem, st>>>(d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt);
+  hub_reduce_kernel<VEC><<<d.k + 2 * hub_ctas, 32 * UPD_WARPS, red_smem, st>>>(d, wb, w, keys, vals, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 1, us.per_batch, us.sum);
+  hub_update_kernel<VEC, RULE_EMB><<<hub_ctas, 32 * UPD_WARPS, hub_smem, st>>>(d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, us.bigtab);
   ++launches;
   launches += 2;
   if (has_op) {
     if (d.dynamic) {
       pbg_opt_in_smem((const void *)hub_update_kernel<VEC, RULE_REL>, (int)hub_smem_max);
-      cudaMemsetAsync(us.hubcnt, 0, 2 * sizeof(int), st);
+      int *t = hubcnt; hubcnt = hubcnt_next; hubcnt_next = t;
+      ++*us.turn;
       if (dyn_first) {
         const size_t rel_smem = (size_t)UPD_WARPS * TILE * d.Dp * sizeof(float);
         pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_REL, 1>, (int)((size_t)UPD_WARPS * TILE * VEC * 128 * sizeof(float)));
-        tile_update_kernel<VEC, RULE_REL, 1><<<ctas, 32 * UPD_WARPS, rel_smem, st>>>(d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, us.hubcnt);
+        tile_update_kernel<VEC, RULE_REL, 1><<<ctas, 32 * UPD_WARPS, rel_smem, st>>>(d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt);
       }
       else if (d.cmp == PBG_CMP_DOT && d.reg_coef == 0.f)
-        tile_update_kernel<VEC, RULE_REL, 3><<<ctas, 32 * UPD_WARPS, 0, st>>>(d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, us.hubcnt);
+        tile_update_kernel<VEC, RULE_REL, 3><<<ctas, 32 * UPD_WARPS, 0, st>>>(d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt);
       else
-        tile_update_kernel<VEC, RULE_REL, 0><<<ctas, 32 * UPD_WARPS, 0, st>>>(d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, us.hubcnt);
-      hub_reduce_kernel<VEC><<<2 * hub_ctas, 32 * UPD_WARPS, red_smem, st>>>(d, keys, vals, us.psum, us.hublist, us.hubcnt, us.bigtab);
-      hub_update_kernel<VEC, RULE_REL><<<hub_ctas, 32 * UPD_WARPS, hub_smem, st>>>(d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, us.hubcnt, us.bigtab);
+        tile_update_kernel<VEC, RULE_REL, 0><<<ctas, 32 * UPD_WARPS, 0, st>>>(d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt);
+      hub_reduce_kernel<VEC><<<2 * hub_ctas, 32 * UPD_WARPS, red_smem, st>>>(d, wb, w, keys, vals, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 0, nullptr, nullptr);
+      hub_update_kernel<VEC, RULE_REL><<<hub_ctas, 32 * UPD_WARPS, hub_smem, st>>>(d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt, us.bigtab);
       ++launches;
       launches += 2;
     } else if (d.matrix_op) {
@@ -1228,10 +1272,8 @@ static int launch_update_vec(const WaveDims &d_in, const WaveBatches &wb, const 
   return launches;
 }
 
-int launch_update(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, const unsigned long long *keys,
-                  const unsigned int *vals, float lr, float rel_lr, float *psum, long long *hublist, int *hubcnt,
-                  long long *bigtab, cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
-  UpdateScratch us{psum, hublist, hubcnt, bigtab, side, fork, join};
+int launch_update(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, const unsigned long long *keys, const unsigned int *vals,
+                  float lr, float rel_lr, const UpdateScratch &us, cudaStream_t st) {
   int vec = (d.D + 127) / 128;
   if (vec <= 1) return launch_update_vec<1>(d, wb, w, keys, vals, lr, rel_lr, us, st);
   if (vec <= 2) return launch_update_vec<2>(d, wb, w, keys, vals, lr, rel_lr, us, st);
