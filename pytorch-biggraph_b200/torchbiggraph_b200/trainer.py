@@ -9,6 +9,7 @@ import time
 from abc import ABC, abstractmethod
 from typing import Dict, Iterable, List, Optional, Tuple
 
+import numpy as np
 import torch
 
 from . import _lib
@@ -21,6 +22,20 @@ from .types import EdgeList, Stats
 
 def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else C.c_void_p(t.data_ptr())
+
+
+# the C structures pbg_batch and pbg_batch_stats as array records
+_BATCH = np.dtype([("offset", np.int64), ("count", np.int32), ("rel", np.int32)])
+_STATS = np.dtype([("loss", np.float32), ("reg", np.float32), ("violators_lhs", np.int64), ("violators_rhs", np.int64), ("count", np.int64)])
+
+
+def _even_batches(n: int, batch_size: int, rel: int) -> np.ndarray:
+    """Descriptors of n edges of one relation cut into batches of batch_size."""
+    out = np.empty(-(-n // batch_size), dtype=_BATCH)
+    out["offset"] = np.arange(len(out), dtype=np.int64) * batch_size
+    out["count"] = np.minimum(batch_size, n - out["offset"])
+    out["rel"] = rel
+    return out
 
 
 class _Native:
@@ -57,6 +72,7 @@ class _Native:
         self.cfg = c
         self.max_batch = max_batch
         self.device_index = model.device.index if model.device.index is not None else torch.cuda.current_device()
+        self._bucket, self._bucket_key = None, ()
         self.ctx = C.c_void_p()
         stream = torch.cuda.current_stream(self.device_index).cuda_stream
         st = self.lib.pbg_create(C.byref(c), self.device_index, C.c_void_p(stream), C.byref(self.ctx))
@@ -76,8 +92,17 @@ class _Native:
     def set_hyper(self, lr, relation_lr, margin):
         check(self.lib.pbg_set_hyperparameters(self.ctx, lr, lr if relation_lr is None else relation_lr, margin), self.ctx)
 
-    def bucket(self, model, relation_idx, states, weights_arr) -> PbgBucket:
+    def bucket(self, model, relation_idx, states, weights) -> PbgBucket:
+        """The call's tables as the library takes them.  `weights`: relation weights of the context's operator group, or
+        None.  The structure is kept for as long as every address in it stays the same (filling its fifteen fields
+        costs a single-batch call as much as three kernel launches)."""
         wl, wr = model.tables_for(relation_idx)
+        rhs_tab, lhs_tab = model.op_table_for(self.op_name)
+        glob = model.globals_for(relation_idx)
+        tensors = (wl, wr, rhs_tab, lhs_tab) + glob + (() if states is None else states)
+        key = (wl.shape[0], wr.shape[0], None if weights is None else tuple(weights)) + tuple([None if t is None else t.data_ptr() for t in tensors])
+        if key == self._bucket_key:
+            return self._bucket
         b = PbgBucket()
         b.lhs_emb, b.lhs_rows = wl.data_ptr(), wl.shape[0]
         b.rhs_emb, b.rhs_rows = wr.data_ptr(), wr.shape[0]
@@ -86,15 +111,15 @@ class _Native:
             b.lhs_state, b.rhs_state = gl.data_ptr(), gr.data_ptr()
             b.rhs_op_state = None if ar is None else ar.data_ptr()
             b.lhs_op_state = None if al is None else al.data_ptr()
-        rhs_tab, lhs_tab = model.op_table_for(self.op_name)
         b.rhs_op = None if rhs_tab is None else rhs_tab.data_ptr()
         b.lhs_op = None if lhs_tab is None else lhs_tab.data_ptr()
-        b.relation_weights = weights_arr
-        gl_, gr_ = model.globals_for(relation_idx)
+        b.relation_weights = None if weights is None else (C.c_float * len(weights))(*weights)
+        gl_, gr_ = glob
         if gl_ is not None:
             b.lhs_global, b.rhs_global = gl_.data_ptr(), gr_.data_ptr()
             if states is not None and len(states) > 4:
                 b.lhs_global_state, b.rhs_global_state = states[4].data_ptr(), states[5].data_ptr()
+        self._bucket, self._bucket_key = b, key
         return b
 
     def score(self, model, edges: EdgeList, ul, ur, seed) -> Scores:
@@ -172,14 +197,15 @@ class B200Trainer(AbstractBatchProcessor):
         self._native_key = None
         self.seed = 0
         self._calls = 0
-        self._batch_arrays = {}
 
     # ---- plumbing ------------------------------------------------------------------------------
     def _state_for(self, table: torch.Tensor) -> torch.Tensor:
-        for opt in list(self.partitioned_optimizers.values()) + list(self.unpartitioned_optimizers.values()):
-            for p in opt.params:
-                if p.data_ptr() == table.data_ptr():
-                    return opt.sum_for(p)
+        ptr = table.data_ptr()
+        for opts in (self.partitioned_optimizers, self.unpartitioned_optimizers):
+            for opt in opts.values():
+                for p in opt.params:
+                    if p.data_ptr() == ptr:
+                        return opt.sum_for(p)
         raise RuntimeError("no RowAdagrad optimizer registered for an embedding table of this batch")
 
     def _lr(self) -> float:
@@ -224,41 +250,47 @@ class B200Trainer(AbstractBatchProcessor):
         per-edge weights parallel to the edge arrays (EdgeList.weight), moved to the device here."""
         if not batches:
             return []
-        if any(model.relations[0 if model.num_dynamic_rels > 0 else b[2]].all_negs for b in batches):
-            raise NotImplementedError("relations with all_negs=True are not trained by torchbiggraph_b200 (the evaluator ranks them)")
-        relation_idx = 0 if model.num_dynamic_rels > 0 else batches[0][2]
-        op_name = model.operator_of(relation_idx)
-        nat = self._context(model, max(b[1] for b in batches), op_name)
-        wl, wr = model.tables_for(relation_idx)
-        if model.num_dynamic_rels == 0:
-            for b in batches:
-                if model.tables_for(b[2])[0] is not wl or model.tables_for(b[2])[1] is not wr or model.operator_of(b[2]) != op_name:
+        if model.num_dynamic_rels == 0 and len(batches) > 1:
+            relation_idx = batches[0][2]
+            op_name = model.operator_of(relation_idx)
+            wl, wr = model.tables_for(relation_idx)
+            for r in {b[2] for b in batches}:
+                if model.tables_for(r)[0] is not wl or model.tables_for(r)[1] is not wr or model.operator_of(r) != op_name:
                     raise NotImplementedError("batches of one call must read the same pair of tables through the same operator "
                                               "(process_in_batches cuts a list into such runs)")
+        stats = self._train_run(model, lhs, rhs, rel, np.array(batches, dtype=_BATCH), uniform_lhs, uniform_rhs, want_per_batch, weights)
+        if stats is None:
+            return []
+        return [Stats(loss=l, reg=g, violators_lhs=vl, violators_rhs=vr, count=n) for l, g, vl, vr, n in stats.tolist()]
+
+    def _train_run(self, model: MultiRelationEmbedder, lhs, rhs, rel, batches: np.ndarray, uniform_lhs=None, uniform_rhs=None,
+                   want_stats: bool = True, weights: Optional[torch.Tensor] = None) -> Optional[np.ndarray]:
+        """One library call over _BATCH records that read one pair of tables through one operator; the _STATS records of
+        the batches, or None when they are not wanted."""
+        dyn = model.num_dynamic_rels > 0
+        rels = np.zeros(1, np.int32) if dyn else batches["rel"]
+        relation_idx = int(rels[0])
+        for r in (relation_idx,) if len(batches) == 1 else np.unique(rels).tolist():
+            if model.relations[r].all_negs:
+                raise NotImplementedError("relations with all_negs=True are not trained by torchbiggraph_b200 (the evaluator ranks them)")
+        op_name = model.operator_of(relation_idx)
+        nat = self._context(model, int(batches["count"].max()), op_name)
+        wl, wr = model.tables_for(relation_idx)
         al, ar = self._op_states(model, op_name)
-        states = (self._state_for(wl), self._state_for(wr), al, ar)
+        gl = self._state_for(wl)
+        states = (gl, gl if wr is wl else self._state_for(wr), al, ar)
         gl_, gr_ = model.globals_for(relation_idx)
         if gl_ is not None:
             if not isinstance(self.model_optimizer, AsyncAdagrad):
                 raise RuntimeError("the model has global embeddings but model_optimizer is not an AsyncAdagrad over them")
             states = states + (self.model_optimizer.sum_for(gl_), self.model_optimizer.sum_for(gr_))
         # the library indexes operator rows and relation weights by the relation's place in its operator group
-        dyn = model.num_dynamic_rels > 0
         members = [0] if dyn else model.op_groups[op_name]
-        warr = (C.c_float * len(members))(*[self.relation_weights[g] for g in members])
-        bucket = nat.bucket(model, relation_idx, states, warr)
-        # the descriptor array of a batch list is built once (a trainer is handed the same bucket layout
-        # over and over; filling a few hundred ctypes structs costs more host time than launching a wave)
-        key = tuple(batches)
-        barr = self._batch_arrays.get(key)
-        if barr is None:
-            barr = (PbgBatch * len(batches))()
-            for i, (o, n, r) in enumerate(batches):
-                barr[i].offset, barr[i].count, barr[i].rel = o, n, (0 if dyn else model.group_of[r][1])
-            if len(self._batch_arrays) > 64:
-                self._batch_arrays.clear()
-            self._batch_arrays[key] = barr
-        sarr = (PbgBatchStats * len(batches))() if want_per_batch else None
+        bucket = nat.bucket(model, relation_idx, states, [self.relation_weights[g] for g in members])
+        desc = batches
+        if dyn or len(members) != len(model.relations):
+            desc = batches.copy()
+            desc["rel"] = 0 if dyn else np.array([g[1] for g in model.group_of], dtype=np.int32)[rels]
         on_host = lhs.device.type == "cpu"
         fn = nat.lib.pbg_train_batches_host if on_host else nat.lib.pbg_train_batches
         for t in (lhs, rhs, rel, uniform_lhs, uniform_rhs):
@@ -270,12 +302,11 @@ class B200Trainer(AbstractBatchProcessor):
                 raise ValueError("one weight per edge is needed")
             weights = weights.to(device=model.device, dtype=torch.float32).contiguous()     # kept alive until the call returns
             check(nat.lib.pbg_set_edge_weights(nat.ctx, _ptr(weights)), nat.ctx)
-        check(fn(nat.ctx, C.byref(bucket), _ptr(lhs), _ptr(rhs), _ptr(rel), lhs.shape[0], barr, len(batches),
-                 _ptr(uniform_lhs), _ptr(uniform_rhs), self.seed + self._calls, sarr), nat.ctx)
-        if not want_per_batch:
-            return []
-        return [Stats(loss=float(s.loss), reg=float(s.reg), violators_lhs=int(s.violators_lhs),
-                      violators_rhs=int(s.violators_rhs), count=int(s.count)) for s in sarr]
+        stats = np.empty(len(desc), dtype=_STATS) if want_stats else None
+        check(fn(nat.ctx, C.byref(bucket), _ptr(lhs), _ptr(rhs), _ptr(rel), lhs.shape[0],
+                 C.cast(desc.ctypes.data, C.POINTER(PbgBatch)), len(desc), _ptr(uniform_lhs), _ptr(uniform_rhs), self.seed + self._calls,
+                 C.cast(stats.ctypes.data, C.POINTER(PbgBatchStats)) if want_stats else None), nat.ctx)
+        return stats
 
     def read_stats(self) -> Stats:
         s = PbgBatchStats()
@@ -368,8 +399,7 @@ class B200RankingEvaluator(AbstractBatchProcessor):
         ul = None if uniform_lhs is None else nat._uniform(uniform_lhs, dev)
         ur = None if uniform_rhs is None else nat._uniform(uniform_rhs, dev)
         members = [0] if dyn else model.op_groups[op_name]
-        warr = (C.c_float * len(members))(*[self.relation_weights[g] for g in members])
-        bucket = nat.bucket(model, r, None, warr)
+        bucket = nat.bucket(model, r, None, [self.relation_weights[g] for g in members])
         full_r, r = r, (0 if dyn else model.group_of[r][1])     # the library's relation index is local to the operator group
         out = _lib.PbgEvalStats()
         self._calls += 1
@@ -393,21 +423,37 @@ class B200RankingEvaluator(AbstractBatchProcessor):
         return self._process_one_batch(model, batch_edges, uniform_lhs, uniform_rhs)
 
 
-def _batches_group_by_relation(rel_sorted: torch.Tensor, batch_size: int, generator=None):
-    """Batch descriptors over edges sorted by relation: repeatedly pick a relation with
-    probability proportional to its remaining edges and emit its next <= batch_size edges
-    (batching.py:58-79)."""
-    rels, counts = torch.unique_consecutive(rel_sorted, return_counts=True)
-    starts = torch.cumsum(counts, 0) - counts
-    left = counts.clone()
+def _draw_batches(counts: List[int], batch_size: int, generator=None) -> List[Tuple[int, int, int]]:
+    """Batch descriptors over edges sorted by relation (counts[r] edges of relation r): repeatedly pick a relation with
+    probability proportional to its remaining edges and emit its next <= batch_size edges (batching.py:58-79).
+    The pick is an exponential race -- relation r arrives after Exp(1) / remaining[r], the first one wins (Efraimidis and
+    Spirakis, weighted random sampling) -- which takes the same draws as torch.multinomial and gives the same picks at a
+    fraction of its overhead; it runs once per batch."""
+    rels = [r for r, n in enumerate(counts) if n > 0]
+    remaining = [counts[r] for r in rels]
+    starts = np.concatenate([[0], np.cumsum(remaining)[:-1]]).astype(np.int64).tolist()
+    left = np.array(remaining, dtype=np.float32)
+    arrival = torch.empty(len(rels), dtype=torch.float32)
+    speed = arrival.numpy()
     out = []
-    while int(left.sum()) > 0:
-        idx = int(torch.multinomial(left.float(), 1, generator=generator))
-        off = int(starts[idx] + counts[idx] - left[idx])
-        n = min(batch_size, int(left[idx]))
-        out.append((off, n, int(rels[idx])))
-        left[idx] -= n
+    total = sum(remaining)
+    while total > 0:
+        arrival.exponential_(1, generator=generator)
+        with np.errstate(divide="ignore"):
+            np.divide(left, speed, out=speed)
+        i = int(speed.argmax())
+        n = min(batch_size, remaining[i])
+        out.append((starts[i], n, rels[i]))
+        starts[i] += n
+        remaining[i] -= n
+        left[i] = remaining[i]
+        total -= n
     return out
+
+
+def _batches_group_by_relation(rel_sorted: torch.Tensor, batch_size: int, generator=None):
+    """The same over the sorted relation ids themselves."""
+    return _draw_batches(torch.bincount(rel_sorted, minlength=1).tolist(), batch_size, generator)
 
 
 def process_in_batches(batch_size: int, model: MultiRelationEmbedder, batch_processor: B200Trainer,
@@ -426,39 +472,38 @@ def process_in_batches(batch_size: int, model: MultiRelationEmbedder, batch_proc
         return Stats(count=0)
     lhs, rhs = edges.lhs.to_tensor().contiguous(), edges.rhs.to_tensor().contiguous()
     weights = torch.as_tensor(edges.weight) if edges.has_weight() else None
+    rel = None
     if model.num_dynamic_rels > 0:
         rel = edges.get_relation_type_as_vector().contiguous()
-        batches = [(o, min(batch_size, n - o), 0) for o in range(0, n, batch_size)]
+        batches = _even_batches(n, batch_size, 0)
     elif edges.has_scalar_relation_type():
-        rel = None
-        r = edges.get_relation_type_as_scalar()
-        batches = [(o, min(batch_size, n - o), r) for o in range(0, n, batch_size)]
+        batches = _even_batches(n, batch_size, edges.get_relation_type_as_scalar())
     else:
-        order = torch.argsort(edges.rel, stable=True)
-        lhs, rhs, rel_sorted = lhs[order].contiguous(), rhs[order].contiguous(), edges.rel[order]
+        # sorted by relation on the device, wherever the edges are: it is a fraction of the copy there
+        dev = model.device
+        counts = torch.bincount(edges.rel, minlength=1).tolist()
+        order = torch.argsort(edges.rel.to(dev, non_blocking=True), stable=True)
+        lhs, rhs = lhs.to(dev, non_blocking=True)[order], rhs.to(dev, non_blocking=True)[order]
         if weights is not None:
-            weights = weights[order.to(weights.device)]
-        rel = None
-        batches = _batches_group_by_relation(rel_sorted.cpu(), batch_size)
-    stats: List[Stats] = []
-    for run in _runs_by_table_pair(model, batches):
-        stats.extend(batch_processor.train_batches(model, lhs, rhs, rel, run, weights=weights))
-    return Stats.sum(stats)
+            weights = weights.to(dev, non_blocking=True)[order]
+        batches = np.array(_draw_batches(counts, batch_size), dtype=_BATCH)
+    runs = _runs_by_table_pair(model, batches)
+    stats = [batch_processor._train_run(model, lhs, rhs, rel, run, weights=weights) for run in runs]
+    s = stats[0] if len(stats) == 1 else np.concatenate(stats)
+    return Stats(loss=float(s["loss"].sum(dtype=np.float64)), reg=float(s["reg"].sum(dtype=np.float64)),
+                 violators_lhs=int(s["violators_lhs"].sum()), violators_rhs=int(s["violators_rhs"].sum()), count=int(s["count"].sum()))
 
 
 def _runs_by_table_pair(model: MultiRelationEmbedder, batches):
-    """Cuts a batch list into maximal runs of consecutive batches whose relations read the same
+    """Cuts a batch list (tuples or _BATCH records) into maximal runs of consecutive batches whose relations read the same
     (lhs table, rhs table) pair through the same operator; one library call trains one run."""
-    if model.num_dynamic_rels > 0 or not batches:
-        return [batches] if batches else []
-    runs, cur, cur_key = [], [], None
-    for b in batches:
-        wl, wr = model.tables_for(b[2])
-        key = (wl.data_ptr(), wr.data_ptr(), model.operator_of(b[2]))
-        if cur and key != cur_key:
-            runs.append(cur)
-            cur = []
-        cur_key = key
-        cur.append(b)
-    runs.append(cur)
-    return runs
+    if model.num_dynamic_rels > 0 or len(batches) < 2:
+        return [batches] if len(batches) else []
+    rels = batches["rel"] if isinstance(batches, np.ndarray) else np.array([b[2] for b in batches])
+    pairs: Dict[Tuple, int] = {}
+    group = np.zeros(int(rels.max()) + 1, dtype=np.int64)
+    for r in np.unique(rels).tolist():
+        wl, wr = model.tables_for(r)
+        group[r] = pairs.setdefault((wl.data_ptr(), wr.data_ptr(), model.operator_of(r)), len(pairs))
+    cuts = [0] + (np.flatnonzero(np.diff(group[rels])) + 1).tolist() + [len(batches)]
+    return [batches[a:b] for a, b in zip(cuts, cuts[1:])]
