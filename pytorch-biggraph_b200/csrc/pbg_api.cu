@@ -48,8 +48,6 @@ struct pbg_context {
   int *hubcnt = nullptr;        // two sets of counters, used in turn
   unsigned hub_turn = 0;
   long long *bigtab = nullptr;  // batch boundaries of the rows with 256 and more slots in a wave
-  cudaStream_t upd_side = nullptr;                          // operator-row kernels that run beside the embedding rows' update
-  cudaEvent_t ev_upd_fork = nullptr, ev_upd_join = nullptr;
   long long *edge_dev[3] = {nullptr, nullptr, nullptr};
   long long edge_cap = 0;
   long long *uni_dev[2] = {nullptr, nullptr};
@@ -238,8 +236,8 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
     oRank[p] = take(nQ * 4);
   }
   oCoef[0] = take(nN * 4); oCoef[1] = take(nN * 4); oCoef[2] = take(nQ * 4); oCoef[3] = take(nQ * 4);
-  size_t oRel = take(nblk * 8 * (size_t)cfg->dim * 4);
-  size_t oGlobPart = take(nblk * 2 * 8 * (size_t)cfg->dim * 4);
+  size_t oRel = take(nblk * (size_t)cfg->dim * 4);
+  size_t oGlobPart = take(nblk * 2 * (size_t)cfg->dim * 4);
   const size_t opw = matrix_op ? (size_t)cfg->dim * cfg->dim + (cfg->op == PBG_OP_AFFINE ? cfg->dim : 0) : (size_t)cfg->dim;
   size_t oR1 = 0, oR2 = 0, oDA = 0;
   if (matrix_op) { oR1 = take(nN * c->Dp * 4); oR2 = take(nN * c->Dp * 4); oDA = take((size_t)c->kmax * opw * 4); }
@@ -259,6 +257,8 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   size_t oGR[2] = {0, 0};
   const bool keep_gr = dyn && cfg->op != PBG_OP_NONE && !matrix_op;
   if (keep_gr) { oGR[0] = take(nQ * c->Dp * 4); oGR[1] = take(nQ * c->Dp * 4); }
+  const bool keep_pg = !dyn && (cfg->op == PBG_OP_DIAGONAL || cfg->op == PBG_OP_COMPLEX_DIAGONAL);
+  const size_t oPG = keep_pg ? take(nN * c->Dp * 4) : 0;
   c->ws_bytes = off;
   CU(c, cudaMalloc(&c->ws, c->ws_bytes));
   CU(c, cudaMemsetAsync(c->ws, 0, c->ws_bytes, c->stream));
@@ -281,6 +281,7 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   b.xrows[0] = b.xrows[1] = c->Mm;
   b.xrows[2] = b.xrows[3] = dyn ? c->Pm : c->Mm;
   for (int t = 0; t < 2; ++t) b.GR[t] = keep_gr ? (float *)(c->ws + oGR[t]) : nullptr;
+  b.PG = keep_pg ? (float *)(c->ws + oPG) : nullptr;
   b.grows[0] = b.grows[1] = c->Mm;
   b.grows[2] = b.grows[3] = c->Pm;
   for (int p = 0; p < 2; ++p) {
@@ -319,11 +320,6 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   CU(c, cudaHostAlloc((void **)&c->box, sizeof *c->box, cudaHostAllocMapped | cudaHostAllocPortable));
   memset(c->box, 0, sizeof *c->box);
   CU(c, cudaHostGetDevicePointer((void **)&c->box_dev, c->box, 0));
-  if (!(getenv("PBG_REL_ASIDE") && getenv("PBG_REL_ASIDE")[0] == '0')) {        // PBG_REL_ASIDE=0: everything on one stream (for comparisons)
-    CU(c, cudaStreamCreateWithFlags(&c->upd_side, cudaStreamNonBlocking));
-    CU(c, cudaEventCreateWithFlags(&c->ev_upd_fork, cudaEventDisableTiming));
-    CU(c, cudaEventCreateWithFlags(&c->ev_upd_join, cudaEventDisableTiming));
-  }
   c->sum_dev = (double *)(c->ws + oSum);
   c->errflag = &c->box_dev->err;
   c->eval_dev = (double *)(c->ws + oEval);
@@ -368,9 +364,6 @@ extern "C" int pbg_destroy(pbg_context *c) {
   if (c->ev_inputs) cudaEventDestroy(c->ev_inputs);
   if (c->side) cudaStreamDestroy(c->side);
   if (c->part2) cudaStreamDestroy(c->part2);
-  if (c->upd_side) cudaStreamDestroy(c->upd_side);
-  if (c->ev_upd_fork) cudaEventDestroy(c->ev_upd_fork);
-  if (c->ev_upd_join) cudaEventDestroy(c->ev_upd_join);
   if (c->ev_wave) cudaEventDestroy(c->ev_wave);
   if (c->ev_part2) cudaEventDestroy(c->ev_part2);
   for (auto &s : c->spans) { cudaEventDestroy(s.a); cudaEventDestroy(s.b); }
@@ -607,8 +600,7 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
     CU(c, cudaEventRecord(c->ev_sorted[g & 1], c->side));
     return PBG_OK;
   };
-  UpdateScratch us{c->psum, c->hublist, c->hubcnt, &c->hub_turn, c->bigtab, c->upd_side, c->ev_upd_fork, c->ev_upd_join,
-                   stats_out ? c->stats_dev : nullptr, c->sum_dev};
+  UpdateScratch us{c->psum, c->hublist, c->hubcnt, &c->hub_turn, c->bigtab, stats_out ? c->stats_dev : nullptr, c->sum_dev};
   int wave = 0;
   for (int b0 = 0; b0 < num_batches; ++wave) {
     const int kk = kks[wave];

@@ -74,6 +74,7 @@ struct WaveBufs {
   float *GX[4];      int grows[4];   // gradient arrays GN0,GN1,GQ0,GQ1
   float *GR[2];                      // dynamic relations with an operator: per edge the gradient of its operator row,
                                      // [0] rhs table (slots ARR_R0), [1] lhs table (ARR_R1), rows like GQ; null: not kept
+  float *PG;                         // standard relations, diagonal / complex_diagonal: per N1 row its contribution to the operator row's gradient; else null
   float *S[2];                       // scores / coefficient matrices
   // Standard relations: combined coefficient matrices, one per side, [nblk][Mm][Ma]:
   //   A[0][m][j] = (j < Pm ? T0[j][m] : 0) + (m < Pm ? T1[m][j] : 0)   gradient of the lhs rows  = A[0] . N1
@@ -105,10 +106,10 @@ struct WaveBufs {
   // linear / affine operators: R1 = raw rhs rows, R2 = A.x (forward) then g.A (backward), both laid
   // out like N1; dA = per-batch gradient of the operator row [k][opw]
   float *R1, *R2, *dA;
-  float *relpart;                    // standard mode: [k][Cm][D] partial operator gradients
+  float *relpart;                    // standard mode: [blk][D] partial operator gradients
   float *glob[2], *gacc[2];          // global embedding of the lhs / rhs entity type + AsyncAdagrad accumulator, or null
   int glob_shared;                   // both sides are of one entity type: glob[0] == glob[1], one step per batch
-  float *globpart;                   // [blk][side][warp][D] partial sums of the row gradients (global-embedding gradient)
+  float *globpart;                   // [side][blk][D] partial sums of the row gradients (global-embedding gradient)
   int *errflag;                      // device error word (bit 0: id out of range)
 };
 
@@ -400,12 +401,10 @@ int launch_loss(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cud
 int launch_export_scores(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w,
                          float *lhs_pos, float *rhs_pos, float *lhs_neg, float *rhs_neg, cudaStream_t st);
 // What the optimizer kernels of a wave work with.  hubcnt: two sets of counters, 64 ints apart, used in turn (*turn):
-// while one set counts, the kernel behind it clears the other for the next user.  side / fork / join: a second stream and
-// two events for the parts of the update that can run beside the embedding rows' kernels (null: everything on the main
-// stream).  per_batch (may be null) / sum: where the Stats of the wave's batches go.
+// while one set counts, the kernel behind it clears the other for the next user.  per_batch (may be null) / sum: where
+// the Stats of the wave's batches go.
 struct UpdateScratch {
   float *psum; long long *hublist; int *hubcnt; unsigned *turn; long long *bigtab;
-  cudaStream_t side; cudaEvent_t fork, join;
   pbg_batch_stats *per_batch; double *sum;
 };
 int launch_update(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, const unsigned long long *keys, const unsigned int *vals,

@@ -1,9 +1,12 @@
 // Optimizer steps of one wave.
 //
+// First the pull-back: what a gradient slot contributes depends on nothing but the slot's own rows, so one pass over
+// the slots (std_pullback_kernel, dyn_pullback_kernel) takes every gradient row back through comparator.prepare and
+// the relation operator in place, and sums or stores what the operator rows and global vectors get.
+//
 // The sorted occurrence list (pbg_sort.cu) puts all gradient slots of a table row next to each
 // other, in batch order.  A warp keeps a row in registers, and for every batch of the wave that
-// touched it sums the slots' gradients -- each taken back through comparator.prepare and the
-// relation operator on the fly -- and applies one optimizer step:
+// touched it sums the slots' gradient rows and applies one optimizer step:
 //   embedding rows  RowAdagrad   G += mean(g^2); w -= lr g / (sqrt(G) + 1e-10)
 //                                (torchbiggraph/row_adagrad.py:84-96; duplicates are summed first,
 //                                 the `coalesce` of line 83)
@@ -16,130 +19,224 @@
 
 #define UPD_WARPS 8
 
-// Everything needed to pull one gradient slot back to the embedding row it came from.
-// CMPK >= 0 fixes the comparator at compile time, OPK == 0 states that the operator does not scale
-// the gradient (none / translation): the kernels instantiated that way carry no dead branches.
-template <int VEC, int CMPK = -1, int OPK = -1>
-#define REL_UNKNOWN (-(1ll << 62))
-struct SlotGrad {
-  const float *g, *y;      // gradient row, prepared operand row
-  const float *theta;      // operator row or null
-  float dotgy, inv, cf;    // cos: <g', y> and 1/|z|; l2 family: coefficient of y
-  float rc;                // N3 regularizer weight if the slot is an adjusted positive row, else 0
-  bool rcplx;              // ... with the complex modulus (complex_diagonal)
-  int op, cmp, D;
+enum { CK_DOT = 0, CK_COS = 1, CK_L2 = 2 };      // comparator kinds of the pull-back
 
-  // gstage: the gradient row already staged in shared memory (null: read it from global memory)
-  // pre_op: (linear / affine only) stop at the operator output instead of reading the finished
-  //         gradient of the raw row from R2
-  // rl_known: (dynamic relations) the slot's relation id where the caller has looked it up already (REL_UNKNOWN: look
-  //           it up here); reg_known: 1 / 0 = the slot is / is not a regularized row (-1: work it out here)
-  __device__ __forceinline__ void init(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w,
-                                       int a, int blk, int r, int b, int lane, const float *gstage = nullptr,
-                                       bool pre_op = false, long long rl_known = REL_UNKNOWN, int reg_known = -1) {
-    D = d.D; op = OPK == 0 ? PBG_OP_NONE : d.op; cmp = CMPK >= 0 ? CMPK : d.cmp;
-    size_t xr = (size_t)blk * w.xrows[a] + r, gr = (size_t)blk * w.grows[a] + r;
-    y = w.X[a] + xr * d.Dp;
-    g = gstage ? gstage : w.GX[a] + gr * d.Dp;
-    theta = nullptr;
-    cf = 0.f; inv = 1.f; dotgy = 0.f;
-    rc = 0.f; rcplx = d.op == PBG_OP_COMPLEX_DIAGONAL;
-    if (d.reg_coef != 0.f) {
-      // regularized rows: the edges of the chunk (not the uniform negatives) in every operand array
-      if (reg_known >= 0) { if (reg_known) rc = d.reg_coef; }
-      else {
-        BlockInfo rbi = block_info(d, wb, blk);
-        if (r < rbi.n && (a >= ARR_Q0 || r < d.Pm)) rc = d.reg_coef;
-      }
-    }
-    if (d.matrix_op) {
-      op = PBG_OP_NONE;
-      if (a == ARR_N1 && !pre_op) {            // R2 already holds d(loss)/d(raw row)
-        if (!gstage) g = w.R2 + gr * d.Dp;
-        cmp = PBG_CMP_DOT;
-        return;
-      }
-    }
-    if (OPK != 0 && op != PBG_OP_NONE) {
-      if (!d.dynamic) {
-        if ((a == ARR_N1 || a == ARR_Q0) && w.theta[0]) theta = w.theta[0] + (size_t)wb.rel[b] * D;
-      } else if (a == ARR_Q0 || a == ARR_Q1) {
-        long long rl = rl_known;
-        if (rl == REL_UNKNOWN) {
-          BlockInfo bi = block_info(d, wb, blk);
-          rl = w.rel[bi.e0 + r];
-        }
-        const float *tab = w.theta[a == ARR_Q0 ? 0 : 1];
-        if (tab && rl >= 0 && rl < d.num_rels) theta = tab + (size_t)rl * D;
-      }
-    }
-    const int cmp = CMPK >= 0 ? CMPK : this->cmp;
-    if (cmp >= PBG_CMP_L2) {
-      // dynamic: ga = T.N - rowsum(T) a ;  gb = T^T.Q - colsum(T) b.  standard: g = A.N' - rowsum(A) y
-      const float *cp = (a == ARR_N0) ? w.coef[0] : (a == ARR_N1) ? w.coef[1] : (a == ARR_Q0) ? w.coef[2] : w.coef[3];
-      cf = cp[gr];
-    } else if (cmp == PBG_CMP_COS) {
-      inv = w.aux[a][xr];
-      float s = 0.f;
+// v = gradient of the operator output behind slot (a, blk, r): the contraction's row, plus the regularizer's own
+// gradient on the rows it covers (reg), back through comparator.prepare -- cos: (g - y <g, y>) / |z|; l2 family: the
+// row's own |y|^2 term (dynamic: ga = T.N - rowsum(T) a, gb = T^T.Q - colsum(T) b; standard: g = A.N' - rowsum(A) y).
+template <int VEC, int CK>
+__device__ __forceinline__ void gz_row(float4 (&v)[VEC], const WaveDims &d, const WaveBufs &w, int a, int blk, int r, int lane, bool reg) {
+  const int D = d.D;
+  const size_t xr = (size_t)blk * w.xrows[a] + r, gr = (size_t)blk * w.grows[a] + r;
+  const float *y = w.X[a] + xr * d.Dp, *g = w.GX[a] + gr * d.Dp;
+  float4 yv[VEC];
 #pragma unroll
-      for (int c = 0; c < VEC; ++c) {
-        int dd = c * 128 + lane * 4;
-        if (dd < D) s += f4dot(graw(dd), yv(dd));
-      }
-      dotgy = warp_sum(s);
+  for (int c = 0; c < VEC; ++c) {
+    const int dd = c * 128 + lane * 4;
+    v[c] = dd < D ? ld4(g + dd) : f4zero();
+    if (CK != CK_DOT) yv[c] = dd < D ? ld4(y + dd) : f4zero();
+  }
+  const float cf = CK == CK_L2 ? w.coef[a][gr] : 0.f, inv = CK == CK_COS ? w.aux[a][xr] : 1.f;
+  if (reg) {
+#pragma unroll
+    for (int c = 0; c < VEC; ++c) {
+      const int dd = c * 128 + lane * 4;
+      if (dd < D) v[c] = v[c] + n3_grad4(y, dd, D, d.op == PBG_OP_COMPLEX_DIAGONAL) * d.reg_coef;
     }
   }
-  __device__ __forceinline__ float4 yv(int dd) const {
-    return ld4(y + dd);
+  if (CK == CK_COS) {
+    float s = 0.f;
+#pragma unroll
+    for (int c = 0; c < VEC; ++c)     // rounding order spelled out: it must not depend on what the compiler contracts around it
+      s += __fmaf_rn(v[c].w, yv[c].w, __fmaf_rn(v[c].z, yv[c].z, __fmaf_rn(v[c].x, yv[c].x, __fmul_rn(v[c].y, yv[c].y))));
+    s = warp_sum(s);
+#pragma unroll
+    for (int c = 0; c < VEC; ++c) v[c] = (v[c] - yv[c] * s) * inv;
+  } else if (CK == CK_L2) {
+#pragma unroll
+    for (int c = 0; c < VEC; ++c) v[c] = v[c] - yv[c] * cf;
   }
-  // gradient w.r.t. the operator output z at elements [dd, dd+4)
-  // gradient that reaches the prepared row: from the contractions, plus the regularizer's own
-  __device__ __forceinline__ float4 graw(int dd) const {
-    float4 v = ld4(g + dd);
-    if (rc != 0.f) v = v + n3_grad4(y, dd, D, rcplx) * rc;
-    return v;
-  }
-  __device__ __forceinline__ float4 gz(int dd) const {
-    float4 v = graw(dd);
-    const int cmp = CMPK >= 0 ? CMPK : this->cmp;
-    if (cmp >= PBG_CMP_L2) v = v - yv(dd) * cf;
-    else if (cmp == PBG_CMP_COS) v = (v - yv(dd) * dotgy) * inv;   // (g - y <g,y>) / |z|
-    return v;
-  }
-  // gradient w.r.t. the embedding row at elements [dd, dd+4)
-  __device__ __forceinline__ float4 gx(int dd) const {
-    float4 v = gz(dd);
-    if (OPK == 0 || theta == nullptr || op == PBG_OP_TRANSLATION) return v;
-    float4 t = ld4(theta + dd);
-    if (op == PBG_OP_DIAGONAL) return v * t;
-    int h = D >> 1;
-    int dp = dd < h ? dd + h : dd - h;
-    float4 vp = gz(dp), tp = ld4(theta + dp);
-    // gx_re = g_re p_re + g_im p_im ;  gx_im = -g_re p_im + g_im p_re
-    return dd < h ? v * t + vp * tp : v * tp - vp * t;
-  }
-};
+}
 
-// d(loss)/d(operator row) contributed by one slot whose operand went through the operator:
-// needs the gradient at the operator output (gz) and the raw embedding row x.
-template <int VEC, int CMPK = -1>
-__device__ __forceinline__ float4 op_param_grad(const SlotGrad<VEC, CMPK, -1> &sg, const float *x, float xscale, int dd,
-                                                const float *xadd = nullptr) {
-  // xadd: global embedding added to the raw row before the operator (null: none)
-  float4 v = sg.gz(dd);
-  if (sg.op == PBG_OP_TRANSLATION) return v;
+// Back through the operator: v (gradient of its output) becomes the gradient of the raw row, pg the contribution to
+// the operator row.  x: the raw row, used as x * xs (+ xadd).  complex_diagonal pairs element d with d +- D/2, which
+// another lane holds: v goes through `part` (D floats of the warp's own shared memory), the partners of x and theta are
+// read again (L1 / L2).
+template <int VEC>
+__device__ __forceinline__ void operator_back(float4 (&v)[VEC], float4 (&pg)[VEC], const WaveDims &d, const float *theta, const float *x,
+                                              float xs, const float *xadd, float *part, int lane) {
+  const int D = d.D;
   auto raw = [&](int e) {
-    float4 r = ld4(x + e) * xscale;
-    if (xadd) r = r + ld4(xadd + e);
-    return r;
+    float4 q = ld4(x + e) * xs;
+    if (xadd) q = q + ld4(xadd + e);
+    return q;
   };
-  float4 xv = raw(dd);
-  if (sg.op == PBG_OP_DIAGONAL) return v * xv;
-  int h = sg.D >> 1;
-  int dp = dd < h ? dd + h : dd - h;
-  float4 vp = sg.gz(dp), xp = raw(dp);
-  // d real = g_re a_re + g_im a_im ;  d imag = -g_re a_im + g_im a_re
-  return dd < h ? v * xv + vp * xp : v * xp - vp * xv;
+  if (d.op == PBG_OP_TRANSLATION) {
+#pragma unroll
+    for (int c = 0; c < VEC; ++c) pg[c] = v[c];
+    return;
+  }
+  if (d.op == PBG_OP_DIAGONAL) {
+#pragma unroll
+    for (int c = 0; c < VEC; ++c) {
+      const int dd = c * 128 + lane * 4;
+      if (dd < D) { pg[c] = v[c] * raw(dd); v[c] = v[c] * ld4(theta + dd); }
+    }
+    return;
+  }
+  const int h = D >> 1;
+  __syncwarp();                                              // the previous row's partners have been read
+#pragma unroll
+  for (int c = 0; c < VEC; ++c) {
+    const int dd = c * 128 + lane * 4;
+    if (dd < D) st4(part + dd, v[c]);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < VEC; ++c) {
+    const int dd = c * 128 + lane * 4;
+    if (dd < D) {
+      const int dp = dd < h ? dd + h : dd - h;
+      const float4 vp = ld4(part + dp), xv = raw(dd), xp = raw(dp), t = ld4(theta + dd), tp = ld4(theta + dp);
+      // d real = g_re a_re + g_im a_im ;  d imag = -g_re a_im + g_im a_re
+      pg[c] = dd < h ? v[c] * xv + vp * xp : v[c] * xp - vp * xv;
+      // gx_re = g_re p_re + g_im p_im ;  gx_im = -g_re p_im + g_im p_re
+      v[c] = dd < h ? v[c] * t + vp * tp : v[c] * tp - vp * t;
+    }
+  }
+}
+
+// Standard relations: the pull-back of a wave's gradient slots, one warp per row of a chunk block and side -- the
+// gradient of the raw row written over the slot's own gradient row.  Under diagonal and complex_diagonal the row's
+// contribution to the relation's operator row goes to PG beside it (under a translation it IS the gradient row).
+// first_side / sides: what is left out needs no change.  (One warp per row and no sums in here: a kernel that also
+// summed per chunk block ran 20 CTAs on a single batch.)
+template <int VEC, int CK>
+__global__ void __launch_bounds__(32 * UPD_WARPS) std_pullback_kernel(WaveDims d, WaveBatches wb, WaveBufs w, int side0) {
+  extern __shared__ __align__(16) float wpart[];             // [UPD_WARPS][VEC * 128]
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const int side = side0 + blockIdx.y, a = side ? ARR_N1 : ARR_N0;
+  const long long item = (long long)blockIdx.x * UPD_WARPS + wl;
+  if (item >= (long long)d.nblk * d.Mm) return;
+  const int lb = (int)(item / d.Mm), r = (int)(item - (long long)lb * d.Mm), blk = d.blk0 + lb;
+  if (side == 1 && d.matrix_op) return;                      // linear / affine: R2 holds the gradient of the raw row already
+  const BlockInfo bi = block_info(d, wb, blk);
+  if (bi.n <= 0) return;
+  const long long row = slot_row(d, wb, w, bi, side, r);
+  if (row < 0 || row >= d.n_rows[side]) return;
+  const int D = d.D;
+  float4 v[VEC], pg[VEC];
+  gz_row<VEC, CK>(v, d, w, a, blk, r, lane, d.reg_coef != 0.f && r < bi.n && r < d.Pm);
+  if (side == 1 && w.PG) {
+    const float xs = d.max_norm > 0.f ? w.rscale[(size_t)blk * d.Mm + r] : 1.0f;   // the raw row entered the operator scaled
+    operator_back<VEC>(v, pg, d, w.theta[0] + (size_t)wb.rel[bi.b] * D, w.W[1] + (size_t)row * D, xs, w.glob[1], wpart + (size_t)wl * VEC * 128, lane);
+    float *out = w.PG + ((size_t)blk * d.Mm + r) * d.Dp;
+#pragma unroll
+    for (int c = 0; c < VEC; ++c) { const int dd = c * 128 + lane * 4; if (dd < D) st4(out + dd, pg[c]); }
+  }
+  __syncwarp();
+  float *out = w.GX[a] + ((size_t)blk * w.grows[a] + r) * d.Dp;
+#pragma unroll
+  for (int c = 0; c < VEC; ++c) { const int dd = c * 128 + lane * 4; if (dd < D) st4(out + dd, v[c]); }
+}
+
+// The vectors that every row of a batch shares in standard relations: the relation's operator row, and the vector of
+// each entity type (config.global_emb: added to every row of the type before the operator, so its gradient is the sum of
+// the raw rows' gradients).  Both steps ride on launches that are there anyway, as CTAs beside the embedding rows' work
+// -- what they step is read by nothing before the next wave -- where they were four kernels of 14 to 27 us on a batch
+// of 1000 edges at dimension 128, two of them a single CTA:
+//   param_sums   beside the tiles: CTA (vector, chunk block, 128 columns) adds up the block's rows, warp u rows u, u + 8, ...
+//                (two such sequences per warp here), the eight sums in order, into one partial row per block
+//   param_step   beside the big hub rows: adds up a batch's partial rows and takes the dense AsyncAdagrad steps batch
+//                after batch (torchbiggraph/async_adagrad.py:75-85, train_cpu.py:215-230)
+// kinds: 0 operator row, 1 / 2 vector of the lhs / rhs entity type (one vector for both sides: two sums, one step)
+struct ParamJob { int sums, sum_kind[3], steps, step_kind[3]; float lr; };
+static inline int param_sum_ctas(const WaveDims &d, const ParamJob &job) { return job.sums * d.nblk * ((d.D + 127) / 128); }
+static inline int param_step_ctas(const WaveDims &d, const ParamJob &job) { return job.steps * ((d.D + 31) / 32); }
+
+// (128 threads)
+__device__ __forceinline__ void param_sums(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, const ParamJob &job, int cta, float *sm) {
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const int cols = (d.D + 127) / 128;
+  const int dd = (cta % cols) * 128 + lane * 4;
+  const int blk = cta / cols % d.nblk, kind = job.sum_kind[cta / cols / d.nblk];
+  const int side = kind == 1 ? 0 : 1;
+  const BlockInfo bi = block_info(d, wb, blk);
+  const float *src = kind == 0 ? (w.PG ? w.PG : w.GX[ARR_N1]) : kind == 1 ? w.GX[ARR_N0] : d.matrix_op ? w.R2 : w.GX[ARR_N1];
+  src += (size_t)blk * d.Mm * d.Dp + dd;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int y = wl + 4 * h;
+    float4 s = f4zero();
+    if (bi.n > 0 && dd < d.D) {
+      for (int r0 = y; r0 < d.Mm; r0 += 32) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int r = r0 + 8 * u;
+          const long long row = r < d.Mm ? slot_row(d, wb, w, bi, side, r) : -1;
+          v[u] = row >= 0 && row < d.n_rows[side] ? ld4(src + (size_t)r * d.Dp) : f4zero();
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s = s + v[u];
+      }
+      if (kind == 0 && y == 0 && d.reg_coef != 0.f)
+        // N3 regularizer on the relation's parameters: sum(params^3) * number of chunks
+        // (regularizers.py:88-92), i.e. once per chunk block; theta is still the wave's snapshot here
+        s = s + n3_grad4(w.theta[0] + (size_t)wb.rel[bi.b] * d.D, dd, d.D, d.op == PBG_OP_COMPLEX_DIAGONAL) * d.reg_coef;
+    }
+    st4(sm + y * 128 + lane * 4, s);
+  }
+  __syncthreads();
+  if (wl == 0 && dd < d.D) {
+    float4 t = ld4(sm + lane * 4);
+#pragma unroll
+    for (int u = 1; u < 8; ++u) t = t + ld4(sm + u * 128 + lane * 4);
+    float *out = kind == 0 ? w.relpart : w.globpart + (kind == 2 ? (size_t)d.nblk * d.D : 0);
+    st4(out + (size_t)blk * d.D + dd, t);
+  }
+}
+
+// (256 threads; sm: PBG_KMAX * 32 floats)
+__device__ __forceinline__ void param_step(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, const ParamJob &job, int cta, float *sm) {
+  const int colctas = (d.D + 31) / 32;
+  const int kind = job.step_kind[cta / colctas];
+  const int col = threadIdx.x & 31, y = threadIdx.x >> 5, dd = (cta % colctas) * 32 + col;
+  const float *part = (kind == 0 ? w.relpart : w.globpart + (kind == 2 ? (size_t)d.nblk * d.D : 0)) + dd;
+  const float *part2 = kind == 1 && w.glob_shared ? w.globpart + (size_t)d.nblk * d.D + dd : nullptr;   // one vector: both sides' gradients add up
+  if (dd < d.D) {
+    for (int b = y; b < d.k; b += UPD_WARPS) {
+      float s = 0.f, s2 = 0.f;
+#pragma unroll 4
+      for (int c = 0; c < d.Cm; ++c) s += part[((size_t)b * d.Cm + c) * d.D];
+      if (part2) {
+#pragma unroll 4
+        for (int c = 0; c < d.Cm; ++c) s2 += part2[((size_t)b * d.Cm + c) * d.D];
+        s += s2;
+      }
+      sm[b * 32 + col] = s;
+    }
+  }
+  __syncthreads();
+  if (y != 0 || dd >= d.D) return;
+  float *acc = kind == 0 ? w.acc[0] : w.gacc[kind - 1], *val = kind == 0 ? w.theta[0] : w.glob[kind - 1];
+  // the row of the relation in hand stays in registers (a global vector is one row)
+  int cur = -1;
+  float a = 0.f, v = 0.f;
+  for (int b = 0; b < d.k; ++b) {
+    if (wb.n[b] <= 0) continue;
+    const int row = kind == 0 ? wb.rel[b] : 0;
+    if (kind == 0 && (row < 0 || row >= d.num_rels)) continue;
+    const float g = sm[b * 32 + col];
+    if (row != cur) {
+      if (cur >= 0) { acc[(size_t)cur * d.D + dd] = a; val[(size_t)cur * d.D + dd] = v; }
+      cur = row;
+      a = acc[(size_t)row * d.D + dd]; v = val[(size_t)row * d.D + dd];
+    }
+    a += g * g;
+    v -= job.lr * g / (sqrtf(a) + PBG_ADAGRAD_EPS);
+  }
+  if (cur >= 0) { acc[(size_t)cur * d.D + dd] = a; val[(size_t)cur * d.D + dd] = v; }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -253,84 +350,43 @@ struct RowState {
   }
 };
 
-// acc += the contribution of one slot to its row's gradient
-template <int VEC, int RULE, int CMPK = -1, int OPK = -1>
-__device__ __forceinline__ void add_slot(float4 (&acc)[VEC], const WaveDims &d, const WaveBatches &wb,
-                                         const WaveBufs &w, const Occ &oc, int lane, const float *gstage = nullptr,
-                                         long long rl_known = REL_UNKNOWN, int reg_known = -1) {
-  const int D = d.D;
-  if (RULE == RULE_EMB) {
-    SlotGrad<VEC, CMPK, OPK> sg;
-    sg.init(d, wb, w, oc.a, oc.blk, oc.r, oc.b, lane, gstage, false, rl_known, reg_known);
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) {
-      int dd = c * 128 + lane * 4;
-      if (dd < D) acc[c] = acc[c] + sg.gx(dd);
-    }
-  } else {
-    SlotGrad<VEC, CMPK, -1> sg;
-    int qa = oc.a == ARR_R0 ? ARR_Q0 : ARR_Q1;             // slot that carried the operator
-    int na = oc.a == ARR_R0 ? ARR_N1 : ARR_N0;             // its operator-free copy (raw row)
-    sg.init(d, wb, w, qa, oc.blk, oc.r, oc.b, lane, nullptr, false, rl_known, reg_known);
-    size_t nrow = (size_t)oc.blk * w.xrows[na] + oc.r;
-    const float *x = w.X[na] + nrow * d.Dp;
-    float xscale = (CMPK >= 0 ? CMPK : d.cmp) == PBG_CMP_COS ? 1.0f / w.aux[na][nrow] : 1.0f;
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) {
-      int dd = c * 128 + lane * 4;
-      if (dd < D) {
-        acc[c] = acc[c] + op_param_grad<VEC, CMPK>(sg, x, xscale, dd);
-        // N3 regularizer on the edge's own parameter row (still as the wave found it in global memory)
-        if (d.reg_coef != 0.f && sg.theta) acc[c] = acc[c] + n3_grad4(sg.theta, dd, D, d.op == PBG_OP_COMPLEX_DIAGONAL) * d.reg_coef;
-      }
-    }
-  }
-}
-
 // Embedding rows: 4 warps per CTA, each with TILE row buffers in shared memory that it fills with
 // bulk asynchronous copies (cp.async.bulk, completion on the warp's mbarrier): the gradient rows
 // of a whole tile are in flight at once instead of one dependent 16-byte-per-lane load at a time.
 #define TILE_WARPS_EMB 4
 #define UPD_WAIT_LIMIT 4000000
 
-// MODE 1 (plain): the slot's gradient row is already the gradient of the table row (dot comparator, no
-// operator or a translation) -- compiled without the comparator / operator pull-back, whose
-// predicated-off copies in the unrolled loops cost more issue slots than the additions themselves.
-// MODE 2: cos comparator with no operator or a translation, comparator fixed at compile time.
-// MODE 3: dot comparator fixed at compile time, any operator (the pull-back through complex_diagonal
-// evaluates the comparator's part twice per element).
-// MODE 0: everything decided at run time.
-// Resident CTAs per SM: rows of up to 256 floats with an operator or a non-trivial comparator are bound by the latency
-// of a slot's chain of loads, not by bytes, and gain from twice the warps at the price of a few dozen bytes of spills
-// (dimension 200, dynamic complex_diagonal / l2: update 55.8 -> 52.5 ms per 2.16 M edges); the wide rows stay at the
-// register count that keeps them spill-free.
-template <int VEC, int RULE, int MODE>
-__global__ void __launch_bounds__(32 * (RULE == RULE_EMB ? TILE_WARPS_EMB : UPD_WARPS), RULE == RULE_EMB ? (VEC == 2 ? 6 : 3) : (VEC == 2 ? 4 : 2))
+// The operator rows' slots are staged from GR (dyn_pullback_kernel), eight warps per CTA.
+// Resident CTAs per SM: rows of up to 256 floats are bound by the latency of a slot's chain of loads, not by bytes, and
+// gain from twice the warps at the price of a few dozen bytes of spills (dimension 200: update 55.8 -> 52.5 ms per 2.16 M
+// edges); the wide rows stay at the register count that keeps them spill-free.
+template <int VEC, int RULE>
+struct TileWarps { enum { N = RULE == RULE_EMB ? TILE_WARPS_EMB : VEC > 8 ? UPD_WARPS / 2 : UPD_WARPS }; };
+
+template <int VEC, int RULE>
+__global__ void __launch_bounds__(32 * TileWarps<VEC, RULE>::N, RULE == RULE_EMB ? (VEC == 2 ? 6 : 3) : (VEC == 2 ? 4 : 2))
 tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys,
                    const unsigned int *__restrict__ vals, float lr, float *__restrict__ psum,
-                   long long *__restrict__ hublist, int *__restrict__ hubcnt) {
-  constexpr int WARPS = RULE == RULE_EMB ? TILE_WARPS_EMB : UPD_WARPS;
-  constexpr bool PLAIN = MODE == 1;
-  constexpr bool STAGED = RULE == RULE_EMB || PLAIN;          // (the plain form of the operator rows stages its GR rows too)
-  extern __shared__ __align__(128) float stage_all[];        // [WARPS][TILE][Dp] (STAGED only)
+                   long long *__restrict__ hublist, int *__restrict__ hubcnt, ParamJob job, int aside) {
+  constexpr int WARPS = TileWarps<VEC, RULE>::N;
+  extern __shared__ __align__(128) float stage_all[];        // [WARPS][TILE][Dp]
   __shared__ __align__(8) unsigned long long sbar[WARPS];
   const unsigned FULL = 0xffffffffu;
   const unsigned long long SENT = ~0ull;
   int lane = threadIdx.x & 31;
   const int wl = threadIdx.x >> 5;
-  long long t0 = ((long long)blockIdx.x * WARPS + wl) * TILE;
+  if (RULE == RULE_EMB && blockIdx.x < aside) { param_sums(d, wb, w, job, blockIdx.x, stage_all); return; }
+  long long t0 = ((long long)(blockIdx.x - aside) * WARPS + wl) * TILE;
   if (t0 >= d.nocc) return;
-  float *stage = STAGED ? stage_all + (size_t)wl * TILE * d.Dp : nullptr;
+  float *stage = stage_all + (size_t)wl * TILE * d.Dp;
   const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&sbar[wl]);
   uint32_t phase = 0;
   int staged_lo = 0, staged_hi = 0;                           // window slots whose rows are in `stage`
-  if (STAGED) {
-    if (lane == 0) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar));
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncwarp();
+  if (lane == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  __syncwarp();
   const int D = d.D;
   const float invD = 1.0f / (float)D;
   const unsigned long long lo = RULE == RULE_EMB ? 0ull : d.key_rel_base;
@@ -340,37 +396,19 @@ tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
   unsigned long long kB = pb < d.nocc ? keys[pb] : SENT;
   unsigned int vB = pb < d.nocc ? vals[pb] : 0u;
   const int bB = (int)(vB / (unsigned int)d.spb);              // batch of this lane's slot
-  // Every lane resolves its own slot once -- the integer divisions of the decoding, and with dynamic relations the
-  // relation id of the slot's edge (a load that the operator row's address depends on) -- so that the slot-by-slot
-  // loop below starts from shuffles instead of redoing both as one dependent chain per slot.
-  Occ ocB; ocB.b = bB; ocB.a = 0; ocB.blk = 0; ocB.r = 0;
-  long long rlB = REL_UNKNOWN;
-  int regB = -1;
-  if ((!PLAIN || RULE == RULE_REL) && pb < d.nocc && kB < hi) {
-    ocB = occ_decode(d, (int)vB);
-    if (!PLAIN && (d.dynamic || d.reg_coef != 0.f)) {
-      const int qa = ocB.a == ARR_R0 ? ARR_Q0 : ocB.a == ARR_R1 ? ARR_Q1 : ocB.a;
-      BlockInfo bi = block_info(d, wb, ocB.blk);
-      if (d.dynamic && d.op != PBG_OP_NONE && (qa == ARR_Q0 || qa == ARR_Q1) && ocB.r < bi.n) rlB = w.rel[bi.e0 + ocB.r];
-      regB = (ocB.r < bi.n && (qa >= ARR_Q0 || ocB.r < d.Pm)) ? 1 : 0;
-    }
-  }
   if (__shfl_sync(FULL, kB, TILE - 1) < lo) return;          // tile holds only the other rule's rows
   // Copies the gradient rows of window slots j0 .. j0+cnt-1 (cnt <= TILE) into the stage buffers and
   // waits for them; the wait is bounded (bit 1 of the error word when it runs out).
   auto stage_rows = [&](int j0, int cnt) {
     __syncwarp();                                            // everyone is done with the old rows
-    const int src = j0 + (lane < cnt ? lane : 0);
-    Occ oc;
-    oc.a = __shfl_sync(FULL, ocB.a, src); oc.blk = __shfl_sync(FULL, ocB.blk, src); oc.r = __shfl_sync(FULL, ocB.r, src);
-    unsigned int v = __shfl_sync(FULL, vB, src);
+    unsigned int v = __shfl_sync(FULL, vB, j0 + (lane < cnt ? lane : 0));
     if (lane == 0) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"((uint32_t)(cnt * d.D * 4)) : "memory");
     }
     __syncwarp();
     if (lane < cnt) {
-      if (PLAIN && RULE == RULE_EMB) oc = occ_decode(d, (int)v);   // the plain embedding kernel decodes only what it stages
+      const Occ oc = occ_decode(d, (int)v);
       const float *g;
       if (RULE == RULE_REL) g = w.GR[oc.a == ARR_R1 ? 1 : 0] + ((size_t)oc.blk * d.Pm + oc.r) * d.Dp;
       else {
@@ -404,8 +442,8 @@ tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
     }
     int nvalid = __popc(__ballot_sync(FULL, lane < TILE && kB < hi));
     if (nvalid > 0) stage_rows(0, nvalid);
-  } else if (STAGED) {
-    // operator rows, plain form: the tile's slots of this rule (they follow the embedding rows' slots in the sorted list)
+  } else {
+    // operator rows: the tile's slots of this rule (they follow the embedding rows' slots in the sorted list)
     const int first = __popc(__ballot_sync(FULL, lane < TILE && kB < lo));
     const int nvalid = __popc(__ballot_sync(FULL, lane < TILE && kB >= lo && kB < hi));
     if (nvalid > 0) stage_rows(first, nvalid);
@@ -433,12 +471,8 @@ tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
     int cur_b = -1, run_start = 0;
     for (int j = i; j <= i + nproc; ++j) {
       bool in = j < i + nproc;
-      Occ oc;
-      if (in) {
-        oc.b = __shfl_sync(FULL, ocB.b, j);
-        if (!PLAIN || RULE == RULE_REL) { oc.a = __shfl_sync(FULL, ocB.a, j); oc.blk = __shfl_sync(FULL, ocB.blk, j); oc.r = __shfl_sync(FULL, ocB.r, j); }
-      }
-      if (cur_b >= 0 && (!in || oc.b != cur_b)) {             // a batch of this row is complete
+      const int b = in ? __shfl_sync(FULL, bB, j) : -1;
+      if (cur_b >= 0 && b != cur_b) {                                     // a batch of this row is complete
         if (hub) {
           float *dst = psum + (size_t)(t0 + run_start) * d.Dp;
 #pragma unroll
@@ -453,28 +487,16 @@ tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
         for (int c = 0; c < VEC; ++c) acc[c] = f4zero();
       }
       if (!in) break;
-      if (oc.b != cur_b) { cur_b = oc.b; run_start = j; }
-      const float *gs = nullptr;
-      if (STAGED) {
-        if (j >= staged_hi) {                                 // a short row that runs past the tile
-          int left = i + nproc - j;
-          stage_rows(j, left < TILE ? left : TILE);
-        }
-        gs = stage + (size_t)(j - staged_lo) * d.Dp;
+      if (b != cur_b) { cur_b = b; run_start = j; }
+      if (j >= staged_hi) {                                   // a short row that runs past the tile
+        int left = i + nproc - j;
+        stage_rows(j, left < TILE ? left : TILE);
       }
-      if (PLAIN) {
-        // the staged row: the slot's gradient row, or for operator rows the edge's row of GR (dyn_pullback_kernel)
+      const float *gs = stage + (size_t)(j - staged_lo) * d.Dp;
 #pragma unroll
-        for (int c = 0; c < VEC; ++c) {
-          int dd = c * 128 + lane * 4;
-          if (dd < D) acc[c] = acc[c] + ld4(gs + dd);
-        }
-      } else {
-        const long long rl = __shfl_sync(FULL, rlB, j);
-        const int reg = __shfl_sync(FULL, regB, j);
-        if (MODE == 2) add_slot<VEC, RULE, PBG_CMP_COS, 0>(acc, d, wb, w, oc, lane, gs, rl, reg);
-        else if (MODE == 3) add_slot<VEC, RULE, PBG_CMP_DOT, -1>(acc, d, wb, w, oc, lane, gs, rl, reg);
-        else add_slot<VEC, RULE>(acc, d, wb, w, oc, lane, gs, rl, reg);
+      for (int c = 0; c < VEC; ++c) {
+        int dd = c * 128 + lane * 4;
+        if (dd < D) acc[c] = acc[c] + ld4(gs + dd);
       }
     }
     if (!hub) rs.store(D, lane);
@@ -575,11 +597,16 @@ template <int VEC>
 __global__ void __launch_bounds__(32 * UPD_WARPS)
 hub_reduce_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys, const unsigned int *__restrict__ vals,
                   float *__restrict__ psum, const long long *__restrict__ hublist, const int *__restrict__ hubcnt,
-                  int *__restrict__ hubcnt_next, long long *__restrict__ bigtab, int stats, pbg_batch_stats *per_batch, double *sum) {
+                  int *__restrict__ hubcnt_next, long long *__restrict__ bigtab, int aside, ParamJob job, pbg_batch_stats *per_batch, double *sum) {
   extern __shared__ __align__(16) float part[];              // [UPD_WARPS][VEC * 128]
   if (blockIdx.x == 0 && threadIdx.x < 2) hubcnt_next[threadIdx.x] = 0;      // its last reader is behind us in the stream
-  if (stats && blockIdx.x < d.k) { batch_stats(d, wb, w, blockIdx.x, per_batch, sum); return; }
-  const int cta0 = stats ? d.k : 0;
+  // the first CTAs of the embedding rows' launch (aside) have other work
+  int cta0 = 0;
+  if (aside) {
+    cta0 = d.k + job.steps * ((d.D + 31) / 32);               // param_step_ctas
+    if (blockIdx.x < d.k) { batch_stats(d, wb, w, blockIdx.x, per_batch, sum); return; }
+    if (blockIdx.x < cta0) { param_step(d, wb, w, job, blockIdx.x - d.k, part); return; }
+  }
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int D = d.D;
   const long long *biglist = hub_biglist(hublist, d.nocc);
@@ -801,100 +828,10 @@ hub_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long lo
   }
 }
 
-// Standard relations: every rhs row of a batch went through the same operator row.  Stage 1: one
-// CTA per chunk sums the parameter gradient of its rows (N1 slots: chunk rows + uniform rows)
-// into relpart[b][c][D] (the eight warps added up in shared memory); the raw rows are re-read from the rhs table, which this wave has not
-// updated yet.  Stage 2 (relupdate_std_kernel) adds the chunks up and steps theta, batch by batch.
-template <int VEC>
-__global__ void __launch_bounds__(32 * UPD_WARPS) relgrad_std_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
-  int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  int blk = blockIdx.x;
-  BlockInfo bi = block_info(d, wb, blk);
-  const int D = d.D;
-  float4 acc[VEC];
-#pragma unroll
-  for (int c = 0; c < VEC; ++c) acc[c] = f4zero();
-  int items = d.Mm;                                          // the chunk's rhs rows: GN1 slots
-  if (bi.n > 0) {
-    for (int it = wl; it < items; it += UPD_WARPS) {
-      int a = ARR_N1;
-      int r = it;
-      long long row = slot_row(d, wb, w, bi, 1, r);
-      if (row < 0 || row >= d.n_rows[1]) continue;
-      SlotGrad<VEC> sg;
-      sg.init(d, wb, w, a, blk, r, bi.b, lane);
-      const float *x = w.W[1] + (size_t)row * D;
-      const float xsc = d.max_norm > 0.f ? w.rscale[(size_t)blk * d.Mm + r] : 1.0f;    // the raw row entered the operator scaled
-#pragma unroll
-      for (int c = 0; c < VEC; ++c) {
-        int dd = c * 128 + lane * 4;
-        if (dd < D) acc[c] = acc[c] + op_param_grad<VEC>(sg, x, xsc, dd, w.glob[1]);
-      }
-    }
-  }
-  if (d.reg_coef != 0.f && wl == 0 && bi.n > 0) {
-    // N3 regularizer on the relation's parameters: sum(params^3) * number of chunks
-    // (regularizers.py:88-92), i.e. once per chunk block; theta is still the wave's snapshot here
-    const float *th = w.theta[0] + (size_t)wb.rel[bi.b] * D;
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) {
-      int dd = c * 128 + lane * 4;
-      if (dd < D) acc[c] = acc[c] + n3_grad4(th, dd, D, d.op == PBG_OP_COMPLEX_DIAGONAL) * d.reg_coef;
-    }
-  }
-  // the eight warps' sums are added in warp order: one partial row per chunk block, so that the
-  // single-CTA stage 2 reads Cm rows per batch instead of 8 Cm (its loads are one dependent chain)
-  extern __shared__ __align__(16) float wpart_raw[];
-  float (*wpart)[VEC * 128] = reinterpret_cast<float (*)[VEC * 128]>(wpart_raw);
-#pragma unroll
-  for (int c = 0; c < VEC; ++c) st4(&wpart[wl][c * 128 + lane * 4], acc[c]);
-  __syncthreads();
-  float *out = w.relpart + (size_t)blk * D;
-  for (int dd = threadIdx.x * 4; dd < D; dd += 4 * blockDim.x) {
-    float4 t = ld4(&wpart[0][dd]);
-#pragma unroll
-    for (int u = 1; u < UPD_WARPS; ++u) t = t + ld4(&wpart[u][dd]);
-    st4(out + dd, t);
-  }
-}
-
-__global__ void relupdate_std_kernel(WaveDims d, WaveBatches wb, WaveBufs w, float lr) {
-  int dd = blockIdx.x * blockDim.x + threadIdx.x;
-  if (dd >= d.D) return;
-  // The gradient sums of all batches first: these loads do not depend on the steps, and with the
-  // batch loop innermost they are all in flight together (one dependent chain of k * Cm loads took
-  // 76 us per wave).  Chunks are added in the same order as before.
-  float g[PBG_KMAX];
-#pragma unroll
-  for (int b = 0; b < PBG_KMAX; ++b) g[b] = 0.f;
-  for (int c = 0; c < d.Cm; ++c) {
-#pragma unroll
-    for (int b = 0; b < PBG_KMAX; ++b)
-      if (b < d.k) g[b] += w.relpart[((size_t)b * d.Cm + c) * d.D + dd];
-  }
-  // the steps in batch order; the row of the relation in hand stays in registers
-  int cur = -1;
-  float a = 0.f, th = 0.f;
-#pragma unroll
-  for (int b = 0; b < PBG_KMAX; ++b) {
-    if (b >= d.k || wb.n[b] <= 0) continue;
-    int rl = wb.rel[b];
-    if (rl < 0 || rl >= d.num_rels) continue;
-    if (rl != cur) {
-      if (cur >= 0) { w.acc[0][(size_t)cur * d.D + dd] = a; w.theta[0][(size_t)cur * d.D + dd] = th; }
-      cur = rl;
-      a = w.acc[0][(size_t)rl * d.D + dd]; th = w.theta[0][(size_t)rl * d.D + dd];
-    }
-    a += g[b] * g[b];
-    th -= lr * g[b] / (sqrtf(a) + PBG_ADAGRAD_EPS);
-  }
-  if (cur >= 0) { w.acc[0][(size_t)cur * d.D + dd] = a; w.theta[0][(size_t)cur * d.D + dd] = th; }
-}
-
 // linear / affine operators: turns GN1 rows (gradient w.r.t. the prepared operand) into the
 // gradient w.r.t. the operator output, in place; slots without a row get zeros.  The two
 // contractions of launch_matrix_backward read the result.
-template <int VEC>
+template <int VEC, int CK>
 __global__ void __launch_bounds__(32 * UPD_WARPS) gz_rows_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   int lane = threadIdx.x & 31;
   long long item = (long long)blockIdx.x * UPD_WARPS + (threadIdx.x >> 5);
@@ -910,13 +847,7 @@ __global__ void __launch_bounds__(32 * UPD_WARPS) gz_rows_kernel(WaveDims d, Wav
 #pragma unroll
     for (int c = 0; c < VEC; ++c) v[c] = f4zero();
   } else {
-    SlotGrad<VEC> sg;
-    sg.init(d, wb, w, ARR_N1, blk, r, bi.b, lane, nullptr, true);
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) {
-      int dd = c * 128 + lane * 4;
-      v[c] = dd < D ? sg.gz(dd) : f4zero();
-    }
+    gz_row<VEC, CK>(v, d, w, ARR_N1, blk, r, lane, false);
   }
   __syncwarp();
 #pragma unroll
@@ -926,11 +857,21 @@ __global__ void __launch_bounds__(32 * UPD_WARPS) gz_rows_kernel(WaveDims d, Wav
   }
 }
 
+static inline int comparator_kind(const WaveDims &d) { return d.cmp >= PBG_CMP_L2 ? CK_L2 : d.cmp == PBG_CMP_COS ? CK_COS : CK_DOT; }
+// KERNEL<VEC, CK> with the row width and comparator of the wave
+#define PBG_ROWS_CK(VEC, KERNEL, ...)                                        \
+  do {                                                                       \
+    const int ck_ = comparator_kind(d);                                      \
+    if (ck_ == CK_DOT) KERNEL<VEC, CK_DOT> __VA_ARGS__;                      \
+    else if (ck_ == CK_COS) KERNEL<VEC, CK_COS> __VA_ARGS__;                 \
+    else KERNEL<VEC, CK_L2> __VA_ARGS__;                                     \
+  } while (0)
+
 int launch_gz_rows(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st) {
   long long items = (long long)d.nblk * d.Mm;
   int ctas = (int)((items + UPD_WARPS - 1) / UPD_WARPS);
   int vec = (d.D + 127) / 128;
-#define GZ(V) gz_rows_kernel<V><<<ctas, 32 * UPD_WARPS, 0, st>>>(d, wb, w)
+#define GZ(V) PBG_ROWS_CK(V, gz_rows_kernel, <<<ctas, 32 * UPD_WARPS, 0, st>>>(d, wb, w))
   if (vec <= 1) GZ(1); else if (vec <= 2) GZ(2); else if (vec <= 4) GZ(4); else if (vec <= 8) GZ(8); else GZ(16);
 #undef GZ
   return 1;
@@ -962,140 +903,22 @@ __global__ void relupdate_matrix_kernel(WaveDims d, WaveBatches wb, WaveBufs w, 
   }
 }
 
-// Global embeddings (config.global_emb): the vector of an entity type is added to every row of that
-// type before the operator, so its gradient is the sum of the row gradients of all slots of its
-// side(s).  Stage 1: one CTA per chunk block, warp w sums the slots w, w + 8, ... of the lhs and of
-// the rhs operand array, the eight sums are added in warp order into globpart[blk][side][D]; stage 2
-// adds the partial sums of a batch
-// in a fixed order and applies the dense AsyncAdagrad step, batch after batch
-// (torchbiggraph/async_adagrad.py:75-85; the vector is one of model.parameters(), train_cpu.py:215-230).
-template <int VEC>
-__global__ void __launch_bounds__(32 * UPD_WARPS) globgrad_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
-  extern __shared__ __align__(16) float wpart_raw[];
-  float (*wpart)[VEC * 128] = reinterpret_cast<float (*)[VEC * 128]>(wpart_raw);
-  int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  int blk = blockIdx.x;
-  BlockInfo bi = block_info(d, wb, blk);
-  const int D = d.D;
-#pragma unroll 1
-  for (int side = 0; side < 2; ++side) {
-    float4 acc[VEC];
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) acc[c] = f4zero();
-    if (bi.n > 0 && w.glob[side]) {
-      for (int r = wl; r < d.Mm; r += UPD_WARPS) {
-        long long row = slot_row(d, wb, w, bi, side, r);
-        if (row < 0 || row >= d.n_rows[side]) continue;
-        SlotGrad<VEC> sg;
-        sg.init(d, wb, w, side == 0 ? ARR_N0 : ARR_N1, blk, r, bi.b, lane);
-#pragma unroll
-        for (int c = 0; c < VEC; ++c) {
-          int dd = c * 128 + lane * 4;
-          if (dd < D) acc[c] = acc[c] + sg.gx(dd);
-        }
-      }
-    }
-    __syncthreads();                                   // wpart of the previous side has been read
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) st4(&wpart[wl][c * 128 + lane * 4], acc[c]);
-    __syncthreads();
-    float *out = w.globpart + ((size_t)blk * 2 + side) * D;
-    for (int dd = threadIdx.x * 4; dd < D; dd += 4 * blockDim.x) {
-      float4 t = ld4(&wpart[0][dd]);
-#pragma unroll
-      for (int u = 1; u < UPD_WARPS; ++u) t = t + ld4(&wpart[u][dd]);
-      st4(out + dd, t);
-    }
-  }
-}
-
-__global__ void globupdate_kernel(WaveDims d, WaveBatches wb, WaveBufs w, float lr) {
-  int dd = blockIdx.x * blockDim.x + threadIdx.x;
-  if (dd >= d.D) return;
-  // gradient sums of all batches first (independent loads, all in flight), then the steps in batch order
-  float g0[PBG_KMAX], g1[PBG_KMAX];
-#pragma unroll
-  for (int b = 0; b < PBG_KMAX; ++b) { g0[b] = 0.f; g1[b] = 0.f; }
-  for (int c = 0; c < d.Cm; ++c) {
-#pragma unroll
-    for (int b = 0; b < PBG_KMAX; ++b) {
-      if (b < d.k) {
-        const float *part = w.globpart + (((size_t)b * d.Cm + c) * 2) * d.D + dd;
-        if (w.glob[0]) g0[b] += part[0];
-        if (w.glob[1]) g1[b] += part[d.D];
-      }
-    }
-  }
-  const bool two = !w.glob_shared && w.glob[1] != nullptr;       // a second vector of its own
-  const bool one = w.glob[0] != nullptr;
-  float a0 = 0.f, v0 = 0.f, a1 = 0.f, v1 = 0.f;
-  if (one) { a0 = w.gacc[0][dd]; v0 = w.glob[0][dd]; }
-  if (two) { a1 = w.gacc[1][dd]; v1 = w.glob[1][dd]; }
-#pragma unroll
-  for (int b = 0; b < PBG_KMAX; ++b) {
-    if (b >= d.k || wb.n[b] <= 0) continue;
-    float gs0 = g0[b], gs1 = g1[b];
-    if (w.glob_shared) { gs0 += gs1; gs1 = 0.f; }
-    if (one) { a0 += gs0 * gs0; v0 -= lr * gs0 / (sqrtf(a0) + PBG_ADAGRAD_EPS); }
-    if (two) { a1 += gs1 * gs1; v1 -= lr * gs1 / (sqrtf(a1) + PBG_ADAGRAD_EPS); }
-  }
-  if (one) { w.gacc[0][dd] = a0; w.glob[0][dd] = v0; }
-  if (two) { w.gacc[1][dd] = a1; w.glob[1][dd] = v1; }
-}
-
 int launch_matrix_update(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, float lr, cudaStream_t st) {
   relupdate_matrix_kernel<<<(d.opw + 255) / 256, 256, 0, st>>>(d, wb, w, lr);
   return 1;
 }
 
-// Standard relations under the cos comparator with no operator or a translation: the pull-back of a slot's gradient
-// through the normalisation, g <- (g - y <g, y>) / |z|, needs nothing but the slot's own rows.  Done here for all
-// slots at once, one warp per slot, in place -- the same expression SlotGrad::gz evaluates -- it leaves the sorted,
-// row-by-row update kernel nothing to do per slot but add (its plain form), instead of a dot product, a warp reduction
-// and two more row reads inside that kernel's chain of dependent steps.
-template <int VEC>
-__global__ void __launch_bounds__(32 * UPD_WARPS) cos_pullback_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
-  const int lane = threadIdx.x & 31;
-  long long item = (long long)blockIdx.x * UPD_WARPS + (threadIdx.x >> 5);
-  const long long per_side = (long long)d.nblk * d.Mm;
-  if (item >= 2 * per_side) return;
-  const int side = item >= per_side ? 1 : 0;
-  item -= (long long)side * per_side;
-  const int lb = (int)(item / d.Mm), r = (int)(item - (long long)lb * d.Mm);
-  const int blk = d.blk0 + lb;
-  BlockInfo bi = block_info(d, wb, blk);
-  if (bi.n <= 0) return;
-  const long long id = slot_row(d, wb, w, bi, side, r);
-  if (id < 0 || id >= d.n_rows[side]) return;
-  const int a = side ? ARR_N1 : ARR_N0;
-  SlotGrad<VEC, PBG_CMP_COS, 0> sg;
-  sg.init(d, wb, w, a, blk, r, bi.b, lane);
-  float4 v[VEC];
-#pragma unroll
-  for (int c = 0; c < VEC; ++c) {
-    int dd = c * 128 + lane * 4;
-    v[c] = dd < d.D ? sg.gz(dd) : f4zero();
-  }
-  __syncwarp();
-  float *row = w.GX[a] + ((size_t)blk * w.grows[a] + r) * d.Dp;
-#pragma unroll
-  for (int c = 0; c < VEC; ++c) {
-    int dd = c * 128 + lane * 4;
-    if (dd < d.D) st4(row + dd, v[c]);
-  }
-}
-
-// Dynamic relations with a diagonal, translation or complex_diagonal operator (no regularizer): everything a gradient
-// slot contributes is worked out here for all slots at once, one warp per slot -- the gradient of the table row
-// (comparator and operator pull-back: SlotGrad::gx) written over the slot's own gradient row, and for the slots that
-// went through an operator the gradient of the edge's operator row (op_param_grad) into GR -- so that both sorted,
-// row-by-row update kernels run in their plain form (add the slot's row) instead of evaluating ~570 instructions and a
-// chain of dependent loads per slot.  The expressions are the ones those kernels evaluated.
-template <int VEC>
-__global__ void __launch_bounds__(32 * UPD_WARPS, VEC <= 2 ? 4 : 2) dyn_pullback_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
-  const int lane = threadIdx.x & 31;
-  long long item = (long long)blockIdx.x * UPD_WARPS + (threadIdx.x >> 5);
+// Dynamic relations: the pull-back, one warp per slot -- the gradient of the table row written over the slot's own
+// gradient row, and for the slots that went through an operator the gradient of the edge's operator row into GR -- so
+// that both sorted, row-by-row update kernels only add rows.  first_q: the slots of N0 and N1 are left out (dot
+// comparator, no regularizer: what they hold is the row's gradient already; on a dimension-400 graph of 1000-row chunks
+// they are half of the slots).
+template <int VEC, int CK>
+__global__ void __launch_bounds__(32 * UPD_WARPS, VEC <= 4 ? 4 : 1) dyn_pullback_kernel(WaveDims d, WaveBatches wb, WaveBufs w, int first_q) {
+  extern __shared__ __align__(16) float wpart[];             // [UPD_WARPS][VEC * 128]
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const long long nN = (long long)d.nblk * d.Mm, nQ = (long long)d.nblk * d.Pm;
+  long long item = (long long)blockIdx.x * UPD_WARPS + wl + (first_q ? 2 * nN : 0);
   if (item >= 2 * nN + 2 * nQ) return;
   int a, rows;
   if (item < nN) { a = ARR_N0; rows = d.Mm; }
@@ -1103,170 +926,135 @@ __global__ void __launch_bounds__(32 * UPD_WARPS, VEC <= 2 ? 4 : 2) dyn_pullback
   else if ((item -= nN) < nQ) { a = ARR_Q0; rows = d.Pm; }
   else { item -= nQ; a = ARR_Q1; rows = d.Pm; }
   const int lb = (int)(item / rows), r = (int)(item - (long long)lb * rows);
-  const int blk = d.blk0 + lb;
+  const int blk = d.blk0 + lb, D = d.D;
   BlockInfo bi = block_info(d, wb, blk);
   if (bi.n <= 0) return;
   // the entity of the slot: N arrays hold lhs / rhs rows (chunk, then uniform), Q0 = op_rhs(rhs), Q1 = op_lhs(lhs)
   const int side = (a == ARR_N0 || a == ARR_Q1) ? 0 : 1;
-  if (a >= ARR_Q0 && r >= bi.n) return;
+  const bool q = a >= ARR_Q0;
+  if (q && r >= bi.n) return;
+  float *prow = q && w.GR[a - ARR_Q0] ? w.GR[a - ARR_Q0] + ((size_t)blk * d.Pm + r) * d.Dp : nullptr;
   const long long id = slot_row(d, wb, w, bi, side, r);
   if (id < 0 || id >= d.n_rows[side]) {
     // an entity id outside its table (the call reports it): the edge's operator-row slot may still be a valid one
     // (its key depends on the relation id only), so it gets a zero gradient rather than whatever the row held
-    if (a >= ARR_Q0 && w.GR[a - ARR_Q0]) {
-      float *prow0 = w.GR[a - ARR_Q0] + ((size_t)blk * d.Pm + r) * d.Dp;
-      for (int dd = lane * 4; dd < d.D; dd += 128) st4(prow0 + dd, f4zero());
-    }
+    if (prow)
+      for (int dd = lane * 4; dd < D; dd += 128) st4(prow + dd, f4zero());
     return;
   }
-  SlotGrad<VEC> sg;
-  sg.init(d, wb, w, a, blk, r, bi.b, lane);
-  const int D = d.D;
-  float4 gxv[VEC], pg[VEC];
-  const bool param = a >= ARR_Q0 && sg.theta != nullptr;
-#pragma unroll
-  for (int c = 0; c < VEC; ++c) {
-    int dd = c * 128 + lane * 4;
-    gxv[c] = dd < D ? sg.gx(dd) : f4zero();
-    pg[c] = f4zero();
+  const float *theta = nullptr;
+  if (prow) {
+    const long long rl = w.rel[bi.e0 + r];
+    const float *tab = w.theta[a - ARR_Q0];
+    if (tab && rl >= 0 && rl < d.num_rels) theta = tab + (size_t)rl * D;
   }
-  if (param) {
+  const bool reg = d.reg_coef != 0.f && r < bi.n && r < d.Pm;    // regularized: the chunk's edges in every operand array
+  float4 v[VEC], pg[VEC];
+  gz_row<VEC, CK>(v, d, w, a, blk, r, lane, reg);
+  if (theta) {
     const int na = a == ARR_Q0 ? ARR_N1 : ARR_N0;              // the slot's operator-free copy (prepared raw row)
     const size_t nrow = (size_t)blk * w.xrows[na] + r;
-    const float *x = w.X[na] + nrow * d.Dp;
-    const float xscale = d.cmp == PBG_CMP_COS ? 1.0f / w.aux[na][nrow] : 1.0f;
+    const float xs = CK == CK_COS ? 1.0f / w.aux[na][nrow] : 1.0f;
+    operator_back<VEC>(v, pg, d, theta, w.X[na] + nrow * d.Dp, xs, nullptr, wpart + (size_t)wl * VEC * 128, lane);
 #pragma unroll
     for (int c = 0; c < VEC; ++c) {
-      int dd = c * 128 + lane * 4;
-      if (dd < D) pg[c] = op_param_grad<VEC>(sg, x, xscale, dd);
+      const int dd = c * 128 + lane * 4;
+      if (dd < D) {
+        // N3 regularizer on the edge's own parameter row (still as the wave found it)
+        if (d.reg_coef != 0.f) pg[c] = pg[c] + n3_grad4(theta, dd, D, d.op == PBG_OP_COMPLEX_DIAGONAL) * d.reg_coef;
+        st4(prow + dd, pg[c]);
+      }
     }
   }
   __syncwarp();
   float *row = w.GX[a] + ((size_t)blk * w.grows[a] + r) * d.Dp;
-  float *prow = a >= ARR_Q0 ? w.GR[a - ARR_Q0] + ((size_t)blk * d.Pm + r) * d.Dp : nullptr;
 #pragma unroll
   for (int c = 0; c < VEC; ++c) {
-    int dd = c * 128 + lane * 4;
-    if (dd < D) {
-      st4(row + dd, gxv[c]);
-      if (param) st4(prow + dd, pg[c]);
-    }
+    const int dd = c * 128 + lane * 4;
+    if (dd < D) st4(row + dd, v[c]);
   }
 }
 
+// The pull-back of a wave (what is left to do depends on the comparator, the operator and the options) and the job it
+// leaves for param_step.
 template <int VEC>
-static int launch_update_vec(const WaveDims &d_in, const WaveBatches &wb, const WaveBufs &w,
+static int launch_pullback(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, float rel_lr, ParamJob &job, cudaStream_t st) {
+  const size_t smem = (size_t)UPD_WARPS * VEC * 128 * sizeof(float);
+  const bool has_op = d.op != PBG_OP_NONE && w.theta[0] != nullptr;
+  const bool rows_change = d.cmp != PBG_CMP_DOT || d.reg_coef != 0.f;
+  pbg_opt_in_smem((const void *)std_pullback_kernel<VEC, CK_DOT>, (int)smem);
+  pbg_opt_in_smem((const void *)std_pullback_kernel<VEC, CK_COS>, (int)smem);
+  pbg_opt_in_smem((const void *)std_pullback_kernel<VEC, CK_L2>, (int)smem);
+  pbg_opt_in_smem((const void *)dyn_pullback_kernel<VEC, CK_DOT>, (int)smem);
+  pbg_opt_in_smem((const void *)dyn_pullback_kernel<VEC, CK_COS>, (int)smem);
+  pbg_opt_in_smem((const void *)dyn_pullback_kernel<VEC, CK_L2>, (int)smem);
+  job.sums = job.steps = 0; job.lr = rel_lr;
+  if (d.dynamic) {
+    if (!rows_change && !has_op) return 0;
+    const int first_q = rows_change ? 0 : 1;
+    const long long rows = 2ll * d.nblk * d.Pm + (first_q ? 0 : 2ll * d.nblk * d.Mm);
+    PBG_ROWS_CK(VEC, dyn_pullback_kernel, <<<(unsigned)((rows + UPD_WARPS - 1) / UPD_WARPS), 32 * UPD_WARPS, smem, st>>>(d, wb, w, first_q));
+    return 1;
+  }
+  const bool row_op = has_op && !d.matrix_op;
+  if (row_op) { job.sum_kind[job.sums++] = 0; job.step_kind[job.steps++] = 0; }
+  if (w.glob[0]) { job.sum_kind[job.sums++] = 1; job.step_kind[job.steps++] = 1; }
+  if (w.glob[1]) {
+    job.sum_kind[job.sums++] = 2;
+    if (!w.glob_shared) job.step_kind[job.steps++] = 2;
+  }
+  if (!rows_change && !(row_op && w.PG)) return 0;
+  const dim3 grid((unsigned)(((long long)d.nblk * d.Mm + UPD_WARPS - 1) / UPD_WARPS), rows_change ? 2 : 1);
+  PBG_ROWS_CK(VEC, std_pullback_kernel, <<<grid, 32 * UPD_WARPS, smem, st>>>(d, wb, w, rows_change ? 0 : 1));
+  return 1;
+}
+
+template <int VEC>
+static int launch_update_vec(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w,
                              const unsigned long long *keys, const unsigned int *vals, float lr, float rel_lr,
                              const UpdateScratch &us, cudaStream_t st) {
-  WaveDims d = d_in;            // (the comparator becomes dot once the cos pull-back has been applied to all slots, below)
-  int launches = 0;
-  long long warps = ((long long)d.nocc + TILE - 1) / TILE;
-  int ctas = (int)((warps + UPD_WARPS - 1) / UPD_WARPS);
-  int ctas_emb = (int)((warps + TILE_WARPS_EMB - 1) / TILE_WARPS_EMB);
-  size_t stage_smem = (size_t)TILE_WARPS_EMB * TILE * d.Dp * sizeof(float);
+  constexpr int EMB_WARPS = TileWarps<VEC, RULE_EMB>::N, REL_WARPS = TileWarps<VEC, RULE_REL>::N;
+  const long long tiles = ((long long)d.nocc + TILE - 1) / TILE;
   const int hub_ctas = 296;     // (two and four times as many measured the same: the kernels take as long as their longest row)
-  size_t hub_smem = (size_t)d.k * VEC * 128 * sizeof(float);            // per-batch totals of one hub row
-  size_t red_smem = (size_t)UPD_WARPS * VEC * 128 * sizeof(float);       // eight partial sums of one batch of a big row
+  const size_t hub_smem = (size_t)d.k * VEC * 128 * sizeof(float);            // per-batch totals of one hub row
+  const size_t red_smem = (size_t)UPD_WARPS * VEC * 128 * sizeof(float);       // eight partial sums of one batch of a big row
+  static_assert(PBG_KMAX * 32 <= UPD_WARPS * 128, "param_step works in the same shared memory");
   // the attribute is set once for the largest wave this row width allows in 227 KB
   size_t hub_smem_max = (size_t)PBG_KMAX * VEC * 128 * sizeof(float);
   if (hub_smem_max > 227 * 1024) hub_smem_max = 227 * 1024;
   // per device (a process may hold contexts on several GPUs); a failed opt-in makes the launch fail,
   // which the caller's cudaGetLastError reports
-  const int tile_smem_max = (int)((size_t)TILE_WARPS_EMB * TILE * VEC * 128 * sizeof(float));
   pbg_opt_in_smem((const void *)hub_update_kernel<VEC, RULE_EMB>, (int)hub_smem_max);
   pbg_opt_in_smem((const void *)hub_reduce_kernel<VEC>, (int)red_smem);
-  pbg_opt_in_smem((const void *)relgrad_std_kernel<VEC>, (int)red_smem);
-  pbg_opt_in_smem((const void *)globgrad_kernel<VEC>, (int)red_smem);
-  pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_EMB, 0>, tile_smem_max);
-  pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_EMB, 1>, tile_smem_max);
-  pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_EMB, 2>, tile_smem_max);
-  pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_EMB, 3>, tile_smem_max);
-  bool has_op = d.op != PBG_OP_NONE && w.theta[0] != nullptr;
-  const bool has_glob = w.glob[0] || w.glob[1];
-  // Standard relations under a translation: the operator row's two kernels (one CTA per chunk block, then ONE CTA that
-  // steps the row batch after batch: 35 + 37 us of latency per wave at dimension 100) touch nothing the embedding
-  // rows' kernels read or write -- the pull-back through a translation is the identity and its parameter gradient
-  // is the sum of the rhs rows' gradients -- so they run on a side stream beside them.
-  const bool cos_first = !d.dynamic && d.cmp == PBG_CMP_COS && !d.matrix_op && d.reg_coef == 0.f && !has_glob &&
-                         (d.op == PBG_OP_NONE || d.op == PBG_OP_TRANSLATION);
-  if (cos_first) {
-    const long long rows2 = 2ll * d.nblk * d.Mm;
-    cos_pullback_kernel<VEC><<<(unsigned)((rows2 + UPD_WARPS - 1) / UPD_WARPS), 32 * UPD_WARPS, 0, st>>>(d_in, wb, w);
-    ++launches;
-    d.cmp = PBG_CMP_DOT;        // what the gradient slots hold now is the gradient of the operator's output
-  }
-  // (rows of more than 1024 floats keep the per-slot form: the staging buffers of the plain operator-row kernel would
-  // not fit in shared memory)
-  const bool dyn_first = d.dynamic && has_op && !d.matrix_op && d.reg_coef == 0.f && !has_glob && w.GR[0] != nullptr && VEC <= 8;
-  if (dyn_first) {
-    const long long rows4 = 2ll * d.nblk * d.Mm + 2ll * d.nblk * d.Pm;
-    dyn_pullback_kernel<VEC><<<(unsigned)((rows4 + UPD_WARPS - 1) / UPD_WARPS), 32 * UPD_WARPS, 0, st>>>(d_in, wb, w);
-    ++launches;
-    d.cmp = PBG_CMP_DOT;        // the gradient slots hold the gradients of the table rows now
-  }
-  const bool rel_side = has_op && !d.dynamic && !d.matrix_op && d.op == PBG_OP_TRANSLATION && !has_glob && us.side != nullptr;
-  if (has_op && !d.dynamic && !d.matrix_op) {
-    if (rel_side) {
-      cudaEventRecord(us.fork, st);
-      cudaStreamWaitEvent(us.side, us.fork, 0);
-      relgrad_std_kernel<VEC><<<d.nblk, 32 * UPD_WARPS, red_smem, us.side>>>(d, wb, w);
-      relupdate_std_kernel<<<(d.D + 127) / 128, 128, 0, us.side>>>(d, wb, w, rel_lr);
-      cudaEventRecord(us.join, us.side);
-      launches += 2;
-    } else {
-      relgrad_std_kernel<VEC><<<d.nblk, 32 * UPD_WARPS, red_smem, st>>>(d, wb, w);
-      ++launches;
-    }
-  }
-  // gradient sums of the global embeddings: before any operator parameter of this wave is stepped
-  if (has_glob) {
-    globgrad_kernel<VEC><<<d.nblk, 32 * UPD_WARPS, red_smem, st>>>(d, wb, w);
-    ++launches;
-  }
+  pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_EMB>, EMB_WARPS * TILE * VEC * 512);
+  ParamJob job;
+  int launches = launch_pullback<VEC>(d, wb, w, rel_lr, job, st);
   int *hubcnt = us.hubcnt + 64 * (*us.turn & 1), *hubcnt_next = us.hubcnt + 64 * ((*us.turn + 1) & 1);
   ++*us.turn;
-  // the gradient slot is the row's gradient as it stands: dot comparator, and no operator or a translation
-  const bool plain = dyn_first || (d.cmp == PBG_CMP_DOT && !d.matrix_op && d.reg_coef == 0.f && (d.op == PBG_OP_NONE || d.op == PBG_OP_TRANSLATION));
-  if (plain) tile_update_kernel<VEC, RULE_EMB, 1><<<ctas_emb, 32 * TILE_WARPS_EMB, stage_smem, st>>>(d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt);
-  else if (d.cmp == PBG_CMP_COS && !d.matrix_op && d.reg_coef == 0.f && (d.op == PBG_OP_NONE || d.op == PBG_OP_TRANSLATION))
-    tile_update_kernel<VEC, RULE_EMB, 2><<<ctas_emb, 32 * TILE_WARPS_EMB, stage_smem, st>>>(d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt);
-  else if (d.cmp == PBG_CMP_DOT && !d.matrix_op && d.reg_coef == 0.f)
-    tile_update_kernel<VEC, RULE_EMB, 3><<<ctas_emb, 32 * TILE_WARPS_EMB, stage_smem, st>>>(d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt);
-  else tile_update_kernel<VEC, RULE_EMB, 0><<<ctas_emb, 32 * TILE_WARPS_EMB, stage_smem, st>>>(d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt);
-  hub_reduce_kernel<VEC><<<d.k + 2 * hub_ctas, 32 * UPD_WARPS, red_smem, st>>>(d, wb, w, keys, vals, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 1, us.per_batch, us.sum);
+  const int sum_ctas = param_sum_ctas(d, job);
+  size_t tile_smem = (size_t)EMB_WARPS * TILE * d.Dp * 4;
+  if (sum_ctas && tile_smem < 8 * 128 * 4) tile_smem = 8 * 128 * 4;
+  tile_update_kernel<VEC, RULE_EMB><<<sum_ctas + (unsigned)((tiles + EMB_WARPS - 1) / EMB_WARPS), 32 * EMB_WARPS, tile_smem, st>>>(
+      d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, job, sum_ctas);
+  hub_reduce_kernel<VEC><<<d.k + param_step_ctas(d, job) + 2 * hub_ctas, 32 * UPD_WARPS, red_smem, st>>>(
+      d, wb, w, keys, vals, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 1, job, us.per_batch, us.sum);
   hub_update_kernel<VEC, RULE_EMB><<<hub_ctas, 32 * UPD_WARPS, hub_smem, st>>>(d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, us.bigtab);
-  ++launches;
-  launches += 2;
-  if (has_op) {
+  launches += 3;
+  if (d.op != PBG_OP_NONE && w.theta[0] != nullptr) {
     if (d.dynamic) {
       pbg_opt_in_smem((const void *)hub_update_kernel<VEC, RULE_REL>, (int)hub_smem_max);
+      pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_REL>, REL_WARPS * TILE * VEC * 512);
       int *t = hubcnt; hubcnt = hubcnt_next; hubcnt_next = t;
       ++*us.turn;
-      if (dyn_first) {
-        const size_t rel_smem = (size_t)UPD_WARPS * TILE * d.Dp * sizeof(float);
-        pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_REL, 1>, (int)((size_t)UPD_WARPS * TILE * VEC * 128 * sizeof(float)));
-        tile_update_kernel<VEC, RULE_REL, 1><<<ctas, 32 * UPD_WARPS, rel_smem, st>>>(d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt);
-      }
-      else if (d.cmp == PBG_CMP_DOT && d.reg_coef == 0.f)
-        tile_update_kernel<VEC, RULE_REL, 3><<<ctas, 32 * UPD_WARPS, 0, st>>>(d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt);
-      else
-        tile_update_kernel<VEC, RULE_REL, 0><<<ctas, 32 * UPD_WARPS, 0, st>>>(d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt);
-      hub_reduce_kernel<VEC><<<2 * hub_ctas, 32 * UPD_WARPS, red_smem, st>>>(d, wb, w, keys, vals, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 0, nullptr, nullptr);
+      tile_update_kernel<VEC, RULE_REL><<<(unsigned)((tiles + REL_WARPS - 1) / REL_WARPS), 32 * REL_WARPS, (size_t)REL_WARPS * TILE * d.Dp * 4, st>>>(
+          d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt, job, 0);
+      hub_reduce_kernel<VEC><<<2 * hub_ctas, 32 * UPD_WARPS, red_smem, st>>>(
+          d, wb, w, keys, vals, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 0, job, nullptr, nullptr);
       hub_update_kernel<VEC, RULE_REL><<<hub_ctas, 32 * UPD_WARPS, hub_smem, st>>>(d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt, us.bigtab);
-      ++launches;
-      launches += 2;
+      launches += 3;
     } else if (d.matrix_op) {
       launches += launch_matrix_update(d, wb, w, rel_lr, st);
-    } else if (rel_side) {
-      cudaStreamWaitEvent(st, us.join, 0);
-    } else {
-      relupdate_std_kernel<<<(d.D + 127) / 128, 128, 0, st>>>(d, wb, w, rel_lr);
-      ++launches;
     }
-  }
-  if (has_glob) {
-    globupdate_kernel<<<(d.D + 127) / 128, 128, 0, st>>>(d, wb, w, rel_lr);
-    ++launches;
   }
   pbg_note_launch();
   return launches;
