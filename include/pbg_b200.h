@@ -219,7 +219,7 @@ int pbg_eval_batch(pbg_context *ctx, const pbg_bucket *bucket,
  * of a side are ALL rows of its table, one chunk holds the whole batch, and the score of an edge against its
  * own true entity is ignored.  rank = 1 + #(candidates scoring >= the positive) over lhs_rows - 1 (rhs_rows - 1)
  * candidates; the loss is calc_loss over those score rows; Stats as pbg_eval_batch returns them.  The score rows
- * are never stored: the table is scored in slabs of 8192 rows.  num_batch_negs / num_uniform_negs of the
+ * are never stored: the table is scored slab by slab.  num_batch_negs / num_uniform_negs of the
  * context are not used.  Not for the linear / affine operators. */
 int pbg_eval_batch_all_negs(pbg_context *ctx, const pbg_bucket *bucket,
                             const int64_t *lhs_dev, const int64_t *rhs_dev, const int64_t *rel_dev,

@@ -37,7 +37,8 @@ struct pbg_context {
   pbg_batch_stats *stats_host = nullptr, *stats_dev = nullptr;
   int stats_cap = 0;
   double *sum_dev = nullptr;
-  double *eval_dev = nullptr;
+  double *eval_part = nullptr;      // per-CTA sums of an evaluation, and the counter of the CTAs that have left theirs
+  unsigned *eval_done = nullptr;
   int *errflag = nullptr;
   void *tcplan = nullptr;       // tensor maps of the tcgen05 contractions
   void *pairplan = nullptr;     // tensor maps of the fused score + loss kernel (standard relations, plane tiers)
@@ -59,6 +60,8 @@ struct pbg_context {
   char *esort_mem = nullptr;
   long long *etab_dev = nullptr;      // per-relation tables of a sub_bucket call + its counts
   long long etab_cap = 0;
+  int allnegs_slab = 0;
+  long long allnegs_rows = 0;         // rows of the largest table it was sized for
   char *allnegs_mem = nullptr;        // scratch of pbg_eval_batch_all_negs, allocated at its first call
   int split_min_k = 2;                // waves of at least this many batches run as two halves on two streams (PBG_SPLIT_MIN_K)
   // optional event timing per kernel class
@@ -194,7 +197,7 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   size_t off = 0;
   auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
   size_t oReg = 0, oRscale = 0;
-  size_t oX[4], oAux[4], oG[4], oS[2], oSpos[2], oCoef[4], oLoss[2], oViol[2], oRank[2];
+  size_t oX[4], oAux[4], oG[4], oS[2], oSpos[2], oCoef[4], oLoss[2], oViol[2];
   oX[0] = take(nN * c->Dp * 4); oX[1] = take(nN * c->Dp * 4);
   oAux[0] = take(nN * 4); oAux[1] = take(nN * 4);
   if (dyn) { oX[2] = take(nQ * c->Dp * 4); oX[3] = take(nQ * c->Dp * 4); oAux[2] = take(nQ * 4); oAux[3] = take(nQ * 4); }
@@ -233,7 +236,6 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   for (int p = 0; p < 2; ++p) {
     oS[p] = take(nQ * c->Ms * 4); oSpos[p] = take(nQ * 4); oLoss[p] = take(nQ * 4); oViol[p] = take(nQ * 4);
     if (p == 0) { oReg = take(nQ * 4); oRscale = take(nN * 4); }
-    oRank[p] = take(nQ * 4);
   }
   oCoef[0] = take(nN * 4); oCoef[1] = take(nN * 4); oCoef[2] = take(nQ * 4); oCoef[3] = take(nQ * 4);
   size_t oRel = take(nblk * (size_t)cfg->dim * 4);
@@ -250,7 +252,7 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   size_t oWK[2][PBG_SORT_WAVES], oWV[2][PBG_SORT_WAVES];
   for (int s = 0; s < 2; ++s)
     for (int i = 0; i < PBG_SORT_WAVES; ++i) { oWK[s][i] = take((size_t)nocc * 8); oWV[s][i] = take((size_t)nocc * 4); }
-  size_t oSum = take(8 * sizeof(double)), oEval = take(8 * sizeof(double));
+  size_t oSum = take(8 * sizeof(double)), oEval = take((size_t)pbg_eval_ctas(c->Cm, c->Pm) * 8 * sizeof(double)), oEvalDone = take(4);
   size_t oPsum = take((size_t)nocc * c->Dp * 4), oHub = take(((size_t)nocc / 8 + 64) * 8), oHubCnt = take(512);
   size_t oBigTab = take(pbg_bigtab_bytes((long long)nocc));
   // dynamic relations with a (vector) operator: the operator-row gradient of every edge, written by the pull-back pass
@@ -290,7 +292,6 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
     b.lossrow[p] = (float *)(c->ws + oLoss[p]);
     if (p == 0) { b.regrow = (float *)(c->ws + oReg); b.rscale = (float *)(c->ws + oRscale); }
     b.violrow[p] = (int *)(c->ws + oViol[p]);
-    b.rankrow[p] = (int *)(c->ws + oRank[p]);
   }
   b.relpart = (float *)(c->ws + oRel);
   b.globpart = (float *)(c->ws + oGlobPart);
@@ -322,7 +323,8 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   CU(c, cudaHostGetDevicePointer((void **)&c->box_dev, c->box, 0));
   c->sum_dev = (double *)(c->ws + oSum);
   c->errflag = &c->box_dev->err;
-  c->eval_dev = (double *)(c->ws + oEval);
+  c->eval_part = (double *)(c->ws + oEval);
+  c->eval_done = (unsigned *)(c->ws + oEvalDone);
   b.errflag = c->errflag;
   c->psum = (float *)(c->ws + oPsum);
   c->hublist = (long long *)(c->ws + oHub);
@@ -770,10 +772,9 @@ extern "C" int pbg_eval_batch(pbg_context *c, const pbg_bucket *bk, const int64_
   wb.wrel[0] = bk->relation_weights ? bk->relation_weights[d.dynamic ? 0 : relidx] : 1.0f;
   d.k = 1; d.nblk = d.Cm; d.nocc = d.spb; d.blk0 = 0;
   run_forward(c, d, wb, w, c->stream);
-  c->launches += launch_eval(d, wb, w, c->eval_dev, c->stream);
+  c->launches += launch_eval(d, wb, w, c->eval_part, c->eval_done, c->box_dev->eval, c->stream);
   CU(c, pbg_take_launch_error());
-  double *h = c->box->eval;
-  CU(c, cudaMemcpyAsync(h, c->eval_dev, sizeof c->box->eval, cudaMemcpyDeviceToHost, c->stream));
+  const double *h = c->box->eval;
   rc = check_errflag(c);
   int sides = (d.neg_enabled[0] ? 1 : 0) + (d.neg_enabled[1] ? 1 : 0);
   double div = sides > 0 ? sides : 1;
@@ -784,8 +785,6 @@ extern "C" int pbg_eval_batch(pbg_context *c, const pbg_bucket *bk, const int64_
   out->count = count;
   return rc;
 }
-
-#define PBG_ALLNEGS_SLAB 8192     // candidate rows transformed and scored at a time
 
 extern "C" int pbg_eval_batch_all_negs(pbg_context *c, const pbg_bucket *bk, const int64_t *lhs, const int64_t *rhs,
                                        const int64_t *rel, int32_t count, int32_t relidx, uint64_t seed, pbg_eval_stats *out) {
@@ -802,15 +801,21 @@ extern "C" int pbg_eval_batch_all_negs(pbg_context *c, const pbg_bucket *bk, con
   if (d.matrix_op) return fail(c, PBG_ERR_UNSUPPORTED, "ranking against all entities has no device code for the linear / affine operators");
   if (!d.dynamic && (relidx < 0 || relidx >= c->cfg.num_rels)) return fail(c, PBG_ERR_INDEX_RANGE, "relation %d outside [0, %d)", relidx, c->cfg.num_rels);
   if (d.dynamic && d.op != PBG_OP_NONE && !rel) return fail(c, PBG_ERR_BAD_ARGUMENT, "dynamic relations need the rel array");
-  if (!c->allnegs_mem) CU(c, cudaMalloc(&c->allnegs_mem, pbg_allnegs_bytes(c->cfg.max_batch_size, c->Dp, PBG_ALLNEGS_SLAB)));
+  const bool planes = c->cfg.precision != PBG_PREC_FP32;
+  const long long most_rows = bk->lhs_rows > bk->rhs_rows ? bk->lhs_rows : bk->rhs_rows;
+  if (!c->allnegs_mem || most_rows > c->allnegs_rows) {
+    if (c->allnegs_mem) { cudaFree(c->allnegs_mem); c->allnegs_mem = nullptr; }
+    CU(c, cudaMalloc(&c->allnegs_mem, pbg_allnegs_bytes(c->cfg.max_batch_size, c->cfg.dim, planes, most_rows, c->allnegs_slab)));
+    c->allnegs_rows = most_rows;
+  }
   w.lhs = (const long long *)lhs; w.rhs = (const long long *)rhs; w.rel = (const long long *)rel;
   w.ew = c->edge_w; c->edge_w = nullptr;
   w.seed = seed;
   const float wrel = bk->relation_weights ? bk->relation_weights[d.dynamic ? 0 : relidx] : 1.0f;
-  c->launches += launch_allnegs_eval(d, w, c->allnegs_mem, count, PBG_ALLNEGS_SLAB, d.dynamic ? 0 : relidx, wrel, c->eval_dev, c->stream);
+  c->launches += launch_allnegs_eval(d, w, c->allnegs_mem, c->cfg.max_batch_size, count, c->allnegs_slab, planes, d.dynamic ? 0 : relidx, wrel,
+                                   c->eval_done, c->box_dev->eval, c->stream);
   CU(c, pbg_take_launch_error());
-  double *h = c->box->eval;
-  CU(c, cudaMemcpyAsync(h, c->eval_dev, sizeof c->box->eval, cudaMemcpyDeviceToHost, c->stream));
+  const double *h = c->box->eval;
   rc = check_errflag(c);
   int sides = (d.neg_enabled[0] ? 1 : 0) + (d.neg_enabled[1] ? 1 : 0);
   double div = sides > 0 ? sides : 1;

@@ -96,7 +96,6 @@ struct WaveBufs {
   float *rscale;                     // max_norm: scale applied to the raw row of every N1 slot [blk][Mm] (1 = none)
   float *regrow;                     // per positive row: its share of the N3 regularizer (reg_coef != 0)
   int *violrow[2];                   // per positive row: #(neg > pos)
-  int *rankrow[2];                   // evaluation: per positive row, 1 + #(neg >= pos)
   const long long *lhs, *rhs, *rel;  // edge arrays
   const float *ew;                  // per-edge weights parallel to the edge arrays, or null
   const long long *ul, *ur;          // uniform ids [batches][Cm][U] or null
@@ -411,10 +410,47 @@ int launch_update(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, c
                   float lr, float rel_lr, const UpdateScratch &us, cudaStream_t st);
 // bigtab: (nocc / 256 + 2) rows of PBG_KMAX + 1 entries: where the batches of a row with 256 and more slots start, and its end
 inline size_t pbg_bigtab_bytes(long long nocc) { return (size_t)(nocc / 256 + 2) * (PBG_KMAX + 1) * sizeof(long long); }
-int launch_eval(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, double *out8_dev, cudaStream_t st);
-size_t pbg_allnegs_bytes(int B, int Dp, int slab);
-int launch_allnegs_eval(const WaveDims &d, const WaveBufs &w, char *mem, int B, int slab, int rel_std, float wrel,
-                        double *out8_dev, cudaStream_t st);
+// Evaluation of one batch after its scores.  out8 (host or device memory): loss, then pos_rank, mrr, r1, r10, r50 summed over
+// both sides, then the AUC hits per side.  part: 8 doubles for each of the kernel's CTAs; done: a counter, zero at first.
+inline int pbg_eval_ctas(int nblk, int Pm) { return (int)((2ll * nblk * Pm + 7) / 8); }
+int launch_eval(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, double *part, unsigned *done, double *out8, cudaStream_t st);
+// The evaluator's last step, by the last CTA of a kernel (256 threads): the CTAs' partial sums [ctas][8] added up in a
+// fixed order (32 runs, then the runs), the counter cleared for the next call.
+__device__ __forceinline__ void close_eval(const double *part, int ctas, unsigned *done, double *out8) {
+  __shared__ double run[32][8];
+  const int k = threadIdx.x & 7, y = threadIdx.x >> 3;
+  double s = 0.0;
+  __threadfence();
+  for (int c = y; c < ctas; c += 32) s += ((const volatile double *)part)[(size_t)c * 8 + k];
+  run[y][k] = s;
+  __syncthreads();
+  if (threadIdx.x < 8) {
+    double t = 0.0;
+    for (int u = 0; u < 32; ++u) t += run[u][k];
+    out8[k] = t;
+    if (k == 0) *done = 0u;
+    __threadfence_system();
+  }
+}
+
+// Ranking against all entities (pbg_gather.cu, pbg_rank_tc.cu): one chunk holds the batch of B edges, the candidates of a
+// side come in slabs of its table.
+struct AllNegs {
+  float *Q[2];            // [B][Dp]  Q[0]: scored against lhs candidates (op_rhs(rhs) rows), Q[1]: against rhs candidates
+  float *qn[2], *pos[2];  // [B] |q|^2 (l2 family); positive score of problem 0 / 1
+  float *Y[2], *yn[2];    // candidate slab [slab][Dp] (fp32 tier), |y|^2
+  unsigned short *QB, *YB;              // other tiers: bf16 planes [2][3][qrows][Dpb], [2][3][slab][Dpb]
+  int *pcnt[2]; float *pa[2], *pb[2];   // per (tile of the slab, edge): count, loss partials
+  int *cnt[2]; float *ra[2], *rb[2];    // per-edge state over the slabs so far
+  int *auc[2];                          // per edge: did its sample of the randomized AUC hit
+  double *part; unsigned *done;         // per-CTA sums of the last kernel, and how many CTAs have left theirs
+  int B, slab, qrows, Dpb, tiles;       // tiles: partials per edge and slab
+};
+size_t pbg_allnegs_bytes(int maxB, int D, bool planes, long long table_rows, int &slab);
+// out8: what the evaluator returns (see launch_eval), in host or device memory
+int launch_allnegs_eval(const WaveDims &d, const WaveBufs &w, char *mem, int maxB, int B, int slab, bool planes, int rel_std, float wrel,
+                        unsigned *done, double *out8, cudaStream_t st);
+int launch_allnegs_score_tc(const WaveDims &d, const WaveBufs &w, const AllNegs &a, long long row0, cudaStream_t st);
 int launch_reg_value(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st);
 int launch_row_adagrad_sorted(float *emb, float *state, int dim, const unsigned long long *keys,
                               const unsigned int *vals, const float *grads, int n, float lr,

@@ -494,22 +494,37 @@ int launch_build_keys(const WaveDims &d, const WaveBatches &wb, const WaveBufs &
 // batch, the negatives of a side are every row of its table, and an edge's own true entity is ignored.
 //   allnegs_rows_kernel     per edge: the two scored rows (prepared, operator applied where the mode says so)
 //                           and the positive score(s)
-//   allnegs_slab_kernel     a slab of table rows as candidates: global embedding, operator (standard relations,
-//                           rhs side), prepare -> Y[slab][Dp] and the row's |y|^2
-//   allnegs_score_kernel    64 x 64 tiles of scores between the batch's scored rows and the slab, never stored:
-//                           per (tile, edge) the count of candidates scoring >= the positive and the loss partials
-//   allnegs_merge_kernel    folds a slab's tiles into the per-edge running state, in tile order
-//   allnegs_finish_kernel   ranks, loss and the evaluator's sums
+//   allnegs_slab_kernel     a slab of both tables' rows as candidates: global embedding, operator (standard relations,
+//                           rhs side), prepare -> rows of Y (planes of YB) and the row's |y|^2; with the first slab
+//                           also the samples of the randomized AUC
+//   scores, never stored: per (tile of candidates, edge) the count scoring >= the positive and the loss partials --
+//                           allnegs_tc_kernel (pbg_rank_tc.cu), or in the fp32 tier allnegs_score_kernel's 64 x 64 tiles
+//   allnegs_merge_kernel    one warp per edge and side folds the slab's tiles into the running state; after the last
+//                           slab ranks, loss and the evaluator's sums
+// Both sides go through every launch together: a table that fits one slab takes four launches in all.
 // ------------------------------------------------------------------------------------------------
-struct AllNegs {
-  float *Q[2];            // [B][Dp]  Q[0]: scored against lhs candidates (op_rhs(rhs) rows), Q[1]: against rhs candidates
-  float *qn[2];           // [B] |q|^2 (l2 family)
-  float *pos[2];          // [B] positive score of problem 0 / 1
-  float *Y, *yn;          // candidate slab [slab][Dp], |y|^2
-  int *pcnt; float *pa, *pb;      // per (tile of the slab, edge): count, loss partials
-  int *cnt[2]; float *ra[2], *rb[2];   // running per-edge state of side 0 / 1
-  int B, slab;
-};
+__device__ __forceinline__ int allnegs_rows_of(const WaveDims &d, const AllNegs &a, int side, long long row0) {
+  if (!d.neg_enabled[side]) return 0;
+  const long long left = d.n_rows[side] - row0;
+  return left < 0 ? 0 : left < a.slab ? (int)left : a.slab;
+}
+template <int VEC>
+__device__ __forceinline__ void store_planes(unsigned short *x, size_t plane, const float4 (&v)[VEC], int D, int lane) {
+#pragma unroll
+  for (int c = 0; c < VEC; ++c) {
+    const int dd = c * 128 + lane * 4;
+    if (dd < D) {
+      uint2 p0, p1, p2;
+      bf16_planes4(v[c], p0, p1, p2);
+      *(uint2 *)(x + dd) = p0; *(uint2 *)(x + plane + dd) = p1; *(uint2 *)(x + 2 * plane + dd) = p2;
+    }
+  }
+}
+template <int VEC>
+__device__ __forceinline__ void allnegs_q_planes(const AllNegs &a, int side, int e, const float4 (&v)[VEC], int D, int lane) {
+  const size_t plane = (size_t)a.qrows * a.Dpb;
+  store_planes<VEC>(a.QB + (size_t)side * 3 * plane + (size_t)e * a.Dpb, plane, v, D, lane);
+}
 
 template <int VEC>
 __global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_rows_kernel(WaveDims d, WaveBufs w, AllNegs a, int rel_std) {
@@ -524,6 +539,12 @@ __global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_rows_kernel(WaveDim
   if (!ok) {
     if (lane == 0) { atomicOr(w.errflag, 1); a.pos[0][e] = 0.f; a.pos[1][e] = 0.f; a.qn[0][e] = 0.f; a.qn[1][e] = 0.f; }
     zero_row<VEC>(q0, D, lane); zero_row<VEC>(q1, D, lane);
+    if (a.QB) {
+      float4 z[VEC];
+#pragma unroll
+      for (int c = 0; c < VEC; ++c) z[c] = f4zero();
+      allnegs_q_planes<VEC>(a, 0, e, z, D, lane); allnegs_q_planes<VEC>(a, 1, e, z, D, lane);
+    }
     return;
   }
   const float *xl = w.W[0] + (size_t)il * D, *xr = w.W[1] + (size_t)ir * D;
@@ -542,8 +563,10 @@ __global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_rows_kernel(WaveDim
     apply_operator<VEC>(z, x, xl, th1, d.op, D, lane, nullptr, scl);
     a1 = prepare_row<VEC>(z, d.cmp);
     store_row<VEC>(q1, z, D, lane);
+    if (a.QB) allnegs_q_planes<VEC>(a, 1, e, z, D, lane);
   } else {
     store_row<VEC>(q1, yl, D, lane);
+    if (a.QB) allnegs_q_planes<VEC>(a, 1, e, yl, D, lane);
   }
   // rhs row through the rhs operator, prepared
   load_row<VEC>(x, xr, D, lane);
@@ -553,6 +576,7 @@ __global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_rows_kernel(WaveDim
   apply_operator<VEC>(yr, x, xr, th0, d.op, D, lane, w.glob[1], scr);
   float a0 = prepare_row<VEC>(yr, d.cmp);
   store_row<VEC>(q0, yr, D, lane);
+  if (a.QB) allnegs_q_planes<VEC>(a, 0, e, yr, D, lane);
   float s0 = positive_score<VEC>(yl, yr, d.cmp);          // problem 0: c(lhs, op_rhs(rhs))
   if (d.dynamic) {
     // problem 1: c(prepared rhs without operator, op_lhs(lhs))
@@ -570,33 +594,74 @@ __global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_rows_kernel(WaveDim
   }
 }
 
-// candidates: rows [row0, row0 + n) of the table of `side`
+// one candidate: row `row` of the table of `side` through global embedding, operator and prepare; returns its |y|^2
 template <int VEC>
-__global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_slab_kernel(WaveDims d, WaveBufs w, AllNegs a, int side, long long row0, int n, int rel_std) {
-  int lane = threadIdx.x & 31;
-  int r = blockIdx.x * GATHER_WARPS + (threadIdx.x >> 5);
-  if (r >= n) return;
+__device__ __forceinline__ float allnegs_candidate(float4 (&z)[VEC], const WaveDims &d, const WaveBufs &w, int side, long long row, int rel_std, int lane) {
   const int D = d.D;
-  const float *xrow = w.W[side] + (size_t)(row0 + r) * D;
-  float4 x[VEC], z[VEC];
+  const float *xrow = w.W[side] + (size_t)row * D;
+  float4 x[VEC];
   load_row<VEC>(x, xrow, D, lane);
   const float sc = renorm_row<VEC>(x, d.max_norm);
   add_global<VEC>(x, w.glob[side], D, lane);
   // standard relations apply the operator to every rhs row, negatives included; with dynamic relations negatives get none
   const float *th = (side == 1 && !d.dynamic && d.op != PBG_OP_NONE && w.theta[0]) ? w.theta[0] + (size_t)rel_std * D : nullptr;
   apply_operator<VEC>(z, x, xrow, th, d.op, D, lane, w.glob[side], sc);
-  float aux = prepare_row<VEC>(z, d.cmp);
-  store_row<VEC>(a.Y + (size_t)r * d.Dp, z, D, lane);
-  if (lane == 0) a.yn[r] = d.cmp >= PBG_CMP_L2 ? aux : 0.f;
+  return prepare_row<VEC>(z, d.cmp);
+}
+
+// grid (row groups, sides): candidates row0 .. of both tables; warps past them take the AUC's samples (auc: B of them),
+// torchbiggraph/util.py:415-428: `count` random (positive, (edge, candidate)) pairs per side, hits left in cnt[side]
+template <int VEC>
+__global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_slab_kernel(WaveDims d, WaveBufs w, AllNegs a, long long row0, int rel_std, int slab_ctas, int auc) {
+  const int lane = threadIdx.x & 31, side = blockIdx.y, D = d.D;
+  float4 z[VEC];
+  if (blockIdx.x < slab_ctas) {
+    const int r = blockIdx.x * GATHER_WARPS + (threadIdx.x >> 5);
+    if (r >= allnegs_rows_of(d, a, side, row0)) return;
+    const float aux = allnegs_candidate<VEC>(z, d, w, side, row0 + r, rel_std, lane);
+    if (a.YB) {
+      const size_t plane = (size_t)a.slab * a.Dpb;
+      store_planes<VEC>(a.YB + (size_t)side * 3 * plane + (size_t)r * a.Dpb, plane, z, D, lane);
+    } else {
+      store_row<VEC>(a.Y[side] + (size_t)r * d.Dp, z, D, lane);
+    }
+    if (lane == 0) a.yn[side][r] = d.cmp >= PBG_CMP_L2 ? aux : 0.f;
+    return;
+  }
+  const int smp = (blockIdx.x - slab_ctas) * GATHER_WARPS + (threadIdx.x >> 5);
+  if (!auc || smp >= a.B || !d.neg_enabled[side]) return;
+  unsigned long long h = pbg_mix64(w.seed ^ pbg_mix64(0xA11CE5ull + (unsigned long long)side * 0x10001ull + smp));
+  const int ei = (int)(h % (unsigned long long)a.B);
+  h = pbg_mix64(h);
+  const int er = (int)(h % (unsigned long long)a.B);
+  h = pbg_mix64(h);
+  const long long cand = (long long)(h % (unsigned long long)d.n_rows[side]);
+  float neg = PBG_MASKED;
+  if (cand != (side == 0 ? w.lhs : w.rhs)[er]) {
+    const float yn = allnegs_candidate<VEC>(z, d, w, side, cand, rel_std, lane);
+    const float *qr = a.Q[side] + (size_t)er * d.Dp;
+    float s = 0.f;
+#pragma unroll
+    for (int c = 0; c < VEC; ++c) { const int dd = c * 128 + lane * 4; if (dd < D) s += f4dot(ld4(qr + dd), z[c]); }
+    s = warp_sum(s);
+    if (d.cmp >= PBG_CMP_L2) {
+      const float qv = (yn - 2.0f * s) + a.qn[side][er];
+      s = d.cmp == PBG_CMP_L2 ? -sqrtf(fmaxf(qv, 1e-30f)) : -qv;
+    }
+    neg = s;
+  }
+  if (lane == 0) a.auc[side][smp] = a.pos[side][ei] > neg ? 1 : 0;
 }
 
 #define AN_TILE 64
-// grid (edge tiles, candidate tiles of the slab); 256 threads, each a 4 x 4 block of the 64 x 64 score tile
-__global__ void __launch_bounds__(256) allnegs_score_kernel(WaveDims d, WaveBufs w, AllNegs a, int side, long long row0, int n) {
+// grid (edge tiles, candidate tiles of the slab, sides); 256 threads, each a 4 x 4 block of the 64 x 64 score tile
+__global__ void __launch_bounds__(256) allnegs_score_kernel(WaveDims d, WaveBufs w, AllNegs a, long long row0) {
   __shared__ float sq[16][AN_TILE + 1], sy[16][AN_TILE + 1];
   __shared__ int scnt[16][AN_TILE];
   __shared__ float sa[16][AN_TILE], sb[16][AN_TILE];
-  const int te = blockIdx.x, tc = blockIdx.y, t = threadIdx.x;
+  const int te = blockIdx.x, tc = blockIdx.y, side = blockIdx.z, t = threadIdx.x;
+  const int n = allnegs_rows_of(d, a, side, row0);
+  if (tc * AN_TILE >= n) return;
   const int ty = t >> 4, tx = t & 15;                        // rows 4 ty .. 4 ty + 3 (edges), cols 4 tx .. (candidates)
   const float *Q = a.Q[side];
   float acc[4][4];
@@ -610,7 +675,7 @@ __global__ void __launch_bounds__(256) allnegs_score_kernel(WaveDims d, WaveBufs
     int lr = t >> 2, lk = (t & 3) * 4;
     float4 vq = f4zero(), vy = f4zero();
     if (e0 + lr < a.B && k0 + lk < d.D) vq = ld4(Q + (size_t)(e0 + lr) * d.Dp + k0 + lk);
-    if (c0 + lr < n && k0 + lk < d.D) vy = ld4(a.Y + (size_t)(c0 + lr) * d.Dp + k0 + lk);
+    if (c0 + lr < n && k0 + lk < d.D) vy = ld4(a.Y[side] + (size_t)(c0 + lr) * d.Dp + k0 + lk);
     __syncthreads();
     sq[lk][lr] = vq.x; sq[lk + 1][lr] = vq.y; sq[lk + 2][lr] = vq.z; sq[lk + 3][lr] = vq.w;
     sy[lk][lr] = vy.x; sy[lk + 1][lr] = vy.y; sy[lk + 2][lr] = vy.z; sy[lk + 3][lr] = vy.w;
@@ -644,7 +709,7 @@ __global__ void __launch_bounds__(256) allnegs_score_kernel(WaveDims d, WaveBufs
         live[j] = c < n && row0 + c != tid;
         float s = acc[i][j];
         if (d.cmp >= PBG_CMP_L2) {
-          float qv = (a.yn[c < n ? c : 0] - 2.0f * s) + a.qn[side][e];       // model.py:226-246
+          float qv = (a.yn[side][c < n ? c : 0] - 2.0f * s) + a.qn[side][e];       // model.py:226-246
           s = d.cmp == PBG_CMP_L2 ? -sqrtf(fmaxf(qv, 1e-30f)) : -qv;
         }
         sv[j] = s;
@@ -679,152 +744,149 @@ __global__ void __launch_bounds__(256) allnegs_score_kernel(WaveDims d, WaveBufs
         } else pa += sa[x][t];
       }
       size_t o = (size_t)tc * a.B + e;
-      a.pcnt[o] = cnt; a.pa[o] = pa; a.pb[o] = pb;
+      a.pcnt[side][o] = cnt; a.pa[side][o] = pa; a.pb[side][o] = pb;
     }
   }
 }
 
-__global__ void allnegs_merge_kernel(WaveDims d, AllNegs a, int side, int ntiles, int first) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= a.B) return;
-  int cnt = first ? 0 : a.cnt[side][e];
-  float ra = first ? 0.f : a.ra[side][e];
-  float rb = first ? (d.loss == PBG_LOSS_SOFTMAX ? -INFINITY : 0.f) : a.rb[side][e];
-  for (int tcl = 0; tcl < ntiles; ++tcl) {
-    size_t o = (size_t)tcl * a.B + e;
-    cnt += a.pcnt[o];
+// One warp per (side, edge).  The partials of the slab's tiles are folded across the lanes and into the running state;
+// with the last slab every warp turns its state into rank and loss, the CTA's eight are summed, and the last CTA to
+// finish adds up the CTAs' sums in CTA order.
+// out8: loss, pos_rank, mrr, r1, r10, r50 sums over both sides' ranks, AUC hits per side.
+__global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_merge_kernel(WaveDims d, WaveBufs w, AllNegs a, long long row0, int first, int last, float wrel, double *out8) {
+  __shared__ double sm[GATHER_WARPS][8];
+  __shared__ bool closing;
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const int item = blockIdx.x * GATHER_WARPS + wl;
+  const int side = item >= a.B ? 1 : 0, e = item - side * a.B;
+  const bool live = item < 2 * a.B && d.neg_enabled[side];
+  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  if (live) {
+    const int n = allnegs_rows_of(d, a, side, row0);
+    const int per = a.slab / a.tiles, ntiles = (n + per - 1) / per;       // candidates per partial; partials that hold any
+    int cnt = 0;
+    float ra = 0.f, rb = -INFINITY;
+    for (int t = lane; t < ntiles; t += 32) {
+      const size_t o = (size_t)t * a.B + e;
+      cnt += a.pcnt[side][o];
+      if (d.loss == PBG_LOSS_SOFTMAX) {
+        const float m2 = a.pb[side][o], m = fmaxf(rb, m2);
+        if (m2 > -INFINITY) { ra = (rb > -INFINITY ? ra * expf(rb - m) : 0.f) + a.pa[side][o] * expf(m2 - m); rb = m; }
+      } else ra += a.pa[side][o];
+    }
+    cnt = warp_sum_int(cnt);
     if (d.loss == PBG_LOSS_SOFTMAX) {
-      float m2 = a.pb[o];
-      if (m2 > -INFINITY) {
-        float m = fmaxf(rb, m2);
-        ra = (rb > -INFINITY ? ra * expf(rb - m) : 0.f) + a.pa[o] * expf(m2 - m);
-        rb = m;
+      const float m = warp_max(rb);
+      ra = warp_sum(rb > -INFINITY ? ra * expf(rb - m) : 0.f);
+      rb = m;
+    } else ra = warp_sum(ra);
+    if (lane == 0) {
+      if (!first) {
+        cnt += a.cnt[side][e];
+        if (d.loss == PBG_LOSS_SOFTMAX) {
+          const float pb = a.rb[side][e], m = fmaxf(rb, pb);
+          if (m > -INFINITY) ra = (pb > -INFINITY ? a.ra[side][e] * expf(pb - m) : 0.f) + (rb > -INFINITY ? ra * expf(rb - m) : 0.f);
+          rb = m;
+        } else ra += a.ra[side][e];
       }
-    } else ra += a.pa[o];
-  }
-  a.cnt[side][e] = cnt; a.ra[side][e] = ra; a.rb[side][e] = rb;
-}
-
-// out8: loss, pos_rank, mrr, r1, r10, r50 sums over both sides' ranks (as eval_reduce_kernel); AUC slots are filled by allnegs_auc_kernel
-__global__ void __launch_bounds__(256) allnegs_finish_kernel(WaveDims d, WaveBufs w, AllNegs a, float wrel, double *out8) {
-  __shared__ double sm[6][256];
-  int t = threadIdx.x;
-  double acc[6] = {0, 0, 0, 0, 0, 0};
-  for (int e = t; e < a.B; e += 256) {
-    const float wgt = wrel * (w.ew ? w.ew[e] : 1.0f);
-    for (int side = 0; side < 2; ++side) {
-      if (!d.neg_enabled[side]) continue;
-      const float pos = a.pos[side][e];
-      const long long n = d.n_rows[side];
-      float lossv;
-      if (d.loss == PBG_LOSS_RANKING) lossv = a.ra[side][e];
-      else if (d.loss == PBG_LOSS_LOGISTIC) lossv = a.ra[side][e] / (float)n + (fmaxf(-pos, 0.f) + log1pf(expf(-fabsf(pos))));   // M counts the ignored column
+      if (!last) { a.cnt[side][e] = cnt; a.ra[side][e] = ra; a.rb[side][e] = rb; }
       else {
-        float m = fmaxf(a.rb[side][e], pos);
-        float z = (a.rb[side][e] > -INFINITY ? a.ra[side][e] * expf(a.rb[side][e] - m) : 0.f) + expf(pos - m);
-        lossv = -pos + m + logf(z);
+        const float wgt = wrel * (w.ew ? w.ew[e] : 1.0f), pos = a.pos[side][e];
+        float lossv;
+        if (d.loss == PBG_LOSS_RANKING) lossv = ra;
+        else if (d.loss == PBG_LOSS_LOGISTIC) lossv = ra / (float)d.n_rows[side] + (fmaxf(-pos, 0.f) + log1pf(expf(-fabsf(pos))));   // M counts the ignored column
+        else {
+          const float m = fmaxf(rb, pos);
+          lossv = -pos + m + logf((rb > -INFINITY ? ra * expf(rb - m) : 0.f) + expf(pos - m));
+        }
+        const int rk = cnt + 1;
+        v[0] = (double)(wgt * lossv); v[1] = rk; v[2] = 1.0 / rk; v[3] = rk <= 1; v[4] = rk <= 10; v[5] = rk <= 50;
+        v[6 + side] = a.auc[side][e];
       }
-      acc[0] += (double)(wgt * lossv);
-      int rk = a.cnt[side][e] + 1;
-      acc[1] += rk; acc[2] += 1.0 / rk; acc[3] += rk <= 1; acc[4] += rk <= 10; acc[5] += rk <= 50;
     }
   }
-  for (int k = 0; k < 6; ++k) sm[k][t] = acc[k];
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (t < o) for (int k = 0; k < 6; ++k) sm[k][t] += sm[k][t + o];
-    __syncthreads();
-  }
-  if (t < 6) out8[t] = sm[t][0];
-}
-
-// randomized AUC (torchbiggraph/util.py:415-428): `count` random (positive, (edge, candidate)) pairs per side; one warp per sample
-template <int VEC>
-__global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_auc_kernel(WaveDims d, WaveBufs w, AllNegs a, int rel_std, double *out8) {
-  int lane = threadIdx.x & 31;
-  int smp = blockIdx.x * GATHER_WARPS + (threadIdx.x >> 5);
-  int side = blockIdx.y;
-  if (smp >= a.B || !d.neg_enabled[side]) return;
-  const int D = d.D;
-  unsigned long long h = pbg_mix64(w.seed ^ pbg_mix64(0xA11CE5ull + (unsigned long long)side * 0x10001ull + smp));
-  int ei = (int)(h % (unsigned long long)a.B);
-  h = pbg_mix64(h);
-  int er = (int)(h % (unsigned long long)a.B);
-  h = pbg_mix64(h);
-  long long cand = (long long)(h % (unsigned long long)d.n_rows[side]);
-  const long long *truth = side == 0 ? w.lhs : w.rhs;
-  float neg;
-  if (cand == truth[er]) neg = PBG_MASKED;
-  else {
-    const float *xrow = w.W[side] + (size_t)cand * D;
-    float4 x[VEC], z[VEC], q[VEC];
-    load_row<VEC>(x, xrow, D, lane);
-    const float sc = renorm_row<VEC>(x, d.max_norm);
-    add_global<VEC>(x, w.glob[side], D, lane);
-    const float *th = (side == 1 && !d.dynamic && d.op != PBG_OP_NONE && w.theta[0]) ? w.theta[0] + (size_t)rel_std * D : nullptr;
-    apply_operator<VEC>(z, x, xrow, th, d.op, D, lane, w.glob[side], sc);
-    float yn = prepare_row<VEC>(z, d.cmp);
-    load_row<VEC>(q, a.Q[side] + (size_t)er * d.Dp, D, lane);
-    float s = 0.f;
+  if (!last) return;
+  if (lane == 0)
 #pragma unroll
-    for (int c = 0; c < VEC; ++c) s += f4dot(q[c], z[c]);
-    s = warp_sum(s);
-    if (d.cmp >= PBG_CMP_L2) {
-      float qv = (yn - 2.0f * s) + a.qn[side][er];
-      s = d.cmp == PBG_CMP_L2 ? -sqrtf(fmaxf(qv, 1e-30f)) : -qv;
-    }
-    neg = s;
+    for (int k = 0; k < 8; ++k) sm[wl][k] = v[k];
+  __syncthreads();
+  if (threadIdx.x < 8) {
+    double s = 0.0;
+    for (int u = 0; u < GATHER_WARPS; ++u) s += sm[u][threadIdx.x];
+    a.part[(size_t)blockIdx.x * 8 + threadIdx.x] = s;
+    __threadfence();
   }
-  if (lane == 0 && a.pos[side][ei] > neg) atomicAdd(&out8[6 + side], 1.0);
+  __syncthreads();
+  if (threadIdx.x == 0) closing = atomicAdd(a.done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (closing) close_eval(a.part, gridDim.x, a.done, out8);
 }
 
-size_t pbg_allnegs_bytes(int B, int Dp, int slab) {
-  size_t f = 2ull * B * Dp + 2ull * B + 2ull * B + (size_t)slab * Dp + slab;      // Q, qn, pos, Y, yn
-  size_t tiles = (size_t)(slab + AN_TILE - 1) / AN_TILE;
-  f += 3ull * tiles * B + 6ull * B;                                               // partials, running state
-  return f * 4 + 4096;
+// scratch of the evaluation; `slab`: candidates per side prepared at a time
+static void allnegs_layout(AllNegs &a, char *mem, int maxB, int Dp, int Dpb, int slab, bool planes, size_t &bytes) {
+  size_t off = 0;
+  auto take = [&](size_t n) { char *r = mem ? mem + off : nullptr; off += (n + 255) / 256 * 256; return r; };
+  const int tiles = planes ? slab / 128 : slab / AN_TILE;
+  const size_t ctas = (2 * (size_t)maxB + GATHER_WARPS - 1) / GATHER_WARPS;
+  for (int s = 0; s < 2; ++s) {
+    a.Q[s] = (float *)take((size_t)maxB * Dp * 4);
+    a.qn[s] = (float *)take((size_t)maxB * 4); a.pos[s] = (float *)take((size_t)maxB * 4); a.auc[s] = (int *)take((size_t)maxB * 4);
+    a.Y[s] = planes ? nullptr : (float *)take((size_t)slab * Dp * 4);
+    a.yn[s] = (float *)take((size_t)slab * 4);
+    a.pcnt[s] = (int *)take((size_t)tiles * maxB * 4); a.pa[s] = (float *)take((size_t)tiles * maxB * 4); a.pb[s] = (float *)take((size_t)tiles * maxB * 4);
+    a.cnt[s] = (int *)take((size_t)maxB * 4); a.ra[s] = (float *)take((size_t)maxB * 4); a.rb[s] = (float *)take((size_t)maxB * 4);
+  }
+  a.QB = planes ? (unsigned short *)take(6 * (size_t)maxB * Dpb * 2) : nullptr;
+  a.YB = planes ? (unsigned short *)take(6 * (size_t)slab * Dpb * 2) : nullptr;
+  a.part = (double *)take(ctas * 8 * 8);
+  a.slab = slab; a.qrows = maxB; a.Dpb = Dpb; a.tiles = tiles;
+  bytes = off;
+}
+
+// Slabs of 8192 candidates, or with planes as many as keep both sides inside about 96 MB (they are read from L2): a
+// slab's launches have a last round of tiles that leaves SMs idle, so fewer and larger ones are better; never more than
+// the largest table has.
+size_t pbg_allnegs_bytes(int maxB, int D, bool planes, long long table_rows, int &slab) {
+  const int Dp = (D + 31) / 32 * 32, Dpb = (D + 7) / 8 * 8;
+  long long rows = 8192;
+  if (planes) {
+    rows = 96ll * 1024 * 1024 / (12ll * Dpb);
+    if (rows < 8192) rows = 8192;
+    if (rows > 65536) rows = 65536;
+  }
+  if (rows > table_rows) rows = table_rows;
+  slab = (int)((rows + 255) / 256 * 256);
+  AllNegs a;
+  size_t bytes;
+  allnegs_layout(a, nullptr, maxB, Dp, Dpb, slab, planes, bytes);
+  return bytes;
 }
 
 // Runs the whole evaluation of one batch against all rows of both tables; `mem` holds pbg_allnegs_bytes bytes.
-int launch_allnegs_eval(const WaveDims &d, const WaveBufs &w, char *mem, int B, int slab, int rel_std, float wrel,
-                        double *out8_dev, cudaStream_t st) {
+int launch_allnegs_eval(const WaveDims &d, const WaveBufs &w, char *mem, int maxB, int B, int slab, bool planes, int rel_std, float wrel,
+                        unsigned *done, double *out8, cudaStream_t st) {
   AllNegs a;
-  float *p = (float *)mem;
-  auto take = [&](size_t n) { float *r = p; p += (n + 63) / 64 * 64; return r; };
-  a.B = B; a.slab = slab;
-  a.Q[0] = take((size_t)B * d.Dp); a.Q[1] = take((size_t)B * d.Dp);
-  a.qn[0] = take(B); a.qn[1] = take(B); a.pos[0] = take(B); a.pos[1] = take(B);
-  a.Y = take((size_t)slab * d.Dp); a.yn = take(slab);
-  const int tiles_slab = (slab + AN_TILE - 1) / AN_TILE;
-  a.pcnt = (int *)take((size_t)tiles_slab * B); a.pa = take((size_t)tiles_slab * B); a.pb = take((size_t)tiles_slab * B);
-  for (int s = 0; s < 2; ++s) { a.cnt[s] = (int *)take(B); a.ra[s] = take(B); a.rb[s] = take(B); }
+  size_t bytes;
+  allnegs_layout(a, mem, maxB, d.Dp, (d.D + 7) / 8 * 8, slab, planes, bytes);
+  a.B = B; a.done = done;
   int launches = 0;
   const int vec = (d.D + 127) / 128;
   const int ectas = (B + GATHER_WARPS - 1) / GATHER_WARPS;
-  cudaMemsetAsync(out8_dev, 0, 8 * sizeof(double), st);
 #define AN_V(K, ...) do { if (vec <= 1) K<1>__VA_ARGS__; else if (vec <= 2) K<2>__VA_ARGS__; else if (vec <= 4) K<4>__VA_ARGS__; else if (vec <= 8) K<8>__VA_ARGS__; else K<16>__VA_ARGS__; } while (0)
   AN_V(allnegs_rows_kernel, <<<ectas, 32 * GATHER_WARPS, 0, st>>>(d, w, a, rel_std));
   ++launches;
-  for (int side = 0; side < 2; ++side) {
-    if (!d.neg_enabled[side]) continue;
-    const long long N = d.n_rows[side];
-    bool first = true;
-    for (long long row0 = 0; row0 < N; row0 += slab) {
-      const int n = (int)(N - row0 < slab ? N - row0 : slab);
-      const int sctas = (n + GATHER_WARPS - 1) / GATHER_WARPS;
-      AN_V(allnegs_slab_kernel, <<<sctas, 32 * GATHER_WARPS, 0, st>>>(d, w, a, side, row0, n, rel_std));
-      const int ntiles = (n + AN_TILE - 1) / AN_TILE;
-      dim3 g((B + AN_TILE - 1) / AN_TILE, ntiles);
-      allnegs_score_kernel<<<g, 256, 0, st>>>(d, w, a, side, row0, n);
-      allnegs_merge_kernel<<<(B + 127) / 128, 128, 0, st>>>(d, a, side, ntiles, first ? 1 : 0);
-      first = false;
-      launches += 3;
-    }
+  long long most = 0;
+  for (int s = 0; s < 2; ++s) if (d.neg_enabled[s] && d.n_rows[s] > most) most = d.n_rows[s];
+  for (long long row0 = 0; row0 == 0 || row0 < most; row0 += slab) {
+    const int n = (int)(most - row0 < slab ? most - row0 : slab);
+    const int sctas = (n + GATHER_WARPS - 1) / GATHER_WARPS, first = row0 == 0, last = row0 + slab >= most;
+    AN_V(allnegs_slab_kernel, <<<dim3(sctas + (first ? ectas : 0), 2), 32 * GATHER_WARPS, 0, st>>>(d, w, a, row0, rel_std, sctas, first));
+    if (planes) launch_allnegs_score_tc(d, w, a, row0, st);
+    else allnegs_score_kernel<<<dim3((B + AN_TILE - 1) / AN_TILE, (n + AN_TILE - 1) / AN_TILE, 2), 256, 0, st>>>(d, w, a, row0);
+    allnegs_merge_kernel<<<(2 * B + GATHER_WARPS - 1) / GATHER_WARPS, 32 * GATHER_WARPS, 0, st>>>(d, w, a, row0, first, last, wrel, out8);
+    launches += 3;
   }
-  allnegs_finish_kernel<<<1, 256, 0, st>>>(d, w, a, wrel, out8_dev);
-  dim3 ga(ectas, 2);
-  AN_V(allnegs_auc_kernel, <<<ga, 32 * GATHER_WARPS, 0, st>>>(d, w, a, rel_std, out8_dev));
 #undef AN_V
   pbg_note_launch();
-  return launches + 2;
+  return launches;
 }

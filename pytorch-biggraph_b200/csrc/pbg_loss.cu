@@ -489,87 +489,108 @@ int launch_export_scores(const WaveDims &d, const WaveBatches &wb, const WaveBuf
 }
 
 // ---- evaluation (RankingEvaluator, torchbiggraph/eval.py:43-81), one batch at a time -------------
-// rank of every positive among its negatives, before the loss kernel turns S into coefficients
-__global__ void __launch_bounds__(32 * LOSS_WARPS) rank_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
-  int lane = threadIdx.x & 31;
-  long long item = (long long)blockIdx.x * LOSS_WARPS + (threadIdx.x >> 5);
-  long long per_prob = (long long)d.nblk * d.Pm;
-  if (item >= 2 * per_prob) return;
-  int p = (int)(item / per_prob);
-  long long rem = item - p * per_prob;
-  int blk = (int)(rem / d.Pm), i = (int)(rem - (long long)blk * d.Pm);
-  BlockInfo bi = block_info(d, wb, blk);
-  size_t prow = (size_t)blk * d.Pm + i;
-  if (i >= bi.n || !d.neg_enabled[p]) { if (lane == 0) w.rankrow[p][prow] = 0; return; }
-  const float *S = w.S[p] + prow * d.Ms;
-  const float s = w.spos[p][prow];
-  int ge = 0;
-  for (int j = lane; j < d.Mm; j += 32) {
-    if (j < d.Pm && (!d.batch_negs || j >= bi.Pl)) continue;             // column does not exist in the reference's matrix
-    float v = col_masked(d, bi, 1, i, j) ? PBG_MASKED : S[j];
-    ge += v >= s;
-  }
-  ge = warp_sum_int(ge);
-  if (lane == 0) w.rankrow[p][prow] = ge + 1;
-}
-
-// randomized AUC (torchbiggraph/util.py:415-428): `count` random (positive, negative) pairs per side
-__global__ void auc_kernel(WaveDims d, WaveBatches wb, WaveBufs w, double *out8) {
-  int p = blockIdx.y;
-  int smp = blockIdx.x * blockDim.x + threadIdx.x;
-  int count = wb.n[0];
-  if (smp >= count || !d.neg_enabled[p]) return;
-  BlockInfo b0 = block_info(d, wb, 0);
-  int Pl = b0.Pl, cols = d.batch_negs ? Pl + d.U : d.U;
-  if (Pl == 0 || cols == 0) return;
-  unsigned long long h = pbg_mix64(w.seed ^ pbg_mix64(0xA0C0FFEEull + (unsigned long long)p * 0x10001ull + smp));
-  int ei = (int)(h % (unsigned long long)count);
-  h = pbg_mix64(h);
-  long long flat = (long long)(h % ((unsigned long long)count * cols));
-  int er = (int)(flat / cols), j = (int)(flat - (long long)er * cols);
-  int src = d.batch_negs ? (j < Pl ? j : d.Pm + (j - Pl)) : d.Pm + j;
-  int c = er / Pl, i = er - c * Pl;
-  BlockInfo bi = block_info(d, wb, c);
-  float neg = col_masked(d, bi, 1, i, src) ? PBG_MASKED : w.S[p][((size_t)c * d.Pm + i) * d.Ms + src];
-  float pos = w.spos[p][(size_t)(ei / Pl) * d.Pm + (ei % Pl)];
-  if (pos > neg) atomicAdd(&out8[6 + 0], p == 0 ? 1.0 : 0.0), atomicAdd(&out8[7], p == 1 ? 1.0 : 0.0);
-}
-
-// out8: loss, pos_rank, mrr, r1, r10, r50 (sums over both sides' ranks), then AUC hit counts per side
-__global__ void __launch_bounds__(256) eval_reduce_kernel(WaveDims d, WaveBatches wb, WaveBufs w, double *out8) {
-  __shared__ double sm[6][256];
-  int t = threadIdx.x;
-  double acc[6] = {0, 0, 0, 0, 0, 0};
-  int rows = d.Cm * d.Pm;
-  for (int r = t; r < rows; r += 256) {
-    int c = r / d.Pm, i = r - c * d.Pm;
-    BlockInfo bi = block_info(d, wb, c);
-    if (i >= bi.n) continue;
-    size_t prow = (size_t)c * d.Pm + i;
-    acc[0] += (double)w.lossrow[0][prow] + (double)w.lossrow[1][prow];
-    for (int p = 0; p < 2; ++p) {
-      int rk = w.rankrow[p][prow];
-      if (rk <= 0) continue;
-      acc[1] += rk; acc[2] += 1.0 / rk; acc[3] += rk <= 1; acc[4] += rk <= 10; acc[5] += rk <= 50;
+// One warp per positive row and problem, one pass over its scores (16-byte loads): rank among the negatives, the loss
+// (softmax with a running maximum), the row's sample of the randomized AUC (torchbiggraph/util.py:415-428: `count` random
+// (positive, negative) pairs per side); the CTA's eight rows are summed and the last CTA adds up the CTAs' sums.
+// The score matrix is read once and not written.  (Rank, AUC, loss and sum as kernels of their own, the loss with the
+// coefficient matrix it writes for training, took 107 us on 5000 edges against 1000 negatives a side.)
+__global__ void __launch_bounds__(32 * LOSS_WARPS) eval_rows_kernel(WaveDims d, WaveBatches wb, WaveBufs w, double *part, unsigned *done, double *out8) {
+  __shared__ double sm[LOSS_WARPS][8];
+  __shared__ bool closing;
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const long long item = (long long)blockIdx.x * LOSS_WARPS + wl, per_prob = (long long)d.nblk * d.Pm;
+  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  const int p = item >= per_prob ? 1 : 0;
+  const long long rem = item - p * per_prob;
+  const int blk = (int)(rem / d.Pm), i = (int)(rem - (long long)blk * d.Pm);
+  if (item < 2 * per_prob) {
+    const BlockInfo bi = block_info(d, wb, blk);
+    if (i < bi.n) {
+      const size_t prow = (size_t)blk * d.Pm + i;
+      const float *S = w.S[p] + prow * d.Ms;
+      const float s = w.spos[p][prow];
+      const float wr = wb.wrel[bi.b] * (w.ew ? w.ew[bi.e0 + i] : 1.0f);
+      const bool enabled = d.neg_enabled[p] != 0;
+      const int Mlog = !enabled ? 0 : (d.batch_negs ? bi.Pl + d.U : d.U);
+      int ge = 0;
+      float acc = 0.f, m = -INFINITY;
+      if (enabled) {
+        for (int j0 = lane * 4; j0 < d.Mm; j0 += 128) {
+          const float4 q = ld4(S + j0);
+          float x[4] = {q.x, q.y, q.z, q.w};
+          float mx = -INFINITY;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int j = j0 + u;
+            const bool exists = j < d.Pm ? (d.batch_negs && j < bi.Pl) : j < d.Mm;      // a column of the reference's matrix
+            const bool live = exists && (j >= d.Pm || (j != i && j < bi.n));
+            ge += exists && (live ? x[u] : PBG_MASKED) >= s;
+            x[u] = live ? x[u] : -INFINITY;
+            mx = fmaxf(mx, x[u]);
+          }
+          if (d.loss == PBG_LOSS_SOFTMAX) {
+            if (mx > m) { acc *= expf(m - mx); m = mx; }              // (the first time: 0 x exp(-inf) = 0)
+            if (m > -INFINITY)
+#pragma unroll
+              for (int u = 0; u < 4; ++u) acc += expf(x[u] - m);
+          } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (x[u] > -INFINITY) acc += d.loss == PBG_LOSS_RANKING ? fmaxf(0.f, (x[u] - s) + d.margin) : softplusf(x[u]);
+          }
+        }
+      }
+      ge = warp_sum_int(ge);
+      float lossv = 0.f;
+      if (d.loss == PBG_LOSS_SOFTMAX) {
+        const float mw = warp_max(m);
+        const float z = warp_sum(m > -INFINITY ? acc * expf(m - mw) : 0.f);
+        float mm = fmaxf(mw, s);
+        if (mw == -INFINITY) mm = fmaxf(s, PBG_MASKED);               // every column masked
+        if (Mlog > 0) lossv = -s + mm + logf((mw > -INFINITY ? z * expf(mw - mm) : 0.f) + expf(s - mm));
+      } else {
+        acc = warp_sum(acc);
+        lossv = d.loss == PBG_LOSS_RANKING ? (Mlog > 0 ? acc : 0.f) : (Mlog > 0 ? acc / (float)Mlog : 0.f) + softplusf(-s);
+      }
+      if (lane == 0) {
+        v[0] = (double)(wr * lossv);
+        if (enabled) {
+          const int rk = ge + 1;
+          v[1] = rk; v[2] = 1.0 / rk; v[3] = rk <= 1; v[4] = rk <= 10; v[5] = rk <= 50;
+          const int count = wb.n[0], smp = blk * bi.Pl + i;
+          if (Mlog > 0) {
+            unsigned long long h = pbg_mix64(w.seed ^ pbg_mix64(0xA0C0FFEEull + (unsigned long long)p * 0x10001ull + smp));
+            const int ei = (int)(h % (unsigned long long)count);
+            h = pbg_mix64(h);
+            const long long flat = (long long)(h % ((unsigned long long)count * Mlog));
+            const int er = (int)(flat / Mlog), j = (int)(flat - (long long)er * Mlog);
+            const int src = d.batch_negs ? (j < bi.Pl ? j : d.Pm + (j - bi.Pl)) : d.Pm + j;
+            const int c = er / bi.Pl, ii = er - c * bi.Pl;
+            const BlockInfo b2 = block_info(d, wb, c);
+            const float neg = col_masked(d, b2, 1, ii, src) ? PBG_MASKED : w.S[p][((size_t)c * d.Pm + ii) * d.Ms + src];
+            v[6 + p] = w.spos[p][(size_t)(ei / bi.Pl) * d.Pm + (ei % bi.Pl)] > neg ? 1.0 : 0.0;
+          }
+        }
+      }
     }
   }
-  for (int k = 0; k < 6; ++k) sm[k][t] = acc[k];
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) sm[wl][k] = v[k];
   __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (t < o) for (int k = 0; k < 6; ++k) sm[k][t] += sm[k][t + o];
-    __syncthreads();
+  if (threadIdx.x < 8) {
+    double s = 0.0;
+    for (int u = 0; u < LOSS_WARPS; ++u) s += sm[u][threadIdx.x];
+    part[(size_t)blockIdx.x * 8 + threadIdx.x] = s;
+    __threadfence();
   }
-  if (t < 6) out8[t] = sm[t][0];
+  __syncthreads();
+  if (threadIdx.x == 0) closing = atomicAdd(done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (closing) close_eval(part, gridDim.x, done, out8);
 }
 
-// call order: gather, score, launch_eval_ranks (this), launch_loss, launch_eval_reduce
-int launch_eval(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, double *out8_dev, cudaStream_t st) {
-  long long items = 2ll * d.nblk * d.Pm;
-  cudaMemsetAsync(out8_dev, 0, 8 * sizeof(double), st);
-  rank_kernel<<<(int)((items + LOSS_WARPS - 1) / LOSS_WARPS), 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
-  dim3 g((wb.n[0] + 127) / 128, 2);
-  auc_kernel<<<g, 128, 0, st>>>(d, wb, w, out8_dev);
-  loss_kernel<<<(int)((items + LOSS_WARPS - 1) / LOSS_WARPS), 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
-  eval_reduce_kernel<<<1, 256, 0, st>>>(d, wb, w, out8_dev);
-  return 4;
+int launch_eval(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, double *part, unsigned *done, double *out8, cudaStream_t st) {
+  eval_rows_kernel<<<pbg_eval_ctas(d.nblk, d.Pm), 32 * LOSS_WARPS, 0, st>>>(d, wb, w, part, done, out8);
+  return 1;
 }
