@@ -35,6 +35,10 @@ __device__ __forceinline__ float coef_from_dscore(int cmp, float dS, float S) {
   return dS;
 }
 
+// NV > 0: the row (at most 32 NV columns) is read into registers before the first coefficient is written.  Written column
+// by column behind the reads, every read waited for the write before it (the compiler cannot tell the rows apart): 24 to
+// 31 us for 2 x 70 blocks of 100 rows x 200 columns where the bytes take 4.  NV == 0: rows of any length, column by column.
+template <int NV>
 __global__ void __launch_bounds__(32 * LOSS_WARPS) loss_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   int lane = threadIdx.x & 31;
   long long item = (long long)blockIdx.x * LOSS_WARPS + (threadIdx.x >> 5);
@@ -71,68 +75,85 @@ __global__ void __launch_bounds__(32 * LOSS_WARPS) loss_kernel(WaveDims d, WaveB
   const int Mlog = !enabled ? 0 : (d.batch_negs ? bi.Pl + d.U : d.U);
   float lossv = 0.f, ds = 0.f, rowsum = 0.f;
   int viol = 0;
+  constexpr int NR = NV > 0 ? NV : 1;
+  float sv[NR];
+  unsigned live = 0u;                                 // bit u: column lane + 32 u counts
+  if (NV > 0) {
+#pragma unroll
+    for (int u = 0; u < NR; ++u) {
+      const int j = lane + 32 * u;
+      const bool c = j < Mm && !col_masked(d, bi, enabled, i, j);
+      sv[u] = c ? S[j] : 0.f;
+      live |= c ? 1u << u : 0u;
+    }
+  }
+  // every live column j with its score, in the order j = lane, lane + 32, ...
+  auto each = [&](auto &&f) {
+    if (NV > 0) {
+#pragma unroll
+      for (int u = 0; u < NR; ++u) if (live >> u & 1u) f(lane + 32 * u, sv[u]);
+    } else {
+      for (int j = lane; j < Mm; j += 32) if (!col_masked(d, bi, enabled, i, j)) f(j, S[j]);
+    }
+  };
+  // writes the row: f(score) in the live columns, zeros elsewhere (the diagonal is filled below)
+  auto fill = [&](auto &&f) {
+    if (NV > 0) {
+#pragma unroll
+      for (int u = 0; u < NR; ++u) {
+        const int j = lane + 32 * u;
+        const float t = live >> u & 1u ? f(sv[u]) : 0.f;
+        rowsum += t;
+        if (j < d.Ms) put(j, t);
+      }
+    } else {
+      for (int j = lane; j < d.Ms; j += 32) {
+        const float t = j < Mm && !col_masked(d, bi, enabled, i, j) ? f(S[j]) : 0.f;
+        rowsum += t;
+        put(j, t);
+      }
+    }
+  };
 
   if (d.loss == PBG_LOSS_SOFTMAX) {
     // -s + log(e^s + sum_j e^S_ij); masked entries are e^-1e9 = 0 (losses.py:143-159)
-    float mx = -INFINITY;
-    for (int j = lane; j < Mm; j += 32)
-      if (!col_masked(d, bi, enabled, i, j)) mx = fmaxf(mx, S[j]);
-    mx = warp_max(mx);
     if (Mlog > 0) {
+      float mx = -INFINITY;
+      each([&](int, float x) { mx = fmaxf(mx, x); });
+      mx = warp_max(mx);
       float m = fmaxf(mx, s);
       if (mx == -INFINITY) m = fmaxf(s, PBG_MASKED);      // every column masked
       float z = 0.f;
-      for (int j = lane; j < Mm; j += 32)
-        if (!col_masked(d, bi, enabled, i, j)) { z += expf(S[j] - m); viol += S[j] > s; }
+      each([&](int, float x) { z += expf(x - m); viol += x > s; });
       z = warp_sum(z);
       float es = expf(s - m);
       float Z = z + es;
       lossv = -s + m + logf(Z);
       ds = es / Z - 1.0f;
       float invZ = 1.0f / Z;
-      for (int j = lane; j < d.Ms; j += 32) {
-        float t = 0.f;
-        if (j < Mm && !col_masked(d, bi, enabled, i, j)) t = coef_from_dscore(d.cmp, wr * expf(S[j] - m) * invZ, S[j]);
-        if (j == i) t = 0.f;                                // filled below
-        rowsum += t;
-        put(j, t);
-      }
+      fill([&](float x) { return coef_from_dscore(d.cmp, wr * expf(x - m) * invZ, x); });
     } else {
-      for (int j = lane; j < d.Ms; j += 32) put(j, 0.f);    // losses.py:139-140: loss 0, no gradient
+      fill([&](float) { return 0.f; });                    // losses.py:139-140: loss 0, no gradient
     }
   } else if (d.loss == PBG_LOSS_RANKING) {
     // sum_j max(0, margin - s + S_ij) (losses.py:116-122)
     if (Mlog > 0) {
-      for (int j = lane; j < d.Ms; j += 32) {
-        float t = 0.f;
-        if (j < Mm && !col_masked(d, bi, enabled, i, j)) {
-          float sj = S[j];
-          float v = (sj - s) + d.margin;
-          viol += sj > s;
-          if (v > 0.f) { lossv += v; ds -= 1.0f; t = coef_from_dscore(d.cmp, wr, sj); }
-        }
-        rowsum += t;
-        put(j, t);
-      }
+      each([&](int, float x) {
+        const float v = (x - s) + d.margin;
+        viol += x > s;
+        if (v > 0.f) { lossv += v; ds -= 1.0f; }
+      });
+      fill([&](float x) { return (x - s) + d.margin > 0.f ? coef_from_dscore(d.cmp, wr, x) : 0.f; });
       lossv = warp_sum(lossv);
       ds = warp_sum(ds);
     } else {
-      for (int j = lane; j < d.Ms; j += 32) put(j, 0.f);
+      fill([&](float) { return 0.f; });
     }
   } else {
     // softplus(-s) + (1/M) sum_j softplus(S_ij), M counts masked columns (losses.py:61-80)
     float nw = Mlog > 0 ? 1.0f / (float)Mlog : 0.f;
-    for (int j = lane; j < d.Ms; j += 32) {
-      float t = 0.f;
-      if (j < Mm && !col_masked(d, bi, enabled, i, j)) {
-        float sj = S[j];
-        viol += sj > s;
-        lossv += softplusf(sj);
-        t = coef_from_dscore(d.cmp, wr * nw * sigmoidf(sj), sj);
-      }
-      rowsum += t;
-      put(j, t);
-    }
+    each([&](int, float x) { viol += x > s; lossv += softplusf(x); });
+    fill([&](float x) { return coef_from_dscore(d.cmp, wr * nw * sigmoidf(x), x); });
     lossv = warp_sum(lossv) * nw + softplusf(-s);
     ds = -sigmoidf(-s);
   }
@@ -159,7 +180,13 @@ __global__ void colsum_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   BlockInfo bi = block_info(d, wb, blk);
   float s = 0.f;
   const float *T = w.S[p] + (size_t)blk * d.Pm * d.Ms + j;
-  for (int i = 0; i < bi.n; ++i) s += T[(size_t)i * d.Ms];
+  for (int i0 = 0; i0 < bi.n; i0 += 16) {              // sixteen reads in flight; the sum is one chain
+    float v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) v[u] = i0 + u < bi.n ? T[(size_t)(i0 + u) * d.Ms] : 0.f;
+#pragma unroll
+    for (int u = 0; u < 16; ++u) s += v[u];
+  }
   w.coef[p][(size_t)blk * d.Mm + j] = s;
 }
 
@@ -168,6 +195,7 @@ __global__ void colsum_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
 // (side, block, row m) merges them into the combined coefficient matrix A[side] (see WaveBufs), so
 // that the backward pass is ONE product per side with K = Mm, and keeps the row sum of A for the
 // l2 family (coefficient of the row's own |y|^2 term).
+template <int NV>
 __global__ void __launch_bounds__(32 * LOSS_WARPS) coef_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   int lane = threadIdx.x & 31;
   long long item = (long long)blockIdx.x * LOSS_WARPS + (threadIdx.x >> 5);
@@ -187,15 +215,26 @@ __global__ void __launch_bounds__(32 * LOSS_WARPS) coef_kernel(WaveDims d, WaveB
   float rowsum = 0.f;
   // bf16-plane tier: the planes of the row beside it
   unsigned short *ABr = w.AB[side] ? w.AB[side] + ((size_t)blk * w.npl * d.Mm + m) * w.Kb : nullptr;
-  for (int j = lane; j < w.Ma; j += 32) {
-    float a = 0.f;
-    if (j < d.Mm) {
-      if (j < bi.n) a += Tcol[(size_t)j * d.Ms + m];
-      if (m < bi.n) a += Trow[j];
+  // NV columns per lane at a time, read before the first of them is written (see loss_kernel)
+  for (int j0 = lane; j0 < w.Ma; j0 += 32 * NV) {
+    float a[NV];
+#pragma unroll
+    for (int u = 0; u < NV; ++u) {
+      const int j = j0 + 32 * u;
+      a[u] = 0.f;
+      if (j < d.Mm) {
+        if (j < bi.n) a[u] += Tcol[(size_t)j * d.Ms + m];
+        if (m < bi.n) a[u] += Trow[j];
+      }
     }
-    rowsum += a;
-    A[j] = a;
-    if (ABr) put_planes1(ABr + j, (size_t)d.Mm * w.Kb, a, w.npl);
+#pragma unroll
+    for (int u = 0; u < NV; ++u) {
+      const int j = j0 + 32 * u;
+      if (j >= w.Ma) break;
+      rowsum += a[u];
+      A[j] = a[u];
+      if (ABr) put_planes1(ABr + j, (size_t)d.Mm * w.Kb, a[u], w.npl);
+    }
   }
   if (d.cmp >= PBG_CMP_L2) {
     rowsum = warp_sum(rowsum);
@@ -327,16 +366,23 @@ __global__ void __launch_bounds__(32 * LOSS_WARPS) coef_tile_kernel(WaveDims d, 
     t[4 * q] = v.x; t[4 * q + 1] = v.y; t[4 * q + 2] = v.z; t[4 * q + 3] = v.w;
   }
   const float *orow = w.S[1 - side] + (size_t)blk * d.Pm * d.Ms;              // T_other[m][j]
+  // All 32 values of the direct term are requested before the first is used: added as they came, each read waited for the
+  // one before it (12 us for 20 blocks of 100 rows, 20 us for 70 blocks of 200).
+  float o[32];
+#pragma unroll
+  for (int r = 0; r < 32; ++r) o[r] = m0 + r < bi.n && j < d.Mm ? orow[(size_t)(m0 + r) * d.Ms + j] : 0.f;
+#pragma unroll
+  for (int r = 0; r < 32; ++r) {
+    const float a = t[r] + o[r];
+    t[r] = m0 + r >= bi.n ? t[r] : a;                   // (the sum is left alone where there is no second term)
+    if (j >= d.Mm || m0 + r >= d.Mm) t[r] = 0.f;
+  }
   float *A = w.A[side] + (size_t)blk * d.Mm * w.Ma;
   if (!PL) {
 #pragma unroll
     for (int r = 0; r < 32; ++r) {
       int m = m0 + r;
-      if (m < d.Mm && j < w.Ma) {
-        float a = j < d.Mm ? t[r] : 0.f;
-        if (m < bi.n && j < d.Mm) a += orow[(size_t)m * d.Ms + j];
-        A[(size_t)m * w.Ma + j] = a;
-      }
+      if (m < d.Mm && j < w.Ma) A[(size_t)m * w.Ma + j] = t[r];
     }
     return;
   }
@@ -352,10 +398,7 @@ __global__ void __launch_bounds__(32 * LOSS_WARPS) coef_tile_kernel(WaveDims d, 
     unsigned pl[2][3];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      int m = m0 + r + h;
-      float a = (m < d.Mm && j < d.Mm) ? t[r + h] : 0.f;
-      if (m < bi.n && j < d.Mm) a += orow[(size_t)m * d.Ms + j];
-      bf16_planes(a, pl[h][0], pl[h][1], pl[h][2]);
+      bf16_planes(t[r + h], pl[h][0], pl[h][1], pl[h][2]);
     }
     // what the neighbour stores: its row is m for an even neighbour, m + 1 for an odd one
     unsigned give[3], keep[3];
@@ -384,7 +427,11 @@ int launch_loss(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cud
   else if (dotlike && d.loss == PBG_LOSS_SOFTMAX && d.Ms <= 256) loss_softmax_kernel<8><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
   else if (dotlike && d.loss == PBG_LOSS_SOFTMAX && d.Ms <= 512) loss_softmax_kernel<16><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
   else if (dotlike && d.loss == PBG_LOSS_SOFTMAX && d.Ms <= 1024) loss_softmax_kernel<32><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
-  else loss_kernel<<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
+  else if (d.Ms <= 128) loss_kernel<4><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
+  else if (d.Ms <= 256) loss_kernel<8><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
+  else if (d.Ms <= 512) loss_kernel<16><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
+  else if (d.Ms <= 1024) loss_kernel<32><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
+  else loss_kernel<0><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
   if (!d.dynamic) {
     if (dotlike) {
       const int tiles = (d.Mm + 31) / 32;
@@ -393,7 +440,7 @@ int launch_loss(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cud
       else coef_tile_kernel<false><<<(int)((warps + LOSS_WARPS - 1) / LOSS_WARPS), 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
     } else {
       long long rows = 2ll * d.nblk * d.Mm;
-      coef_kernel<<<(int)((rows + LOSS_WARPS - 1) / LOSS_WARPS), 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
+      coef_kernel<8><<<(int)((rows + LOSS_WARPS - 1) / LOSS_WARPS), 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
     }
     return 2;
   }

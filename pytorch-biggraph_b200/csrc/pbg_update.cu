@@ -123,9 +123,19 @@ __global__ void __launch_bounds__(32 * UPD_WARPS) std_pullback_kernel(WaveDims d
   const BlockInfo bi = block_info(d, wb, blk);
   if (bi.n <= 0) return;
   const long long row = slot_row(d, wb, w, bi, side, r);
-  if (row < 0 || row >= d.n_rows[side]) return;
   const int D = d.D;
   float4 v[VEC], pg[VEC];
+  if (row < 0 || row >= d.n_rows[side]) {                    // no row behind the slot: nothing for param_sums to add
+#pragma unroll
+    for (int c = 0; c < VEC; ++c) {
+      const int dd = c * 128 + lane * 4;
+      if (dd < D) {
+        st4(w.GX[a] + ((size_t)blk * w.grows[a] + r) * d.Dp + dd, f4zero());
+        if (side == 1 && w.PG) st4(w.PG + ((size_t)blk * d.Mm + r) * d.Dp + dd, f4zero());
+      }
+    }
+    return;
+  }
   gz_row<VEC, CK>(v, d, w, a, blk, r, lane, d.reg_coef != 0.f && r < bi.n && r < d.Pm);
   if (side == 1 && w.PG) {
     const float xs = d.max_norm > 0.f ? w.rscale[(size_t)blk * d.Mm + r] : 1.0f;   // the raw row entered the operator scaled
@@ -150,7 +160,8 @@ __global__ void __launch_bounds__(32 * UPD_WARPS) std_pullback_kernel(WaveDims d
 //   param_step   beside the big hub rows: adds up a batch's partial rows and takes the dense AsyncAdagrad steps batch
 //                after batch (torchbiggraph/async_adagrad.py:75-85, train_cpu.py:215-230)
 // kinds: 0 operator row, 1 / 2 vector of the lhs / rhs entity type (one vector for both sides: two sums, one step)
-struct ParamJob { int sums, sum_kind[3], steps, step_kind[3]; float lr; };
+// cleared0 / cleared1: the pull-back has been over every row of that side
+struct ParamJob { int sums, sum_kind[3], steps, step_kind[3], cleared0, cleared1; float lr; };
 static inline int param_sum_ctas(const WaveDims &d, const ParamJob &job) { return job.sums * d.nblk * ((d.D + 127) / 128); }
 static inline int param_step_ctas(const WaveDims &d, const ParamJob &job) { return job.steps * ((d.D + 31) / 32); }
 
@@ -164,29 +175,30 @@ __device__ __forceinline__ void param_sums(const WaveDims &d, const WaveBatches 
   const BlockInfo bi = block_info(d, wb, blk);
   const float *src = kind == 0 ? (w.PG ? w.PG : w.GX[ARR_N1]) : kind == 1 ? w.GX[ARR_N0] : d.matrix_op ? w.R2 : w.GX[ARR_N1];
   src += (size_t)blk * d.Mm * d.Dp + dd;
+  // the rows of both sequences of this warp, four each in flight; rows without an entity behind them hold zeros where the
+  // pull-back has been over them, else (checked) their ids are looked at
+  const bool checked = kind == 0 ? !job.cleared1 : kind == 1 ? !job.cleared0 : !job.cleared1 || d.matrix_op;
+  float4 s[2] = {f4zero(), f4zero()};
+  if (bi.n > 0 && dd < d.D) {
+    for (int r0 = wl; r0 < d.Mm; r0 += 32) {
+      float4 v[8];
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int y = wl + 4 * h;
-    float4 s = f4zero();
-    if (bi.n > 0 && dd < d.D) {
-      for (int r0 = y; r0 < d.Mm; r0 += 32) {
-        float4 v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int r = r0 + 8 * u;
-          const long long row = r < d.Mm ? slot_row(d, wb, w, bi, side, r) : -1;
-          v[u] = row >= 0 && row < d.n_rows[side] ? ld4(src + (size_t)r * d.Dp) : f4zero();
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) s = s + v[u];
+      for (int u = 0; u < 8; ++u) {
+        const int r = r0 + 4 * u;
+        bool real = r < d.Mm;
+        if (checked && real) { const long long row = slot_row(d, wb, w, bi, side, r); real = row >= 0 && row < d.n_rows[side]; }
+        v[u] = real ? ld4(src + (size_t)r * d.Dp) : f4zero();
       }
-      if (kind == 0 && y == 0 && d.reg_coef != 0.f)
-        // N3 regularizer on the relation's parameters: sum(params^3) * number of chunks
-        // (regularizers.py:88-92), i.e. once per chunk block; theta is still the wave's snapshot here
-        s = s + n3_grad4(w.theta[0] + (size_t)wb.rel[bi.b] * d.D, dd, d.D, d.op == PBG_OP_COMPLEX_DIAGONAL) * d.reg_coef;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s[u & 1] = s[u & 1] + v[u];
     }
-    st4(sm + y * 128 + lane * 4, s);
+    if (kind == 0 && wl == 0 && d.reg_coef != 0.f)
+      // N3 regularizer on the relation's parameters: sum(params^3) * number of chunks
+      // (regularizers.py:88-92), i.e. once per chunk block; theta is still the wave's snapshot here
+      s[0] = s[0] + n3_grad4(w.theta[0] + (size_t)wb.rel[bi.b] * d.D, dd, d.D, d.op == PBG_OP_COMPLEX_DIAGONAL) * d.reg_coef;
   }
+  st4(sm + wl * 128 + lane * 4, s[0]);
+  st4(sm + (wl + 4) * 128 + lane * 4, s[1]);
   __syncthreads();
   if (wl == 0 && dd < d.D) {
     float4 t = ld4(sm + lane * 4);
@@ -207,10 +219,10 @@ __device__ __forceinline__ void param_step(const WaveDims &d, const WaveBatches 
   if (dd < d.D) {
     for (int b = y; b < d.k; b += UPD_WARPS) {
       float s = 0.f, s2 = 0.f;
-#pragma unroll 4
+#pragma unroll 10
       for (int c = 0; c < d.Cm; ++c) s += part[((size_t)b * d.Cm + c) * d.D];
       if (part2) {
-#pragma unroll 4
+#pragma unroll 10
         for (int c = 0; c < d.Cm; ++c) s2 += part2[((size_t)b * d.Cm + c) * d.D];
         s += s2;
       }
@@ -350,7 +362,13 @@ struct RowState {
   }
 };
 
-// Embedding rows: 4 warps per CTA, each with TILE row buffers in shared memory that it fills with
+// Rows a warp stages at once.  Narrow rows get more buffers than a tile has slots: a row of five to twelve slots, which
+// belongs to the tile of its first slot, is then on its way in one round instead of two or three one after the other --
+// the longest chain of the kernel.
+template <int VEC, int RULE>
+struct StageRows { enum { N = RULE == RULE_REL ? TILE : VEC == 1 ? 12 : TILE }; };
+
+// Embedding rows: 4 warps per CTA, each with row buffers in shared memory that it fills with
 // bulk asynchronous copies (cp.async.bulk, completion on the warp's mbarrier): the gradient rows
 // of a whole tile are in flight at once instead of one dependent 16-byte-per-lane load at a time.
 #define TILE_WARPS_EMB 4
@@ -364,12 +382,12 @@ template <int VEC, int RULE>
 struct TileWarps { enum { N = RULE == RULE_EMB ? TILE_WARPS_EMB : VEC > 8 ? UPD_WARPS / 2 : UPD_WARPS }; };
 
 template <int VEC, int RULE>
-__global__ void __launch_bounds__(32 * TileWarps<VEC, RULE>::N, RULE == RULE_EMB ? (VEC == 2 ? 6 : 3) : (VEC == 2 ? 4 : 2))
+__global__ void __launch_bounds__(32 * TileWarps<VEC, RULE>::N, RULE == RULE_EMB ? (VEC == 1 ? 8 : VEC == 2 ? 6 : 3) : (VEC == 2 ? 4 : 2))
 tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys,
                    const unsigned int *__restrict__ vals, float lr, float *__restrict__ psum,
                    long long *__restrict__ hublist, int *__restrict__ hubcnt, ParamJob job, int aside) {
-  constexpr int WARPS = TileWarps<VEC, RULE>::N;
-  extern __shared__ __align__(128) float stage_all[];        // [WARPS][TILE][Dp]
+  constexpr int WARPS = TileWarps<VEC, RULE>::N, STAGE = StageRows<VEC, RULE>::N;
+  extern __shared__ __align__(128) float stage_all[];        // [WARPS][STAGE][Dp]
   __shared__ __align__(8) unsigned long long sbar[WARPS];
   const unsigned FULL = 0xffffffffu;
   const unsigned long long SENT = ~0ull;
@@ -378,7 +396,7 @@ tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
   if (RULE == RULE_EMB && blockIdx.x < aside) { param_sums(d, wb, w, job, blockIdx.x, stage_all); return; }
   long long t0 = ((long long)(blockIdx.x - aside) * WARPS + wl) * TILE;
   if (t0 >= d.nocc) return;
-  float *stage = stage_all + (size_t)wl * TILE * d.Dp;
+  float *stage = stage_all + (size_t)wl * STAGE * d.Dp;
   const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&sbar[wl]);
   uint32_t phase = 0;
   int staged_lo = 0, staged_hi = 0;                           // window slots whose rows are in `stage`
@@ -397,7 +415,7 @@ tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
   unsigned int vB = pb < d.nocc ? vals[pb] : 0u;
   const int bB = (int)(vB / (unsigned int)d.spb);              // batch of this lane's slot
   if (__shfl_sync(FULL, kB, TILE - 1) < lo) return;          // tile holds only the other rule's rows
-  // Copies the gradient rows of window slots j0 .. j0+cnt-1 (cnt <= TILE) into the stage buffers and
+  // Copies the gradient rows of window slots j0 .. j0+cnt-1 (cnt <= STAGE) into the stage buffers and
   // waits for them; the wait is bounded (bit 1 of the error word when it runs out).
   auto stage_rows = [&](int j0, int cnt) {
     __syncwarp();                                            // everyone is done with the old rows
@@ -430,38 +448,53 @@ tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
     phase ^= 1u;
     staged_lo = j0; staged_hi = j0 + cnt;
   };
+  // What the tile's row segments are, from ballots alone: [first, last) are the window slots whose rows this warp reads --
+  // without a leading short row that belongs to an earlier tile, and with the rest of a trailing short row that begins here.
+  auto segment = [&](int i, unsigned long long key, int &run, bool &hub, bool &head_here) {
+    unsigned fm = __ballot_sync(FULL, kB == key);
+    unsigned rest = ~(fm >> i);
+    run = rest ? __ffs(rest) - 1 : 32 - i;                   // slots i .. i+run-1 of the window share the key
+    int back = 0;
+    if (i == 0) back = __clz(~__ballot_sync(FULL, kA == key)); // slots of this row just before the tile
+    head_here = back == 0;
+    hub = i + run >= 32 || back == 32 || back + run > SHORT_MAX;
+  };
+  int first = __popc(__ballot_sync(FULL, lane < TILE && kB < lo)), last = __popc(__ballot_sync(FULL, lane < TILE && kB < hi));
+  if (first >= last) return;
+  {
+    int run;
+    bool hub, head_here;
+    if (first == 0) {
+      segment(0, __shfl_sync(FULL, kB, 0), run, hub, head_here);
+      if (!hub && !head_here) first = run < TILE ? run : TILE;
+    }
+    if (first >= last) return;
+    if (last == TILE) {
+      const unsigned long long key = __shfl_sync(FULL, kB, TILE - 1);
+      const int start = __ffs(__ballot_sync(FULL, kB == key)) - 1;
+      segment(start, key, run, hub, head_here);
+      if (!hub && head_here) last = start + run;
+    }
+  }
   if (RULE == RULE_EMB) {
     // get the rows this tile will need moving towards L2 before the dependent loads start
 #pragma unroll
     for (int i = 0; i < TILE; ++i) {
+      if (i < first || i >= last) continue;
       unsigned long long key = __shfl_sync(FULL, kB, i);
-      if (key >= hi) break;
       int side = (!d.shared_table && key >= (unsigned long long)d.n_rows[0]) ? 1 : 0;
       const float *wr = w.W[side] + (size_t)(side ? key - (unsigned long long)d.n_rows[0] : key) * D;
       for (int f = lane * 32; f < D; f += 1024) asm volatile("prefetch.global.L2 [%0];" :: "l"(wr + f));
     }
-    int nvalid = __popc(__ballot_sync(FULL, lane < TILE && kB < hi));
-    if (nvalid > 0) stage_rows(0, nvalid);
-  } else {
-    // operator rows: the tile's slots of this rule (they follow the embedding rows' slots in the sorted list)
-    const int first = __popc(__ballot_sync(FULL, lane < TILE && kB < lo));
-    const int nvalid = __popc(__ballot_sync(FULL, lane < TILE && kB >= lo && kB < hi));
-    if (nvalid > 0) stage_rows(first, nvalid);
   }
-  int i = 0;
+  stage_rows(first, last - first < STAGE ? last - first : STAGE);
+  int i = first;
   while (i < TILE) {
     unsigned long long key = __shfl_sync(FULL, kB, i);
     if (key >= hi) return;                                   // sorted: nothing of this rule follows
-    if (key < lo) { ++i; continue; }
-    unsigned fm = __ballot_sync(FULL, kB == key);
-    unsigned rest = ~(fm >> i);
-    int run = rest ? __ffs(rest) - 1 : 32 - i;               // slots i .. i+run-1 of the window share the key
-    bool hits_end = i + run >= 32;
-    int back = 0;
-    if (i == 0) back = __clz(~__ballot_sync(FULL, kA == key)); // slots of this row just before the tile
-    bool head_here = back == 0;
-    bool hub = hits_end || back == 32 || back + run > SHORT_MAX;
-    if (!hub && !head_here) { i += run; continue; }          // short row owned by an earlier tile
+    int run;
+    bool hub, head_here;
+    segment(i, key, run, hub, head_here);
     int nproc = hub ? (run < TILE - i ? run : TILE - i) : run;
     RowState<VEC, RULE> rs;
     if (!hub) rs.load(d, w, key, lane);
@@ -488,10 +521,7 @@ tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
       }
       if (!in) break;
       if (b != cur_b) { cur_b = b; run_start = j; }
-      if (j >= staged_hi) {                                   // a short row that runs past the tile
-        int left = i + nproc - j;
-        stage_rows(j, left < TILE ? left : TILE);
-      }
+      if (j >= staged_hi) stage_rows(j, last - j < STAGE ? last - j : STAGE);       // more slots than buffers
       const float *gs = stage + (size_t)(j - staged_lo) * d.Dp;
 #pragma unroll
       for (int c = 0; c < VEC; ++c) {
@@ -988,7 +1018,7 @@ static int launch_pullback(const WaveDims &d, const WaveBatches &wb, const WaveB
   pbg_opt_in_smem((const void *)dyn_pullback_kernel<VEC, CK_DOT>, (int)smem);
   pbg_opt_in_smem((const void *)dyn_pullback_kernel<VEC, CK_COS>, (int)smem);
   pbg_opt_in_smem((const void *)dyn_pullback_kernel<VEC, CK_L2>, (int)smem);
-  job.sums = job.steps = 0; job.lr = rel_lr;
+  job.sums = job.steps = job.cleared0 = job.cleared1 = 0; job.lr = rel_lr;
   if (d.dynamic) {
     if (!rows_change && !has_op) return 0;
     const int first_q = rows_change ? 0 : 1;
@@ -1004,6 +1034,7 @@ static int launch_pullback(const WaveDims &d, const WaveBatches &wb, const WaveB
     if (!w.glob_shared) job.step_kind[job.steps++] = 2;
   }
   if (!rows_change && !(row_op && w.PG)) return 0;
+  job.cleared0 = rows_change; job.cleared1 = 1;
   const dim3 grid((unsigned)(((long long)d.nblk * d.Mm + UPD_WARPS - 1) / UPD_WARPS), rows_change ? 2 : 1);
   PBG_ROWS_CK(VEC, std_pullback_kernel, <<<grid, 32 * UPD_WARPS, smem, st>>>(d, wb, w, rows_change ? 0 : 1));
   return 1;
@@ -1026,13 +1057,13 @@ static int launch_update_vec(const WaveDims &d, const WaveBatches &wb, const Wav
   // which the caller's cudaGetLastError reports
   pbg_opt_in_smem((const void *)hub_update_kernel<VEC, RULE_EMB>, (int)hub_smem_max);
   pbg_opt_in_smem((const void *)hub_reduce_kernel<VEC>, (int)red_smem);
-  pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_EMB>, EMB_WARPS * TILE * VEC * 512);
+  pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_EMB>, EMB_WARPS * StageRows<VEC, RULE_EMB>::N * VEC * 512);
   ParamJob job;
   int launches = launch_pullback<VEC>(d, wb, w, rel_lr, job, st);
   int *hubcnt = us.hubcnt + 64 * (*us.turn & 1), *hubcnt_next = us.hubcnt + 64 * ((*us.turn + 1) & 1);
   ++*us.turn;
   const int sum_ctas = param_sum_ctas(d, job);
-  size_t tile_smem = (size_t)EMB_WARPS * TILE * d.Dp * 4;
+  size_t tile_smem = (size_t)EMB_WARPS * StageRows<VEC, RULE_EMB>::N * d.Dp * 4;
   if (sum_ctas && tile_smem < 8 * 128 * 4) tile_smem = 8 * 128 * 4;
   tile_update_kernel<VEC, RULE_EMB><<<sum_ctas + (unsigned)((tiles + EMB_WARPS - 1) / EMB_WARPS), 32 * EMB_WARPS, tile_smem, st>>>(
       d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, job, sum_ctas);
