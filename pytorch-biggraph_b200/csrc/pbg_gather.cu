@@ -155,6 +155,7 @@ __device__ __forceinline__ float positive_score(const float4 (&a)[VEC], const fl
 
 template <int VEC, bool PL>
 __global__ void __launch_bounds__(32 * GATHER_WARPS, VEC >= 8 ? 2 : 3) gather_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
+  pdl_begin();
   int lane = threadIdx.x & 31;
   long long item = (long long)blockIdx.x * GATHER_WARPS + (threadIdx.x >> 5);
   if (item >= (long long)d.nblk * d.Mm) return;
@@ -303,6 +304,7 @@ __global__ void __launch_bounds__(32 * GATHER_WARPS, VEC >= 8 ? 2 : 3) gather_ke
 // one (half the registers, three CTAs per SM instead of two).
 template <int VEC, bool PL>
 __global__ void __launch_bounds__(32 * GATHER_WARPS, VEC >= 16 ? 1 : VEC >= 8 ? 3 : 4) gather_plain_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
+  pdl_begin();
   int lane = threadIdx.x & 31;
   long long item = (long long)blockIdx.x * GATHER_WARPS + (threadIdx.x >> 5);
   if (item >= (long long)d.nblk * d.Mm) return;
@@ -382,6 +384,7 @@ __global__ void __launch_bounds__(32 * GATHER_WARPS, VEC >= 16 ? 1 : VEC >= 8 ? 
 // chunk's edges, the positive score against the lhs row already in N0.
 template <int VEC>
 __global__ void __launch_bounds__(32 * GATHER_WARPS) postop_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
+  pdl_begin();
   int lane = threadIdx.x & 31;
   long long item = (long long)blockIdx.x * GATHER_WARPS + (threadIdx.x >> 5);
   if (item >= (long long)d.nblk * d.Mm) return;
@@ -429,11 +432,11 @@ int launch_postop(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, c
   long long items = (long long)d.nblk * d.Mm;
   int ctas = (int)((items + GATHER_WARPS - 1) / GATHER_WARPS);
   int vec = (d.D + 127) / 128;
-  if (vec <= 1) postop_kernel<1><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-  else if (vec <= 2) postop_kernel<2><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-  else if (vec <= 4) postop_kernel<4><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-  else if (vec <= 8) postop_kernel<8><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-  else postop_kernel<16><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
+  if (vec <= 1) pbg_launch(postop_kernel<1>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+  else if (vec <= 2) pbg_launch(postop_kernel<2>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+  else if (vec <= 4) pbg_launch(postop_kernel<4>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+  else if (vec <= 8) pbg_launch(postop_kernel<8>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+  else pbg_launch(postop_kernel<16>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
   return 1;
 }
 
@@ -443,39 +446,40 @@ int launch_gather(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, c
   int vec = (d.D + 127) / 128;
   const bool plain = !d.dynamic && !d.matrix_op && d.max_norm <= 0.f && d.cmp == PBG_CMP_DOT && (d.op == PBG_OP_NONE || w.theta[0] == nullptr);
   if (plain && w.XB[0] && d.reg_coef == 0.f) {      // planes only: nothing reads the fp32 operand rows then
-    if (vec <= 1) gather_plain_kernel<1, true><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-    else if (vec <= 2) gather_plain_kernel<2, true><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-    else if (vec <= 4) gather_plain_kernel<4, true><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-    else if (vec <= 8) gather_plain_kernel<8, true><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-    else gather_plain_kernel<16, true><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
+    if (vec <= 1) pbg_launch(gather_plain_kernel<1, true>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+    else if (vec <= 2) pbg_launch(gather_plain_kernel<2, true>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+    else if (vec <= 4) pbg_launch(gather_plain_kernel<4, true>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+    else if (vec <= 8) pbg_launch(gather_plain_kernel<8, true>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+    else pbg_launch(gather_plain_kernel<16, true>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
     return 1;
   }
   if (plain && !w.XB[0]) {
-    if (vec <= 1) gather_plain_kernel<1, false><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-    else if (vec <= 2) gather_plain_kernel<2, false><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-    else if (vec <= 4) gather_plain_kernel<4, false><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-    else if (vec <= 8) gather_plain_kernel<8, false><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-    else gather_plain_kernel<16, false><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
+    if (vec <= 1) pbg_launch(gather_plain_kernel<1, false>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+    else if (vec <= 2) pbg_launch(gather_plain_kernel<2, false>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+    else if (vec <= 4) pbg_launch(gather_plain_kernel<4, false>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+    else if (vec <= 8) pbg_launch(gather_plain_kernel<8, false>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+    else pbg_launch(gather_plain_kernel<16, false>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
     return 1;
   }
   if (w.XB[0]) {
-    if (vec <= 1) gather_kernel<1, true><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-    else if (vec <= 2) gather_kernel<2, true><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-    else if (vec <= 4) gather_kernel<4, true><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-    else if (vec <= 8) gather_kernel<8, true><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-    else gather_kernel<16, true><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
+    if (vec <= 1) pbg_launch(gather_kernel<1, true>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+    else if (vec <= 2) pbg_launch(gather_kernel<2, true>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+    else if (vec <= 4) pbg_launch(gather_kernel<4, true>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+    else if (vec <= 8) pbg_launch(gather_kernel<8, true>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+    else pbg_launch(gather_kernel<16, true>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
     return 1;
   }
-  if (vec <= 1) gather_kernel<1, false><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-  else if (vec <= 2) gather_kernel<2, false><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-  else if (vec <= 4) gather_kernel<4, false><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-  else if (vec <= 8) gather_kernel<8, false><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
-  else gather_kernel<16, false><<<ctas, 32 * GATHER_WARPS, 0, st>>>(d, wb, w);
+  if (vec <= 1) pbg_launch(gather_kernel<1, false>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+  else if (vec <= 2) pbg_launch(gather_kernel<2, false>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+  else if (vec <= 4) pbg_launch(gather_kernel<4, false>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+  else if (vec <= 8) pbg_launch(gather_kernel<8, false>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
+  else pbg_launch(gather_kernel<16, false>, ctas, 32 * GATHER_WARPS, 0, st, d, wb, w);
   return 1;
 }
 
 // One thread per occurrence slot (waves too large for the one-kernel sort, which builds its keys itself).
 __global__ void build_keys_kernel(WaveDims d, WaveBatches wb, WaveBufs w, unsigned long long *keys, unsigned int *vals) {
+  pdl_begin();
   int o = blockIdx.x * blockDim.x + threadIdx.x;
   if (o >= d.nocc) return;
   keys[o] = slot_key(d, wb, w, o);
@@ -484,7 +488,7 @@ __global__ void build_keys_kernel(WaveDims d, WaveBatches wb, WaveBufs w, unsign
 
 int launch_build_keys(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w,
                       unsigned long long *keys, unsigned int *vals, cudaStream_t st) {
-  build_keys_kernel<<<(d.nocc + 255) / 256, 256, 0, st>>>(d, wb, w, keys, vals);
+  pbg_launch(build_keys_kernel, (d.nocc + 255) / 256, 256, 0, st, d, wb, w, keys, vals);
   return 1;
 }
 
@@ -528,6 +532,7 @@ __device__ __forceinline__ void allnegs_q_planes(const AllNegs &a, int side, int
 
 template <int VEC>
 __global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_rows_kernel(WaveDims d, WaveBufs w, AllNegs a, int rel_std) {
+  pdl_begin();
   int lane = threadIdx.x & 31;
   int e = blockIdx.x * GATHER_WARPS + (threadIdx.x >> 5);
   if (e >= a.B) return;
@@ -613,6 +618,7 @@ __device__ __forceinline__ float allnegs_candidate(float4 (&z)[VEC], const WaveD
 // torchbiggraph/util.py:415-428: `count` random (positive, (edge, candidate)) pairs per side, hits left in cnt[side]
 template <int VEC>
 __global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_slab_kernel(WaveDims d, WaveBufs w, AllNegs a, long long row0, int rel_std, int slab_ctas, int auc) {
+  pdl_begin();
   const int lane = threadIdx.x & 31, side = blockIdx.y, D = d.D;
   float4 z[VEC];
   if (blockIdx.x < slab_ctas) {
@@ -656,6 +662,7 @@ __global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_slab_kernel(WaveDim
 #define AN_TILE 64
 // grid (edge tiles, candidate tiles of the slab, sides); 256 threads, each a 4 x 4 block of the 64 x 64 score tile
 __global__ void __launch_bounds__(256) allnegs_score_kernel(WaveDims d, WaveBufs w, AllNegs a, long long row0) {
+  pdl_begin();
   __shared__ float sq[16][AN_TILE + 1], sy[16][AN_TILE + 1];
   __shared__ int scnt[16][AN_TILE];
   __shared__ float sa[16][AN_TILE], sb[16][AN_TILE];
@@ -754,6 +761,7 @@ __global__ void __launch_bounds__(256) allnegs_score_kernel(WaveDims d, WaveBufs
 // finish adds up the CTAs' sums in CTA order.
 // out8: loss, pos_rank, mrr, r1, r10, r50 sums over both sides' ranks, AUC hits per side.
 __global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_merge_kernel(WaveDims d, WaveBufs w, AllNegs a, long long row0, int first, int last, float wrel, double *out8) {
+  pdl_begin();
   __shared__ double sm[GATHER_WARPS][8];
   __shared__ bool closing;
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
@@ -872,18 +880,19 @@ int launch_allnegs_eval(const WaveDims &d, const WaveBufs &w, char *mem, int max
   int launches = 0;
   const int vec = (d.D + 127) / 128;
   const int ectas = (B + GATHER_WARPS - 1) / GATHER_WARPS;
-#define AN_V(K, ...) do { if (vec <= 1) K<1>__VA_ARGS__; else if (vec <= 2) K<2>__VA_ARGS__; else if (vec <= 4) K<4>__VA_ARGS__; else if (vec <= 8) K<8>__VA_ARGS__; else K<16>__VA_ARGS__; } while (0)
-  AN_V(allnegs_rows_kernel, <<<ectas, 32 * GATHER_WARPS, 0, st>>>(d, w, a, rel_std));
+#define AN_V(K, ...) do { if (vec <= 1) pbg_launch(K<1>, __VA_ARGS__); else if (vec <= 2) pbg_launch(K<2>, __VA_ARGS__); else if (vec <= 4) pbg_launch(K<4>, __VA_ARGS__); \
+                            else if (vec <= 8) pbg_launch(K<8>, __VA_ARGS__); else pbg_launch(K<16>, __VA_ARGS__); } while (0)
+  AN_V(allnegs_rows_kernel, ectas, 32 * GATHER_WARPS, 0, st, d, w, a, rel_std);
   ++launches;
   long long most = 0;
   for (int s = 0; s < 2; ++s) if (d.neg_enabled[s] && d.n_rows[s] > most) most = d.n_rows[s];
   for (long long row0 = 0; row0 == 0 || row0 < most; row0 += slab) {
     const int n = (int)(most - row0 < slab ? most - row0 : slab);
     const int sctas = (n + GATHER_WARPS - 1) / GATHER_WARPS, first = row0 == 0, last = row0 + slab >= most;
-    AN_V(allnegs_slab_kernel, <<<dim3(sctas + (first ? ectas : 0), 2), 32 * GATHER_WARPS, 0, st>>>(d, w, a, row0, rel_std, sctas, first));
+    AN_V(allnegs_slab_kernel, dim3(sctas + (first ? ectas : 0), 2), 32 * GATHER_WARPS, 0, st, d, w, a, row0, rel_std, sctas, first);
     if (planes) launch_allnegs_score_tc(d, w, a, row0, st);
-    else allnegs_score_kernel<<<dim3((B + AN_TILE - 1) / AN_TILE, (n + AN_TILE - 1) / AN_TILE, 2), 256, 0, st>>>(d, w, a, row0);
-    allnegs_merge_kernel<<<(2 * B + GATHER_WARPS - 1) / GATHER_WARPS, 32 * GATHER_WARPS, 0, st>>>(d, w, a, row0, first, last, wrel, out8);
+    else pbg_launch(allnegs_score_kernel, dim3((B + AN_TILE - 1) / AN_TILE, (n + AN_TILE - 1) / AN_TILE, 2), 256, 0, st, d, w, a, row0);
+    pbg_launch(allnegs_merge_kernel, (2 * B + GATHER_WARPS - 1) / GATHER_WARPS, 32 * GATHER_WARPS, 0, st, d, w, a, row0, first, last, wrel, out8);
     launches += 3;
   }
 #undef AN_V

@@ -32,6 +32,7 @@ struct GemmTasks { GemmTask t[2]; };
 
 template <int BM, bool A_KCONTIG, bool B_KCONTIG, bool SCORE>
 __global__ void __launch_bounds__(256) gemm_tile_kernel(GemmTasks tasks, WaveDims d, WaveBatches wb) {
+  pdl_begin();
   constexpr int TM = BM / 16;
   __shared__ __align__(16) float As[BK][BM + 4];
   __shared__ __align__(16) float Bs[BK][BN + 4];
@@ -159,10 +160,10 @@ static void launch_tiles(const GemmTasks &ts, const WaveDims &d, const WaveBatch
   int M = ts.t[0].M, N = ts.t[0].N;
   if (M <= 64) {
     dim3 g((N + BN - 1) / BN, (M + 63) / 64, d.nblk * 2);
-    gemm_tile_kernel<64, A_KCONTIG, B_KCONTIG, SCORE><<<g, 256, 0, st>>>(ts, d, wb);
+    pbg_launch(gemm_tile_kernel<64, A_KCONTIG, B_KCONTIG, SCORE>, g, 256, 0, st, ts, d, wb);
   } else {
     dim3 g((N + BN - 1) / BN, (M + 127) / 128, d.nblk * 2);
-    gemm_tile_kernel<128, A_KCONTIG, B_KCONTIG, SCORE><<<g, 256, 0, st>>>(ts, d, wb);
+    pbg_launch(gemm_tile_kernel<128, A_KCONTIG, B_KCONTIG, SCORE>, g, 256, 0, st, ts, d, wb);
   }
 }
 

@@ -115,6 +115,7 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base_s;
+  pdl_begin();                                               // barriers and tensor memory are set up beside the kernel before this one
   const int nkb = (g.K + KB - 1) / KB;
   const int b_atoms = PLANES ? (g.BN + 63) / 64 : (g.BN + 31) / 32;     // MN-major boxes per B tile (per plane)
   const uint32_t b_plane = B_MN ? (uint32_t)b_atoms * BOX_BYTES : (uint32_t)g.BN * ROW_BYTES;   // bytes of one B tile (plane)
@@ -520,7 +521,7 @@ static void launch_tc_inst(const TcMaps &maps, const TcGeom &g, const WaveDims &
   // if the opt-in fails the launch below fails too, and the caller's cudaGetLastError reports it
   pbg_opt_in_smem((const void *)tc_gemm_kernel<A_MN, B_MN, NTERMS, L2EPI>, (int)smem);
   // the plane tier has no split warps: producer, MMA issuer and the four epilogue warps
-  tc_gemm_kernel<A_MN, B_MN, NTERMS, L2EPI><<<grid, planes ? 192 : TC_THREADS, smem, st>>>(maps, gg, d, wb, errflag);
+  pbg_launch(tc_gemm_kernel<A_MN, B_MN, NTERMS, L2EPI>, grid, planes ? 192 : TC_THREADS, smem, st, maps, gg, d, wb, errflag);
   pbg_note_launch();
 }
 

@@ -40,6 +40,7 @@ __device__ __forceinline__ float coef_from_dscore(int cmp, float dS, float S) {
 // 31 us for 2 x 70 blocks of 100 rows x 200 columns where the bytes take 4.  NV == 0: rows of any length, column by column.
 template <int NV>
 __global__ void __launch_bounds__(32 * LOSS_WARPS) loss_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
+  pdl_begin();
   int lane = threadIdx.x & 31;
   long long item = (long long)blockIdx.x * LOSS_WARPS + (threadIdx.x >> 5);
   long long per_prob = (long long)d.nblk * d.Pm;
@@ -174,6 +175,7 @@ __global__ void __launch_bounds__(32 * LOSS_WARPS) loss_kernel(WaveDims d, WaveB
 // l2 family: column sums of T_p over the chunk's positives (coefficient of the negative row's
 // own |b|^2 term).  One thread per column.
 __global__ void colsum_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
+  pdl_begin();
   int p = blockIdx.z, blk = d.blk0 + blockIdx.y;
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= d.Mm) return;
@@ -197,6 +199,7 @@ __global__ void colsum_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
 // l2 family (coefficient of the row's own |y|^2 term).
 template <int NV>
 __global__ void __launch_bounds__(32 * LOSS_WARPS) coef_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
+  pdl_begin();
   int lane = threadIdx.x & 31;
   long long item = (long long)blockIdx.x * LOSS_WARPS + (threadIdx.x >> 5);
   long long per_side = (long long)d.nblk * d.Mm;
@@ -247,6 +250,7 @@ __global__ void __launch_bounds__(32 * LOSS_WARPS) coef_kernel(WaveDims d, WaveB
 // taken once (the general kernel makes three passes).  Same arithmetic, same summation order.
 template <int NV>
 __global__ void __launch_bounds__(32 * LOSS_WARPS) loss_softmax_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
+  pdl_begin();
   int lane = threadIdx.x & 31;
   long long item = (long long)blockIdx.x * LOSS_WARPS + (threadIdx.x >> 5);
   long long per_prob = (long long)d.nblk * d.Pm;
@@ -344,6 +348,7 @@ __global__ void __launch_bounds__(32 * LOSS_WARPS) loss_softmax_kernel(WaveDims 
 // whole lines without a shuffle or shared memory.
 template <bool PL>
 __global__ void __launch_bounds__(32 * LOSS_WARPS) coef_tile_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
+  pdl_begin();
   int lane = threadIdx.x & 31;
   long long item = (long long)blockIdx.x * LOSS_WARPS + (threadIdx.x >> 5);
   const int tiles = (d.Mm + 31) / 32;
@@ -423,30 +428,30 @@ int launch_loss(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cud
   long long items = 2ll * d.nblk * d.Pm;
   const int loss_ctas = (int)((items + LOSS_WARPS - 1) / LOSS_WARPS);
   const bool dotlike = d.cmp < PBG_CMP_L2;
-  if (dotlike && d.loss == PBG_LOSS_SOFTMAX && d.Ms <= 128) loss_softmax_kernel<4><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
-  else if (dotlike && d.loss == PBG_LOSS_SOFTMAX && d.Ms <= 256) loss_softmax_kernel<8><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
-  else if (dotlike && d.loss == PBG_LOSS_SOFTMAX && d.Ms <= 512) loss_softmax_kernel<16><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
-  else if (dotlike && d.loss == PBG_LOSS_SOFTMAX && d.Ms <= 1024) loss_softmax_kernel<32><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
-  else if (d.Ms <= 128) loss_kernel<4><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
-  else if (d.Ms <= 256) loss_kernel<8><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
-  else if (d.Ms <= 512) loss_kernel<16><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
-  else if (d.Ms <= 1024) loss_kernel<32><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
-  else loss_kernel<0><<<loss_ctas, 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
+  if (dotlike && d.loss == PBG_LOSS_SOFTMAX && d.Ms <= 128) pbg_launch(loss_softmax_kernel<4>, loss_ctas, 32 * LOSS_WARPS, 0, st, d, wb, w);
+  else if (dotlike && d.loss == PBG_LOSS_SOFTMAX && d.Ms <= 256) pbg_launch(loss_softmax_kernel<8>, loss_ctas, 32 * LOSS_WARPS, 0, st, d, wb, w);
+  else if (dotlike && d.loss == PBG_LOSS_SOFTMAX && d.Ms <= 512) pbg_launch(loss_softmax_kernel<16>, loss_ctas, 32 * LOSS_WARPS, 0, st, d, wb, w);
+  else if (dotlike && d.loss == PBG_LOSS_SOFTMAX && d.Ms <= 1024) pbg_launch(loss_softmax_kernel<32>, loss_ctas, 32 * LOSS_WARPS, 0, st, d, wb, w);
+  else if (d.Ms <= 128) pbg_launch(loss_kernel<4>, loss_ctas, 32 * LOSS_WARPS, 0, st, d, wb, w);
+  else if (d.Ms <= 256) pbg_launch(loss_kernel<8>, loss_ctas, 32 * LOSS_WARPS, 0, st, d, wb, w);
+  else if (d.Ms <= 512) pbg_launch(loss_kernel<16>, loss_ctas, 32 * LOSS_WARPS, 0, st, d, wb, w);
+  else if (d.Ms <= 1024) pbg_launch(loss_kernel<32>, loss_ctas, 32 * LOSS_WARPS, 0, st, d, wb, w);
+  else pbg_launch(loss_kernel<0>, loss_ctas, 32 * LOSS_WARPS, 0, st, d, wb, w);
   if (!d.dynamic) {
     if (dotlike) {
       const int tiles = (d.Mm + 31) / 32;
       long long warps = 2ll * d.nblk * tiles * tiles;
-      if (w.AB[0]) coef_tile_kernel<true><<<(int)((warps + LOSS_WARPS - 1) / LOSS_WARPS), 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
-      else coef_tile_kernel<false><<<(int)((warps + LOSS_WARPS - 1) / LOSS_WARPS), 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
+      if (w.AB[0]) pbg_launch(coef_tile_kernel<true>, (int)((warps + LOSS_WARPS - 1) / LOSS_WARPS), 32 * LOSS_WARPS, 0, st, d, wb, w);
+      else pbg_launch(coef_tile_kernel<false>, (int)((warps + LOSS_WARPS - 1) / LOSS_WARPS), 32 * LOSS_WARPS, 0, st, d, wb, w);
     } else {
       long long rows = 2ll * d.nblk * d.Mm;
-      coef_kernel<8><<<(int)((rows + LOSS_WARPS - 1) / LOSS_WARPS), 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
+      pbg_launch(coef_kernel<8>, (int)((rows + LOSS_WARPS - 1) / LOSS_WARPS), 32 * LOSS_WARPS, 0, st, d, wb, w);
     }
     return 2;
   }
   if (d.cmp >= PBG_CMP_L2) {
     dim3 g((d.Mm + 127) / 128, d.nblk, 2);
-    colsum_kernel<<<g, 128, 0, st>>>(d, wb, w);
+    pbg_launch(colsum_kernel, g, 128, 0, st, d, wb, w);
     return 2;
   }
   return 1;
@@ -459,6 +464,7 @@ int launch_loss(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cud
 // (sum(params^3) * len(src_pos) where src_pos is the [chunks, P, D] view, regularizers.py:88-92),
 // which row 0 of the block carries.  Runs after the gather, on the snapshot the wave reads.
 __global__ void __launch_bounds__(32 * LOSS_WARPS) reg_value_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
+  pdl_begin();
   int lane = threadIdx.x & 31;
   long long item = (long long)blockIdx.x * LOSS_WARPS + (threadIdx.x >> 5);
   if (item >= (long long)d.nblk * d.Pm) return;
@@ -499,7 +505,7 @@ __global__ void __launch_bounds__(32 * LOSS_WARPS) reg_value_kernel(WaveDims d, 
 
 int launch_reg_value(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st) {
   long long items = (long long)d.nblk * d.Pm;
-  reg_value_kernel<<<(int)((items + LOSS_WARPS - 1) / LOSS_WARPS), 32 * LOSS_WARPS, 0, st>>>(d, wb, w);
+  pbg_launch(reg_value_kernel, (int)((items + LOSS_WARPS - 1) / LOSS_WARPS), 32 * LOSS_WARPS, 0, st, d, wb, w);
   return 1;
 }
 
@@ -507,6 +513,7 @@ int launch_reg_value(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w
 // [count, Pl + U] negatives per side with ignored entries set to -1e9; single batch (wave of 1).
 __global__ void export_scores_kernel(WaveDims d, WaveBatches wb, WaveBufs w, float *lhs_pos, float *rhs_pos,
                                      float *lhs_neg, float *rhs_neg) {
+  pdl_begin();
   int e = blockIdx.x;                       // edge of the batch
   int p = blockIdx.y;
   BlockInfo b0 = block_info(d, wb, 0);
@@ -531,7 +538,7 @@ int launch_export_scores(const WaveDims &d, const WaveBatches &wb, const WaveBuf
                          float *rhs_pos, float *lhs_neg, float *rhs_neg, cudaStream_t st) {
   if (wb.n[0] <= 0) return 0;
   dim3 g(wb.n[0], 2);
-  export_scores_kernel<<<g, 128, 0, st>>>(d, wb, w, lhs_pos, rhs_pos, lhs_neg, rhs_neg);
+  pbg_launch(export_scores_kernel, g, 128, 0, st, d, wb, w, lhs_pos, rhs_pos, lhs_neg, rhs_neg);
   return 1;
 }
 
@@ -542,6 +549,7 @@ int launch_export_scores(const WaveDims &d, const WaveBatches &wb, const WaveBuf
 // The score matrix is read once and not written.  (Rank, AUC, loss and sum as kernels of their own, the loss with the
 // coefficient matrix it writes for training, took 107 us on 5000 edges against 1000 negatives a side.)
 __global__ void __launch_bounds__(32 * LOSS_WARPS) eval_rows_kernel(WaveDims d, WaveBatches wb, WaveBufs w, double *part, unsigned *done, double *out8) {
+  pdl_begin();
   __shared__ double sm[LOSS_WARPS][8];
   __shared__ bool closing;
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
@@ -638,6 +646,6 @@ __global__ void __launch_bounds__(32 * LOSS_WARPS) eval_rows_kernel(WaveDims d, 
 }
 
 int launch_eval(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, double *part, unsigned *done, double *out8, cudaStream_t st) {
-  eval_rows_kernel<<<pbg_eval_ctas(d.nblk, d.Pm), 32 * LOSS_WARPS, 0, st>>>(d, wb, w, part, done, out8);
+  pbg_launch(eval_rows_kernel, pbg_eval_ctas(d.nblk, d.Pm), 32 * LOSS_WARPS, 0, st, d, wb, w, part, done, out8);
   return 1;
 }

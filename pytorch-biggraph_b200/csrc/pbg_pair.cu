@@ -81,6 +81,7 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base_s;
+  pdl_begin();                                               // barriers and tensor memory are set up beside the kernel before this one
   const int STAGES = g.nst;
   const uint32_t plane_bytes = (uint32_t)g.rows_pad * 64u;               // one plane of one operand array: rows of 32 bf16
   const uint32_t arr_bytes = (uint32_t)NPL * plane_bytes;
@@ -391,10 +392,10 @@ int launch_pair_score(const WaveDims &d, const WaveBatches &wb, const WaveBufs &
   // the opt-in covers the largest stage ring this kernel is ever launched with (227 KB less its static shared memory)
   if (pl->npl == 3) {
     pbg_opt_in_smem((const void *)pair_score_kernel<3>, PAIR_SMEM_MAX);
-    pair_score_kernel<3><<<grid, PAIR_THREADS, smem, st>>>(pl->maps, pl->geom, d, wb, w);
+    pbg_launch(pair_score_kernel<3>, grid, PAIR_THREADS, smem, st, pl->maps, pl->geom, d, wb, w);
   } else {
     pbg_opt_in_smem((const void *)pair_score_kernel<2>, PAIR_SMEM_MAX);
-    pair_score_kernel<2><<<grid, PAIR_THREADS, smem, st>>>(pl->maps, pl->geom, d, wb, w);
+    pbg_launch(pair_score_kernel<2>, grid, PAIR_THREADS, smem, st, pl->maps, pl->geom, d, wb, w);
   }
   pbg_note_launch();
   return 1;

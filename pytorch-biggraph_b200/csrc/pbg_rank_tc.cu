@@ -51,6 +51,7 @@ allnegs_tc_kernel(const __grid_constant__ RankMaps maps, WaveDims d, WaveBufs w,
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base_s;
+  pdl_begin();                                               // barriers and tensor memory are set up beside the kernel before this one
   const int nkb = (d.D + 31) / 32;
   const int tiles_m = (a.B + 127) / 128, tiles_n = a.slab / RK_BN;
   const int ntiles = 2 * tiles_m * tiles_n;
@@ -194,7 +195,7 @@ int launch_allnegs_score_tc(const WaveDims &d, const WaveBufs &w, const AllNegs 
   const size_t smem = RK_STAGES * RK_STAGE + 1024;
   pbg_opt_in_smem((const void *)allnegs_tc_kernel, (int)smem);
   const int tiles = 2 * ((a.B + 127) / 128) * (a.slab / RK_BN), sms = pbg_sm_count();
-  allnegs_tc_kernel<<<tiles < sms ? tiles : sms, RK_THREADS, smem, st>>>(maps, d, w, a, row0);
+  pbg_launch(allnegs_tc_kernel, tiles < sms ? tiles : sms, RK_THREADS, smem, st, maps, d, w, a, row0);
   pbg_note_launch();
   return 1;
 }

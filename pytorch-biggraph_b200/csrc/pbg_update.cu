@@ -113,6 +113,7 @@ __device__ __forceinline__ void operator_back(float4 (&v)[VEC], float4 (&pg)[VEC
 // summed per chunk block ran 20 CTAs on a single batch.)
 template <int VEC, int CK>
 __global__ void __launch_bounds__(32 * UPD_WARPS) std_pullback_kernel(WaveDims d, WaveBatches wb, WaveBufs w, int side0) {
+  pdl_begin();
   extern __shared__ __align__(16) float wpart[];             // [UPD_WARPS][VEC * 128]
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int side = side0 + blockIdx.y, a = side ? ARR_N1 : ARR_N0;
@@ -386,6 +387,7 @@ __global__ void __launch_bounds__(32 * TileWarps<VEC, RULE>::N, RULE == RULE_EMB
 tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys,
                    const unsigned int *__restrict__ vals, float lr, float *__restrict__ psum,
                    long long *__restrict__ hublist, int *__restrict__ hubcnt, ParamJob job, int aside) {
+  pdl_begin();
   constexpr int WARPS = TileWarps<VEC, RULE>::N, STAGE = StageRows<VEC, RULE>::N;
   extern __shared__ __align__(128) float stage_all[];        // [WARPS][STAGE][Dp]
   __shared__ __align__(8) unsigned long long sbar[WARPS];
@@ -628,6 +630,7 @@ __global__ void __launch_bounds__(32 * UPD_WARPS)
 hub_reduce_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys, const unsigned int *__restrict__ vals,
                   float *__restrict__ psum, const long long *__restrict__ hublist, const int *__restrict__ hubcnt,
                   int *__restrict__ hubcnt_next, long long *__restrict__ bigtab, int aside, ParamJob job, pbg_batch_stats *per_batch, double *sum) {
+  pdl_begin();
   extern __shared__ __align__(16) float part[];              // [UPD_WARPS][VEC * 128]
   if (blockIdx.x == 0 && threadIdx.x < 2) hubcnt_next[threadIdx.x] = 0;      // its last reader is behind us in the stream
   // the first CTAs of the embedding rows' launch (aside) have other work
@@ -708,6 +711,7 @@ hub_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long lo
                   const unsigned int *__restrict__ vals, float lr, const float *__restrict__ psum,
                   const long long *__restrict__ hublist, const int *__restrict__ hubcnt,
                   const long long *__restrict__ bigtab) {
+  pdl_begin();
   static_assert(32 * UPD_WARPS == HUB_BIG, "one probe per thread covers exactly the rows that are not big");
   extern __shared__ __align__(16) float tot[];               // [k][VEC * 128]
   __shared__ long long bstart[PBG_KMAX + 1];
@@ -863,6 +867,7 @@ hub_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long lo
 // contractions of launch_matrix_backward read the result.
 template <int VEC, int CK>
 __global__ void __launch_bounds__(32 * UPD_WARPS) gz_rows_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
+  pdl_begin();
   int lane = threadIdx.x & 31;
   long long item = (long long)blockIdx.x * UPD_WARPS + (threadIdx.x >> 5);
   if (item >= (long long)d.nblk * d.Mm) return;
@@ -892,16 +897,16 @@ static inline int comparator_kind(const WaveDims &d) { return d.cmp >= PBG_CMP_L
 #define PBG_ROWS_CK(VEC, KERNEL, ...)                                        \
   do {                                                                       \
     const int ck_ = comparator_kind(d);                                      \
-    if (ck_ == CK_DOT) KERNEL<VEC, CK_DOT> __VA_ARGS__;                      \
-    else if (ck_ == CK_COS) KERNEL<VEC, CK_COS> __VA_ARGS__;                 \
-    else KERNEL<VEC, CK_L2> __VA_ARGS__;                                     \
+    if (ck_ == CK_DOT) pbg_launch(KERNEL<VEC, CK_DOT>, __VA_ARGS__);         \
+    else if (ck_ == CK_COS) pbg_launch(KERNEL<VEC, CK_COS>, __VA_ARGS__);    \
+    else pbg_launch(KERNEL<VEC, CK_L2>, __VA_ARGS__);                        \
   } while (0)
 
 int launch_gz_rows(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st) {
   long long items = (long long)d.nblk * d.Mm;
   int ctas = (int)((items + UPD_WARPS - 1) / UPD_WARPS);
   int vec = (d.D + 127) / 128;
-#define GZ(V) PBG_ROWS_CK(V, gz_rows_kernel, <<<ctas, 32 * UPD_WARPS, 0, st>>>(d, wb, w))
+#define GZ(V) PBG_ROWS_CK(V, gz_rows_kernel, ctas, 32 * UPD_WARPS, 0, st, d, wb, w)
   if (vec <= 1) GZ(1); else if (vec <= 2) GZ(2); else if (vec <= 4) GZ(4); else if (vec <= 8) GZ(8); else GZ(16);
 #undef GZ
   return 1;
@@ -911,6 +916,7 @@ int launch_gz_rows(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, 
 // (async_adagrad.py:75-85).  dA[b] comes from launch_matrix_backward; the gradient of an affine
 // translation is the column sum of the batch's GN1 rows.
 __global__ void relupdate_matrix_kernel(WaveDims d, WaveBatches wb, WaveBufs w, float lr) {
+  pdl_begin();
   long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= d.opw) return;
   const long long DD = (long long)d.D * d.D;
@@ -934,7 +940,7 @@ __global__ void relupdate_matrix_kernel(WaveDims d, WaveBatches wb, WaveBufs w, 
 }
 
 int launch_matrix_update(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, float lr, cudaStream_t st) {
-  relupdate_matrix_kernel<<<(d.opw + 255) / 256, 256, 0, st>>>(d, wb, w, lr);
+  pbg_launch(relupdate_matrix_kernel, (d.opw + 255) / 256, 256, 0, st, d, wb, w, lr);
   return 1;
 }
 
@@ -945,6 +951,7 @@ int launch_matrix_update(const WaveDims &d, const WaveBatches &wb, const WaveBuf
 // they are half of the slots).
 template <int VEC, int CK>
 __global__ void __launch_bounds__(32 * UPD_WARPS, VEC <= 4 ? 4 : 1) dyn_pullback_kernel(WaveDims d, WaveBatches wb, WaveBufs w, int first_q) {
+  pdl_begin();
   extern __shared__ __align__(16) float wpart[];             // [UPD_WARPS][VEC * 128]
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const long long nN = (long long)d.nblk * d.Mm, nQ = (long long)d.nblk * d.Pm;
@@ -1023,7 +1030,7 @@ static int launch_pullback(const WaveDims &d, const WaveBatches &wb, const WaveB
     if (!rows_change && !has_op) return 0;
     const int first_q = rows_change ? 0 : 1;
     const long long rows = 2ll * d.nblk * d.Pm + (first_q ? 0 : 2ll * d.nblk * d.Mm);
-    PBG_ROWS_CK(VEC, dyn_pullback_kernel, <<<(unsigned)((rows + UPD_WARPS - 1) / UPD_WARPS), 32 * UPD_WARPS, smem, st>>>(d, wb, w, first_q));
+    PBG_ROWS_CK(VEC, dyn_pullback_kernel, (unsigned)((rows + UPD_WARPS - 1) / UPD_WARPS), 32 * UPD_WARPS, smem, st, d, wb, w, first_q);
     return 1;
   }
   const bool row_op = has_op && !d.matrix_op;
@@ -1036,7 +1043,7 @@ static int launch_pullback(const WaveDims &d, const WaveBatches &wb, const WaveB
   if (!rows_change && !(row_op && w.PG)) return 0;
   job.cleared0 = rows_change; job.cleared1 = 1;
   const dim3 grid((unsigned)(((long long)d.nblk * d.Mm + UPD_WARPS - 1) / UPD_WARPS), rows_change ? 2 : 1);
-  PBG_ROWS_CK(VEC, std_pullback_kernel, <<<grid, 32 * UPD_WARPS, smem, st>>>(d, wb, w, rows_change ? 0 : 1));
+  PBG_ROWS_CK(VEC, std_pullback_kernel, grid, 32 * UPD_WARPS, smem, st, d, wb, w, rows_change ? 0 : 1);
   return 1;
 }
 
@@ -1065,11 +1072,9 @@ static int launch_update_vec(const WaveDims &d, const WaveBatches &wb, const Wav
   const int sum_ctas = param_sum_ctas(d, job);
   size_t tile_smem = (size_t)EMB_WARPS * StageRows<VEC, RULE_EMB>::N * d.Dp * 4;
   if (sum_ctas && tile_smem < 8 * 128 * 4) tile_smem = 8 * 128 * 4;
-  tile_update_kernel<VEC, RULE_EMB><<<sum_ctas + (unsigned)((tiles + EMB_WARPS - 1) / EMB_WARPS), 32 * EMB_WARPS, tile_smem, st>>>(
-      d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, job, sum_ctas);
-  hub_reduce_kernel<VEC><<<d.k + param_step_ctas(d, job) + 2 * hub_ctas, 32 * UPD_WARPS, red_smem, st>>>(
-      d, wb, w, keys, vals, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 1, job, us.per_batch, us.sum);
-  hub_update_kernel<VEC, RULE_EMB><<<hub_ctas, 32 * UPD_WARPS, hub_smem, st>>>(d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, us.bigtab);
+  pbg_launch(tile_update_kernel<VEC, RULE_EMB>, sum_ctas + (unsigned)((tiles + EMB_WARPS - 1) / EMB_WARPS), 32 * EMB_WARPS, tile_smem, st, d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, job, sum_ctas);
+  pbg_launch(hub_reduce_kernel<VEC>, d.k + param_step_ctas(d, job) + 2 * hub_ctas, 32 * UPD_WARPS, red_smem, st, d, wb, w, keys, vals, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 1, job, us.per_batch, us.sum);
+  pbg_launch(hub_update_kernel<VEC, RULE_EMB>, hub_ctas, 32 * UPD_WARPS, hub_smem, st, d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, us.bigtab);
   launches += 3;
   if (d.op != PBG_OP_NONE && w.theta[0] != nullptr) {
     if (d.dynamic) {
@@ -1077,11 +1082,9 @@ static int launch_update_vec(const WaveDims &d, const WaveBatches &wb, const Wav
       pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_REL>, REL_WARPS * TILE * VEC * 512);
       int *t = hubcnt; hubcnt = hubcnt_next; hubcnt_next = t;
       ++*us.turn;
-      tile_update_kernel<VEC, RULE_REL><<<(unsigned)((tiles + REL_WARPS - 1) / REL_WARPS), 32 * REL_WARPS, (size_t)REL_WARPS * TILE * d.Dp * 4, st>>>(
-          d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt, job, 0);
-      hub_reduce_kernel<VEC><<<2 * hub_ctas, 32 * UPD_WARPS, red_smem, st>>>(
-          d, wb, w, keys, vals, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 0, job, nullptr, nullptr);
-      hub_update_kernel<VEC, RULE_REL><<<hub_ctas, 32 * UPD_WARPS, hub_smem, st>>>(d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt, us.bigtab);
+      pbg_launch(tile_update_kernel<VEC, RULE_REL>, (unsigned)((tiles + REL_WARPS - 1) / REL_WARPS), 32 * REL_WARPS, (size_t)REL_WARPS * TILE * d.Dp * 4, st, d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt, job, 0);
+      pbg_launch(hub_reduce_kernel<VEC>, 2 * hub_ctas, 32 * UPD_WARPS, red_smem, st, d, wb, w, keys, vals, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 0, job, nullptr, nullptr);
+      pbg_launch(hub_update_kernel<VEC, RULE_REL>, hub_ctas, 32 * UPD_WARPS, hub_smem, st, d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt, us.bigtab);
       launches += 3;
     } else if (d.matrix_op) {
       launches += launch_matrix_update(d, wb, w, rel_lr, st);
@@ -1108,6 +1111,7 @@ __global__ void __launch_bounds__(32 * UPD_WARPS)
 row_adagrad_sorted_kernel(float *emb, float *state, int D, const unsigned long long *__restrict__ keys,
                           const unsigned int *__restrict__ vals, const float *__restrict__ grads, int n,
                           float lr, unsigned long long key_invalid) {
+  pdl_begin();
   int lane = threadIdx.x & 31;
   long long pos = (long long)blockIdx.x * UPD_WARPS + (threadIdx.x >> 5);
   if (pos >= n) return;
@@ -1145,7 +1149,7 @@ int launch_row_adagrad_sorted(float *emb, float *state, int dim, const unsigned 
                               unsigned long long key_invalid, cudaStream_t st) {
   int ctas = (n + UPD_WARPS - 1) / UPD_WARPS;
   int vec = (dim + 127) / 128;
-#define RA(V) row_adagrad_sorted_kernel<V><<<ctas, 32 * UPD_WARPS, 0, st>>>(emb, state, dim, keys, vals, grads, n, lr, key_invalid)
+#define RA(V) pbg_launch(row_adagrad_sorted_kernel<V>, ctas, 32 * UPD_WARPS, 0, st, emb, state, dim, keys, vals, grads, n, lr, key_invalid)
   if (vec <= 1) RA(1); else if (vec <= 2) RA(2); else if (vec <= 4) RA(4); else if (vec <= 8) RA(8); else RA(16);
 #undef RA
   return 1;
