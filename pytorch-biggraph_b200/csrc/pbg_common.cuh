@@ -265,7 +265,10 @@ __device__ __forceinline__ float4 operator+(float4 a, float4 b) { return make_fl
 __device__ __forceinline__ float4 operator-(float4 a, float4 b) { return make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w); }
 __device__ __forceinline__ float4 operator*(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
 __device__ __forceinline__ float4 operator*(float4 a, float s) { return make_float4(a.x * s, a.y * s, a.z * s, a.w * s); }
-__device__ __forceinline__ float f4dot(float4 a, float4 b) { return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
+// (Rounding orders spelled out: which products the compiler contracts would otherwise depend on the code around the call.
+// Two are in use, so that sums stay bit for bit what they were when their kernels were written.)
+__device__ __forceinline__ float f4dot(float4 a, float4 b) { return __fmaf_rn(a.w, b.w, __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x)))); }
+__device__ __forceinline__ float f4dot_yx(float4 a, float4 b) { return __fmaf_rn(a.w, b.w, __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)))); }
 __device__ __forceinline__ float f4sum(float4 a) { return a.x + a.y + a.z + a.w; }
 // tf32(x): round to nearest, 10 mantissa bits kept -- the part of x a kind::tf32 MMA sees exactly
 __device__ __forceinline__ float tf32_hi(float x) {
@@ -428,8 +431,8 @@ struct UpdateScratch {
 };
 int launch_update(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, const unsigned long long *keys, const unsigned int *vals,
                   float lr, float rel_lr, const UpdateScratch &us, cudaStream_t st);
-// bigtab: (nocc / 256 + 2) rows of PBG_KMAX + 1 entries: where the batches of a row with 256 and more slots start, and its end
-inline size_t pbg_bigtab_bytes(long long nocc) { return (size_t)(nocc / 256 + 2) * (PBG_KMAX + 1) * sizeof(long long); }
+// bigtab: a line for each row with 256 and more slots: where its batches start, its end, a counter (zero between waves)
+inline size_t pbg_bigtab_bytes(long long nocc) { return (size_t)(nocc / 256 + 2) * (PBG_KMAX + 2) * sizeof(long long); }
 // Evaluation of one batch after its scores.  out8 (host or device memory): loss, then pos_rank, mrr, r1, r10, r50 summed over
 // both sides, then the AUC hits per side.  part: 8 doubles for each of the kernel's CTAs; done: a counter, zero at first.
 inline int pbg_eval_ctas(int nblk, int Pm) { return (int)((2ll * nblk * Pm + 7) / 8); }

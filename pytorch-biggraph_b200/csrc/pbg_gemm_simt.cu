@@ -57,58 +57,73 @@ __global__ void __launch_bounds__(256) gemm_tile_kernel(GemmTasks tasks, WaveDim
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
 
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    // ---- stage A ----
-    if (A_KCONTIG) {   // A[m][k], k contiguous: BM rows x 16 k = BM*4 float4
+  // The next k-block's values are requested into registers before this one's are multiplied (a block is 16 k-values: without
+  // it every block began with a wait for global memory, most of a 100-wide product's time).
+  constexpr int NA = (BM * 4) / 256;
+  float4 ra[NA], rb;
+  auto fetch = [&](int k0) {
 #pragma unroll
-      for (int it = 0; it < (BM * 4) / 256; ++it) {
-        int idx = tid + it * 256, row = idx >> 2, kq = (idx & 3) * 4;
-        float4 v = f4zero();
+    for (int it = 0; it < NA; ++it) {
+      const int idx = tid + it * 256;
+      float4 v = f4zero();
+      if (A_KCONTIG) {   // A[m][k], k contiguous: BM rows x 16 k = BM*4 float4
+        const int row = idx >> 2, kq = (idx & 3) * 4;
         if (m0 + row < M && k0 + kq < K) {
           v = ld4(A + (size_t)(m0 + row) * t.lda + k0 + kq);
           if (k0 + kq + 1 >= K) v.y = 0.f;
           if (k0 + kq + 2 >= K) v.z = 0.f;
           if (k0 + kq + 3 >= K) v.w = 0.f;
         }
-        As[kq + 0][row] = v.x; As[kq + 1][row] = v.y; As[kq + 2][row] = v.z; As[kq + 3][row] = v.w;
-      }
-    } else {           // A[k][m], m contiguous: 16 k rows x BM = BM*4 float4
-#pragma unroll
-      for (int it = 0; it < (BM * 4) / 256; ++it) {
-        int idx = tid + it * 256, kr = idx / (BM / 4), c4 = (idx % (BM / 4)) * 4;
-        float4 v = f4zero();
+      } else {           // A[k][m], m contiguous: 16 k rows x BM = BM*4 float4
+        const int kr = idx / (BM / 4), c4 = (idx % (BM / 4)) * 4;
         if (k0 + kr < K && m0 + c4 < M) {
           v = ld4(A + (size_t)(k0 + kr) * t.lda + m0 + c4);
           if (m0 + c4 + 1 >= M) v.y = 0.f;
           if (m0 + c4 + 2 >= M) v.z = 0.f;
           if (m0 + c4 + 3 >= M) v.w = 0.f;
         }
-        st4(&As[kr][c4], v);
+      }
+      ra[it] = v;
+    }
+    rb = f4zero();
+    if (B_KCONTIG) {   // B[n][k]
+      const int row = tid >> 2, kq = (tid & 3) * 4;
+      if (n0 + row < N && k0 + kq < K) {
+        rb = ld4(B + (size_t)(n0 + row) * t.ldb + k0 + kq);
+        if (k0 + kq + 1 >= K) rb.y = 0.f;
+        if (k0 + kq + 2 >= K) rb.z = 0.f;
+        if (k0 + kq + 3 >= K) rb.w = 0.f;
+      }
+    } else {           // B[k][n]
+      const int kr = tid >> 4, c4 = (tid & 15) * 4;
+      if (k0 + kr < K && n0 + c4 < N) {
+        rb = ld4(B + (size_t)(k0 + kr) * t.ldb + n0 + c4);
+        if (n0 + c4 + 1 >= N) rb.y = 0.f;
+        if (n0 + c4 + 2 >= N) rb.z = 0.f;
+        if (n0 + c4 + 3 >= N) rb.w = 0.f;
       }
     }
-    // ---- stage B ----
-    if (B_KCONTIG) {   // B[n][k]
-      int row = tid >> 2, kq = (tid & 3) * 4;
-      float4 v = f4zero();
-      if (n0 + row < N && k0 + kq < K) {
-        v = ld4(B + (size_t)(n0 + row) * t.ldb + k0 + kq);
-        if (k0 + kq + 1 >= K) v.y = 0.f;
-        if (k0 + kq + 2 >= K) v.z = 0.f;
-        if (k0 + kq + 3 >= K) v.w = 0.f;
+  };
+  fetch(0);
+  for (int k0 = 0; k0 < K; k0 += BK) {
+#pragma unroll
+    for (int it = 0; it < NA; ++it) {
+      const int idx = tid + it * 256;
+      if (A_KCONTIG) {
+        const int row = idx >> 2, kq = (idx & 3) * 4;
+        As[kq + 0][row] = ra[it].x; As[kq + 1][row] = ra[it].y; As[kq + 2][row] = ra[it].z; As[kq + 3][row] = ra[it].w;
+      } else {
+        st4(&As[idx / (BM / 4)][(idx % (BM / 4)) * 4], ra[it]);
       }
-      Bs[kq + 0][row] = v.x; Bs[kq + 1][row] = v.y; Bs[kq + 2][row] = v.z; Bs[kq + 3][row] = v.w;
-    } else {           // B[k][n]
-      int kr = tid >> 4, c4 = (tid & 15) * 4;
-      float4 v = f4zero();
-      if (k0 + kr < K && n0 + c4 < N) {
-        v = ld4(B + (size_t)(k0 + kr) * t.ldb + n0 + c4);
-        if (n0 + c4 + 1 >= N) v.y = 0.f;
-        if (n0 + c4 + 2 >= N) v.z = 0.f;
-        if (n0 + c4 + 3 >= N) v.w = 0.f;
-      }
-      st4(&Bs[kr][c4], v);
+    }
+    if (B_KCONTIG) {
+      const int row = tid >> 2, kq = (tid & 3) * 4;
+      Bs[kq + 0][row] = rb.x; Bs[kq + 1][row] = rb.y; Bs[kq + 2][row] = rb.z; Bs[kq + 3][row] = rb.w;
+    } else {
+      st4(&Bs[tid >> 4][(tid & 15) * 4], rb);
     }
     __syncthreads();
+    if (k0 + BK < K) fetch(k0 + BK);
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
       float a[TM];

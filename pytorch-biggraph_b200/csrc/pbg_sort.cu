@@ -226,9 +226,11 @@ __device__ __forceinline__ void cluster_sort_body(uint2 (&item)[IPT], int n, int
     }
     __syncthreads();
     if (t < bins) {
-      unsigned int run = 0u;
-#pragma unroll 8
-      for (int w = 0; w < CS_WARPS; ++w) { const unsigned int c = cnt[w * bins + t]; cnt[w * bins + t] = run; run += c; }
+      unsigned int run = 0u, c[CS_WARPS];
+#pragma unroll
+      for (int w = 0; w < CS_WARPS; ++w) c[w] = cnt[w * bins + t];
+#pragma unroll
+      for (int w = 0; w < CS_WARPS; ++w) { cnt[w * bins + t] = run; run += c[w]; }
       for (int c = 0; c < nct; ++c) cluster.map_shared_rank(all, c)[rank * CS_BINS + t] = run;
     }
     cluster.sync();                                                     // totals are everywhere; every pair is in registers
@@ -309,13 +311,24 @@ __global__ void __launch_bounds__(CS_THREADS, 1) sort_rows_kernel(SortRows a, in
   cluster_sort_body<IPT>(item, a.n, bits, a.keys, a.vals, cs_smem);
 }
 
-// CTAs and pairs per thread for a list of n: four pairs per thread as long as the cluster can grow (a pass costs about
-// the same with one CTA as with sixteen, and more pairs per thread lengthen it), then 8 and 16 on sixteen CTAs.
+// CTAs and pairs per thread for a list of n: one pair per thread as long as the cluster can grow, then up to sixteen on
+// sixteen CTAs.  A barrier of a large cluster costs less than building and ranking more pairs per thread: a list of
+// 4,000 slots took 21 us on one CTA with four pairs per thread.
 static void cluster_shape(int n, int &ctas, int &ipt) {
-  ipt = 4;
-  for (ctas = 1; ctas < 16 && ctas * CS_THREADS * 4 < n; ctas *= 2) {}
+  ipt = 1;
+  for (ctas = 1; ctas < 16 && ctas * CS_THREADS < n; ctas *= 2) {}
   while (ctas * CS_THREADS * ipt < n) ipt *= 2;
 }
+
+// KERNEL<pairs per thread>(args) on `lists` clusters
+#define CS_LAUNCH(KERNEL, LISTS, ...)                                                                       \
+  do {                                                                                                      \
+    if (ipt == 1) launch_cluster(KERNEL<1>, LISTS, ctas, cluster_sort_smem<1>(), st, __VA_ARGS__);          \
+    else if (ipt == 2) launch_cluster(KERNEL<2>, LISTS, ctas, cluster_sort_smem<2>(), st, __VA_ARGS__);     \
+    else if (ipt == 4) launch_cluster(KERNEL<4>, LISTS, ctas, cluster_sort_smem<4>(), st, __VA_ARGS__);     \
+    else if (ipt == 8) launch_cluster(KERNEL<8>, LISTS, ctas, cluster_sort_smem<8>(), st, __VA_ARGS__);     \
+    else launch_cluster(KERNEL<16>, LISTS, ctas, cluster_sort_smem<16>(), st, __VA_ARGS__);                 \
+  } while (0)
 
 template <class... Args>
 static void launch_cluster(void (*kernel)(Args...), int lists, int ctas, size_t smem, cudaStream_t st, Args... args) {
@@ -334,9 +347,7 @@ int launch_sort_waves(const WaveDims &d, const WaveBufs &w, const SortWaves &wav
   int most = 0, ctas, ipt;
   for (int i = 0; i < waves.count; ++i) if (waves.w[i].k > most) most = waves.w[i].k;
   cluster_shape(most * d.spb, ctas, ipt);
-  if (ipt == 4) launch_cluster(sort_waves_kernel<4>, waves.count, ctas, cluster_sort_smem<4>(), st, d, w, waves, bits);
-  else if (ipt == 8) launch_cluster(sort_waves_kernel<8>, waves.count, ctas, cluster_sort_smem<8>(), st, d, w, waves, bits);
-  else launch_cluster(sort_waves_kernel<16>, waves.count, ctas, cluster_sort_smem<16>(), st, d, w, waves, bits);
+  CS_LAUNCH(sort_waves_kernel, waves.count, d, w, waves, bits);
   return 1;
 }
 
@@ -345,8 +356,6 @@ int launch_sort_rows(const long long *rows, long long num_rows, int n, int bits,
   SortRows a{rows, num_rows, n, keys, vals, errflag};
   int ctas, ipt;
   cluster_shape(n, ctas, ipt);
-  if (ipt == 4) launch_cluster(sort_rows_kernel<4>, 1, ctas, cluster_sort_smem<4>(), st, a, bits);
-  else if (ipt == 8) launch_cluster(sort_rows_kernel<8>, 1, ctas, cluster_sort_smem<8>(), st, a, bits);
-  else launch_cluster(sort_rows_kernel<16>, 1, ctas, cluster_sort_smem<16>(), st, a, bits);
+  CS_LAUNCH(sort_rows_kernel, 1, a, bits);
   return 1;
 }

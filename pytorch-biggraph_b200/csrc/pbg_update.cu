@@ -47,8 +47,7 @@ __device__ __forceinline__ void gz_row(float4 (&v)[VEC], const WaveDims &d, cons
   if (CK == CK_COS) {
     float s = 0.f;
 #pragma unroll
-    for (int c = 0; c < VEC; ++c)     // rounding order spelled out: it must not depend on what the compiler contracts around it
-      s += __fmaf_rn(v[c].w, yv[c].w, __fmaf_rn(v[c].z, yv[c].z, __fmaf_rn(v[c].x, yv[c].x, __fmul_rn(v[c].y, yv[c].y))));
+    for (int c = 0; c < VEC; ++c) s += f4dot_yx(v[c], yv[c]);
     s = warp_sum(s);
 #pragma unroll
     for (int c = 0; c < VEC; ++c) v[c] = (v[c] - yv[c] * s) * inv;
@@ -263,13 +262,14 @@ __device__ __forceinline__ void param_step(const WaveDims &d, const WaveBatches 
 //     slot: row and state in registers, one optimizer step per batch that touched it;
 //   * a longer row (a hub of the graph) is summed tile by tile: every warp writes, for each
 //     (batch, tile) run of its slots, one partial gradient row to psum[first slot of the run]; the
-//     warp that holds the head registers the row in hublist, and hub_update_kernel finishes it
+//     warp that holds the head registers the row in hublist, and hub_kernel finishes it
 //     with one CTA per row (eight warps add the partial rows of a batch in a fixed order).
 // RULE selects the table and its optimizer: embedding rows / RowAdagrad, or (dynamic relations)
 // operator rows / AsyncAdagrad.
 // ------------------------------------------------------------------------------------------------
 #define TILE 4
 #define SHORT_MAX 24
+#define BIGTAB_LINE (PBG_KMAX + 2)
 #define HUB_BIG 256     // rows with at least this many slots in a wave get their batches summed by separate CTAs
 // hublist holds nocc / 8 + 64 entries; a hub row has more than SHORT_MAX slots, so the rows themselves need fewer than
 // nocc / 16 + 32 of them and the list of big rows (at most nocc / HUB_BIG) lives in the rest.  hubcnt[0] counts hub
@@ -581,7 +581,7 @@ __device__ __forceinline__ long long warp_prefix_end(long long lo, long long hi,
 
 // Per-batch Stats (train_cpu.py:95-101) of batch b of the wave, summed by one CTA in a fixed order; the running totals
 // live in `sum` (loss, violators_lhs, violators_rhs, count, reg).  The first k CTAs of the embedding rows'
-// hub_reduce_kernel do this: as a kernel of its own it was 5 to 29 us per wave of one CTA per batch, and a launch.
+// hub_kernel do this: as a kernel of its own it was 5 to 29 us per wave of one CTA per batch, and a launch.
 __device__ __forceinline__ void batch_stats(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, int b, pbg_batch_stats *per_batch, double *sum) {
   __shared__ double sl[UPD_WARPS], sr[UPD_WARPS];
   __shared__ long long sv0[UPD_WARPS], sv1[UPD_WARPS];
@@ -620,120 +620,116 @@ __device__ __forceinline__ void batch_stats(const WaveDims &d, const WaveBatches
   }
 }
 
-// The few rows that collect hundreds of slots per wave (the top nodes of a power-law partition)
-// would keep one CTA of hub_update_kernel busy long after every other row is done.  One CTA per
-// (big row, batch) adds that batch's partial rows up first -- warp w takes runs w, w + 8, ..., the
-// eight sums are added in warp order -- and leaves the total in the batch's first partial row, so
-// that hub_update_kernel reads one row per batch of a big row.
-template <int VEC>
-__global__ void __launch_bounds__(32 * UPD_WARPS)
-hub_reduce_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys, const unsigned int *__restrict__ vals,
-                  float *__restrict__ psum, const long long *__restrict__ hublist, const int *__restrict__ hubcnt,
-                  int *__restrict__ hubcnt_next, long long *__restrict__ bigtab, int aside, ParamJob job, pbg_batch_stats *per_batch, double *sum) {
-  pdl_begin();
-  extern __shared__ __align__(16) float part[];              // [UPD_WARPS][VEC * 128]
-  if (blockIdx.x == 0 && threadIdx.x < 2) hubcnt_next[threadIdx.x] = 0;      // its last reader is behind us in the stream
-  // the first CTAs of the embedding rows' launch (aside) have other work
-  int cta0 = 0;
-  if (aside) {
-    cta0 = d.k + job.steps * ((d.D + 31) / 32);               // param_step_ctas
-    if (blockIdx.x < d.k) { batch_stats(d, wb, w, blockIdx.x, per_batch, sum); return; }
-    if (blockIdx.x < cta0) { param_step(d, wb, w, job, blockIdx.x - d.k, part); return; }
-  }
-  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  const int D = d.D;
-  const long long *biglist = hub_biglist(hublist, d.nocc);
-  const long long items = (long long)hubcnt[1] * d.k;        // the tile kernel listed the big rows
-  for (long long item = blockIdx.x - cta0; item < items; item += gridDim.x - cta0) {
-    const int h = (int)(item / d.k), b = (int)(item % d.k);
-    const long long head = biglist[h];
-    const unsigned long long key = keys[head];
-    const long long end = coop_prefix_end(head + HUB_BIG, (long long)d.nocc, [&](long long pos) { return keys[pos] == key; });
-    // where batch b starts and ends inside the row.  hub_update_kernel reads the answers from bigtab[h] ([b] = first
-    // slot of batch b or -1, [PBG_KMAX] = end of the row) instead of searching again.  (Both searches in the same
-    // rounds, half of the CTA each, measured slower: 14.2 against 11.8 us.)
-    const long long q = coop_prefix_end(head, end, [&](long long pos) { return (int)(vals[pos] / (unsigned int)d.spb) < b; });
-    const long long eb = coop_prefix_end(q, end, [&](long long pos) { return (int)(vals[pos] / (unsigned int)d.spb) <= b; });
-    if (threadIdx.x == 0) {
-      bigtab[(size_t)h * (PBG_KMAX + 1) + b] = q < eb ? q : -1;
-      if (b == 0) bigtab[(size_t)h * (PBG_KMAX + 1) + PBG_KMAX] = end;
-    }
-    if (q >= eb) continue;
-    const long long ftb = (q / TILE + 1) * TILE;
-    const long long nruns = 1 + (eb > ftb ? (eb - 1 - ftb) / TILE + 1 : 0);
-    if (nruns == 1) continue;
-    float4 acc[VEC];
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) acc[c] = f4zero();
-    // warp w takes runs w, w + 8, ...: four of its partial rows in flight at a time, added in run order
-    for (long long r0 = wl; r0 < nruns; r0 += 4 * UPD_WARPS) {
-      const float *src[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        long long r = r0 + (long long)u * UPD_WARPS;
-        src[u] = r < nruns ? psum + (size_t)(r == 0 ? q : ftb + (r - 1) * TILE) * d.Dp : nullptr;
-      }
-#pragma unroll
-      for (int c = 0; c < VEC; ++c) {
-        int dd = c * 128 + lane * 4;
-        if (dd < D) {
-          float4 v[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) v[u] = src[u] ? ld4(src[u] + dd) : f4zero();
-#pragma unroll
-          for (int u = 0; u < 4; ++u) acc[c] = acc[c] + v[u];
-        }
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) st4(&part[(size_t)wl * VEC * 128 + c * 128 + lane * 4], acc[c]);
-    __syncthreads();
-    float *dst = psum + (size_t)q * d.Dp;
-    for (int dd = threadIdx.x * 4; dd < D; dd += 4 * blockDim.x) {
-      float4 t = ld4(&part[dd]);
-#pragma unroll
-      for (int u = 1; u < UPD_WARPS; ++u) t = t + ld4(&part[(size_t)u * VEC * 128 + dd]);
-      st4(dst + dd, t);
-    }
-    __syncthreads();
-  }
-}
-
-// One CTA per hub row.  Its slots [head, end) are in batch order.  One probe per thread over the row's first 256
-// slots gives, in a single round of loads, the row's end and where each of its batches starts (rows of 256 and more
-// slots: searches); then warp w adds up the partial rows of batches w, w+8, ... (a batch's slots [q, eb) were summed
-// by the tile warps in runs that start at q and at every multiple of TILE inside (q, eb)) into tot[batch][] and,
-// for embedding rows, takes the batch's squared norm while it has the sum in registers; warp 0 applies the optimizer
-// steps in batch order from shared memory.  All sums run in a fixed order.
+// What is left after the tiles: the hub rows, and (aside) the work that rides along.
+//
+// A hub row's slots [head, end) are in batch order; the tile warps have summed them in runs that start at a batch's first
+// slot q and at every multiple of TILE inside the batch.  One CTA finishes a row: a probe per thread over its first 256
+// slots gives, in a single round of loads, the row's end and where each of its batches starts; warp w adds up the
+// partial rows of batches w, w + 8, ... into tot[batch][] and, for embedding rows, takes the batch's squared norm while it
+// has the sum in registers; then the optimizer steps are taken in batch order.
+//
+// The few rows that collect 256 and more slots per wave (the top nodes of a power-law partition) would keep one CTA busy
+// long after every other row is done.  For them one CTA per (row, batch) adds that batch's partial rows up first -- warp w
+// takes runs w, w + 8, ..., the eight sums are added in warp order -- leaves the total in the batch's first partial row and
+// the batch's start in the row's line of bigtab, and the CTA that finds itself the last of the row's batches finishes the
+// row.  (A kernel for the sums and one for the rows cost a launch and 9 us more per wave of 56,000 slots at dimension
+// 100: the second waited for the longest search of the first.)  All sums run in a fixed order.
 template <int VEC, int RULE>
 __global__ void __launch_bounds__(32 * UPD_WARPS)
-hub_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys,
-                  const unsigned int *__restrict__ vals, float lr, const float *__restrict__ psum,
-                  const long long *__restrict__ hublist, const int *__restrict__ hubcnt,
-                  const long long *__restrict__ bigtab) {
+hub_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys, const unsigned int *__restrict__ vals, float lr,
+           float *psum, const long long *__restrict__ hublist, const int *__restrict__ hubcnt, int *__restrict__ hubcnt_next,
+           long long *bigtab, int aside, ParamJob job, pbg_batch_stats *per_batch, double *sum) {
   pdl_begin();
   static_assert(32 * UPD_WARPS == HUB_BIG, "one probe per thread covers exactly the rows that are not big");
-  extern __shared__ __align__(16) float tot[];               // [k][VEC * 128]
+  extern __shared__ __align__(16) float tot[];               // [k][VEC * 128]; sums of a big row's batch: [UPD_WARPS][VEC * 128]
   __shared__ long long bstart[PBG_KMAX + 1];
   __shared__ float bnorm[PBG_KMAX];                           // mean squared gradient of a batch (embedding rows)
   __shared__ int sbatch[32 * UPD_WARPS];
   __shared__ unsigned long long skey;
   __shared__ long long bend;
+  __shared__ bool closing;
+  if (blockIdx.x == 0 && threadIdx.x < 2) hubcnt_next[threadIdx.x] = 0;      // its last reader is behind us in the stream
+  // the first CTAs of the embedding rows' launch (aside) have other work
+  int cta0 = 0;
+  if (RULE == RULE_EMB && aside) {
+    cta0 = d.k + job.steps * ((d.D + 31) / 32);               // param_step_ctas
+    if (blockIdx.x < d.k) { batch_stats(d, wb, w, blockIdx.x, per_batch, sum); return; }
+    if (blockIdx.x < cta0) { param_step(d, wb, w, job, blockIdx.x - d.k, tot); return; }
+  }
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int D = d.D;
   const float invD = 1.0f / (float)D;
-  const int nh = hubcnt[0], nbig = hubcnt[1];
+  const int nh = hubcnt[0], nbig = hubcnt[1];                 // the tile kernel listed the rows
   const long long *biglist = hub_biglist(hublist, d.nocc);
-  // the big rows first (theirs is the longest chain of dependent loads), then the list of all hub rows without them
-  for (int item = blockIdx.x; item < nbig + nh; item += gridDim.x) {
-    const bool from_big = item < nbig;
-    const long long head = from_big ? biglist[item] : hublist[item - nbig];
+  // the batches of the big rows first, then the list of all hub rows, big ones skipped
+  const int ctas = gridDim.x - cta0, items = nbig * d.k + nh;
+  for (int item = blockIdx.x - cta0; item < items; item += ctas) {
+    const bool from_big = item < nbig * d.k;
+    const int h = item / d.k;
+    const long long head = from_big ? biglist[h] : hublist[item - nbig * d.k];
+    long long *line = bigtab + (size_t)h * BIGTAB_LINE;       // [b] first slot of batch b or -1, then the row's end, then a counter
+    if (from_big) {
+      const int b = item - h * d.k;
+      const unsigned long long key = keys[head];
+      const long long end = coop_prefix_end(head + HUB_BIG, (long long)d.nocc, [&](long long pos) { return keys[pos] == key; });
+      // where batch b starts and ends inside the row.  (Both searches in the same rounds, half of the CTA each, measured
+      // slower: 14.2 against 11.8 us.)
+      const long long q = coop_prefix_end(head, end, [&](long long pos) { return (int)(vals[pos] / (unsigned int)d.spb) < b; });
+      const long long eb = coop_prefix_end(q, end, [&](long long pos) { return (int)(vals[pos] / (unsigned int)d.spb) <= b; });
+      const long long ftb = (q / TILE + 1) * TILE;
+      const long long nruns = q < eb ? 1 + (eb > ftb ? (eb - 1 - ftb) / TILE + 1 : 0) : 0;
+      if (nruns > 1) {
+        float4 acc[VEC];
+#pragma unroll
+        for (int c = 0; c < VEC; ++c) acc[c] = f4zero();
+        // four of the warp's partial rows in flight at a time, added in run order
+        for (long long r0 = wl; r0 < nruns; r0 += 4 * UPD_WARPS) {
+          const float *src[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            long long r = r0 + (long long)u * UPD_WARPS;
+            src[u] = r < nruns ? psum + (size_t)(r == 0 ? q : ftb + (r - 1) * TILE) * d.Dp : nullptr;
+          }
+#pragma unroll
+          for (int c = 0; c < VEC; ++c) {
+            int dd = c * 128 + lane * 4;
+            if (dd < D) {
+              float4 v[4];
+#pragma unroll
+              for (int u = 0; u < 4; ++u) v[u] = src[u] ? ld4(src[u] + dd) : f4zero();
+#pragma unroll
+              for (int u = 0; u < 4; ++u) acc[c] = acc[c] + v[u];
+            }
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < VEC; ++c) st4(&tot[(size_t)wl * VEC * 128 + c * 128 + lane * 4], acc[c]);
+        __syncthreads();
+        float *dst = psum + (size_t)q * d.Dp;
+        for (int dd = threadIdx.x * 4; dd < D; dd += 4 * blockDim.x) {
+          float4 t = ld4(&tot[dd]);
+#pragma unroll
+          for (int u = 1; u < UPD_WARPS; ++u) t = t + ld4(&tot[(size_t)u * VEC * 128 + dd]);
+          st4(dst + dd, t);
+        }
+      }
+      if (threadIdx.x == 0) {
+        line[b] = q < eb ? q : -1;
+        if (b == 0) line[PBG_KMAX] = end;
+      }
+      __threadfence();
+      __syncthreads();
+      if (threadIdx.x == 0) closing = atomicAdd((unsigned long long *)&line[PBG_KMAX + 1], 1ull) == (unsigned long long)(d.k - 1);
+      __syncthreads();
+      if (!closing) continue;                                 // another batch of the row is still being summed
+      __threadfence();
+      if (threadIdx.x == 0) line[PBG_KMAX + 1] = 0;           // for the next wave
+    }
     const long long p = head + threadIdx.x;
     const unsigned long long kp = p < (long long)d.nocc ? keys[p] : ~0ull;
     const int bp = p < (long long)d.nocc ? (int)(vals[p] / (unsigned int)d.spb) : -1;
-    // what hub_reduce_kernel found out about a big row: the starts of its batches and its end, one load each
-    long long tabv = -1;
-    if (from_big && threadIdx.x <= PBG_KMAX) tabv = bigtab[(size_t)item * (PBG_KMAX + 1) + threadIdx.x];
+    // what the CTAs of a big row's batches left (past L1: this CTA may have read the lines before)
+    const long long tabv = from_big && threadIdx.x <= PBG_KMAX ? __ldcg(line + threadIdx.x) : -1;
     if (threadIdx.x == 0) skey = kp;
     for (int i = threadIdx.x; i <= PBG_KMAX; i += blockDim.x) bstart[i] = -1;
     __syncthreads();
@@ -750,7 +746,7 @@ hub_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long lo
       }
     }
     const int cnt = __syncthreads_count(in);                  // slots of the row among the first 256 (they are contiguous)
-    const bool big = cnt == (int)blockDim.x;                  // hub_reduce_kernel left one row per batch
+    const bool big = cnt == (int)blockDim.x;                  // one row per batch is left of it
     if (big && !from_big) continue;                           // taken from the list of big rows
     long long end = head + cnt;
     if (!big) {
@@ -787,7 +783,7 @@ hub_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long lo
           if (dd < D) {
             float4 v[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = src[u] ? ld4(src[u] + dd) : f4zero();
+            for (int u = 0; u < 4; ++u) v[u] = src[u] ? (big ? __ldcg((const float4 *)(src[u] + dd)) : ld4(src[u] + dd)) : f4zero();
 #pragma unroll
             for (int u = 0; u < 4; ++u) acc[c] = acc[c] + v[u];
           }
@@ -799,9 +795,9 @@ hub_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long lo
         // the same expression, on the same values, as RowState::step evaluates
         float ss = 0.f;
 #pragma unroll
-        for (int c = 0; c < VEC; ++c) ss += f4dot(acc[c], acc[c]);
+        for (int c = 0; c < VEC; ++c) ss += f4dot_yx(acc[c], acc[c]);
         ss = warp_sum(ss);
-        if (lane == 0) bnorm[bq] = ss * invD;
+        if (lane == 0) bnorm[bq] = __fmul_rn(ss, invD);
       }
     }
     __syncthreads();
@@ -812,7 +808,7 @@ hub_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long lo
     // rescale first needs its norm: that case keeps the one-warp form.)
     // With more hub rows than CTAs (a small graph, where every row is one) the kernel is bound by the instructions it
     // executes, not by one row's chain, and the one-warp form executes fewer.
-    if ((RULE == RULE_EMB && d.max_norm > 0.f) || nh + nbig > (int)gridDim.x) {
+    if ((RULE == RULE_EMB && d.max_norm > 0.f) || items > ctas) {
       if (wl == 0) {
         RowState<VEC, RULE> rs;
         rs.load(d, w, key, lane);
@@ -1053,17 +1049,16 @@ static int launch_update_vec(const WaveDims &d, const WaveBatches &wb, const Wav
                              const UpdateScratch &us, cudaStream_t st) {
   constexpr int EMB_WARPS = TileWarps<VEC, RULE_EMB>::N, REL_WARPS = TileWarps<VEC, RULE_REL>::N;
   const long long tiles = ((long long)d.nocc + TILE - 1) / TILE;
-  const int hub_ctas = 296;     // (two and four times as many measured the same: the kernels take as long as their longest row)
-  const size_t hub_smem = (size_t)d.k * VEC * 128 * sizeof(float);            // per-batch totals of one hub row
-  const size_t red_smem = (size_t)UPD_WARPS * VEC * 128 * sizeof(float);       // eight partial sums of one batch of a big row
+  const int hub_ctas = 592;     // (half and twice as many measured the same: the kernel takes as long as its longest row)
+  // per-batch totals of one hub row, or eight partial sums of one batch of a big row
+  const size_t hub_smem = (size_t)(d.k > UPD_WARPS ? d.k : UPD_WARPS) * VEC * 128 * sizeof(float);
   static_assert(PBG_KMAX * 32 <= UPD_WARPS * 128, "param_step works in the same shared memory");
   // the attribute is set once for the largest wave this row width allows in 227 KB
   size_t hub_smem_max = (size_t)PBG_KMAX * VEC * 128 * sizeof(float);
   if (hub_smem_max > 227 * 1024) hub_smem_max = 227 * 1024;
   // per device (a process may hold contexts on several GPUs); a failed opt-in makes the launch fail,
   // which the caller's cudaGetLastError reports
-  pbg_opt_in_smem((const void *)hub_update_kernel<VEC, RULE_EMB>, (int)hub_smem_max);
-  pbg_opt_in_smem((const void *)hub_reduce_kernel<VEC>, (int)red_smem);
+  pbg_opt_in_smem((const void *)hub_kernel<VEC, RULE_EMB>, (int)hub_smem_max);
   pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_EMB>, EMB_WARPS * StageRows<VEC, RULE_EMB>::N * VEC * 512);
   ParamJob job;
   int launches = launch_pullback<VEC>(d, wb, w, rel_lr, job, st);
@@ -1073,19 +1068,19 @@ static int launch_update_vec(const WaveDims &d, const WaveBatches &wb, const Wav
   size_t tile_smem = (size_t)EMB_WARPS * StageRows<VEC, RULE_EMB>::N * d.Dp * 4;
   if (sum_ctas && tile_smem < 8 * 128 * 4) tile_smem = 8 * 128 * 4;
   pbg_launch(tile_update_kernel<VEC, RULE_EMB>, sum_ctas + (unsigned)((tiles + EMB_WARPS - 1) / EMB_WARPS), 32 * EMB_WARPS, tile_smem, st, d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, job, sum_ctas);
-  pbg_launch(hub_reduce_kernel<VEC>, d.k + param_step_ctas(d, job) + 2 * hub_ctas, 32 * UPD_WARPS, red_smem, st, d, wb, w, keys, vals, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 1, job, us.per_batch, us.sum);
-  pbg_launch(hub_update_kernel<VEC, RULE_EMB>, hub_ctas, 32 * UPD_WARPS, hub_smem, st, d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, us.bigtab);
-  launches += 3;
+  pbg_launch(hub_kernel<VEC, RULE_EMB>, d.k + param_step_ctas(d, job) + hub_ctas, 32 * UPD_WARPS, hub_smem, st,
+             d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 1, job, us.per_batch, us.sum);
+  launches += 2;
   if (d.op != PBG_OP_NONE && w.theta[0] != nullptr) {
     if (d.dynamic) {
-      pbg_opt_in_smem((const void *)hub_update_kernel<VEC, RULE_REL>, (int)hub_smem_max);
+      pbg_opt_in_smem((const void *)hub_kernel<VEC, RULE_REL>, (int)hub_smem_max);
       pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_REL>, REL_WARPS * TILE * VEC * 512);
       int *t = hubcnt; hubcnt = hubcnt_next; hubcnt_next = t;
       ++*us.turn;
       pbg_launch(tile_update_kernel<VEC, RULE_REL>, (unsigned)((tiles + REL_WARPS - 1) / REL_WARPS), 32 * REL_WARPS, (size_t)REL_WARPS * TILE * d.Dp * 4, st, d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt, job, 0);
-      pbg_launch(hub_reduce_kernel<VEC>, 2 * hub_ctas, 32 * UPD_WARPS, red_smem, st, d, wb, w, keys, vals, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 0, job, nullptr, nullptr);
-      pbg_launch(hub_update_kernel<VEC, RULE_REL>, hub_ctas, 32 * UPD_WARPS, hub_smem, st, d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt, us.bigtab);
-      launches += 3;
+      pbg_launch(hub_kernel<VEC, RULE_REL>, hub_ctas, 32 * UPD_WARPS, hub_smem, st,
+                 d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 0, job, (pbg_batch_stats *)nullptr, (double *)nullptr);
+      launches += 2;
     } else if (d.matrix_op) {
       launches += launch_matrix_update(d, wb, w, rel_lr, st);
     }

@@ -59,10 +59,11 @@ SYMBOLS = [
     ("pbg_last_error", C.c_char_p, [_P]),
     ("pbg_workspace_bytes", C.c_int64, [_P]),
     ("pbg_set_hyperparameters", C.c_int, [_P, C.c_float, C.c_float, C.c_float]),
-    ("pbg_train_batches", C.c_int, [_P, C.POINTER(PbgBucket), _P, _P, _P, C.c_int64, C.POINTER(PbgBatch),
-                                    C.c_int32, _P, _P, C.c_uint64, C.POINTER(PbgBatchStats)]),
-    ("pbg_train_batches_host", C.c_int, [_P, C.POINTER(PbgBucket), _P, _P, _P, C.c_int64, C.POINTER(PbgBatch),
-                                         C.c_int32, _P, _P, C.c_uint64, C.POINTER(PbgBatchStats)]),
+    # (batch lists and Stats by address: arrays of PbgBatch / PbgBatchStats, NumPy records or byref())
+    ("pbg_train_batches", C.c_int, [_P, C.POINTER(PbgBucket), _P, _P, _P, C.c_int64, _P,
+                                    C.c_int32, _P, _P, C.c_uint64, _P]),
+    ("pbg_train_batches_host", C.c_int, [_P, C.POINTER(PbgBucket), _P, _P, _P, C.c_int64, _P,
+                                         C.c_int32, _P, _P, C.c_uint64, _P]),
     ("pbg_read_stats", C.c_int, [_P, C.POINTER(PbgBatchStats)]),
     ("pbg_score_batch", C.c_int, [_P, C.POINTER(PbgBucket), _P, _P, _P, C.c_int32, C.c_int32, _P, _P,
                                   C.c_uint64, _P, _P, _P, _P]),

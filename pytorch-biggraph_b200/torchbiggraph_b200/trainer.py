@@ -21,7 +21,7 @@ from .types import EdgeList, Stats
 
 
 def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 # the C structures pbg_batch and pbg_batch_stats as array records
@@ -135,10 +135,12 @@ class _Native:
         rel = edges.rel.to(dev).contiguous() if dyn else None
         relidx = 0 if dyn else edges.get_relation_type_as_scalar()
         local = 0 if dyn else model.group_of[relidx][1]
-        P, Cn, lc, rc = (C.c_int32() for _ in range(4))
-        check(self.lib.pbg_neg_columns(self.ctx, n, C.byref(P), C.byref(Cn), C.byref(lc), C.byref(rc)), self.ctx)
-        lp = torch.empty(n, device=dev); rp = torch.empty(n, device=dev)
-        ln = torch.empty((n, lc.value), device=dev); rn = torch.empty((n, rc.value), device=dev)
+        # negative columns per side (pbg_neg_columns; model.py:648-656)
+        nb, nu = self.cfg.num_batch_negs, self.cfg.num_uniform_negs
+        cols = (min(nb, n) if nb > 0 else 0) + nu
+        lc, rc = 0 if self.cfg.disable_lhs_negs else cols, 0 if self.cfg.disable_rhs_negs else cols
+        lp, rp, ln, rn = torch.empty(n * (2 + lc + rc), device=dev).split((n, n, n * lc, n * rc))
+        ln, rn = ln.view(n, lc), rn.view(n, rc)
         ul = None if ul is None else self._uniform(ul, dev)
         ur = None if ur is None else self._uniform(ur, dev)
         b = self.bucket(model, relidx, None, None)
@@ -268,13 +270,24 @@ class B200Trainer(AbstractBatchProcessor):
         """One library call over _BATCH records that read one pair of tables through one operator; the _STATS records of
         the batches, or None when they are not wanted."""
         dyn = model.num_dynamic_rels > 0
-        rels = np.zeros(1, np.int32) if dyn else batches["rel"]
-        relation_idx = int(rels[0])
-        for r in (relation_idx,) if len(batches) == 1 else np.unique(rels).tolist():
+        rels = [0] if dyn else np.unique(batches["rel"]).tolist()
+        nat, bucket, local = self._bound(model, 0 if dyn else int(batches["rel"][0]), rels, int(batches["count"].max()))
+        if local is not None:
+            batches = batches.copy()
+            batches["rel"] = local[batches["rel"]] if not dyn else 0
+        stats = np.empty(len(batches), dtype=_STATS) if want_stats else None
+        self._call(nat, bucket, model, lhs, rhs, rel, batches.ctypes.data, len(batches), uniform_lhs, uniform_rhs,
+                   stats.ctypes.data if want_stats else None, weights)
+        return stats
+
+    def _bound(self, model, relation_idx: int, rels, max_count: int):
+        """(context, bucket structure, place of every relation in its operator group -- or None where it is its index) for
+        batches of relations `rels`, which read the tables of `relation_idx`."""
+        for r in rels:
             if model.relations[r].all_negs:
                 raise NotImplementedError("relations with all_negs=True are not trained by torchbiggraph_b200 (the evaluator ranks them)")
         op_name = model.operator_of(relation_idx)
-        nat = self._context(model, int(batches["count"].max()), op_name)
+        nat = self._context(model, max_count, op_name)
         wl, wr = model.tables_for(relation_idx)
         al, ar = self._op_states(model, op_name)
         gl = self._state_for(wl)
@@ -285,12 +298,15 @@ class B200Trainer(AbstractBatchProcessor):
                 raise RuntimeError("the model has global embeddings but model_optimizer is not an AsyncAdagrad over them")
             states = states + (self.model_optimizer.sum_for(gl_), self.model_optimizer.sum_for(gr_))
         # the library indexes operator rows and relation weights by the relation's place in its operator group
+        dyn = model.num_dynamic_rels > 0
         members = [0] if dyn else model.op_groups[op_name]
         bucket = nat.bucket(model, relation_idx, states, [self.relation_weights[g] for g in members])
-        desc = batches
         if dyn or len(members) != len(model.relations):
-            desc = batches.copy()
-            desc["rel"] = 0 if dyn else np.array([g[1] for g in model.group_of], dtype=np.int32)[rels]
+            return nat, bucket, np.array([g[1] for g in model.group_of], dtype=np.int32)
+        return nat, bucket, None
+
+    def _call(self, nat, bucket, model, lhs, rhs, rel, batches: int, num_batches: int, uniform_lhs, uniform_rhs, stats: Optional[int], weights):
+        """pbg_train_batches, or with edges on the host pbg_train_batches_host; `batches` and `stats` are addresses."""
         on_host = lhs.device.type == "cpu"
         fn = nat.lib.pbg_train_batches_host if on_host else nat.lib.pbg_train_batches
         for t in (lhs, rhs, rel, uniform_lhs, uniform_rhs):
@@ -302,11 +318,8 @@ class B200Trainer(AbstractBatchProcessor):
                 raise ValueError("one weight per edge is needed")
             weights = weights.to(device=model.device, dtype=torch.float32).contiguous()     # kept alive until the call returns
             check(nat.lib.pbg_set_edge_weights(nat.ctx, _ptr(weights)), nat.ctx)
-        stats = np.empty(len(desc), dtype=_STATS) if want_stats else None
-        check(fn(nat.ctx, C.byref(bucket), _ptr(lhs), _ptr(rhs), _ptr(rel), lhs.shape[0],
-                 C.cast(desc.ctypes.data, C.POINTER(PbgBatch)), len(desc), _ptr(uniform_lhs), _ptr(uniform_rhs), self.seed + self._calls,
-                 C.cast(stats.ctypes.data, C.POINTER(PbgBatchStats)) if want_stats else None), nat.ctx)
-        return stats
+        check(fn(nat.ctx, C.byref(bucket), _ptr(lhs), _ptr(rhs), _ptr(rel), lhs.shape[0], batches, num_batches,
+                 _ptr(uniform_lhs), _ptr(uniform_rhs), self.seed + self._calls, stats), nat.ctx)
 
     def read_stats(self) -> Stats:
         s = PbgBatchStats()
@@ -330,11 +343,13 @@ class B200Trainer(AbstractBatchProcessor):
         rhs = batch_edges.rhs.to_tensor().to(dev).contiguous()
         rel = batch_edges.rel.to(dev).contiguous() if dyn else None
         r = 0 if dyn else batch_edges.get_relation_type_as_scalar()
-        nat = self._context(model, n, model.operator_of(r))
+        nat, bucket, local = self._bound(model, r, (r,), n)
         ul = None if uniform_lhs is None else nat._uniform(uniform_lhs, dev)
         ur = None if uniform_rhs is None else nat._uniform(uniform_rhs, dev)
         wgt = torch.as_tensor(batch_edges.weight) if batch_edges.has_weight() else None
-        return self.train_batches(model, lhs, rhs, rel, [(0, n, r)], ul, ur, weights=wgt)[0]
+        b, s = PbgBatch(0, n, r if local is None else int(local[r])), PbgBatchStats()
+        self._call(nat, bucket, model, lhs, rhs, rel, C.addressof(b), 1, ul, ur, C.addressof(s), wgt)
+        return Stats(loss=s.loss, reg=s.reg, violators_lhs=s.violators_lhs, violators_rhs=s.violators_rhs, count=s.count)
 
     def process_one_batch(self, model, batch_edges, uniform_lhs=None, uniform_rhs=None) -> Stats:
         if self.overrides is not None:
