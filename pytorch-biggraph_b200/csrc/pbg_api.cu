@@ -58,8 +58,13 @@ struct pbg_context {
   // scratch of the edge-list utilities (pbg_randperm, pbg_sub_bucket): grown on demand
   SortPlan esort = {{nullptr, nullptr}, {nullptr, nullptr}, nullptr, 0, 0};
   char *esort_mem = nullptr;
-  long long *etab_dev = nullptr;      // per-relation tables of a sub_bucket call + its counts
+  char *rp_mem = nullptr;             // buckets and counters of pbg_randperm
+  size_t rp_bytes = 0;
+  unsigned rp_turn = 0;
+  long long *etab_dev = nullptr;      // per-relation tables of a sub_bucket call of many relations
   long long etab_cap = 0;
+  long long *counts_host = nullptr, *counts_dev = nullptr;   // sub-bucket sizes, written by the kernels
+  long long counts_cap = 0;
   int allnegs_slab = 0;
   long long allnegs_rows = 0;         // rows of the largest table it was sized for
   char *allnegs_mem = nullptr;        // scratch of pbg_eval_batch_all_negs, allocated at its first call
@@ -357,6 +362,8 @@ extern "C" int pbg_destroy(pbg_context *c) {
   for (int i = 0; i < 3; ++i) if (c->edge_dev[i]) cudaFree(c->edge_dev[i]);
   for (int i = 0; i < 2; ++i) if (c->uni_dev[i]) cudaFree(c->uni_dev[i]);
   if (c->esort_mem) cudaFree(c->esort_mem);
+  if (c->rp_mem) cudaFree(c->rp_mem);
+  if (c->counts_host) cudaFreeHost(c->counts_host);
   if (c->allnegs_mem) cudaFree(c->allnegs_mem);
   if (c->etab_dev) cudaFree(c->etab_dev);
   for (int s = 0; s < 2; ++s) {
@@ -904,6 +911,19 @@ extern "C" int pbg_randperm(pbg_context *c, int64_t n, uint64_t seed, int64_t *o
   if (n == 0) return PBG_OK;
   if (!out || n < 0) return fail(c, PBG_ERR_BAD_ARGUMENT, "bad randperm arguments");
   CU(c, cudaSetDevice(c->device));
+  const size_t need = pbg_randperm_bytes(n);
+  if (need) {
+    if (need > c->rp_bytes) {
+      if (c->rp_mem) { cudaFree(c->rp_mem); c->rp_mem = nullptr; c->rp_bytes = 0; }
+      CU(c, cudaMalloc(&c->rp_mem, need));
+      CU(c, cudaMemsetAsync(c->rp_mem, 0, need, c->stream));
+      c->rp_bytes = need;
+    }
+    c->launches += launch_randperm_dealt(c->rp_mem, c->rp_turn++, n, seed, (long long *)out, c->errflag, c->stream);
+    CU(c, pbg_take_launch_error());
+    int flag = 0, rcf = wait_for_flag(c, flag);
+    if (rcf || !(flag & 256)) return rcf;                    // 256: a bucket overflowed; the general sort below
+  }
   int rc = ensure_edge_sort(c, n);
   if (rc) return rc;
   c->launches += launch_randperm(c->esort, n, seed, (long long *)out, c->stream);
@@ -927,12 +947,21 @@ extern "C" int pbg_sub_bucket(pbg_context *c, const int64_t *lhs_in, const int64
   CU(c, cudaSetDevice(c->device));
   int rc = ensure_edge_sort(c, num_edges);
   if (rc) return rc;
-  const long long need = 6ll * R + (long long)nl * nr;
-  if (need > c->etab_cap) {
-    if (c->etab_dev) cudaFree(c->etab_dev);
-    c->etab_dev = nullptr;
-    CU(c, cudaMalloc(&c->etab_dev, (size_t)(need + 64) * sizeof(long long)));
-    c->etab_cap = need + 64;
+  const long long need = 6ll * R, nb = (long long)nl * nr;
+  if (!pbg_sub_bucket_inline(R) || nb >= 1024) {
+    if (need > c->etab_cap) {
+      if (c->etab_dev) cudaFree(c->etab_dev);
+      c->etab_dev = nullptr;
+      CU(c, cudaMalloc(&c->etab_dev, (size_t)(need + 64) * sizeof(long long)));
+      c->etab_cap = need + 64;
+    }
+  }
+  if (nb > c->counts_cap) {                                   // sizes come back through pinned memory the kernel writes
+    if (c->counts_host) cudaFreeHost(c->counts_host);
+    c->counts_host = nullptr; c->counts_cap = 0;
+    CU(c, cudaHostAlloc((void **)&c->counts_host, (size_t)(nb + 64) * sizeof(long long), cudaHostAllocMapped | cudaHostAllocPortable));
+    CU(c, cudaHostGetDevicePointer((void **)&c->counts_dev, c->counts_host, 0));
+    c->counts_cap = nb + 64;
   }
   std::vector<long long> tab((size_t)need, 0);
   for (int r = 0; r < R; ++r) {
@@ -945,13 +974,16 @@ extern "C" int pbg_sub_bucket(pbg_context *c, const int64_t *lhs_in, const int64
     tab[4 * R + r] = (lhs_entity_counts[r] + nl - 1) / nl;                               // util.cpp:296-315
     tab[5 * R + r] = (rhs_entity_counts[r] + nr - 1) / nr;
   }
-  CU(c, cudaMemcpyAsync(c->etab_dev, tab.data(), (size_t)6 * R * sizeof(long long), cudaMemcpyHostToDevice, c->stream));
-  CU(c, cudaStreamSynchronize(c->stream));                                               // tab is a local: the copy must have left it
-  long long *counts_dev = c->etab_dev + 6 * R;
-  c->launches += launch_sub_bucket(c->esort, (const long long *)lhs_in, (const long long *)rhs_in, (const long long *)rel_in, num_edges, R,
+  if (!pbg_sub_bucket_inline(R) || nb >= 1024) {
+    CU(c, cudaMemcpyAsync(c->etab_dev, tab.data(), (size_t)6 * R * sizeof(long long), cudaMemcpyHostToDevice, c->stream));
+    CU(c, cudaStreamSynchronize(c->stream));                                             // tab is a local: the copy must have left it
+  }
+  c->launches += launch_sub_bucket(c->esort, (const long long *)lhs_in, (const long long *)rhs_in, (const long long *)rel_in, num_edges, R, tab.data(),
                                    c->etab_dev, nl, nr, dynamic_relations != 0, (long long *)lhs_out, (long long *)rhs_out,
-                                   (long long *)rel_out, counts_dev, c->errflag, c->stream);
+                                   (long long *)rel_out, c->counts_dev, c->errflag, c->stream);
   CU(c, pbg_take_launch_error());
-  CU(c, cudaMemcpyAsync(sub_bucket_counts, counts_dev, (size_t)nl * nr * sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
-  return check_errflag_edges(c, "sub_bucket");
+  const int rcs = check_errflag_edges(c, "sub_bucket");
+  if (num_edges == 0) memset(c->counts_host, 0, (size_t)nb * sizeof(long long));
+  memcpy(sub_bucket_counts, c->counts_host, (size_t)nb * sizeof(long long));
+  return rcs;
 }

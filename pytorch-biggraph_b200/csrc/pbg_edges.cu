@@ -20,23 +20,107 @@ __global__ void reverse_permutation_kernel(const long long *__restrict__ perm, l
   out[p] = i;
 }
 
-// out row perm[r] = in row r, rows of `units` elements of type T
+// out row perm[r] = in row r.  A group of G threads moves a row of `units` elements of type T, four elements per thread in
+// flight; G is the power of two that covers a row in at most four steps.  (One thread per element divided a 64-bit index
+// by the row length for every 16 bytes: 4.4 TB/s on 303,000 rows of 400 bytes.)
 template <class T>
-__global__ void shuffle_rows_kernel(const T *__restrict__ in, T *__restrict__ out, long long rows, long long units,
-                                    const long long *__restrict__ perm, int *errflag) {
-  long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= rows * units) return;
-  long long r = idx / units, u = idx - r * units;
-  long long p = perm[r];
-  if (p < 0 || p >= rows) { if (u == 0) atomicOr(errflag, 1); return; }
-  out[p * units + u] = in[idx];
+__global__ void __launch_bounds__(256) shuffle_rows_kernel(const T *__restrict__ in, T *__restrict__ out, long long rows, int units, int G,
+                                                           const long long *__restrict__ perm, int *errflag) {
+  const int per = 256 / G, sub = threadIdx.x % G;
+  const long long r = (long long)blockIdx.x * per + threadIdx.x / G;
+  if (r >= rows) return;
+  const long long p = perm[r];
+  if (p < 0 || p >= rows) { if (sub == 0) atomicOr(errflag, 1); return; }
+  const T *src = in + r * units;
+  T *dst = out + p * units;
+  for (int u0 = sub; u0 < units; u0 += 4 * G) {
+    T v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) if (u0 + k * G < units) v[k] = src[u0 + k * G];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) if (u0 + k * G < units) dst[u0 + k * G] = v[k];
+  }
 }
 
-// keys of a random permutation: 44 hashed bits per index (ties, vanishingly rare, keep index order: still a permutation)
+// A random permutation is the indices in the order of (44 hashed bits, index); ties, vanishingly rare, keep index order.
+__device__ __forceinline__ unsigned long long randperm_hash(unsigned long long seed, long long i) {
+  return pbg_mix64(seed ^ pbg_mix64((unsigned long long)i + 0x51ED270B0F1ull)) >> 20;
+}
+
+// Up to RP_MAX indices in two kernels: the hash is uniform, so its top bits deal the indices to buckets of about 1,000 to
+// 2,000, which a CTA sorts in shared memory.  A bucket has room for RP_CAP; one that overflows (a thousand standard
+// deviations away) raises the error word's bit 8 and the caller takes the general sort.  Keys in a bucket: the remaining
+// hash bits above the index (55 bits together), one comparison for both.  (Four radix passes of three launches took 260 us for
+// 269,507 indices.)
+#define RP_CAP 4096
+#define RP_MAX (1ll << 22)
+#define RP_MAX_BUCKETS 2048
+static int rp_index_bits(long long n) { int b = 1; while ((n - 1) >> b) ++b; return b; }
+static int rp_bits(long long n) { int b = 0; while ((n >> b) > 2048 && (1 << b) < RP_MAX_BUCKETS) ++b; return b; }
+
+__global__ void __launch_bounds__(256) randperm_deal_kernel(long long n, unsigned long long seed, int bits, int index_bits, unsigned long long *buckets, unsigned int *count,
+                                                            unsigned int *count_next, int *errflag) {
+  __shared__ unsigned int cnt[RP_MAX_BUCKETS];
+  const int nb = 1 << bits, t = threadIdx.x;
+  if (blockIdx.x == 0) for (int i = t; i < RP_MAX_BUCKETS; i += 256) count_next[i] = 0u;      // last read by the call before this one
+  for (int i = t; i < nb; i += 256) cnt[i] = 0u;
+  __syncthreads();
+  unsigned long long h[8];
+  unsigned int at[8];
+  const long long i0 = (long long)blockIdx.x * 2048 + t;
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const long long i = i0 + u * 256;
+    if (i < n) { h[u] = randperm_hash(seed, i); at[u] = atomicAdd(&cnt[h[u] >> (44 - bits)], 1u); }
+  }
+  __syncthreads();
+  for (int i = t; i < nb; i += 256) cnt[i] = cnt[i] ? atomicAdd(&count[i], cnt[i]) : 0u;   // where this CTA's part of the bucket begins
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const long long i = i0 + u * 256;
+    if (i >= n) continue;
+    const unsigned int b = (unsigned int)(h[u] >> (44 - bits)), pos = cnt[b] + at[u];
+    if (pos < RP_CAP) buckets[(size_t)b * RP_CAP + pos] = (h[u] & ((1ull << (44 - bits)) - 1ull)) << index_bits | (unsigned long long)i;
+    else atomicOr(errflag, 256);
+  }
+}
+
+// one CTA per bucket: bitonic sort of its keys (padded to a power of two), indices out behind the smaller buckets'
+__global__ void __launch_bounds__(1024) randperm_sort_kernel(const unsigned long long *__restrict__ buckets, const unsigned int *__restrict__ count,
+                                                             int index_bits, long long *__restrict__ out) {
+  __shared__ unsigned long long key[RP_CAP];
+  __shared__ unsigned int below[32];
+  const int t = threadIdx.x, b = blockIdx.x;
+  const int n = count[b] < RP_CAP ? (int)count[b] : RP_CAP;
+  unsigned int s = 0u;
+  for (int i = t; i < b; i += 1024) s += count[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((t & 31) == 0) below[t >> 5] = s;
+  int size = 2;
+  while (size < n) size <<= 1;
+  for (int i = t; i < size; i += 1024) key[i] = i < n ? buckets[(size_t)b * RP_CAP + i] : ~0ull;
+  __syncthreads();
+  for (int k = 2; k <= size; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int p = t; p < size / 2; p += 1024) {
+        const int lo = (p / j) * 2 * j + p % j, hi = lo + j;
+        const unsigned long long x = key[lo], y = key[hi];
+        if ((x > y) == ((lo & k) == 0)) { key[lo] = y; key[hi] = x; }
+      }
+      __syncthreads();
+    }
+  unsigned int base = 0u;
+  for (int u = 0; u < 32; ++u) base += below[u];
+  for (int i = t; i < n; i += 1024) out[base + i] = (long long)(key[i] & ((1ull << index_bits) - 1ull));
+}
+
+// the general form, any length: keys for the radix sort
 __global__ void randperm_keys_kernel(long long n, unsigned long long seed, unsigned long long *keys, unsigned int *vals) {
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  keys[i] = pbg_mix64(seed ^ pbg_mix64((unsigned long long)i + 0x51ED270B0F1ull)) >> 20;
+  keys[i] = randperm_hash(seed, i);
   vals[i] = (unsigned int)i;
 }
 __global__ void widen_kernel(const unsigned int *__restrict__ vals, long long n, long long *__restrict__ out) {
@@ -53,6 +137,18 @@ struct SubBucketArgs {
   const long long *lcount, *rcount, *lsize, *rsize;
   int R, nl, nr, dynamic;
 };
+// The same tables inside the kernel's parameters, for up to SB_INLINE relations (no upload, no wait for it).
+#define SB_INLINE 16
+struct SubBucketTables { long long v[6 * SB_INLINE]; };
+
+// the argument structure with its table pointers aimed at the tables in the parameters (in_dev null) or in device memory
+__device__ __forceinline__ SubBucketArgs sub_bucket_bind(SubBucketArgs a, const SubBucketTables &in, const long long *in_dev) {
+  const long long *t = in_dev ? in_dev : in.v;
+  a.lperm = (const long long *const *)t;
+  a.rperm = (const long long *const *)(t + a.R);
+  a.lcount = t + 2 * a.R; a.rcount = t + 3 * a.R; a.lsize = t + 4 * a.R; a.rsize = t + 5 * a.R;
+  return a;
+}
 
 // permuted offsets of edge e; false (and the error word set) when an id is outside its table
 __device__ __forceinline__ bool sub_bucket_offsets(const SubBucketArgs &a, long long e, long long &lo, long long &ro, long long &relid, int *errflag) {
@@ -66,6 +162,106 @@ __device__ __forceinline__ bool sub_bucket_offsets(const SubBucketArgs &a, long 
   return true;
 }
 
+// Up to SB_BINS - 1 sub-buckets (127 x 127 need more): stable counting sort in three launches that carry the edges along --
+//   sub_bucket_hist     every warp owns a run of SB_RUN consecutive edges, keeps their keys and counts them into
+//                       hist[key][warp]
+//   sub_bucket_scan     one CTA per key: exclusive scan of its row of warp counts; the row's total is the sub-bucket's size
+//   sub_bucket_scatter  every warp walks its run in order and writes each edge's offsets to its place
+// (Keys, a radix pass over (key, index) pairs, a gather and binary searches for the sizes were six launches.)
+#define SB_RUN 256
+#define SB_WARPS 4
+#define SB_BINS 1024
+__global__ void __launch_bounds__(32 * SB_WARPS) sub_bucket_hist(SubBucketArgs args, const __grid_constant__ SubBucketTables in, const long long *in_dev, unsigned short *keys,
+                                                                 unsigned int *hist, int nwarps, int *errflag) {
+  __shared__ unsigned int cnt[SB_WARPS][SB_BINS];
+  const SubBucketArgs a = sub_bucket_bind(args, in, in_dev);
+  const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31, wg = blockIdx.x * SB_WARPS + wl, nb = a.nl * a.nr;
+  if (wg >= nwarps) return;
+  for (int i = lane; i <= nb; i += 32) cnt[wl][i] = 0u;
+  __syncwarp();
+#pragma unroll
+  for (int it = 0; it < SB_RUN / 32; ++it) {
+    const long long e = (long long)wg * SB_RUN + it * 32 + lane;
+    int key = nb;                                            // edges that cannot be placed come last
+    if (e < a.n) {
+      long long lo, ro, relid;
+      if (sub_bucket_offsets(a, e, lo, ro, relid, errflag)) key = (int)(lo / a.lsize[relid]) * a.nr + (int)(ro / a.rsize[relid]);
+      keys[e] = (unsigned short)key;
+      atomicAdd(&cnt[wl][key], 1u);
+    }
+  }
+  __syncwarp();
+  for (int i = lane; i <= nb; i += 32) hist[(size_t)i * nwarps + wg] = cnt[wl][i];
+}
+
+__global__ void __launch_bounds__(256) sub_bucket_scan(unsigned int *hist, int nwarps, int nb, unsigned int *totals, long long *counts) {
+  __shared__ unsigned int part[8];
+  unsigned int *row = hist + (size_t)blockIdx.x * nwarps;
+  const int t = threadIdx.x, lane = t & 31, wl = t >> 5;
+  unsigned int carry = 0u;
+  for (int i0 = 0; i0 < nwarps; i0 += 256) {
+    const int i = i0 + t;
+    const unsigned int v = i < nwarps ? row[i] : 0u;
+    unsigned int incl = v;
+    for (int o = 1; o < 32; o <<= 1) { const unsigned int x = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += x; }
+    if (lane == 31) part[wl] = incl;
+    __syncthreads();
+    unsigned int before = carry, all = carry;
+    for (int u = 0; u < 8; ++u) { if (u < wl) before += part[u]; all += part[u]; }
+    if (i < nwarps) row[i] = before + incl - v;
+    carry = all;
+    __syncthreads();
+  }
+  if (t == 0) {
+    totals[blockIdx.x] = carry;
+    if (blockIdx.x < nb) counts[blockIdx.x] = carry;
+  }
+}
+
+__global__ void __launch_bounds__(32 * SB_WARPS) sub_bucket_scatter(SubBucketArgs args, const __grid_constant__ SubBucketTables in, const long long *in_dev,
+                                                                    const unsigned short *__restrict__ keys, const unsigned int *__restrict__ hist,
+                                                                    const unsigned int *__restrict__ totals, int nwarps, long long *lhs_out, long long *rhs_out,
+                                                                    long long *rel_out, int *errflag) {
+  __shared__ unsigned int base[SB_BINS], pos[SB_WARPS][SB_BINS];
+  __shared__ unsigned int wsum[SB_WARPS];
+  const SubBucketArgs a = sub_bucket_bind(args, in, in_dev);
+  const int t = threadIdx.x, wl = t >> 5, lane = t & 31, wg = blockIdx.x * SB_WARPS + wl, nb = a.nl * a.nr;
+  // where each sub-bucket begins: exclusive scan of the totals, a contiguous part per thread
+  {
+    const int per = (nb + 32 * SB_WARPS - 1) / (32 * SB_WARPS), lo = t * per < nb ? t * per : nb, hi = lo + per < nb ? lo + per : nb;
+    unsigned int s = 0u;
+    for (int i = lo; i < hi; ++i) s += totals[i];
+    unsigned int incl = s;
+    for (int o = 1; o < 32; o <<= 1) { const unsigned int x = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += x; }
+    if (lane == 31) wsum[wl] = incl;
+    __syncthreads();
+    unsigned int run = incl - s;
+    for (int u = 0; u < wl; ++u) run += wsum[u];
+    for (int i = lo; i < hi; ++i) { base[i] = run; run += totals[i]; }
+    __syncthreads();
+  }
+  if (wg >= nwarps) return;
+  for (int i = lane; i < nb; i += 32) pos[wl][i] = base[i] + hist[(size_t)i * nwarps + wg];
+  __syncwarp();
+  for (int it = 0; it < SB_RUN / 32; ++it) {
+    const long long e = (long long)wg * SB_RUN + it * 32 + lane;
+    const int key = e < a.n ? (int)keys[e] : nb;
+    const unsigned int peers = __match_any_sync(0xffffffffu, key), before = __popc(peers & ((1u << lane) - 1u));
+    unsigned int dst = 0u;
+    if (key < nb) dst = pos[wl][key] + before;
+    __syncwarp();                                            // every peer has read pos[] by now
+    if (key < nb && before == 0u) pos[wl][key] += __popc(peers);
+    __syncwarp();
+    long long lo, ro, relid;
+    if (key < nb && sub_bucket_offsets(a, e, lo, ro, relid, errflag)) {
+      lhs_out[dst] = lo % a.lsize[relid];
+      rhs_out[dst] = ro % a.rsize[relid];
+      rel_out[dst] = a.rel[e];
+    }
+  }
+}
+
+// The general form: keys and edge numbers through the radix sort.
 __global__ void sub_bucket_keys_kernel(SubBucketArgs a, unsigned long long *keys, unsigned int *vals, int *errflag) {
   long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= a.n) return;
@@ -108,22 +304,37 @@ int launch_reverse_permutation(const long long *perm, long long n, long long *ou
   return n > 0;
 }
 
+template <class T>
+static void shuffle_as(const void *in, void *out, long long rows, long long row_bytes, const long long *perm, int *errflag, cudaStream_t st) {
+  const int units = (int)(row_bytes / (long long)sizeof(T));
+  int G = 1;
+  while (G < 256 && 4 * G < units) G *= 2;
+  shuffle_rows_kernel<T><<<grid_for(rows, 256 / G), 256, 0, st>>>((const T *)in, (T *)out, rows, units, G, perm, errflag);
+}
+
 int launch_shuffle_rows(const void *in, void *out, long long rows, long long row_bytes, const long long *perm, int *errflag, cudaStream_t st) {
   if (rows <= 0 || row_bytes <= 0) return 0;
   const uintptr_t al = (uintptr_t)in | (uintptr_t)out | (uintptr_t)row_bytes;
-  if (al % 16 == 0) {
-    long long u = row_bytes / 16;
-    shuffle_rows_kernel<uint4><<<grid_for(rows * u, 256), 256, 0, st>>>((const uint4 *)in, (uint4 *)out, rows, u, perm, errflag);
-  } else if (al % 8 == 0) {
-    long long u = row_bytes / 8;
-    shuffle_rows_kernel<unsigned long long><<<grid_for(rows * u, 256), 256, 0, st>>>((const unsigned long long *)in, (unsigned long long *)out, rows, u, perm, errflag);
-  } else if (al % 4 == 0) {
-    long long u = row_bytes / 4;
-    shuffle_rows_kernel<unsigned int><<<grid_for(rows * u, 256), 256, 0, st>>>((const unsigned int *)in, (unsigned int *)out, rows, u, perm, errflag);
-  } else {
-    shuffle_rows_kernel<unsigned char><<<grid_for(rows * row_bytes, 256), 256, 0, st>>>((const unsigned char *)in, (unsigned char *)out, rows, row_bytes, perm, errflag);
-  }
+  if (al % 16 == 0) shuffle_as<uint4>(in, out, rows, row_bytes, perm, errflag, st);
+  else if (al % 8 == 0) shuffle_as<unsigned long long>(in, out, rows, row_bytes, perm, errflag, st);
+  else if (al % 4 == 0) shuffle_as<unsigned int>(in, out, rows, row_bytes, perm, errflag, st);
+  else shuffle_as<unsigned char>(in, out, rows, row_bytes, perm, errflag, st);
   return 1;
+}
+
+// scratch of the two-kernel randperm (0: n is too large for it): counters, which start at zero, then the buckets
+size_t pbg_randperm_bytes(long long n) {
+  if (n > RP_MAX) return 0;
+  return 2 * RP_MAX_BUCKETS * 4 + ((size_t)RP_CAP * 8 << rp_bits(n));
+}
+int launch_randperm_dealt(char *mem, unsigned turn, long long n, unsigned long long seed, long long *out, int *errflag, cudaStream_t st) {
+  const int bits = rp_bits(n), index_bits = rp_index_bits(n);
+  unsigned int *counts = (unsigned int *)mem;
+  unsigned int *cur = counts + (turn & 1) * RP_MAX_BUCKETS, *next = counts + ((turn + 1) & 1) * RP_MAX_BUCKETS;
+  unsigned long long *buckets = (unsigned long long *)(mem + 2 * RP_MAX_BUCKETS * 4);
+  randperm_deal_kernel<<<grid_for(n, 2048), 256, 0, st>>>(n, seed, bits, index_bits, buckets, cur, next, errflag);
+  randperm_sort_kernel<<<1 << bits, 1024, 0, st>>>(buckets, cur, index_bits, out);
+  return 2;
 }
 
 int launch_randperm(SortPlan &sp, long long n, unsigned long long seed, long long *out, cudaStream_t st) {
@@ -134,21 +345,35 @@ int launch_randperm(SortPlan &sp, long long n, unsigned long long seed, long lon
   return launches + 1;
 }
 
-int launch_sub_bucket(SortPlan &sp, const long long *lhs, const long long *rhs, const long long *rel, long long n, int R,
-                      const long long *tables_dev, int nl, int nr, int dynamic, long long *lhs_out, long long *rhs_out,
-                      long long *rel_out, long long *counts_dev, int *errflag, cudaStream_t st) {
+// tables: [6 R] in host memory; tables_dev: where they lie on the device when R is above SB_INLINE (pbg_sub_bucket_inline)
+bool pbg_sub_bucket_inline(int R) { return R <= SB_INLINE; }
+int launch_sub_bucket(SortPlan &sp, const long long *lhs, const long long *rhs, const long long *rel, long long n, int R, const long long *tables,
+                      const long long *tables_dev, int nl, int nr, int dynamic, long long *lhs_out, long long *rhs_out, long long *rel_out,
+                      long long *counts, int *errflag, cudaStream_t st) {
   SubBucketArgs a;
   a.lhs = lhs; a.rhs = rhs; a.rel = rel; a.n = n; a.R = R; a.nl = nl; a.nr = nr; a.dynamic = dynamic;
   a.lperm = (const long long *const *)tables_dev;
   a.rperm = (const long long *const *)(tables_dev + R);
   a.lcount = tables_dev + 2 * R; a.rcount = tables_dev + 3 * R; a.lsize = tables_dev + 4 * R; a.rsize = tables_dev + 5 * R;
   const int nb = nl * nr;
-  if (n <= 0) { cudaMemsetAsync(counts_dev, 0, (size_t)nb * sizeof(long long), st); return 0; }
+  if (n <= 0) return 0;
+  if (nb < SB_BINS) {
+    SubBucketTables in;
+    const bool inl = pbg_sub_bucket_inline(R);
+    for (int i = 0; i < 6 * SB_INLINE; ++i) in.v[i] = inl && i < 6 * R ? tables[i] : 0;
+    const int nwarps = (int)((n + SB_RUN - 1) / SB_RUN), ctas = (nwarps + SB_WARPS - 1) / SB_WARPS;
+    unsigned short *keys = (unsigned short *)sp.keys[0];
+    unsigned int *totals = sp.hist + (size_t)(nb + 1) * nwarps;
+    sub_bucket_hist<<<ctas, 32 * SB_WARPS, 0, st>>>(a, in, inl ? nullptr : tables_dev, keys, sp.hist, nwarps, errflag);
+    sub_bucket_scan<<<nb + 1, 256, 0, st>>>(sp.hist, nwarps, nb, totals, counts);
+    sub_bucket_scatter<<<ctas, 32 * SB_WARPS, 0, st>>>(a, in, inl ? nullptr : tables_dev, keys, sp.hist, totals, nwarps, lhs_out, rhs_out, rel_out, errflag);
+    return 3;
+  }
   sub_bucket_keys_kernel<<<grid_for(n, 256), 256, 0, st>>>(a, sp.keys[0], sp.vals[0], errflag);
   int bits = 1;
   while ((1ll << bits) <= nb) ++bits;                                   // keys run up to nb (the "cannot be placed" key)
   int launches = 1 + pbg_sort(sp, (int)n, bits, st);
   sub_bucket_emit_kernel<<<grid_for(n, 256), 256, 0, st>>>(a, sp.keys[sp.result], sp.vals[sp.result], lhs_out, rhs_out, rel_out, errflag);
-  sub_bucket_counts_kernel<<<grid_for(nb, 128), 128, 0, st>>>(sp.keys[sp.result], n, nb, counts_dev);
+  sub_bucket_counts_kernel<<<grid_for(nb, 128), 128, 0, st>>>(sp.keys[sp.result], n, nb, counts);
   return launches + 2;
 }

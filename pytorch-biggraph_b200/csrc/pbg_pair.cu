@@ -46,13 +46,20 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-template <int NPL>
+// NARROW: score rows of at most 128 columns.  The accumulators of a block are then two of 128 columns, of which tensor
+// memory holds two sets: the products of the next block run beside the epilogue of this one.  And the two halves of a row
+// (two column groups of 64) leave eight of the sixteen epilogue warps without work, so the other eight take the second
+// problem at the same time.  (With one set and both problems on the same warps, 280 blocks of 50 edges and 100 columns took
+// 47 us on 148 SMs, two blocks one after the other on each.)
+template <int NPL, bool NARROW>
 // (18 warps are allocated as 20: 96 registers per thread is what fits, which is what ptxas settles on)
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d, WaveBatches wb, WaveBufs w) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) unsigned long long bars[2 * PAIR_SMAX + 2];
+  constexpr int SETS = NARROW ? 2 : 1;
+  constexpr uint32_t ACC = NARROW ? 128u : 256u;                         // columns of one accumulator
+  __shared__ __align__(8) unsigned long long bars[2 * PAIR_SMAX + 4];
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int failed;
   __shared__ volatile int epi_go;
@@ -63,13 +70,15 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
   const uint32_t bar0 = smem_u32(&bars[0]);
   auto full_bar = [&](int s) { return bar0 + 8u * s; };                  // TMA landed
   auto empty_bar = [&](int s) { return bar0 + 8u * (PAIR_SMAX + s); };   // MMAs have read the stage
-  const uint32_t accf_bar = bar0 + 8u * (2 * PAIR_SMAX);                 // both accumulators complete
-  const uint32_t acce_bar = bar0 + 8u * (2 * PAIR_SMAX + 1);             // both accumulators drained
+  auto accf_bar = [&](int a) { return bar0 + 8u * (2 * PAIR_SMAX + a); };        // both accumulators of set a complete
+  auto acce_bar = [&](int a) { return bar0 + 8u * (2 * PAIR_SMAX + 2 + a); };    // both accumulators of set a drained
   int *errflag = w.errflag;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2 * PAIR_SMAX; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar0 + 8u * i));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(accf_bar));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 512;" :: "r"(acce_bar));
+    for (int a = 0; a < SETS; ++a) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(accf_bar(a)));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 512;" :: "r"(acce_bar(a)));
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     failed = 0;
   }
@@ -123,7 +132,9 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
     long long git = 0, j = 0;
     for (int t = blockIdx.x; t < d.nblk && !failed; t += gridDim.x) {
       if (!tile_live(t)) continue;
-      if (j >= 1 && !mbar_wait(acce_bar, (uint32_t)(j - 1) & 1, errflag)) { failed = 1; break; }
+      const int set = (int)(j % SETS);
+      const uint32_t tset = tmem + (uint32_t)set * 2u * ACC;
+      if (j >= SETS && !mbar_wait(acce_bar(set), (uint32_t)(j / SETS - 1) & 1, errflag)) { failed = 1; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       bool ok = true;
       for (int kb = 0; kb < nkb; ++kb, ++git) {
@@ -146,14 +157,14 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
               const uint64_t da = smem_desc(st + aarr * arr_bytes + pa[tt] * plane_bytes + k16 * 32, 0, 512, 4);
               const uint64_t db = smem_desc(st + barr * arr_bytes + pb[tt] * plane_bytes + k16 * 32, 0, 512, 4);
               asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-                           :: "r"(tmem + (uint32_t)p * 256u), "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
+                           :: "r"(tset + (uint32_t)p * ACC), "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
             }
           }
         }
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(empty_bar(s)) : "memory");
       }
       if (!ok) break;
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(accf_bar) : "memory");
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(accf_bar(set)) : "memory");
       ++j;
     }
   } else if (warp >= 2) {
@@ -164,9 +175,20 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
     // that every score costs one exponential and no more than 32 values are ever held in registers.
     long long j = 0;
     const int q = warp & 3;                            // the 32 tensor-memory lanes this warp may read
-    const int cg = (warp - 2) >> 2;                    // column group: chunks 2 cg and 2 cg + 1
+    const int wg = (warp - 2) >> 2;
+    const int cg = NARROW ? wg & 1 : wg;               // column group: chunks 2 cg and 2 cg + 1
+    const int p0 = NARROW ? wg >> 1 : 0, p1 = NARROW ? p0 + 1 : 2;       // the problems of this warp
     const int i = q * 32 + lane;                       // positive row of the chunk
     const int Mm = d.Mm, Pm = d.Pm;
+    // a row's sums over its column groups (the narrow form has two of them)
+    auto groups_f = [&](int what, int p, int i) {
+      const float s = red_f[what][p][0][i] + red_f[what][p][1][i];
+      return NARROW ? s : s + (red_f[what][p][2][i] + red_f[what][p][3][i]);
+    };
+    auto groups_i = [&](int p, int i) {
+      const int s = red_i[p][0][i] + red_i[p][1][i];
+      return NARROW ? s : s + red_i[p][2][i] + red_i[p][3][i];
+    };
     auto epi_sync = [] { asm volatile("bar.sync 1, 512;" ::: "memory"); };     // the sixteen epilogue warps
     for (int t = blockIdx.x; t < d.nblk; t += gridDim.x) {
       if (!tile_live(t)) continue;
@@ -174,7 +196,7 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
       // One thread waits for the accumulators (a bounded wait) and tells the others through shared memory: all
       // sixteen warps take the same decision, so that none is left alone at the named barrier further down.
       if (warp == 2 && lane == 0) {
-        bool go = failed == 0 && mbar_wait(accf_bar, (uint32_t)j & 1, errflag);
+        bool go = failed == 0 && mbar_wait(accf_bar((int)(j % SETS)), (uint32_t)(j / SETS) & 1, errflag);
         if (!go) failed = 1;
         epi_go = go ? 1 : 0;
       }
@@ -186,12 +208,12 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
       const size_t prow = (size_t)blk * Pm + (i < Pm ? i : 0);
       const float wr = row_valid ? wb.wrel[bi.b] * (w.ew ? w.ew[bi.e0 + i] : 1.0f) : 0.f;   // relation weight x edge weight
 #pragma unroll 1
-      for (int p = 0; p < 2; ++p) {
+      for (int p = p0; p < p1; ++p) {
         const int enabled = d.neg_enabled[p];
         const int Mlog = !enabled ? 0 : (d.batch_negs ? bi.Pl + d.U : d.U);   // columns of the reference's score matrix
         const float s = row_valid ? w.spos[p][prow] : 0.f;
         const int col0 = cg * 64;                                // first column of this warp's part of the row
-        const uint32_t trow = tmem + (uint32_t)p * 256u + ((uint32_t)(q * 32) << 16) + (uint32_t)col0;
+        const uint32_t trow = tmem + (uint32_t)(j % SETS) * 2u * ACC + (uint32_t)p * ACC + ((uint32_t)(q * 32) << 16) + (uint32_t)col0;
         const int nch = col0 >= w.Kb ? 0 : (col0 + 32 >= w.Kb ? 1 : 2);      // chunks of this warp that hold coefficient columns
         // Which columns of this warp's chunks count for this row (model.py:566-580): bit jj of live[c] is set when
         // column col0 + 32 c + jj exists (< Mm) and is not ignored -- uniform negatives (>= Pm) never are; a batch
@@ -232,8 +254,9 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
           red_f[0][p][cg][i] = mx;
           red_i[p][cg][i] = viol;
           epi_sync();
-          mx = fmaxf(fmaxf(red_f[0][p][0][i], red_f[0][p][1][i]), fmaxf(red_f[0][p][2][i], red_f[0][p][3][i]));
-          viol = red_i[p][0][i] + red_i[p][1][i] + red_i[p][2][i] + red_i[p][3][i];
+          mx = fmaxf(red_f[0][p][0][i], red_f[0][p][1][i]);
+          if (!NARROW) mx = fmaxf(mx, fmaxf(red_f[0][p][2][i], red_f[0][p][3][i]));
+          viol = groups_i(p, i);
           float m = fmaxf(mx, s);
           if (mx == -INFINITY) m = fmaxf(s, PBG_MASKED);         // every column masked
           float z = 0.f;
@@ -251,7 +274,7 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
           }
           red_f[1][p][cg][i] = z;
           epi_sync();
-          z = (red_f[1][p][0][i] + red_f[1][p][1][i]) + (red_f[1][p][2][i] + red_f[1][p][3][i]);
+          z = groups_f(1, p, i);
           const float es = expf(s - m), Z = z + es;
           if (Mlog > 0) { lossv = -s + m + logf(Z); ds = es / Z - 1.0f; scale = wr / Z; }
           else viol = 0;                                          // losses.py:139-140: no negatives, loss 0, no gradient
@@ -276,9 +299,9 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
           }
           red_f[0][p][cg][i] = lossv; red_f[1][p][cg][i] = ds; red_i[p][cg][i] = viol;
           epi_sync();
-          lossv = (red_f[0][p][0][i] + red_f[0][p][1][i]) + (red_f[0][p][2][i] + red_f[0][p][3][i]);
-          ds = (red_f[1][p][0][i] + red_f[1][p][1][i]) + (red_f[1][p][2][i] + red_f[1][p][3][i]);
-          viol = red_i[p][0][i] + red_i[p][1][i] + red_i[p][2][i] + red_i[p][3][i];
+          lossv = groups_f(0, p, i);
+          ds = groups_f(1, p, i);
+          viol = groups_i(p, i);
           scale = wr;
         } else {
           // softplus(-s) + (1/M) sum_j softplus(S_ij), M counts masked columns (losses.py:61-80); the scores are replaced by sigmoid(S)
@@ -298,8 +321,8 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
           }
           red_f[0][p][cg][i] = lossv; red_i[p][cg][i] = viol;
           epi_sync();
-          lossv = ((red_f[0][p][0][i] + red_f[0][p][1][i]) + (red_f[0][p][2][i] + red_f[0][p][3][i])) * nw + pair_softplus(-s);
-          viol = red_i[p][0][i] + red_i[p][1][i] + red_i[p][2][i] + red_i[p][3][i];
+          lossv = groups_f(0, p, i) * nw + pair_softplus(-s);
+          viol = groups_i(p, i);
           ds = -pair_sigmoid(-s);
           scale = wr * nw;
         }
@@ -338,7 +361,7 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(acce_bar) : "memory");
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(acce_bar((int)(j % SETS))) : "memory");
       ++j;
     }
   }
@@ -390,13 +413,9 @@ int launch_pair_score(const WaveDims &d, const WaveBatches &wb, const WaveBufs &
   const dim3 grid((unsigned)(d.nblk < sms ? d.nblk : sms));
   const size_t smem = (size_t)pl->geom.nst * pl->geom.stage_bytes + 1024;
   // the opt-in covers the largest stage ring this kernel is ever launched with (227 KB less its static shared memory)
-  if (pl->npl == 3) {
-    pbg_opt_in_smem((const void *)pair_score_kernel<3>, PAIR_SMEM_MAX);
-    pbg_launch(pair_score_kernel<3>, grid, PAIR_THREADS, smem, st, pl->maps, pl->geom, d, wb, w);
-  } else {
-    pbg_opt_in_smem((const void *)pair_score_kernel<2>, PAIR_SMEM_MAX);
-    pbg_launch(pair_score_kernel<2>, grid, PAIR_THREADS, smem, st, pl->maps, pl->geom, d, wb, w);
-  }
-  pbg_note_launch();
+  auto kernel = pl->npl == 3 ? (d.Mm <= 128 ? pair_score_kernel<3, true> : pair_score_kernel<3, false>)
+                             : (d.Mm <= 128 ? pair_score_kernel<2, true> : pair_score_kernel<2, false>);
+  pbg_opt_in_smem((const void *)kernel, PAIR_SMEM_MAX);
+  pbg_launch(kernel, grid, PAIR_THREADS, smem, st, pl->maps, pl->geom, d, wb, w);
   return 1;
 }

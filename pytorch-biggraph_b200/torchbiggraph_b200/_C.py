@@ -35,12 +35,15 @@ def _ctx(device: torch.device) -> C.c_void_p:
 
 
 def _p(t: torch.Tensor):
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def _sync_torch(device):
-    # the library works on the legacy default stream of its context; order it after PyTorch's current stream
-    torch.cuda.current_stream(device).synchronize()
+    # the library works on the legacy default stream of its context: PyTorch's own default stream is the same one,
+    # any other current stream is waited for
+    s = torch.cuda.current_stream(device)
+    if s.cuda_stream != 0:
+        s.synchronize()
 
 
 def randperm(num_items: int, num_threads: int = 1, seed: int = -1, device="cuda") -> torch.Tensor:
