@@ -416,6 +416,7 @@ static int bind_bucket(pbg_context *c, const pbg_bucket *bk, WaveDims &d, WaveBu
   d.op = cfg.op; d.cmp = cfg.comparator; d.loss = cfg.loss; d.dynamic = cfg.dynamic_relations != 0;
   d.batch_negs = cfg.num_batch_negs > 0;
   d.neg_enabled[0] = !cfg.disable_lhs_negs; d.neg_enabled[1] = !cfg.disable_rhs_negs;
+  d.byMm = FastDiv(c->Mm); d.byPm = FastDiv(c->Pm); d.byCm = FastDiv(c->Cm); d.bySpb = FastDiv(c->spb);
   d.num_batch_negs = cfg.num_batch_negs; d.spb = c->spb; d.margin = cfg.margin; d.reg_coef = cfg.regularization_coef; d.max_norm = cfg.max_norm > 0.f ? cfg.max_norm : 0.f;
   d.matrix_op = cfg.op == PBG_OP_LINEAR || cfg.op == PBG_OP_AFFINE;
   d.opw = d.matrix_op ? cfg.dim * cfg.dim + (cfg.op == PBG_OP_AFFINE ? cfg.dim : 0) : cfg.dim;
@@ -656,7 +657,8 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
       const unsigned int *wvals = cluster ? c->wvals[grp & 1][in_grp] : sp.vals[sp.result];
       t.done(launch_update(d, wb, w, wkeys, wvals, c->cfg.lr, c->cfg.relation_lr, us, c->stream));
     }
-    if (wave == nwaves - 1 || group_of(wave + 1) != grp) CU(c, cudaEventRecord(c->ev_updated[grp & 1], c->stream));
+    // (the next call's sorts come behind everything of this one)
+    if (grp + 2 < ngroups && group_of(wave + 1) != grp) CU(c, cudaEventRecord(c->ev_updated[grp & 1], c->stream));
     b0 += kk;
   }
   c->batches_done += (unsigned long long)num_batches;

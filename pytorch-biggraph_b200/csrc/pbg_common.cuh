@@ -36,10 +36,29 @@
 
 enum { ARR_N0 = 0, ARR_N1 = 1, ARR_Q0 = 2, ARR_Q1 = 3, ARR_R0 = 4, ARR_R1 = 5 };
 
+// Division of slot and block numbers (below 2^31) by a size that is fixed for the launch: one high multiply and a shift
+// instead of the twenty-odd instructions of an integer division.  With l = ceil(log2 d) and m = ceil(2^(31 + l) / d),
+// n / d = floor(n m / 2^(31 + l)): m exceeds the exact quotient by less than 1, so the product exceeds n / d by less
+// than n / 2^(31 + l) < 1 / d.  Kernels of a few hundred instructions per row of 100 floats spend a quarter of them on five
+// such divisions.
+struct FastDiv {
+  unsigned m;
+  int s;                // l - 1; -1: division by 1
+  FastDiv() = default;
+  explicit FastDiv(int d) {
+    int l = 0;
+    while ((1ll << l) < d) ++l;
+    s = l - 1;
+    m = l == 0 ? 0u : (unsigned)(((1ull << (31 + l)) + (unsigned)d - 1) / (unsigned)d);
+  }
+  __device__ __forceinline__ int div(int n) const { return s < 0 ? n : (int)(__umulhi((unsigned)n, m) >> s); }
+};
+
 struct WaveDims {
   int D, Dp;            // dim, workspace row stride (floats)
   int Pm, U, Mm, Ms;    // chunk slots, uniform negatives, Pm+U, score row stride
   int Cm;               // chunks per batch (max)
+  FastDiv byMm, byPm, byCm, bySpb;
   int k, nblk;          // batches in this wave; chunk blocks THIS LAUNCH covers (k*Cm for a whole wave)
   int blk0;             // first chunk block of this launch (a wave may be launched in two parts)
   int op, cmp, loss, dynamic;
@@ -118,7 +137,7 @@ struct BlockInfo { int b, c, Pl, n; long long e0; };
 // edges) (model.py:648-656) and how many of its Pm slots hold real edges.
 __device__ __forceinline__ BlockInfo block_info(const WaveDims &d, const WaveBatches &wb, int blk) {
   BlockInfo bi;
-  bi.b = blk / d.Cm;
+  bi.b = d.byCm.div(blk);
   bi.c = blk - bi.b * d.Cm;
   int nb = wb.n[bi.b];
   int lim = d.batch_negs ? d.num_batch_negs : d.U;
@@ -167,18 +186,18 @@ __device__ __forceinline__ long long slot_row(const WaveDims &d, const WaveBatch
 struct Occ { int b, a, blk, r; };
 __device__ __forceinline__ Occ occ_decode(const WaveDims &d, int o) {
   Occ q;
-  q.b = o / d.spb;
+  q.b = d.bySpb.div(o);
   int w = o - q.b * d.spb;
   int nN = d.Cm * d.Mm, nQ = d.dynamic ? d.Cm * d.Pm : 0;   // standard relations: N slots only
-  int rows;
-  if (w < nN) { q.a = ARR_N0; rows = d.Mm; }
-  else if ((w -= nN) < nN) { q.a = ARR_N1; rows = d.Mm; }
-  else if ((w -= nN) < nQ) { q.a = ARR_Q0; rows = d.Pm; }
-  else if ((w -= nQ) < nQ) { q.a = ARR_Q1; rows = d.Pm; }
-  else if ((w -= nQ) < nQ) { q.a = ARR_R0; rows = d.Pm; }
-  else { w -= nQ; q.a = ARR_R1; rows = d.Pm; }
-  int c = w / rows;
-  q.r = w - c * rows;
+  bool whole = false;                                      // rows of Mm slots (N arrays) or of Pm
+  if (w < nN) { q.a = ARR_N0; whole = true; }
+  else if ((w -= nN) < nN) { q.a = ARR_N1; whole = true; }
+  else if ((w -= nN) < nQ) q.a = ARR_Q0;
+  else if ((w -= nQ) < nQ) q.a = ARR_Q1;
+  else if ((w -= nQ) < nQ) q.a = ARR_R0;
+  else { w -= nQ; q.a = ARR_R1; }
+  int c = whole ? d.byMm.div(w) : d.byPm.div(w);
+  q.r = w - c * (whole ? d.Mm : d.Pm);
   q.blk = q.b * d.Cm + c;
   return q;
 }

@@ -47,8 +47,8 @@ __device__ __forceinline__ unsigned long long randperm_hash(unsigned long long s
   return pbg_mix64(seed ^ pbg_mix64((unsigned long long)i + 0x51ED270B0F1ull)) >> 20;
 }
 
-// Up to RP_MAX indices in two kernels: the hash is uniform, so its top bits deal the indices to buckets of about 1,000 to
-// 2,000, which a CTA sorts in shared memory.  A bucket has room for RP_CAP; one that overflows (a thousand standard
+// Up to RP_MAX indices in two kernels: the hash is uniform, so its top bits deal the indices to buckets of 350 to 700 (of up
+// to 2,048 beyond 1.4 million indices), which a CTA sorts in shared memory.  A bucket has room for RP_CAP; one that overflows (a thousand standard
 // deviations away) raises the error word's bit 8 and the caller takes the general sort.  Keys in a bucket: the remaining
 // hash bits above the index (55 bits together), one comparison for both.  (Four radix passes of three launches took 260 us for
 // 269,507 indices.)
@@ -56,7 +56,7 @@ __device__ __forceinline__ unsigned long long randperm_hash(unsigned long long s
 #define RP_MAX (1ll << 22)
 #define RP_MAX_BUCKETS 2048
 static int rp_index_bits(long long n) { int b = 1; while ((n - 1) >> b) ++b; return b; }
-static int rp_bits(long long n) { int b = 0; while ((n >> b) > 2048 && (1 << b) < RP_MAX_BUCKETS) ++b; return b; }
+static int rp_bits(long long n) { int b = 0; while ((n >> b) > 700 && (1 << b) < RP_MAX_BUCKETS) ++b; return b; }
 
 __global__ void __launch_bounds__(256) randperm_deal_kernel(long long n, unsigned long long seed, int bits, int index_bits, unsigned long long *buckets, unsigned int *count,
                                                             unsigned int *count_next, int *errflag) {
@@ -86,34 +86,38 @@ __global__ void __launch_bounds__(256) randperm_deal_kernel(long long n, unsigne
   }
 }
 
-// one CTA per bucket: bitonic sort of its keys (padded to a power of two), indices out behind the smaller buckets'
-__global__ void __launch_bounds__(1024) randperm_sort_kernel(const unsigned long long *__restrict__ buckets, const unsigned int *__restrict__ count,
-                                                             int index_bits, long long *__restrict__ out) {
+// one CTA per bucket: bitonic sort of its keys (padded to a power of two), indices out behind the smaller buckets'.  Pairs at
+// a distance of 32 and less lie inside one warp's 64 keys: between two such steps the warp waits for itself only.
+#define RP_SORT_THREADS 512
+__global__ void __launch_bounds__(RP_SORT_THREADS) randperm_sort_kernel(const unsigned long long *__restrict__ buckets, const unsigned int *__restrict__ count,
+                                                                        int index_bits, long long *__restrict__ out) {
   __shared__ unsigned long long key[RP_CAP];
-  __shared__ unsigned int below[32];
+  __shared__ unsigned int below[RP_SORT_THREADS / 32];
   const int t = threadIdx.x, b = blockIdx.x;
   const int n = count[b] < RP_CAP ? (int)count[b] : RP_CAP;
   unsigned int s = 0u;
-  for (int i = t; i < b; i += 1024) s += count[i];
+  for (int i = t; i < b; i += RP_SORT_THREADS) s += count[i];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if ((t & 31) == 0) below[t >> 5] = s;
-  int size = 2;
+  int size = 64;
   while (size < n) size <<= 1;
-  for (int i = t; i < size; i += 1024) key[i] = i < n ? buckets[(size_t)b * RP_CAP + i] : ~0ull;
+  for (int i = t; i < size; i += RP_SORT_THREADS) key[i] = i < n ? buckets[(size_t)b * RP_CAP + i] : ~0ull;
   __syncthreads();
   for (int k = 2; k <= size; k <<= 1)
     for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int p = t; p < size / 2; p += 1024) {
-        const int lo = (p / j) * 2 * j + p % j, hi = lo + j;
+      for (int p = t; p < size / 2; p += RP_SORT_THREADS) {
+        const int lo = ((p & ~(j - 1)) << 1) | (p & (j - 1)), hi = lo + j;
         const unsigned long long x = key[lo], y = key[hi];
         if ((x > y) == ((lo & k) == 0)) { key[lo] = y; key[hi] = x; }
       }
-      __syncthreads();
+      const int next = j > 1 ? j >> 1 : k;                    // distance of the step that follows
+      if (j > 32 || next > 32) __syncthreads(); else __syncwarp();
     }
+  __syncthreads();
   unsigned int base = 0u;
-  for (int u = 0; u < 32; ++u) base += below[u];
-  for (int i = t; i < n; i += 1024) out[base + i] = (long long)(key[i] & ((1ull << index_bits) - 1ull));
+  for (int u = 0; u < RP_SORT_THREADS / 32; ++u) base += below[u];
+  for (int i = t; i < n; i += RP_SORT_THREADS) out[base + i] = (long long)(key[i] & ((1ull << index_bits) - 1ull));
 }
 
 // the general form, any length: keys for the radix sort
@@ -163,25 +167,25 @@ __device__ __forceinline__ bool sub_bucket_offsets(const SubBucketArgs &a, long 
 }
 
 // Up to SB_BINS - 1 sub-buckets (127 x 127 need more): stable counting sort in three launches that carry the edges along --
-//   sub_bucket_hist     every warp owns a run of SB_RUN consecutive edges, keeps their keys and counts them into
-//                       hist[key][warp]
+//   sub_bucket_hist     every warp owns a run of consecutive edges, keeps their keys and counts them into hist[key][warp]
 //   sub_bucket_scan     one CTA per key: exclusive scan of its row of warp counts; the row's total is the sub-bucket's size
 //   sub_bucket_scatter  every warp walks its run in order and writes each edge's offsets to its place
 // (Keys, a radix pass over (key, index) pairs, a gather and binary searches for the sizes were six launches.)
-#define SB_RUN 256
+// Runs are 64 edges up to 255 sub-buckets (an edge is a chain of three dependent reads, and a run walks its 32-edge rows
+// one after the other), 256 above (the table of counts grows with both).
+static inline int sb_run(int nb) { return nb < 256 ? 64 : 256; }
 #define SB_WARPS 4
 #define SB_BINS 1024
 __global__ void __launch_bounds__(32 * SB_WARPS) sub_bucket_hist(SubBucketArgs args, const __grid_constant__ SubBucketTables in, const long long *in_dev, unsigned short *keys,
-                                                                 unsigned int *hist, int nwarps, int *errflag) {
+                                                                 unsigned int *hist, int nwarps, int run, int *errflag) {
   __shared__ unsigned int cnt[SB_WARPS][SB_BINS];
   const SubBucketArgs a = sub_bucket_bind(args, in, in_dev);
   const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31, wg = blockIdx.x * SB_WARPS + wl, nb = a.nl * a.nr;
   if (wg >= nwarps) return;
   for (int i = lane; i <= nb; i += 32) cnt[wl][i] = 0u;
   __syncwarp();
-#pragma unroll
-  for (int it = 0; it < SB_RUN / 32; ++it) {
-    const long long e = (long long)wg * SB_RUN + it * 32 + lane;
+  for (int it = 0; it < run / 32; ++it) {
+    const long long e = (long long)wg * run + it * 32 + lane;
     int key = nb;                                            // edges that cannot be placed come last
     if (e < a.n) {
       long long lo, ro, relid;
@@ -194,12 +198,12 @@ __global__ void __launch_bounds__(32 * SB_WARPS) sub_bucket_hist(SubBucketArgs a
   for (int i = lane; i <= nb; i += 32) hist[(size_t)i * nwarps + wg] = cnt[wl][i];
 }
 
-__global__ void __launch_bounds__(256) sub_bucket_scan(unsigned int *hist, int nwarps, int nb, unsigned int *totals, long long *counts) {
-  __shared__ unsigned int part[8];
+__global__ void __launch_bounds__(1024) sub_bucket_scan(unsigned int *hist, int nwarps, int nb, unsigned int *totals, long long *counts) {
+  __shared__ unsigned int part[32];
   unsigned int *row = hist + (size_t)blockIdx.x * nwarps;
   const int t = threadIdx.x, lane = t & 31, wl = t >> 5;
   unsigned int carry = 0u;
-  for (int i0 = 0; i0 < nwarps; i0 += 256) {
+  for (int i0 = 0; i0 < nwarps; i0 += 1024) {
     const int i = i0 + t;
     const unsigned int v = i < nwarps ? row[i] : 0u;
     unsigned int incl = v;
@@ -207,7 +211,7 @@ __global__ void __launch_bounds__(256) sub_bucket_scan(unsigned int *hist, int n
     if (lane == 31) part[wl] = incl;
     __syncthreads();
     unsigned int before = carry, all = carry;
-    for (int u = 0; u < 8; ++u) { if (u < wl) before += part[u]; all += part[u]; }
+    for (int u = 0; u < 32; ++u) { if (u < wl) before += part[u]; all += part[u]; }
     if (i < nwarps) row[i] = before + incl - v;
     carry = all;
     __syncthreads();
@@ -220,7 +224,7 @@ __global__ void __launch_bounds__(256) sub_bucket_scan(unsigned int *hist, int n
 
 __global__ void __launch_bounds__(32 * SB_WARPS) sub_bucket_scatter(SubBucketArgs args, const __grid_constant__ SubBucketTables in, const long long *in_dev,
                                                                     const unsigned short *__restrict__ keys, const unsigned int *__restrict__ hist,
-                                                                    const unsigned int *__restrict__ totals, int nwarps, long long *lhs_out, long long *rhs_out,
+                                                                    const unsigned int *__restrict__ totals, int nwarps, int run, long long *lhs_out, long long *rhs_out,
                                                                     long long *rel_out, int *errflag) {
   __shared__ unsigned int base[SB_BINS], pos[SB_WARPS][SB_BINS];
   __shared__ unsigned int wsum[SB_WARPS];
@@ -235,16 +239,16 @@ __global__ void __launch_bounds__(32 * SB_WARPS) sub_bucket_scatter(SubBucketArg
     for (int o = 1; o < 32; o <<= 1) { const unsigned int x = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += x; }
     if (lane == 31) wsum[wl] = incl;
     __syncthreads();
-    unsigned int run = incl - s;
-    for (int u = 0; u < wl; ++u) run += wsum[u];
-    for (int i = lo; i < hi; ++i) { base[i] = run; run += totals[i]; }
+    unsigned int at = incl - s;
+    for (int u = 0; u < wl; ++u) at += wsum[u];
+    for (int i = lo; i < hi; ++i) { base[i] = at; at += totals[i]; }
     __syncthreads();
   }
   if (wg >= nwarps) return;
   for (int i = lane; i < nb; i += 32) pos[wl][i] = base[i] + hist[(size_t)i * nwarps + wg];
   __syncwarp();
-  for (int it = 0; it < SB_RUN / 32; ++it) {
-    const long long e = (long long)wg * SB_RUN + it * 32 + lane;
+  for (int it = 0; it < run / 32; ++it) {
+    const long long e = (long long)wg * run + it * 32 + lane;
     const int key = e < a.n ? (int)keys[e] : nb;
     const unsigned int peers = __match_any_sync(0xffffffffu, key), before = __popc(peers & ((1u << lane) - 1u));
     unsigned int dst = 0u;
@@ -333,7 +337,7 @@ int launch_randperm_dealt(char *mem, unsigned turn, long long n, unsigned long l
   unsigned int *cur = counts + (turn & 1) * RP_MAX_BUCKETS, *next = counts + ((turn + 1) & 1) * RP_MAX_BUCKETS;
   unsigned long long *buckets = (unsigned long long *)(mem + 2 * RP_MAX_BUCKETS * 4);
   randperm_deal_kernel<<<grid_for(n, 2048), 256, 0, st>>>(n, seed, bits, index_bits, buckets, cur, next, errflag);
-  randperm_sort_kernel<<<1 << bits, 1024, 0, st>>>(buckets, cur, index_bits, out);
+  randperm_sort_kernel<<<1 << bits, RP_SORT_THREADS, 0, st>>>(buckets, cur, index_bits, out);
   return 2;
 }
 
@@ -361,12 +365,12 @@ int launch_sub_bucket(SortPlan &sp, const long long *lhs, const long long *rhs, 
     SubBucketTables in;
     const bool inl = pbg_sub_bucket_inline(R);
     for (int i = 0; i < 6 * SB_INLINE; ++i) in.v[i] = inl && i < 6 * R ? tables[i] : 0;
-    const int nwarps = (int)((n + SB_RUN - 1) / SB_RUN), ctas = (nwarps + SB_WARPS - 1) / SB_WARPS;
+    const int run = sb_run(nb), nwarps = (int)((n + run - 1) / run), ctas = (nwarps + SB_WARPS - 1) / SB_WARPS;
     unsigned short *keys = (unsigned short *)sp.keys[0];
     unsigned int *totals = sp.hist + (size_t)(nb + 1) * nwarps;
-    sub_bucket_hist<<<ctas, 32 * SB_WARPS, 0, st>>>(a, in, inl ? nullptr : tables_dev, keys, sp.hist, nwarps, errflag);
-    sub_bucket_scan<<<nb + 1, 256, 0, st>>>(sp.hist, nwarps, nb, totals, counts);
-    sub_bucket_scatter<<<ctas, 32 * SB_WARPS, 0, st>>>(a, in, inl ? nullptr : tables_dev, keys, sp.hist, totals, nwarps, lhs_out, rhs_out, rel_out, errflag);
+    sub_bucket_hist<<<ctas, 32 * SB_WARPS, 0, st>>>(a, in, inl ? nullptr : tables_dev, keys, sp.hist, nwarps, run, errflag);
+    sub_bucket_scan<<<nb + 1, 1024, 0, st>>>(sp.hist, nwarps, nb, totals, counts);
+    sub_bucket_scatter<<<ctas, 32 * SB_WARPS, 0, st>>>(a, in, inl ? nullptr : tables_dev, keys, sp.hist, totals, nwarps, run, lhs_out, rhs_out, rel_out, errflag);
     return 3;
   }
   sub_bucket_keys_kernel<<<grid_for(n, 256), 256, 0, st>>>(a, sp.keys[0], sp.vals[0], errflag);

@@ -157,9 +157,9 @@ template <int VEC, bool PL>
 __global__ void __launch_bounds__(32 * GATHER_WARPS, VEC >= 8 ? 2 : 3) gather_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   pdl_begin();
   int lane = threadIdx.x & 31;
-  long long item = (long long)blockIdx.x * GATHER_WARPS + (threadIdx.x >> 5);
-  if (item >= (long long)d.nblk * d.Mm) return;
-  int lb = (int)(item / d.Mm), r = (int)(item - (long long)lb * d.Mm);
+  const int item = (int)blockIdx.x * GATHER_WARPS + (int)(threadIdx.x >> 5);
+  if (item >= d.nblk * d.Mm) return;
+  const int lb = d.byMm.div(item), r = item - lb * d.Mm;
   const int blk = d.blk0 + lb;
   BlockInfo bi = block_info(d, wb, blk);
   const int D = d.D;
@@ -203,6 +203,17 @@ __global__ void __launch_bounds__(32 * GATHER_WARPS, VEC >= 8 ? 2 : 3) gather_ke
     }
     const float *xl = w.W[0] + (size_t)il * D, *xr = w.W[1] + (size_t)ir * D;
     const float *th0 = (d.op != PBG_OP_NONE && w.theta[0]) ? w.theta[0] + (size_t)rl * D : nullptr;
+    // Up to 256 floats the rhs row is requested with the lhs row, before anything is written (behind the writes of the lhs
+    // row it waited for them); wider rows leave no registers for it.
+    constexpr bool EARLY = VEC <= 2;
+    float4 xe[EARLY ? VEC : 1];
+    if constexpr (EARLY) load_row<VEC>(xe, xr, D, lane);
+    auto rhs_row = [&] {
+      if constexpr (EARLY) {
+#pragma unroll
+        for (int c = 0; c < VEC; ++c) x[c] = xe[c];
+      } else load_row<VEC>(x, xr, D, lane);
+    };
     // lhs row without operator -> N0
     load_row<VEC>(x, xl, D, lane);
     const float scl = renorm_row<VEC>(x, d.max_norm);
@@ -215,14 +226,14 @@ __global__ void __launch_bounds__(32 * GATHER_WARPS, VEC >= 8 ? 2 : 3) gather_ke
     if (d.matrix_op) {
       // linear / affine: the raw rhs row goes to R1; operator, prepare and the positive score
       // follow in the contraction and postop_kernel
-      load_row<VEC>(x, xr, D, lane);
+      rhs_row();
       renorm_row<VEC>(x, d.max_norm);
       add_global<VEC>(x, w.glob[1], D, lane);
       store_row<VEC>(w.R1 + noff, x, D, lane);
       if (lane == 0) w.aux[ARR_N0][nrow] = a0;
     } else if (!d.dynamic) {
       // rhs row through the operator -> N1; one positive score shared by both problems
-      load_row<VEC>(x, xr, D, lane);
+      rhs_row();
       const float scr = renorm_row<VEC>(x, d.max_norm);
       if (d.max_norm > 0.f && lane == 0) w.rscale[nrow] = scr;
       add_global<VEC>(x, w.glob[1], D, lane);
@@ -243,7 +254,7 @@ __global__ void __launch_bounds__(32 * GATHER_WARPS, VEC >= 8 ? 2 : 3) gather_ke
       put_row<VEC>(w.X[ARR_Q1], qoff, z, D, lane);
       if (PL) put_row_planes<VEC>(w, ARR_Q1, blk, r, z, D, lane);
       // rhs row without operator -> N1
-      load_row<VEC>(x, xr, D, lane);
+      rhs_row();
       const float scr = renorm_row<VEC>(x, d.max_norm);
 #pragma unroll
       for (int c = 0; c < VEC; ++c) y1[c] = x[c];
@@ -266,10 +277,16 @@ __global__ void __launch_bounds__(32 * GATHER_WARPS, VEC >= 8 ? 2 : 3) gather_ke
     return;
   }
   // ---- a uniformly drawn negative row, one per side ------------------------------------------
+  // (both rows are requested before the first is written, as above)
+  constexpr bool BOTH = VEC <= 2;
+  const long long ids[2] = {slot_row(d, wb, w, bi, 0, r), slot_row(d, wb, w, bi, 1, r)};
+  float4 xb[BOTH ? VEC : 1];
+  if constexpr (BOTH)
+    if (ids[1] >= 0 && ids[1] < d.n_rows[1]) load_row<VEC>(xb, w.W[1] + (size_t)ids[1] * D, D, lane);
 #pragma unroll
   for (int side = 0; side < 2; ++side) {
     float *dst = side == 0 ? n0 : n1;
-    long long id = slot_row(d, wb, w, bi, side, r);
+    long long id = ids[side];
     if (id >= d.n_rows[side]) { if (lane == 0) atomicOr(w.errflag, 1); id = -1; }
     if (id < 0) {
       zero_row<VEC>(dst, D, lane);
@@ -279,7 +296,10 @@ __global__ void __launch_bounds__(32 * GATHER_WARPS, VEC >= 8 ? 2 : 3) gather_ke
       continue;
     }
     const float *xrow = w.W[side] + (size_t)id * D;
-    load_row<VEC>(x, xrow, D, lane);
+    if (BOTH && side == 1) {
+#pragma unroll
+      for (int c = 0; c < VEC; ++c) x[c] = xb[BOTH ? c : 0];
+    } else load_row<VEC>(x, xrow, D, lane);
     const float scu = renorm_row<VEC>(x, d.max_norm);
     if (side == 1 && d.max_norm > 0.f && lane == 0) w.rscale[nrow] = scu;
     add_global<VEC>(x, w.glob[side], D, lane);
@@ -306,9 +326,9 @@ template <int VEC, bool PL>
 __global__ void __launch_bounds__(32 * GATHER_WARPS, VEC >= 16 ? 1 : VEC >= 8 ? 3 : 4) gather_plain_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   pdl_begin();
   int lane = threadIdx.x & 31;
-  long long item = (long long)blockIdx.x * GATHER_WARPS + (threadIdx.x >> 5);
-  if (item >= (long long)d.nblk * d.Mm) return;
-  int lb = (int)(item / d.Mm), r = (int)(item - (long long)lb * d.Mm);
+  const int item = (int)blockIdx.x * GATHER_WARPS + (int)(threadIdx.x >> 5);
+  if (item >= d.nblk * d.Mm) return;
+  const int lb = d.byMm.div(item), r = item - lb * d.Mm;
   const int blk = d.blk0 + lb;
   BlockInfo bi = block_info(d, wb, blk);
   const int D = d.D;
@@ -386,9 +406,9 @@ template <int VEC>
 __global__ void __launch_bounds__(32 * GATHER_WARPS) postop_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   pdl_begin();
   int lane = threadIdx.x & 31;
-  long long item = (long long)blockIdx.x * GATHER_WARPS + (threadIdx.x >> 5);
-  if (item >= (long long)d.nblk * d.Mm) return;
-  int lb = (int)(item / d.Mm), r = (int)(item - (long long)lb * d.Mm);
+  const int item = (int)blockIdx.x * GATHER_WARPS + (int)(threadIdx.x >> 5);
+  if (item >= d.nblk * d.Mm) return;
+  const int lb = d.byMm.div(item), r = item - lb * d.Mm;
   const int blk = d.blk0 + lb;
   BlockInfo bi = block_info(d, wb, blk);
   const int D = d.D;

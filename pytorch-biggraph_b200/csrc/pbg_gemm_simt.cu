@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(256) gemm_tile_kernel(GemmTasks tasks, WaveDim
   const GemmTask &t = tasks.t[p];
   if (t.M <= 0) return;
   const float *A = t.A + (size_t)blk * t.a_blk, *B = t.B + (size_t)blk * t.b_blk;
-  if (t.b_rel) B += (size_t)wb.rel[blk / d.Cm] * t.b_rel;
+  if (t.b_rel) B += (size_t)wb.rel[d.byCm.div(blk)] * t.b_rel;
   float *C = t.C + (size_t)blk * t.c_blk;
   const int M = t.M, N = t.N, K = t.K;
   int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
@@ -269,7 +269,7 @@ int launch_matrix_backward(const WaveDims &d, const WaveBatches &wb, const WaveB
   launch_tiles<true, false, false>(ts, d, wb, st);
   // per batch: treat the Cm chunk blocks of a batch as one block of Cm*Mm rows
   WaveDims db = d;
-  db.Cm = 1; db.blk0 = d.blk0 / d.Cm; db.nblk = d.nblk / d.Cm;
+  db.Cm = 1; db.byCm = FastDiv(1); db.blk0 = d.blk0 / d.Cm; db.nblk = d.nblk / d.Cm;
   long long bstride = (long long)d.Cm * d.Mm * d.Dp;
   matrix_task(ts, w.GX[ARR_N1], bstride, d.Dp, w.R1, bstride, d.Dp, 0, w.dA, d.opw, d.D, d.D, d.D, d.Cm * d.Mm);
   launch_tiles<false, false, false>(ts, db, wb, st);

@@ -342,6 +342,9 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         const int ncol0 = n0 + c0;
         if (mrow0 >= g.M || ncol0 >= g.N) continue;    // block entirely outside the matrix (warp-uniform)
+        // l2 family: |b|^2 of the block's 32 columns, one per lane, handed round by shuffles below (read column by column
+        // between the writes into the staging buffer, each read waited for the write before it: half of the kernel)
+        const float bl = l2 && ncol0 + lane < g.N ? bn[ncol0 + lane] : 0.f;
         // the buffer used two blocks ago must have been read by its store before it is rewritten
         if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
         __syncwarp();
@@ -361,8 +364,7 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
           for (int tt = 0; tt < 4; ++tt) {
             v[tt] = __uint_as_float(r[jj + tt]);
             if (l2) {
-              int n = ncol0 + jj + tt;
-              float qv = ((n < g.N ? bn[n] : 0.f) - 2.0f * v[tt]) + an;     // model.py:226-246
+              float qv = (__shfl_sync(0xffffffffu, bl, jj + tt) - 2.0f * v[tt]) + an;     // model.py:226-246
               v[tt] = g.cmp == PBG_CMP_L2 ? -sqrtf(fmaxf(qv, 1e-30f)) : -qv;
             }
           }

@@ -42,12 +42,11 @@ template <int NV>
 __global__ void __launch_bounds__(32 * LOSS_WARPS) loss_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   pdl_begin();
   int lane = threadIdx.x & 31;
-  long long item = (long long)blockIdx.x * LOSS_WARPS + (threadIdx.x >> 5);
-  long long per_prob = (long long)d.nblk * d.Pm;
+  const int item = (int)blockIdx.x * LOSS_WARPS + (int)(threadIdx.x >> 5);
+  const int per_prob = d.nblk * d.Pm;
   if (item >= 2 * per_prob) return;
-  int p = (int)(item / per_prob);
-  long long rem = item - p * per_prob;
-  int lb = (int)(rem / d.Pm), i = (int)(rem - (long long)lb * d.Pm);
+  const int p = item >= per_prob ? 1 : 0, rem = item - p * per_prob;
+  const int lb = d.byPm.div(rem), i = rem - lb * d.Pm;
   const int blk = d.blk0 + lb;
   BlockInfo bi = block_info(d, wb, blk);
   if (bi.n == 0) return;
@@ -201,12 +200,11 @@ template <int NV>
 __global__ void __launch_bounds__(32 * LOSS_WARPS) coef_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   pdl_begin();
   int lane = threadIdx.x & 31;
-  long long item = (long long)blockIdx.x * LOSS_WARPS + (threadIdx.x >> 5);
-  long long per_side = (long long)d.nblk * d.Mm;
+  const int item = (int)blockIdx.x * LOSS_WARPS + (int)(threadIdx.x >> 5);
+  const int per_side = d.nblk * d.Mm;
   if (item >= 2 * per_side) return;
-  int side = (int)(item / per_side);
-  long long rem = item - side * per_side;
-  int lb = (int)(rem / d.Mm), m = (int)(rem - (long long)lb * d.Mm);
+  const int side = item >= per_side ? 1 : 0, rem = item - side * per_side;
+  const int lb = d.byMm.div(rem), m = rem - lb * d.Mm;
   const int blk = d.blk0 + lb;
   BlockInfo bi = block_info(d, wb, blk);
   if (bi.n == 0) return;
@@ -252,12 +250,11 @@ template <int NV>
 __global__ void __launch_bounds__(32 * LOSS_WARPS) loss_softmax_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   pdl_begin();
   int lane = threadIdx.x & 31;
-  long long item = (long long)blockIdx.x * LOSS_WARPS + (threadIdx.x >> 5);
-  long long per_prob = (long long)d.nblk * d.Pm;
+  const int item = (int)blockIdx.x * LOSS_WARPS + (int)(threadIdx.x >> 5);
+  const int per_prob = d.nblk * d.Pm;
   if (item >= 2 * per_prob) return;
-  int p = (int)(item / per_prob);
-  long long rem = item - p * per_prob;
-  int lb = (int)(rem / d.Pm), i = (int)(rem - (long long)lb * d.Pm);
+  const int p = item >= per_prob ? 1 : 0, rem = item - p * per_prob;
+  const int lb = d.byPm.div(rem), i = rem - lb * d.Pm;
   const int blk = d.blk0 + lb;
   BlockInfo bi = block_info(d, wb, blk);
   if (bi.n == 0) return;
@@ -350,13 +347,13 @@ template <bool PL>
 __global__ void __launch_bounds__(32 * LOSS_WARPS) coef_tile_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   pdl_begin();
   int lane = threadIdx.x & 31;
-  long long item = (long long)blockIdx.x * LOSS_WARPS + (threadIdx.x >> 5);
+  const int item = (int)blockIdx.x * LOSS_WARPS + (int)(threadIdx.x >> 5);
   const int tiles = (d.Mm + 31) / 32;
-  long long per_side = (long long)d.nblk * tiles * tiles;
+  const long long per_side = (long long)d.nblk * tiles * tiles;
   if (item >= 2 * per_side) return;
-  int side = (int)(item / per_side);
-  long long rem = item - side * per_side;
-  int lb = (int)(rem / (tiles * tiles)), tt = (int)(rem - (long long)lb * tiles * tiles);
+  const int side = item >= per_side ? 1 : 0;
+  const unsigned rem = (unsigned)(item - side * per_side);
+  int lb = (int)(rem / (unsigned)(tiles * tiles)), tt = (int)(rem - (unsigned)lb * tiles * tiles);
   int m0 = (tt / tiles) * 32, j0 = (tt % tiles) * 32;
   const int blk = d.blk0 + lb;
   BlockInfo bi = block_info(d, wb, blk);
@@ -466,9 +463,9 @@ int launch_loss(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cud
 __global__ void __launch_bounds__(32 * LOSS_WARPS) reg_value_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   pdl_begin();
   int lane = threadIdx.x & 31;
-  long long item = (long long)blockIdx.x * LOSS_WARPS + (threadIdx.x >> 5);
-  if (item >= (long long)d.nblk * d.Pm) return;
-  int lb = (int)(item / d.Pm), i = (int)(item - (long long)lb * d.Pm);
+  const int item = (int)blockIdx.x * LOSS_WARPS + (int)(threadIdx.x >> 5);
+  if (item >= d.nblk * d.Pm) return;
+  const int lb = d.byPm.div(item), i = item - lb * d.Pm;
   const int blk = d.blk0 + lb;
   BlockInfo bi = block_info(d, wb, blk);
   if (bi.n == 0) return;
@@ -553,11 +550,11 @@ __global__ void __launch_bounds__(32 * LOSS_WARPS) eval_rows_kernel(WaveDims d, 
   __shared__ double sm[LOSS_WARPS][8];
   __shared__ bool closing;
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  const long long item = (long long)blockIdx.x * LOSS_WARPS + wl, per_prob = (long long)d.nblk * d.Pm;
+  const int item = (int)blockIdx.x * LOSS_WARPS + wl, per_prob = d.nblk * d.Pm;
   double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   const int p = item >= per_prob ? 1 : 0;
-  const long long rem = item - p * per_prob;
-  const int blk = (int)(rem / d.Pm), i = (int)(rem - (long long)blk * d.Pm);
+  const int rem = item - p * per_prob;
+  const int blk = d.byPm.div(rem), i = rem - blk * d.Pm;
   if (item < 2 * per_prob) {
     const BlockInfo bi = block_info(d, wb, blk);
     if (i < bi.n) {

@@ -116,9 +116,9 @@ __global__ void __launch_bounds__(32 * UPD_WARPS) std_pullback_kernel(WaveDims d
   extern __shared__ __align__(16) float wpart[];             // [UPD_WARPS][VEC * 128]
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int side = side0 + blockIdx.y, a = side ? ARR_N1 : ARR_N0;
-  const long long item = (long long)blockIdx.x * UPD_WARPS + wl;
-  if (item >= (long long)d.nblk * d.Mm) return;
-  const int lb = (int)(item / d.Mm), r = (int)(item - (long long)lb * d.Mm), blk = d.blk0 + lb;
+  const int item = (int)blockIdx.x * UPD_WARPS + wl;
+  if (item >= d.nblk * d.Mm) return;
+  const int lb = d.byMm.div(item), r = item - lb * d.Mm, blk = d.blk0 + lb;
   if (side == 1 && d.matrix_op) return;                      // linear / affine: R2 holds the gradient of the raw row already
   const BlockInfo bi = block_info(d, wb, blk);
   if (bi.n <= 0) return;
@@ -415,7 +415,7 @@ tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
   unsigned long long kA = pa >= 0 ? keys[pa] : SENT;
   unsigned long long kB = pb < d.nocc ? keys[pb] : SENT;
   unsigned int vB = pb < d.nocc ? vals[pb] : 0u;
-  const int bB = (int)(vB / (unsigned int)d.spb);              // batch of this lane's slot
+  const int bB = d.bySpb.div((int)vB);              // batch of this lane's slot
   if (__shfl_sync(FULL, kB, TILE - 1) < lo) return;          // tile holds only the other rule's rows
   // Copies the gradient rows of window slots j0 .. j0+cnt-1 (cnt <= STAGE) into the stage buffers and
   // waits for them; the wait is bounded (bit 1 of the error word when it runs out).
@@ -592,7 +592,7 @@ __device__ __forceinline__ void batch_stats(const WaveDims &d, const WaveBatches
   const int lim = d.batch_negs ? d.num_batch_negs : d.U, nb = wb.n[b], Pl = nb < lim ? nb : lim;
 #pragma unroll 4
   for (int r = t; r < rows; r += blockDim.x) {
-    const int c = r / d.Pm, i = r - c * d.Pm;
+    const int c = d.byPm.div(r), i = r - c * d.Pm;
     if (i >= Pl || c * Pl + i >= nb) continue;
     const size_t prow = (size_t)b * rows + r;
     l += (double)w.lossrow[0][prow] + (double)w.lossrow[1][prow];
@@ -674,8 +674,8 @@ hub_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__r
       const long long end = coop_prefix_end(head + HUB_BIG, (long long)d.nocc, [&](long long pos) { return keys[pos] == key; });
       // where batch b starts and ends inside the row.  (Both searches in the same rounds, half of the CTA each, measured
       // slower: 14.2 against 11.8 us.)
-      const long long q = coop_prefix_end(head, end, [&](long long pos) { return (int)(vals[pos] / (unsigned int)d.spb) < b; });
-      const long long eb = coop_prefix_end(q, end, [&](long long pos) { return (int)(vals[pos] / (unsigned int)d.spb) <= b; });
+      const long long q = coop_prefix_end(head, end, [&](long long pos) { return d.bySpb.div((int)vals[pos]) < b; });
+      const long long eb = coop_prefix_end(q, end, [&](long long pos) { return d.bySpb.div((int)vals[pos]) <= b; });
       const long long ftb = (q / TILE + 1) * TILE;
       const long long nruns = q < eb ? 1 + (eb > ftb ? (eb - 1 - ftb) / TILE + 1 : 0) : 0;
       if (nruns > 1) {
@@ -727,7 +727,7 @@ hub_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__r
     }
     const long long p = head + threadIdx.x;
     const unsigned long long kp = p < (long long)d.nocc ? keys[p] : ~0ull;
-    const int bp = p < (long long)d.nocc ? (int)(vals[p] / (unsigned int)d.spb) : -1;
+    const int bp = p < (long long)d.nocc ? d.bySpb.div((int)vals[p]) : -1;
     // what the CTAs of a big row's batches left (past L1: this CTA may have read the lines before)
     const long long tabv = from_big && threadIdx.x <= PBG_KMAX ? __ldcg(line + threadIdx.x) : -1;
     if (threadIdx.x == 0) skey = kp;
@@ -865,9 +865,9 @@ template <int VEC, int CK>
 __global__ void __launch_bounds__(32 * UPD_WARPS) gz_rows_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   pdl_begin();
   int lane = threadIdx.x & 31;
-  long long item = (long long)blockIdx.x * UPD_WARPS + (threadIdx.x >> 5);
-  if (item >= (long long)d.nblk * d.Mm) return;
-  int lb = (int)(item / d.Mm), r = (int)(item - (long long)lb * d.Mm);
+  const int item = (int)blockIdx.x * UPD_WARPS + (int)(threadIdx.x >> 5);
+  if (item >= d.nblk * d.Mm) return;
+  const int lb = d.byMm.div(item), r = item - lb * d.Mm;
   const int blk = d.blk0 + lb;
   BlockInfo bi = block_info(d, wb, blk);
   const int D = d.D;
@@ -950,15 +950,15 @@ __global__ void __launch_bounds__(32 * UPD_WARPS, VEC <= 4 ? 4 : 1) dyn_pullback
   pdl_begin();
   extern __shared__ __align__(16) float wpart[];             // [UPD_WARPS][VEC * 128]
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  const long long nN = (long long)d.nblk * d.Mm, nQ = (long long)d.nblk * d.Pm;
-  long long item = (long long)blockIdx.x * UPD_WARPS + wl + (first_q ? 2 * nN : 0);
+  const int nN = d.nblk * d.Mm, nQ = d.nblk * d.Pm;
+  int item = (int)blockIdx.x * UPD_WARPS + wl + (first_q ? 2 * nN : 0);
   if (item >= 2 * nN + 2 * nQ) return;
-  int a, rows;
-  if (item < nN) { a = ARR_N0; rows = d.Mm; }
-  else if ((item -= nN) < nN) { a = ARR_N1; rows = d.Mm; }
-  else if ((item -= nN) < nQ) { a = ARR_Q0; rows = d.Pm; }
-  else { item -= nQ; a = ARR_Q1; rows = d.Pm; }
-  const int lb = (int)(item / rows), r = (int)(item - (long long)lb * rows);
+  int a;
+  if (item < nN) a = ARR_N0;
+  else if ((item -= nN) < nN) a = ARR_N1;
+  else if ((item -= nN) < nQ) a = ARR_Q0;
+  else { item -= nQ; a = ARR_Q1; }
+  const int rows = a <= ARR_N1 ? d.Mm : d.Pm, lb = a <= ARR_N1 ? d.byMm.div(item) : d.byPm.div(item), r = item - lb * rows;
   const int blk = d.blk0 + lb, D = d.D;
   BlockInfo bi = block_info(d, wb, blk);
   if (bi.n <= 0) return;
