@@ -118,8 +118,11 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
   pdl_begin();                                               // barriers and tensor memory are set up beside the kernel before this one
   const int nkb = (g.K + KB - 1) / KB;
   const int b_atoms = PLANES ? (g.BN + 63) / 64 : (g.BN + 31) / 32;     // MN-major boxes per B tile (per plane)
-  const uint32_t b_plane = B_MN ? (uint32_t)b_atoms * BOX_BYTES : (uint32_t)g.BN * ROW_BYTES;   // bytes of one B tile (plane)
-  const uint32_t b_used = PLANES ? (uint32_t)NPL * b_plane : b_plane;
+  const uint32_t b_tile = B_MN ? (uint32_t)b_atoms * BOX_BYTES : (uint32_t)g.BN * ROW_BYTES;    // bytes of one B tile (of one plane)
+  const uint32_t b_used = PLANES ? (uint32_t)NPL * b_tile : b_tile;
+  // planes: distance between the planes of an operand; MN-major ones lie as [column block][plane][32 k][64 columns]
+  constexpr uint32_t a_plane = A_MN ? BOX_BYTES : A_PLANE, MN_STRIDE = NPL * BOX_BYTES;
+  const uint32_t b_plane = B_MN ? BOX_BYTES : b_tile;
   const uint32_t stage_tx = A_BYTES + b_used;
   const bool dual = PLANES && A_MN && B_MN && g.dual != 0;
   const int nkb1 = dual ? (g.K1 + KB - 1) / KB : 0;                    // k-blocks that carry B1
@@ -138,11 +141,7 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
   };
 
   if (warp == 0) {
-    // ---------------- TMA producer (whole warp: every box of a stage is issued by its own lane) ----------------
-    // Issuing one cp.async.bulk.tensor costs the issuing thread a few hundred cycles; an MN-major
-    // B tile is up to eight 32 x 32 boxes, which issued from one lane made the producer the
-    // longest link of the stage's chain.
-    const int a_boxes = PLANES ? (A_MN ? 2 * NPL : NPL) : (A_MN ? 4 : 1), b_boxes = PLANES ? NPL * (B_MN ? b_atoms : 1) : (B_MN ? b_atoms : 1);
+    // ---------------- TMA producer (one box per operand, each from its own lane) ----------------
     long long git = 0;
     bool stop = false;
     for (long long t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
@@ -162,25 +161,14 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
         unsigned char *st = smem + (size_t)s * stage_bytes;
         int k0 = kb * KB;
         uint32_t dA = smem_u32(st), dB = smem_u32(st + A_BYTES);
-        if (PLANES) {
-          if (lane < a_boxes) {
-            if (!A_MN) tma_load_4d(dA + lane * A_PLANE, &maps.a[p], k0, m0, lane, blk, fb);
-            else { int pl = lane >> 1, mb = lane & 1; tma_load_4d(dA + pl * A_PLANE + mb * BOX_BYTES, &maps.a[p], m0 + mb * 64, k0, pl, blk, fb); }
-          } else if (lane < a_boxes + b_boxes) {
-            int ib = lane - a_boxes;
-            if (!B_MN) tma_load_4d(dB + ib * b_plane, &maps.b[p], k0, n0, ib, blk, fb);
-            else if (with_b1) { int pl = ib / b_atoms, nb = ib - pl * b_atoms; tma_load_4d(dB + pl * b_plane + nb * BOX_BYTES, &maps.b[p], n0 + nb * 64, k0, pl, blk, fb); }
-          } else if (dual && lane < a_boxes + b_boxes + NPL) {
-            int ib = lane - a_boxes - b_boxes;
-            tma_load_4d(dB + b_used + ib * b2_plane, &maps.b2[p], k0, 0, ib, blk, fb);
-          }
-        } else if (lane < a_boxes) {
-          if (!A_MN) tma_load_3d(dA, &maps.a[p], k0, m0, blk, fb);
-          else tma_load_3d(dA + lane * BOX_BYTES, &maps.a[p], m0 + lane * 32, k0, blk, fb);
-        } else if (lane < a_boxes + b_boxes) {
-          int nb = lane - a_boxes;
-          if (!B_MN) tma_load_3d(dB, &maps.b[p], k0, n0, blk, fb);
-          else tma_load_3d(dB + nb * BOX_BYTES, &maps.b[p], n0 + nb * 32, k0, blk, fb);
+        if (lane == 0) {
+          if (PLANES) { if (A_MN) tma_load_5d(dA, &maps.a[p], 0, k0, 0, m0 / 64, blk, fb); else tma_load_4d(dA, &maps.a[p], k0, m0, 0, blk, fb); }
+          else { if (A_MN) tma_load_4d(dA, &maps.a[p], 0, k0, m0 / 32, blk, fb); else tma_load_3d(dA, &maps.a[p], k0, m0, blk, fb); }
+        } else if (lane == 1) {
+          if (PLANES) { if (!B_MN) tma_load_4d(dB, &maps.b[p], k0, n0, 0, blk, fb); else if (with_b1) tma_load_5d(dB, &maps.b[p], 0, k0, 0, n0 / 64, blk, fb); }
+          else { if (B_MN) tma_load_4d(dB, &maps.b[p], 0, k0, n0 / 32, blk, fb); else tma_load_3d(dB, &maps.b[p], k0, n0, blk, fb); }
+        } else if (dual && lane == 2) {
+          tma_load_4d(dB + b_used, &maps.b2[p], k0, 0, 0, blk, fb);
         }
       }
     }
@@ -188,9 +176,8 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
     // ---------------- MMA issuer ----------------
     // instruction descriptor: D fp32, A/B tf32, operand majors, N >> 3, M >> 4
     const uint32_t fmt = PLANES ? 1u : 2u;            // operand format: bf16 (kind::f16) or tf32
-    const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((A_MN ? 1u : 0u) << 15) | ((B_MN ? 1u : 0u) << 16) |
-                           ((uint32_t)(g.BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-    const uint32_t idesc2 = (idesc & ~((0x3Fu << 17) | (1u << 16))) | ((uint32_t)(g.BN2 >> 3) << 17);   // dual: the B2 products are K-major, BN2 columns wide
+    const uint32_t idesc0 = (1u << 4) | (fmt << 7) | (fmt << 10) | ((A_MN ? 1u : 0u) << 15) | ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(128 >> 4) << 24);
+    const uint32_t idesc2 = (idesc0 & ~(1u << 16)) | ((uint32_t)(g.BN2 >> 3) << 17);   // dual: the B2 products are K-major, BN2 columns wide
     long long git = 0, j = 0;
     for (long long t = blockIdx.x; t < ntiles && !failed; t += gridDim.x) {
       int p, blk, m0, n0;
@@ -199,6 +186,8 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
       if (j >= 2 && !mbar_wait(acce_bar(ab), (uint32_t)((j >> 1) - 1) & 1, errflag)) { failed = 1; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tacc = tmem + (uint32_t)ab * 256u;
+      const int ncols = g.N - n0 < g.BN ? (g.N - n0 + 15) / 16 * 16 : g.BN;                 // columns of this tile that exist
+      const uint32_t idesc = idesc0 | ((uint32_t)(ncols >> 3) << 17);
       bool ok = true;
       for (int kb = 0; kb < nkb; ++kb, ++git) {
         int s = (int)(git % STAGES);
@@ -221,9 +210,9 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
             if (k16 * 16 >= kleft) break;                     // the tail of K: those k-values are zero fill
 #pragma unroll
             for (int t = T0; t < 6; ++t) {
-              uint64_t da = A_MN ? smem_desc(aH + pa[t] * A_PLANE + k16 * 2048, BOX_BYTES, 1024, 2)
-                                 : smem_desc(aH + pa[t] * A_PLANE + k16 * 32, 0, 512, 4);
-              uint64_t db = B_MN ? smem_desc(bH + pb[t] * b_plane + k16 * 2048, BOX_BYTES, 1024, 2)
+              uint64_t da = A_MN ? smem_desc(aH + pa[t] * a_plane + k16 * 2048, MN_STRIDE, 1024, 2)
+                                 : smem_desc(aH + pa[t] * a_plane + k16 * 32, 0, 512, 4);
+              uint64_t db = B_MN ? smem_desc(bH + pb[t] * b_plane + k16 * 2048, MN_STRIDE, 1024, 2)
                                  : smem_desc(bH + pb[t] * b_plane + k16 * 32, 0, 512, 4);
               uint32_t acc = (kb > 0 || k16 > 0 || t > T0) ? 1u : 0u;
               if (dual && k16 * 16 >= kleft1) continue;       // past K1: no B1 product for these k-values
@@ -236,7 +225,7 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
               // which initialises all BN columns
 #pragma unroll
               for (int t = T0; t < 6; ++t) {
-                uint64_t da = smem_desc(aH + pa[t] * A_PLANE + k16 * 2048, BOX_BYTES, 1024, 2);
+                uint64_t da = smem_desc(aH + pa[t] * a_plane + k16 * 2048, MN_STRIDE, 1024, 2);
                 uint64_t db = smem_desc(bH + b_used + pb[t] * b2_plane + k16 * 32, 0, 512, 4);
                 asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
                              :: "r"(tacc), "l"(da), "l"(db), "r"(idesc2), "r"(1u) : "memory");
@@ -410,9 +399,11 @@ struct TcPlan {
 // Columns per tile: equal tiles of at most 256.  With more than one tile the width is a multiple of
 // 32, the width of the epilogue's store blocks (a block must not reach into the next tile); a single
 // tile may end on a multiple of 16, what lies beyond it is outside the matrix and clipped.
-static int tile_cols(int n) {
+// With an MN-major B operand it is a multiple of the operand's column blocks (`atom`: 32 floats, 64 bf16 values); the last
+// tile multiplies only the columns that are left.
+static int tile_cols(int n, int atom = 32) {
   int tiles = (n + 255) / 256;
-  int unit = tiles > 1 ? 32 : 16;
+  int unit = tiles > 1 ? atom : 16;
   int bn = ((n + tiles - 1) / tiles + unit - 1) / unit * unit;
   return bn > 256 ? 256 : bn;
 }
@@ -425,43 +416,42 @@ void *pbg_tc_plan_create(const WaveDims &d, const WaveBufs &w, int nblk_max, int
   pl->dynamic = d.dynamic != 0;
   pl->nterms = precision == PBG_PREC_TF32X3 ? 3 : precision == PBG_PREC_BF16X6 ? 6 : precision == PBG_PREC_BF16X3 ? 2 : 1;
   pl->bn_score = tile_cols(d.Mm);
-  pl->bn_grad = tile_cols(d.D);
+  const bool planes = pl->nterms == 6 || pl->nterms == 2;
+  pl->bn_grad = tile_cols(d.D, planes ? 64 : 32);
+  const int score_atoms = (pl->bn_score + (planes ? 63 : 31)) / (planes ? 64 : 32), grad_atoms = (pl->bn_grad + (planes ? 63 : 31)) / (planes ? 64 : 32);
   bool ok = true;
-  if (pl->nterms == 6 || pl->nterms == 2) {
+  if (planes) {
     const int npl = w.npl;
     // bf16-plane tiers: the same products on the plane arrays (K-major boxes {32 k, rows}, MN-major boxes {64, 32 k})
     for (int p = 0; p < 2; ++p) {
       int q = ARR_Q0 + p, n = ARR_N0 + p;
-      ok &= encode4_planes(&pl->score.a[p], w.XB[q], npl, d.D, d.Pm, w.xrows[q], nblk_max, w.Dpb, 32, 128);
-      ok &= encode4_planes(&pl->score.b[p], w.XB[n], npl, d.D, w.xrows[n], w.xrows[n], nblk_max, w.Dpb, 32, pl->bn_score);
-      ok &= encode3(&pl->score.c[p], w.S[p], d.Mm, d.Pm, nblk_max, d.Ms, (long long)d.Pm * d.Ms, 32, 32, false);
+      ok &= encode4_planes(&pl->score.a[p], w.XB[q], npl, d.D, d.Pm, w.xrows[q], nblk_max, w.Dpb, 128);
+      ok &= encode4_planes(&pl->score.b[p], w.XB[n], npl, d.D, w.xrows[n], w.xrows[n], nblk_max, w.Dpb, pl->bn_score);
+      ok &= encode3(&pl->score.c[p], w.S[p], d.Mm, d.Pm, nblk_max, d.Ms, (long long)d.Pm * d.Ms, 32, 32);
       if (pl->dynamic) {
         // grad Q: A = T (K-major, k = Mm), B = N (MN-major); grad N: A = T^T (MN-major: k rows = Pm), B = Q (MN-major)
-        ok &= encode4_planes(&pl->gradq.a[p], w.TB[p], npl, d.Mm, d.Pm, d.Pm, nblk_max, w.Kb, 32, 128);
-        ok &= encode4_planes(&pl->gradq.b[p], w.XB[n], npl, d.D, w.xrows[n], w.xrows[n], nblk_max, w.Dpb, 64, 32);
-        ok &= encode4_planes(&pl->gradn.a[p], w.TB[p], npl, d.Mm, d.Pm, d.Pm, nblk_max, w.Kb, 64, 32);
-        ok &= encode4_planes(&pl->gradn.b[p], w.XB[q], npl, d.D, w.xrows[q], w.xrows[q], nblk_max, w.Dpb, 64, 32);
-        ok &= encode3(&pl->gradq.c[p], w.GX[q], d.D, d.Pm, nblk_max, d.Dp, (long long)w.grows[q] * d.Dp, 32, 32, false);
-        ok &= encode3(&pl->gradn.c[p], w.GX[n], d.D, d.Mm, nblk_max, d.Dp, (long long)w.grows[n] * d.Dp, 32, 32, false);
+        ok &= encode4_planes(&pl->gradq.a[p], w.TB[p], npl, d.Mm, d.Pm, d.Pm, nblk_max, w.Kb, 128);
+        ok &= encode4_planes_mn(&pl->gradq.b[p], w.XB[n], npl, d.D, w.xrows[n], w.xrows[n], nblk_max, w.Dpb, grad_atoms);
+        ok &= encode4_planes_mn(&pl->gradn.a[p], w.TB[p], npl, d.Mm, d.Pm, d.Pm, nblk_max, w.Kb, 2);
+        ok &= encode4_planes_mn(&pl->gradn.b[p], w.XB[q], npl, d.D, w.xrows[q], w.xrows[q], nblk_max, w.Dpb, grad_atoms);
+        ok &= encode3(&pl->gradq.c[p], w.GX[q], d.D, d.Pm, nblk_max, d.Dp, (long long)w.grows[q] * d.Dp, 32, 32);
+        ok &= encode3(&pl->gradn.c[p], w.GX[n], d.D, d.Mm, nblk_max, d.Dp, (long long)w.grows[n] * d.Dp, 32, 32);
       } else {
         int o = ARR_N0 + (1 - p);
-        ok &= encode4_planes(&pl->gradm.a[p], w.AB[p], npl, d.Mm, d.Mm, d.Mm, nblk_max, w.Kb, 32, 128);
-        ok &= encode4_planes(&pl->gradm.b[p], w.XB[o], npl, d.D, w.xrows[o], w.xrows[o], nblk_max, w.Dpb, 64, 32);
-        ok &= encode3(&pl->gradm.c[p], w.GX[n], d.D, d.Mm, nblk_max, d.Dp, (long long)d.Mm * d.Dp, 32, 32, false);
-        // the same product transposed, GN^T = N_other^T . A^T: tile rows run over D (every 128-row tile full,
-        // where Mm = 200 leaves the second one 56 % used), tile columns over the Mm coefficient rows
-        pl->gradt.a[p] = pl->gradm.b[p];
-        ok &= encode4_planes(&pl->gradt.b[p], w.AB[p], npl, d.Mm, d.Mm, d.Mm, nblk_max, w.Kb, 32, pl->bn_score);
-        pl->gradt.c[p] = pl->gradm.c[p];
+        // transposed, GN^T = N_other^T . A^T: tile rows run over D (every 128-row tile full, where Mm = 200 would leave
+        // the second one 56 % used), tile columns over the Mm coefficient rows
+        ok &= encode4_planes_mn(&pl->gradt.a[p], w.XB[o], npl, d.D, w.xrows[o], w.xrows[o], nblk_max, w.Dpb, 2);
+        ok &= encode4_planes(&pl->gradt.b[p], w.AB[p], npl, d.Mm, d.Mm, d.Mm, nblk_max, w.Kb, pl->bn_score);
+        ok &= encode3(&pl->gradt.c[p], w.GX[n], d.D, d.Mm, nblk_max, d.Dp, (long long)d.Mm * d.Dp, 32, 32);
         if (w.TB[0]) {
           // dual mode: B1 = TB[side] read MN-major (k = i < Pm rows, n = m < Mm), B2 = TB[other side] read K-major (rows
           // i < Pm, k = j < Mm); what lies beyond those extents is outside the maps and arrives as zeros
           pl->has_dual = true;
           pl->bn2 = (d.Pm + 15) / 16 * 16;
-          pl->gradu.a[p] = pl->gradm.b[p];
-          ok &= encode4_planes(&pl->gradu.b[p], w.TB[p], npl, d.Mm, d.Pm, d.Pm, nblk_max, w.Kb, 64, 32);
-          ok &= encode4_planes(&pl->gradu.b2[p], w.TB[1 - p], npl, d.Mm, d.Pm, d.Pm, nblk_max, w.Kb, 32, pl->bn2);
-          pl->gradu.c[p] = pl->gradm.c[p];
+          pl->gradu.a[p] = pl->gradt.a[p];
+          ok &= encode4_planes_mn(&pl->gradu.b[p], w.TB[p], npl, d.Mm, d.Pm, d.Pm, nblk_max, w.Kb, score_atoms);
+          ok &= encode4_planes(&pl->gradu.b2[p], w.TB[1 - p], npl, d.Mm, d.Pm, d.Pm, nblk_max, w.Kb, pl->bn2);
+          pl->gradu.c[p] = pl->gradt.c[p];
         }
       }
     }
@@ -474,29 +464,29 @@ void *pbg_tc_plan_create(const WaveDims &d, const WaveBufs &w, int nblk_max, int
     long long qblk = (long long)w.xrows[q] * d.Dp, nblk_s = (long long)w.xrows[n] * d.Dp, tblk = (long long)d.Pm * d.Ms;
     // score: A = Q (K-major, k = D), B = N (K-major)
     // only the Pm scored rows exist for the map: the rest of the 128-row box is filled with zeros without touching L2
-    ok &= encode3(&pl->score.a[p], Xq, d.D, d.Pm, nblk_max, d.Dp, qblk, TC_KB, 128, false);
-    ok &= encode3(&pl->score.b[p], Xn, d.D, w.xrows[n], nblk_max, d.Dp, nblk_s, TC_KB, pl->bn_score, false);
+    ok &= encode3(&pl->score.a[p], Xq, d.D, d.Pm, nblk_max, d.Dp, qblk, TC_KB, 128);
+    ok &= encode3(&pl->score.b[p], Xn, d.D, w.xrows[n], nblk_max, d.Dp, nblk_s, TC_KB, pl->bn_score);
     // outputs leave through 32 x 32 bulk stores (128-byte swizzle in shared memory), clipped at the matrix edge
-    ok &= encode3(&pl->score.c[p], w.S[p], d.Mm, d.Pm, nblk_max, d.Ms, tblk, 32, 32, false);
+    ok &= encode3(&pl->score.c[p], w.S[p], d.Mm, d.Pm, nblk_max, d.Ms, tblk, 32, 32);
     if (pl->dynamic) {
       // grad Q: A = T (K-major, k = Mm), B = N (MN-major: k rows = Mm, contiguous D)
-      ok &= encode3(&pl->gradq.a[p], T, d.Mm, d.Pm, nblk_max, d.Ms, tblk, TC_KB, 128, false);
-      ok &= encode3(&pl->gradq.b[p], Xn, d.D, w.xrows[n], nblk_max, d.Dp, nblk_s, 32, TC_KB, true);
+      ok &= encode3(&pl->gradq.a[p], T, d.Mm, d.Pm, nblk_max, d.Ms, tblk, TC_KB, 128);
+      ok &= encode3_mn(&pl->gradq.b[p], Xn, d.D, w.xrows[n], nblk_max, d.Dp, nblk_s, TC_KB, grad_atoms);
       // grad N: A = T^T (MN-major: k rows = Pm, contiguous Mm), B = Q (MN-major: k rows = Pm, contiguous D)
-      ok &= encode3(&pl->gradn.a[p], T, d.Mm, d.Pm, nblk_max, d.Ms, tblk, 32, TC_KB, true);
-      ok &= encode3(&pl->gradn.b[p], Xq, d.D, w.xrows[q], nblk_max, d.Dp, qblk, 32, TC_KB, true);
-      ok &= encode3(&pl->gradq.c[p], w.GX[q], d.D, d.Pm, nblk_max, d.Dp, (long long)w.grows[q] * d.Dp, 32, 32, false);
-      ok &= encode3(&pl->gradn.c[p], w.GX[n], d.D, d.Mm, nblk_max, d.Dp, (long long)w.grows[n] * d.Dp, 32, 32, false);
+      ok &= encode3_mn(&pl->gradn.a[p], T, d.Mm, d.Pm, nblk_max, d.Ms, tblk, TC_KB, 4);
+      ok &= encode3_mn(&pl->gradn.b[p], Xq, d.D, w.xrows[q], nblk_max, d.Dp, qblk, TC_KB, grad_atoms);
+      ok &= encode3(&pl->gradq.c[p], w.GX[q], d.D, d.Pm, nblk_max, d.Dp, (long long)w.grows[q] * d.Dp, 32, 32);
+      ok &= encode3(&pl->gradn.c[p], w.GX[n], d.D, d.Mm, nblk_max, d.Dp, (long long)w.grows[n] * d.Dp, 32, 32);
     } else {
       // merged: side p: A = A[p] (K-major, k = Mm), B = the other side's operand rows (MN-major)
       int o = ARR_N0 + (1 - p);
-      ok &= encode3(&pl->gradm.a[p], w.A[p], d.Mm, d.Mm, nblk_max, w.Ma, (long long)d.Mm * w.Ma, TC_KB, 128, false);
-      ok &= encode3(&pl->gradm.b[p], w.X[o], d.D, w.xrows[o], nblk_max, d.Dp, (long long)w.xrows[o] * d.Dp, 32, TC_KB, true);
-      ok &= encode3(&pl->gradm.c[p], w.GX[n], d.D, d.Mm, nblk_max, d.Dp, (long long)d.Mm * d.Dp, 32, 32, false);
+      ok &= encode3(&pl->gradm.a[p], w.A[p], d.Mm, d.Mm, nblk_max, w.Ma, (long long)d.Mm * w.Ma, TC_KB, 128);
+      ok &= encode3_mn(&pl->gradm.b[p], w.X[o], d.D, w.xrows[o], nblk_max, d.Dp, (long long)w.xrows[o] * d.Dp, TC_KB, grad_atoms);
+      ok &= encode3(&pl->gradm.c[p], w.GX[n], d.D, d.Mm, nblk_max, d.Dp, (long long)d.Mm * d.Dp, 32, 32);
       // the same product transposed (see the bf16-plane tier above): A = the other side's operand rows (MN-major),
       // B = the coefficient rows (K-major)
-      pl->gradt.a[p] = pl->gradm.b[p];
-      ok &= encode3(&pl->gradt.b[p], w.A[p], d.Mm, d.Mm, nblk_max, w.Ma, (long long)d.Mm * w.Ma, TC_KB, pl->bn_score, false);
+      ok &= encode3_mn(&pl->gradt.a[p], w.X[o], d.D, w.xrows[o], nblk_max, d.Dp, (long long)w.xrows[o] * d.Dp, TC_KB, 4);
+      ok &= encode3(&pl->gradt.b[p], w.A[p], d.Mm, d.Mm, nblk_max, w.Ma, (long long)d.Mm * w.Ma, TC_KB, pl->bn_score);
       pl->gradt.c[p] = pl->gradm.c[p];
     }
   }

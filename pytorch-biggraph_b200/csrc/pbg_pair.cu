@@ -100,7 +100,7 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
   auto tile_live = [&](int t) { return block_info(d, wb, d.blk0 + t).n != 0; };
 
   if (warp == 0) {
-    // ---------------- TMA producer: one box per (operand array, plane), each from its own lane ----------------
+    // ---------------- TMA producer: one box (all planes) per operand array, each from its own lane ----------------
     long long git = 0;
     bool stop = false;
     for (int t = blockIdx.x; t < d.nblk && !stop; t += gridDim.x) {
@@ -115,11 +115,7 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
         const uint32_t fb = full_bar(s);
         if (lane == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(fb), "r"(stage_tx) : "memory");
         __syncwarp();
-        if (lane < 2 * NPL) {
-          const int arr = lane / NPL, pl = lane - arr * NPL;
-          const uint32_t dst = smem_u32(smem + (size_t)s * g.stage_bytes) + arr * arr_bytes + pl * plane_bytes;
-          tma_load_4d(dst, &maps.n[arr], kb * 32, 0, pl, blk, fb);
-        }
+        if (lane < 2) tma_load_4d(smem_u32(smem + (size_t)s * g.stage_bytes) + lane * arr_bytes, &maps.n[lane], kb * 32, 0, 0, blk, fb);
       }
     }
   } else if (warp == 1 && lane == 0) {
@@ -400,7 +396,7 @@ void *pbg_pair_plan_create(const WaveDims &d, const WaveBufs &w, int nblk_max) {
   bool ok = g.nst >= 2 && w.TB[0];
   // rows beyond the Mm operand rows of a block are outside the map: the box brings zeros for them
   for (int a = 0; a < 2; ++a)
-    ok = ok && encode4_planes(&pl->maps.n[a], w.XB[a], w.npl, d.D, d.Mm, d.Mm, nblk_max, w.Dpb, 32, g.rows_pad);
+    ok = ok && encode4_planes(&pl->maps.n[a], w.XB[a], w.npl, d.D, d.Mm, d.Mm, nblk_max, w.Dpb, g.rows_pad);
   if (!ok) { delete pl; return nullptr; }
   return pl;
 }

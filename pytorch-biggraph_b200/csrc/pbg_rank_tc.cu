@@ -8,7 +8,7 @@
 // 144 KB read per 32 k-values), as in the training contractions.
 //
 // Persistent CTAs walk the tiles of both sides (n fastest):
-//   warp 0     TMA producer, every plane's box from its own lane
+//   warp 0     TMA producer, one box (all planes) per operand
 //   warp 1     tensor memory and MMA issue; two accumulators alternate
 //   warps 2-9  epilogue: thread = edge, two warps per 32 tensor-memory lanes, each one half of the columns
 // Every mbarrier wait is bounded (bit 1 of the error word); every TMA load is CTA-local.
@@ -79,8 +79,8 @@ allnegs_tc_kernel(const __grid_constant__ RankMaps maps, WaveDims d, WaveBufs w,
         const uint32_t fb = full_bar(s), st = smem_u32(smem + (size_t)s * RK_STAGE);
         if (lane == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(fb), "r"(RK_STAGE) : "memory");
         __syncwarp();
-        if (lane < 3) tma_load_4d(st + lane * RK_PLANE_A, &maps.q, kb * 32, m0, lane, side, fb);
-        else if (lane < 6) tma_load_4d(st + 3 * RK_PLANE_A + (lane - 3) * RK_PLANE_B, &maps.y, kb * 32, n0, lane - 3, side, fb);
+        if (lane == 0) tma_load_4d(st, &maps.q, kb * 32, m0, 0, side, fb);
+        else if (lane == 1) tma_load_4d(st + 3 * RK_PLANE_A, &maps.y, kb * 32, n0, 0, side, fb);
       }
     }
   } else if (warp == 1 && lane == 0) {
@@ -187,8 +187,8 @@ allnegs_tc_kernel(const __grid_constant__ RankMaps maps, WaveDims d, WaveBufs w,
 int launch_allnegs_score_tc(const WaveDims &d, const WaveBufs &w, const AllNegs &a, long long row0, cudaStream_t st) {
   // (encoding two maps is a microsecond of host time beside a call of a hundred)
   RankMaps maps;
-  if (!encode4_planes(&maps.q, a.QB, 3, d.D, a.B, a.qrows, 2, a.Dpb, 32, 128) ||
-      !encode4_planes(&maps.y, a.YB, 3, d.D, a.slab, a.slab, 2, a.Dpb, 32, RK_BN)) {
+  if (!encode4_planes(&maps.q, a.QB, 3, d.D, a.B, a.qrows, 2, a.Dpb, 128) ||
+      !encode4_planes(&maps.y, a.YB, 3, d.D, a.slab, a.slab, 2, a.Dpb, RK_BN)) {
     pbg_note_launch(cudaErrorUnknown);
     return 0;
   }

@@ -30,6 +30,11 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map
                :: "r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar) : "memory");
 }
 
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, int c4, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+               :: "r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar) : "memory");
+}
+
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo, uint32_t layout) {
   return ((uint64_t)((addr >> 4) & 0x3FFF)) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
          ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46) | ((uint64_t)layout << 61);
@@ -60,34 +65,49 @@ inline EncodeFn get_encode() {
   return fn;
 }
 
-// 3-D map over an array laid out [nblk][rows][ld] floats: dims {inner extent, rows, nblk}.
-inline bool encode3(CUtensorMap *tm, const float *base, int inner, int rows, int nblk, int ld, long long blk_stride,
-                    int box_inner, int box_rows, bool mn_major) {
+// Every operand tile of a stage is ONE box, whatever it holds: a bulk tensor copy costs its issue and its own walk
+// through the copy engine, a few hundred cycles each, and a stage of 32 k-values used to be up to fifteen of them (a box
+// per plane, and per 32 or 64 columns of an MN-major operand).  An array is therefore described with its planes and its
+// column blocks as dimensions of their own.
+inline bool encode_map(CUtensorMap *tm, CUtensorMapDataType type, const void *base, int rank, const cuuint64_t *dims, const cuuint64_t *strides,
+                       const cuuint32_t *box, CUtensorMapSwizzle swizzle) {
   EncodeFn enc = get_encode();
   if (!enc) return false;
-  cuuint64_t dims[3] = {(cuuint64_t)inner, (cuuint64_t)rows, (cuuint64_t)nblk};
-  cuuint64_t strides[2] = {(cuuint64_t)ld * 4, (cuuint64_t)blk_stride * 4};
-  cuuint32_t box[3] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1};
-  cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void *)base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   mn_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : (box_inner * 4 == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B),
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
+  cuuint32_t es[5] = {1, 1, 1, 1, 1};
+  return enc(tm, type, (cuuint32_t)rank, (void *)base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// bf16 plane arrays [nblk][3][rows][ld]: a 4-D map (inner, rows, plane, block).  K-major operands
-// (box_inner = 32 k-values, 64-byte swizzle) or MN-major (box = 64 contiguous x 32 k rows, 128-byte swizzle).
-inline bool encode4_planes(CUtensorMap *tm, const unsigned short *base, int npl, int inner, int rows, int rows_alloc, int nblk, int ld,
-                           int box_inner, int box_rows) {
-  EncodeFn enc = get_encode();
-  if (!enc) return false;
-  cuuint64_t dims[4] = {(cuuint64_t)inner, (cuuint64_t)rows, (cuuint64_t)npl, (cuuint64_t)nblk};
-  cuuint64_t strides[3] = {(cuuint64_t)ld * 2, (cuuint64_t)rows_alloc * ld * 2, (cuuint64_t)npl * rows_alloc * ld * 2};
-  cuuint32_t box[4] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1, 1};
-  cuuint32_t es[4] = {1, 1, 1, 1};
-  CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   box_inner * 2 == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
+// fp32 arrays [nblk][rows][ld].  K-major operands and outputs: boxes of box_inner floats x box_rows rows (128-byte swizzle;
+// 64 bytes wide: 64-byte swizzle), coordinates (column, row, block).
+inline bool encode3(CUtensorMap *tm, const float *base, int inner, int rows, int nblk, int ld, long long blk_stride, int box_inner, int box_rows) {
+  const cuuint64_t dims[3] = {(cuuint64_t)inner, (cuuint64_t)rows, (cuuint64_t)nblk};
+  const cuuint64_t strides[2] = {(cuuint64_t)ld * 4, (cuuint64_t)blk_stride * 4};
+  const cuuint32_t box[3] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1};
+  return encode_map(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, base, 3, dims, strides, box, box_inner * 4 == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
+}
+// MN-major operands: `atoms` blocks of 32 columns x box_k rows, coordinates (0, k row, column block, block).  The last block
+// of columns may reach past the row's end: what it brings belongs to output columns that are clipped.
+inline bool encode3_mn(CUtensorMap *tm, const float *base, int inner, int rows, int nblk, int ld, long long blk_stride, int box_k, int atoms) {
+  const cuuint64_t dims[4] = {32, (cuuint64_t)rows, (cuuint64_t)((inner + 31) / 32), (cuuint64_t)nblk};
+  const cuuint64_t strides[3] = {(cuuint64_t)ld * 4, 128, (cuuint64_t)blk_stride * 4};
+  const cuuint32_t box[4] = {32, (cuuint32_t)box_k, (cuuint32_t)atoms, 1};
+  return encode_map(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, base, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
 }
 
+// bf16 plane arrays [nblk][npl][rows][ld].  K-major: all planes of 32 k-values x box_rows rows (64-byte swizzle), coordinates
+// (k, row, 0, block).
+inline bool encode4_planes(CUtensorMap *tm, const unsigned short *base, int npl, int inner, int rows, int rows_alloc, int nblk, int ld, int box_rows) {
+  const cuuint64_t dims[4] = {(cuuint64_t)inner, (cuuint64_t)rows, (cuuint64_t)npl, (cuuint64_t)nblk};
+  const cuuint64_t strides[3] = {(cuuint64_t)ld * 2, (cuuint64_t)rows_alloc * ld * 2, (cuuint64_t)npl * rows_alloc * ld * 2};
+  const cuuint32_t box[4] = {32, (cuuint32_t)box_rows, (cuuint32_t)npl, 1};
+  return encode_map(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B);
+}
+// MN-major: `atoms` blocks of 64 columns, each all planes of 32 rows (128-byte swizzle), coordinates (0, k row, 0, column
+// block, block)
+inline bool encode4_planes_mn(CUtensorMap *tm, const unsigned short *base, int npl, int inner, int rows, int rows_alloc, int nblk, int ld, int atoms) {
+  const cuuint64_t dims[5] = {64, (cuuint64_t)rows, (cuuint64_t)npl, (cuuint64_t)((inner + 63) / 64), (cuuint64_t)nblk};
+  const cuuint64_t strides[4] = {(cuuint64_t)ld * 2, (cuuint64_t)rows_alloc * ld * 2, 128, (cuuint64_t)npl * rows_alloc * ld * 2};
+  const cuuint32_t box[5] = {64, 32, (cuuint32_t)npl, (cuuint32_t)atoms, 1};
+  return encode_map(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, 5, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
