@@ -15,7 +15,7 @@
 // Ranking inside a run uses __match_any_sync, so equal digits keep their input order (stable).
 //
 // That is the form for long lists.  A list that fits in the shared memory of one thread-block cluster -- every wave
-// up to 262,144 slots -- is sorted by ONE kernel (cluster_sort_kernel, at the end of this file).
+// up to 262,144 slots -- is sorted by ONE kernel (sort_waves_kernel, at the end of this file).
 #include <cooperative_groups.h>
 
 #include "pbg_common.cuh"
