@@ -236,10 +236,9 @@ __device__ __forceinline__ unsigned long long slot_key(const WaveDims &d, const 
 // Programmatic dependent launch: every kernel of the step is launched while the kernel before it in the stream still
 // runs (pbg_launch) and begins with this -- it waits until that one is complete and its writes are visible, then lets
 // the next one be scheduled.  What overlaps is the launch itself, one to two microseconds per kernel of a step of ten.
-__device__ __forceinline__ void pdl_begin() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_begin() { pdl_wait(); pdl_release(); }
 
 // N3 regularizer pieces at elements [dd, dd + 4) of a row y: the term is sum m^3 with m = |y_d|, or for
 // complex_diagonal the modulus of the pair (y_d, y_{d +- D/2}) counted once per pair

@@ -59,6 +59,10 @@ struct TcGeom {
   // B1 as an MN-major operand (K1 = Pm rows), B2 as a K-major one (BN2 = Pm rounded up to 16 rows, K = Mm).
   // A stage holds the A tile, B1 (for the k-blocks below K1) and B2.
   int dual, K1, BN2;
+  // The launch before this one is its sibling (the other gradient of dynamic relations): same inputs, other outputs.  A
+  // launch's tiles are a few rounds of one per SM and the last round is half empty, so the CTAs of this one start as the
+  // sibling's leave, and wait for its end only before they end themselves (what comes next may count on both).
+  int sibling;
 };
 
 template <bool A_MN, bool B_MN, int NTERMS, bool L2EPI>
@@ -115,7 +119,9 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base_s;
-  pdl_begin();                                               // barriers and tensor memory are set up beside the kernel before this one
+  // barriers and tensor memory are set up beside the kernel before this one
+  if (g.sibling) pdl_release();                              // the sibling has waited for our inputs, and bulk copies read them from L2
+  else pdl_begin();
   const int nkb = (g.K + KB - 1) / KB;
   const int b_atoms = PLANES ? (g.BN + 63) / 64 : (g.BN + 31) / 32;     // MN-major boxes per B tile (per plane)
   const uint32_t b_tile = B_MN ? (uint32_t)b_atoms * BOX_BYTES : (uint32_t)g.BN * ROW_BYTES;    // bytes of one B tile (of one plane)
@@ -129,12 +135,12 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
   const uint32_t b2_plane = (uint32_t)g.BN2 * ROW_BYTES;                 // dual: one plane of the B2 tile
   // persistent tile loop: tile t -> (n tile, m tile, chunk block, problem); every role walks the same list
   const int tiles_n = (g.N + g.BN - 1) / g.BN, tiles_m = (g.M + 127) / 128;
-  const long long ntiles = (long long)tiles_n * tiles_m * d.nblk * 2;
-  auto tile_live = [&](long long t, int &p, int &blk, int &m0, int &n0) {
-    int x = (int)(t % tiles_n);
-    long long r = t / tiles_n;
-    int y = (int)(r % tiles_m);
-    int z = (int)(r / tiles_m);
+  const int ntiles = tiles_n * tiles_m * d.nblk * 2;
+  auto tile_live = [&](int t, int &p, int &blk, int &m0, int &n0) {
+    // the column tiles of a row are dealt in turn: where they differ in width (400 columns: 224 + 176) and their number
+    // divides the grid's, a CTA would otherwise get the wide one every time
+    const int r = t / tiles_n, x = (t + r * tiles_n / (int)gridDim.x) % tiles_n;
+    const int z = r / tiles_m, y = r - z * tiles_m;
     p = z & 1; blk = d.blk0 + (z >> 1); m0 = y * 128; n0 = x * g.BN;
     BlockInfo bi = block_info(d, wb, blk);
     return bi.n != 0 && !(g.score && !d.neg_enabled[p]);
@@ -144,7 +150,7 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
     // ---------------- TMA producer (one box per operand, each from its own lane) ----------------
     long long git = 0;
     bool stop = false;
-    for (long long t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
+    for (int t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
       int p, blk, m0, n0;
       if (__any_sync(0xffffffffu, failed != 0)) break;
       if (!tile_live(t, p, blk, m0, n0)) continue;
@@ -179,7 +185,7 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
     const uint32_t idesc0 = (1u << 4) | (fmt << 7) | (fmt << 10) | ((A_MN ? 1u : 0u) << 15) | ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(128 >> 4) << 24);
     const uint32_t idesc2 = (idesc0 & ~(1u << 16)) | ((uint32_t)(g.BN2 >> 3) << 17);   // dual: the B2 products are K-major, BN2 columns wide
     long long git = 0, j = 0;
-    for (long long t = blockIdx.x; t < ntiles && !failed; t += gridDim.x) {
+    for (int t = blockIdx.x; t < ntiles && !failed; t += gridDim.x) {
       int p, blk, m0, n0;
       if (!tile_live(t, p, blk, m0, n0)) continue;
       const int ab = (int)(j & 1);
@@ -266,7 +272,7 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
     const uint32_t nchunks = stage_tx / 16;
     long long git = 0;
     bool stop = false;
-    for (long long t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
+    for (int t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
       int p, blk, m0, n0;
       if (__any_sync(0xffffffffu, failed != 0)) break;           // warp-uniform exit
       if (!tile_live(t, p, blk, m0, n0)) continue;
@@ -303,7 +309,7 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
     // ---------------- epilogue: drains accumulator j & 1 while the next tile is being multiplied ----------------
     long long j = 0, nst = 0;
     const int q = warp & 3;                           // the 32 TMEM lanes this warp may read
-    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
       int p, blk, m0, n0;
       if (__any_sync(0xffffffffu, failed != 0)) break;           // warp-uniform exit (tcgen05.ld is warp-wide)
       if (!tile_live(t, p, blk, m0, n0)) continue;
@@ -374,6 +380,7 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // the stores have left shared memory and are performed
   }
+  if (g.sibling) pdl_wait();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 1) {
@@ -602,7 +609,7 @@ int launch_grad_tc(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, 
   for (int p = 0; p < 2; ++p) g.C[p] = w.GX[ARR_Q0 + p];
   launch_tc<false, true>(pl->gradq, g, pl->nterms, d, wb, w.errflag, st);
   // GN_p = T_p^T . Q_p
-  g.M = d.Mm; g.K = d.Pm; g.c_blk = (long long)w.grows[ARR_N0] * d.Dp;
+  g.M = d.Mm; g.K = d.Pm; g.c_blk = (long long)w.grows[ARR_N0] * d.Dp; g.sibling = 1;
   for (int p = 0; p < 2; ++p) g.C[p] = w.GX[ARR_N0 + p];
   launch_tc<true, true>(pl->gradn, g, pl->nterms, d, wb, w.errflag, st);
   return 2;

@@ -1,0 +1,52 @@
+"""One batch against the oracle where the step's kernels change form: score rows at the widths of the loss kernels' register
+rows (128, 256, 512, 1024), the fused score kernel's narrow form (up to 128 score columns a side), column tiles that do not divide the
+gradient's width, chunks and column counts of one, and operator rows above 1024 floats."""
+import numpy as np
+import pytest
+
+from oracle import pbg_step as O
+from test_gpu_step import RTOL, _close, _random_case, _tier_tolerance
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(case, precision):
+    from b200_util import Rig
+    c, ocfg, ost, batches = case
+    rig = Rig.from_oracle_state(c, ost, precision=precision)
+    W0 = ost.W_lhs.copy()
+    b = batches[0]
+    want = O.train_batch(ocfg, ost, *b)
+    got = rig.trainer.process_one_batch(rig.model, rig.edges(b[0], b[1], b[2]), b[3], b[4])
+    assert got.metrics["loss"] == pytest.approx(want["loss"], rel=RTOL if precision != "bf16x3" else 10 * RTOL)
+    step = float(np.abs(ost.W_lhs - W0).max())
+    _close(rig.W_lhs.cpu().numpy(), ost.W_lhs, atol=max(1e-6, RTOL * step), what="W")
+    _close(rig.G("lhs"), ost.G_lhs, atol=1e-8, what="G")
+    if ost.theta_rhs is not None:
+        _close(rig.theta("rhs"), ost.theta_rhs, atol=1e-6, what="theta_rhs")
+
+
+@pytest.mark.parametrize("cols", [128, 129, 256, 257, 512, 513, 1024, 1025])
+@pytest.mark.parametrize("comp,loss", [("dot", "ranking"), ("dot", "logistic"), ("l2", "softmax")])
+def test_score_rows_at_the_loss_kernels_widths(cols, comp, loss):
+    nb = cols // 2
+    _run(_random_case(5, 24, 4000, 2 * nb + 3, nb, cols - nb, "none", comp, loss), "tf32x3")
+
+
+@pytest.mark.parametrize("tier", ["bf16x6", "bf16x3"])
+@pytest.mark.parametrize("nb,nu", [(1, 1), (64, 64), (64, 65), (100, 28), (100, 29), (128, 1)])
+def test_fused_scores_at_the_narrow_form_s_edge(nb, nu, tier):
+    with _tier_tolerance(tier):
+        _run(_random_case(6, 100, 4000, 5 * nb + 1, nb, nu, "none", "dot", "softmax"), tier)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "tf32x3", "bf16x6", "bf16x3"])
+@pytest.mark.parametrize("D,nb,nu", [(400, 260, 37), (260, 129, 0), (516, 1, 300), (776, 100, 1)])
+def test_column_tiles_of_both_gradients(D, nb, nu, precision):
+    with _tier_tolerance(precision):
+        _run(_random_case(7, D, 3000, 2 * nb + 1, nb, nu, "diagonal", "dot", "softmax", dyn=True, R=9), precision)
+
+
+@pytest.mark.parametrize("D", [1024, 1028])
+def test_operator_rows_of_wide_models(D):
+    _run(_random_case(8, D, 2000, 300, 50, 20, "translation", "dot", "softmax", dyn=True, R=4, zipf=True), "tf32x3")
