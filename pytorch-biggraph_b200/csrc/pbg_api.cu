@@ -258,8 +258,8 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   for (int s = 0; s < 2; ++s)
     for (int i = 0; i < PBG_SORT_WAVES; ++i) { oWK[s][i] = take((size_t)nocc * 8); oWV[s][i] = take((size_t)nocc * 4); }
   size_t oSum = take(8 * sizeof(double)), oEval = take((size_t)pbg_eval_ctas(c->Cm, c->Pm) * 8 * sizeof(double)), oEvalDone = take(4);
-  size_t oPsum = take((size_t)nocc * c->Dp * 4), oHub = take(((size_t)nocc / 8 + 64) * 8), oHubCnt = take(512);
-  size_t oBigTab = take(pbg_bigtab_bytes((long long)nocc));
+  size_t oPsum = take((size_t)nocc * c->Dp * 4), oHub = take(2 * (size_t)pbg_hublist_entries(nocc) * 8), oHubCnt = take(512);
+  size_t oBigTab = take(2 * pbg_bigtab_bytes((long long)nocc));
   // dynamic relations with a (vector) operator: the operator-row gradient of every edge, written by the pull-back pass
   size_t oGR[2] = {0, 0};
   const bool keep_gr = dyn && cfg->op != PBG_OP_NONE && !matrix_op;

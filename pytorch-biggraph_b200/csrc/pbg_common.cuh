@@ -449,6 +449,8 @@ struct UpdateScratch {
 };
 int launch_update(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, const unsigned long long *keys, const unsigned int *vals,
                   float lr, float rel_lr, const UpdateScratch &us, cudaStream_t st);
+// hublist and bigtab: a part for the embedding rows and one for the operator rows (as are hubcnt[0..1] and hubcnt[32..33] of a set).
+inline long long pbg_hublist_entries(long long nocc) { return nocc / 8 + 64; }
 // bigtab: a line for each row with 256 and more slots: where its batches start, its end, a counter (zero between waves)
 inline size_t pbg_bigtab_bytes(long long nocc) { return (size_t)(nocc / 256 + 2) * (PBG_KMAX + 2) * sizeof(long long); }
 // Evaluation of one batch after its scores.  out8 (host or device memory): loss, then pos_rank, mrr, r1, r10, r50 summed over

@@ -278,6 +278,18 @@ __device__ __forceinline__ long long *hub_biglist(long long *hublist, int nocc) 
 __device__ __forceinline__ const long long *hub_biglist(const long long *hublist, int nocc) { return hublist + nocc / 16 + 32; }
 enum { RULE_EMB = 0, RULE_REL = 1 };
 
+// The kernels of the operator rows (dynamic relations) work beside those of the embedding rows launched just before them:
+// other rows, other places in psum, lists and counters of their own.  Each of the four is bound by the chain of one row, so
+// in turn they took as long as all their chains together (dimension 400, 1,345 relations, every row a hub: the update 172 us a wave, 157 so; dimension 200, 14,824 relations: 169 and 164).  Such a kernel does not wait for the one before
+// it -- that one has waited for everything both read, and the fence keeps reads from lines of before -- but must not be
+// complete before it is, because the next launch counts on both: its last CTA waits for that and has no other work.
+__device__ __forceinline__ bool sibling_begin() {
+  pdl_release();
+  if (blockIdx.x == gridDim.x - 1) { pdl_wait(); return false; }
+  __threadfence();
+  return true;
+}
+
 template <int VEC, int RULE>
 struct RowState {
   float4 v[VEC], a[VEC];     // row; per-element accumulator (RULE_REL only)
@@ -387,7 +399,8 @@ __global__ void __launch_bounds__(32 * TileWarps<VEC, RULE>::N, RULE == RULE_EMB
 tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys,
                    const unsigned int *__restrict__ vals, float lr, float *__restrict__ psum,
                    long long *__restrict__ hublist, int *__restrict__ hubcnt, ParamJob job, int aside) {
-  pdl_begin();
+  if (RULE == RULE_EMB) pdl_begin();
+  else if (!sibling_begin()) return;
   constexpr int WARPS = TileWarps<VEC, RULE>::N, STAGE = StageRows<VEC, RULE>::N;
   extern __shared__ __align__(128) float stage_all[];        // [WARPS][STAGE][Dp]
   __shared__ __align__(8) unsigned long long sbar[WARPS];
@@ -639,7 +652,8 @@ __global__ void __launch_bounds__(32 * UPD_WARPS)
 hub_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys, const unsigned int *__restrict__ vals, float lr,
            float *psum, const long long *__restrict__ hublist, const int *__restrict__ hubcnt, int *__restrict__ hubcnt_next,
            long long *bigtab, int aside, ParamJob job, pbg_batch_stats *per_batch, double *sum) {
-  pdl_begin();
+  if (RULE == RULE_EMB) pdl_begin();
+  else if (!sibling_begin()) return;
   static_assert(32 * UPD_WARPS == HUB_BIG, "one probe per thread covers exactly the rows that are not big");
   extern __shared__ __align__(16) float tot[];               // [k][VEC * 128]; sums of a big row's batch: [UPD_WARPS][VEC * 128]
   __shared__ long long bstart[PBG_KMAX + 1];
@@ -662,7 +676,7 @@ hub_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__r
   const int nh = hubcnt[0], nbig = hubcnt[1];                 // the tile kernel listed the rows
   const long long *biglist = hub_biglist(hublist, d.nocc);
   // the batches of the big rows first, then the list of all hub rows, big ones skipped
-  const int ctas = gridDim.x - cta0, items = nbig * d.k + nh;
+  const int ctas = (int)gridDim.x - (RULE == RULE_REL) - cta0, items = nbig * d.k + nh;
   for (int item = blockIdx.x - cta0; item < items; item += ctas) {
     const bool from_big = item < nbig * d.k;
     const int h = item / d.k;
@@ -1055,7 +1069,7 @@ static int launch_update_vec(const WaveDims &d, const WaveBatches &wb, const Wav
   static_assert(PBG_KMAX * 32 <= UPD_WARPS * 128, "param_step works in the same shared memory");
   // the attribute is set once for the largest wave this row width allows in 227 KB
   size_t hub_smem_max = (size_t)PBG_KMAX * VEC * 128 * sizeof(float);
-  if (hub_smem_max > 227 * 1024) hub_smem_max = 227 * 1024;
+  if (hub_smem_max > 222 * 1024) hub_smem_max = 222 * 1024;    // of 227 KB: the kernel has up to 5 KB of static shared memory
   // per device (a process may hold contexts on several GPUs); a failed opt-in makes the launch fail,
   // which the caller's cudaGetLastError reports
   pbg_opt_in_smem((const void *)hub_kernel<VEC, RULE_EMB>, (int)hub_smem_max);
@@ -1068,20 +1082,23 @@ static int launch_update_vec(const WaveDims &d, const WaveBatches &wb, const Wav
   size_t tile_smem = (size_t)EMB_WARPS * StageRows<VEC, RULE_EMB>::N * d.Dp * 4;
   if (sum_ctas && tile_smem < 8 * 128 * 4) tile_smem = 8 * 128 * 4;
   pbg_launch(tile_update_kernel<VEC, RULE_EMB>, sum_ctas + (unsigned)((tiles + EMB_WARPS - 1) / EMB_WARPS), 32 * EMB_WARPS, tile_smem, st, d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, job, sum_ctas);
+  const bool rel_rows = d.dynamic && d.op != PBG_OP_NONE && w.theta[0] != nullptr;
+  long long *rel_hublist = us.hublist + pbg_hublist_entries(d.nocc), *rel_bigtab = us.bigtab + pbg_bigtab_bytes(d.nocc) / sizeof(long long);
+  if (rel_rows) {
+    pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_REL>, REL_WARPS * TILE * VEC * 512);
+    pbg_launch(tile_update_kernel<VEC, RULE_REL>, (unsigned)((tiles + REL_WARPS - 1) / REL_WARPS) + 1, 32 * REL_WARPS, (size_t)REL_WARPS * TILE * d.Dp * 4, st, d, wb, w, keys, vals, rel_lr, us.psum, rel_hublist, hubcnt + 32, job, 0);
+  }
   pbg_launch(hub_kernel<VEC, RULE_EMB>, d.k + param_step_ctas(d, job) + hub_ctas, 32 * UPD_WARPS, hub_smem, st,
              d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 1, job, us.per_batch, us.sum);
   launches += 2;
+  if (rel_rows) {
+    pbg_opt_in_smem((const void *)hub_kernel<VEC, RULE_REL>, (int)hub_smem_max);
+    pbg_launch(hub_kernel<VEC, RULE_REL>, hub_ctas + 1, 32 * UPD_WARPS, hub_smem, st,
+               d, wb, w, keys, vals, rel_lr, us.psum, rel_hublist, hubcnt + 32, hubcnt_next + 32, rel_bigtab, 0, job, (pbg_batch_stats *)nullptr, (double *)nullptr);
+    launches += 2;
+  }
   if (d.op != PBG_OP_NONE && w.theta[0] != nullptr) {
-    if (d.dynamic) {
-      pbg_opt_in_smem((const void *)hub_kernel<VEC, RULE_REL>, (int)hub_smem_max);
-      pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_REL>, REL_WARPS * TILE * VEC * 512);
-      int *t = hubcnt; hubcnt = hubcnt_next; hubcnt_next = t;
-      ++*us.turn;
-      pbg_launch(tile_update_kernel<VEC, RULE_REL>, (unsigned)((tiles + REL_WARPS - 1) / REL_WARPS), 32 * REL_WARPS, (size_t)REL_WARPS * TILE * d.Dp * 4, st, d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt, job, 0);
-      pbg_launch(hub_kernel<VEC, RULE_REL>, hub_ctas, 32 * UPD_WARPS, hub_smem, st,
-                 d, wb, w, keys, vals, rel_lr, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 0, job, (pbg_batch_stats *)nullptr, (double *)nullptr);
-      launches += 2;
-    } else if (d.matrix_op) {
+    if (d.matrix_op) {
       launches += launch_matrix_update(d, wb, w, rel_lr, st);
     }
   }
