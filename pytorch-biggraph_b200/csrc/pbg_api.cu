@@ -141,6 +141,22 @@ static int chunk_geometry(const pbg_config &cfg, int *Pm, int *Cm) {
   return PBG_OK;
 }
 
+// Whether the fused score + loss kernel and the dual gradient product take less time than the kernels they replace (score,
+// loss, merged coefficients, gradient).  The fused kernel gives a chunk block to one CTA, its loss included: fewer and
+// shorter launches where the blocks of a full wave fill the SMs, a long single epilogue where they do not.  Measured time
+// of the separate kernels over that of the fused ones (whole buckets, 50 to 200 score columns, dimensions 64 / 256 / 512 / 1024):
+//   softmax   12 to 24 blocks 0.85-1.0 (any dimension); 32 and more: three planes 1.1 / 1.03 / 0.98 / 0.96,
+//             two planes 1.15 / 1.09 / 1.05 / 1.01 (512 below 72 blocks: 0.98)
+//   logistic  (log1p and exp of every score in the epilogue) 0.65-0.98, but two planes up to dimension 128 on
+//             nearly full rounds of CTAs 1.04-1.13
+// Ranking keeps to the dimension alone: hinges turn the two forms' different roundings into different trajectories.
+static bool fused_pays(const pbg_config &cfg, int npl, long long blocks) {
+  if (cfg.loss == PBG_LOSS_RANKING) return cfg.dim <= 256;
+  if (cfg.loss == PBG_LOSS_SOFTMAX) return blocks > 24 && (cfg.dim <= 256 || (npl == 2 && cfg.dim <= 512 && blocks >= 72));
+  const long long sms = pbg_sm_count(), rounds = (blocks + sms - 1) / sms;
+  return npl == 2 && cfg.dim <= 128 && 4 * blocks >= 3 * rounds * sms;
+}
+
 extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_context **out) {
   if (!cfg || !out) return PBG_ERR_BAD_ARGUMENT;
   *out = nullptr;
@@ -217,15 +233,13 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   }
   const int Dpb = (cfg->dim + 7) / 8 * 8, Kb = (c->Mm + 7) / 8 * 8;
   size_t oXB[4] = {0, 0, 0, 0}, oAB[2] = {0, 0}, oTB[2] = {0, 0};
-  // Standard relations under the dot / cos comparators with one score tile per chunk block: the fused
-  // score + loss kernel and the dual gradient product (pbg_pair.cu).  Measured on a B200 it wins at dimension 100
-  // (+2.5 % and +5 % on the two such workloads, fewer and shorter launches) and loses at dimension 1024 (-4 %: the
-  // dual product's second operand costs more there than the merged coefficient matrix it saves), so it is the
-  // default up to dimension 256.  PBG_FUSED=1 / 0 in the environment forces one or the other.
+  // Standard relations under the dot / cos comparators with one score tile per chunk block: the fused score + loss kernel and
+  // the dual gradient product (pbg_pair.cu), where fused_pays says so.  PBG_FUSED=1 / 0 in the environment forces one or
+  // the other.
   {
     const char *env = getenv("PBG_FUSED");
     const bool eligible = planes && !dyn && !matrix_op && cfg->comparator < PBG_CMP_L2 && c->Pm <= 128 && c->Mm <= 256;
-    c->fused = eligible && (env && (env[0] == '0' || env[0] == '1') ? env[0] == '1' : cfg->dim <= 256);
+    c->fused = eligible && (env && (env[0] == '0' || env[0] == '1') ? env[0] == '1' : fused_pays(*cfg, npl, (long long)c->kmax * c->Cm));
     const char *envh = getenv("PBG_HALVES");
     c->fused_halves = envh && envh[0] == '1';
     const char *envk = getenv("PBG_SPLIT_MIN_K");

@@ -35,7 +35,8 @@ def test_score_rows_at_the_loss_kernels_widths(cols, comp, loss):
 
 @pytest.mark.parametrize("tier", ["bf16x6", "bf16x3"])
 @pytest.mark.parametrize("nb,nu", [(1, 1), (64, 64), (64, 65), (100, 28), (100, 29), (128, 1)])
-def test_fused_scores_at_the_narrow_form_s_edge(nb, nu, tier):
+def test_fused_scores_at_the_narrow_form_s_edge(nb, nu, tier, monkeypatch):
+    monkeypatch.setenv("PBG_FUSED", "1")
     with _tier_tolerance(tier):
         _run(_random_case(6, 100, 4000, 5 * nb + 1, nb, nu, "none", "dot", "softmax"), tier)
 
