@@ -375,12 +375,6 @@ struct RowState {
   }
 };
 
-// Rows a warp stages at once.  Narrow rows get more buffers than a tile has slots: a row of five to twelve slots, which
-// belongs to the tile of its first slot, is then on its way in one round instead of two or three one after the other --
-// the longest chain of the kernel.
-template <int VEC, int RULE>
-struct StageRows { enum { N = RULE == RULE_REL ? TILE : VEC == 1 ? 12 : TILE }; };
-
 // Embedding rows: 4 warps per CTA, each with row buffers in shared memory that it fills with
 // bulk asynchronous copies (cp.async.bulk, completion on the warp's mbarrier): the gradient rows
 // of a whole tile are in flight at once instead of one dependent 16-byte-per-lane load at a time.
@@ -395,13 +389,13 @@ template <int VEC, int RULE>
 struct TileWarps { enum { N = RULE == RULE_EMB ? TILE_WARPS_EMB : VEC > 8 ? UPD_WARPS / 2 : UPD_WARPS }; };
 
 template <int VEC, int RULE>
-__global__ void __launch_bounds__(32 * TileWarps<VEC, RULE>::N, RULE == RULE_EMB ? (VEC == 1 ? 8 : VEC == 2 ? 6 : 3) : (VEC == 2 ? 4 : 2))
+__global__ void __launch_bounds__(32 * TileWarps<VEC, RULE>::N, RULE == RULE_EMB ? (VEC == 2 ? 6 : 3) : (VEC == 2 ? 4 : 2))
 tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys,
                    const unsigned int *__restrict__ vals, float lr, float *__restrict__ psum,
                    long long *__restrict__ hublist, int *__restrict__ hubcnt, ParamJob job, int aside) {
   if (RULE == RULE_EMB) pdl_begin();
   else if (!sibling_begin()) return;
-  constexpr int WARPS = TileWarps<VEC, RULE>::N, STAGE = StageRows<VEC, RULE>::N;
+  constexpr int WARPS = TileWarps<VEC, RULE>::N, STAGE = TILE;
   extern __shared__ __align__(128) float stage_all[];        // [WARPS][STAGE][Dp]
   __shared__ __align__(8) unsigned long long sbar[WARPS];
   const unsigned FULL = 0xffffffffu;
@@ -554,6 +548,188 @@ tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
         hub_biglist(hublist, d.nocc)[atomicAdd(hubcnt + 1, 1)] = head;
     }
     i += nproc;
+  }
+}
+
+// The same for embedding rows of up to 128 floats, two tiles and two rows at a time.  A row of 100 floats is 25 of a warp's 32
+// 16-byte lanes, and what the tile kernel executes is mostly not its arithmetic: segment ballots, slot decoding, pointer and
+// loop bookkeeping, the sum over the warp, a square root and a division, some 400 instructions for each slot's 100 additions
+// (issue slots 58 % busy at 2 % of the DRAM bandwidth, 30 us for 48,000 slots).  Here a half-warp holds a row as two
+// pieces of 64 floats, and the two halves work on two row segments with the same instructions; slots are decoded and segments
+// found one per lane, once for both tiles.  Sums keep their order: lane l of a half has what lanes l and l + 16 have there.
+//
+// A segment is what one of the tile kernel's loops handles: a short row that begins in one of the two tiles, with all its
+// slots, or the part of a hub row inside one tile.
+#define NARROW_STAGE 16
+#define NARROW_WARPS 4
+__global__ void __launch_bounds__(32 * NARROW_WARPS, 6)
+narrow_tile_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys, const unsigned int *__restrict__ vals,
+                   float lr, float *__restrict__ psum, long long *__restrict__ hublist, int *__restrict__ hubcnt, ParamJob job, int aside) {
+  pdl_begin();
+  extern __shared__ __align__(128) float stage_all[];        // [NARROW_WARPS][NARROW_STAGE][Dp]
+  __shared__ __align__(8) unsigned long long sbar[NARROW_WARPS];
+  if (blockIdx.x < aside) { param_sums(d, wb, w, job, blockIdx.x, stage_all); return; }
+  const unsigned FULL = 0xffffffffu;
+  const unsigned long long SENT = ~0ull;
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5, half = lane >> 4, l16 = lane & 15;
+  const int t0 = ((int)(blockIdx.x - aside) * NARROW_WARPS + wl) * 2 * TILE;
+  if (t0 >= d.nocc) return;
+  float *stage = stage_all + (size_t)wl * NARROW_STAGE * d.Dp;
+  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&sbar[wl]);
+  if (lane == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncwarp();
+  const int D = d.D;
+  const float invD = 1.0f / (float)D;
+  // a lane per slot: the window [t0, t0 + 32), and the 32 keys before it
+  const unsigned long long kA = t0 - 32 + lane >= 0 ? keys[t0 - 32 + lane] : SENT;
+  const unsigned long long kB = t0 + lane < d.nocc ? keys[t0 + lane] : SENT;
+  const unsigned int vB = t0 + lane < d.nocc ? vals[t0 + lane] : 0u;
+  const unsigned same = __match_any_sync(FULL, kB);          // equal keys are neighbours
+  const int row0 = __ffs(same) - 1, row_end = 32 - __clz(same);
+  const int back = __clz(~__ballot_sync(FULL, kA == __shfl_sync(FULL, kB, 0)));      // slots of the window's first row before it
+  const bool begins = row0 == lane && (lane > 0 || back == 0);
+  const bool hub = row_end - row0 + (row0 == 0 ? back : 0) > SHORT_MAX;              // (a row that leaves the window has 25 and more slots in it)
+  const bool starts = lane < 2 * TILE && kB < d.key_rel_base && (begins || (hub && (lane & (TILE - 1)) == 0));
+  int count = row_end - lane;                                // slots of the segment that starts here
+  if (hub && count > TILE - (lane & (TILE - 1))) count = TILE - (lane & (TILE - 1));
+  unsigned rest = __ballot_sync(FULL, starts);
+  if (rest == 0) return;
+  const int first = __ffs(rest) - 1;
+  const int last = __reduce_max_sync(FULL, starts ? lane + count : 0);
+  const int staged = last - first < NARROW_STAGE ? last - first : NARROW_STAGE;
+  const int attr = count | (hub ? 64 : 0) | (begins ? 128 : 0);
+  // gradient rows: into shared memory by bulk copies, all in flight together; what finds no room is read where it lies
+  const float *src = nullptr;
+  int bB = 0;
+  if (lane >= first && lane < last) {
+    const Occ oc = occ_decode(d, (int)vB);
+    const float *gbase = (d.matrix_op && oc.a == ARR_N1) ? w.R2 : w.GX[oc.a];
+    src = gbase + ((size_t)oc.blk * w.grows[oc.a] + oc.r) * d.Dp;
+    bB = d.bySpb.div((int)vB);
+  }
+  if (lane == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"((uint32_t)(staged * D * 4)) : "memory");
+  __syncwarp();
+  if (lane >= first && lane < first + staged) {
+    float *to = stage + (size_t)(lane - first) * d.Dp;
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :: "r"((uint32_t)__cvta_generic_to_shared(to)), "l"(src), "r"((uint32_t)(D * 4)), "r"(bar) : "memory");
+    src = to;
+  }
+  // where the rows of the short segments are; each lane of a segment's half, a few of a slot's for the prefetch
+  auto place = [&](unsigned long long key, float *&prow, float *&pacc) {
+    const int side = (!d.shared_table && key >= (unsigned long long)d.n_rows[0]) ? 1 : 0;
+    const size_t row = (size_t)(side ? key - (unsigned long long)d.n_rows[0] : key);
+    prow = w.W[side] + row * D;
+    pacc = w.G[side] + row;
+  };
+  {
+    const int slot = lane >> 2, line = (lane & 3) * 32;      // 2 * TILE slots x four 128-byte lines
+    const unsigned long long key = __shfl_sync(FULL, kB, slot);
+    const int a = __shfl_sync(FULL, starts ? attr : 64, slot);
+    if (!(a & 64) && line < D) {
+      float *prow, *pacc;
+      place(key, prow, pacc);
+      asm volatile("prefetch.global.L2 [%0];" :: "l"(prow + line));
+    }
+  }
+  const int dd0 = l16 * 4, dd1 = 64 + l16 * 4;
+  const bool ok0 = dd0 < D, ok1 = dd1 < D;
+  float4 nv0, nv1;
+  float nG;
+  float *nrow, *nacc;
+  int nstart, nattr;
+  auto next = [&]() {                                        // the next two segments, one a half; their rows requested
+    const int a = __ffs(rest) - 1;
+    rest &= rest - 1;
+    const int b = __ffs(rest) - 1;
+    rest &= rest - 1;
+    nstart = half ? b : a;                                   // -1: none
+    const int at = nstart < 0 ? 0 : nstart;
+    const unsigned long long key = __shfl_sync(FULL, kB, at);
+    nattr = __shfl_sync(FULL, attr, at);
+    if (nstart < 0) nattr = 64;
+    nv0 = nv1 = f4zero(); nG = 0.f;
+    nrow = nacc = nullptr;
+    if (!(nattr & 64)) {
+      place(key, nrow, nacc);
+      if (ok0) nv0 = ld4(nrow + dd0);
+      if (ok1) nv1 = ld4(nrow + dd1);
+      nG = *nacc;
+    }
+  };
+  next();
+  {
+    bool done = false;
+    for (int it = 0; it < UPD_WAIT_LIMIT && !done; ++it) {
+      uint32_t ok;
+      asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(bar), "r"(0u) : "memory");
+      done = ok != 0;
+    }
+    if (!done && lane == 0) atomicOr(w.errflag, 2);
+  }
+  __syncwarp();
+  for (bool more = true; more;) {
+    float4 v0 = nv0, v1 = nv1;
+    float G = nG;
+    float *prow = nrow, *pacc = nacc;
+    const int start = nstart, n = nattr & 63;
+    const bool is_hub = nattr & 64, head = nattr & 128;
+    more = rest != 0;
+    if (more) next();
+    if (d.max_norm > 0.f) {                                  // as RowState::load
+      float ss = f4dot(v0, v0) + f4dot(v1, v1);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(FULL, ss, o);
+      const float norm = sqrtf(ss);
+      if (norm > d.max_norm) {
+        const float sc = d.max_norm / (norm + 1e-7f);
+        v0 = v0 * sc; v1 = v1 * sc;
+      }
+    }
+    const int other = __shfl_xor_sync(FULL, n, 16), most = n > other ? n : other;
+    float4 a0 = f4zero(), a1 = f4zero();
+    int cur = -1, run_start = 0;
+    for (int j = 0; j <= most; ++j) {
+      const int at = (start + j) & 31;
+      const int bs = __shfl_sync(FULL, bB, at);
+      const float *g = (const float *)__shfl_sync(FULL, (unsigned long long)src, at);
+      const int b = j < n ? bs : -1;
+      const bool flush = j <= n && cur >= 0 && b != cur;     // a batch of this row is complete
+      if (__any_sync(FULL, flush && !is_hub)) {
+        float ss = f4dot(a0, a0) + f4dot(a1, a1);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(FULL, ss, o);
+        if (flush && !is_hub) {
+          G += ss * invD;
+          const float stepv = lr / (sqrtf(G) + PBG_ADAGRAD_EPS);
+          v0 = v0 - a0 * stepv; v1 = v1 - a1 * stepv;
+        }
+      }
+      if (flush && is_hub) {
+        float *dst = psum + (size_t)(t0 + run_start) * d.Dp;
+        if (ok0) st4(dst + dd0, a0);
+        if (ok1) st4(dst + dd1, a1);
+      }
+      if (flush) { a0 = f4zero(); a1 = f4zero(); }
+      if (j < n) {
+        if (b != cur) { cur = b; run_start = start + j; }
+        if (ok0) a0 = a0 + ld4(g + dd0);
+        if (ok1) a1 = a1 + ld4(g + dd1);
+      }
+    }
+    if (start >= 0 && !is_hub) {
+      if (ok0) st4(prow + dd0, v0);
+      if (ok1) st4(prow + dd1, v1);
+      if (l16 == 0) *pacc = G;
+    } else if (start >= 0 && head && l16 == 0) {
+      const long long at = t0 + start;
+      hublist[atomicAdd(hubcnt, 1)] = at;
+      // (big rows: see the tile kernel)
+      if (at + HUB_BIG - 1 < (long long)d.nocc && keys[at + HUB_BIG - 1] == keys[at]) hub_biglist(hublist, d.nocc)[atomicAdd(hubcnt + 1, 1)] = at;
+    }
   }
 }
 
@@ -1061,7 +1237,7 @@ template <int VEC>
 static int launch_update_vec(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w,
                              const unsigned long long *keys, const unsigned int *vals, float lr, float rel_lr,
                              const UpdateScratch &us, cudaStream_t st) {
-  constexpr int EMB_WARPS = TileWarps<VEC, RULE_EMB>::N, REL_WARPS = TileWarps<VEC, RULE_REL>::N;
+  constexpr int REL_WARPS = TileWarps<VEC, RULE_REL>::N;
   const long long tiles = ((long long)d.nocc + TILE - 1) / TILE;
   const int hub_ctas = 592;     // (half and twice as many measured the same: the kernel takes as long as its longest row)
   // per-batch totals of one hub row, or eight partial sums of one batch of a big row
@@ -1073,15 +1249,22 @@ static int launch_update_vec(const WaveDims &d, const WaveBatches &wb, const Wav
   // per device (a process may hold contexts on several GPUs); a failed opt-in makes the launch fail,
   // which the caller's cudaGetLastError reports
   pbg_opt_in_smem((const void *)hub_kernel<VEC, RULE_EMB>, (int)hub_smem_max);
-  pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_EMB>, EMB_WARPS * StageRows<VEC, RULE_EMB>::N * VEC * 512);
   ParamJob job;
   int launches = launch_pullback<VEC>(d, wb, w, rel_lr, job, st);
   int *hubcnt = us.hubcnt + 64 * (*us.turn & 1), *hubcnt_next = us.hubcnt + 64 * ((*us.turn + 1) & 1);
   ++*us.turn;
   const int sum_ctas = param_sum_ctas(d, job);
-  size_t tile_smem = (size_t)EMB_WARPS * StageRows<VEC, RULE_EMB>::N * d.Dp * 4;
-  if (sum_ctas && tile_smem < 8 * 128 * 4) tile_smem = 8 * 128 * 4;
-  pbg_launch(tile_update_kernel<VEC, RULE_EMB>, sum_ctas + (unsigned)((tiles + EMB_WARPS - 1) / EMB_WARPS), 32 * EMB_WARPS, tile_smem, st, d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, job, sum_ctas);
+  if (VEC == 1) {
+    const size_t smem = (size_t)NARROW_WARPS * NARROW_STAGE * d.Dp * 4;          // (also enough for param_sums, from a Dp of 32 up)
+    const long long units = ((long long)d.nocc + 2 * TILE - 1) / (2 * TILE);
+    pbg_opt_in_smem((const void *)narrow_tile_kernel, NARROW_WARPS * NARROW_STAGE * 512);
+    pbg_launch(narrow_tile_kernel, sum_ctas + (unsigned)((units + NARROW_WARPS - 1) / NARROW_WARPS), 32 * NARROW_WARPS, smem, st, d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, job, sum_ctas);
+  } else {
+    constexpr int V = VEC == 1 ? 2 : VEC;
+    constexpr int EMB_WARPS = TileWarps<V, RULE_EMB>::N;
+    pbg_opt_in_smem((const void *)tile_update_kernel<V, RULE_EMB>, EMB_WARPS * TILE * V * 512);
+    pbg_launch(tile_update_kernel<V, RULE_EMB>, sum_ctas + (unsigned)((tiles + EMB_WARPS - 1) / EMB_WARPS), 32 * EMB_WARPS, (size_t)EMB_WARPS * TILE * d.Dp * 4, st, d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, job, sum_ctas);
+  }
   const bool rel_rows = d.dynamic && d.op != PBG_OP_NONE && w.theta[0] != nullptr;
   long long *rel_hublist = us.hublist + pbg_hublist_entries(d.nocc), *rel_bigtab = us.bigtab + pbg_bigtab_bytes(d.nocc) / sizeof(long long);
   if (rel_rows) {

@@ -51,3 +51,10 @@ def test_column_tiles_of_both_gradients(D, nb, nu, precision):
 @pytest.mark.parametrize("D", [1024, 1028])
 def test_operator_rows_of_wide_models(D):
     _run(_random_case(8, D, 2000, 300, 50, 20, "translation", "dot", "softmax", dyn=True, R=4, zipf=True), "tf32x3")
+
+
+@pytest.mark.parametrize("D", [4, 64, 68, 128, 132, 192, 196, 256, 260])
+@pytest.mark.parametrize("N,nb,nu", [(9, 30, 5), (150, 40, 11), (6000, 50, 50)])
+def test_update_rows_at_the_half_warp_kernels_widths(D, N, nb, nu):
+    """Hub rows only, short rows across tiles and hubs, and rows of a single slot, at the edges of a half-warp's row."""
+    _run(_random_case(9, D, N, 5 * nb + 2, nb, nu, "none", "dot", "softmax", zipf=N > 10), "tf32x3")
