@@ -560,12 +560,14 @@ tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
 //
 // A segment is what one of the tile kernel's loops handles: a short row that begins in one of the two tiles, with all its
 // slots, or the part of a hub row inside one tile.
-#define NARROW_STAGE 16
 #define NARROW_WARPS 4
-__global__ void __launch_bounds__(32 * NARROW_WARPS, 6)
+template <int NP> struct NarrowStage { enum { N = NP == 2 ? 16 : 8 }; };
+template <int NP>
+__global__ void __launch_bounds__(32 * NARROW_WARPS, NP == 2 ? 6 : 4)
 narrow_tile_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys, const unsigned int *__restrict__ vals,
                    float lr, float *__restrict__ psum, long long *__restrict__ hublist, int *__restrict__ hubcnt, ParamJob job, int aside) {
   pdl_begin();
+  constexpr int NARROW_STAGE = NarrowStage<NP>::N;
   extern __shared__ __align__(128) float stage_all[];        // [NARROW_WARPS][NARROW_STAGE][Dp]
   __shared__ __align__(8) unsigned long long sbar[NARROW_WARPS];
   if (blockIdx.x < aside) { param_sums(d, wb, w, job, blockIdx.x, stage_all); return; }
@@ -626,18 +628,29 @@ narrow_tile_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
     pacc = w.G[side] + row;
   };
   {
-    const int slot = lane >> 2, line = (lane & 3) * 32;      // 2 * TILE slots x four 128-byte lines
+    const int slot = lane >> 2;                              // 2 * TILE slots x four 128-byte lines at a time
     const unsigned long long key = __shfl_sync(FULL, kB, slot);
     const int a = __shfl_sync(FULL, starts ? attr : 64, slot);
-    if (!(a & 64) && line < D) {
+    if (!(a & 64)) {
       float *prow, *pacc;
       place(key, prow, pacc);
-      asm volatile("prefetch.global.L2 [%0];" :: "l"(prow + line));
+      for (int f = (lane & 3) * 32; f < D; f += 128) asm volatile("prefetch.global.L2 [%0];" :: "l"(prow + f));
     }
   }
-  const int dd0 = l16 * 4, dd1 = 64 + l16 * 4;
-  const bool ok0 = dd0 < D, ok1 = dd1 < D;
-  float4 nv0, nv1;
+  bool ok[NP];
+#pragma unroll
+  for (int c = 0; c < NP; ++c) ok[c] = c * 64 + l16 * 4 < D;
+  // |x|^2 of a half's row, summed as the tile kernel's warp does
+  auto square = [&](const float4 (&x)[NP]) {
+    float even = f4dot(x[0], x[0]), odd = f4dot(x[1], x[1]);
+#pragma unroll
+    for (int c = 2; c < NP; c += 2) { even += f4dot(x[c], x[c]); odd += f4dot(x[c + 1], x[c + 1]); }
+    float ss = even + odd;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(FULL, ss, o);
+    return ss;
+  };
+  float4 nv[NP];
   float nG;
   float *nrow, *nacc;
   int nstart, nattr;
@@ -651,12 +664,14 @@ narrow_tile_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
     const unsigned long long key = __shfl_sync(FULL, kB, at);
     nattr = __shfl_sync(FULL, attr, at);
     if (nstart < 0) nattr = 64;
-    nv0 = nv1 = f4zero(); nG = 0.f;
+    nG = 0.f;
     nrow = nacc = nullptr;
+#pragma unroll
+    for (int c = 0; c < NP; ++c) nv[c] = f4zero();
     if (!(nattr & 64)) {
       place(key, nrow, nacc);
-      if (ok0) nv0 = ld4(nrow + dd0);
-      if (ok1) nv1 = ld4(nrow + dd1);
+#pragma unroll
+      for (int c = 0; c < NP; ++c) if (ok[c]) nv[c] = ld4(nrow + c * 64 + l16 * 4);
       nG = *nacc;
     }
   };
@@ -672,7 +687,9 @@ narrow_tile_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
   }
   __syncwarp();
   for (bool more = true; more;) {
-    float4 v0 = nv0, v1 = nv1;
+    float4 v[NP], acc[NP];
+#pragma unroll
+    for (int c = 0; c < NP; ++c) { v[c] = nv[c]; acc[c] = f4zero(); }
     float G = nG;
     float *prow = nrow, *pacc = nacc;
     const int start = nstart, n = nattr & 63;
@@ -680,17 +697,15 @@ narrow_tile_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
     more = rest != 0;
     if (more) next();
     if (d.max_norm > 0.f) {                                  // as RowState::load
-      float ss = f4dot(v0, v0) + f4dot(v1, v1);
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(FULL, ss, o);
+      const float ss = square(v);
       const float norm = sqrtf(ss);
       if (norm > d.max_norm) {
         const float sc = d.max_norm / (norm + 1e-7f);
-        v0 = v0 * sc; v1 = v1 * sc;
+#pragma unroll
+        for (int c = 0; c < NP; ++c) v[c] = v[c] * sc;
       }
     }
     const int other = __shfl_xor_sync(FULL, n, 16), most = n > other ? n : other;
-    float4 a0 = f4zero(), a1 = f4zero();
     int cur = -1, run_start = 0;
     for (int j = 0; j <= most; ++j) {
       const int at = (start + j) & 31;
@@ -699,30 +714,32 @@ narrow_tile_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
       const int b = j < n ? bs : -1;
       const bool flush = j <= n && cur >= 0 && b != cur;     // a batch of this row is complete
       if (__any_sync(FULL, flush && !is_hub)) {
-        float ss = f4dot(a0, a0) + f4dot(a1, a1);
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(FULL, ss, o);
+        const float ss = square(acc);
         if (flush && !is_hub) {
           G += ss * invD;
           const float stepv = lr / (sqrtf(G) + PBG_ADAGRAD_EPS);
-          v0 = v0 - a0 * stepv; v1 = v1 - a1 * stepv;
+#pragma unroll
+          for (int c = 0; c < NP; ++c) v[c] = v[c] - acc[c] * stepv;
         }
       }
       if (flush && is_hub) {
         float *dst = psum + (size_t)(t0 + run_start) * d.Dp;
-        if (ok0) st4(dst + dd0, a0);
-        if (ok1) st4(dst + dd1, a1);
+#pragma unroll
+        for (int c = 0; c < NP; ++c) if (ok[c]) st4(dst + c * 64 + l16 * 4, acc[c]);
       }
-      if (flush) { a0 = f4zero(); a1 = f4zero(); }
+      if (flush) {
+#pragma unroll
+        for (int c = 0; c < NP; ++c) acc[c] = f4zero();
+      }
       if (j < n) {
         if (b != cur) { cur = b; run_start = start + j; }
-        if (ok0) a0 = a0 + ld4(g + dd0);
-        if (ok1) a1 = a1 + ld4(g + dd1);
+#pragma unroll
+        for (int c = 0; c < NP; ++c) if (ok[c]) acc[c] = acc[c] + ld4(g + c * 64 + l16 * 4);
       }
     }
     if (start >= 0 && !is_hub) {
-      if (ok0) st4(prow + dd0, v0);
-      if (ok1) st4(prow + dd1, v1);
+#pragma unroll
+      for (int c = 0; c < NP; ++c) if (ok[c]) st4(prow + c * 64 + l16 * 4, v[c]);
       if (l16 == 0) *pacc = G;
     } else if (start >= 0 && head && l16 == 0) {
       const long long at = t0 + start;
@@ -1254,13 +1271,14 @@ static int launch_update_vec(const WaveDims &d, const WaveBatches &wb, const Wav
   int *hubcnt = us.hubcnt + 64 * (*us.turn & 1), *hubcnt_next = us.hubcnt + 64 * ((*us.turn + 1) & 1);
   ++*us.turn;
   const int sum_ctas = param_sum_ctas(d, job);
-  if (VEC == 1) {
-    const size_t smem = (size_t)NARROW_WARPS * NARROW_STAGE * d.Dp * 4;          // (also enough for param_sums, from a Dp of 32 up)
+  if (VEC <= 2) {
+    constexpr int NP = VEC == 1 ? 2 : 4, STAGE = NarrowStage<NP>::N;
+    const size_t smem = (size_t)NARROW_WARPS * STAGE * d.Dp * 4;                 // (also enough for param_sums, from a Dp of 32 up)
     const long long units = ((long long)d.nocc + 2 * TILE - 1) / (2 * TILE);
-    pbg_opt_in_smem((const void *)narrow_tile_kernel, NARROW_WARPS * NARROW_STAGE * 512);
-    pbg_launch(narrow_tile_kernel, sum_ctas + (unsigned)((units + NARROW_WARPS - 1) / NARROW_WARPS), 32 * NARROW_WARPS, smem, st, d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, job, sum_ctas);
+    pbg_opt_in_smem((const void *)narrow_tile_kernel<NP>, NARROW_WARPS * STAGE * VEC * 512);
+    pbg_launch(narrow_tile_kernel<NP>, sum_ctas + (unsigned)((units + NARROW_WARPS - 1) / NARROW_WARPS), 32 * NARROW_WARPS, smem, st, d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, job, sum_ctas);
   } else {
-    constexpr int V = VEC == 1 ? 2 : VEC;
+    constexpr int V = VEC <= 2 ? 4 : VEC;
     constexpr int EMB_WARPS = TileWarps<V, RULE_EMB>::N;
     pbg_opt_in_smem((const void *)tile_update_kernel<V, RULE_EMB>, EMB_WARPS * TILE * V * 512);
     pbg_launch(tile_update_kernel<V, RULE_EMB>, sum_ctas + (unsigned)((tiles + EMB_WARPS - 1) / EMB_WARPS), 32 * EMB_WARPS, (size_t)EMB_WARPS * TILE * d.Dp * 4, st, d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, job, sum_ctas);
