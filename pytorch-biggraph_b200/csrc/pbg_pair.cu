@@ -230,16 +230,15 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
           }
           live[c] = m;
         }
-        auto masked = [&](int c, int jj) { return ((live[c] >> jj) & 1u) == 0u; };
+        auto masked = [&](int c, int jj) { return (((c ? live[1] : live[0]) >> jj) & 1u) == 0u; };
         uint32_t r[32];
         float lossv = 0.f, ds = 0.f, scale = 0.f;
         int viol = 0;
         if (d.loss == PBG_LOSS_SOFTMAX) {
           // -s + log(e^s + sum_j e^S_ij), masked entries are e^-1e9 = 0 (losses.py:143-159)
           float mx = -INFINITY;
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            if (c >= nch) break;
+#pragma unroll 1
+          for (int c = 0; c < nch; ++c) {
             tmem_ld32(trow + (uint32_t)c * 32u, r);
 #pragma unroll
             for (int jj = 0; jj < 32; ++jj) {
@@ -256,9 +255,8 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
           float m = fmaxf(mx, s);
           if (mx == -INFINITY) m = fmaxf(s, PBG_MASKED);         // every column masked
           float z = 0.f;
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            if (c >= nch) break;
+#pragma unroll 1
+          for (int c = 0; c < nch; ++c) {
             tmem_ld32(trow + (uint32_t)c * 32u, r);
 #pragma unroll
             for (int jj = 0; jj < 32; ++jj) {
@@ -276,9 +274,8 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
           else viol = 0;                                          // losses.py:139-140: no negatives, loss 0, no gradient
         } else if (d.loss == PBG_LOSS_RANKING) {
           // sum_j max(0, margin - s + S_ij) (losses.py:116-122); the scores are replaced by the 0 / 1 indicator of an active column
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            if (c >= nch) break;
+#pragma unroll 1
+          for (int c = 0; c < nch; ++c) {
             tmem_ld32(trow + (uint32_t)c * 32u, r);
 #pragma unroll
             for (int jj = 0; jj < 32; ++jj) {
@@ -302,9 +299,8 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
         } else {
           // softplus(-s) + (1/M) sum_j softplus(S_ij), M counts masked columns (losses.py:61-80); the scores are replaced by sigmoid(S)
           const float nw = Mlog > 0 ? 1.0f / (float)Mlog : 0.f;
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            if (c >= nch) break;
+#pragma unroll 1
+          for (int c = 0; c < nch; ++c) {
             tmem_ld32(trow + (uint32_t)c * 32u, r);
 #pragma unroll
             for (int jj = 0; jj < 32; ++jj) {
@@ -326,7 +322,7 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
         // ---- coefficient row: planes into TB[p][i][:] (16-byte stores) ----
         unsigned short *tb = w.TB[p] + ((size_t)blk * NPL * Pm + (i < Pm ? i : 0)) * w.Kb;
         const size_t tb_plane = (size_t)Pm * w.Kb;
-#pragma unroll
+#pragma unroll 1
         for (int c = 0; c < 2; ++c) {
           if (c >= nch) break;
           tmem_ld32(trow + (uint32_t)c * 32u, r);
