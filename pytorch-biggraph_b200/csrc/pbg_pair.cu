@@ -9,7 +9,7 @@
 // block crosses L2 -> shared memory once per k-stage instead of 1.5 times, and one CTA ends up with the
 // score rows of both problems in tensor memory (two accumulators of up to 256 columns).
 //
-// Epilogue (sixteen warps, four threads per positive row i, each with two 32-column chunks of the row): what loss_kernel / loss_softmax_kernel do for a
+// Epilogue (sixteen warps, four threads per positive row i, each with four 16-column chunks of the row): what loss_kernel / loss_softmax_kernel do for a
 // row, straight from tensor memory -- masks (model.py:566-580, 836-844), logistic / ranking / softmax
 // (losses.py:53-161), relation and edge weight (batching.py:139-150), violators (train_cpu.py:98-99) --
 // and the coefficient rows T_p[i][:] = d(loss)/d(score) with the positive pair in the diagonal, written
@@ -36,13 +36,18 @@ struct PairGeom {
 __device__ __forceinline__ float pair_softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
 __device__ __forceinline__ float pair_sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }
 
-// 32 columns of this thread's tensor-memory lane back (the epilogue keeps per-score intermediates there)
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-               :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-                  "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
-                  "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]),
-                  "r"(r[30]), "r"(r[31]) : "memory");
+// 16 columns of this thread's tensor-memory lane, and back (the epilogue keeps per-score intermediates there).  The epilogue
+// works in chunks of 16 in a loop: every warp runs it a few times per block, so the code's size counts -- unrolled over two
+// chunks of 32 a fifth of the warps' time went into waiting for instructions (a wave of 140 blocks of 100 columns, ranking: 44.7 us,
+// 41.3 with the two chunks in a loop, 38.6 so) -- and the last chunk of a row has less beyond its end.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
@@ -210,7 +215,7 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
         const float s = row_valid ? w.spos[p][prow] : 0.f;
         const int col0 = cg * 64;                                // first column of this warp's part of the row
         const uint32_t trow = tmem + (uint32_t)(j % SETS) * 2u * ACC + (uint32_t)p * ACC + ((uint32_t)(q * 32) << 16) + (uint32_t)col0;
-        const int nch = col0 >= w.Kb ? 0 : (col0 + 32 >= w.Kb ? 1 : 2);      // chunks of this warp that hold coefficient columns
+        const int nch = col0 >= w.Kb ? 0 : (w.Kb - col0 < 64 ? w.Kb - col0 + 15 : 64) / 16;      // chunks of this warp that hold coefficient columns
         // Which columns of this warp's chunks count for this row (model.py:566-580): bit jj of live[c] is set when
         // column col0 + 32 c + jj exists (< Mm) and is not ignored -- uniform negatives (>= Pm) never are; a batch
         // negative is when the mode has none, when it is the row's own positive, or padding of the last chunk.
@@ -230,8 +235,8 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
           }
           live[c] = m;
         }
-        auto masked = [&](int c, int jj) { return (((c ? live[1] : live[0]) >> jj) & 1u) == 0u; };
-        uint32_t r[32];
+        auto masked = [&](int c, int jj) { return (((c & 2 ? live[1] : live[0]) >> ((c & 1) * 16 + jj)) & 1u) == 0u; };
+        uint32_t r[16];
         float lossv = 0.f, ds = 0.f, scale = 0.f;
         int viol = 0;
         if (d.loss == PBG_LOSS_SOFTMAX) {
@@ -239,9 +244,9 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
           float mx = -INFINITY;
 #pragma unroll 1
           for (int c = 0; c < nch; ++c) {
-            tmem_ld32(trow + (uint32_t)c * 32u, r);
+            tmem_ld16(trow + (uint32_t)c * 16u, r);
 #pragma unroll
-            for (int jj = 0; jj < 32; ++jj) {
+            for (int jj = 0; jj < 16; ++jj) {
               const float sv = __uint_as_float(r[jj]);
               if (!masked(c, jj)) { mx = fmaxf(mx, sv); viol += sv > s; }
             }
@@ -257,14 +262,14 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
           float z = 0.f;
 #pragma unroll 1
           for (int c = 0; c < nch; ++c) {
-            tmem_ld32(trow + (uint32_t)c * 32u, r);
+            tmem_ld16(trow + (uint32_t)c * 16u, r);
 #pragma unroll
-            for (int jj = 0; jj < 32; ++jj) {
+            for (int jj = 0; jj < 16; ++jj) {
               const float e = masked(c, jj) ? 0.f : __expf(__uint_as_float(r[jj]) - m);
               r[jj] = __float_as_uint(e);                        // kept in tensor memory: the coefficient is scale * e
               z += e;
             }
-            tmem_st32(trow + (uint32_t)c * 32u, r);
+            tmem_st16(trow + (uint32_t)c * 16u, r);
           }
           red_f[1][p][cg][i] = z;
           epi_sync();
@@ -276,9 +281,9 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
           // sum_j max(0, margin - s + S_ij) (losses.py:116-122); the scores are replaced by the 0 / 1 indicator of an active column
 #pragma unroll 1
           for (int c = 0; c < nch; ++c) {
-            tmem_ld32(trow + (uint32_t)c * 32u, r);
+            tmem_ld16(trow + (uint32_t)c * 16u, r);
 #pragma unroll
-            for (int jj = 0; jj < 32; ++jj) {
+            for (int jj = 0; jj < 16; ++jj) {
               const float sj = __uint_as_float(r[jj]);
               float act = 0.f;
               if (Mlog > 0 && !masked(c, jj)) {
@@ -288,7 +293,7 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
               }
               r[jj] = __float_as_uint(act);
             }
-            tmem_st32(trow + (uint32_t)c * 32u, r);
+            tmem_st16(trow + (uint32_t)c * 16u, r);
           }
           red_f[0][p][cg][i] = lossv; red_f[1][p][cg][i] = ds; red_i[p][cg][i] = viol;
           epi_sync();
@@ -301,15 +306,15 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
           const float nw = Mlog > 0 ? 1.0f / (float)Mlog : 0.f;
 #pragma unroll 1
           for (int c = 0; c < nch; ++c) {
-            tmem_ld32(trow + (uint32_t)c * 32u, r);
+            tmem_ld16(trow + (uint32_t)c * 16u, r);
 #pragma unroll
-            for (int jj = 0; jj < 32; ++jj) {
+            for (int jj = 0; jj < 16; ++jj) {
               const float sj = __uint_as_float(r[jj]);
               float sg = 0.f;
               if (!masked(c, jj)) { viol += sj > s; lossv += pair_softplus(sj); sg = pair_sigmoid(sj); }
               r[jj] = __float_as_uint(sg);
             }
-            tmem_st32(trow + (uint32_t)c * 32u, r);
+            tmem_st16(trow + (uint32_t)c * 16u, r);
           }
           red_f[0][p][cg][i] = lossv; red_i[p][cg][i] = viol;
           epi_sync();
@@ -323,15 +328,14 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
         unsigned short *tb = w.TB[p] + ((size_t)blk * NPL * Pm + (i < Pm ? i : 0)) * w.Kb;
         const size_t tb_plane = (size_t)Pm * w.Kb;
 #pragma unroll 1
-        for (int c = 0; c < 2; ++c) {
-          if (c >= nch) break;
-          tmem_ld32(trow + (uint32_t)c * 32u, r);
+        for (int c = 0; c < nch; ++c) {
+          tmem_ld16(trow + (uint32_t)c * 16u, r);
 #pragma unroll
-          for (int g8 = 0; g8 < 4; ++g8) {
+          for (int g8 = 0; g8 < 2; ++g8) {
             unsigned pk[3][4];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-              const int jj = g8 * 8 + u, jc = col0 + c * 32 + jj;
+              const int jj = g8 * 8 + u, jc = col0 + c * 16 + jj;
               float tv = row_valid ? scale * __uint_as_float(r[jj]) : 0.f;        // masked columns hold 0
               if (row_valid && jc == i) tv = tdiag;
               unsigned b0, b1, b2;
@@ -339,7 +343,7 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
               if (u & 1) { pk[0][u >> 1] |= b0 << 16; pk[1][u >> 1] |= b1 << 16; pk[2][u >> 1] |= b2 << 16; }
               else { pk[0][u >> 1] = b0; pk[1][u >> 1] = b1; pk[2][u >> 1] = b2; }
             }
-            const int j0 = col0 + c * 32 + g8 * 8;
+            const int j0 = col0 + c * 16 + g8 * 8;
             if (i < Pm && j0 < w.Kb) {
 #pragma unroll
               for (int pl = 0; pl < NPL; ++pl)
