@@ -145,16 +145,15 @@ static int chunk_geometry(const pbg_config &cfg, int *Pm, int *Cm) {
 // loss, merged coefficients, gradient).  The fused kernel gives a chunk block to one CTA, its loss included: fewer and
 // shorter launches where the blocks of a full wave fill the SMs, a long single epilogue where they do not.  Measured time
 // of the separate kernels over that of the fused ones (whole buckets, 50 to 200 score columns, dimensions 64 / 256 / 512 / 1024):
-//   softmax   12 to 24 blocks 0.85-1.0 (any dimension); 32 and more: three planes 1.1 / 1.03 / 0.98 / 0.96,
-//             two planes 1.15 / 1.09 / 1.05 / 1.01 (512 below 72 blocks: 0.98)
-//   logistic  (log1p and exp of every score in the epilogue) 0.65-0.98, but two planes up to dimension 128 on
-//             nearly full rounds of CTAs 1.04-1.13
+//   softmax   12 to 24 blocks 0.8-1.0 (any dimension); 80 to 280: three planes 1.15 / 1.09 / 1.02 / 0.99, two planes 1.25 / 1.16 /
+//             1.08 / 1.03; 32 and 60: three planes 1.15 / 1.0 / 0.94, two planes 1.15 / 1.09 / 1.02
+//   logistic  (log1p and exp of every score in the epilogue) 12 to 60 blocks 0.73-1.0; 80 to 280: three planes 1.1 / 1.03 /
+//             0.99 / 0.97, two planes 1.17 / 1.1 / 1.05 / 1.0
 // Ranking keeps to the dimension alone: hinges turn the two forms' different roundings into different trajectories.
 static bool fused_pays(const pbg_config &cfg, int npl, long long blocks) {
   if (cfg.loss == PBG_LOSS_RANKING) return cfg.dim <= 256;
-  if (cfg.loss == PBG_LOSS_SOFTMAX) return blocks > 24 && (cfg.dim <= 256 || (npl == 2 && cfg.dim <= 512 && blocks >= 72));
-  const long long sms = pbg_sm_count(), rounds = (blocks + sms - 1) / sms;
-  return npl == 2 && cfg.dim <= 128 && 4 * blocks >= 3 * rounds * sms;
+  if (cfg.loss == PBG_LOSS_SOFTMAX) return blocks > 24 && cfg.dim <= (blocks < 72 ? 256 : npl == 2 ? 1024 : 512);
+  return blocks >= 72 && cfg.dim <= (npl == 2 ? 512 : 256);
 }
 
 extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_context **out) {
