@@ -311,7 +311,12 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
             for (int jj = 0; jj < 16; ++jj) {
               const float sj = __uint_as_float(r[jj]);
               float sg = 0.f;
-              if (!masked(c, jj)) { viol += sj > s; lossv += pair_softplus(sj); sg = pair_sigmoid(sj); }
+              if (!masked(c, jj)) {
+                const float e = expf(-fabsf(sj));                 // one exponential for softplus and sigmoid
+                viol += sj > s;
+                lossv += fmaxf(sj, 0.f) + log1pf(e);
+                sg = (sj >= 0.f ? 1.0f : e) / (1.0f + e);
+              }
               r[jj] = __float_as_uint(sg);
             }
             tmem_st16(trow + (uint32_t)c * 16u, r);
