@@ -551,12 +551,13 @@ tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
   }
 }
 
-// The same for embedding rows of up to 128 floats, two tiles and two rows at a time.  A row of 100 floats is 25 of a warp's 32
+// The same for embedding rows of up to 256 floats, two tiles and two rows at a time.  A row of 100 floats is 25 of a warp's 32
 // 16-byte lanes, and what the tile kernel executes is mostly not its arithmetic: segment ballots, slot decoding, pointer and
 // loop bookkeeping, the sum over the warp, a square root and a division, some 400 instructions for each slot's 100 additions
-// (issue slots 58 % busy at 2 % of the DRAM bandwidth, 30 us for 48,000 slots).  Here a half-warp holds a row as two
+// (issue slots 58 % busy at 2 % of the DRAM bandwidth, 30 us for 48,000 slots).  Here a half-warp holds a row as NP
 // pieces of 64 floats, and the two halves work on two row segments with the same instructions; slots are decoded and segments
-// found one per lane, once for both tiles.  Sums keep their order: lane l of a half has what lanes l and l + 16 have there.
+// found one per lane, once for both tiles.  Tiles and hubs of such a wave together: 54 us before, 49 so.  Sums keep their
+// order: lane l of a half has what lanes l and l + 16 have there.
 //
 // A segment is what one of the tile kernel's loops handles: a short row that begins in one of the two tiles, with all its
 // slots, or the part of a hub row inside one tile.
