@@ -192,6 +192,9 @@ int launch_iota_keys(const long long *rows, long long num_rows, int n, unsigned 
 
 struct SortRows { const long long *rows; long long num_rows; int n; unsigned long long *keys; unsigned int *vals; int *errflag; };
 
+// Another CTA's shared memory may be written only once that CTA is known to run.  The kernels therefore arrive at the
+// cluster's barrier first thing, and the wait that belongs to it stands in front of the first remote store; the key build
+// and the first ranking lie between the two.
 template <int IPT>
 __device__ __forceinline__ void cluster_sort_body(uint2 (&item)[IPT], int n, int bits, unsigned long long *keys_out, unsigned int *vals_out,
                                                   unsigned char *smem) {
@@ -225,6 +228,7 @@ __device__ __forceinline__ void cluster_sort_body(uint2 (&item)[IPT], int n, int
       off[i] = before + __popc(peers & lt);
     }
     __syncthreads();
+    if (pass == 0) cluster.barrier_wait();                              // every CTA of the cluster runs: its shared memory may be written
     if (t < bins) {
       unsigned int run = 0u, c[CS_WARPS];
 #pragma unroll
@@ -278,6 +282,7 @@ template <int IPT>
 __global__ void __launch_bounds__(CS_THREADS, 1)
 sort_waves_kernel(WaveDims d, WaveBufs w, const __grid_constant__ SortWaves waves, int bits) {
   extern __shared__ __align__(16) unsigned char cs_smem[];
+  cg::this_cluster().barrier_arrive();
   const int nct = (int)cg::this_cluster().num_blocks(), rank = (int)cg::this_cluster().block_rank();
   const SortWave &sw = waves.w[blockIdx.x / nct];
   const int n = sw.k * d.spb;
@@ -294,6 +299,7 @@ sort_waves_kernel(WaveDims d, WaveBufs w, const __grid_constant__ SortWaves wave
 template <int IPT>
 __global__ void __launch_bounds__(CS_THREADS, 1) sort_rows_kernel(SortRows a, int bits) {
   extern __shared__ __align__(16) unsigned char cs_smem[];
+  cg::this_cluster().barrier_arrive();
   const int first = (int)cg::this_cluster().block_rank() * CS_THREADS * IPT + (threadIdx.x >> 5) * 32 * IPT + (threadIdx.x & 31);
   uint2 item[IPT];
 #pragma unroll
