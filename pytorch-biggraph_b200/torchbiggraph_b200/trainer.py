@@ -24,6 +24,10 @@ def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()
 
 
+# Device index -> handle of PyTorch's current stream.  (The public form is the same at 3 us a call, which a call of 50 us shows.)
+_current_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
+
+
 # the C structures pbg_batch and pbg_batch_stats as array records
 _BATCH = np.dtype([("offset", np.int64), ("count", np.int32), ("rel", np.int32)])
 _STATS = np.dtype([("loss", np.float32), ("reg", np.float32), ("violators_lhs", np.int64), ("violators_rhs", np.int64), ("count", np.int64)])
@@ -74,8 +78,9 @@ class _Native:
         self.device_index = model.device.index if model.device.index is not None else torch.cuda.current_device()
         self._bucket, self._bucket_key = None, ()
         self.ctx = C.c_void_p()
-        stream = torch.cuda.current_stream(self.device_index).cuda_stream
-        st = self.lib.pbg_create(C.byref(c), self.device_index, C.c_void_p(stream), C.byref(self.ctx))
+        self.stream = torch.cuda.current_stream(self.device_index)      # the library's, whatever is current at later calls
+        self.stream_handle = self.stream.cuda_stream
+        st = self.lib.pbg_create(C.byref(c), self.device_index, C.c_void_p(self.stream_handle), C.byref(self.ctx))
         if st != 0:
             msg = self.lib.pbg_last_error(self.ctx).decode() if self.ctx else ""
             self.lib.pbg_destroy(self.ctx)
@@ -88,6 +93,19 @@ class _Native:
         if getattr(self, "ctx", None):
             self.lib.pbg_destroy(self.ctx)
             self.ctx = None
+
+    def ordered(self, fn, *args) -> int:
+        """fn(context, *args), in step with the caller's current stream: behind what PyTorch has queued there (the copies
+        and index kernels that made the arguments, the last use of memory handed out for outputs) and in front of what it
+        queues next (temporaries among the arguments go back to its allocator, tables are read)."""
+        if _current_stream(self.device_index) == self.stream_handle:
+            return fn(self.ctx, *args)
+        current = torch.cuda.current_stream(self.device_index)
+        self.stream.wait_stream(current)
+        try:
+            return fn(self.ctx, *args)
+        finally:
+            current.wait_stream(self.stream)
 
     def set_hyper(self, lr, relation_lr, margin):
         check(self.lib.pbg_set_hyperparameters(self.ctx, lr, lr if relation_lr is None else relation_lr, margin), self.ctx)
@@ -144,8 +162,8 @@ class _Native:
         ul = None if ul is None else self._uniform(ul, dev)
         ur = None if ur is None else self._uniform(ur, dev)
         b = self.bucket(model, relidx, None, None)
-        check(self.lib.pbg_score_batch(self.ctx, C.byref(b), _ptr(lhs), _ptr(rhs), _ptr(rel), n, local,
-                                       _ptr(ul), _ptr(ur), seed, _ptr(lp), _ptr(rp), _ptr(ln), _ptr(rn)), self.ctx)
+        check(self.ordered(self.lib.pbg_score_batch, C.byref(b), _ptr(lhs), _ptr(rhs), _ptr(rel), n, local,
+                           _ptr(ul), _ptr(ur), seed, _ptr(lp), _ptr(rp), _ptr(ln), _ptr(rn)), self.ctx)
         return Scores(lp, rp, ln, rn)
 
     def _uniform(self, u, dev):
@@ -318,8 +336,8 @@ class B200Trainer(AbstractBatchProcessor):
                 raise ValueError("one weight per edge is needed")
             weights = weights.to(device=model.device, dtype=torch.float32).contiguous()     # kept alive until the call returns
             check(nat.lib.pbg_set_edge_weights(nat.ctx, _ptr(weights)), nat.ctx)
-        check(fn(nat.ctx, C.byref(bucket), _ptr(lhs), _ptr(rhs), _ptr(rel), lhs.shape[0], batches, num_batches,
-                 _ptr(uniform_lhs), _ptr(uniform_rhs), self.seed + self._calls, stats), nat.ctx)
+        check(nat.ordered(fn, C.byref(bucket), _ptr(lhs), _ptr(rhs), _ptr(rel), lhs.shape[0], batches, num_batches,
+                          _ptr(uniform_lhs), _ptr(uniform_rhs), self.seed + self._calls, stats), nat.ctx)
 
     def read_stats(self) -> Stats:
         s = PbgBatchStats()
@@ -423,14 +441,14 @@ class B200RankingEvaluator(AbstractBatchProcessor):
             check(nat.lib.pbg_set_edge_weights(nat.ctx, _ptr(wgt)), nat.ctx)
         if model.relations[0 if dyn else full_r].all_negs:
             # every entity of a side's table is a negative (model.py:582-617): ranks among the whole partition
-            st = nat.lib.pbg_eval_batch_all_negs(nat.ctx, C.byref(bucket), _ptr(lhs), _ptr(rhs), _ptr(rel), n, r,
-                                                 self.seed + self._calls, C.byref(out))
+            st = nat.ordered(nat.lib.pbg_eval_batch_all_negs, C.byref(bucket), _ptr(lhs), _ptr(rhs), _ptr(rel), n, r,
+                             self.seed + self._calls, C.byref(out))
             if st == _lib.PBG_ERR_UNSUPPORTED:
                 raise NotImplementedError(nat.lib.pbg_last_error(nat.ctx).decode())
             check(st, nat.ctx)
         else:
-            check(nat.lib.pbg_eval_batch(nat.ctx, C.byref(bucket), _ptr(lhs), _ptr(rhs), _ptr(rel), n, r, _ptr(ul), _ptr(ur),
-                                         self.seed + self._calls, C.byref(out)), nat.ctx)
+            check(nat.ordered(nat.lib.pbg_eval_batch, C.byref(bucket), _ptr(lhs), _ptr(rhs), _ptr(rel), n, r, _ptr(ul), _ptr(ur),
+                              self.seed + self._calls, C.byref(out)), nat.ctx)
         return Stats(loss=float(out.loss), pos_rank=out.pos_rank, mrr=out.mrr, r1=out.r1, r10=out.r10, r50=out.r50,
                      auc=out.auc, count=int(out.count))
 
