@@ -909,11 +909,14 @@ int launch_allnegs_eval(const WaveDims &d, const WaveBufs &w, char *mem, int max
   for (long long row0 = 0; row0 == 0 || row0 < most; row0 += slab) {
     const int n = (int)(most - row0 < slab ? most - row0 : slab);
     const int sctas = (n + GATHER_WARPS - 1) / GATHER_WARPS, first = row0 == 0, last = row0 + slab >= most;
-    AN_V(allnegs_slab_kernel, dim3(sctas + (first ? ectas : 0), 2), 32 * GATHER_WARPS, 0, st, d, w, a, row0, rel_std, sctas, first);
-    if (planes) launch_allnegs_score_tc(d, w, a, row0, st);
-    else pbg_launch(allnegs_score_kernel, dim3((B + AN_TILE - 1) / AN_TILE, (n + AN_TILE - 1) / AN_TILE, 2), 256, 0, st, d, w, a, row0);
+    if (n > 0) {                                              // (neither side has negatives: no candidates, and zeros from the merge)
+      AN_V(allnegs_slab_kernel, dim3(sctas + (first ? ectas : 0), 2), 32 * GATHER_WARPS, 0, st, d, w, a, row0, rel_std, sctas, first);
+      if (planes) launch_allnegs_score_tc(d, w, a, row0, st);
+      else pbg_launch(allnegs_score_kernel, dim3((B + AN_TILE - 1) / AN_TILE, (n + AN_TILE - 1) / AN_TILE, 2), 256, 0, st, d, w, a, row0);
+      launches += 2;
+    }
     pbg_launch(allnegs_merge_kernel, (2 * B + GATHER_WARPS - 1) / GATHER_WARPS, 32 * GATHER_WARPS, 0, st, d, w, a, row0, first, last, wrel, out8);
-    launches += 3;
+    ++launches;
   }
 #undef AN_V
   pbg_note_launch();

@@ -8,11 +8,11 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _stats(rows, D, B, comp, loss, precision, seed=3):
+def _stats(rows, D, B, comp, loss, precision, seed=3, **options):
     import torchbiggraph_b200 as T
     g = torch.Generator().manual_seed(seed)
     cfg = T.ConfigSchema(entities={"e": T.EntitySchema()}, relations=[T.RelationSchema("r", "e", "e", operator="translation", all_negs=True)],
-                         dimension=D, comparator=comp, loss_fn=loss, batch_size=200, num_batch_negs=50, num_uniform_negs=50, precision=precision)
+                         dimension=D, comparator=comp, loss_fn=loss, batch_size=200, num_batch_negs=50, num_uniform_negs=50, precision=precision, **options)
     m = T.make_model(cfg, "cuda")
     W = (torch.randn(rows, D, generator=g) * D ** -0.5)
     t = torch.randn(1, D, generator=g) * 0.3 * D ** -0.5
@@ -47,3 +47,24 @@ def test_ranks_agree_with_double_precision(rows, D, B, comp, loss):
         assert abs(s.metrics["pos_rank"] - total / 2) <= max(1.0, 2e-4 * total), (p, s.metrics["pos_rank"], total / 2)
         np.testing.assert_allclose(s.metrics["loss"], got["fp32"][0].metrics["loss"], rtol=2e-5)
         assert abs(s.metrics["auc"] - got["fp32"][0].metrics["auc"]) <= 1.0
+
+
+@pytest.mark.parametrize("precision", ["fp32", "tf32x3", "bf16x3"])
+@pytest.mark.parametrize("off", [("lhs",), ("rhs",), ("lhs", "rhs")], ids="+".join)
+def test_sides_without_negatives_count_for_nothing(precision, off):
+    """Neither side: no candidates, so no slab and no score tile is launched, and every sum is zero.  One side: the averages of the
+    evaluator are the other side's."""
+    options = {f"disable_{side}_negs": True for side in off}
+    s, W, t, lhs, rhs = _stats(300, 36, 70, "dot", "softmax", precision, **options)
+    assert s.count == 70
+    if len(off) == 2:
+        assert all(s.metrics[m] == 0 for m in ("loss", "pos_rank", "mrr", "r1", "r10", "r50", "auc"))
+        return
+    X, Y = W, W + t
+    S, true = (Y[rhs] @ X.T, lhs) if off == ("rhs",) else (X[lhs] @ Y.T, rhs)
+    i = torch.arange(70)
+    pos = S[i, true].clone()
+    np.testing.assert_allclose(s.metrics["loss"], float((torch.logsumexp(S, 1) - pos).sum()), rtol=1e-5)
+    S[i, true] = -float("inf")
+    total = float((1 + (S >= pos[:, None]).sum(1)).sum())
+    assert abs(s.metrics["pos_rank"] - total) <= 1.0
