@@ -43,7 +43,6 @@ struct pbg_context {
   void *tcplan = nullptr;       // tensor maps of the tcgen05 contractions
   void *pairplan = nullptr;     // tensor maps of the fused score + loss kernel (standard relations, plane tiers)
   bool fused = false;           // training runs gather -> fused score / loss -> dual gradient product
-  bool fused_halves = false;    // ... as two halves of the wave on two streams (PBG_HALVES=1; for comparisons)
   float *psum = nullptr;        // partial gradient rows of hub rows, indexed by slot position
   long long *hublist = nullptr;
   int *hubcnt = nullptr;        // two sets of counters, used in turn
@@ -239,8 +238,6 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
     const char *env = getenv("PBG_FUSED");
     const bool eligible = planes && !dyn && !matrix_op && cfg->comparator < PBG_CMP_L2 && c->Pm <= 128 && c->Mm <= 256;
     c->fused = eligible && (env && (env[0] == '0' || env[0] == '1') ? env[0] == '1' : fused_pays(*cfg, npl, (long long)c->kmax * c->Cm));
-    const char *envh = getenv("PBG_HALVES");
-    c->fused_halves = envh && envh[0] == '1';
     const char *envk = getenv("PBG_SPLIT_MIN_K");
     if (envk && atoi(envk) >= 2) c->split_min_k = atoi(envk);
   }
@@ -634,7 +631,7 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
     // kernels can run as two independent halves on two streams: the memory-bound kernels of one
     // half fill the SMs' idle issue slots while the other half's contractions run.
     d.blk0 = 0;
-    if (c->fused && !c->fused_halves) {
+    if (c->fused) {
       // the fused score kernel computes both problems of a chunk block in one CTA: a wave of 14 batches of 10
       // chunks is one round of 140 CTAs, where its halves would each leave half of the SMs idle
       run_part(c, d, wb, w, c->stream);

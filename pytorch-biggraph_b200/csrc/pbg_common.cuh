@@ -288,16 +288,6 @@ __device__ __forceinline__ float4 operator*(float4 a, float s) { return make_flo
 __device__ __forceinline__ float f4dot(float4 a, float4 b) { return __fmaf_rn(a.w, b.w, __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x)))); }
 __device__ __forceinline__ float f4dot_yx(float4 a, float4 b) { return __fmaf_rn(a.w, b.w, __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)))); }
 __device__ __forceinline__ float f4sum(float4 a) { return a.x + a.y + a.z + a.w; }
-// tf32(x): round to nearest, 10 mantissa bits kept -- the part of x a kind::tf32 MMA sees exactly
-__device__ __forceinline__ float tf32_hi(float x) {
-  uint32_t u;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(x));
-  return __uint_as_float(u);
-}
-__device__ __forceinline__ float4 tf32_hi4(float4 v) { return make_float4(tf32_hi(v.x), tf32_hi(v.y), tf32_hi(v.z), tf32_hi(v.w)); }
-// The same rounding with two integer instructions (add half an ulp of the 10-bit mantissa, clear the
-// low 13 bits): cvt runs at a fraction of the ALU rate, which is what bounds a kernel that splits
-// whole operand tiles.  Differs from cvt only on NaN payloads and when rounding carries into Inf.
 // The three bf16 planes of x (round to nearest each time; the remainders are exact in fp32):
 // float(b0) + float(b1) + float(b2) == x to 24 mantissa bits.
 __device__ __forceinline__ void bf16_planes(float x, unsigned &b0, unsigned &b1, unsigned &b2) {
@@ -322,6 +312,10 @@ __device__ __forceinline__ void put_planes1(unsigned short *dst, size_t plane, f
   dst[0] = (unsigned short)b0; dst[plane] = (unsigned short)b1;
   if (npl > 2) dst[2 * plane] = (unsigned short)b2;
 }
+// tf32(x), the part of x a kind::tf32 MMA sees exactly: round to nearest, 10 mantissa bits kept, by two integer instructions
+// (add half an ulp of the 10-bit mantissa, clear the low 13 bits): cvt.rna.tf32 runs at a fraction of the ALU rate, which is
+// what bounds a kernel that splits whole operand tiles.  Differs from cvt only on NaN payloads and when rounding carries
+// into Inf.
 __device__ __forceinline__ float tf32_round(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u); }
 __device__ __forceinline__ float4 tf32_round4(float4 v) { return make_float4(tf32_round(v.x), tf32_round(v.y), tf32_round(v.z), tf32_round(v.w)); }
 
@@ -423,7 +417,6 @@ int launch_gather(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, c
 void *pbg_tc_plan_create(const WaveDims &d, const WaveBufs &w, int nblk_max, int precision);
 void pbg_tc_plan_destroy(void *plan);
 // standard relations, plane tiers: score contraction of both problems + loss + coefficient planes in one kernel
-bool pbg_pair_eligible(const WaveDims &d, int precision);
 void *pbg_pair_plan_create(const WaveDims &d, const WaveBufs &w, int nblk_max);
 void pbg_pair_plan_destroy(void *plan);
 int launch_pair_score(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, void *plan, cudaStream_t st);

@@ -44,14 +44,11 @@ struct TcMaps { CUtensorMap a[2]; CUtensorMap b[2]; CUtensorMap c[2]; CUtensorMa
 struct TcGeom {
   int M, N, K;          // output rows, columns, contraction length (per block)
   int BN;               // tile columns (multiple of 16, <= 256)
-  int ldc;
-  long long c_blk;
-  float *C[2];
   const float *auxA[2]; long long auxa_blk;   // score epilogue (l2 family): |a|^2, |b|^2
   const float *auxB[2]; long long auxb_blk;
   int cmp, score;
   int nst, stage_bytes;  // bf16-plane tier: stages in flight and bytes of one (three planes of A and of the B tile)
-  int tr;                // the output map is that of the transposed matrix: tile element (row, col) goes to C[col][row]
+  int tr;                // the output map is that of the transposed matrix: tile element (row, col) goes to row col, column row
   // Dual mode (standard relations, plane tiers, transposed gradient without a merged coefficient matrix):
   //   GN_side^T (D x Mm) = N_other^T[:, k < K1] . B1   +   N_other^T[:, k < K] . B2   (B2 fills the first BN2 columns)
   // with B1[k = i][n = m] = T_side[i][m] and B2[n = i][k = j] = T_other[i][j]: the two halves of the combined
@@ -552,10 +549,9 @@ int launch_score_tc(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w,
   TcPlan *pl = (TcPlan *)plan;
   TcGeom g;
   memset(&g, 0, sizeof g);
-  g.M = d.Pm; g.N = d.Mm; g.K = d.D; g.BN = pl->bn_score; g.ldc = d.Ms; g.c_blk = (long long)d.Pm * d.Ms;
+  g.M = d.Pm; g.N = d.Mm; g.K = d.D; g.BN = pl->bn_score;
   g.cmp = d.cmp; g.score = 1;
   for (int p = 0; p < 2; ++p) {
-    g.C[p] = w.S[p];
     g.auxA[p] = w.aux[ARR_Q0 + p]; g.auxB[p] = w.aux[ARR_N0 + p];
   }
   g.auxa_blk = w.xrows[ARR_Q0]; g.auxb_blk = w.xrows[ARR_N0];
@@ -569,9 +565,8 @@ int launch_grad_dual_tc(const WaveDims &d, const WaveBatches &wb, const WaveBufs
   TcPlan *pl = (TcPlan *)plan;
   TcGeom g;
   memset(&g, 0, sizeof g);
-  g.M = d.D; g.N = d.Mm; g.K = d.Mm; g.BN = pl->bn_score; g.ldc = d.Dp; g.tr = 1;
+  g.M = d.D; g.N = d.Mm; g.K = d.Mm; g.BN = pl->bn_score; g.tr = 1;
   g.dual = 1; g.K1 = d.Pm; g.BN2 = pl->bn2;
-  for (int p = 0; p < 2; ++p) g.C[p] = w.GX[ARR_N0 + p];
   long long tiles = (long long)((g.N + g.BN - 1) / g.BN) * ((g.M + 127) / 128) * d.nblk * 2;
   const int sms = pbg_sm_count();
   const dim3 grid((unsigned)(tiles < sms ? tiles : sms));
@@ -585,11 +580,10 @@ int launch_grad_tc(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, 
   TcPlan *pl = (TcPlan *)plan;
   TcGeom g;
   memset(&g, 0, sizeof g);
-  g.N = d.D; g.BN = pl->bn_grad; g.ldc = d.Dp;
+  g.N = d.D; g.BN = pl->bn_grad;
   if (!pl->dynamic && pl->nterms != 1) {     // standard relations: the transposed product (see pbg_tc_plan_create)
     g.M = d.D; g.N = d.Mm; g.K = d.Mm; g.BN = pl->bn_score; g.tr = 1;
-    for (int p = 0; p < 2; ++p) g.C[p] = w.GX[ARR_N0 + p];
-    long long tiles = (long long)((g.N + g.BN - 1) / g.BN) * ((g.M + 127) / 128) * d.nblk * 2;
+      long long tiles = (long long)((g.N + g.BN - 1) / g.BN) * ((g.M + 127) / 128) * d.nblk * 2;
     const int sms = pbg_sm_count();
     const dim3 grid((unsigned)(tiles < sms ? tiles : sms));
     const size_t smem = 4 * (128 * 128 + 256 * 128) + 4 * 2 * 4096 + 1024;
@@ -599,18 +593,15 @@ int launch_grad_tc(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, 
     return 1;
   }
   if (!pl->dynamic) {          // GN_side = A[side] . N_(1-side)
-    g.M = d.Mm; g.K = d.Mm; g.c_blk = (long long)d.Mm * d.Dp;
-    for (int p = 0; p < 2; ++p) g.C[p] = w.GX[ARR_N0 + p];
-    launch_tc<false, true>(pl->gradm, g, pl->nterms, d, wb, w.errflag, st);
+    g.M = d.Mm; g.K = d.Mm;
+      launch_tc<false, true>(pl->gradm, g, pl->nterms, d, wb, w.errflag, st);
     return 1;
   }
   // GQ_p = T_p . N_p
-  g.M = d.Pm; g.K = d.Mm; g.c_blk = (long long)w.grows[ARR_Q0] * d.Dp;
-  for (int p = 0; p < 2; ++p) g.C[p] = w.GX[ARR_Q0 + p];
+  g.M = d.Pm; g.K = d.Mm;
   launch_tc<false, true>(pl->gradq, g, pl->nterms, d, wb, w.errflag, st);
   // GN_p = T_p^T . Q_p
-  g.M = d.Mm; g.K = d.Pm; g.c_blk = (long long)w.grows[ARR_N0] * d.Dp; g.sibling = 1;
-  for (int p = 0; p < 2; ++p) g.C[p] = w.GX[ARR_N0 + p];
+  g.M = d.Mm; g.K = d.Pm; g.sibling = 1;
   launch_tc<true, true>(pl->gradn, g, pl->nterms, d, wb, w.errflag, st);
   return 2;
 }

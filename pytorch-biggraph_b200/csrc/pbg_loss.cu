@@ -21,7 +21,6 @@ __device__ __forceinline__ float softplusf(float x) {           // log(1 + e^x),
 __device__ __forceinline__ float sigmoidf(float x) { return 1.0f / (1.0f + expf(-x)); }
 
 // column j of the negatives of a chunk: is it ignored, and does it exist at all?
-struct ColMask { bool masked; };
 __device__ __forceinline__ bool col_masked(const WaveDims &d, const BlockInfo &bi, int enabled, int i, int j) {
   if (!enabled) return true;
   if (j >= d.Pm) return false;                       // uniform negatives are never masked

@@ -384,11 +384,6 @@ struct PairPlan {
   int npl;
 };
 
-bool pbg_pair_eligible(const WaveDims &d, int precision) {
-  const bool planes = precision == PBG_PREC_BF16X6 || precision == PBG_PREC_BF16X3;
-  return planes && !d.dynamic && !d.matrix_op && d.cmp < PBG_CMP_L2 && d.Pm <= 128 && d.Mm <= 256;
-}
-
 void *pbg_pair_plan_create(const WaveDims &d, const WaveBufs &w, int nblk_max) {
   PairPlan *pl = new PairPlan();
   pl->npl = w.npl;
