@@ -73,6 +73,11 @@ def csrc_digest():
     return h.hexdigest()[:16]
 
 
+def waves_of(edges, batch, k):
+    """Waves of one library call: its batches dealt to the fewest waves of at most k."""
+    return -(-(-(-edges // batch)) // k)
+
+
 def ncu_traffic_per_edge(workload, precision):
     """(per-class DRAM bytes per trained edge, source note) from the profile summary of this pair, or
     (None, why) when there is none for the kernels in the tree."""
@@ -569,7 +574,7 @@ def run_b200_epoch(args, w, world, rank, dev):
         for _ in range(2):
             cur["edges"] = presplit(drv.step_index, plan_step(drv.step_index))
             drv.run_step(train_fn, after_step)
-        msc, lc = (C.c_double * 7)(), (C.c_int64 * 7)()
+        msc, lc = (C.c_double * len(_lib.KERNEL_CLASSES))(), (C.c_int64 * len(_lib.KERNEL_CLASSES))()
         _lib.check(nat.lib.pbg_kernel_times(nat.ctx, msc, lc), nat.ctx)
         _lib.check(nat.lib.pbg_set_profiling(nat.ctx, 0), nat.ctx)
         ne = max(cur["edges_done"] - done0, 1)
@@ -840,8 +845,8 @@ def run_b200(args, w):
     check(nat.lib.pbg_set_profiling(nat.ctx, 2), nat.ctx)     # halves of a wave one after the other: a pair brackets its kernels alone
     for s in range(total_steps, total_steps + nprof):
         step_device(s)
-    msc = (C.c_double * 7)()
-    lc = (C.c_int64 * 7)()
+    msc = (C.c_double * len(_lib.KERNEL_CLASSES))()
+    lc = (C.c_int64 * len(_lib.KERNEL_CLASSES))()
     check(nat.lib.pbg_kernel_times(nat.ctx, msc, lc), nat.ctx)
     check(nat.lib.pbg_set_profiling(nat.ctx, 0), nat.ctx)
     alg = algorithmic(w)
@@ -866,8 +871,8 @@ def run_b200(args, w):
     per_class_traffic, traffic_source = ncu_traffic_per_edge(args.workload, args.precision)
     per_edge = None if per_class_traffic is None else per_class_traffic.get(dom)
     # ncu's DRAM bytes of the dominant class, per launch of this run (edges of the timing pass / its launches)
-    # (the update class is several kernels per wave, the tile kernel carries its traffic: one launch per wave, as the statistics kernel)
-    dom_kernel_launches = max(per_class["stats"]["launches"], 1) if dom == "update" else launches_dom
+    # (the update class is several kernels per wave of which the tile kernel carries the traffic: one launch per wave)
+    dom_kernel_launches = nprof * bps * waves_of(step_edges, B, args.k) if dom == "update" else launches_dom
     traffic = None if per_edge is None else per_edge * edges_prof / dom_kernel_launches
     if dom in model_flops:
         ach = per_class[dom]["TFLOPs"]

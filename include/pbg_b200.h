@@ -301,9 +301,9 @@ int64_t pbg_launch_count(const pbg_context *ctx);
  * enable = 2: the halves are launched one after the other on the context's stream, so that a pair
  * brackets its kernels alone -- the durations to hold against a roofline.
  * Classes: 0 sort keys + radix sort, 1 gather/operator/prepare, 2 score contraction, 3 loss,
- * 4 gradient contractions, 5 optimizer updates (the batches' Stats are summed inside them), 6 no longer used.  ms_out / launches_out: HOST arrays of
+ * 4 gradient contractions, 5 optimizer updates (the batches' Stats are summed inside them).  ms_out / launches_out: HOST arrays of
  * PBG_NUM_KERNEL_CLASSES entries. */
-#define PBG_NUM_KERNEL_CLASSES 7
+#define PBG_NUM_KERNEL_CLASSES 6
 int pbg_set_profiling(pbg_context *ctx, int enable);
 int pbg_kernel_times(pbg_context *ctx, double *ms_out, int64_t *launches_out);
 

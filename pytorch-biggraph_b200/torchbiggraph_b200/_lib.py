@@ -85,7 +85,7 @@ SYMBOLS = [
     ("pbg_set_profiling", C.c_int, [_P, C.c_int]),
     ("pbg_kernel_times", C.c_int, [_P, C.POINTER(C.c_double), C.POINTER(C.c_int64)]),
 ]
-KERNEL_CLASSES = ("sort", "gather", "score", "loss", "grad", "update", "stats")
+KERNEL_CLASSES = ("sort", "gather", "score", "loss", "grad", "update")          # PBG_NUM_KERNEL_CLASSES of them
 
 _lib = None
 

@@ -57,3 +57,17 @@ def test_algorithmic_figures_of_the_headline_workload():
     # per trained edge, dim 1024 with 100 chunk + 100 uniform negatives: 12 D (P + U) flops, (2 + 2 U / P)(12 D + 8) + 24 bytes
     assert alg["flops"] == 12 * 1024 * 200
     assert alg["bytes"] == 4 * (12 * 1024 + 8) + 24
+
+
+def test_launches_behind_a_class_s_traffic_are_counted():
+    """The update class is several kernels a wave; its traffic belongs to one of them, so it is divided by the waves of the timed
+    calls (270 batches at fourteen in flight: twenty waves), and every class the library reports has a name."""
+    import re
+    b = _bench()
+    assert b.waves_of(269_506, 1000, 14) == 20 and b.waves_of(1, 1000, 14) == 1 and b.waves_of(14_000, 1000, 14) == 1 and b.waves_of(14_001, 1000, 14) == 2
+    from torchbiggraph_b200 import _lib
+    with open(os.path.join(ROOT, "include", "pbg_b200.h")) as f:
+        assert int(re.search(r"#define PBG_NUM_KERNEL_CLASSES (\d+)", f.read()).group(1)) == len(_lib.KERNEL_CLASSES)
+    with open(os.path.join(ROOT, "bench.py")) as f:
+        used = set(re.findall(r'per_class\["(\w+)"\]', f.read()))
+    assert used <= set(_lib.KERNEL_CLASSES)
