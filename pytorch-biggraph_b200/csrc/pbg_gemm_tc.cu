@@ -321,8 +321,9 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
       // comparator epilogue of the l2 family: compiled in only where it is used (predicated-off
       // copies of it in the unrolled loop cost more issue slots than the stores themselves)
       constexpr bool l2 = L2EPI;
-      if (l2 && m < g.M) an = g.auxA[p][(size_t)blk * g.auxa_blk + m];
-      const float *bn = l2 ? g.auxB[p] + (size_t)blk * g.auxb_blk : nullptr;
+      // (picked by selects: an index into the parameters made the compiler copy them to the stack, 8 % of the kernel)
+      if (l2 && m < g.M) an = (p ? g.auxA[1] : g.auxA[0])[(size_t)blk * g.auxa_blk + m];
+      const float *bn = l2 ? (p ? g.auxB[1] : g.auxB[0]) + (size_t)blk * g.auxb_blk : nullptr;
       for (int c0 = 0; c0 < g.BN; c0 += 32) {
         uint32_t r[32];
         uint32_t taddr = tmem + (uint32_t)ab * 256u + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
