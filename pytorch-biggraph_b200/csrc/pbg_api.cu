@@ -47,6 +47,7 @@ struct pbg_context {
   long long *hublist = nullptr;
   int *hubcnt = nullptr;        // two sets of counters, used in turn
   unsigned hub_turn = 0;
+  unsigned *seams = nullptr;    // words of the gradients' sibling launches
   long long *bigtab = nullptr;  // batch boundaries of the rows with 256 and more slots in a wave
   long long *edge_dev[3] = {nullptr, nullptr, nullptr};
   long long edge_cap = 0;
@@ -268,7 +269,7 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   for (int s = 0; s < 2; ++s)
     for (int i = 0; i < PBG_SORT_WAVES; ++i) { oWK[s][i] = take((size_t)nocc * 8); oWV[s][i] = take((size_t)nocc * 4); }
   size_t oSum = take(8 * sizeof(double)), oEval = take((size_t)pbg_eval_ctas(c->Cm, c->Pm) * 8 * sizeof(double)), oEvalDone = take(4);
-  size_t oPsum = take((size_t)nocc * c->Dp * 4), oHub = take(2 * (size_t)pbg_hublist_entries(nocc) * 8), oHubCnt = take(512);
+  size_t oPsum = take((size_t)nocc * c->Dp * 4), oHub = take(2 * (size_t)pbg_hublist_entries(nocc) * 8), oHubCnt = take(2 * HUB_SET * sizeof(int)), oSeam = take(64);
   size_t oBigTab = take(2 * pbg_bigtab_bytes((long long)nocc));
   // dynamic relations with a (vector) operator: the operator-row gradient of every edge, written by the pull-back pass
   size_t oGR[2] = {0, 0};
@@ -345,12 +346,13 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   c->hublist = (long long *)(c->ws + oHub);
   c->hubcnt = (int *)(c->ws + oHubCnt);
   c->bigtab = (long long *)(c->ws + oBigTab);
+  c->seams = (unsigned *)(c->ws + oSeam);
   if (cfg->precision != PBG_PREC_FP32) {
     WaveDims gd;
     memset(&gd, 0, sizeof gd);
     gd.D = cfg->dim; gd.Dp = c->Dp; gd.Pm = c->Pm; gd.U = c->U; gd.Mm = c->Mm; gd.Ms = c->Ms; gd.Cm = c->Cm;
     gd.dynamic = dyn;
-    c->tcplan = pbg_tc_plan_create(gd, b, (int)nblk, cfg->precision);
+    c->tcplan = pbg_tc_plan_create(gd, b, (int)nblk, cfg->precision, c->seams);
     if (!c->tcplan) return fail(c, PBG_ERR_CUDA, "could not encode the TMA tensor maps of the tensor-core contractions");
     if (c->fused) {
       c->pairplan = pbg_pair_plan_create(gd, b, (int)nblk);
@@ -672,7 +674,11 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
     b0 += kk;
   }
   c->batches_done += (unsigned long long)num_batches;
-  CU(c, pbg_take_launch_error());
+  if (const cudaError_t e = pbg_take_launch_error()) {
+    cudaMemsetAsync(c->seams, 0, 64, c->stream);             // (the first of two siblings may be without its second)
+    cudaMemsetAsync(c->hubcnt, 0, 2 * HUB_SET * sizeof(int), c->stream);
+    return fail(c, PBG_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
+  }
   if (stats_out) {
     rc = check_errflag(c);
     memcpy(stats_out, c->stats_host, (size_t)num_batches * sizeof(pbg_batch_stats));

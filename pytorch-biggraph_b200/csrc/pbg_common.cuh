@@ -240,6 +240,37 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_begin() { pdl_wait(); pdl_release(); }
 
+// Siblings: two launches in a row that read the same inputs and write different places.  The second starts as the first
+// one's CTAs leave (their last round is half empty) and is complete only after it (what comes next counts on both).  What it
+// reads has been waited for by the first, but the memory model gives that to the first alone, so the first hands it on: one
+// thread, behind the wait, releases a word, and the second acquires it before it reads anything -- by causality it then sees
+// what the first saw.  Where the word is not there yet, or not any more, it waits like every other kernel.  The
+// second clears the word behind its wait for the first's end, so each pair starts from zero.
+//   first:   pdl_begin_open(word)         (all threads; a null word: no sibling follows)
+//   second:  pdl_release(), then seam_enter(word) by every thread that reads, each for itself, and by whole warps;
+//            pdl_wait() and seam_close(word) before it ends.  Inputs through plain or __ldcg loads and bulk copies only:
+//            the read-only path (const __restrict__ pointers) is outside of the memory model's order.
+__device__ __forceinline__ void pdl_begin_open(unsigned *seam) {
+  int opens = seam != nullptr && blockIdx.x == 0;
+  asm volatile("" : "+r"(opens));                            // (the parameter is fetched in front of the wait, not behind it)
+  pdl_wait();
+  if (opens) {
+    if (threadIdx.x == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" :: "l"(seam), "r"(1u) : "memory");
+    __syncthreads();                                         // (the dependents are let go by the first thread that gets there)
+  }
+  pdl_release();
+}
+__device__ __forceinline__ void seam_enter(const unsigned *seam) {
+  unsigned open;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(open) : "l"(seam) : "memory");
+  if (open == 0u) pdl_wait();
+  __syncwarp();
+  asm volatile("fence.proxy.async.global;" ::: "memory");    // bulk copies read behind it too
+}
+__device__ __forceinline__ void seam_close(unsigned *seam) {
+  if (threadIdx.x == 0) *seam = 0u;
+}
+
 // N3 regularizer pieces at elements [dd, dd + 4) of a row y: the term is sum m^3 with m = |y_d|, or for
 // complex_diagonal the modulus of the pair (y_d, y_{d +- D/2}) counted once per pair
 // (torchbiggraph/operators.py:42-43, 151-157).  n3_grad4: d(sum m^3)/dy = 3 m y.
@@ -414,7 +445,8 @@ int launch_sort_rows(const long long *rows, long long num_rows, int n, int bits,
 int launch_build_keys(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w,
                       unsigned long long *keys, unsigned int *vals, cudaStream_t st);
 int launch_gather(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st);
-void *pbg_tc_plan_create(const WaveDims &d, const WaveBufs &w, int nblk_max, int precision);
+// seams: 16 words of device memory, zero, for the sibling launches of the gradients
+void *pbg_tc_plan_create(const WaveDims &d, const WaveBufs &w, int nblk_max, int precision, unsigned *seams);
 void pbg_tc_plan_destroy(void *plan);
 // standard relations, plane tiers: score contraction of both problems + loss + coefficient planes in one kernel
 void *pbg_pair_plan_create(const WaveDims &d, const WaveBufs &w, int nblk_max);
@@ -433,8 +465,9 @@ int launch_grad_simt(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w
 int launch_loss(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st);
 int launch_export_scores(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w,
                          float *lhs_pos, float *rhs_pos, float *lhs_neg, float *rhs_neg, cudaStream_t st);
-// What the optimizer kernels of a wave work with.  hubcnt: two sets of counters, 64 ints apart, used in turn (*turn):
-// while one set counts, the kernel behind it clears the other for the next user.  per_batch (may be null) / sum: where
+// What the optimizer kernels of a wave work with.  hubcnt: two sets of counters, HUB_SET ints apart, used in turn
+// (*turn): while one set counts, the kernel behind it clears the other for the next user; a set holds the words of the
+// sibling launches too (HUB_SEAM_*).  per_batch (may be null) / sum: where
 // the Stats of the wave's batches go.
 struct UpdateScratch {
   float *psum; long long *hublist; int *hubcnt; unsigned *turn; long long *bigtab;
@@ -442,7 +475,10 @@ struct UpdateScratch {
 };
 int launch_update(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, const unsigned long long *keys, const unsigned int *vals,
                   float lr, float rel_lr, const UpdateScratch &us, cudaStream_t st);
-// hublist and bigtab: a part for the embedding rows and one for the operator rows (as are hubcnt[0..1] and hubcnt[32..33] of a set).
+// hublist and bigtab: a part for the embedding rows and one for the operator rows (as are hubcnt[0..1] and hubcnt[HUB_REL ..] of a set).
+// Places in a set of hubcnt, a line each: the operator rows' counters, the words (pdl_begin_open) of the two tile and the two
+// hub kernels.
+enum { HUB_REL = 32, HUB_SEAM_TILE = 64, HUB_SEAM_HUB = 96, HUB_SET = 128 };
 inline long long pbg_hublist_entries(long long nocc) { return nocc / 8 + 64; }
 // bigtab: a line for each row with 256 and more slots: where its batches start, its end, a counter (zero between waves)
 inline size_t pbg_bigtab_bytes(long long nocc) { return (size_t)(nocc / 256 + 2) * (PBG_KMAX + 2) * sizeof(long long); }

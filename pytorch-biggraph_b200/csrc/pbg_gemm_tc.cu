@@ -56,10 +56,10 @@ struct TcGeom {
   // B1 as an MN-major operand (K1 = Pm rows), B2 as a K-major one (BN2 = Pm rounded up to 16 rows, K = Mm).
   // A stage holds the A tile, B1 (for the k-blocks below K1) and B2.
   int dual, K1, BN2;
-  // The launch before this one is its sibling (the other gradient of dynamic relations): same inputs, other outputs.  A
-  // launch's tiles are a few rounds of one per SM and the last round is half empty, so the CTAs of this one start as the
-  // sibling's leave, and wait for its end only before they end themselves (what comes next may count on both).
+  // The two gradients of dynamic relations are siblings (pdl_begin_open): 1 the first of them, 2 the second, 0 no sibling.  A
+  // launch's tiles are a few rounds of one per SM and the last round is half empty: the second's CTAs start in it.
   int sibling;
+  unsigned *seam;       // their word, else null
 };
 
 template <bool A_MN, bool B_MN, int NTERMS, bool L2EPI>
@@ -116,9 +116,6 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base_s;
-  // barriers and tensor memory are set up beside the kernel before this one
-  if (g.sibling) pdl_release();                              // the sibling has waited for our inputs, and bulk copies read them from L2
-  else pdl_begin();
   const int nkb = (g.K + KB - 1) / KB;
   const int b_atoms = PLANES ? (g.BN + 63) / 64 : (g.BN + 31) / 32;     // MN-major boxes per B tile (per plane)
   const uint32_t b_tile = B_MN ? (uint32_t)b_atoms * BOX_BYTES : (uint32_t)g.BN * ROW_BYTES;    // bytes of one B tile (of one plane)
@@ -142,6 +139,15 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
     BlockInfo bi = block_info(d, wb, blk);
     return bi.n != 0 && !(g.score && !d.neg_enabled[p]);
   };
+  // Barriers, tensor memory and the list of tiles are set up beside the kernel before this one.  (The list's divisions behind
+  // the wait cost 0.6 us of a 66 us batch.)
+  asm volatile("" :: "r"(ntiles), "r"(nkb), "r"(stage_tx));
+  const bool second = B_MN && g.sibling == 2;                // (both gradients of dynamic relations have an MN-major B)
+  if (second) {
+    pdl_release();
+    if (warp == 0) seam_enter(g.seam);                       // the producer's warp: nothing else here reads the inputs
+  } else if (B_MN) pdl_begin_open(g.seam);
+  else pdl_begin();
 
   if (warp == 0) {
     // ---------------- TMA producer (one box per operand, each from its own lane) ----------------
@@ -378,7 +384,10 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // the stores have left shared memory and are performed
   }
-  if (g.sibling) pdl_wait();
+  if (second) {
+    pdl_wait();
+    if (blockIdx.x == 0) seam_close(g.seam);
+  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 1) {
@@ -397,6 +406,7 @@ struct TcPlan {
   bool has_dual;
   int bn2;
   bool dynamic;
+  unsigned *seams;      // two words, 8 apart (pdl_begin_open): the gradients of a wave's first part, of its second
   int bn_score, bn_grad;
   int nterms;
 };
@@ -415,8 +425,9 @@ static int tile_cols(int n, int atom = 32) {
 
 // Builds the tensor maps for the context's workspace.  Returns null when the driver entry point
 // is missing or an encode fails.
-void *pbg_tc_plan_create(const WaveDims &d, const WaveBufs &w, int nblk_max, int precision) {
+void *pbg_tc_plan_create(const WaveDims &d, const WaveBufs &w, int nblk_max, int precision, unsigned *seams) {
   TcPlan *pl = new TcPlan();
+  pl->seams = seams;
   pl->has_dual = false; pl->bn2 = 0;
   pl->dynamic = d.dynamic != 0;
   pl->nterms = precision == PBG_PREC_TF32X3 ? 3 : precision == PBG_PREC_BF16X6 ? 6 : precision == PBG_PREC_BF16X3 ? 2 : 1;
@@ -599,10 +610,10 @@ int launch_grad_tc(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, 
     return 1;
   }
   // GQ_p = T_p . N_p
-  g.M = d.Pm; g.K = d.Mm;
+  g.M = d.Pm; g.K = d.Mm; g.sibling = 1; g.seam = pl->seams + (d.blk0 > 0 ? 8 : 0);   // (a wave's parts run on two streams)
   launch_tc<false, true>(pl->gradq, g, pl->nterms, d, wb, w.errflag, st);
   // GN_p = T_p^T . Q_p
-  g.M = d.Mm; g.K = d.Pm; g.sibling = 1;
+  g.M = d.Mm; g.K = d.Pm; g.sibling = 2;
   launch_tc<true, true>(pl->gradn, g, pl->nterms, d, wb, w.errflag, st);
   return 2;
 }

@@ -278,17 +278,26 @@ __device__ __forceinline__ long long *hub_biglist(long long *hublist, int nocc) 
 __device__ __forceinline__ const long long *hub_biglist(const long long *hublist, int nocc) { return hublist + nocc / 16 + 32; }
 enum { RULE_EMB = 0, RULE_REL = 1 };
 
-// The kernels of the operator rows (dynamic relations) work beside those of the embedding rows launched just before them:
-// other rows, other places in psum, lists and counters of their own.  Each of the four is bound by the chain of one row, so
-// in turn they took as long as all their chains together (dimension 400, 1,345 relations, every row a hub: the update 172 us a wave, 157 so; dimension 200, 14,824 relations: 169 and 164).  Such a kernel does not wait for the one before
-// it -- that one has waited for everything both read, and the fence keeps reads from lines of before -- but must not be
-// complete before it is, because the next launch counts on both: its last CTA waits for that and has no other work.
-__device__ __forceinline__ bool sibling_begin() {
+// The kernels of the operator rows (dynamic relations) work beside those of the embedding rows launched just before them, as
+// their siblings (pdl_begin_open): other rows, other places in psum, lists and counters of their own.  Each of the four is
+// bound by the chain of one row, so in turn they took as long as all their chains together (dimension 400, 1,345 relations,
+// every row a hub: the update 172 us a wave, 157 so; dimension 200, 14,824 relations: 169 and 164).  The last CTA of such a
+// kernel has no other work than to wait for the end of the one before.
+__host__ __device__ __forceinline__ bool has_operator_rows(const WaveDims &d) { return d.dynamic && d.op != PBG_OP_NONE; }
+__device__ __forceinline__ bool sibling_begin(unsigned *seam) {
   pdl_release();
-  if (blockIdx.x == gridDim.x - 1) { pdl_wait(); return false; }
-  __threadfence();
+  if (blockIdx.x == gridDim.x - 1) {
+    pdl_wait();
+    seam_close(seam);
+    return false;
+  }
+  seam_enter(seam);
   return true;
 }
+// The sorted list, the hub lists and their counters: written before the launch, so the operator rows' kernels, which do not
+// wait for the launch before them, read past the read-only path.
+template <int RULE, class T>
+__device__ __forceinline__ T ld_list(const T *p) { return RULE == RULE_REL ? __ldcg(p) : *p; }
 
 template <int VEC, int RULE>
 struct RowState {
@@ -393,8 +402,8 @@ __global__ void __launch_bounds__(32 * TileWarps<VEC, RULE>::N, RULE == RULE_EMB
 tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys,
                    const unsigned int *__restrict__ vals, float lr, float *__restrict__ psum,
                    long long *__restrict__ hublist, int *__restrict__ hubcnt, ParamJob job, int aside) {
-  if (RULE == RULE_EMB) pdl_begin();
-  else if (!sibling_begin()) return;
+  if (RULE == RULE_EMB) pdl_begin_open(has_operator_rows(d) ? (unsigned *)hubcnt + HUB_SEAM_TILE : nullptr);
+  else if (!sibling_begin((unsigned *)hubcnt - HUB_REL + HUB_SEAM_TILE)) return;
   constexpr int WARPS = TileWarps<VEC, RULE>::N, STAGE = TILE;
   extern __shared__ __align__(128) float stage_all[];        // [WARPS][STAGE][Dp]
   __shared__ __align__(8) unsigned long long sbar[WARPS];
@@ -419,9 +428,9 @@ tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
   const unsigned long long lo = RULE == RULE_EMB ? 0ull : d.key_rel_base;
   const unsigned long long hi = RULE == RULE_EMB ? d.key_rel_base : d.key_invalid;
   long long pa = t0 - 32 + lane, pb = t0 + lane;
-  unsigned long long kA = pa >= 0 ? keys[pa] : SENT;
-  unsigned long long kB = pb < d.nocc ? keys[pb] : SENT;
-  unsigned int vB = pb < d.nocc ? vals[pb] : 0u;
+  unsigned long long kA = pa >= 0 ? ld_list<RULE>(keys + pa) : SENT;
+  unsigned long long kB = pb < d.nocc ? ld_list<RULE>(keys + pb) : SENT;
+  unsigned int vB = pb < d.nocc ? ld_list<RULE>(vals + pb) : 0u;
   const int bB = d.bySpb.div((int)vB);              // batch of this lane's slot
   if (__shfl_sync(FULL, kB, TILE - 1) < lo) return;          // tile holds only the other rule's rows
   // Copies the gradient rows of window slots j0 .. j0+cnt-1 (cnt <= STAGE) into the stage buffers and
@@ -544,7 +553,7 @@ tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
       hublist[atomicAdd(hubcnt, 1)] = head;
       // a row's slots are contiguous in the sorted list: it has HUB_BIG or more of them exactly when the slot
       // HUB_BIG - 1 places after its head still carries its key; those few rows go on a second list
-      if (head + HUB_BIG - 1 < (long long)d.nocc && keys[head + HUB_BIG - 1] == key)
+      if (head + HUB_BIG - 1 < (long long)d.nocc && ld_list<RULE>(keys + head + HUB_BIG - 1) == key)
         hub_biglist(hublist, d.nocc)[atomicAdd(hubcnt + 1, 1)] = head;
     }
     i += nproc;
@@ -567,7 +576,7 @@ template <int NP>
 __global__ void __launch_bounds__(32 * NARROW_WARPS, NP == 2 ? 6 : 4)
 narrow_tile_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys, const unsigned int *__restrict__ vals,
                    float lr, float *__restrict__ psum, long long *__restrict__ hublist, int *__restrict__ hubcnt, ParamJob job, int aside) {
-  pdl_begin();
+  pdl_begin_open(has_operator_rows(d) ? (unsigned *)hubcnt + HUB_SEAM_TILE : nullptr);
   constexpr int NARROW_STAGE = NarrowStage<NP>::N;
   extern __shared__ __align__(128) float stage_all[];        // [NARROW_WARPS][NARROW_STAGE][Dp]
   __shared__ __align__(8) unsigned long long sbar[NARROW_WARPS];
@@ -846,8 +855,8 @@ __global__ void __launch_bounds__(32 * UPD_WARPS)
 hub_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys, const unsigned int *__restrict__ vals, float lr,
            float *psum, const long long *__restrict__ hublist, const int *__restrict__ hubcnt, int *__restrict__ hubcnt_next,
            long long *bigtab, int aside, ParamJob job, pbg_batch_stats *per_batch, double *sum) {
-  if (RULE == RULE_EMB) pdl_begin();
-  else if (!sibling_begin()) return;
+  if (RULE == RULE_EMB) pdl_begin_open(has_operator_rows(d) ? (unsigned *)hubcnt + HUB_SEAM_HUB : nullptr);
+  else if (!sibling_begin((unsigned *)hubcnt - HUB_REL + HUB_SEAM_HUB)) return;
   static_assert(32 * UPD_WARPS == HUB_BIG, "one probe per thread covers exactly the rows that are not big");
   extern __shared__ __align__(16) float tot[];               // [k][VEC * 128]; sums of a big row's batch: [UPD_WARPS][VEC * 128]
   __shared__ long long bstart[PBG_KMAX + 1];
@@ -867,23 +876,23 @@ hub_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__r
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int D = d.D;
   const float invD = 1.0f / (float)D;
-  const int nh = hubcnt[0], nbig = hubcnt[1];                 // the tile kernel listed the rows
+  const int nh = ld_list<RULE>(hubcnt), nbig = ld_list<RULE>(hubcnt + 1);                 // the tile kernel listed the rows
   const long long *biglist = hub_biglist(hublist, d.nocc);
   // the batches of the big rows first, then the list of all hub rows, big ones skipped
   const int ctas = (int)gridDim.x - (RULE == RULE_REL) - cta0, items = nbig * d.k + nh;
   for (int item = blockIdx.x - cta0; item < items; item += ctas) {
     const bool from_big = item < nbig * d.k;
     const int h = item / d.k;
-    const long long head = from_big ? biglist[h] : hublist[item - nbig * d.k];
+    const long long head = ld_list<RULE>(from_big ? biglist + h : hublist + (item - nbig * d.k));
     long long *line = bigtab + (size_t)h * BIGTAB_LINE;       // [b] first slot of batch b or -1, then the row's end, then a counter
     if (from_big) {
       const int b = item - h * d.k;
-      const unsigned long long key = keys[head];
-      const long long end = coop_prefix_end(head + HUB_BIG, (long long)d.nocc, [&](long long pos) { return keys[pos] == key; });
+      const unsigned long long key = ld_list<RULE>(keys + head);
+      const long long end = coop_prefix_end(head + HUB_BIG, (long long)d.nocc, [&](long long pos) { return ld_list<RULE>(keys + pos) == key; });
       // where batch b starts and ends inside the row.  (Both searches in the same rounds, half of the CTA each, measured
       // slower: 14.2 against 11.8 us.)
-      const long long q = coop_prefix_end(head, end, [&](long long pos) { return d.bySpb.div((int)vals[pos]) < b; });
-      const long long eb = coop_prefix_end(q, end, [&](long long pos) { return d.bySpb.div((int)vals[pos]) <= b; });
+      const long long q = coop_prefix_end(head, end, [&](long long pos) { return d.bySpb.div((int)ld_list<RULE>(vals + pos)) < b; });
+      const long long eb = coop_prefix_end(q, end, [&](long long pos) { return d.bySpb.div((int)ld_list<RULE>(vals + pos)) <= b; });
       const long long ftb = (q / TILE + 1) * TILE;
       const long long nruns = q < eb ? 1 + (eb > ftb ? (eb - 1 - ftb) / TILE + 1 : 0) : 0;
       if (nruns > 1) {
@@ -934,8 +943,8 @@ hub_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__r
       if (threadIdx.x == 0) line[PBG_KMAX + 1] = 0;           // for the next wave
     }
     const long long p = head + threadIdx.x;
-    const unsigned long long kp = p < (long long)d.nocc ? keys[p] : ~0ull;
-    const int bp = p < (long long)d.nocc ? d.bySpb.div((int)vals[p]) : -1;
+    const unsigned long long kp = p < (long long)d.nocc ? ld_list<RULE>(keys + p) : ~0ull;
+    const int bp = p < (long long)d.nocc ? d.bySpb.div((int)ld_list<RULE>(vals + p)) : -1;
     // what the CTAs of a big row's batches left (past L1: this CTA may have read the lines before)
     const long long tabv = from_big && threadIdx.x <= PBG_KMAX ? __ldcg(line + threadIdx.x) : -1;
     if (threadIdx.x == 0) skey = kp;
@@ -1269,7 +1278,7 @@ static int launch_update_vec(const WaveDims &d, const WaveBatches &wb, const Wav
   pbg_opt_in_smem((const void *)hub_kernel<VEC, RULE_EMB>, (int)hub_smem_max);
   ParamJob job;
   int launches = launch_pullback<VEC>(d, wb, w, rel_lr, job, st);
-  int *hubcnt = us.hubcnt + 64 * (*us.turn & 1), *hubcnt_next = us.hubcnt + 64 * ((*us.turn + 1) & 1);
+  int *hubcnt = us.hubcnt + HUB_SET * (*us.turn & 1), *hubcnt_next = us.hubcnt + HUB_SET * ((*us.turn + 1) & 1);
   ++*us.turn;
   const int sum_ctas = param_sum_ctas(d, job);
   if (VEC <= 2) {
@@ -1284,11 +1293,11 @@ static int launch_update_vec(const WaveDims &d, const WaveBatches &wb, const Wav
     pbg_opt_in_smem((const void *)tile_update_kernel<V, RULE_EMB>, EMB_WARPS * TILE * V * 512);
     pbg_launch(tile_update_kernel<V, RULE_EMB>, sum_ctas + (unsigned)((tiles + EMB_WARPS - 1) / EMB_WARPS), 32 * EMB_WARPS, (size_t)EMB_WARPS * TILE * d.Dp * 4, st, d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, job, sum_ctas);
   }
-  const bool rel_rows = d.dynamic && d.op != PBG_OP_NONE && w.theta[0] != nullptr;
+  const bool rel_rows = has_operator_rows(d);
   long long *rel_hublist = us.hublist + pbg_hublist_entries(d.nocc), *rel_bigtab = us.bigtab + pbg_bigtab_bytes(d.nocc) / sizeof(long long);
   if (rel_rows) {
     pbg_opt_in_smem((const void *)tile_update_kernel<VEC, RULE_REL>, REL_WARPS * TILE * VEC * 512);
-    pbg_launch(tile_update_kernel<VEC, RULE_REL>, (unsigned)((tiles + REL_WARPS - 1) / REL_WARPS) + 1, 32 * REL_WARPS, (size_t)REL_WARPS * TILE * d.Dp * 4, st, d, wb, w, keys, vals, rel_lr, us.psum, rel_hublist, hubcnt + 32, job, 0);
+    pbg_launch(tile_update_kernel<VEC, RULE_REL>, (unsigned)((tiles + REL_WARPS - 1) / REL_WARPS) + 1, 32 * REL_WARPS, (size_t)REL_WARPS * TILE * d.Dp * 4, st, d, wb, w, keys, vals, rel_lr, us.psum, rel_hublist, hubcnt + HUB_REL, job, 0);
   }
   pbg_launch(hub_kernel<VEC, RULE_EMB>, d.k + param_step_ctas(d, job) + hub_ctas, 32 * UPD_WARPS, hub_smem, st,
              d, wb, w, keys, vals, lr, us.psum, us.hublist, hubcnt, hubcnt_next, us.bigtab, 1, job, us.per_batch, us.sum);
@@ -1296,7 +1305,7 @@ static int launch_update_vec(const WaveDims &d, const WaveBatches &wb, const Wav
   if (rel_rows) {
     pbg_opt_in_smem((const void *)hub_kernel<VEC, RULE_REL>, (int)hub_smem_max);
     pbg_launch(hub_kernel<VEC, RULE_REL>, hub_ctas + 1, 32 * UPD_WARPS, hub_smem, st,
-               d, wb, w, keys, vals, rel_lr, us.psum, rel_hublist, hubcnt + 32, hubcnt_next + 32, rel_bigtab, 0, job, (pbg_batch_stats *)nullptr, (double *)nullptr);
+               d, wb, w, keys, vals, rel_lr, us.psum, rel_hublist, hubcnt + HUB_REL, hubcnt_next + HUB_REL, rel_bigtab, 0, job, (pbg_batch_stats *)nullptr, (double *)nullptr);
     launches += 2;
   }
   if (d.op != PBG_OP_NONE && w.theta[0] != nullptr) {

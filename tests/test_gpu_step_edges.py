@@ -58,3 +58,34 @@ def test_operator_rows_of_wide_models(D):
 def test_update_rows_at_the_half_warp_kernels_widths(D, N, nb, nu):
     """Hub rows only, short rows across tiles and hubs, and rows of a single slot, at the edges of a half-warp's row."""
     _run(_random_case(9, D, N, 5 * nb + 2, nb, nu, "none", "dot", "softmax", zipf=N > 10), "tf32x3")
+
+
+@pytest.mark.parametrize("precision", ["tf32x3", "bf16x6"])
+@pytest.mark.parametrize("D,R,k", [(36, 5, 1), (100, 900, 4), (260, 40, 3)])
+def test_sibling_launches_wave_after_wave(D, R, k, precision):
+    """Dynamic relations: the two gradients, and the tile and hub kernels of embedding and operator rows, run into one another.
+    Several waves in one call (k >= 2: halves on two streams), against the oracle, and the same bits every time."""
+    import torch
+    from b200_util import Rig
+    c, ocfg, ost, batches = _random_case(10, D, 700, 310, 30, 20, "diagonal", "dot", "softmax", dyn=True, R=R, zipf=True, nbatches=2 * k + 1)
+    start = [ost.W_lhs.copy(), ost.G_lhs.copy(), ost.theta_rhs.copy(), ost.theta_lhs.copy()]
+    lhs, rhs, rel = (np.concatenate([b[i] for b in batches]) for i in range(3))
+    runs = []
+    for _ in range(3):
+        rig = Rig.from_oracle_state(c, ost, precision=precision, k=k)
+        nat = rig.trainer._context(rig.model, 310)
+        ul, ur = (torch.stack([nat._uniform(b[i], "cuda") for b in batches]).contiguous() for i in (3, 4))
+        t = lambda a: torch.tensor(a).cuda()
+        rig.trainer.train_batches(rig.model, t(lhs), t(rhs), t(rel), [(i * 310, 310, 0) for i in range(len(batches))], ul, ur)
+        runs.append((rig.W_lhs.cpu().numpy(), rig.G("lhs"), rig.theta("rhs"), rig.theta("lhs"), rig.acc("rhs"), rig.acc("lhs")))
+    for other in runs[1:]:
+        for a, b in zip(runs[0], other):
+            np.testing.assert_array_equal(a, b)
+    nwaves = -(-len(batches) // k)
+    sizes = [len(batches) // nwaves + (w < len(batches) % nwaves) for w in range(nwaves)]      # dealt evenly
+    for n in sizes:
+        O.train_wave(ocfg, ost, batches[:n])
+        batches = batches[n:]
+    with _tier_tolerance(precision):
+        for got, want, was, what in zip(runs[0], (ost.W_lhs, ost.G_lhs, ost.theta_rhs, ost.theta_lhs), start, ("W", "G", "theta_rhs", "theta_lhs")):
+            _close(got, want, atol=max(1e-6, RTOL * float(np.abs(want - was).max())), what=what)
