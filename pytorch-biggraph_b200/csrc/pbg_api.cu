@@ -22,6 +22,7 @@ struct pbg_context {
   size_t ws_bytes = 0;
   WaveBufs bufs;           // workspace pointers (table pointers filled per call)
   SortPlan sort[2];        // double-buffered scratch of the three-launch sort: wave w+1 is sorted on `side` while wave w trains
+  bool cluster_sort = false;        // the device can hold the clusters of sort_waves_kernel (pbg_cluster_sort_available)
   // sorted lists of two groups of waves: the next group is sorted on `side` while this one trains
   unsigned long long *wkeys[2][PBG_SORT_WAVES];
   unsigned int *wvals[2][PBG_SORT_WAVES];
@@ -259,6 +260,9 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   const size_t opw = matrix_op ? (size_t)cfg->dim * cfg->dim + (cfg->op == PBG_OP_AFFINE ? cfg->dim : 0) : (size_t)cfg->dim;
   size_t oR1 = 0, oR2 = 0, oDA = 0;
   if (matrix_op) { oR1 = take(nN * c->Dp * 4); oR2 = take(nN * c->Dp * 4); oDA = take((size_t)c->kmax * opw * 4); }
+  // PBG_CLUSTER_SORT=0 in the environment: the three-launch sort for every list
+  const char *envc = getenv("PBG_CLUSTER_SORT");
+  c->cluster_sort = !(envc && envc[0] == '0') && pbg_cluster_sort_available(nocc);
   size_t oK[2][2], oV[2][2], oH[2];
   for (int s = 0; s < 2; ++s) {
     oK[s][0] = take((size_t)nocc * 8); oK[s][1] = take((size_t)nocc * 8);
@@ -597,7 +601,7 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
   // trains: few launches, and the sort of the next group has a whole group's training to hide behind.  The call's
   // first group is one wave, so that its update waits for the shortest sort there is.  Waves beyond what a cluster
   // holds are sorted one by one, one wave ahead.
-  const bool cluster = pbg_cluster_sort_fits((long long)(kbase + (kextra ? 1 : 0)) * d.spb, bits);
+  const bool cluster = c->cluster_sort && pbg_cluster_sort_fits((long long)(kbase + (kextra ? 1 : 0)) * d.spb, bits);
   const int gsize = cluster ? PBG_SORT_WAVES : 1;
   auto group_of = [&](int wv) { return wv == 0 ? 0 : 1 + (wv - 1) / gsize; };
   auto group_first = [&](int g) { return g == 0 ? 0 : 1 + (g - 1) * gsize; };
@@ -860,7 +864,7 @@ extern "C" int pbg_row_adagrad(pbg_context *c, float *emb, float *state, int64_t
   if (n > sp.max_n) return fail(c, PBG_ERR_TOO_LARGE, "%d gradient rows exceed this context's sort capacity %d", n, sp.max_n);
   CU(c, cudaSetDevice(c->device));
   const int bits = bit_length((unsigned long long)num_rows);
-  if (pbg_cluster_sort_fits(n, bits)) {
+  if (c->cluster_sort && pbg_cluster_sort_fits(n, bits)) {
     sp.result = 0;
     c->launches += launch_sort_rows((const long long *)rows, num_rows, n, bits, sp.keys[0], sp.vals[0], c->errflag, c->stream);
   } else {

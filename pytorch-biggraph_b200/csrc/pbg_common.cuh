@@ -433,6 +433,7 @@ int pbg_sort(SortPlan &sp, int n, int bits, cudaStream_t st);
 // Stable sort in one kernel, a thread-block cluster per list: lists of at most PBG_CLUSTER_SORT_MAX pairs, keys below 2^32.
 #define PBG_CLUSTER_SORT_MAX (16 * 1024 * 16)
 inline bool pbg_cluster_sort_fits(long long n, int bits) { return n <= PBG_CLUSTER_SORT_MAX && bits <= 32; }
+bool pbg_cluster_sort_available(long long n);   // on the current device, for lists of up to n pairs
 #define PBG_SORT_WAVES 4            // most waves of one launch
 struct SortWave { WaveBatches wb; int k; unsigned long long *keys; unsigned int *vals; };
 struct SortWaves { SortWave w[PBG_SORT_WAVES]; int count; };

@@ -349,6 +349,34 @@ static void launch_cluster(void (*kernel)(Args...), int lists, int ctas, size_t 
   pbg_note_launch(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
+// Whether clusters of this shape can be resident on the device at all: with part of its SMs (MPS, MIG, green contexts) there may
+// be no sixteen of them close enough together that each have the shared memory free.
+template <int IPT>
+static bool cluster_resident(int ctas) {
+  for (const void *kernel : {(const void *)sort_waves_kernel<IPT>, (const void *)sort_rows_kernel<IPT>}) {
+    if (pbg_opt_in_smem(kernel, (int)cluster_sort_smem<IPT>()) != cudaSuccess) return false;
+    if (ctas > 8 && pbg_opt_in_cluster16(kernel) != cudaSuccess) return false;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas); cfg.blockDim = dim3(CS_THREADS); cfg.dynamicSmemBytes = cluster_sort_smem<IPT>();
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = ctas; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cfg.attrs = &at; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) return false;
+  }
+  return true;
+}
+
+// The largest list takes the most CTAs and shared memory; where its clusters fit, those of shorter lists do.
+bool pbg_cluster_sort_available(long long n) {
+  int ctas, ipt;
+  cluster_shape((int)(n < PBG_CLUSTER_SORT_MAX ? n : PBG_CLUSTER_SORT_MAX), ctas, ipt);
+  const bool ok = ipt == 1 ? cluster_resident<1>(ctas) : ipt == 2 ? cluster_resident<2>(ctas) : ipt == 4 ? cluster_resident<4>(ctas) : ipt == 8 ? cluster_resident<8>(ctas) : cluster_resident<16>(ctas);
+  if (!ok) pbg_take_launch_error();                          // (an answer, not a failure of the call that asked)
+  return ok;
+}
+
 int launch_sort_waves(const WaveDims &d, const WaveBufs &w, const SortWaves &waves, int bits, cudaStream_t st) {
   int most = 0, ctas, ipt;
   for (int i = 0; i < waves.count; ++i) if (waves.w[i].k > most) most = waves.w[i].k;
