@@ -21,7 +21,10 @@ struct pbg_context {
   char *ws = nullptr;
   size_t ws_bytes = 0;
   WaveBufs bufs;           // workspace pointers (table pointers filled per call)
-  SortPlan sort[2];        // double-buffered scratch of the three-launch sort: wave w+1 is sorted on `side` while wave w trains
+  // Scratch of the three-launch sort, double-buffered: wave w+1 is sorted on `side` while wave w trains.  The second is there
+  // where waves can be longer than a cluster sorts, else from the first call with keys beyond 32 bits (second_sort).
+  SortPlan sort[2];
+  char *sort_mem = nullptr;
   bool cluster_sort = false;        // the device can hold the clusters of sort_waves_kernel (pbg_cluster_sort_available)
   // sorted lists of two groups of waves: the next group is sorted on `side` while this one trains
   unsigned long long *wkeys[2][PBG_SORT_WAVES];
@@ -132,6 +135,19 @@ extern "C" int64_t pbg_workspace_bytes(const pbg_context *c) { return c ? (int64
 extern "C" int64_t pbg_launch_count(const pbg_context *c) { return c ? c->launches : 0; }
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
+
+// scratch of the three-launch sort of n pairs
+static size_t sort_plan_bytes(long long n) {
+  return 2 * align_up((size_t)n * 8, 256) + 2 * align_up((size_t)n * 4, 256) + align_up(pbg_sort_hist_entries((int)n) * 4, 256);
+}
+static void carve_sort(SortPlan &sp, char *p, long long n) {
+  const size_t kb = align_up((size_t)n * 8, 256), vb = align_up((size_t)n * 4, 256);
+  sp.keys[0] = (unsigned long long *)p; sp.keys[1] = (unsigned long long *)(p + kb);
+  sp.vals[0] = (unsigned int *)(p + 2 * kb); sp.vals[1] = (unsigned int *)(p + 2 * kb + vb);
+  sp.hist = (unsigned int *)(p + 2 * kb + 2 * vb);
+  sp.max_n = (int)n;
+  sp.result = 0;
+}
 
 static int chunk_geometry(const pbg_config &cfg, int *Pm, int *Cm) {
   int B = cfg.max_batch_size;
@@ -263,15 +279,13 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   // PBG_CLUSTER_SORT=0 in the environment: the three-launch sort for every list
   const char *envc = getenv("PBG_CLUSTER_SORT");
   c->cluster_sort = !(envc && envc[0] == '0') && pbg_cluster_sort_available(nocc);
-  size_t oK[2][2], oV[2][2], oH[2];
-  for (int s = 0; s < 2; ++s) {
-    oK[s][0] = take((size_t)nocc * 8); oK[s][1] = take((size_t)nocc * 8);
-    oV[s][0] = take((size_t)nocc * 4); oV[s][1] = take((size_t)nocc * 4);
-    oH[s] = take(pbg_sort_hist_entries((int)nocc) * 4);
-  }
+  size_t oSort[2] = {take(sort_plan_bytes(nocc)), 0};
+  const bool two_sorts = !c->cluster_sort || nocc > PBG_CLUSTER_SORT_MAX;
+  if (two_sorts) oSort[1] = take(sort_plan_bytes(nocc));
+  const size_t list = !c->cluster_sort ? 0 : nocc < PBG_CLUSTER_SORT_MAX ? (size_t)nocc : PBG_CLUSTER_SORT_MAX;     // longest list a cluster sorts
   size_t oWK[2][PBG_SORT_WAVES], oWV[2][PBG_SORT_WAVES];
   for (int s = 0; s < 2; ++s)
-    for (int i = 0; i < PBG_SORT_WAVES; ++i) { oWK[s][i] = take((size_t)nocc * 8); oWV[s][i] = take((size_t)nocc * 4); }
+    for (int i = 0; i < PBG_SORT_WAVES; ++i) { oWK[s][i] = take(list * 8); oWV[s][i] = take(list * 4); }
   size_t oSum = take(8 * sizeof(double)), oEval = take((size_t)pbg_eval_ctas(c->Cm, c->Pm) * 8 * sizeof(double)), oEvalDone = take(4);
   size_t oPsum = take((size_t)nocc * c->Dp * 4), oHub = take(2 * (size_t)pbg_hublist_entries(nocc) * 8), oHubCnt = take(2 * HUB_SET * sizeof(int)), oSeam = take(64);
   size_t oBigTab = take(2 * pbg_bigtab_bytes((long long)nocc));
@@ -319,13 +333,8 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   b.R2 = matrix_op ? (float *)(c->ws + oR2) : nullptr;
   b.dA = matrix_op ? (float *)(c->ws + oDA) : nullptr;
   for (int s = 0; s < 2; ++s) {
-    c->sort[s].keys[0] = (unsigned long long *)(c->ws + oK[s][0]);
-    c->sort[s].keys[1] = (unsigned long long *)(c->ws + oK[s][1]);
-    c->sort[s].vals[0] = (unsigned int *)(c->ws + oV[s][0]);
-    c->sort[s].vals[1] = (unsigned int *)(c->ws + oV[s][1]);
-    c->sort[s].hist = (unsigned int *)(c->ws + oH[s]);
-    c->sort[s].max_n = (int)nocc;
-    c->sort[s].result = 0;
+    if (s == 0 || two_sorts) carve_sort(c->sort[s], c->ws + oSort[s], nocc);
+    else c->sort[s].max_n = 0;
     for (int i = 0; i < PBG_SORT_WAVES; ++i) {
       c->wkeys[s][i] = (unsigned long long *)(c->ws + oWK[s][i]);
       c->wvals[s][i] = (unsigned int *)(c->ws + oWV[s][i]);
@@ -378,6 +387,7 @@ extern "C" int pbg_destroy(pbg_context *c) {
   for (int i = 0; i < 3; ++i) if (c->edge_dev[i]) cudaFree(c->edge_dev[i]);
   for (int i = 0; i < 2; ++i) if (c->uni_dev[i]) cudaFree(c->uni_dev[i]);
   if (c->esort_mem) cudaFree(c->esort_mem);
+  if (c->sort_mem) cudaFree(c->sort_mem);
   if (c->rp_mem) cudaFree(c->rp_mem);
   if (c->counts_host) cudaFreeHost(c->counts_host);
   if (c->allnegs_mem) cudaFree(c->allnegs_mem);
@@ -532,6 +542,15 @@ extern "C" int pbg_kernel_times(pbg_context *c, double *ms_out, int64_t *launche
   return PBG_OK;
 }
 
+// The second scratch of the three-launch sort, where pbg_create saw no need for it: keys of more than 32 bits.
+static int second_sort(pbg_context *c) {
+  if (c->sort[1].max_n) return PBG_OK;
+  const int n = c->sort[0].max_n;
+  CU(c, cudaMalloc(&c->sort_mem, sort_plan_bytes(n)));
+  carve_sort(c->sort[1], c->sort_mem, n);
+  return PBG_OK;
+}
+
 extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int64_t *lhs, const int64_t *rhs,
                                  const int64_t *rel, int64_t num_edges, const pbg_batch *batches,
                                  int32_t num_batches, const int64_t *ul, const int64_t *ur, uint64_t seed,
@@ -603,6 +622,7 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
   // holds are sorted one by one, one wave ahead.
   const bool cluster = c->cluster_sort && pbg_cluster_sort_fits((long long)(kbase + (kextra ? 1 : 0)) * d.spb, bits);
   const int gsize = cluster ? PBG_SORT_WAVES : 1;
+  if (!cluster && nwaves > 1) { rc = second_sort(c); if (rc) return rc; }
   auto group_of = [&](int wv) { return wv == 0 ? 0 : 1 + (wv - 1) / gsize; };
   auto group_first = [&](int g) { return g == 0 ? 0 : 1 + (g - 1) * gsize; };
   const int ngroups = group_of(nwaves - 1) + 1;
@@ -895,14 +915,8 @@ static int ensure_edge_sort(pbg_context *c, long long n) {
   if (n <= c->esort.max_n) return PBG_OK;
   if (c->esort_mem) { cudaFree(c->esort_mem); c->esort_mem = nullptr; c->esort.max_n = 0; }
   const long long cap = n + n / 4 + 1024 > 0x7fffffffll ? 0x7fffffffll : n + n / 4 + 1024;
-  const size_t kb = align_up((size_t)cap * 8, 256), vb = align_up((size_t)cap * 4, 256);
-  const size_t hb = align_up(pbg_sort_hist_entries((int)cap) * 4, 256);
-  CU(c, cudaMalloc(&c->esort_mem, 2 * kb + 2 * vb + hb));
-  char *p = c->esort_mem;
-  c->esort.keys[0] = (unsigned long long *)p; c->esort.keys[1] = (unsigned long long *)(p + kb);
-  c->esort.vals[0] = (unsigned int *)(p + 2 * kb); c->esort.vals[1] = (unsigned int *)(p + 2 * kb + vb);
-  c->esort.hist = (unsigned int *)(p + 2 * kb + 2 * vb);
-  c->esort.max_n = (int)cap;
+  CU(c, cudaMalloc(&c->esort_mem, sort_plan_bytes(cap)));
+  carve_sort(c->esort, c->esort_mem, cap);
   return PBG_OK;
 }
 

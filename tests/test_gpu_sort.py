@@ -86,7 +86,7 @@ def _train(rows_told=None, batches=30):
 
 def test_without_clusters_and_with_keys_beyond_32_bits_the_sort_takes_the_radix_passes(monkeypatch):
     """The same order, so the same bits.  PBG_CLUSTER_SORT=0 stands for a device that cannot hold the clusters (part of its SMs);
-    2^33 rows need keys of 34 bits.  Keys of 12 bits take two passes of three
+    2^33 rows need keys of 34 bits, for which a second scratch is made at the first call.  Keys of 12 bits take two passes of three
     launches, keys of 34 four, and the key build; the cluster kernel takes the eight waves in three launches."""
     W, G, launches = _train()
     monkeypatch.setenv("PBG_CLUSTER_SORT", "0")
@@ -95,3 +95,16 @@ def test_without_clusters_and_with_keys_beyond_32_bits_the_sort_takes_the_radix_
     Wl, Gl, wide = _train(rows_told=2 ** 33)
     assert torch.equal(W, Wr) and torch.equal(G, Gr) and torch.equal(W, Wl) and torch.equal(G, Gl)
     assert radix - launches == 8 * 7 - 3 and wide - launches == 8 * 13 - 3
+
+
+def test_sort_scratch_follows_what_the_waves_need():
+    """Bytes per slot of the workspace, below and above the longest list a cluster sorts (262,144): below, eight lists of 12 bytes a
+    slot and one scratch of 56 (pairs twice, counters); above, a second scratch, and no more lists: 96 - 56 bytes less."""
+    def slope(small, large):
+        size = {}
+        for edges in (small, large):
+            L, ctx = _create(max_batch_size=edges, batches_in_flight=1)
+            size[edges] = L.pbg_workspace_bytes(ctx)
+            L.pbg_destroy(ctx)
+        return (size[large] - size[small]) / (4.0 * (large - small))          # 50 + 50 negatives a side: four slots an edge
+    assert slope(25_000, 50_000) - slope(100_000, 200_000) == pytest.approx(40.0, abs=1.0)
