@@ -6,6 +6,7 @@ and the batch loop around it (torchbiggraph/batching.py:91-125).
 library in one call, which trains `batches_in_flight` batches per wave on the device."""
 import ctypes as C
 import time
+import weakref
 from abc import ABC, abstractmethod
 from typing import Dict, Iterable, List, Optional, Tuple
 
@@ -213,7 +214,8 @@ class B200Trainer(AbstractBatchProcessor):
         self.unpartitioned_optimizers: Dict[str, RowAdagrad] = {}
         self.partitioned_optimizers: Dict[Tuple, RowAdagrad] = {}
         self._native: Optional[_Native] = None          # the context used last
-        self._natives: Dict[str, _Native] = {}          # one per operator group
+        self._natives: Dict[str, _Native] = {}          # one per operator group of the model they were made for
+        self._native_model = lambda: None               # (a weak reference: an id would be the next model's too)
         self._native_key = None
         self.seed = 0
         self._calls = 0
@@ -237,10 +239,10 @@ class B200Trainer(AbstractBatchProcessor):
         """The library context of an operator group (one per operator the relations use)."""
         cfg = model.config
         op_name = model.operator_name if op_name is None else op_name
-        key = (id(model), cfg.batches_in_flight, cfg.precision)
-        if self._native_key != key:
+        key = (cfg.batches_in_flight, cfg.precision)
+        if self._native_model() is not model or self._native_key != key:
             self._natives = {}
-            self._native_key = key
+            self._native_model, self._native_key = weakref.ref(model), key
         nat = self._natives.get(op_name)
         if nat is None or nat.max_batch < need_batch:
             margin = getattr(self.loss_fn, "margin", cfg.margin)
@@ -392,16 +394,15 @@ class B200RankingEvaluator(AbstractBatchProcessor):
         self.neg_overrides = dict(overrides or {})
         self._native: Optional[_Native] = None
         self._natives: Dict[str, _Native] = {}
-        self._key = None
+        self._native_model = lambda: None
         self.seed = 0
         self._calls = 0
 
     def _context(self, model, need_batch, op_name=None):
         op_name = model.operator_name if op_name is None else op_name
-        key = (id(model),)
-        if self._key != key:
+        if self._native_model() is not model:
             self._natives = {}
-            self._key = key
+            self._native_model = weakref.ref(model)
         nat = self._natives.get(op_name)
         if nat is None or nat.max_batch < need_batch:
             cfg = model.config

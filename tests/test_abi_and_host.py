@@ -249,3 +249,32 @@ def test_bench_names_a_default_tier_per_workload():
     for name, w in bench.WORKLOADS.items():
         assert w.get("precision", "tf32x3") in ("tf32x3", "bf16x6"), name
     assert set(bench.PRECISION_NOTES) == set(_lib.PRECISION_CODES)
+
+
+@pytest.mark.parametrize("kind", ["trainer", "evaluator"])
+def test_contexts_belong_to_a_model_and_not_to_its_address(monkeypatch, kind):
+    """A model made where a freed one lay has the same id() and other sizes: the context of the old one would read its tables with
+    the wrong row width."""
+    from torchbiggraph_b200 import trainer as trainer_module
+    made = []
+
+    class Native:
+        def __init__(self, model, max_batch, *a, **kw):
+            made.append(model.config.dimension)
+            self.max_batch = max_batch
+    monkeypatch.setattr(trainer_module, "_Native", Native)
+    loss_fn = T.LOSS_FUNCTIONS.get_class("softmax")(margin=0.1)
+
+    def model(dim):
+        cfg = T.ConfigSchema(entities={"e": T.EntitySchema()}, relations=[T.RelationSchema("r", "e", "e")], dimension=dim,
+                             comparator="dot", loss_fn="softmax", batch_size=100)
+        return T.make_model(cfg, "cpu")
+    user = T.B200Trainer(None, loss_fn, [1.0]) if kind == "trainer" else T.B200RankingEvaluator(loss_fn, [1.0])
+    if kind == "trainer":
+        user.unpartitioned_optimizers["e"] = T.RowAdagrad([torch.zeros(1, 4)], lr=0.1)
+    monkeypatch.setattr(trainer_module, "id", lambda o: 4711, raising=False)       # every model lies where the last one lay
+    a = model(8)
+    first = user._context(a, 10)
+    assert user._context(a, 100) is first and made == [8]
+    del a
+    assert user._context(model(16), 10) is not first and made == [8, 16]
