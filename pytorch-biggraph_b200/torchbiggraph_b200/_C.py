@@ -96,9 +96,10 @@ def shuffle(tensor: torch.Tensor, permutation: torch.Tensor, num_threads: int = 
         raise ValueError("Tensor and permutation must be on the same device")
     out = torch.empty_like(tensor)
     ctx = _ctx(tensor.device)
-    _sync_torch(tensor.device)
+    permutation = permutation.contiguous()
+    _sync_torch(tensor.device)                              # (behind the last thing PyTorch does for the call)
     row_bytes = tensor[0].numel() * tensor.element_size()
-    _check_value(_lib.lib().pbg_shuffle_rows(ctx, _p(tensor), _p(out), rows, row_bytes, _p(permutation.contiguous())), ctx)
+    _check_value(_lib.lib().pbg_shuffle_rows(ctx, _p(tensor), _p(out), rows, row_bytes, _p(permutation)), ctx)
     tensor.copy_(out)
 
 

@@ -115,3 +115,29 @@ def test_calls_under_another_busy_stream_see_their_arguments():
     got = _calls(model, tr, ev, W, under=busy)
     for i, (a, b) in enumerate(zip(got, want)):
         assert torch.equal(a, b), f"output {i}"
+
+
+def test_shuffle_hands_over_a_permutation_that_is_complete_and_stays(monkeypatch):
+    """A permutation that is not contiguous is copied by PyTorch: in front of the wait for PyTorch's stream, and kept until the
+    library is done with it.  (CPU: a library that only writes down when it is called)"""
+    import weakref
+
+    from torchbiggraph_b200 import _C as native
+    log, copies, contiguous = [], [], torch.Tensor.contiguous
+
+    def copy(self, *a):
+        out = contiguous(self, *a)
+        log.append("copy")
+        copies.append(weakref.ref(out))
+        return out
+
+    def call(*a):
+        assert copies[-1]() is not None and a[-1] == copies[-1]().data_ptr()
+        log.append("call")
+        return 0
+    monkeypatch.setattr(native, "_ctx", lambda device: None)
+    monkeypatch.setattr(native, "_sync_torch", lambda device: log.append("wait"))
+    monkeypatch.setattr(native._lib, "lib", lambda: SimpleNamespace(pbg_shuffle_rows=call))
+    monkeypatch.setattr(torch.Tensor, "contiguous", copy)
+    native.shuffle(torch.zeros(10, 3), torch.arange(20)[::2])
+    assert log == ["copy", "wait", "call"]
