@@ -542,6 +542,13 @@ extern "C" int pbg_kernel_times(pbg_context *c, double *ms_out, int64_t *launche
   return PBG_OK;
 }
 
+// Per-edge weights apply to the next call, whatever becomes of it: the caller may free them when it returns.
+static const float *take_edge_weights(pbg_context *c) {
+  const float *ew = c->edge_w;
+  c->edge_w = nullptr;
+  return ew;
+}
+
 // The second scratch of the three-launch sort, where pbg_create saw no need for it: keys of more than 32 bits.
 static int second_sort(pbg_context *c) {
   if (c->sort[1].max_n) return PBG_OK;
@@ -556,6 +563,7 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
                                  int32_t num_batches, const int64_t *ul, const int64_t *ur, uint64_t seed,
                                  pbg_batch_stats *stats_out) {
   if (!c) return PBG_ERR_BAD_ARGUMENT;
+  const float *ew = take_edge_weights(c);
   if (num_batches == 0) return PBG_OK;
   if (!lhs || !rhs || !batches || num_batches < 0 || num_edges < 0) return fail(c, PBG_ERR_BAD_ARGUMENT, "null edge arrays or batch list");
   CU(c, cudaSetDevice(c->device));
@@ -579,7 +587,7 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
   }
   w.lhs = (const long long *)lhs; w.rhs = (const long long *)rhs; w.rel = (const long long *)rel;
   w.ul = (const long long *)ul; w.ur = (const long long *)ur;
-  w.ew = c->edge_w; c->edge_w = nullptr;                    // per-edge weights apply to one call
+  w.ew = ew;
   w.seed = seed ^ (c->batches_done * 0x9E3779B97F4A7C15ull);
   if (stats_out && num_batches > c->stats_cap) {
     CU(c, cudaStreamSynchronize(c->stream));                 // an earlier call may still write the old array
@@ -723,6 +731,7 @@ extern "C" int pbg_train_batches_host(pbg_context *c, const pbg_bucket *bk, cons
                                       int32_t num_batches, const int64_t *ul, const int64_t *ur, uint64_t seed,
                                       pbg_batch_stats *stats_out) {
   if (!c) return PBG_ERR_BAD_ARGUMENT;
+  const float *ew = take_edge_weights(c);
   if (num_batches == 0) return PBG_OK;
   if (!lhs || !rhs || num_edges < 0) return fail(c, PBG_ERR_BAD_ARGUMENT, "null edge arrays");
   CU(c, cudaSetDevice(c->device));
@@ -745,6 +754,7 @@ extern "C" int pbg_train_batches_host(pbg_context *c, const pbg_bucket *bk, cons
     if (ul) { CU(c, cudaMemcpyAsync(c->uni_dev[0], ul, (size_t)per * 8, cudaMemcpyHostToDevice, c->stream)); uld = c->uni_dev[0]; }
     if (ur) { CU(c, cudaMemcpyAsync(c->uni_dev[1], ur, (size_t)per * 8, cudaMemcpyHostToDevice, c->stream)); urd = c->uni_dev[1]; }
   }
+  c->edge_w = ew;
   return pbg_train_batches(c, bk, (const int64_t *)c->edge_dev[0], (const int64_t *)c->edge_dev[1],
                            rel ? (const int64_t *)c->edge_dev[2] : nullptr, num_edges, batches, num_batches,
                            (const int64_t *)uld, (const int64_t *)urd, seed, stats_out);
@@ -800,7 +810,9 @@ extern "C" int pbg_score_batch(pbg_context *c, const pbg_bucket *bk, const int64
 extern "C" int pbg_eval_batch(pbg_context *c, const pbg_bucket *bk, const int64_t *lhs, const int64_t *rhs,
                               const int64_t *rel, int32_t count, int32_t relidx, const int64_t *ul, const int64_t *ur,
                               uint64_t seed, pbg_eval_stats *out) {
-  if (!c || !out) return PBG_ERR_BAD_ARGUMENT;
+  if (!c) return PBG_ERR_BAD_ARGUMENT;
+  const float *ew = take_edge_weights(c);
+  if (!out) return PBG_ERR_BAD_ARGUMENT;
   memset(out, 0, sizeof *out);
   if (count == 0) return PBG_OK;
   if (!lhs || !rhs || count < 0 || count > c->cfg.max_batch_size)
@@ -813,7 +825,7 @@ extern "C" int pbg_eval_batch(pbg_context *c, const pbg_bucket *bk, const int64_
   if (!d.dynamic && (relidx < 0 || relidx >= c->cfg.num_rels)) return fail(c, PBG_ERR_INDEX_RANGE, "relation %d outside [0, %d)", relidx, c->cfg.num_rels);
   if (d.dynamic && d.op != PBG_OP_NONE && !rel) return fail(c, PBG_ERR_BAD_ARGUMENT, "dynamic relations need the rel array");
   w.lhs = (const long long *)lhs; w.rhs = (const long long *)rhs; w.rel = (const long long *)rel;
-  w.ew = c->edge_w; c->edge_w = nullptr;
+  w.ew = ew;
   w.ul = (const long long *)ul; w.ur = (const long long *)ur; w.seed = seed;
   WaveBatches wb;
   memset(&wb, 0, sizeof wb);
@@ -837,7 +849,9 @@ extern "C" int pbg_eval_batch(pbg_context *c, const pbg_bucket *bk, const int64_
 
 extern "C" int pbg_eval_batch_all_negs(pbg_context *c, const pbg_bucket *bk, const int64_t *lhs, const int64_t *rhs,
                                        const int64_t *rel, int32_t count, int32_t relidx, uint64_t seed, pbg_eval_stats *out) {
-  if (!c || !out) return PBG_ERR_BAD_ARGUMENT;
+  if (!c) return PBG_ERR_BAD_ARGUMENT;
+  const float *ew = take_edge_weights(c);
+  if (!out) return PBG_ERR_BAD_ARGUMENT;
   memset(out, 0, sizeof *out);
   if (count == 0) return PBG_OK;
   if (!lhs || !rhs || count < 0 || count > c->cfg.max_batch_size)
@@ -858,7 +872,7 @@ extern "C" int pbg_eval_batch_all_negs(pbg_context *c, const pbg_bucket *bk, con
     c->allnegs_rows = most_rows;
   }
   w.lhs = (const long long *)lhs; w.rhs = (const long long *)rhs; w.rel = (const long long *)rel;
-  w.ew = c->edge_w; c->edge_w = nullptr;
+  w.ew = ew;
   w.seed = seed;
   const float wrel = bk->relation_weights ? bk->relation_weights[d.dynamic ? 0 : relidx] : 1.0f;
   c->launches += launch_allnegs_eval(d, w, c->allnegs_mem, c->cfg.max_batch_size, count, c->allnegs_slab, planes, d.dynamic ? 0 : relidx, wrel,

@@ -143,3 +143,21 @@ def test_relations_with_different_operators_train_like_the_oracle():
     np.testing.assert_allclose(W.cpu().numpy(), Wo, rtol=RTOL, atol=2e-6)
     for o in th:
         np.testing.assert_allclose(model.op_tables[o].cpu().numpy(), states[o].theta_rhs, rtol=RTOL, atol=2e-6, err_msg=o)
+
+
+@pytest.mark.parametrize("edges", ["cuda", "cpu"])
+def test_edge_weights_of_a_refused_call_are_not_the_next_call_s(edges):
+    """The weights belong to the caller, who frees them when the call fails: the library must not have kept their address."""
+    from torchbiggraph_b200 import _lib
+    T, build, lhs, rhs, _, wgt = _setup(False)
+    t = lambda a: torch.tensor(np.asarray(a)).to(edges)
+    results = []
+    for refused in (False, True):
+        model, tr, W, _ = build()
+        nat = tr._context(model, 100)
+        if refused:
+            with pytest.raises(_lib.PbgError, match="max_batch_size"):       # a batch that reaches past the list's end
+                tr.train_batches(model, t(lhs), t(rhs), None, [(len(lhs) - 50, 100, 0)], weights=torch.tensor(wgt))
+        stats = tr.train_batches(model, t(lhs), t(rhs), None, [(i * 100, 100, 0) for i in range(7)])
+        results.append((W.cpu(), [s.metrics["loss"] for s in stats]))
+    assert torch.equal(results[0][0], results[1][0]) and results[0][1] == results[1][1]
