@@ -168,7 +168,8 @@ int pbg_train_batches(pbg_context *ctx, const pbg_bucket *bucket,
 
 /* Same, with the edge arrays (and optional uniform ids) in HOST memory: copies them to the
  * device asynchronously on the context's stream ahead of the first wave (8 to 24 bytes per
- * edge, against ~50 KB per edge of table traffic).  This is the call that stands where
+ * edge, against ~50 KB per edge of table traffic; pinned arrays stay as they are until the
+ * stream has passed the copies, which with stats_out it has when the call returns).  This is the call that stands where
  * GPUProcess.do_one_job moves a bucket's edges to the GPU and trains on them
  * (torchbiggraph/train_gpu.py:243-266). */
 int pbg_train_batches_host(pbg_context *ctx, const pbg_bucket *bucket,
@@ -180,8 +181,8 @@ int pbg_train_batches_host(pbg_context *ctx, const pbg_bucket *bucket,
 /* Per-edge weights (EdgeList.weight of the reference: every loss multiplies the loss of a positive
  * and of its negatives by the edge's weight, torchbiggraph/losses.py:65-78, 104-113, 145-157).
  * weights_dev: DEVICE float array parallel to the edge arrays of the NEXT pbg_train_batches,
- * pbg_train_batches_host or pbg_eval_batch call on this context; that call uses it and clears
- * it.  NULL clears it at once.  Without this call every edge weighs 1. */
+ * pbg_train_batches_host or pbg_eval_batch(_all_negs) call on this context; that call uses it
+ * and clears it, refused or not.  NULL clears it at once.  Without this call every edge weighs 1. */
 int pbg_set_edge_weights(pbg_context *ctx, const float *weights_dev);
 
 /* Sum of the stats of every batch trained since the last call of this function (device

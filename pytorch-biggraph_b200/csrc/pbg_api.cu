@@ -161,12 +161,35 @@ static int chunk_geometry(const pbg_config &cfg, int *Pm, int *Cm) {
 // Whether the fused score + loss kernel and the dual gradient product take less time than the kernels they replace (score,
 // loss, merged coefficients, gradient).  The fused kernel gives a chunk block to one CTA, its loss included: fewer and
 // shorter launches where the blocks of a full wave fill the SMs, a long single epilogue where they do not.  Measured time
-// of the separate kernels over that of the fused ones (whole buckets, 50 to 200 score columns, dimensions 64 / 256 / 512 / 1024):
-//   softmax   12 to 24 blocks 0.8-1.0 (any dimension); 80 to 280: three planes 1.15 / 1.09 / 1.02 / 0.99, two planes 1.25 / 1.16 /
-//             1.08 / 1.03; 32 and 60: three planes 1.15 / 1.0 / 0.94, two planes 1.15 / 1.09 / 1.02
-//   logistic  (log1p and exp of every score in the epilogue) 12 to 60 blocks 0.73-1.0; 80 to 280: three planes 1.1 / 1.03 /
-//             0.99 / 0.97, two planes 1.17 / 1.1 / 1.05 / 1.0
-// Ranking keeps to the dimension alone: hinges turn the two forms' different roundings into different trajectories.
+// of the separate kernels over that of the fused ones (whole buckets, 300,000 rows; 100 / 200 score columns):
+//                        dimension 64    256          512          1024
+//   softmax, three planes
+//     12, 24 blocks      1.01 / 0.89     0.94 / 0.86  0.86 / 0.84  0.79 / 0.81
+//     32, 60             1.12 / 1.02     1.03 / 0.98  0.97 / 0.94  0.94 / 0.93
+//     80, 140, 280       1.17 / 1.15     1.09 / 1.10  1.03 / 1.03  0.99 / 0.97
+//   softmax, two planes
+//     12, 24             1.06 / 0.96     1.00 / 0.94  0.95 / 0.92  0.91 / 0.90
+//     32, 60             1.16 / 1.08     1.09 / 1.04  1.05 / 1.02  1.04 / 0.98
+//     80, 140, 280       1.21 / 1.26     1.15 / 1.17  1.09 / 1.09  1.05 / 1.03
+//   logistic (log1p and exp of every score in the epilogue), three planes
+//     12 to 60           0.97 / 0.85     0.91 / 0.83  0.86 / 0.82  0.83 / 0.83
+//     80, 140, 280       1.08 / 1.14     1.07 / 1.07  1.01 / 1.02  0.97 / 0.98
+//   logistic, two planes
+//     12 to 60           0.98 / 0.88     0.96 / 0.88  0.94 / 0.88  0.93 / 0.88
+//     80, 140, 280       1.12 / 1.21     1.11 / 1.13  1.07 / 1.07  1.04 / 1.02
+//   ranking, three planes
+//     12, 24             1.04 / 0.90     0.95 / 0.86  0.87 / 0.84  0.80 / 0.81
+//     32, 60             1.12 / 1.05     1.03 / 0.98  0.98 / 0.95  0.95 / 0.93
+//     80, 140, 280       1.17 / 1.18     1.10 / 1.12  1.04 / 1.04  0.99 / 1.01
+//   ranking, two planes
+//     12, 24             1.13 / 0.97     1.05 / 0.94  0.97 / 0.92  0.92 / 0.90
+//     32, 60             1.18 / 1.10     1.10 / 1.06  1.06 / 1.02  1.05 / 1.00
+//     80, 140, 280       1.21 / 1.30     1.16 / 1.19  1.10 / 1.10  1.06 / 1.05
+// The lines follow the table where it is clear of the few percent by which runs differ; left on the table are softmax in two
+// planes at dimension 512 with 32 to 60 blocks and logistic in two planes above 512.  Ranking does not follow it: the forms
+// round differently, hinges turn that into other trajectories, and its line at dimension 256 is the one its results were
+// made with.  That costs up to 16 % below 25 blocks with 200 columns, and 10 % in two planes at dimension 512.
+// `blocks` are those of a full wave: a list of fewer batches is launched in the form chosen for it all the same.
 static bool fused_pays(const pbg_config &cfg, int npl, long long blocks) {
   if (cfg.loss == PBG_LOSS_RANKING) return cfg.dim <= 256;
   if (cfg.loss == PBG_LOSS_SOFTMAX) return blocks > 24 && cfg.dim <= (blocks < 72 ? 256 : npl == 2 ? 1024 : 512);

@@ -37,7 +37,8 @@
 enum { ARR_N0 = 0, ARR_N1 = 1, ARR_Q0 = 2, ARR_Q1 = 3, ARR_R0 = 4, ARR_R1 = 5 };
 
 // Division of slot and block numbers (below 2^31) by a size that is fixed for the launch: one high multiply and a shift
-// instead of the twenty-odd instructions of an integer division.  With l = ceil(log2 d) and m = ceil(2^(31 + l) / d),
+// instead of the twenty-odd instructions of an integer division (Granlund and Montgomery, division by invariant integers
+// using multiplication).  With l = ceil(log2 d) and m = ceil(2^(31 + l) / d),
 // n / d = floor(n m / 2^(31 + l)): m exceeds the exact quotient by less than 1, so the product exceeds n / d by less
 // than n / 2^(31 + l) < 1 / d.  Kernels of a few hundred instructions per row of 100 floats spend a quarter of them on five
 // such divisions.

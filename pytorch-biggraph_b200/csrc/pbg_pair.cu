@@ -170,14 +170,15 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
     }
   } else if (warp >= 2) {
     // ---------------- epilogue: loss, statistics and coefficient planes of both problems ----------------
-    // Sixteen warps: the four warps that share a tensor-memory lane group (rows i = q * 32 + lane) take two
-    // 32-column chunks of the row each and combine their partial maxima / sums through shared memory.  A chunk
-    // is read from tensor memory, reduced, and (softmax) its exponentials are written back over the scores, so
-    // that every score costs one exponential and no more than 32 values are ever held in registers.
+    // Sixteen warps: the four warps that share a tensor-memory lane group (rows i = q * 32 + lane) take four
+    // 16-column chunks of the row each (two of them in the narrow form) and combine their partial maxima / sums through
+    // shared memory.  A chunk is read from tensor memory, reduced, and what its coefficients are made of (exponentials,
+    // indicators, sigmoids) is written back over the scores, so that every score costs one exponential and no more than 16
+    // values are ever held in registers.
     long long j = 0;
     const int q = warp & 3;                            // the 32 tensor-memory lanes this warp may read
     const int wg = (warp - 2) >> 2;
-    const int cg = NARROW ? wg & 1 : wg;               // column group: chunks 2 cg and 2 cg + 1
+    const int cg = NARROW ? wg & 1 : wg;               // column group: 64 columns
     const int p0 = NARROW ? wg >> 1 : 0, p1 = NARROW ? p0 + 1 : 2;       // the problems of this warp
     const int i = q * 32 + lane;                       // positive row of the chunk
     const int Mm = d.Mm, Pm = d.Pm;

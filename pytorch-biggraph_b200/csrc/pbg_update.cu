@@ -390,15 +390,16 @@ struct RowState {
 #define TILE_WARPS_EMB 4
 #define UPD_WAIT_LIMIT 4000000
 
-// The operator rows' slots are staged from GR (dyn_pullback_kernel), eight warps per CTA.
-// Resident CTAs per SM: rows of up to 256 floats are bound by the latency of a slot's chain of loads, not by bytes, and
-// gain from twice the warps at the price of a few dozen bytes of spills (dimension 200: update 55.8 -> 52.5 ms per 2.16 M
-// edges); the wide rows stay at the register count that keeps them spill-free.
+// (Embedding rows of up to 256 floats have a kernel of their own, narrow_tile_kernel.)
+// The operator rows' slots are staged from GR (dyn_pullback_kernel), eight warps per CTA, four above 1024 floats.
+// Resident CTAs per SM: operator rows of up to 256 floats are bound by the latency of a slot's chain of loads, not by bytes,
+// and gain from twice the warps (dimension 200, when both kinds of rows had it: update 55.8 -> 52.5 ms per 2.16 M edges); the
+// wide rows stay at the register count that keeps them all but free of spills.
 template <int VEC, int RULE>
 struct TileWarps { enum { N = RULE == RULE_EMB ? TILE_WARPS_EMB : VEC > 8 ? UPD_WARPS / 2 : UPD_WARPS }; };
 
 template <int VEC, int RULE>
-__global__ void __launch_bounds__(32 * TileWarps<VEC, RULE>::N, RULE == RULE_EMB ? (VEC == 2 ? 6 : 3) : (VEC == 2 ? 4 : 2))
+__global__ void __launch_bounds__(32 * TileWarps<VEC, RULE>::N, RULE == RULE_EMB ? 3 : VEC == 2 ? 4 : 2)
 tile_update_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__restrict__ keys,
                    const unsigned int *__restrict__ vals, float lr, float *__restrict__ psum,
                    long long *__restrict__ hublist, int *__restrict__ hubcnt, ParamJob job, int aside) {
