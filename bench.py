@@ -57,8 +57,7 @@ EDGES_PER_STEP_CAP = 269_507
 #   traffic_per_edge_bytes: gather=... score=... grad=... update=... csrc_sha256=<digest>
 # where the digest is csrc_digest() of the kernel sources the capture ran.  A summary whose digest is
 # not that of the sources in the tree describes other kernels: its figures are then not used.
-PROFILE_FILES = {("c3", "tf32x3"): "kernels_c3_tf32x3.md", ("c3", "bf16x6"): "kernels_c3_bf16x6.md",
-                 ("c3", "bf16x3"): "kernels_c3_bf16x3.md"}
+PROFILE_FILES = {("c3", "bf16x6"): "kernels_c3_bf16x6.md"}
 
 
 def csrc_digest():
