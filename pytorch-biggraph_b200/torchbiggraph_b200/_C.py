@@ -6,6 +6,7 @@ The reference runs them on host threads over CPU tensors; here the tensors live 
 PyTorch only owns the memory.  Errors keep the reference's types: what util.cpp throws as
 std::invalid_argument arrives as ValueError, std::runtime_error as RuntimeError."""
 import ctypes as C
+import threading
 from typing import Dict, List, Sequence, Tuple
 
 import torch
@@ -13,6 +14,9 @@ import torch
 from . import _lib
 
 _contexts: Dict[int, C.c_void_p] = {}
+# Held around every call: the reference's functions may run on several threads, and a context has one error word, one scratch
+# that grows, one set of counters.
+_lock = threading.Lock()
 
 
 def _ctx(device: torch.device) -> C.c_void_p:
@@ -46,6 +50,13 @@ def _sync_torch(device):
         s.synchronize()
 
 
+def _ready(device: torch.device) -> C.c_void_p:
+    """The device's context, behind everything PyTorch has been asked to do for the call so far."""
+    ctx = _ctx(device)
+    _sync_torch(device)
+    return ctx
+
+
 def randperm(num_items: int, num_threads: int = 1, seed: int = -1, device="cuda") -> torch.Tensor:
     """util.cpp:14-101: a random permutation of range(num_items) as an int64 tensor.  seed < 0 draws one from
     PyTorch's generator (the reference then uses its default seed)."""
@@ -53,9 +64,9 @@ def randperm(num_items: int, num_threads: int = 1, seed: int = -1, device="cuda"
     if seed < 0:
         seed = int(torch.randint(0, 2**62, (1,)).item())
     out = torch.empty(num_items, dtype=torch.long, device=device)
-    ctx = _ctx(out.device)
-    _sync_torch(out.device)
-    _lib.check(_lib.lib().pbg_randperm(ctx, num_items, seed, _p(out)), ctx)
+    with _lock:
+        ctx = _ready(out.device)
+        _lib.check(_lib.lib().pbg_randperm(ctx, num_items, seed, _p(out)), ctx)
     return out
 
 
@@ -65,9 +76,9 @@ def reverse_permutation(perm: torch.Tensor, num_threads: int = 1) -> torch.Tenso
         raise ValueError("Permutation must be a 1-dimensional int64 tensor")
     perm = perm.contiguous()
     out = torch.empty_like(perm)
-    ctx = _ctx(perm.device)
-    _sync_torch(perm.device)
-    _check_value(_lib.lib().pbg_reverse_permutation(ctx, _p(perm), perm.shape[0], _p(out)), ctx)
+    with _lock:
+        ctx = _ready(perm.device)
+        _check_value(_lib.lib().pbg_reverse_permutation(ctx, _p(perm), perm.shape[0], _p(out)), ctx)
     return out
 
 
@@ -95,11 +106,11 @@ def shuffle(tensor: torch.Tensor, permutation: torch.Tensor, num_threads: int = 
     if tensor.device != permutation.device:
         raise ValueError("Tensor and permutation must be on the same device")
     out = torch.empty_like(tensor)
-    ctx = _ctx(tensor.device)
     permutation = permutation.contiguous()
-    _sync_torch(tensor.device)                              # (behind the last thing PyTorch does for the call)
     row_bytes = tensor[0].numel() * tensor.element_size()
-    _check_value(_lib.lib().pbg_shuffle_rows(ctx, _p(tensor), _p(out), rows, row_bytes, _p(permutation)), ctx)
+    with _lock:
+        ctx = _ready(tensor.device)
+        _check_value(_lib.lib().pbg_shuffle_rows(ctx, _p(tensor), _p(out), rows, row_bytes, _p(permutation)), ctx)
     tensor.copy_(out)
 
 
@@ -116,7 +127,6 @@ def sub_bucket(lhs_in: torch.Tensor, rhs_in: torch.Tensor, rel_in: torch.Tensor,
     for t in (lhs_in, rhs_in, rel_in, lhs_out, rhs_out, rel_out):
         if t.dtype != torch.long or t.dim() != 1 or t.shape[0] != n or not t.is_contiguous():
             raise ValueError("edge tensors must be contiguous 1-dimensional int64 tensors of one length")
-    ctx = _ctx(lhs_in.device)
     lperms = [p.contiguous() for p in lhs_perms]
     rperms = [p.contiguous() for p in rhs_perms]
     lc = (C.c_int64 * R)(*[int(x) for x in lhs_entity_counts])
@@ -125,12 +135,13 @@ def sub_bucket(lhs_in: torch.Tensor, rhs_in: torch.Tensor, rel_in: torch.Tensor,
     rp = (C.c_void_p * R)(*[p.data_ptr() for p in rperms])
     nb = num_lhs_sub_parts * num_rhs_sub_parts
     counts = (C.c_int64 * nb)()
-    _sync_torch(lhs_in.device)
-    st = _lib.lib().pbg_sub_bucket(ctx, _p(lhs_in), _p(rhs_in), _p(rel_in), n, R, lc, lp, rc, rp, _p(lhs_out), _p(rhs_out),
-                                   _p(rel_out), num_lhs_sub_parts, num_rhs_sub_parts, int(bool(dynamic_relations)), counts)
-    if st == _lib.PBG_ERR_INDEX_RANGE:
-        raise RuntimeError(_lib.lib().pbg_last_error(ctx).decode())
-    _lib.check(st, ctx)
+    with _lock:
+        ctx = _ready(lhs_in.device)
+        st = _lib.lib().pbg_sub_bucket(ctx, _p(lhs_in), _p(rhs_in), _p(rel_in), n, R, lc, lp, rc, rp, _p(lhs_out), _p(rhs_out),
+                                       _p(rel_out), num_lhs_sub_parts, num_rhs_sub_parts, int(bool(dynamic_relations)), counts)
+        if st == _lib.PBG_ERR_INDEX_RANGE:
+            raise RuntimeError(_lib.lib().pbg_last_error(ctx).decode())
+        _lib.check(st, ctx)
     res, start = {}, 0
     for i in range(num_lhs_sub_parts):
         for j in range(num_rhs_sub_parts):

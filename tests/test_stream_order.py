@@ -141,3 +141,33 @@ def test_shuffle_hands_over_a_permutation_that_is_complete_and_stays(monkeypatch
     monkeypatch.setattr(torch.Tensor, "contiguous", copy)
     native.shuffle(torch.zeros(10, 3), torch.arange(20)[::2])
     assert log == ["copy", "wait", "call"]
+
+
+def test_edge_list_utilities_use_a_context_for_one_thread_at_a_time(monkeypatch):
+    """The reference's functions may run on several threads; here they share a device's context (one error word, scratch that
+    grows).  (CPU: a library that writes down who is inside it)"""
+    import threading
+    import time
+
+    from torchbiggraph_b200 import _C as native
+    inside, most = [], []
+
+    def call(*a):
+        inside.append(1)
+        most.append(len(inside))
+        time.sleep(0.02)
+        inside.pop()
+        return 0
+    fake = SimpleNamespace(pbg_shuffle_rows=call, pbg_reverse_permutation=call, pbg_randperm=call, pbg_sub_bucket=call)
+    monkeypatch.setattr(native, "_ctx", lambda device: None)
+    monkeypatch.setattr(native, "_sync_torch", lambda device: None)
+    monkeypatch.setattr(native._lib, "lib", lambda: fake)
+    e = torch.zeros(4, dtype=torch.long)
+    calls = [lambda: native.randperm(4, seed=1, device="cpu"), lambda: native.reverse_permutation(e), lambda: native.shuffle(torch.zeros(4, 2), e),
+             lambda: native.sub_bucket(e, e, e, [4], [e], [4], [e], e.clone(), e.clone(), e.clone(), 1, 1)]
+    threads = [threading.Thread(target=c) for c in calls * 2]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(most) == 8 and max(most) == 1
