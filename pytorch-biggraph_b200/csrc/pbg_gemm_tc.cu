@@ -151,16 +151,16 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
 
   if (warp == 0) {
     // ---------------- TMA producer (one box per operand, each from its own lane) ----------------
-    long long git = 0;
+    StageRing at;
     bool stop = false;
     for (int t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
       int p, blk, m0, n0;
       if (__any_sync(0xffffffffu, failed != 0)) break;
       if (!tile_live(t, p, blk, m0, n0)) continue;
-      for (int kb = 0; kb < nkb; ++kb, ++git) {
-        int s = (int)(git % STAGES);
+      for (int kb = 0; kb < nkb; ++kb, at.next(STAGES)) {
+        const int s = at.s;
         bool okw = true;
-        if (git >= STAGES && lane == 0) okw = mbar_wait(empty_bar(s), (uint32_t)((git / STAGES) - 1) & 1, errflag);
+        if (lane == 0) okw = mbar_wait(empty_bar(s), at.parity ^ 1u, errflag);
         if (!__all_sync(0xffffffffu, okw)) { failed = 1; stop = true; break; }
         uint32_t fb = full_bar(s);
         const bool with_b1 = !dual || kb < nkb1;
@@ -187,20 +187,21 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
     const uint32_t fmt = PLANES ? 1u : 2u;            // operand format: bf16 (kind::f16) or tf32
     const uint32_t idesc0 = (1u << 4) | (fmt << 7) | (fmt << 10) | ((A_MN ? 1u : 0u) << 15) | ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(128 >> 4) << 24);
     const uint32_t idesc2 = (idesc0 & ~(1u << 16)) | ((uint32_t)(g.BN2 >> 3) << 17);   // dual: the B2 products are K-major, BN2 columns wide
-    long long git = 0, j = 0;
+    StageRing at;
+    int j = 0;
     for (int t = blockIdx.x; t < ntiles && !failed; t += gridDim.x) {
       int p, blk, m0, n0;
       if (!tile_live(t, p, blk, m0, n0)) continue;
-      const int ab = (int)(j & 1);
+      const int ab = j & 1;
       if (j >= 2 && !mbar_wait(acce_bar(ab), (uint32_t)((j >> 1) - 1) & 1, errflag)) { failed = 1; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tacc = tmem + (uint32_t)ab * 256u;
       const int ncols = g.N - n0 < g.BN ? (g.N - n0 + 15) / 16 * 16 : g.BN;                 // columns of this tile that exist
       const uint32_t idesc = idesc0 | ((uint32_t)(ncols >> 3) << 17);
       bool ok = true;
-      for (int kb = 0; kb < nkb; ++kb, ++git) {
-        int s = (int)(git % STAGES);
-        if (!mbar_wait(SPLIT ? conv_bar(s) : full_bar(s), (uint32_t)(git / STAGES) & 1, errflag)) { failed = 1; ok = false; break; }
+      for (int kb = 0; kb < nkb; ++kb, at.next(STAGES)) {
+        const int s = at.s;
+        if (!mbar_wait(SPLIT ? conv_bar(s) : full_bar(s), at.parity, errflag)) { failed = 1; ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         unsigned char *st = smem + (size_t)s * stage_bytes;
         uint32_t aH = smem_u32(st), bH = smem_u32(st + A_BYTES);
@@ -273,18 +274,18 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
     // ---------------- hi / lo split of every landed stage (warps 6-13) ----------------
     const int ct = threadIdx.x - 192;                             // 0..255
     const uint32_t nchunks = stage_tx / 16;
-    long long git = 0;
+    StageRing at;
     bool stop = false;
     for (int t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
       int p, blk, m0, n0;
       if (__any_sync(0xffffffffu, failed != 0)) break;           // warp-uniform exit
       if (!tile_live(t, p, blk, m0, n0)) continue;
-      for (int kb = 0; kb < nkb; ++kb, ++git) {
-        int s = (int)(git % STAGES);
+      for (int kb = 0; kb < nkb; ++kb, at.next(STAGES)) {
+        const int s = at.s;
         // one lane per warp polls the barrier (256 polling threads would take issue slots from the warps
         // that have work); the warp-wide vote that follows orders the other lanes' reads after it
         bool okw = true;
-        if (lane == 0) okw = mbar_wait(full_bar(s), (uint32_t)(git / STAGES) & 1, errflag);
+        if (lane == 0) okw = mbar_wait(full_bar(s), at.parity, errflag);
         if (!__all_sync(0xffffffffu, okw)) { failed = 1; stop = true; break; }
         unsigned char *st = smem + (size_t)s * stage_bytes;
         for (uint32_t c0 = ct; c0 < nchunks; c0 += 4 * TC_SPLIT_THREADS) {
@@ -310,13 +311,13 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
     }
   } else if (warp >= 2 && warp < 6) {
     // ---------------- epilogue: drains accumulator j & 1 while the next tile is being multiplied ----------------
-    long long j = 0, nst = 0;
+    int j = 0, nst = 0;
     const int q = warp & 3;                           // the 32 TMEM lanes this warp may read
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
       int p, blk, m0, n0;
       if (__any_sync(0xffffffffu, failed != 0)) break;           // warp-uniform exit (tcgen05.ld is warp-wide)
       if (!tile_live(t, p, blk, m0, n0)) continue;
-      const int ab = (int)(j & 1);
+      const int ab = j & 1;
       bool okw = true;
       if (lane == 0) okw = mbar_wait(accf_bar(ab), (uint32_t)(j >> 1) & 1, errflag);
       if (!__all_sync(0xffffffffu, okw)) { failed = 1; break; }
@@ -347,7 +348,7 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
         // the buffer used two blocks ago must have been read by its store before it is rewritten
         if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
         __syncwarp();
-        unsigned char *buf = ostage + (size_t)(q * 2 + (int)(nst & 1)) * 4096;
+        unsigned char *buf = ostage + (size_t)(q * 2 + (nst & 1)) * 4096;
         ++nst;
         if (g.tr) {
           // transposed output: column jj of the block is row jj of the store box, this lane's tile row its

@@ -106,16 +106,16 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
 
   if (warp == 0) {
     // ---------------- TMA producer: one box (all planes) per operand array, each from its own lane ----------------
-    long long git = 0;
+    StageRing at;
     bool stop = false;
     for (int t = blockIdx.x; t < d.nblk && !stop; t += gridDim.x) {
       if (__any_sync(0xffffffffu, failed != 0)) break;
       if (!tile_live(t)) continue;
       const int blk = d.blk0 + t;
-      for (int kb = 0; kb < nkb; ++kb, ++git) {
-        const int s = (int)(git % STAGES);
+      for (int kb = 0; kb < nkb; ++kb, at.next(STAGES)) {
+        const int s = at.s;
         bool okw = true;
-        if (git >= STAGES && lane == 0) okw = mbar_wait(empty_bar(s), (uint32_t)((git / STAGES) - 1) & 1, errflag);
+        if (lane == 0) okw = mbar_wait(empty_bar(s), at.parity ^ 1u, errflag);
         if (!__all_sync(0xffffffffu, okw)) { failed = 1; stop = true; break; }
         const uint32_t fb = full_bar(s);
         if (lane == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(fb), "r"(stage_tx) : "memory");
@@ -130,17 +130,18 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
     // plane pairs (a, b) of order a + b <= 2, the smallest contributions first; two planes: the last three
     const int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
     constexpr int T0 = NPL == 3 ? 0 : 3;
-    long long git = 0, j = 0;
+    StageRing at;
+    int j = 0;
     for (int t = blockIdx.x; t < d.nblk && !failed; t += gridDim.x) {
       if (!tile_live(t)) continue;
-      const int set = (int)(j % SETS);
+      const int set = j % SETS;
       const uint32_t tset = tmem + (uint32_t)set * 2u * ACC;
       if (j >= SETS && !mbar_wait(acce_bar(set), (uint32_t)(j / SETS - 1) & 1, errflag)) { failed = 1; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       bool ok = true;
-      for (int kb = 0; kb < nkb; ++kb, ++git) {
-        const int s = (int)(git % STAGES);
-        if (!mbar_wait(full_bar(s), (uint32_t)(git / STAGES) & 1, errflag)) { failed = 1; ok = false; break; }
+      for (int kb = 0; kb < nkb; ++kb, at.next(STAGES)) {
+        const int s = at.s;
+        if (!mbar_wait(full_bar(s), at.parity, errflag)) { failed = 1; ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t st = smem_u32(smem + (size_t)s * g.stage_bytes);
         const int kleft = d.D - kb * 32;
@@ -175,7 +176,7 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
     // shared memory.  A chunk is read from tensor memory, reduced, and what its coefficients are made of (exponentials,
     // indicators, sigmoids) is written back over the scores, so that every score costs one exponential and no more than 16
     // values are ever held in registers.
-    long long j = 0;
+    int j = 0;
     const int q = warp & 3;                            // the 32 tensor-memory lanes this warp may read
     const int wg = (warp - 2) >> 2;
     const int cg = NARROW ? wg & 1 : wg;               // column group: 64 columns
@@ -198,7 +199,7 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
       // One thread waits for the accumulators (a bounded wait) and tells the others through shared memory: all
       // sixteen warps take the same decision, so that none is left alone at the named barrier further down.
       if (warp == 2 && lane == 0) {
-        bool go = failed == 0 && mbar_wait(accf_bar((int)(j % SETS)), (uint32_t)(j / SETS) & 1, errflag);
+        bool go = failed == 0 && mbar_wait(accf_bar(j % SETS), (uint32_t)(j / SETS) & 1, errflag);
         if (!go) failed = 1;
         epi_go = go ? 1 : 0;
       }
@@ -363,7 +364,7 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(acce_bar((int)(j % SETS))) : "memory");
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(acce_bar(j % SETS)) : "memory");
       ++j;
     }
   }

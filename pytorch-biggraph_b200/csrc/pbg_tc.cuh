@@ -20,6 +20,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int *er
   return false;
 }
 
+// Place in a ring of stages: which one, and the parity of the pass over the ring.  The consumer of a stage waits for `parity`,
+// its producer for the other one (a fresh barrier lets it through).  Counted, not divided out of a running number: in the plane
+// tiers, whose number of stages is known at run time, a 64-bit division by it stood in front of every wait of the producer and
+// of the thread that issues the products (two planes, 1000-row chunks at dimension 400: gradients 7.83 ms with it, 6.80 without;
+// dual gradient of 20-chunk waves at dimension 100, three planes: 28.8 and 26.1 us).
+struct StageRing {
+  int s = 0;
+  uint32_t parity = 0;
+  __device__ __forceinline__ void next(int stages) { if (++s == stages) { s = 0; parity ^= 1u; } }
+};
+
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, uint32_t bar) {
   asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                :: "r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar) : "memory");
