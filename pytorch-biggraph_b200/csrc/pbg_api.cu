@@ -47,6 +47,7 @@ struct pbg_context {
   void *tcplan = nullptr;       // tensor maps of the tcgen05 contractions
   void *pairplan = nullptr;     // tensor maps of the fused score + loss kernel (standard relations, plane tiers)
   bool fused = false;           // training runs gather -> fused score / loss -> dual gradient product
+  bool chunk = false;           // training and scoring run one kernel from the ids to the gradient rows (pbg_chunk.cu)
   float *psum = nullptr;        // partial gradient rows of hub rows, indexed by slot position
   long long *hublist = nullptr;
   int *hubcnt = nullptr;        // two sets of counters, used in turn
@@ -196,6 +197,39 @@ static bool fused_pays(const pbg_config &cfg, int npl, long long blocks) {
   return blocks >= 72 && cfg.dim <= (npl == 2 ? 512 : 256);
 }
 
+// Whether the blocks of a full wave go through chunk_kernel, a cluster of CTAs each, in place of gather, score, loss, gradient
+// and pull-back kernels.  Its products run on the CUDA cores and a CTA works through its tiles one after the other, so it takes
+// blocks that leave each CTA with one tile of scores (64 edges) and one of gradient rows.  Measured time of the separate kernels
+// over that of this one (k = 1, lists of 30 batches over 50,000 rows, per batch; 10 / 20 / 28 blocks of a wave, ranges over
+// comparators, losses and operators):
+//                                      dimension 16        104, 128             160              256
+//   fp32, standard    10 + 5 columns   1.05 / 1.03 / 1.04  1.2  / 1.2  / 1.2    1.1              1.2
+//                     30 + 60          1.2  / 1.1  / 1.1   1.3  / 1.4  / 1.45   1.2  / 1.3       1.4  / 1.5
+//                     64 + 64          1.2  / 1.1  / 1.2   1.5  / 1.35 / 1.4    1.3  / 1.15 / 1.04  1.5 / 1.3 / 1.08
+//   fp32, dynamic     30 + 60          1.0 - 1.1           1.1  / 1.2  / 1.3    1.1  / 1.3       1.25 / 1.45
+//                     64 + 20, two     0.95 / 1.04 / 1.07  0.99 / 1.14 / 1.25   0.98 / 1.06      1.05 / 1.17
+//   tf32x3, standard  10 + 5           1.2  / 1.15 / 1.15  1.2                  1.1              1.15
+//   (bf16x6 alike)    30 + 60          1.2  / 1.1  / 1.1   1.25 / 1.1  / 1.15   1.1  / 0.95      1.1  / 0.97
+//                     64 + 64          1.2  / 1.05 / 1.1   1.2  / 1.03 / 1.1    1.0  / 0.86      1.0  / 0.87
+//                     100 + 50, two    0.8  / 0.75         0.8  / 0.7           0.6  / 0.5       0.6  / 0.5
+//                     36 blocks, 50 + 50   0.85            0.83                 0.75             0.74
+//   tf32x3, dynamic   10 + 5           1.1 - 1.2           1.15 - 1.25          1.06 - 1.17      1.1  - 1.2
+//                     30 + 60          0.96 - 1.1          1.0  - 1.15          0.91 - 1.05      0.95 - 1.1
+//                     50 + 50, two     0.85                0.85 - 0.9           0.83 - 0.94      0.83 - 0.96
+//   bf16x3, standard  l2: 1.1 - 1.2, dot and cos: 0.95 - 1.06 (its two-plane products are the shortest there are)
+// The fp32 tier's own products are on the CUDA cores too (and equal to these bit for bit), so it gains at every dimension; the
+// others do up to the 128 columns that one float4 a lane holds.
+static bool chunk_pays(const pbg_config &cfg, int Pm, int Mm, long long blocks) {
+  const char *env = getenv("PBG_CHUNK");
+  if (cfg.op == PBG_OP_LINEAR || cfg.op == PBG_OP_AFFINE || !pbg_chunk_fits(Pm, Mm, cfg.dim) || (env && env[0] == '0')) return false;
+  if (env && env[0] == '1') return pbg_chunk_available();
+  if (getenv("PBG_FUSED") || blocks > 28 || Pm > 64) return false;
+  const int tiles = (Mm + 31) / 32 + (cfg.dynamic_relations ? (Pm + 31) / 32 : 0);
+  if (cfg.precision == PBG_PREC_FP32) return tiles <= 4 && pbg_chunk_available();
+  if (cfg.dim > 128 || (cfg.precision == PBG_PREC_BF16X3 && cfg.comparator < PBG_CMP_L2)) return false;
+  return tiles <= (cfg.dynamic_relations ? 2 : 4) && pbg_chunk_available();
+}
+
 extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_context **out) {
   if (!cfg || !out) return PBG_ERR_BAD_ARGUMENT;
   *out = nullptr;
@@ -282,6 +316,7 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
     const char *envk = getenv("PBG_SPLIT_MIN_K");
     if (envk && atoi(envk) >= 2) c->split_min_k = atoi(envk);
   }
+  c->chunk = chunk_pays(*cfg, c->Pm, c->Mm, (long long)c->kmax * c->Cm);
   if (planes) {
     oXB[0] = take(nN * npl * Dpb * 2); oXB[1] = take(nN * npl * Dpb * 2);
     if (dyn) { oXB[2] = take(nQ * npl * Dpb * 2); oXB[3] = take(nQ * npl * Dpb * 2); oTB[0] = take(nQ * npl * Kb * 2); oTB[1] = take(nQ * npl * Kb * 2); }
@@ -467,6 +502,7 @@ static int bind_bucket(pbg_context *c, const pbg_bucket *bk, WaveDims &d, WaveBu
   d.neg_enabled[0] = !cfg.disable_lhs_negs; d.neg_enabled[1] = !cfg.disable_rhs_negs;
   d.byMm = FastDiv(c->Mm); d.byPm = FastDiv(c->Pm); d.byCm = FastDiv(c->Cm); d.bySpb = FastDiv(c->spb);
   d.num_batch_negs = cfg.num_batch_negs; d.spb = c->spb; d.margin = cfg.margin; d.reg_coef = cfg.regularization_coef; d.max_norm = cfg.max_norm > 0.f ? cfg.max_norm : 0.f;
+  d.pulled_back = c->chunk;
   d.matrix_op = cfg.op == PBG_OP_LINEAR || cfg.op == PBG_OP_AFFINE;
   d.opw = d.matrix_op ? cfg.dim * cfg.dim + (cfg.op == PBG_OP_AFFINE ? cfg.dim : 0) : cfg.dim;
   d.n_rows[0] = bk->lhs_rows; d.n_rows[1] = bk->rhs_rows;
@@ -527,6 +563,11 @@ static int run_forward(pbg_context *c, const WaveDims &d, const WaveBatches &wb,
 
 // gather -> score -> loss -> gradient products of the chunk blocks [d.blk0, d.blk0 + d.nblk) on `st`
 static void run_part(pbg_context *c, const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st) {
+  if (c->chunk) {
+    { ClassTimer t(c, 2, st); t.done(launch_chunk_step(d, wb, w, st)); }
+    if (d.reg_coef != 0.f) { ClassTimer t(c, 3, st); t.done(launch_reg_value(d, wb, w, st)); }
+    return;
+  }
   if (c->fused) {
     { ClassTimer t(c, 1, st); t.done(launch_gather(d, wb, w, st)); }
     { ClassTimer t(c, 2, st); t.done(launch_pair_score(d, wb, w, c->pairplan, st)); }      // scores, loss, coefficient planes
@@ -688,7 +729,7 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
     // kernels can run as two independent halves on two streams: the memory-bound kernels of one
     // half fill the SMs' idle issue slots while the other half's contractions run.
     d.blk0 = 0;
-    if (c->fused) {
+    if (c->fused || c->chunk) {
       // the fused score kernel computes both problems of a chunk block in one CTA: a wave of 14 batches of 10
       // chunks is one round of 140 CTAs, where its halves would each leave half of the SMs idle
       run_part(c, d, wb, w, c->stream);
@@ -824,8 +865,11 @@ extern "C" int pbg_score_batch(pbg_context *c, const pbg_bucket *bk, const int64
   wb.n[0] = count; wb.rel[0] = d.dynamic ? 0 : relidx; wb.wrel[0] = 1.0f;
   d.k = 1; d.nblk = d.Cm; d.nocc = d.spb;
   d.blk0 = 0;
-  run_forward(c, d, wb, w, c->stream);
-  c->launches += launch_export_scores(d, wb, w, lhs_pos, rhs_pos, lhs_neg, rhs_neg, c->stream);
+  if (c->chunk) c->launches += launch_chunk_scores(d, wb, w, lhs_pos, rhs_pos, lhs_neg, rhs_neg, c->stream);
+  else {
+    run_forward(c, d, wb, w, c->stream);
+    c->launches += launch_export_scores(d, wb, w, lhs_pos, rhs_pos, lhs_neg, rhs_neg, c->stream);
+  }
   CU(c, pbg_take_launch_error());
   return check_errflag(c);
 }

@@ -76,6 +76,7 @@ struct WaveDims {
   int num_rels;
   int matrix_op;        // operator is linear / affine (standard relations): applied by contractions, not in the gather
   int opw;              // floats per operator-table row: D, or D*D (+ D) for linear (affine)
+  int pulled_back;      // the gradient slots have been through the pull-back already (chunk_kernel)
   unsigned long long key_rel_base;   // first sort key of operator-table rows
   unsigned long long key_invalid;    // sort key of slots that carry no gradient
 };
@@ -351,6 +352,14 @@ __device__ __forceinline__ void put_planes1(unsigned short *dst, size_t plane, f
 __device__ __forceinline__ float tf32_round(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u); }
 __device__ __forceinline__ float4 tf32_round4(float4 v) { return make_float4(tf32_round(v.x), tf32_round(v.y), tf32_round(v.z), tf32_round(v.w)); }
 
+// 16 bytes from global to shared memory, asynchronously; zeros without `real`.
+__device__ __forceinline__ void cp_async16(float *dst, const float *src, bool real) {
+  const int bytes = real ? 16 : 0;                    // nothing read, zeros written
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
+
 // ---- host-side helpers ---------------------------------------------------------------------------
 // Opt-in to more than 48 KB of dynamic shared memory.  The attribute belongs to the (kernel, device)
 // pair, so a process that drives several GPUs has to set it on each of them: the pairs already done
@@ -418,6 +427,20 @@ inline void pbg_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
   pbg_note_launch(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
 }
 
+// The same for a kernel of clusters of `ctas` CTAs.
+template <class... P, class... A>
+inline void pbg_launch_clusters(void (*kernel)(P...), int clusters, int ctas, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(clusters * ctas)); cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = ctas; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = 2;
+  pbg_note_launch(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
 // ---- host-side launchers (one per translation unit) ------------------------------------------
 struct SortPlan {
   unsigned long long *keys[2];
@@ -464,6 +487,13 @@ int launch_postop(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, c
 int launch_gz_rows(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st);
 int launch_score_simt(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st);
 int launch_grad_simt(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st);
+// Gather, scores, loss, gradients and pull-back of the chunk blocks of a small wave in one kernel, a cluster of CTAs to a block.
+// pbg_chunk_fits: shapes it takes; pbg_chunk_available: the current device can hold its clusters.
+bool pbg_chunk_fits(int Pm, int Mm, int D);
+bool pbg_chunk_available();
+int launch_chunk_step(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st);
+// the forward half of it for one batch, straight into the caller's score arrays (see launch_export_scores)
+int launch_chunk_scores(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, float *lhs_pos, float *rhs_pos, float *lhs_neg, float *rhs_neg, cudaStream_t st);
 int launch_loss(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st);
 int launch_export_scores(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w,
                          float *lhs_pos, float *rhs_pos, float *lhs_neg, float *rhs_neg, cudaStream_t st);

@@ -11,163 +11,20 @@
 //   l2        :  T_ij = -dS_ij / S_ij     (= -2 dLoss/d(squared distance)), same on the diagonal
 //   squared_l2:  T_ij = 2 dS_ij
 // The diagonal of S is always masked, which is what frees it to carry the positive pair.
-#include "pbg_common.cuh"
+#include "pbg_rows.cuh"
 
 #define LOSS_WARPS 8
 
-__device__ __forceinline__ float softplusf(float x) {           // log(1 + e^x), stable
-  return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x)));
-}
-__device__ __forceinline__ float sigmoidf(float x) { return 1.0f / (1.0f + expf(-x)); }
-
-// column j of the negatives of a chunk: is it ignored, and does it exist at all?
-__device__ __forceinline__ bool col_masked(const WaveDims &d, const BlockInfo &bi, int enabled, int i, int j) {
-  if (!enabled) return true;
-  if (j >= d.Pm) return false;                       // uniform negatives are never masked
-  if (!d.batch_negs) return true;                    // uniform-only mode: no batch negatives
-  return j == i || j >= bi.n;                        // own positive; padding of the last chunk
-}
-
-__device__ __forceinline__ float coef_from_dscore(int cmp, float dS, float S) {
-  if (cmp == PBG_CMP_L2) return (-S > 1e-15f) ? -dS / S : 0.f;   // clamp at 1e-30 kills the gradient
-  if (cmp == PBG_CMP_SQUARED_L2) return 2.0f * dS;
-  return dS;
-}
-
-// NV > 0: the row (at most 32 NV columns) is read into registers before the first coefficient is written.  Written column
-// by column behind the reads, every read waited for the write before it (the compiler cannot tell the rows apart): 24 to
-// 31 us for 2 x 70 blocks of 100 rows x 200 columns where the bytes take 4.  NV == 0: rows of any length, column by column.
 template <int NV>
 __global__ void __launch_bounds__(32 * LOSS_WARPS) loss_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   pdl_begin();
-  int lane = threadIdx.x & 31;
   const int item = (int)blockIdx.x * LOSS_WARPS + (int)(threadIdx.x >> 5);
   const int per_prob = d.nblk * d.Pm;
   if (item >= 2 * per_prob) return;
   const int p = item >= per_prob ? 1 : 0, rem = item - p * per_prob;
-  const int lb = d.byPm.div(rem), i = rem - lb * d.Pm;
-  const int blk = d.blk0 + lb;
-  BlockInfo bi = block_info(d, wb, blk);
-  if (bi.n == 0) return;
-  float *S = w.S[p] + ((size_t)blk * d.Pm + i) * d.Ms;
-  // bf16-plane tier with dynamic relations: T is an MMA operand, its planes go beside it
-  unsigned short *TBr = w.TB[p] ? w.TB[p] + ((size_t)blk * w.npl * d.Pm + i) * w.Kb : nullptr;
-  const size_t tplane = (size_t)d.Pm * w.Kb;
-  auto put = [&](int j, float t) {
-    S[j] = t;
-    if (TBr) put_planes1(TBr + j, tplane, t, w.npl);
-  };
-  size_t prow = (size_t)blk * d.Pm + i;
-  const int Mm = d.Mm;
-  if (i >= bi.n) {                                   // padded positive: contributes nothing
-    for (int j = lane; j < d.Ms; j += 32) put(j, 0.f);
-    if (lane == 0) {
-      w.lossrow[p][prow] = 0.f; w.violrow[p][prow] = 0;
-      if (d.cmp >= PBG_CMP_L2) w.coef[2 + p][prow] = 0.f;
-    }
-    return;
-  }
-  const int enabled = d.neg_enabled[p];
-  const float s = w.spos[p][prow];
-  const float wr = wb.wrel[bi.b] * (w.ew ? w.ew[bi.e0 + i] : 1.0f);   // relation weight x edge weight
-  // number of negative columns the reference's score matrix has for this row (masked included)
-  const int Mlog = !enabled ? 0 : (d.batch_negs ? bi.Pl + d.U : d.U);
-  float lossv = 0.f, ds = 0.f, rowsum = 0.f;
-  int viol = 0;
-  constexpr int NR = NV > 0 ? NV : 1;
-  float sv[NR];
-  unsigned live = 0u;                                 // bit u: column lane + 32 u counts
-  if (NV > 0) {
-#pragma unroll
-    for (int u = 0; u < NR; ++u) {
-      const int j = lane + 32 * u;
-      const bool c = j < Mm && !col_masked(d, bi, enabled, i, j);
-      sv[u] = c ? S[j] : 0.f;
-      live |= c ? 1u << u : 0u;
-    }
-  }
-  // every live column j with its score, in the order j = lane, lane + 32, ...
-  auto each = [&](auto &&f) {
-    if (NV > 0) {
-#pragma unroll
-      for (int u = 0; u < NR; ++u) if (live >> u & 1u) f(lane + 32 * u, sv[u]);
-    } else {
-      for (int j = lane; j < Mm; j += 32) if (!col_masked(d, bi, enabled, i, j)) f(j, S[j]);
-    }
-  };
-  // writes the row: f(score) in the live columns, zeros elsewhere (the diagonal is filled below)
-  auto fill = [&](auto &&f) {
-    if (NV > 0) {
-#pragma unroll
-      for (int u = 0; u < NR; ++u) {
-        const int j = lane + 32 * u;
-        const float t = live >> u & 1u ? f(sv[u]) : 0.f;
-        rowsum += t;
-        if (j < d.Ms) put(j, t);
-      }
-    } else {
-      for (int j = lane; j < d.Ms; j += 32) {
-        const float t = j < Mm && !col_masked(d, bi, enabled, i, j) ? f(S[j]) : 0.f;
-        rowsum += t;
-        put(j, t);
-      }
-    }
-  };
-
-  if (d.loss == PBG_LOSS_SOFTMAX) {
-    // -s + log(e^s + sum_j e^S_ij); masked entries are e^-1e9 = 0 (losses.py:143-159)
-    if (Mlog > 0) {
-      float mx = -INFINITY;
-      each([&](int, float x) { mx = fmaxf(mx, x); });
-      mx = warp_max(mx);
-      float m = fmaxf(mx, s);
-      if (mx == -INFINITY) m = fmaxf(s, PBG_MASKED);      // every column masked
-      float z = 0.f;
-      each([&](int, float x) { z += expf(x - m); viol += x > s; });
-      z = warp_sum(z);
-      float es = expf(s - m);
-      float Z = z + es;
-      lossv = -s + m + logf(Z);
-      ds = es / Z - 1.0f;
-      float invZ = 1.0f / Z;
-      fill([&](float x) { return coef_from_dscore(d.cmp, wr * expf(x - m) * invZ, x); });
-    } else {
-      fill([&](float) { return 0.f; });                    // losses.py:139-140: loss 0, no gradient
-    }
-  } else if (d.loss == PBG_LOSS_RANKING) {
-    // sum_j max(0, margin - s + S_ij) (losses.py:116-122)
-    if (Mlog > 0) {
-      each([&](int, float x) {
-        const float v = (x - s) + d.margin;
-        viol += x > s;
-        if (v > 0.f) { lossv += v; ds -= 1.0f; }
-      });
-      fill([&](float x) { return (x - s) + d.margin > 0.f ? coef_from_dscore(d.cmp, wr, x) : 0.f; });
-      lossv = warp_sum(lossv);
-      ds = warp_sum(ds);
-    } else {
-      fill([&](float) { return 0.f; });
-    }
-  } else {
-    // softplus(-s) + (1/M) sum_j softplus(S_ij), M counts masked columns (losses.py:61-80)
-    float nw = Mlog > 0 ? 1.0f / (float)Mlog : 0.f;
-    each([&](int, float x) { viol += x > s; lossv += softplusf(x); });
-    fill([&](float x) { return coef_from_dscore(d.cmp, wr * nw * sigmoidf(x), x); });
-    lossv = warp_sum(lossv) * nw + softplusf(-s);
-    ds = -sigmoidf(-s);
-  }
-  viol = warp_sum_int(viol);
-  rowsum = warp_sum(rowsum);
-  // positive pair folded into the diagonal; the positive score of the l2 family is the direct
-  // form -sqrt(max(sum (a-b)^2, 1e-30)) (model.py:267-274)
-  float tdiag = coef_from_dscore(d.cmp, wr * ds, s);
-  __syncwarp();
-  if (lane == 0) {
-    put(i, tdiag);
-    w.lossrow[p][prow] = wr * lossv;
-    w.violrow[p][prow] = viol;
-    if (d.cmp >= PBG_CMP_L2) w.coef[2 + p][prow] = rowsum + tdiag;
-  }
+  const int lb = d.byPm.div(rem);
+  const int blk = d.blk0 + lb, i = rem - lb * d.Pm;
+  loss_row<NV>(d, wb, w, p, blk, i, threadIdx.x & 31, w.S[p] + ((size_t)blk * d.Pm + i) * d.Ms);
 }
 
 // l2 family: column sums of T_p over the chunk's positives (coefficient of the negative row's own |b|^2 term).  A CTA takes
@@ -252,99 +109,16 @@ __global__ void __launch_bounds__(32 * LOSS_WARPS) coef_kernel(WaveDims d, WaveB
   }
 }
 
-// Softmax under the dot / cos comparators with at most 32 NV negative columns: the warp keeps the
-// row in registers, so the scores are read once, the masks evaluated once and every exponential
-// taken once (the general kernel makes three passes).  Same arithmetic, same summation order.
 template <int NV>
 __global__ void __launch_bounds__(32 * LOSS_WARPS) loss_softmax_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   pdl_begin();
-  int lane = threadIdx.x & 31;
   const int item = (int)blockIdx.x * LOSS_WARPS + (int)(threadIdx.x >> 5);
   const int per_prob = d.nblk * d.Pm;
   if (item >= 2 * per_prob) return;
   const int p = item >= per_prob ? 1 : 0, rem = item - p * per_prob;
-  const int lb = d.byPm.div(rem), i = rem - lb * d.Pm;
-  const int blk = d.blk0 + lb;
-  BlockInfo bi = block_info(d, wb, blk);
-  if (bi.n == 0) return;
-  float *S = w.S[p] + ((size_t)blk * d.Pm + i) * d.Ms;
-  // bf16-plane tier with dynamic relations: T is an MMA operand, its planes go beside it
-  unsigned short *TBr = w.TB[p] ? w.TB[p] + ((size_t)blk * w.npl * d.Pm + i) * w.Kb : nullptr;
-  const size_t tplane = (size_t)d.Pm * w.Kb;
-  const int npl = w.npl;
-  size_t prow = (size_t)blk * d.Pm + i;
-  const int Mm = d.Mm;
-  const int enabled = d.neg_enabled[p];
-  const int Mlog = !enabled ? 0 : (d.batch_negs ? bi.Pl + d.U : d.U);
-  if (i >= bi.n || Mlog == 0) {                      // padded positive, or no negatives at all: no loss, no gradient
-#pragma unroll
-    for (int u = 0; u < NV; ++u) { int j = lane + 32 * u; if (j < d.Ms) S[j] = 0.f; }
-    if (TBr)
-      for (int j = 2 * lane; j < d.Ms; j += 64) { *(unsigned *)(TBr + j) = 0u; *(unsigned *)(TBr + tplane + j) = 0u; if (npl > 2) *(unsigned *)(TBr + 2 * tplane + j) = 0u; }
-    if (lane == 0) { w.lossrow[p][prow] = 0.f; w.violrow[p][prow] = 0; }
-    return;
-  }
-  const float s = w.spos[p][prow];
-  const float wr = wb.wrel[bi.b] * (w.ew ? w.ew[bi.e0 + i] : 1.0f);   // relation weight x edge weight
-  float sv[NV];
-  float mx = -INFINITY;
-#pragma unroll
-  for (int u = 0; u < NV; ++u) {
-    int j = lane + 32 * u;
-    bool valid = j < Mm && !col_masked(d, bi, enabled, i, j);
-    sv[u] = valid ? S[j] : -INFINITY;
-    mx = fmaxf(mx, sv[u]);
-  }
-  mx = warp_max(mx);
-  float m = fmaxf(mx, s);
-  if (mx == -INFINITY) m = fmaxf(s, PBG_MASKED);      // every column masked
-  float z = 0.f;
-  int viol = 0;
-#pragma unroll
-  for (int u = 0; u < NV; ++u) {
-    bool valid = sv[u] != -INFINITY;
-    viol += valid && sv[u] > s;
-    sv[u] = valid ? expf(sv[u] - m) : 0.f;
-    z += sv[u];
-  }
-  z = warp_sum(z);
-  viol = warp_sum_int(viol);
-  float es = expf(s - m);
-  float Z = z + es;
-  float lossv = -s + m + logf(Z);
-  float invZ = 1.0f / Z;
-  float tdiag = wr * (es / Z - 1.0f);
-#pragma unroll
-  for (int u = 0; u < NV; ++u) {
-    int j = lane + 32 * u;
-    if (j < d.Ms) S[j] = j == i ? tdiag : wr * sv[u] * invZ;
-  }
-  if (TBr) {
-    // two column groups at a time: neighbouring lanes swap one group's planes, so that every lane stores
-    // two columns of one group (4-byte stores): even lanes (j, j + 1) of group u, odd lanes (j - 1, j) of u + 1
-    const bool odd = lane & 1;
-#pragma unroll
-    for (int u = 0; u < NV; u += 2) {
-      const int j0 = lane + 32 * u, j1 = j0 + 32;
-      unsigned a[3], b[3], give[3], keep[3];
-      bf16_planes(j0 == i ? tdiag : wr * sv[u] * invZ, a[0], a[1], a[2]);
-      bf16_planes(j1 == i ? tdiag : wr * sv[u + 1] * invZ, b[0], b[1], b[2]);
-#pragma unroll
-      for (int q = 0; q < 3; ++q) { give[q] = odd ? a[q] : b[q]; keep[q] = odd ? b[q] : a[q]; }
-      unsigned g01 = __shfl_xor_sync(0xffffffffu, give[0] | (give[1] << 16), 1);
-      unsigned g2 = __shfl_xor_sync(0xffffffffu, give[2], 1);
-      unsigned got[3] = {g01 & 0xffffu, g01 >> 16, g2};
-      const int col = (odd ? j1 : j0) & ~1;
-      if (col < d.Ms) {
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          unsigned lo = odd ? got[q] : keep[q], hi = odd ? keep[q] : got[q];
-          if (q < npl) *(unsigned *)(TBr + q * tplane + col) = lo | (hi << 16);
-        }
-      }
-    }
-  }
-  if (lane == 0) { w.lossrow[p][prow] = wr * lossv; w.violrow[p][prow] = viol; }
+  const int lb = d.byPm.div(rem);
+  const int blk = d.blk0 + lb, i = rem - lb * d.Pm;
+  loss_softmax_row<NV>(d, wb, w, p, blk, i, threadIdx.x & 31, w.S[p] + ((size_t)blk * d.Pm + i) * d.Ms);
 }
 
 // Combined coefficient matrices under the dot / cos comparators, one warp per 32 x 32 tile of

@@ -15,95 +15,9 @@
 // A row is read once and written once per wave however many batches touched it, and the
 // optimizer state never leaves HBM.  Everything is summed in a fixed order: results are
 // reproducible run to run.
-#include "pbg_common.cuh"
+#include "pbg_rows.cuh"
 
 #define UPD_WARPS 8
-
-enum { CK_DOT = 0, CK_COS = 1, CK_L2 = 2 };      // comparator kinds of the pull-back
-
-// v = gradient of the operator output behind slot (a, blk, r): the contraction's row, plus the regularizer's own
-// gradient on the rows it covers (reg), back through comparator.prepare -- cos: (g - y <g, y>) / |z|; l2 family: the
-// row's own |y|^2 term (dynamic: ga = T.N - rowsum(T) a, gb = T^T.Q - colsum(T) b; standard: g = A.N' - rowsum(A) y).
-template <int VEC, int CK>
-__device__ __forceinline__ void gz_row(float4 (&v)[VEC], const WaveDims &d, const WaveBufs &w, int a, int blk, int r, int lane, bool reg) {
-  const int D = d.D;
-  const size_t xr = (size_t)blk * w.xrows[a] + r, gr = (size_t)blk * w.grows[a] + r;
-  const float *y = w.X[a] + xr * d.Dp, *g = w.GX[a] + gr * d.Dp;
-  float4 yv[VEC];
-#pragma unroll
-  for (int c = 0; c < VEC; ++c) {
-    const int dd = c * 128 + lane * 4;
-    v[c] = dd < D ? ld4(g + dd) : f4zero();
-    if (CK != CK_DOT) yv[c] = dd < D ? ld4(y + dd) : f4zero();
-  }
-  const float cf = CK == CK_L2 ? w.coef[a][gr] : 0.f, inv = CK == CK_COS ? w.aux[a][xr] : 1.f;
-  if (reg) {
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) {
-      const int dd = c * 128 + lane * 4;
-      if (dd < D) v[c] = v[c] + n3_grad4(y, dd, D, d.op == PBG_OP_COMPLEX_DIAGONAL) * d.reg_coef;
-    }
-  }
-  if (CK == CK_COS) {
-    float s = 0.f;
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) s += f4dot_yx(v[c], yv[c]);
-    s = warp_sum(s);
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) v[c] = (v[c] - yv[c] * s) * inv;
-  } else if (CK == CK_L2) {
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) v[c] = v[c] - yv[c] * cf;
-  }
-}
-
-// Back through the operator: v (gradient of its output) becomes the gradient of the raw row, pg the contribution to
-// the operator row.  x: the raw row, used as x * xs (+ xadd).  complex_diagonal pairs element d with d +- D/2, which
-// another lane holds: v goes through `part` (D floats of the warp's own shared memory), the partners of x and theta are
-// read again (L1 / L2).
-template <int VEC>
-__device__ __forceinline__ void operator_back(float4 (&v)[VEC], float4 (&pg)[VEC], const WaveDims &d, const float *theta, const float *x,
-                                              float xs, const float *xadd, float *part, int lane) {
-  const int D = d.D;
-  auto raw = [&](int e) {
-    float4 q = ld4(x + e) * xs;
-    if (xadd) q = q + ld4(xadd + e);
-    return q;
-  };
-  if (d.op == PBG_OP_TRANSLATION) {
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) pg[c] = v[c];
-    return;
-  }
-  if (d.op == PBG_OP_DIAGONAL) {
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) {
-      const int dd = c * 128 + lane * 4;
-      if (dd < D) { pg[c] = v[c] * raw(dd); v[c] = v[c] * ld4(theta + dd); }
-    }
-    return;
-  }
-  const int h = D >> 1;
-  __syncwarp();                                              // the previous row's partners have been read
-#pragma unroll
-  for (int c = 0; c < VEC; ++c) {
-    const int dd = c * 128 + lane * 4;
-    if (dd < D) st4(part + dd, v[c]);
-  }
-  __syncwarp();
-#pragma unroll
-  for (int c = 0; c < VEC; ++c) {
-    const int dd = c * 128 + lane * 4;
-    if (dd < D) {
-      const int dp = dd < h ? dd + h : dd - h;
-      const float4 vp = ld4(part + dp), xv = raw(dd), xp = raw(dp), t = ld4(theta + dd), tp = ld4(theta + dp);
-      // d real = g_re a_re + g_im a_im ;  d imag = -g_re a_im + g_im a_re
-      pg[c] = dd < h ? v[c] * xv + vp * xp : v[c] * xp - vp * xv;
-      // gx_re = g_re p_re + g_im p_im ;  gx_im = -g_re p_im + g_im p_re
-      v[c] = dd < h ? v[c] * t + vp * tp : v[c] * tp - vp * t;
-    }
-  }
-}
 
 // Standard relations: the pull-back of a wave's gradient slots, one warp per row of a chunk block and side -- the
 // gradient of the raw row written over the slot's own gradient row.  Under diagonal and complex_diagonal the row's
@@ -114,40 +28,18 @@ template <int VEC, int CK>
 __global__ void __launch_bounds__(32 * UPD_WARPS) std_pullback_kernel(WaveDims d, WaveBatches wb, WaveBufs w, int side0) {
   pdl_begin();
   extern __shared__ __align__(16) float wpart[];             // [UPD_WARPS][VEC * 128]
-  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  const int side = side0 + blockIdx.y, a = side ? ARR_N1 : ARR_N0;
-  const int item = (int)blockIdx.x * UPD_WARPS + wl;
+  const int wl = threadIdx.x >> 5, item = (int)blockIdx.x * UPD_WARPS + wl;
   if (item >= d.nblk * d.Mm) return;
-  const int lb = d.byMm.div(item), r = item - lb * d.Mm, blk = d.blk0 + lb;
+  const int lb = d.byMm.div(item);
+  const int side = side0 + blockIdx.y, a = side ? ARR_N1 : ARR_N0, blk = d.blk0 + lb, r = item - lb * d.Mm, lane = threadIdx.x & 31;
   if (side == 1 && d.matrix_op) return;                      // linear / affine: R2 holds the gradient of the raw row already
   const BlockInfo bi = block_info(d, wb, blk);
   if (bi.n <= 0) return;
   const long long row = slot_row(d, wb, w, bi, side, r);
-  const int D = d.D;
-  float4 v[VEC], pg[VEC];
-  if (row < 0 || row >= d.n_rows[side]) {                    // no row behind the slot: nothing for param_sums to add
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) {
-      const int dd = c * 128 + lane * 4;
-      if (dd < D) {
-        st4(w.GX[a] + ((size_t)blk * w.grows[a] + r) * d.Dp + dd, f4zero());
-        if (side == 1 && w.PG) st4(w.PG + ((size_t)blk * d.Mm + r) * d.Dp + dd, f4zero());
-      }
-    }
-    return;
-  }
+  if (row < 0 || row >= d.n_rows[side]) { std_pullback_empty<VEC>(d, w, side, blk, r, lane); return; }
+  float4 v[VEC];
   gz_row<VEC, CK>(v, d, w, a, blk, r, lane, d.reg_coef != 0.f && r < bi.n && r < d.Pm);
-  if (side == 1 && w.PG) {
-    const float xs = d.max_norm > 0.f ? w.rscale[(size_t)blk * d.Mm + r] : 1.0f;   // the raw row entered the operator scaled
-    operator_back<VEC>(v, pg, d, w.theta[0] + (size_t)wb.rel[bi.b] * D, w.W[1] + (size_t)row * D, xs, w.glob[1], wpart + (size_t)wl * VEC * 128, lane);
-    float *out = w.PG + ((size_t)blk * d.Mm + r) * d.Dp;
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) { const int dd = c * 128 + lane * 4; if (dd < D) st4(out + dd, pg[c]); }
-  }
-  __syncwarp();
-  float *out = w.GX[a] + ((size_t)blk * w.grows[a] + r) * d.Dp;
-#pragma unroll
-  for (int c = 0; c < VEC; ++c) { const int dd = c * 128 + lane * 4; if (dd < D) st4(out + dd, v[c]); }
+  std_pullback_finish<VEC>(v, d, wb, w, side, bi, blk, r, row, lane, wpart + (size_t)wl * VEC * 128);
 }
 
 // The vectors that every row of a batch shares in standard relations: the relation's operator row, and the vector of
@@ -1167,7 +1059,7 @@ template <int VEC, int CK>
 __global__ void __launch_bounds__(32 * UPD_WARPS, VEC <= 4 ? 4 : 1) dyn_pullback_kernel(WaveDims d, WaveBatches wb, WaveBufs w, int first_q) {
   pdl_begin();
   extern __shared__ __align__(16) float wpart[];             // [UPD_WARPS][VEC * 128]
-  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const int wl = threadIdx.x >> 5;
   const int nN = d.nblk * d.Mm, nQ = d.nblk * d.Pm;
   int item = (int)blockIdx.x * UPD_WARPS + wl + (first_q ? 2 * nN : 0);
   if (item >= 2 * nN + 2 * nQ) return;
@@ -1176,54 +1068,15 @@ __global__ void __launch_bounds__(32 * UPD_WARPS, VEC <= 4 ? 4 : 1) dyn_pullback
   else if ((item -= nN) < nN) a = ARR_N1;
   else if ((item -= nN) < nQ) a = ARR_Q0;
   else { item -= nQ; a = ARR_Q1; }
-  const int rows = a <= ARR_N1 ? d.Mm : d.Pm, lb = a <= ARR_N1 ? d.byMm.div(item) : d.byPm.div(item), r = item - lb * rows;
-  const int blk = d.blk0 + lb, D = d.D;
-  BlockInfo bi = block_info(d, wb, blk);
-  if (bi.n <= 0) return;
-  // the entity of the slot: N arrays hold lhs / rhs rows (chunk, then uniform), Q0 = op_rhs(rhs), Q1 = op_lhs(lhs)
-  const int side = (a == ARR_N0 || a == ARR_Q1) ? 0 : 1;
-  const bool q = a >= ARR_Q0;
-  if (q && r >= bi.n) return;
-  float *prow = q && w.GR[a - ARR_Q0] ? w.GR[a - ARR_Q0] + ((size_t)blk * d.Pm + r) * d.Dp : nullptr;
+  const int rows = a <= ARR_N1 ? d.Mm : d.Pm, lb = a <= ARR_N1 ? d.byMm.div(item) : d.byPm.div(item);
+  const int blk = d.blk0 + lb, r = item - lb * rows, lane = threadIdx.x & 31, side = slot_side(a);
+  const BlockInfo bi = block_info(d, wb, blk);
+  if (bi.n <= 0 || (a >= ARR_Q0 && r >= bi.n)) return;
   const long long id = slot_row(d, wb, w, bi, side, r);
-  if (id < 0 || id >= d.n_rows[side]) {
-    // an entity id outside its table (the call reports it): the edge's operator-row slot may still be a valid one
-    // (its key depends on the relation id only), so it gets a zero gradient rather than whatever the row held
-    if (prow)
-      for (int dd = lane * 4; dd < D; dd += 128) st4(prow + dd, f4zero());
-    return;
-  }
-  const float *theta = nullptr;
-  if (prow) {
-    const long long rl = w.rel[bi.e0 + r];
-    const float *tab = w.theta[a - ARR_Q0];
-    if (tab && rl >= 0 && rl < d.num_rels) theta = tab + (size_t)rl * D;
-  }
-  const bool reg = d.reg_coef != 0.f && r < bi.n && r < d.Pm;    // regularized: the chunk's edges in every operand array
-  float4 v[VEC], pg[VEC];
-  gz_row<VEC, CK>(v, d, w, a, blk, r, lane, reg);
-  if (theta) {
-    const int na = a == ARR_Q0 ? ARR_N1 : ARR_N0;              // the slot's operator-free copy (prepared raw row)
-    const size_t nrow = (size_t)blk * w.xrows[na] + r;
-    const float xs = CK == CK_COS ? 1.0f / w.aux[na][nrow] : 1.0f;
-    operator_back<VEC>(v, pg, d, theta, w.X[na] + nrow * d.Dp, xs, nullptr, wpart + (size_t)wl * VEC * 128, lane);
-#pragma unroll
-    for (int c = 0; c < VEC; ++c) {
-      const int dd = c * 128 + lane * 4;
-      if (dd < D) {
-        // N3 regularizer on the edge's own parameter row (still as the wave found it)
-        if (d.reg_coef != 0.f) pg[c] = pg[c] + n3_grad4(theta, dd, D, d.op == PBG_OP_COMPLEX_DIAGONAL) * d.reg_coef;
-        st4(prow + dd, pg[c]);
-      }
-    }
-  }
-  __syncwarp();
-  float *row = w.GX[a] + ((size_t)blk * w.grows[a] + r) * d.Dp;
-#pragma unroll
-  for (int c = 0; c < VEC; ++c) {
-    const int dd = c * 128 + lane * 4;
-    if (dd < D) st4(row + dd, v[c]);
-  }
+  if (id < 0 || id >= d.n_rows[side]) { dyn_pullback_empty<VEC>(d, w, a, blk, r, lane); return; }
+  float4 v[VEC];
+  gz_row<VEC, CK>(v, d, w, a, blk, r, lane, d.reg_coef != 0.f && r < bi.n && r < d.Pm);    // (regularized: the chunk's edges in every operand array)
+  dyn_pullback_finish<VEC, CK>(v, d, w, a, bi, blk, r, lane, wpart + (size_t)wl * VEC * 128);
 }
 
 // The pull-back of a wave (what is left to do depends on the comparator, the operator and the options) and the job it
@@ -1241,7 +1094,7 @@ static int launch_pullback(const WaveDims &d, const WaveBatches &wb, const WaveB
   pbg_opt_in_smem((const void *)dyn_pullback_kernel<VEC, CK_L2>, (int)smem);
   job.sums = job.steps = job.cleared0 = job.cleared1 = 0; job.lr = rel_lr;
   if (d.dynamic) {
-    if (!rows_change && !has_op) return 0;
+    if (d.pulled_back || (!rows_change && !has_op)) return 0;
     const int first_q = rows_change ? 0 : 1;
     const long long rows = 2ll * d.nblk * d.Pm + (first_q ? 0 : 2ll * d.nblk * d.Mm);
     PBG_ROWS_CK(VEC, dyn_pullback_kernel, (unsigned)((rows + UPD_WARPS - 1) / UPD_WARPS), 32 * UPD_WARPS, smem, st, d, wb, w, first_q);
@@ -1256,6 +1109,7 @@ static int launch_pullback(const WaveDims &d, const WaveBatches &wb, const WaveB
   }
   if (!rows_change && !(row_op && w.PG)) return 0;
   job.cleared0 = rows_change; job.cleared1 = 1;
+  if (d.pulled_back) return 0;
   const dim3 grid((unsigned)(((long long)d.nblk * d.Mm + UPD_WARPS - 1) / UPD_WARPS), rows_change ? 2 : 1);
   PBG_ROWS_CK(VEC, std_pullback_kernel, grid, 32 * UPD_WARPS, smem, st, d, wb, w, rows_change ? 0 : 1);
   return 1;
