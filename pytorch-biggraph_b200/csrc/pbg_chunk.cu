@@ -122,8 +122,8 @@ __device__ __forceinline__ void chunk_scores(const WaveDims &d, const WaveBatche
     __syncwarp();                                     // a warp's two rows are its own
     for (int m = ty * 2; m < ty * 2 + 2 && m0 + m < m_end; ++m) {
       const float *Sr = Ss + m * (CHUNK_MM + 4);
-      if (d.loss == PBG_LOSS_SOFTMAX && d.cmp < PBG_CMP_L2) loss_softmax_row<NV>(d, wb, w, p, blk, m0 + m, lane, Sr);
-      else loss_row<NV>(d, wb, w, p, blk, m0 + m, lane, Sr);
+      if (d.loss == PBG_LOSS_SOFTMAX && d.cmp < PBG_CMP_L2) loss_softmax_row<NV, true>(d, wb, w, p, blk, m0 + m, lane, Sr);
+      else loss_row<NV, true>(d, wb, w, p, blk, m0 + m, lane, Sr);
     }
   }
 }

@@ -23,8 +23,7 @@ __global__ void __launch_bounds__(32 * LOSS_WARPS) loss_kernel(WaveDims d, WaveB
   if (item >= 2 * per_prob) return;
   const int p = item >= per_prob ? 1 : 0, rem = item - p * per_prob;
   const int lb = d.byPm.div(rem);
-  const int blk = d.blk0 + lb, i = rem - lb * d.Pm;
-  loss_row<NV>(d, wb, w, p, blk, i, threadIdx.x & 31, w.S[p] + ((size_t)blk * d.Pm + i) * d.Ms);
+  loss_row<NV>(d, wb, w, p, d.blk0 + lb, rem - lb * d.Pm, threadIdx.x & 31);
 }
 
 // l2 family: column sums of T_p over the chunk's positives (coefficient of the negative row's own |b|^2 term).  A CTA takes
@@ -117,8 +116,7 @@ __global__ void __launch_bounds__(32 * LOSS_WARPS) loss_softmax_kernel(WaveDims 
   if (item >= 2 * per_prob) return;
   const int p = item >= per_prob ? 1 : 0, rem = item - p * per_prob;
   const int lb = d.byPm.div(rem);
-  const int blk = d.blk0 + lb, i = rem - lb * d.Pm;
-  loss_softmax_row<NV>(d, wb, w, p, blk, i, threadIdx.x & 31, w.S[p] + ((size_t)blk * d.Pm + i) * d.Ms);
+  loss_softmax_row<NV>(d, wb, w, p, d.blk0 + lb, rem - lb * d.Pm, threadIdx.x & 31);
 }
 
 // Combined coefficient matrices under the dot / cos comparators, one warp per 32 x 32 tile of

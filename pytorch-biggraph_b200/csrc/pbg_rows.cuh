@@ -330,12 +330,13 @@ __device__ __forceinline__ float coef_from_dscore(int cmp, float dS, float S) {
 // NV > 0: the row (at most 32 NV columns) is read into registers before the first coefficient is written.  Written column
 // by column behind the reads, every read waited for the write before it (the compiler cannot tell the rows apart): 24 to
 // 31 us for 2 x 70 blocks of 100 rows x 200 columns where the bytes take 4.  NV == 0: rows of any length, column by column.
-// Sr: the row's scores, in the place the coefficients go to or in shared memory.
-template <int NV>
-__device__ __forceinline__ void loss_row(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, int p, int blk, int i, int lane, const float *Sr) {
+// The row's scores are where the coefficients go to, or (FROM) somewhere else.
+template <int NV, bool FROM = false>
+__device__ __forceinline__ void loss_row(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, int p, int blk, int i, int lane, const float *from = nullptr) {
   BlockInfo bi = block_info(d, wb, blk);
   if (bi.n == 0) return;
   float *S = w.S[p] + ((size_t)blk * d.Pm + i) * d.Ms;
+  const float *Sr = FROM ? from : S;
   // bf16-plane tier with dynamic relations: T is an MMA operand, its planes go beside it
   unsigned short *TBr = w.TB[p] ? w.TB[p] + ((size_t)blk * w.npl * d.Pm + i) * w.Kb : nullptr;
   const size_t tplane = (size_t)d.Pm * w.Kb;
@@ -459,11 +460,12 @@ __device__ __forceinline__ void loss_row(const WaveDims &d, const WaveBatches &w
 // Softmax under the dot / cos comparators with at most 32 NV negative columns: the warp keeps the
 // row in registers, so the scores are read once, the masks evaluated once and every exponential
 // taken once (the general kernel makes three passes).  Same arithmetic, same summation order.
-template <int NV>
-__device__ __forceinline__ void loss_softmax_row(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, int p, int blk, int i, int lane, const float *Sr) {
+template <int NV, bool FROM = false>
+__device__ __forceinline__ void loss_softmax_row(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, int p, int blk, int i, int lane, const float *from = nullptr) {
   BlockInfo bi = block_info(d, wb, blk);
   if (bi.n == 0) return;
   float *S = w.S[p] + ((size_t)blk * d.Pm + i) * d.Ms;
+  const float *Sr = FROM ? from : S;
   // bf16-plane tier with dynamic relations: T is an MMA operand, its planes go beside it
   unsigned short *TBr = w.TB[p] ? w.TB[p] + ((size_t)blk * w.npl * d.Pm + i) * w.Kb : nullptr;
   const size_t tplane = (size_t)d.Pm * w.Kb;
