@@ -12,8 +12,8 @@
 // tile overlaps the main loop of the next:
 //   warp 0      TMA producer: cp.async.bulk.tensor tiles of 32 k-values into a ring of
 //               shared-memory stages, completion on an mbarrier per stage
-//   warp 1      allocates tensor memory, issues tcgen05.mma.kind::tf32 (one elected lane) and
-//               commits to the stage's "empty" barrier / the final "accumulator ready" barrier
+//   warp 1      allocates tensor memory, issues tcgen05.mma.kind::tf32 (the whole warp runs the loop, one elected
+//               lane issues) and commits to the stage's "empty" barrier / the final "accumulator ready" barrier
 //   warps 2-5   epilogue: tcgen05.ld 32 columns at a time (each warp its 32 TMEM lanes = 32
 //               rows), comparator epilogue for scores; the 32 x 32 block goes through a private
 //               swizzled shared-memory buffer (two per warp) and leaves as one bulk tensor
@@ -22,19 +22,20 @@
 // K-major operands use the 128-byte swizzle; MN-major tf32 operands must use the 128-byte swizzle
 // with 32-byte atoms (descriptor layout type 1, TMA swizzle 128B_ATOM_32B), 32 x 32 element boxes.
 //
-// TF32X3: the fp32 tiles TMA brings in are split in shared memory by eight warps: hi = tf32(x) in place, lo = x - hi into a second buffer of the
-// stage; the tile is lo.hi + hi.lo + hi.hi accumulated in fp32, which restores fp32-level
-// accuracy while every operand crosses HBM/L2 once, as plain fp32.
+// TF32X3: the fp32 tiles TMA brings in are split in shared memory by eight warps: hi = tf32(x) in place, lo = x - hi into a
+// buffer of its own; the tile is lo.hi + hi.lo + hi.hi accumulated in fp32, which restores fp32-level accuracy while every
+// operand crosses HBM/L2 once, as plain fp32.  What bounds the loop: with two stages of raw, hi and lo parts its period was half
+// of load + split + products + hand-overs (one after the other in a stage, 3,400 cycles a k-block of 256 columns where the
+// products take 1,540).  Now the loads run ahead through three raw stages and one buffer of lo parts serves them all: the products
+// that read it come first, and while hi.hi runs the split of the next stage, held in registers, moves in.  Scores of 1000-row
+// chunks at dimension 400 6.18 -> 5.80 ms, gradients 13.35 -> 12.31 (serial); 2,900 cycles a k-block of 208 columns, of which
+// shared memory is busy for 2,400 (TMA writes 45 KB, the split reads as much and writes it twice, the products read 127).
 //
 // Every wait on an mbarrier is bounded; when one runs out the CTA raises bit 1 of the error word,
 // stops issuing work, releases its tensor memory and returns.  Every TMA load is CTA-local.
 #include "pbg_tc.cuh"
 
-// k-values per pipeline stage: 32 (two stages of 96 KB with their low parts in TF32X3) or 16 (four stages of
-// 48 KB; K-major tiles then have 64-byte rows -- TMA 64-byte swizzle, descriptor layout 4, 512 bytes per 8
-// rows -- and MN-major boxes are 32 x 16, descriptor LBO 2048).  Both are verified and give the same speed:
-// the main loop is bound by shared-memory bandwidth (load 1x, split 3x, MMA operand reads 3x the tile per
-// stage), not by the depth of the ring, and a tile takes the same time whether 20 or 148 CTAs run.
+// k-values per pipeline stage
 #define TC_KB 32
 #define TC_THREADS 448          // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue, warps 6-13 split operands (TF32X3)
 #define TC_SPLIT_THREADS 256
@@ -72,35 +73,38 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
   // NTERMS == 2: the same on two planes per operand (x ~ b0 + b1) and the three products b1.b0, b0.b1, b0.b0
   constexpr bool PLANES = NTERMS == 6 || NTERMS == 2;
   constexpr int NPL = NTERMS == 6 ? 3 : 2;                               // planes per operand
-  static_assert(!PLANES || TC_KB == 32, "bf16 planes: 32 k-values per stage");
+  static_assert(TC_KB == 32, "layouts of a stage: 32 k-values");
   constexpr int KB = TC_KB;
-  constexpr int SMAX = PLANES ? 4 : (SPLIT ? 2 : 4) * (32 / KB);      // stages (bf16 planes: as many as fit, at most 4)
+  constexpr int SMAX = PLANES ? 4 : SPLIT ? 3 : 4;                       // stages (bf16 planes: as many as fit, at most 4)
   constexpr uint32_t ROW_BYTES = PLANES ? KB * 2 : KB * 4;               // bytes of one K-major row of a stage
   constexpr uint32_t BOX_BYTES = PLANES ? 4096 : KB * 128;               // one MN-major box: 64 x 32 bf16 or 32 x KB fp32
   constexpr uint32_t A_PLANE = 128 * ROW_BYTES, B_PLANE = 256 * ROW_BYTES;
   constexpr uint32_t A_BYTES = PLANES ? NPL * A_PLANE : A_PLANE, B_BYTES = PLANES ? NPL * B_PLANE : B_PLANE;   // one KB-k tile of 128 / 256 rows
   constexpr uint32_t RAW_BYTES = A_BYTES + B_BYTES;
-  constexpr uint32_t STAGE_BYTES = SPLIT ? 2 * RAW_BYTES : RAW_BYTES;   // [A hi][B hi] ([A lo][B lo]) or [A planes][B planes]
+  constexpr uint32_t STAGE_BYTES = RAW_BYTES;                            // [A][B], or [A planes][B planes]; SPLIT: hi parts in place
 
   extern __shared__ unsigned char smem_raw[];
   unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   // the plane tier sizes its stages by the tile's real width, and takes as many of them as fit
   const int STAGES = PLANES ? g.nst : SMAX;
   const uint32_t stage_bytes = PLANES ? (uint32_t)g.stage_bytes : STAGE_BYTES;
-  unsigned char *ostage = smem + (size_t)STAGES * stage_bytes;          // [4 warps][2][32 rows x 128 B], epilogue staging
-  __shared__ __align__(8) unsigned long long bars[3 * SMAX + 4];
+  unsigned char *lo = smem + (size_t)STAGES * stage_bytes;               // SPLIT: lo parts of one stage
+  unsigned char *ostage = lo + (SPLIT ? RAW_BYTES : 0u);                 // [4 warps][2][32 rows x 128 B], epilogue staging
+  __shared__ __align__(8) unsigned long long bars[2 * SMAX + 6];
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int failed;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t bar0 = smem_u32(&bars[0]);
   auto full_bar = [&](int s) { return bar0 + 8u * s; };                 // TMA landed
   auto empty_bar = [&](int s) { return bar0 + 8u * (SMAX + s); };     // MMAs have read the stage
-  auto conv_bar = [&](int s) { return bar0 + 8u * (2 * SMAX + s); };  // hi / lo written (SPLIT)
-  auto accf_bar = [&](int a) { return bar0 + 8u * (3 * SMAX + a); };      // accumulator a complete
-  auto acce_bar = [&](int a) { return bar0 + 8u * (3 * SMAX + 2 + a); };  // accumulator a drained
+  auto accf_bar = [&](int a) { return bar0 + 8u * (2 * SMAX + a); };      // accumulator a complete
+  auto acce_bar = [&](int a) { return bar0 + 8u * (2 * SMAX + 2 + a); };  // accumulator a drained
+  const uint32_t conv_bar = bar0 + 8u * (2 * SMAX + 4);                   // SPLIT: hi and lo parts of the stage in turn are written
+  const uint32_t lofree_bar = conv_bar + 8u;                              //        the products that read the lo parts are done
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2 * SMAX; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar0 + 8u * i));
-    for (int i = 0; i < SMAX; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(conv_bar(i)), "r"(TC_SPLIT_THREADS));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(conv_bar), "r"(TC_SPLIT_THREADS));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(lofree_bar));
     for (int a = 0; a < 2; ++a) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(accf_bar(a)));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 128;" :: "r"(acce_bar(a)));
@@ -181,19 +185,22 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
         }
       }
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     // instruction descriptor: D fp32, A/B tf32, operand majors, N >> 3, M >> 4
     const uint32_t fmt = PLANES ? 1u : 2u;            // operand format: bf16 (kind::f16) or tf32
     const uint32_t idesc0 = (1u << 4) | (fmt << 7) | (fmt << 10) | ((A_MN ? 1u : 0u) << 15) | ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(128 >> 4) << 24);
     const uint32_t idesc2 = (idesc0 & ~(1u << 16)) | ((uint32_t)(g.BN2 >> 3) << 17);   // dual: the B2 products are K-major, BN2 columns wide
+    const bool leader = elect_one();
     StageRing at;
+    uint32_t turn = 0;                                // SPLIT: parity of the stages so far
     int j = 0;
-    for (int t = blockIdx.x; t < ntiles && !failed; t += gridDim.x) {
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
       int p, blk, m0, n0;
+      if (__any_sync(0xffffffffu, failed != 0)) break;
       if (!tile_live(t, p, blk, m0, n0)) continue;
       const int ab = j & 1;
-      if (j >= 2 && !mbar_wait(acce_bar(ab), (uint32_t)((j >> 1) - 1) & 1, errflag)) { failed = 1; break; }
+      if (j >= 2 && !__all_sync(0xffffffffu, mbar_wait(acce_bar(ab), (uint32_t)((j >> 1) - 1) & 1, errflag))) { failed = 1; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tacc = tmem + (uint32_t)ab * 256u;
       const int ncols = g.N - n0 < g.BN ? (g.N - n0 + 15) / 16 * 16 : g.BN;                 // columns of this tile that exist
@@ -201,11 +208,10 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
       bool ok = true;
       for (int kb = 0; kb < nkb; ++kb, at.next(STAGES)) {
         const int s = at.s;
-        if (!mbar_wait(SPLIT ? conv_bar(s) : full_bar(s), at.parity, errflag)) { failed = 1; ok = false; break; }
+        if (!__all_sync(0xffffffffu, mbar_wait(SPLIT ? conv_bar : full_bar(s), SPLIT ? turn : at.parity, errflag))) { failed = 1; ok = false; break; }
+        turn ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        unsigned char *st = smem + (size_t)s * stage_bytes;
-        uint32_t aH = smem_u32(st), bH = smem_u32(st + A_BYTES);
-        uint32_t aL = aH + RAW_BYTES, bL = bH + RAW_BYTES;
+        const uint32_t aH = smem_u32(smem) + (uint32_t)s * stage_bytes, bH = aH + A_BYTES;
         const int kleft = g.K - kb * KB;                        // k-values of this block that exist (the rest is zero fill)
         if (PLANES) {
           // plane pairs (a, b) of order a + b <= 2, the smallest contributions first; K = 16 per MMA:
@@ -214,67 +220,68 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
           // (two planes: the last three pairs of the list)
           const int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
           constexpr int T0 = NPL == 3 ? 0 : 3;
+          constexpr uint32_t a_step = A_MN ? 2048 : 32, b_step = B_MN ? 2048 : 32;
           const int kleft1 = dual ? g.K1 - kb * KB : kleft;    // k-values of this block under B1
+          const uint64_t da0 = A_MN ? smem_desc(aH, MN_STRIDE, 1024, 2) : smem_desc(aH, 0, 512, 4);
+          const uint64_t db0 = B_MN ? smem_desc(bH, MN_STRIDE, 1024, 2) : smem_desc(bH, 0, 512, 4);
+          const uint64_t dc0 = smem_desc(bH + b_used, 0, 512, 4);
 #pragma unroll
           for (int k16 = 0; k16 < 2; ++k16) {
             if (k16 * 16 >= kleft) break;                     // the tail of K: those k-values are zero fill
+            if (!dual || k16 * 16 < kleft1) {                 // (past K1: no B1 product for these k-values)
 #pragma unroll
-            for (int t = T0; t < 6; ++t) {
-              uint64_t da = A_MN ? smem_desc(aH + pa[t] * a_plane + k16 * 2048, MN_STRIDE, 1024, 2)
-                                 : smem_desc(aH + pa[t] * a_plane + k16 * 32, 0, 512, 4);
-              uint64_t db = B_MN ? smem_desc(bH + pb[t] * b_plane + k16 * 2048, MN_STRIDE, 1024, 2)
-                                 : smem_desc(bH + pb[t] * b_plane + k16 * 32, 0, 512, 4);
-              uint32_t acc = (kb > 0 || k16 > 0 || t > T0) ? 1u : 0u;
-              if (dual && k16 * 16 >= kleft1) continue;       // past K1: no B1 product for these k-values
-              asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-                           :: "r"(tacc), "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
+              for (int t = T0; t < 6; ++t)
+                if (leader) mma_f16(tacc, desc_at(da0, pa[t] * a_plane + k16 * a_step), desc_at(db0, pb[t] * b_plane + k16 * b_step), idesc, kb > 0 || k16 > 0 || t > T0);
             }
             if (dual) {
               // B2 = rows of the other problem's coefficient matrix: every k-block, BN2 columns wide, always
               // accumulating -- the first product of a tile is a B1 product (k-block 0 carries B1 and K1 >= 1),
               // which initialises all BN columns
 #pragma unroll
-              for (int t = T0; t < 6; ++t) {
-                uint64_t da = smem_desc(aH + pa[t] * a_plane + k16 * 2048, MN_STRIDE, 1024, 2);
-                uint64_t db = smem_desc(bH + b_used + pb[t] * b2_plane + k16 * 32, 0, 512, 4);
-                asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-                             :: "r"(tacc), "l"(da), "l"(db), "r"(idesc2), "r"(1u) : "memory");
-              }
+              for (int t = T0; t < 6; ++t)
+                if (leader) mma_f16(tacc, desc_at(da0, pa[t] * a_plane + k16 * a_step), desc_at(dc0, pb[t] * b2_plane + k16 * 32), idesc2, true);
             }
           }
-        } else
-#pragma unroll
-        for (int k8 = 0; k8 < KB / 8; ++k8) {
-          if (k8 * 8 >= kleft) break;                         // the tail of K: those k-values are zero fill
+        } else {
           constexpr uint32_t KSBO = KB == 32 ? 1024 : 512, KLAY = KB == 32 ? 2 : 4;     // K-major: 8 rows of ROW_BYTES; 128- / 64-byte swizzle
-          uint32_t ao = A_MN ? k8 * 1024 : k8 * 32, bo = B_MN ? k8 * 1024 : k8 * 32;
-          uint64_t dAh = A_MN ? smem_desc(aH + ao, BOX_BYTES, 512, 1) : smem_desc(aH + ao, 0, KSBO, KLAY);
-          uint64_t dBh = B_MN ? smem_desc(bH + bo, BOX_BYTES, 512, 1) : smem_desc(bH + bo, 0, KSBO, KLAY);
-          uint32_t acc = (kb > 0 || k8 > 0) ? 1u : 0u;
-          if (SPLIT) {
-            uint64_t dAl = A_MN ? smem_desc(aL + ao, BOX_BYTES, 512, 1) : smem_desc(aL + ao, 0, KSBO, KLAY);
-            uint64_t dBl = B_MN ? smem_desc(bL + bo, BOX_BYTES, 512, 1) : smem_desc(bL + bo, 0, KSBO, KLAY);
-            asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}"
-                         :: "r"(tacc), "l"(dAl), "l"(dBh), "r"(idesc), "r"(acc) : "memory");
-            asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}"
-                         :: "r"(tacc), "l"(dAh), "l"(dBl), "r"(idesc), "r"(1u) : "memory");
-            acc = 1u;
+          constexpr uint32_t a_step = A_MN ? 1024 : 32, b_step = B_MN ? 1024 : 32;
+          const uint64_t da0 = A_MN ? smem_desc(aH, BOX_BYTES, 512, 1) : smem_desc(aH, 0, KSBO, KLAY);
+          const uint64_t db0 = B_MN ? smem_desc(bH, BOX_BYTES, 512, 1) : smem_desc(bH, 0, KSBO, KLAY);
+if (SPLIT) {
+            // the two products with lo parts first: their buffer goes back while hi . hi runs
+            const uint32_t lo0 = smem_u32(lo);
+            const uint64_t dal0 = A_MN ? smem_desc(lo0, BOX_BYTES, 512, 1) : smem_desc(lo0, 0, KSBO, KLAY);
+            const uint64_t dbl0 = B_MN ? smem_desc(lo0 + A_BYTES, BOX_BYTES, 512, 1) : smem_desc(lo0 + A_BYTES, 0, KSBO, KLAY);
+#pragma unroll
+            for (int k8 = 0; k8 < KB / 8; ++k8) {
+              if (k8 * 8 >= kleft) break;
+              if (leader) {
+                mma_tf32(tacc, desc_at(dal0, k8 * a_step), desc_at(db0, k8 * b_step), idesc, kb > 0 || k8 > 0);
+                mma_tf32(tacc, desc_at(da0, k8 * a_step), desc_at(dbl0, k8 * b_step), idesc, true);
+              }
+            }
+            if (leader) mma_commit(lofree_bar);
           }
-          asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}"
-                       :: "r"(tacc), "l"(dAh), "l"(dBh), "r"(idesc), "r"(acc) : "memory");
+#pragma unroll
+          for (int k8 = 0; k8 < KB / 8; ++k8) {
+            if (k8 * 8 >= kleft) break;                       // the tail of K: those k-values are zero fill
+            if (leader) mma_tf32(tacc, desc_at(da0, k8 * a_step), desc_at(db0, k8 * b_step), idesc, SPLIT || kb > 0 || k8 > 0);
+          }
         }
         // frees the stage for the producer once the MMAs above have read it
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(empty_bar(s)) : "memory");
+        if (leader) mma_commit(empty_bar(s));
       }
       if (!ok) break;
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(accf_bar(ab)) : "memory");
+      if (leader) mma_commit(accf_bar(ab));
       ++j;
     }
   } else if (SPLIT && warp >= 6) {
     // ---------------- hi / lo split of every landed stage (warps 6-13) ----------------
     const int ct = threadIdx.x - 192;                             // 0..255
     const uint32_t nchunks = stage_tx / 16;
+    constexpr int SPLIT_PART = (int)(RAW_BYTES / 16 / TC_SPLIT_THREADS);
     StageRing at;
+    uint32_t turn = 0;
     bool stop = false;
     for (int t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
       int p, blk, m0, n0;
@@ -288,25 +295,33 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
         if (lane == 0) okw = mbar_wait(full_bar(s), at.parity, errflag);
         if (!__all_sync(0xffffffffu, okw)) { failed = 1; stop = true; break; }
         unsigned char *st = smem + (size_t)s * stage_bytes;
-        for (uint32_t c0 = ct; c0 < nchunks; c0 += 4 * TC_SPLIT_THREADS) {
-          float4 v[4];
+        // A thread's part of the stage (at most SPLIT_PART pieces of 16 bytes): hi parts in place at once, lo parts kept until
+        // the products of the stage before have read theirs.
+        float4 v[SPLIT_PART];
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            uint32_t c = c0 + u * TC_SPLIT_THREADS;
-            if (c < nchunks) v[u] = *reinterpret_cast<const float4 *>(st + (size_t)c * 16);
-          }
+        for (int u = 0; u < SPLIT_PART; ++u) {
+          const uint32_t c = ct + u * TC_SPLIT_THREADS;
+          if (c < nchunks) v[u] = *reinterpret_cast<const float4 *>(st + (size_t)c * 16);
+        }
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            uint32_t c = c0 + u * TC_SPLIT_THREADS;
-            if (c < nchunks) {
-              float4 h = tf32_round4(v[u]);
-              *reinterpret_cast<float4 *>(st + (size_t)c * 16) = h;
-              *reinterpret_cast<float4 *>(st + RAW_BYTES + (size_t)c * 16) = v[u] - h;
-            }
+        for (int u = 0; u < SPLIT_PART; ++u) {
+          const uint32_t c = ct + u * TC_SPLIT_THREADS;
+          if (c < nchunks) {
+            const float4 h = tf32_round4(v[u]);
+            *reinterpret_cast<float4 *>(st + (size_t)c * 16) = h;
+            v[u] = v[u] - h;
           }
         }
+        if (lane == 0) okw = mbar_wait(lofree_bar, turn ^ 1u, errflag);
+        turn ^= 1u;
+        if (!__all_sync(0xffffffffu, okw)) { failed = 1; stop = true; break; }
+#pragma unroll
+        for (int u = 0; u < SPLIT_PART; ++u) {
+          const uint32_t c = ct + u * TC_SPLIT_THREADS;
+          if (c < nchunks) *reinterpret_cast<float4 *>(lo + (size_t)c * 16) = v[u];
+        }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> tensor-core reads
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(conv_bar(s)) : "memory");
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(conv_bar) : "memory");
       }
     }
   } else if (warp >= 2 && warp < 6) {

@@ -51,6 +51,28 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
          ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46) | ((uint64_t)layout << 61);
 }
 
+// One lane of a converged warp.  The warp that issues products runs its loop as a whole -- waits, counters and descriptors are
+// the same in every lane, so that they live in uniform registers, which is where the instruction takes them from -- and one
+// lane issues.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(one));
+  return one != 0;
+}
+// D (+)= A . B on shared-memory descriptors
+__device__ __forceinline__ void mma_f16(uint32_t acc, uint64_t a, uint64_t b, uint32_t idesc, bool add) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" :: "r"(acc), "l"(a), "l"(b), "r"(idesc), "r"(add ? 1u : 0u) : "memory");
+}
+__device__ __forceinline__ void mma_tf32(uint32_t acc, uint64_t a, uint64_t b, uint32_t idesc, bool add) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}" :: "r"(acc), "l"(a), "l"(b), "r"(idesc), "r"(add ? 1u : 0u) : "memory");
+}
+// arrives on the barrier when the products issued so far are done
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
+}
+// The descriptor of an operand `bytes` (a multiple of 16) further on: shared-memory addresses fit the field without a carry.
+__device__ __forceinline__ uint64_t desc_at(uint64_t desc, uint32_t bytes) { return desc + (bytes >> 4); }
+
 // 32 columns of this thread's tensor-memory lane
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
