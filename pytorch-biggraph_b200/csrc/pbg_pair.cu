@@ -123,50 +123,47 @@ pair_score_kernel(const __grid_constant__ PairMaps maps, PairGeom g, WaveDims d,
         if (lane < 2) tma_load_4d(smem_u32(smem + (size_t)s * g.stage_bytes) + lane * arr_bytes, &maps.n[lane], kb * 32, 0, 0, blk, fb);
       }
     }
-  } else if (warp == 1 && lane == 0) {
-    // ---------------- MMA issuer ----------------
+  } else if (warp == 1) {
+    // ---------------- MMA issuer (elect_one) ----------------
     // instruction descriptor: D fp32, A / B bf16, both K-major, N >> 3, M = 128
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(g.BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
     // plane pairs (a, b) of order a + b <= 2, the smallest contributions first; two planes: the last three
     const int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
     constexpr int T0 = NPL == 3 ? 0 : 3;
+    const bool leader = elect_one();
     StageRing at;
     int j = 0;
-    for (int t = blockIdx.x; t < d.nblk && !failed; t += gridDim.x) {
+    for (int t = blockIdx.x; t < d.nblk; t += gridDim.x) {
+      if (__any_sync(0xffffffffu, failed != 0)) break;
       if (!tile_live(t)) continue;
       const int set = j % SETS;
       const uint32_t tset = tmem + (uint32_t)set * 2u * ACC;
-      if (j >= SETS && !mbar_wait(acce_bar(set), (uint32_t)(j / SETS - 1) & 1, errflag)) { failed = 1; break; }
+      if (j >= SETS && !__all_sync(0xffffffffu, mbar_wait(acce_bar(set), (uint32_t)(j / SETS - 1) & 1, errflag))) { failed = 1; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       bool ok = true;
       for (int kb = 0; kb < nkb; ++kb, at.next(STAGES)) {
         const int s = at.s;
-        if (!mbar_wait(full_bar(s), at.parity, errflag)) { failed = 1; ok = false; break; }
+        if (!__all_sync(0xffffffffu, mbar_wait(full_bar(s), at.parity, errflag))) { failed = 1; ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t st = smem_u32(smem + (size_t)s * g.stage_bytes);
+        const uint32_t st = smem_u32(smem) + (uint32_t)(s * g.stage_bytes);
         const int kleft = d.D - kb * 32;
+        const uint64_t n0 = smem_desc(st, 0, 512, 4), n1 = smem_desc(st + arr_bytes, 0, 512, 4);
 #pragma unroll
         for (int k16 = 0; k16 < 2; ++k16) {
           if (k16 * 16 >= kleft) break;                          // the tail of K is zero fill
 #pragma unroll
           for (int tt = T0; tt < 6; ++tt) {
-            const uint32_t acc = (kb > 0 || k16 > 0 || tt > T0) ? 1u : 0u;
-#pragma unroll
-            for (int p = 0; p < 2; ++p) {
-              if (!d.neg_enabled[p]) continue;
-              // problem 0: A = rows of N1 (array 1), B = rows of N0 (array 0); problem 1 the other way round
-              const uint32_t aarr = p == 0 ? 1u : 0u, barr = 1u - aarr;
-              const uint64_t da = smem_desc(st + aarr * arr_bytes + pa[tt] * plane_bytes + k16 * 32, 0, 512, 4);
-              const uint64_t db = smem_desc(st + barr * arr_bytes + pb[tt] * plane_bytes + k16 * 32, 0, 512, 4);
-              asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-                           :: "r"(tset + (uint32_t)p * ACC), "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
-            }
+            const uint32_t oa = pa[tt] * plane_bytes + k16 * 32, ob = pb[tt] * plane_bytes + k16 * 32;
+            const bool add = kb > 0 || k16 > 0 || tt > T0;
+            // problem 0: A = rows of N1 (array 1), B = rows of N0 (array 0); problem 1 the other way round
+            if (leader && d.neg_enabled[0]) mma_f16(tset, desc_at(n1, oa), desc_at(n0, ob), idesc, add);
+            if (leader && d.neg_enabled[1]) mma_f16(tset + ACC, desc_at(n0, oa), desc_at(n1, ob), idesc, add);
           }
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(empty_bar(s)) : "memory");
+        if (leader) mma_commit(empty_bar(s));
       }
       if (!ok) break;
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(accf_bar(set)) : "memory");
+      if (leader) mma_commit(accf_bar(set));
       ++j;
     }
   } else if (warp >= 2) {

@@ -83,36 +83,36 @@ allnegs_tc_kernel(const __grid_constant__ RankMaps maps, WaveDims d, WaveBufs w,
         else if (lane == 1) tma_load_4d(st + 3 * RK_PLANE_A, &maps.y, kb * 32, n0, 0, side, fb);
       }
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(RK_BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
     const int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};   // smallest contributions first
-    int git = 0, j = 0;
-    for (int t = blockIdx.x; t < ntiles && !failed; t += gridDim.x) {
+    const bool leader = elect_one();
+    StageRing at;
+    int j = 0;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+      if (__any_sync(0xffffffffu, failed != 0)) break;
       if (!tile_live(t, side, m0, n0, n)) continue;
       const int ab = j & 1;
-      if (j >= 2 && !mbar_wait(acce_bar(ab), (uint32_t)((j >> 1) - 1) & 1, errflag)) { failed = 1; break; }
+      if (j >= 2 && !__all_sync(0xffffffffu, mbar_wait(acce_bar(ab), (uint32_t)((j >> 1) - 1) & 1, errflag))) { failed = 1; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       bool ok = true;
-      for (int kb = 0; kb < nkb; ++kb, ++git) {
-        const int s = git % RK_STAGES;
-        if (!mbar_wait(full_bar(s), (uint32_t)(git / RK_STAGES) & 1, errflag)) { failed = 1; ok = false; break; }
+      for (int kb = 0; kb < nkb; ++kb, at.next(RK_STAGES)) {
+        const int s = at.s;
+        if (!__all_sync(0xffffffffu, mbar_wait(full_bar(s), at.parity, errflag))) { failed = 1; ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t sa = smem_u32(smem + (size_t)s * RK_STAGE), sb = sa + 3 * RK_PLANE_A;
+        const uint32_t sa = smem_u32(smem) + (uint32_t)s * RK_STAGE;
+        const uint64_t da = smem_desc(sa, 0, 512, 4), db = smem_desc(sa + 3 * RK_PLANE_A, 0, 512, 4);
 #pragma unroll
         for (int k16 = 0; k16 < 2; ++k16) {
           if (k16 * 16 >= d.D - kb * 32) break;                          // the tail of K is zero fill
 #pragma unroll
-          for (int tt = 0; tt < 6; ++tt) {
-            const uint32_t acc = (kb > 0 || k16 > 0 || tt > 0) ? 1u : 0u;
-            asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-                         :: "r"(tmem + (uint32_t)ab * 256u), "l"(smem_desc(sa + pa[tt] * RK_PLANE_A + k16 * 32, 0, 512, 4)),
-                            "l"(smem_desc(sb + pb[tt] * RK_PLANE_B + k16 * 32, 0, 512, 4)), "r"(idesc), "r"(acc) : "memory");
-          }
+          for (int tt = 0; tt < 6; ++tt)
+            if (leader) mma_f16(tmem + (uint32_t)ab * 256u, desc_at(da, pa[tt] * RK_PLANE_A + k16 * 32), desc_at(db, pb[tt] * RK_PLANE_B + k16 * 32), idesc, kb > 0 || k16 > 0 || tt > 0);
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(empty_bar(s)) : "memory");
+        if (leader) mma_commit(empty_bar(s));
       }
       if (!ok) break;
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(accf_bar(ab)) : "memory");
+      if (leader) mma_commit(accf_bar(ab));
       ++j;
     }
   } else if (warp >= 2) {
