@@ -653,39 +653,43 @@ narrow_tile_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
   }
 }
 
-// End of the prefix of [lo, hi) on which pred holds (pred must hold on a prefix only).  The whole CTA
-// probes blockDim.x evenly spaced positions per round: two rounds for any wave size instead of a
-// chain of ~16 dependent loads by one thread.  Every thread returns the same value.
-template <class Pred>
-__device__ __forceinline__ long long coop_prefix_end(long long lo, long long hi, Pred pred) {
-  while (lo < hi) {
-    long long stride = (hi - lo + blockDim.x - 1) / blockDim.x;
-    long long pos = lo + (long long)threadIdx.x * stride;
-    int cnt = __syncthreads_count(pos < hi && pred(pos));
-    if (cnt == 0) return lo;
-    long long nhi = lo + (long long)cnt * stride;
-    lo = lo + (long long)(cnt - 1) * stride + 1;
-    if (nhi < hi) hi = nhi;
-    if (stride == 1) return hi;
+// First slot of batch b, and first of a later batch, among the slots of the row `key` that starts at head: two such searches in
+// the same rounds.  Row and batch are ascending along the list, so "still in the row and below b" and "still in the row and
+// not above b" hold on prefixes; the first round probes the same positions for both.  (Three searches one after the other -- the
+// row's end, then the batch in it -- were six rounds of a load and a barrier, of about 1,000 cycles each: hub kernel and all of a
+// plumbing wave 115.3 -> 114.5 us.)
+template <class Key, class Batch>
+__device__ __forceinline__ void coop_batch_range(const unsigned long long *keys, const unsigned int *vals, long long head, long long end, unsigned long long key, int b,
+                                                 Key &&key_at, Batch &&batch_at, long long &q, long long &eb) {
+  long long lo[2] = {head, head}, hi[2] = {end, end};
+  bool same = true;                                          // both ranges are the same so far: one probe serves both
+  while (lo[0] < hi[0] || lo[1] < hi[1]) {
+    long long stride[2];
+    int in[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      stride[u] = (hi[u] - lo[u] + blockDim.x - 1) / blockDim.x;
+      const long long pos = lo[u] + (long long)threadIdx.x * stride[u];
+      if (u == 0 || !same) {
+        in[u] = -1;
+        if (pos < hi[u] && key_at(keys + pos) == key) in[u] = batch_at(vals + pos);
+        else if (pos < hi[u]) in[u] = PBG_KMAX;              // behind the row
+      } else in[1] = in[0];
+    }
+    const int cnt[2] = {__syncthreads_count(in[0] >= 0 && in[0] < b), __syncthreads_count(in[1] >= 0 && in[1] <= b)};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (lo[u] >= hi[u]) continue;
+      if (cnt[u] == 0) { hi[u] = lo[u]; continue; }
+      const long long nhi = lo[u] + (long long)cnt[u] * stride[u];
+      lo[u] += (long long)(cnt[u] - 1) * stride[u] + 1;
+      if (nhi < hi[u]) hi[u] = nhi;
+      if (stride[u] == 1) lo[u] = hi[u];
+    }
+    same = same && lo[0] == lo[1] && hi[0] == hi[1];
   }
-  return hi;
-}
-
-// The same for one warp: 32 probes per round.  Every lane returns the same value.
-template <class Pred>
-__device__ __forceinline__ long long warp_prefix_end(long long lo, long long hi, Pred pred) {
-  const int lane = threadIdx.x & 31;
-  while (lo < hi) {
-    long long stride = (hi - lo + 31) / 32;
-    long long pos = lo + (long long)lane * stride;
-    int cnt = __popc(__ballot_sync(0xffffffffu, pos < hi && pred(pos)));
-    if (cnt == 0) return lo;
-    long long nhi = lo + (long long)cnt * stride;
-    lo = lo + (long long)(cnt - 1) * stride + 1;
-    if (nhi < hi) hi = nhi;
-    if (stride == 1) return hi;
-  }
-  return hi;
+  q = hi[0];
+  eb = hi[1];
 }
 
 // Per-batch Stats (train_cpu.py:95-101) of batch b of the wave, summed by one CTA in a fixed order; the running totals
@@ -756,7 +760,6 @@ hub_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__r
   __shared__ float bnorm[PBG_KMAX];                           // mean squared gradient of a batch (embedding rows)
   __shared__ int sbatch[32 * UPD_WARPS];
   __shared__ unsigned long long skey;
-  __shared__ long long bend;
   __shared__ bool closing;
   if (blockIdx.x == 0 && threadIdx.x < 2) hubcnt_next[threadIdx.x] = 0;      // its last reader is behind us in the stream
   // the first CTAs of the embedding rows' launch (aside) have other work
@@ -777,15 +780,14 @@ hub_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__r
     const bool from_big = item < nbig * d.k;
     const int h = item / d.k;
     const long long head = ld_list<RULE>(from_big ? biglist + h : hublist + (item - nbig * d.k));
-    long long *line = bigtab + (size_t)h * BIGTAB_LINE;       // [b] first slot of batch b or -1, then the row's end, then a counter
+    long long *line = bigtab + (size_t)h * BIGTAB_LINE;       // [b] first slot of batch b or -1; last: a counter
     if (from_big) {
       const int b = item - h * d.k;
       const unsigned long long key = ld_list<RULE>(keys + head);
-      const long long end = coop_prefix_end(head + HUB_BIG, (long long)d.nocc, [&](long long pos) { return ld_list<RULE>(keys + pos) == key; });
-      // where batch b starts and ends inside the row.  (Both searches in the same rounds, half of the CTA each, measured
-      // slower: 14.2 against 11.8 us.)
-      const long long q = coop_prefix_end(head, end, [&](long long pos) { return d.bySpb.div((int)ld_list<RULE>(vals + pos)) < b; });
-      const long long eb = coop_prefix_end(q, end, [&](long long pos) { return d.bySpb.div((int)ld_list<RULE>(vals + pos)) <= b; });
+      // where batch b starts and ends inside the row (both right behind it where it has no slot there)
+      long long q, eb;
+      coop_batch_range(keys, vals, head, (long long)d.nocc, key, b, [&](const unsigned long long *p) { return ld_list<RULE>(p); },
+                       [&](const unsigned int *p) { return d.bySpb.div((int)ld_list<RULE>(p)); }, q, eb);
       const long long ftb = (q / TILE + 1) * TILE;
       const long long nruns = q < eb ? 1 + (eb > ftb ? (eb - 1 - ftb) / TILE + 1 : 0) : 0;
       if (nruns > 1) {
@@ -823,10 +825,7 @@ hub_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__r
           st4(dst + dd, t);
         }
       }
-      if (threadIdx.x == 0) {
-        line[b] = q < eb ? q : -1;
-        if (b == 0) line[PBG_KMAX] = end;
-      }
+      if (threadIdx.x == 0) line[b] = q < eb ? q : -1;
       __threadfence();
       __syncthreads();
       if (threadIdx.x == 0) closing = atomicAdd((unsigned long long *)&line[PBG_KMAX + 1], 1ull) == (unsigned long long)(d.k - 1);
@@ -839,7 +838,7 @@ hub_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__r
     const unsigned long long kp = p < (long long)d.nocc ? ld_list<RULE>(keys + p) : ~0ull;
     const int bp = p < (long long)d.nocc ? d.bySpb.div((int)ld_list<RULE>(vals + p)) : -1;
     // what the CTAs of a big row's batches left (past L1: this CTA may have read the lines before)
-    const long long tabv = from_big && threadIdx.x <= PBG_KMAX ? __ldcg(line + threadIdx.x) : -1;
+    const long long tabv = from_big && threadIdx.x < PBG_KMAX ? __ldcg(line + threadIdx.x) : -1;
     if (threadIdx.x == 0) skey = kp;
     for (int i = threadIdx.x; i <= PBG_KMAX; i += blockDim.x) bstart[i] = -1;
     __syncthreads();
@@ -858,15 +857,13 @@ hub_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__r
     const int cnt = __syncthreads_count(in);                  // slots of the row among the first 256 (they are contiguous)
     const bool big = cnt == (int)blockDim.x;                  // one row per batch is left of it
     if (big && !from_big) continue;                           // taken from the list of big rows
-    long long end = head + cnt;
+    const long long end = head + cnt;                         // (not of a big row: it has one partial row per batch)
     if (!big) {
       if (in && (threadIdx.x == 0 || sbatch[threadIdx.x - 1] != bp)) bstart[bp] = p;     // first slot of batch bp
     } else {
       if (threadIdx.x < d.k) bstart[threadIdx.x] = tabv;
-      if (threadIdx.x == PBG_KMAX) bend = tabv;
     }
     __syncthreads();
-    if (big) end = bend;
     // ---- per-batch totals ----
     for (int bq = wl; bq < d.k; bq += UPD_WARPS) {
       long long q = bstart[bq];
