@@ -11,8 +11,16 @@
 
 #define GATHER_WARPS 8
 
+// Resident CTAs per SM, by the float4 a lane holds of a row.  A warp waits for one row after the other, so what counts is warps, as
+// long as registers last (gather class of whole buckets, serial): general kernel, rows of up to 128 floats 5 CTAs (two planes:
+// 0.67 ms at 3, 0.59 at 4, 0.55 at 5), of 256 4 (1.09 at 3, 0.99), of 512 3 (1.87; 2.10 at 4 and 2.15 at 2); plain kernel, rows of
+// up to 256 floats 6 (three planes: 1.57 at 4, 1.43 at 6, 1.44 at 8), of 1024 2 (2.09 at 3 with registers spilled, 1.96, 2.74 at 4).
+template <int VEC> struct GatherCtas {
+  enum { GENERAL = VEC >= 8 ? 2 : VEC == 4 ? 3 : VEC == 2 ? 4 : 5, PLAIN = VEC >= 16 ? 1 : VEC == 8 ? 2 : VEC == 4 ? 4 : 6 };
+};
+
 template <int VEC, bool PL>
-__global__ void __launch_bounds__(32 * GATHER_WARPS, VEC >= 8 ? 2 : 3) gather_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
+__global__ void __launch_bounds__(32 * GATHER_WARPS, GatherCtas<VEC>::GENERAL) gather_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   pdl_begin();
   const int item = (int)blockIdx.x * GATHER_WARPS + (int)(threadIdx.x >> 5);
   if (item >= d.nblk * d.Mm) return;
@@ -26,7 +34,7 @@ __global__ void __launch_bounds__(32 * GATHER_WARPS, VEC >= 8 ? 2 : 3) gather_ke
 // a warp keeps in flight, and the kernel carries none of the operator / prepare code of the general
 // one (half the registers, three CTAs per SM instead of two).
 template <int VEC, bool PL>
-__global__ void __launch_bounds__(32 * GATHER_WARPS, VEC >= 16 ? 1 : VEC >= 8 ? 3 : 4) gather_plain_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
+__global__ void __launch_bounds__(32 * GATHER_WARPS, GatherCtas<VEC>::PLAIN) gather_plain_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   pdl_begin();
   int lane = threadIdx.x & 31;
   const int item = (int)blockIdx.x * GATHER_WARPS + (int)(threadIdx.x >> 5);
