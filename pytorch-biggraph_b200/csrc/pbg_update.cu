@@ -608,6 +608,23 @@ narrow_tile_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
         for (int c = 0; c < NP; ++c) v[c] = v[c] * sc;
       }
     }
+    // A slot each, as for most rows of a wave: no loop over batches (update class of the plumbing bucket 3.55 -> 3.48 ms).
+    if (__all_sync(FULL, n <= 1 && !is_hub)) {
+      const float *g = (const float *)__shfl_sync(FULL, (unsigned long long)src, start & 31);
+      if (n == 1) {
+#pragma unroll
+        for (int c = 0; c < NP; ++c) if (ok[c]) acc[c] = acc[c] + ld4(g + c * 64 + l16 * 4);
+      }
+      const float ss = square(acc);
+      if (n == 1) {
+        G += ss * invD;
+        const float stepv = lr / (sqrtf(G) + PBG_ADAGRAD_EPS);
+#pragma unroll
+        for (int c = 0; c < NP; ++c) if (ok[c]) st4(prow + c * 64 + l16 * 4, v[c] - acc[c] * stepv);
+        if (l16 == 0) *pacc = G;
+      }
+      continue;
+    }
     const int other = __shfl_xor_sync(FULL, n, 16), most = n > other ? n : other;
     int cur = -1, run_start = 0;
     for (int j = 0; j <= most; ++j) {
