@@ -86,38 +86,58 @@ __global__ void __launch_bounds__(256) randperm_deal_kernel(long long n, unsigne
   }
 }
 
-// one CTA per bucket: bitonic sort of its keys (padded to a power of two), indices out behind the smaller buckets'.  Pairs at
-// a distance of 32 and less lie inside one warp's 64 keys: between two such steps the warp waits for itself only.
+// One CTA per bucket orders its keys by counting: a thousand bins of the hash's next bits, at most a few keys in each, then
+// every key counts the smaller ones of its own bin.  Five barriers whatever the size; the bitonic sort of the keys before it
+// was 55 steps in a row, 27 us for 269,507 indices (7.3 us now).  The indices leave behind the smaller buckets'.
 #define RP_SORT_THREADS 512
+#define RP_BIN_BITS 10
 __global__ void __launch_bounds__(RP_SORT_THREADS) randperm_sort_kernel(const unsigned long long *__restrict__ buckets, const unsigned int *__restrict__ count,
-                                                                        int index_bits, long long *__restrict__ out) {
+                                                                        int key_bits, int index_bits, long long *__restrict__ out) {
+  constexpr int PER = RP_CAP / RP_SORT_THREADS, WARPS = RP_SORT_THREADS / 32;
   __shared__ unsigned long long key[RP_CAP];
-  __shared__ unsigned int below[RP_SORT_THREADS / 32];
-  const int t = threadIdx.x, b = blockIdx.x;
+  __shared__ unsigned int start[(1 << RP_BIN_BITS) + 1];      // the bins' counts, then where each begins
+  __shared__ unsigned int below[WARPS], bins[WARPS];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5, b = blockIdx.x, shift = key_bits - RP_BIN_BITS;
   const int n = count[b] < RP_CAP ? (int)count[b] : RP_CAP;
+  start[t] = start[t + RP_SORT_THREADS] = 0u;
   unsigned int s = 0u;
   for (int i = t; i < b; i += RP_SORT_THREADS) s += count[i];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((t & 31) == 0) below[t >> 5] = s;
-  int size = 64;
-  while (size < n) size <<= 1;
-  for (int i = t; i < size; i += RP_SORT_THREADS) key[i] = i < n ? buckets[(size_t)b * RP_CAP + i] : ~0ull;
+  if (lane == 0) below[w] = s;
+  unsigned long long k[PER];
+  unsigned int at[PER];
+#pragma unroll
+  for (int u = 0; u < PER; ++u)
+    if (t + u * RP_SORT_THREADS < n) k[u] = buckets[(size_t)b * RP_CAP + t + u * RP_SORT_THREADS];
   __syncthreads();
-  for (int k = 2; k <= size; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int p = t; p < size / 2; p += RP_SORT_THREADS) {
-        const int lo = ((p & ~(j - 1)) << 1) | (p & (j - 1)), hi = lo + j;
-        const unsigned long long x = key[lo], y = key[hi];
-        if ((x > y) == ((lo & k) == 0)) { key[lo] = y; key[hi] = x; }
-      }
-      const int next = j > 1 ? j >> 1 : k;                    // distance of the step that follows
-      if (j > 32 || next > 32) __syncthreads(); else __syncwarp();
-    }
+#pragma unroll
+  for (int u = 0; u < PER; ++u)
+    if (t + u * RP_SORT_THREADS < n) at[u] = atomicAdd(&start[k[u] >> shift], 1u);
   __syncthreads();
-  unsigned int base = 0u;
-  for (int u = 0; u < RP_SORT_THREADS / 32; ++u) base += below[u];
-  for (int i = t; i < n; i += RP_SORT_THREADS) out[base + i] = (long long)(key[i] & ((1ull << index_bits) - 1ull));
+  const unsigned int c0 = start[2 * t], c1 = start[2 * t + 1];
+  unsigned int incl = c0 + c1;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) { const unsigned int x = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += x; }
+  if (lane == 31) bins[w] = incl;
+  __syncthreads();
+  unsigned int base = 0u, first = incl - c0 - c1;
+#pragma unroll
+  for (int u = 0; u < WARPS; ++u) { base += below[u]; first += u < w ? bins[u] : 0u; }
+  start[2 * t] = first;
+  start[2 * t + 1] = first + c0;
+  if (t == 0) start[1 << RP_BIN_BITS] = (unsigned int)n;
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < PER; ++u)
+    if (t + u * RP_SORT_THREADS < n) key[start[k[u] >> shift] + at[u]] = k[u];
+  __syncthreads();
+  for (int i = t; i < n; i += RP_SORT_THREADS) {
+    const unsigned long long x = key[i];
+    unsigned int pos = start[x >> shift];
+    for (unsigned int j = pos, end = start[(x >> shift) + 1]; j < end; ++j) pos += key[j] < x;
+    out[base + pos] = (long long)(x & ((1ull << index_bits) - 1ull));
+  }
 }
 
 // the general form, any length: keys for the radix sort
@@ -337,7 +357,7 @@ int launch_randperm_dealt(char *mem, unsigned turn, long long n, unsigned long l
   unsigned int *cur = counts + (turn & 1) * RP_MAX_BUCKETS, *next = counts + ((turn + 1) & 1) * RP_MAX_BUCKETS;
   unsigned long long *buckets = (unsigned long long *)(mem + 2 * RP_MAX_BUCKETS * 4);
   randperm_deal_kernel<<<grid_for(n, 2048), 256, 0, st>>>(n, seed, bits, index_bits, buckets, cur, next, errflag);
-  randperm_sort_kernel<<<1 << bits, RP_SORT_THREADS, 0, st>>>(buckets, cur, index_bits, out);
+  randperm_sort_kernel<<<1 << bits, RP_SORT_THREADS, 0, st>>>(buckets, cur, 44 - bits + index_bits, index_bits, out);
   return 2;
 }
 
