@@ -218,22 +218,37 @@ __global__ void __launch_bounds__(32 * SB_WARPS) sub_bucket_hist(SubBucketArgs a
   for (int i = lane; i <= nb; i += 32) hist[(size_t)i * nwarps + wg] = cnt[wl][i];
 }
 
+// Eight counts per thread and round, all in flight together: the rounds are a chain of load, scan and barrier, and one count
+// per thread took five of them for 269,507 edges (9.3 us, 6.1 us now).
 __global__ void __launch_bounds__(1024) sub_bucket_scan(unsigned int *hist, int nwarps, int nb, unsigned int *totals, long long *counts) {
+  constexpr int PER = 8;
   __shared__ unsigned int part[32];
   unsigned int *row = hist + (size_t)blockIdx.x * nwarps;
   const int t = threadIdx.x, lane = t & 31, wl = t >> 5;
   unsigned int carry = 0u;
-  for (int i0 = 0; i0 < nwarps; i0 += 1024) {
-    const int i = i0 + t;
-    const unsigned int v = i < nwarps ? row[i] : 0u;
-    unsigned int incl = v;
+  for (int i0 = 0; i0 < nwarps; i0 += 1024 * PER) {
+    const int i = i0 + t * PER;
+    unsigned int v[PER], sum = 0u;
+#pragma unroll
+    for (int u = 0; u < PER; ++u) v[u] = i + u < nwarps ? row[i + u] : 0u;
+#pragma unroll
+    for (int u = 0; u < PER; ++u) sum += v[u];
+    unsigned int incl = sum;
+#pragma unroll
     for (int o = 1; o < 32; o <<= 1) { const unsigned int x = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += x; }
     if (lane == 31) part[wl] = incl;
     __syncthreads();
-    unsigned int before = carry, all = carry;
-    for (int u = 0; u < 32; ++u) { if (u < wl) before += part[u]; all += part[u]; }
-    if (i < nwarps) row[i] = before + incl - v;
-    carry = all;
+    unsigned int upto = part[lane];                           // every warp scans the 32 parts for itself
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const unsigned int x = __shfl_up_sync(0xffffffffu, upto, o); if (lane >= o) upto += x; }
+    const unsigned int lower = __shfl_sync(0xffffffffu, upto, wl > 0 ? wl - 1 : 0);
+    unsigned int at = carry + (wl > 0 ? lower : 0u) + incl - sum;
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      if (i + u < nwarps) row[i + u] = at;
+      at += v[u];
+    }
+    carry += __shfl_sync(0xffffffffu, upto, 31);
     __syncthreads();
   }
   if (t == 0) {
