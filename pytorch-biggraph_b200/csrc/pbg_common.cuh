@@ -516,7 +516,8 @@ inline long long pbg_hublist_entries(long long nocc) { return nocc / 8 + 64; }
 inline size_t pbg_bigtab_bytes(long long nocc) { return (size_t)(nocc / 256 + 2) * (PBG_KMAX + 2) * sizeof(long long); }
 // Evaluation of one batch after its scores.  out8 (host or device memory): loss, then pos_rank, mrr, r1, r10, r50 summed over
 // both sides, then the AUC hits per side.  part: 8 doubles for each of the kernel's CTAs; done: a counter, zero at first.
-inline int pbg_eval_ctas(int nblk, int Pm) { return (int)((2ll * nblk * Pm + 7) / 8); }
+inline int pbg_eval_auc_ctas(int nblk, int Pm) { return (int)((2ll * nblk * Pm + 255) / 256); }
+inline int pbg_eval_ctas(int nblk, int Pm) { return pbg_eval_auc_ctas(nblk, Pm) + (int)((2ll * nblk * Pm + 7) / 8); }
 int launch_eval(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, double *part, unsigned *done, double *out8, cudaStream_t st);
 // The evaluator's last step, by the last CTA of a kernel (256 threads): the CTAs' partial sums [ctas][8] added up in a
 // fixed order (32 runs, then the runs), the counter cleared for the next call.
@@ -525,7 +526,13 @@ __device__ __forceinline__ void close_eval(const double *part, int ctas, unsigne
   const int k = threadIdx.x & 7, y = threadIdx.x >> 3;
   double s = 0.0;
   __threadfence();
-  for (int c = y; c < ctas; c += 32) s += ((const volatile double *)part)[(size_t)c * 8 + k];
+  for (int c0 = y; c0 < ctas; c0 += 32 * 8) {                // eight reads in flight, past the L1
+    double x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = c0 + 32 * u < ctas ? __ldcg(part + (size_t)(c0 + 32 * u) * 8 + k) : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += x[u];
+  }
   run[y][k] = s;
   __syncthreads();
   if (threadIdx.x < 8) {

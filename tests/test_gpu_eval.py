@@ -114,3 +114,40 @@ def test_all_negs_relations_are_not_trained():
     t = lambda a: torch.tensor(np.asarray(a, np.int64))
     with pytest.raises(NotImplementedError, match="all_negs"):
         tr.process_one_batch(model, T.EdgeList(T.EntityList.from_tensor(t(z["lhs"])), T.EntityList.from_tensor(t(z["rhs"])), t(0)))
+
+
+@pytest.mark.parametrize("loss", ["softmax", "ranking", "logistic"])
+@pytest.mark.parametrize("B,nb,nu", [(1, 1, 3), (23, 7, 3), (130, 130, 390), (513, 513, 0), (515, 128, 2), (70, 0, 35)])
+def test_sampled_ranks_are_the_ranks_of_the_forward_scores(B, nb, nu, loss):
+    """Rows whose own column lies at every place of a group of four, chunks that end inside one, more columns than one pass of a
+    warp takes, no batch negatives: ranks and hits are counts over the scores that the forward call returns for the same
+    candidates (the same kernels, so they are equal), the loss is its formula in double precision over those scores.  The device
+    adds up to 520 terms in single precision: 520 x 2^-24 = 3.1e-5 relative, and the terms' own rounding (exp, log: a few 2^-24)."""
+    import torch
+    import torchbiggraph_b200 as T
+    g = torch.Generator().manual_seed(B + nb)
+    rows, D, margin, chunks = 900, 20, 0.1, -(-B // (nb or nu))
+    cfg = T.ConfigSchema(entities={"e": T.EntitySchema()}, relations=[T.RelationSchema("r", "e", "e", operator="none")], dimension=D,
+                         comparator="dot", loss_fn=loss, margin=margin, batch_size=chunks * (nb or nu), num_batch_negs=nb, num_uniform_negs=nu, precision="fp32")
+    m = T.make_model(cfg, "cuda")
+    W = torch.randn(rows, D, generator=g).cuda()
+    m.set_embeddings("e", T.Side.LHS, W)
+    m.set_embeddings("e", T.Side.RHS, W)
+    edges = T.EdgeList(T.EntityList.from_tensor(torch.randint(0, rows, (B,), generator=g)), T.EntityList.from_tensor(torch.randint(0, rows, (B,), generator=g)), torch.tensor(0))
+    ul, ur = (torch.randint(0, rows, (chunks, nu), generator=g).cuda() if nu else None for _ in range(2))
+    sc = m(edges, ul, ur)
+    st = T.B200RankingEvaluator(T.LOSS_FUNCTIONS.get_class(loss)(margin=margin), [1.0]).process_one_batch(m, edges, ul, ur)
+    want, value = np.zeros(4), 0.0
+    for pos, neg in ((sc.lhs_pos, sc.lhs_neg), (sc.rhs_pos, sc.rhs_neg)):
+        pos, neg = pos.double().cpu(), neg.double().cpu()
+        rk = 1 + (neg >= pos[:, None]).sum(1)
+        want += [float(rk.sum()) / 2] + [float((rk <= k).sum()) / 2 for k in (1, 10, 50)]
+        if loss == "softmax":
+            value += float((torch.logsumexp(torch.cat([pos[:, None], neg], 1), 1) - pos).sum())
+        elif loss == "ranking":
+            value += float((neg - pos[:, None] + margin).clamp(min=0).sum())
+        else:
+            sp = torch.nn.functional.softplus
+            value += float(sp(-pos).sum() + sp(neg).sum() / neg.shape[1])
+    assert [st.metrics[k] for k in ("pos_rank", "r1", "r10", "r50")] == pytest.approx(list(want), abs=1e-9)
+    assert st.metrics["loss"] == pytest.approx(value, rel=4e-5, abs=1e-5)
