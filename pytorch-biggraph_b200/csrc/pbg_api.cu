@@ -52,7 +52,7 @@ struct pbg_context {
   long long *hublist = nullptr;
   int *hubcnt = nullptr;        // two sets of counters, used in turn
   unsigned hub_turn = 0;
-  unsigned *seams = nullptr;    // words of the gradients' sibling launches
+  unsigned *seams = nullptr;    // words of the sibling launches: the gradients' (0 and 8), the full ranking's (16)
   long long *bigtab = nullptr;  // batch boundaries of the rows with 256 and more slots in a wave
   long long *edge_dev[3] = {nullptr, nullptr, nullptr};
   long long edge_cap = 0;
@@ -345,7 +345,7 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   for (int s = 0; s < 2; ++s)
     for (int i = 0; i < PBG_SORT_WAVES; ++i) { oWK[s][i] = take(list * 8); oWV[s][i] = take(list * 4); }
   size_t oSum = take(8 * sizeof(double)), oEval = take((size_t)pbg_eval_ctas(c->Cm, c->Pm) * 8 * sizeof(double)), oEvalDone = take(4);
-  size_t oPsum = take((size_t)nocc * c->Dp * 4), oHub = take(2 * (size_t)pbg_hublist_entries(nocc) * 8), oHubCnt = take(2 * HUB_SET * sizeof(int)), oSeam = take(64);
+  size_t oPsum = take((size_t)nocc * c->Dp * 4), oHub = take(2 * (size_t)pbg_hublist_entries(nocc) * 8), oHubCnt = take(2 * HUB_SET * sizeof(int)), oSeam = take(128);
   size_t oBigTab = take(2 * pbg_bigtab_bytes((long long)nocc));
   // dynamic relations with a (vector) operator: the operator-row gradient of every edge, written by the pull-back pass
   size_t oGR[2] = {0, 0};
@@ -943,7 +943,7 @@ extern "C" int pbg_eval_batch_all_negs(pbg_context *c, const pbg_bucket *bk, con
   w.seed = seed;
   const float wrel = bk->relation_weights ? bk->relation_weights[d.dynamic ? 0 : relidx] : 1.0f;
   c->launches += launch_allnegs_eval(d, w, c->allnegs_mem, c->cfg.max_batch_size, count, c->allnegs_slab, planes, d.dynamic ? 0 : relidx, wrel,
-                                   c->eval_done, c->box_dev->eval, c->stream);
+                                   c->eval_done, c->seams + 16, c->box_dev->eval, c->stream);
   CU(c, pbg_take_launch_error());
   const double *h = c->box->eval;
   rc = check_errflag(c);

@@ -554,13 +554,14 @@ struct AllNegs {
   int *pcnt[2]; float *pa[2], *pb[2];   // per (tile of the slab, edge): count, loss partials
   int *cnt[2]; float *ra[2], *rb[2];    // per-edge state over the slabs so far
   int *auc[2];                          // per edge: did its sample of the randomized AUC hit
+  unsigned *seam;                       // word of the first two kernels, siblings (pdl_begin_open)
   double *part; unsigned *done;         // per-CTA sums of the last kernel, and how many CTAs have left theirs
   int B, slab, qrows, Dpb, tiles;       // tiles: partials per edge and slab
 };
 size_t pbg_allnegs_bytes(int maxB, int D, bool planes, long long table_rows, int &slab);
 // out8: what the evaluator returns (see launch_eval), in host or device memory
 int launch_allnegs_eval(const WaveDims &d, const WaveBufs &w, char *mem, int maxB, int B, int slab, bool planes, int rel_std, float wrel,
-                        unsigned *done, double *out8, cudaStream_t st);
+                        unsigned *done, unsigned *seam, double *out8, cudaStream_t st);
 int launch_allnegs_score_tc(const WaveDims &d, const WaveBufs &w, const AllNegs &a, long long row0, cudaStream_t st);
 int launch_reg_value(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st);
 int launch_row_adagrad_sorted(float *emb, float *state, int dim, const unsigned long long *keys,

@@ -263,7 +263,7 @@ __device__ __forceinline__ void allnegs_q_planes(const AllNegs &a, int side, int
 
 template <int VEC>
 __global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_rows_kernel(WaveDims d, WaveBufs w, AllNegs a, int rel_std) {
-  pdl_begin();
+  pdl_begin_open(a.seam);
   int lane = threadIdx.x & 31;
   int e = blockIdx.x * GATHER_WARPS + (threadIdx.x >> 5);
   if (e >= a.B) return;
@@ -345,28 +345,38 @@ __device__ __forceinline__ float allnegs_candidate(float4 (&z)[VEC], const WaveD
   return prepare_row<VEC>(z, d.cmp);
 }
 
-// grid (row groups, sides): candidates row0 .. of both tables; warps past them take the AUC's samples (auc: B of them),
-// torchbiggraph/util.py:415-428: `count` random (positive, (edge, candidate)) pairs per side, hits left in cnt[side]
+// grid (row groups, sides): candidates row0 .. of both tables; `auc_ctas` CTAs of each side take the AUC's samples (B of
+// them), torchbiggraph/util.py:415-428: `count` random (positive, (edge, candidate)) pairs per side, hits left in auc[side].
+// The candidates need nothing from the edges' rows, so the first slab starts as a sibling of allnegs_rows_kernel; the samples
+// wait for it, in the middle of the grid's order (last of side 0, first of side 1), where neither the wait nor their chain of
+// reads is the end of the kernel.  (One batch of 1000 edges against 14,951 rows of 400 floats a side: 185.2 us behind the rows and with the samples last, 184.3 so.)
 template <int VEC>
-__global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_slab_kernel(WaveDims d, WaveBufs w, AllNegs a, long long row0, int rel_std, int slab_ctas, int auc) {
-  pdl_begin();
+__global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_slab_kernel(WaveDims d, WaveBufs w, AllNegs a, long long row0, int rel_std, int slab_ctas, int auc_ctas) {
   const int lane = threadIdx.x & 31, side = blockIdx.y, D = d.D;
+  const int cta = (int)blockIdx.x - (side == 1 ? auc_ctas : 0);            // candidates: 0 .. slab_ctas - 1
+  const bool samples = cta < 0 || cta >= slab_ctas;
   float4 z[VEC];
-  if (blockIdx.x < slab_ctas) {
-    const int r = blockIdx.x * GATHER_WARPS + (threadIdx.x >> 5);
-    if (r >= allnegs_rows_of(d, a, side, row0)) return;
-    const float aux = allnegs_candidate<VEC>(z, d, w, side, row0 + r, rel_std, lane);
-    if (a.YB) {
-      const size_t plane = (size_t)a.slab * a.Dpb;
-      store_planes<VEC>(a.YB + (size_t)side * 3 * plane + (size_t)r * a.Dpb, plane, z, D, lane);
-    } else {
-      store_row<VEC>(a.Y[side] + (size_t)r * d.Dp, z, D, lane);
+  if (!samples) {
+    const bool sibling = row0 == 0;                                      // (a later slab follows the merge of the one before)
+    if (!sibling) pdl_begin();
+    else { pdl_release(); seam_enter(a.seam); }
+    const int r = cta * GATHER_WARPS + (threadIdx.x >> 5);
+    if (r < allnegs_rows_of(d, a, side, row0)) {
+      const float aux = allnegs_candidate<VEC>(z, d, w, side, row0 + r, rel_std, lane);
+      if (a.YB) {
+        const size_t plane = (size_t)a.slab * a.Dpb;
+        store_planes<VEC>(a.YB + (size_t)side * 3 * plane + (size_t)r * a.Dpb, plane, z, D, lane);
+      } else {
+        store_row<VEC>(a.Y[side] + (size_t)r * d.Dp, z, D, lane);
+      }
+      if (lane == 0) a.yn[side][r] = d.cmp >= PBG_CMP_L2 ? aux : 0.f;
     }
-    if (lane == 0) a.yn[side][r] = d.cmp >= PBG_CMP_L2 ? aux : 0.f;
-    return;
+    return;                                                // (the samples' CTAs wait for the rows' end)
   }
-  const int smp = (blockIdx.x - slab_ctas) * GATHER_WARPS + (threadIdx.x >> 5);
-  if (!auc || smp >= a.B || !d.neg_enabled[side]) return;
+  pdl_begin();
+  const int smp = (cta < 0 ? (int)blockIdx.x : cta - slab_ctas) * GATHER_WARPS + (threadIdx.x >> 5);
+  if (smp == 0 && side == 0) seam_close(a.seam);
+  if (smp >= a.B || !d.neg_enabled[side]) return;
   unsigned long long h = pbg_mix64(w.seed ^ pbg_mix64(0xA11CE5ull + (unsigned long long)side * 0x10001ull + smp));
   const int ei = (int)(h % (unsigned long long)a.B);
   h = pbg_mix64(h);
@@ -505,13 +515,25 @@ __global__ void __launch_bounds__(32 * GATHER_WARPS) allnegs_merge_kernel(WaveDi
     const int per = a.slab / a.tiles, ntiles = (n + per - 1) / per;       // candidates per partial; partials that hold any
     int cnt = 0;
     float ra = 0.f, rb = -INFINITY;
-    for (int t = lane; t < ntiles; t += 32) {
-      const size_t o = (size_t)t * a.B + e;
-      cnt += a.pcnt[side][o];
-      if (d.loss == PBG_LOSS_SOFTMAX) {
-        const float m2 = a.pb[side][o], m = fmaxf(rb, m2);
-        if (m2 > -INFINITY) { ra = (rb > -INFINITY ? ra * expf(rb - m) : 0.f) + a.pa[side][o] * expf(m2 - m); rb = m; }
-      } else ra += a.pa[side][o];
+    for (int t0 = lane; t0 < ntiles; t0 += 128) {                          // four partials in flight
+      int pc[4];
+      float fa[4], fb[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const size_t o = (size_t)(t0 + 32 * u) * a.B + e;
+        const bool on = t0 + 32 * u < ntiles;
+        pc[u] = on ? a.pcnt[side][o] : 0;
+        fa[u] = on ? a.pa[side][o] : 0.f;
+        fb[u] = on && d.loss == PBG_LOSS_SOFTMAX ? a.pb[side][o] : -INFINITY;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        cnt += pc[u];
+        if (d.loss == PBG_LOSS_SOFTMAX) {
+          const float m2 = fb[u], m = fmaxf(rb, m2);
+          if (m2 > -INFINITY) { ra = (rb > -INFINITY ? ra * expf(rb - m) : 0.f) + fa[u] * expf(m2 - m); rb = m; }
+        } else ra += fa[u];
+      }
     }
     cnt = warp_sum_int(cnt);
     if (d.loss == PBG_LOSS_SOFTMAX) {
@@ -603,25 +625,26 @@ size_t pbg_allnegs_bytes(int maxB, int D, bool planes, long long table_rows, int
 
 // Runs the whole evaluation of one batch against all rows of both tables; `mem` holds pbg_allnegs_bytes bytes.
 int launch_allnegs_eval(const WaveDims &d, const WaveBufs &w, char *mem, int maxB, int B, int slab, bool planes, int rel_std, float wrel,
-                        unsigned *done, double *out8, cudaStream_t st) {
+                        unsigned *done, unsigned *seam, double *out8, cudaStream_t st) {
   AllNegs a;
   size_t bytes;
   allnegs_layout(a, mem, maxB, d.Dp, (d.D + 7) / 8 * 8, slab, planes, bytes);
-  a.B = B; a.done = done;
+  a.B = B; a.done = done; a.seam = nullptr;
   int launches = 0;
   const int vec = (d.D + 127) / 128;
   const int ectas = (B + GATHER_WARPS - 1) / GATHER_WARPS;
 #define AN_V(K, ...) do { if (vec <= 1) pbg_launch(K<1>, __VA_ARGS__); else if (vec <= 2) pbg_launch(K<2>, __VA_ARGS__); else if (vec <= 4) pbg_launch(K<4>, __VA_ARGS__); \
                             else if (vec <= 8) pbg_launch(K<8>, __VA_ARGS__); else pbg_launch(K<16>, __VA_ARGS__); } while (0)
-  AN_V(allnegs_rows_kernel, ectas, 32 * GATHER_WARPS, 0, st, d, w, a, rel_std);
-  ++launches;
   long long most = 0;
   for (int s = 0; s < 2; ++s) if (d.neg_enabled[s] && d.n_rows[s] > most) most = d.n_rows[s];
+  if (most > 0) a.seam = seam;                                // (with no candidates there is no second sibling to clear it)
+  AN_V(allnegs_rows_kernel, ectas, 32 * GATHER_WARPS, 0, st, d, w, a, rel_std);
+  ++launches;
   for (long long row0 = 0; row0 == 0 || row0 < most; row0 += slab) {
     const int n = (int)(most - row0 < slab ? most - row0 : slab);
     const int sctas = (n + GATHER_WARPS - 1) / GATHER_WARPS, first = row0 == 0, last = row0 + slab >= most;
     if (n > 0) {                                              // (neither side has negatives: no candidates, and zeros from the merge)
-      AN_V(allnegs_slab_kernel, dim3(sctas + (first ? ectas : 0), 2), 32 * GATHER_WARPS, 0, st, d, w, a, row0, rel_std, sctas, first);
+      AN_V(allnegs_slab_kernel, dim3(sctas + (first ? ectas : 0), 2), 32 * GATHER_WARPS, 0, st, d, w, a, row0, rel_std, sctas, first ? ectas : 0);
       if (planes) launch_allnegs_score_tc(d, w, a, row0, st);
       else pbg_launch(allnegs_score_kernel, dim3((B + AN_TILE - 1) / AN_TILE, (n + AN_TILE - 1) / AN_TILE, 2), 256, 0, st, d, w, a, row0);
       launches += 2;
