@@ -32,7 +32,7 @@ struct pbg_context {
   cudaStream_t side = nullptr;      // sorts of the waves to come
   cudaStream_t part2 = nullptr;     // second half of a wave's gather / score / loss / gradient kernels
   cudaEvent_t ev_wave = nullptr, ev_part2 = nullptr;
-  cudaEvent_t ev_sorted[2] = {nullptr, nullptr}, ev_updated[2] = {nullptr, nullptr}, ev_inputs = nullptr;
+  cudaEvent_t ev_sorted[2] = {nullptr, nullptr}, ev_sort = nullptr, ev_inputs = nullptr;
   // What a call reads back lies in pinned host memory that the kernels write themselves: the error word (written only
   // when something is wrong), the evaluator's sums, a batch's Stats.  Reading it costs the call's one synchronisation
   // and no copy (two pageable copies of a few bytes were 20 us of a 150 us call).
@@ -398,11 +398,11 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
       c->wvals[s][i] = (unsigned int *)(c->ws + oWV[s][i]);
     }
     CU(c, cudaEventCreateWithFlags(&c->ev_sorted[s], cudaEventDisableTiming));
-    CU(c, cudaEventCreateWithFlags(&c->ev_updated[s], cudaEventDisableTiming));
   }
   CU(c, cudaEventCreateWithFlags(&c->ev_inputs, cudaEventDisableTiming));
   CU(c, cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
   CU(c, cudaStreamCreateWithFlags(&c->part2, cudaStreamNonBlocking));
+  CU(c, cudaEventCreateWithFlags(&c->ev_sort, cudaEventDisableTiming));
   CU(c, cudaEventCreateWithFlags(&c->ev_wave, cudaEventDisableTiming));
   CU(c, cudaEventCreateWithFlags(&c->ev_part2, cudaEventDisableTiming));
   CU(c, cudaHostAlloc((void **)&c->box, sizeof *c->box, cudaHostAllocMapped | cudaHostAllocPortable));
@@ -452,11 +452,11 @@ extern "C" int pbg_destroy(pbg_context *c) {
   if (c->etab_dev) cudaFree(c->etab_dev);
   for (int s = 0; s < 2; ++s) {
     if (c->ev_sorted[s]) cudaEventDestroy(c->ev_sorted[s]);
-    if (c->ev_updated[s]) cudaEventDestroy(c->ev_updated[s]);
   }
   if (c->ev_inputs) cudaEventDestroy(c->ev_inputs);
   if (c->side) cudaStreamDestroy(c->side);
   if (c->part2) cudaStreamDestroy(c->part2);
+  if (c->ev_sort) cudaEventDestroy(c->ev_sort);
   if (c->ev_wave) cudaEventDestroy(c->ev_wave);
   if (c->ev_part2) cudaEventDestroy(c->ev_part2);
   for (auto &s : c->spans) { cudaEventDestroy(s.a); cudaEventDestroy(s.b); }
@@ -690,17 +690,26 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
   }
   // Waves are sorted PBG_SORT_WAVES at a time by one kernel, a cluster per wave, one group ahead of the group that
   // trains: few launches, and the sort of the next group has a whole group's training to hide behind.  The call's
-  // first group is one wave, so that its update waits for the shortest sort there is.  Waves beyond what a cluster
-  // holds are sorted one by one, one wave ahead.
+  // first group is one wave, so that its update waits for the shortest sort there is.  On the fused path the sort starts behind
+  // the gradients of a group's first wave: up to four clusters of sixteen CTAs beside its tiles, hub rows and the next gather,
+  // which leave room on their SMs.  Started with that wave, the sort's last CTAs held 64 SMs in front of a score kernel of one
+  // CTA per SM in one round (plumbing graph: 48 us in every fourth wave, 27 in the others; the bucket 8,061 -> 7,682 us, a follower
+  // graph's 2,814 -> 2,763).  Otherwise it starts with the wave: the separate kernels' contractions take several rounds beside
+  // memory-bound halves, and waves of chunk_kernel leave SMs free (the late start changed them by less than 0.5 %).  Waves beyond
+  // what a cluster holds are sorted one by one, one wave ahead.
   const bool cluster = c->cluster_sort && pbg_cluster_sort_fits((long long)(kbase + (kextra ? 1 : 0)) * d.spb, bits);
   const int gsize = cluster ? PBG_SORT_WAVES : 1;
+  const bool sort_late = cluster && c->fused && !c->chunk;
   if (!cluster && nwaves > 1) { rc = second_sort(c); if (rc) return rc; }
   auto group_of = [&](int wv) { return wv == 0 ? 0 : 1 + (wv - 1) / gsize; };
   auto group_first = [&](int g) { return g == 0 ? 0 : 1 + (g - 1) * gsize; };
   const int ngroups = group_of(nwaves - 1) + 1;
   auto sort_group = [&](int g) -> int {                       // into buffer half g & 1
     if (g >= ngroups) return PBG_OK;
-    if (g >= 2) CU(c, cudaStreamWaitEvent(c->side, c->ev_updated[g & 1], 0));   // group g - 2 has been applied
+    if (g >= 2) {                                             // group g - 2, whose buffer half this is, has been applied
+      if (sort_late) CU(c, cudaEventRecord(c->ev_sort, c->stream));
+      CU(c, cudaStreamWaitEvent(c->side, c->ev_sort, 0));
+    }
     const int w0 = group_first(g), w1 = g + 1 < ngroups ? group_first(g + 1) : nwaves;
     ClassTimer t(c, 0, c->side);
     if (cluster) {
@@ -725,6 +734,7 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
     const WaveBatches &wb = wbs[wave];
     d.k = kk; d.nblk = kk * d.Cm; d.nocc = kk * d.spb;
     const int grp = group_of(wave), in_grp = wave - group_first(grp);
+    if (!sort_late && in_grp == 0) CU(c, cudaEventRecord(c->ev_sort, c->stream));
     // The batches of a wave all read the tables as the wave found them, so its forward / backward
     // kernels can run as two independent halves on two streams: the memory-bound kernels of one
     // half fill the SMs' idle issue slots while the other half's contractions run.
@@ -765,8 +775,6 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
       const unsigned int *wvals = cluster ? c->wvals[grp & 1][in_grp] : sp.vals[sp.result];
       t.done(launch_update(d, wb, w, wkeys, wvals, c->cfg.lr, c->cfg.relation_lr, us, c->stream));
     }
-    // (the next call's sorts come behind everything of this one)
-    if (grp + 2 < ngroups && group_of(wave + 1) != grp) CU(c, cudaEventRecord(c->ev_updated[grp & 1], c->stream));
     b0 += kk;
   }
   c->batches_done += (unsigned long long)num_batches;
