@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(32 * GATHER_WARPS, GatherCtas<VEC>::GENERAL) g
 // comparator: the operand rows are plain copies of the table rows, and the positive score is their
 // dot product.  Both rows of a slot (lhs side, rhs side) are loaded at once, which doubles the bytes
 // a warp keeps in flight, and the kernel carries none of the operator / prepare code of the general
-// one (half the registers, three CTAs per SM instead of two).
+// one.
 template <int VEC, bool PL>
 __global__ void __launch_bounds__(32 * GATHER_WARPS, GatherCtas<VEC>::PLAIN) gather_plain_kernel(WaveDims d, WaveBatches wb, WaveBufs w) {
   pdl_begin();
