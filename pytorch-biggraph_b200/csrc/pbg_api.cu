@@ -53,6 +53,8 @@ struct pbg_context {
   int *hubcnt = nullptr;        // two sets of counters, used in turn
   unsigned hub_turn = 0;
   unsigned *seams = nullptr;    // words of the sibling launches: the gradients' (0 and 8), the full ranking's (16)
+  char *zeros = nullptr;        // the words and counters that a call finds at zero and leaves at zero (end_launches)
+  size_t zero_bytes = 0;
   long long *bigtab = nullptr;  // batch boundaries of the rows with 256 and more slots in a wave
   long long *edge_dev[3] = {nullptr, nullptr, nullptr};
   long long edge_cap = 0;
@@ -344,9 +346,10 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   size_t oWK[2][PBG_SORT_WAVES], oWV[2][PBG_SORT_WAVES];
   for (int s = 0; s < 2; ++s)
     for (int i = 0; i < PBG_SORT_WAVES; ++i) { oWK[s][i] = take(list * 8); oWV[s][i] = take(list * 4); }
-  size_t oSum = take(8 * sizeof(double)), oEval = take((size_t)pbg_eval_ctas(c->Cm, c->Pm) * 8 * sizeof(double)), oEvalDone = take(4);
-  size_t oPsum = take((size_t)nocc * c->Dp * 4), oHub = take(2 * (size_t)pbg_hublist_entries(nocc) * 8), oHubCnt = take(2 * HUB_SET * sizeof(int)), oSeam = take(128);
-  size_t oBigTab = take(2 * pbg_bigtab_bytes((long long)nocc));
+  size_t oSum = take(8 * sizeof(double)), oEval = take((size_t)pbg_eval_ctas(c->Cm, c->Pm) * 8 * sizeof(double));
+  size_t oPsum = take((size_t)nocc * c->Dp * 4), oHub = take(2 * (size_t)pbg_hublist_entries(nocc) * 8);
+  const size_t oZero = off, oEvalDone = take(4), oHubCnt = take(2 * HUB_SET * sizeof(int)), oSeam = take(128), oBigTab = take(2 * pbg_bigtab_bytes((long long)nocc));
+  c->zero_bytes = off - oZero;
   // dynamic relations with a (vector) operator: the operator-row gradient of every edge, written by the pull-back pass
   size_t oGR[2] = {0, 0};
   const bool keep_gr = dyn && cfg->op != PBG_OP_NONE && !matrix_op;
@@ -418,6 +421,7 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
   c->hubcnt = (int *)(c->ws + oHubCnt);
   c->bigtab = (long long *)(c->ws + oBigTab);
   c->seams = (unsigned *)(c->ws + oSeam);
+  c->zeros = c->ws + oZero;
   if (cfg->precision != PBG_PREC_FP32) {
     WaveDims gd;
     memset(&gd, 0, sizeof gd);
@@ -548,6 +552,30 @@ static int check_errflag(pbg_context *c) {
   return PBG_OK;
 }
 
+// Start of an entry point that launches: an earlier call's failure on this thread is not this call's.
+#define BEGIN_LAUNCHES(c)                     \
+  do {                                        \
+    CU(c, cudaSetDevice((c)->device));        \
+    pbg_launch_error() = cudaSuccess;         \
+  } while (0)
+
+// End of an entry point's launches.  rc: what went wrong between them, if anything.  The kernels of a call find the words
+// of the sibling launches and their counters at zero and leave them so, the whole sequence of them: where one has not been
+// launched (nor has anything behind it) a word may stay set, and the next call's second sibling would read what its first has
+// not waited for.  A failed call therefore clears them all, and the ids its kernels complained of.
+static int end_launches(pbg_context *c, int rc = PBG_OK) {
+  const cudaError_t e = pbg_take_launch_error();
+  if (rc == PBG_OK && e == cudaSuccess) return PBG_OK;
+  if (rc == PBG_OK) rc = fail(c, PBG_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
+  cudaStreamSynchronize(c->side);                             // (nothing may still read the caller's arrays)
+  cudaStreamSynchronize(c->part2);
+  cudaMemsetAsync(c->zeros, 0, c->zero_bytes, c->stream);
+  if (c->rp_mem) cudaMemsetAsync(c->rp_mem, 0, pbg_randperm_counter_bytes(), c->stream);
+  cudaStreamSynchronize(c->stream);
+  c->box->err = 0;
+  return rc;
+}
+
 static int run_forward(pbg_context *c, const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st) {
   {
     ClassTimer t(c, 1, st);
@@ -622,6 +650,9 @@ static int second_sort(pbg_context *c) {
   return PBG_OK;
 }
 
+static int train_waves(pbg_context *c, const pbg_bucket *bk, WaveDims &d, const WaveBufs &w, const pbg_batch *batches, int num_batches,
+                       bool want_stats);
+
 extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int64_t *lhs, const int64_t *rhs,
                                  const int64_t *rel, int64_t num_edges, const pbg_batch *batches,
                                  int32_t num_batches, const int64_t *ul, const int64_t *ur, uint64_t seed,
@@ -630,7 +661,7 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
   const float *ew = take_edge_weights(c);
   if (num_batches == 0) return PBG_OK;
   if (!lhs || !rhs || !batches || num_batches < 0 || num_edges < 0) return fail(c, PBG_ERR_BAD_ARGUMENT, "null edge arrays or batch list");
-  CU(c, cudaSetDevice(c->device));
+  BEGIN_LAUNCHES(c);
   WaveDims d;
   WaveBufs w;
   int rc = bind_bucket(c, bk, d, w);
@@ -662,6 +693,17 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
     CU(c, cudaHostGetDevicePointer((void **)&c->stats_dev, c->stats_host, 0));
     c->stats_cap = cap;
   }
+  rc = end_launches(c, train_waves(c, bk, d, w, batches, num_batches, stats_out != nullptr));
+  if (rc || !stats_out) return rc;
+  rc = check_errflag(c);
+  memcpy(stats_out, c->stats_host, (size_t)num_batches * sizeof(pbg_batch_stats));
+  return rc;
+}
+
+// the kernels of a call's waves
+static int train_waves(pbg_context *c, const pbg_bucket *bk, WaveDims &d, const WaveBufs &w, const pbg_batch *batches, int num_batches,
+                       bool want_stats) {
+  int rc = PBG_OK;
   const int bits = bit_length(d.key_invalid);
   // The sort keys depend on the edge and negative ids only, never on the tables: the key build
   // and radix sort of a wave run on the side stream and overlap the previous wave's kernels.
@@ -727,7 +769,7 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
     CU(c, cudaEventRecord(c->ev_sorted[g & 1], c->side));
     return PBG_OK;
   };
-  UpdateScratch us{c->psum, c->hublist, c->hubcnt, &c->hub_turn, c->bigtab, stats_out ? c->stats_dev : nullptr, c->sum_dev};
+  UpdateScratch us{c->psum, c->hublist, c->hubcnt, &c->hub_turn, c->bigtab, want_stats ? c->stats_dev : nullptr, c->sum_dev};
   int wave = 0;
   for (int b0 = 0; b0 < num_batches; ++wave) {
     const int kk = kks[wave];
@@ -778,16 +820,6 @@ extern "C" int pbg_train_batches(pbg_context *c, const pbg_bucket *bk, const int
     b0 += kk;
   }
   c->batches_done += (unsigned long long)num_batches;
-  if (const cudaError_t e = pbg_take_launch_error()) {
-    cudaMemsetAsync(c->seams, 0, 64, c->stream);             // (the first of two siblings may be without its second)
-    cudaMemsetAsync(c->hubcnt, 0, 2 * HUB_SET * sizeof(int), c->stream);
-    return fail(c, PBG_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
-  }
-  if (stats_out) {
-    rc = check_errflag(c);
-    memcpy(stats_out, c->stats_host, (size_t)num_batches * sizeof(pbg_batch_stats));
-    return rc;
-  }
   return PBG_OK;
 }
 
@@ -858,7 +890,7 @@ extern "C" int pbg_score_batch(pbg_context *c, const pbg_bucket *bk, const int64
   if (count == 0) return PBG_OK;
   if (!lhs || !rhs || !lhs_pos || !rhs_pos || count < 0 || count > c->cfg.max_batch_size)
     return fail(c, PBG_ERR_BAD_ARGUMENT, "bad score_batch arguments (count %d, max_batch_size %d)", count, c->cfg.max_batch_size);
-  CU(c, cudaSetDevice(c->device));
+  BEGIN_LAUNCHES(c);
   WaveDims d;
   WaveBufs w;
   int rc = bind_bucket(c, bk, d, w);
@@ -878,8 +910,8 @@ extern "C" int pbg_score_batch(pbg_context *c, const pbg_bucket *bk, const int64
     run_forward(c, d, wb, w, c->stream);
     c->launches += launch_export_scores(d, wb, w, lhs_pos, rhs_pos, lhs_neg, rhs_neg, c->stream);
   }
-  CU(c, pbg_take_launch_error());
-  return check_errflag(c);
+  rc = end_launches(c);
+  return rc ? rc : check_errflag(c);
 }
 
 extern "C" int pbg_eval_batch(pbg_context *c, const pbg_bucket *bk, const int64_t *lhs, const int64_t *rhs,
@@ -892,7 +924,7 @@ extern "C" int pbg_eval_batch(pbg_context *c, const pbg_bucket *bk, const int64_
   if (count == 0) return PBG_OK;
   if (!lhs || !rhs || count < 0 || count > c->cfg.max_batch_size)
     return fail(c, PBG_ERR_BAD_ARGUMENT, "bad eval_batch arguments (count %d, max_batch_size %d)", count, c->cfg.max_batch_size);
-  CU(c, cudaSetDevice(c->device));
+  BEGIN_LAUNCHES(c);
   WaveDims d;
   WaveBufs w;
   int rc = bind_bucket(c, bk, d, w);
@@ -909,7 +941,7 @@ extern "C" int pbg_eval_batch(pbg_context *c, const pbg_bucket *bk, const int64_
   d.k = 1; d.nblk = d.Cm; d.nocc = d.spb; d.blk0 = 0;
   run_forward(c, d, wb, w, c->stream);
   c->launches += launch_eval(d, wb, w, c->eval_part, c->eval_done, c->box_dev->eval, c->stream);
-  CU(c, pbg_take_launch_error());
+  if ((rc = end_launches(c))) return rc;
   const double *h = c->box->eval;
   rc = check_errflag(c);
   int sides = (d.neg_enabled[0] ? 1 : 0) + (d.neg_enabled[1] ? 1 : 0);
@@ -931,7 +963,7 @@ extern "C" int pbg_eval_batch_all_negs(pbg_context *c, const pbg_bucket *bk, con
   if (count == 0) return PBG_OK;
   if (!lhs || !rhs || count < 0 || count > c->cfg.max_batch_size)
     return fail(c, PBG_ERR_BAD_ARGUMENT, "bad eval_batch_all_negs arguments (count %d, max_batch_size %d)", count, c->cfg.max_batch_size);
-  CU(c, cudaSetDevice(c->device));
+  BEGIN_LAUNCHES(c);
   WaveDims d;
   WaveBufs w;
   int rc = bind_bucket(c, bk, d, w);
@@ -952,7 +984,7 @@ extern "C" int pbg_eval_batch_all_negs(pbg_context *c, const pbg_bucket *bk, con
   const float wrel = bk->relation_weights ? bk->relation_weights[d.dynamic ? 0 : relidx] : 1.0f;
   c->launches += launch_allnegs_eval(d, w, c->allnegs_mem, c->cfg.max_batch_size, count, c->allnegs_slab, planes, d.dynamic ? 0 : relidx, wrel,
                                    c->eval_done, c->seams + 16, c->box_dev->eval, c->stream);
-  CU(c, pbg_take_launch_error());
+  if ((rc = end_launches(c))) return rc;
   const double *h = c->box->eval;
   rc = check_errflag(c);
   int sides = (d.neg_enabled[0] ? 1 : 0) + (d.neg_enabled[1] ? 1 : 0);
@@ -971,7 +1003,7 @@ extern "C" int pbg_row_adagrad(pbg_context *c, float *emb, float *state, int64_t
   if (!emb || !state || !rows || !grads || n < 0 || num_rows <= 0) return fail(c, PBG_ERR_BAD_ARGUMENT, "bad row_adagrad arguments");
   SortPlan &sp = c->sort[0];
   if (n > sp.max_n) return fail(c, PBG_ERR_TOO_LARGE, "%d gradient rows exceed this context's sort capacity %d", n, sp.max_n);
-  CU(c, cudaSetDevice(c->device));
+  BEGIN_LAUNCHES(c);
   const int bits = bit_length((unsigned long long)num_rows);
   if (c->cluster_sort && pbg_cluster_sort_fits(n, bits)) {
     sp.result = 0;
@@ -982,8 +1014,8 @@ extern "C" int pbg_row_adagrad(pbg_context *c, float *emb, float *state, int64_t
   }
   c->launches += launch_row_adagrad_sorted(emb, state, c->cfg.dim, sp.keys[sp.result], sp.vals[sp.result],
                                            grads, n, lr, (unsigned long long)num_rows, c->stream);
-  CU(c, pbg_take_launch_error());
-  return check_errflag(c);
+  int rc = end_launches(c);
+  return rc ? rc : check_errflag(c);
 }
 
 // ---- edge-list utilities (torchbiggraph/util.cpp) -------------------------------------------------
@@ -1013,20 +1045,20 @@ extern "C" int pbg_reverse_permutation(pbg_context *c, const int64_t *perm, int6
   if (!c) return PBG_ERR_BAD_ARGUMENT;
   if (n == 0) return PBG_OK;
   if (!perm || !out || n < 0) return fail(c, PBG_ERR_BAD_ARGUMENT, "bad reverse_permutation arguments");
-  CU(c, cudaSetDevice(c->device));
+  BEGIN_LAUNCHES(c);
   c->launches += launch_reverse_permutation((const long long *)perm, n, (long long *)out, c->errflag, c->stream);
-  CU(c, pbg_take_launch_error());
-  return check_errflag_edges(c, "reverse_permutation");
+  const int rc = end_launches(c);
+  return rc ? rc : check_errflag_edges(c, "reverse_permutation");
 }
 
 extern "C" int pbg_shuffle_rows(pbg_context *c, const void *in, void *out, int64_t rows, int64_t row_bytes, const int64_t *perm) {
   if (!c) return PBG_ERR_BAD_ARGUMENT;
   if (rows == 0 || row_bytes == 0) return PBG_OK;
   if (!in || !out || !perm || rows < 0 || row_bytes < 0 || in == out) return fail(c, PBG_ERR_BAD_ARGUMENT, "bad shuffle arguments (in and out must be different buffers)");
-  CU(c, cudaSetDevice(c->device));
+  BEGIN_LAUNCHES(c);
   c->launches += launch_shuffle_rows(in, out, rows, row_bytes, (const long long *)perm, c->errflag, c->stream);
-  CU(c, pbg_take_launch_error());
-  int rc = check_errflag_edges(c, "shuffle");
+  int rc = end_launches(c);
+  if (rc == PBG_OK) rc = check_errflag_edges(c, "shuffle");
   if (rc == PBG_ERR_INDEX_RANGE) c->err = "Permutation has out-of-bound values";      // util.cpp:200-202
   return rc;
 }
@@ -1035,7 +1067,7 @@ extern "C" int pbg_randperm(pbg_context *c, int64_t n, uint64_t seed, int64_t *o
   if (!c) return PBG_ERR_BAD_ARGUMENT;
   if (n == 0) return PBG_OK;
   if (!out || n < 0) return fail(c, PBG_ERR_BAD_ARGUMENT, "bad randperm arguments");
-  CU(c, cudaSetDevice(c->device));
+  BEGIN_LAUNCHES(c);
   const size_t need = pbg_randperm_bytes(n);
   if (need) {
     if (need > c->rp_bytes) {
@@ -1045,14 +1077,14 @@ extern "C" int pbg_randperm(pbg_context *c, int64_t n, uint64_t seed, int64_t *o
       c->rp_bytes = need;
     }
     c->launches += launch_randperm_dealt(c->rp_mem, c->rp_turn++, n, seed, (long long *)out, c->errflag, c->stream);
-    CU(c, pbg_take_launch_error());
-    int flag = 0, rcf = wait_for_flag(c, flag);
+    int flag = 0, rcf = end_launches(c);
+    if (rcf == PBG_OK) rcf = wait_for_flag(c, flag);
     if (rcf || !(flag & 256)) return rcf;                    // 256: a bucket overflowed; the general sort below
   }
   int rc = ensure_edge_sort(c, n);
   if (rc) return rc;
   c->launches += launch_randperm(c->esort, n, seed, (long long *)out, c->stream);
-  CU(c, pbg_take_launch_error());
+  if ((rc = end_launches(c))) return rc;
   CU(c, cudaStreamSynchronize(c->stream));
   return PBG_OK;
 }
@@ -1069,7 +1101,7 @@ extern "C" int pbg_sub_bucket(pbg_context *c, const int64_t *lhs_in, const int64
   if (nl <= 0 || nr <= 0 || nl > 127 || nr > 127) return fail(c, PBG_ERR_BAD_ARGUMENT, "sub-partition counts must be in [1, 127] (int8 in the reference)");
   if (num_edges < 0 || (num_edges > 0 && (!lhs_in || !rhs_in || !rel_in || !lhs_out || !rhs_out || !rel_out)))
     return fail(c, PBG_ERR_BAD_ARGUMENT, "null edge arrays");
-  CU(c, cudaSetDevice(c->device));
+  BEGIN_LAUNCHES(c);
   int rc = ensure_edge_sort(c, num_edges);
   if (rc) return rc;
   const long long need = 6ll * R, nb = (long long)nl * nr;
@@ -1106,7 +1138,7 @@ extern "C" int pbg_sub_bucket(pbg_context *c, const int64_t *lhs_in, const int64
   c->launches += launch_sub_bucket(c->esort, (const long long *)lhs_in, (const long long *)rhs_in, (const long long *)rel_in, num_edges, R, tab.data(),
                                    c->etab_dev, nl, nr, dynamic_relations != 0, (long long *)lhs_out, (long long *)rhs_out,
                                    (long long *)rel_out, c->counts_dev, c->errflag, c->stream);
-  CU(c, pbg_take_launch_error());
+  if ((rc = end_launches(c))) return rc;
   const int rcs = check_errflag_edges(c, "sub_bucket");
   if (num_edges == 0) memset(c->counts_host, 0, (size_t)nb * sizeof(long long));
   memcpy(sub_bucket_counts, c->counts_host, (size_t)nb * sizeof(long long));

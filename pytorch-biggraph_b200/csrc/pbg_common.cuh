@@ -374,6 +374,9 @@ inline cudaError_t &pbg_launch_error() {
 inline void pbg_note_launch(cudaError_t e = cudaGetLastError()) {
   if (e != cudaSuccess && pbg_launch_error() == cudaSuccess) pbg_launch_error() = e;
 }
+// Nothing is launched behind a launch that failed: the kernels of a call take what the ones before them left (sorted keys,
+// counts, sums) for places in memory, and would find another call's there.
+inline bool pbg_launch_failed() { return pbg_launch_error() != cudaSuccess; }
 inline cudaError_t pbg_take_launch_error() {
   cudaError_t e = pbg_launch_error();
   pbg_launch_error() = cudaSuccess;
@@ -418,6 +421,7 @@ inline int pbg_sm_count() {
 // Launches a kernel that begins with pdl_begin().
 template <class... P, class... A>
 inline void pbg_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+  if (pbg_launch_failed()) return;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute at;
@@ -427,9 +431,19 @@ inline void pbg_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
   pbg_note_launch(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
 }
 
-// The same for a kernel of clusters of `ctas` CTAs.
+// A kernel that waits for the whole launch before it, as CUDA's stream order has it.
+template <class... P, class... A>
+inline void pbg_launch_in_order(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+  if (pbg_launch_failed()) return;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  pbg_note_launch(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
+// The same as pbg_launch for a kernel of clusters of `ctas` CTAs.
 template <class... P, class... A>
 inline void pbg_launch_clusters(void (*kernel)(P...), int clusters, int ctas, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+  if (pbg_launch_failed()) return;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(clusters * ctas)); cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute at[2];
@@ -470,7 +484,7 @@ int launch_sort_rows(const long long *rows, long long num_rows, int n, int bits,
 int launch_build_keys(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w,
                       unsigned long long *keys, unsigned int *vals, cudaStream_t st);
 int launch_gather(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, cudaStream_t st);
-// seams: 16 words of device memory, zero, for the sibling launches of the gradients
+// seams: words 0 and 8 are those of the gradients' sibling launches (a wave's first and second part); zero between calls
 void *pbg_tc_plan_create(const WaveDims &d, const WaveBufs &w, int nblk_max, int precision, unsigned *seams);
 void pbg_tc_plan_destroy(void *plan);
 // standard relations, plane tiers: score contraction of both problems + loss + coefficient planes in one kernel
@@ -571,6 +585,7 @@ int launch_reverse_permutation(const long long *perm, long long n, long long *ou
 int launch_shuffle_rows(const void *in, void *out, long long rows, long long row_bytes, const long long *perm, int *errflag, cudaStream_t st);
 int launch_randperm(SortPlan &sp, long long n, unsigned long long seed, long long *out, cudaStream_t st);
 size_t pbg_randperm_bytes(long long n);
+size_t pbg_randperm_counter_bytes();     // of it, at its start: the counters
 int launch_randperm_dealt(char *mem, unsigned turn, long long n, unsigned long long seed, long long *out, int *errflag, cudaStream_t st);
 bool pbg_sub_bucket_inline(int R);
 int launch_sub_bucket(SortPlan &sp, const long long *lhs, const long long *rhs, const long long *rel, long long n, int R, const long long *tables,

@@ -339,7 +339,7 @@ __global__ void sub_bucket_counts_kernel(const unsigned long long *__restrict__ 
 static inline int grid_for(long long n, int threads) { return (int)((n + threads - 1) / threads); }
 
 int launch_reverse_permutation(const long long *perm, long long n, long long *out, int *errflag, cudaStream_t st) {
-  if (n > 0) reverse_permutation_kernel<<<grid_for(n, 256), 256, 0, st>>>(perm, n, out, errflag);
+  if (n > 0) pbg_launch_in_order(reverse_permutation_kernel, grid_for(n, 256), 256, 0, st, perm, n, out, errflag);
   return n > 0;
 }
 
@@ -348,7 +348,7 @@ static void shuffle_as(const void *in, void *out, long long rows, long long row_
   const int units = (int)(row_bytes / (long long)sizeof(T));
   int G = 1;
   while (G < 256 && 4 * G < units) G *= 2;
-  shuffle_rows_kernel<T><<<grid_for(rows, 256 / G), 256, 0, st>>>((const T *)in, (T *)out, rows, units, G, perm, errflag);
+  pbg_launch_in_order(shuffle_rows_kernel<T>, grid_for(rows, 256 / G), 256, 0, st, (const T *)in, (T *)out, rows, units, G, perm, errflag);
 }
 
 int launch_shuffle_rows(const void *in, void *out, long long rows, long long row_bytes, const long long *perm, int *errflag, cudaStream_t st) {
@@ -364,23 +364,24 @@ int launch_shuffle_rows(const void *in, void *out, long long rows, long long row
 // scratch of the two-kernel randperm (0: n is too large for it): counters, which start at zero, then the buckets
 size_t pbg_randperm_bytes(long long n) {
   if (n > RP_MAX) return 0;
-  return 2 * RP_MAX_BUCKETS * 4 + ((size_t)RP_CAP * 8 << rp_bits(n));
+  return pbg_randperm_counter_bytes() + ((size_t)RP_CAP * 8 << rp_bits(n));
 }
+size_t pbg_randperm_counter_bytes() { return 2 * RP_MAX_BUCKETS * sizeof(unsigned int); }
 int launch_randperm_dealt(char *mem, unsigned turn, long long n, unsigned long long seed, long long *out, int *errflag, cudaStream_t st) {
   const int bits = rp_bits(n), index_bits = rp_index_bits(n);
   unsigned int *counts = (unsigned int *)mem;
   unsigned int *cur = counts + (turn & 1) * RP_MAX_BUCKETS, *next = counts + ((turn + 1) & 1) * RP_MAX_BUCKETS;
-  unsigned long long *buckets = (unsigned long long *)(mem + 2 * RP_MAX_BUCKETS * 4);
-  randperm_deal_kernel<<<grid_for(n, 2048), 256, 0, st>>>(n, seed, bits, index_bits, buckets, cur, next, errflag);
-  randperm_sort_kernel<<<1 << bits, RP_SORT_THREADS, 0, st>>>(buckets, cur, 44 - bits + index_bits, index_bits, out);
+  unsigned long long *buckets = (unsigned long long *)(mem + pbg_randperm_counter_bytes());
+  pbg_launch_in_order(randperm_deal_kernel, grid_for(n, 2048), 256, 0, st, n, seed, bits, index_bits, buckets, cur, next, errflag);
+  pbg_launch_in_order(randperm_sort_kernel, 1 << bits, RP_SORT_THREADS, 0, st, buckets, cur, 44 - bits + index_bits, index_bits, out);
   return 2;
 }
 
 int launch_randperm(SortPlan &sp, long long n, unsigned long long seed, long long *out, cudaStream_t st) {
   if (n <= 0) return 0;
-  randperm_keys_kernel<<<grid_for(n, 256), 256, 0, st>>>(n, seed, sp.keys[0], sp.vals[0]);
+  pbg_launch_in_order(randperm_keys_kernel, grid_for(n, 256), 256, 0, st, n, seed, sp.keys[0], sp.vals[0]);
   int launches = 1 + pbg_sort(sp, (int)n, 44, st);
-  widen_kernel<<<grid_for(n, 256), 256, 0, st>>>(sp.vals[sp.result], n, out);
+  pbg_launch_in_order(widen_kernel, grid_for(n, 256), 256, 0, st, sp.vals[sp.result], n, out);
   return launches + 1;
 }
 
@@ -403,16 +404,16 @@ int launch_sub_bucket(SortPlan &sp, const long long *lhs, const long long *rhs, 
     const int run = sb_run(nb), nwarps = (int)((n + run - 1) / run), ctas = (nwarps + SB_WARPS - 1) / SB_WARPS;
     unsigned short *keys = (unsigned short *)sp.keys[0];
     unsigned int *totals = sp.hist + (size_t)(nb + 1) * nwarps;
-    sub_bucket_hist<<<ctas, 32 * SB_WARPS, 0, st>>>(a, in, inl ? nullptr : tables_dev, keys, sp.hist, nwarps, run, errflag);
-    sub_bucket_scan<<<nb + 1, 1024, 0, st>>>(sp.hist, nwarps, nb, totals, counts);
-    sub_bucket_scatter<<<ctas, 32 * SB_WARPS, 0, st>>>(a, in, inl ? nullptr : tables_dev, keys, sp.hist, totals, nwarps, run, lhs_out, rhs_out, rel_out, errflag);
+    pbg_launch_in_order(sub_bucket_hist, ctas, 32 * SB_WARPS, 0, st, a, in, inl ? nullptr : tables_dev, keys, sp.hist, nwarps, run, errflag);
+    pbg_launch_in_order(sub_bucket_scan, nb + 1, 1024, 0, st, sp.hist, nwarps, nb, totals, counts);
+    pbg_launch_in_order(sub_bucket_scatter, ctas, 32 * SB_WARPS, 0, st, a, in, inl ? nullptr : tables_dev, keys, sp.hist, totals, nwarps, run, lhs_out, rhs_out, rel_out, errflag);
     return 3;
   }
-  sub_bucket_keys_kernel<<<grid_for(n, 256), 256, 0, st>>>(a, sp.keys[0], sp.vals[0], errflag);
+  pbg_launch_in_order(sub_bucket_keys_kernel, grid_for(n, 256), 256, 0, st, a, sp.keys[0], sp.vals[0], errflag);
   int bits = 1;
   while ((1ll << bits) <= nb) ++bits;                                   // keys run up to nb (the "cannot be placed" key)
   int launches = 1 + pbg_sort(sp, (int)n, bits, st);
-  sub_bucket_emit_kernel<<<grid_for(n, 256), 256, 0, st>>>(a, sp.keys[sp.result], sp.vals[sp.result], lhs_out, rhs_out, rel_out, errflag);
-  sub_bucket_counts_kernel<<<grid_for(nb, 128), 128, 0, st>>>(sp.keys[sp.result], n, nb, counts);
+  pbg_launch_in_order(sub_bucket_emit_kernel, grid_for(n, 256), 256, 0, st, a, sp.keys[sp.result], sp.vals[sp.result], lhs_out, rhs_out, rel_out, errflag);
+  pbg_launch_in_order(sub_bucket_counts_kernel, grid_for(nb, 128), 128, 0, st, sp.keys[sp.result], n, nb, counts);
   return launches + 2;
 }

@@ -63,6 +63,7 @@ extern "C" int pbg_row_adagrad_static(float *emb, float *state, int64_t num_rows
   sp.max_n = NOALLOC_MAX_ROWS;
   sp.result = 0;
   int *errflag = (int *)(base + 2 * NA_KEYS_BYTES + 2 * NA_VALS_BYTES + NA_HIST_BYTES);
+  pbg_launch_error() = cudaSuccess;      // (of an earlier call on this thread)
   // the array keeps whatever the previous call left: the error word has to start at zero
   if (cudaMemsetAsync(errflag, 0, sizeof(int), st) != cudaSuccess) return PBG_ERR_CUDA;
   const int bits = bit_len((unsigned long long)num_rows);

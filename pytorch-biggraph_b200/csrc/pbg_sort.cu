@@ -146,10 +146,10 @@ int pbg_sort(SortPlan &sp, int n, int bits, cudaStream_t st) {
   int nbins = 1 << db;
   unsigned int *totals = sp.hist + (size_t)MAX_BINS * nwarps;
   for (int pass = 0, shift = 0; pass < passes; ++pass, shift += db) {
-    radix_hist<<<ctas, 32 * SORT_WARPS_PER_CTA, 0, st>>>(sp.keys[src], n, shift, nbins, sp.hist, nwarps);
-    radix_scan<<<nbins, 128, 0, st>>>(sp.hist, nwarps, totals);
-    radix_scatter<<<ctas, 32 * SORT_WARPS_PER_CTA, 0, st>>>(sp.keys[src], sp.vals[src], n, shift, nbins, sp.hist, totals,
-                                                           nwarps, sp.keys[src ^ 1], sp.vals[src ^ 1]);
+    pbg_launch_in_order(radix_hist, ctas, 32 * SORT_WARPS_PER_CTA, 0, st, sp.keys[src], n, shift, nbins, sp.hist, nwarps);
+    pbg_launch_in_order(radix_scan, nbins, 128, 0, st, sp.hist, nwarps, totals);
+    pbg_launch_in_order(radix_scatter, ctas, 32 * SORT_WARPS_PER_CTA, 0, st, sp.keys[src], sp.vals[src], n, shift, nbins, sp.hist, totals,
+                        nwarps, sp.keys[src ^ 1], sp.vals[src ^ 1]);
     launches += 3;
     src ^= 1;
   }
@@ -173,7 +173,7 @@ __global__ void iota_keys(const long long *__restrict__ rows, long long num_rows
 
 int launch_iota_keys(const long long *rows, long long num_rows, int n, unsigned long long *keys,
                      unsigned int *vals, int *errflag, cudaStream_t st) {
-  iota_keys<<<(n + 255) / 256, 256, 0, st>>>(rows, num_rows, n, keys, vals, errflag);
+  pbg_launch_in_order(iota_keys, (n + 255) / 256, 256, 0, st, rows, num_rows, n, keys, vals, errflag);
   return 1;
 }
 
@@ -338,6 +338,7 @@ static void cluster_shape(int n, int &ctas, int &ipt) {
 
 template <class... Args>
 static void launch_cluster(void (*kernel)(Args...), int lists, int ctas, size_t smem, cudaStream_t st, Args... args) {
+  if (pbg_launch_failed()) return;
   pbg_opt_in_smem((const void *)kernel, (int)smem);
   if (ctas > 8) pbg_opt_in_cluster16((const void *)kernel);
   cudaLaunchConfig_t cfg = {};
