@@ -7,6 +7,7 @@ import torch
 from golden_util import load_step, step_fixture_names
 from oracle import pbg_step as O
 import test_gpu_step as steps
+import test_gpu_step_edges as edges
 
 pytestmark = pytest.mark.gpu
 
@@ -69,10 +70,41 @@ def test_fp32_tier_keeps_its_bits(monkeypatch):
             np.testing.assert_array_equal(a, b)
 
 
-@pytest.mark.parametrize("precision", ["fp32", "tf32x3", "bf16x6"])
+TIERS = steps.PRECISIONS + steps.PLANE_TIERS
+
+
+@pytest.mark.parametrize("precision", TIERS)
 @pytest.mark.parametrize("name", [n for n in step_fixture_names() if load_step(n)[0]["op"] not in ("linear", "affine")])
 def test_separate_kernels_on_the_reference_fixtures(name, precision, monkeypatch):
     """The fixtures are small enough for the one-kernel path: the kernels of larger waves on them too."""
     monkeypatch.setenv("PBG_CHUNK", "0")
-    steps.test_step_matches_reference_fixture(name, precision)
-    steps.test_forward_scores_match_reference_fixture(name, precision)
+    with steps._tier_tolerance(precision):
+        steps.test_step_matches_reference_fixture(name, precision)
+        steps.test_forward_scores_match_reference_fixture(name, precision)
+
+
+_C1 = steps.BASELINE_SHAPES[0].values
+SMALL = ([("waves-of-fixtures", steps.test_wave_of_three_batches_matches_oracle, (n, t), t) for n in ("sequence_3_batches", "sequence_3_batches_dyn_cos") for t in TIERS]
+         + [("wave-with-global", steps.test_wave_with_global_embeddings_matches_oracle, (t,), t) for t in TIERS]
+         + [("dealt-evenly", steps.test_batches_are_dealt_evenly_to_waves, (), "fp32")]
+         + [("C1", steps.test_baseline_shapes_match_oracle, _C1 + (t,), t) for t in TIERS]
+         + [("C1", steps.test_single_pass_tf32_is_the_1e3_tier, _C1, "tf32")]
+         + [("loss-rows-of-128-%s-%s" % (comp, loss), edges.test_score_rows_at_the_loss_kernels_widths, (128, comp, loss), "tf32x3")
+            for comp, loss in (("dot", "ranking"), ("dot", "logistic"), ("l2", "softmax"))])
+
+
+@pytest.mark.parametrize("test,args,tier", [pytest.param(test, args, tier, id=f"{name}-{tier}") for name, test, args, tier in SMALL])
+def test_separate_kernels_on_small_shapes(test, args, tier, monkeypatch):
+    """The same for the other tests whose shapes the one-kernel path takes by default."""
+    monkeypatch.setenv("PBG_CHUNK", "0")
+    with steps._tier_tolerance(tier):
+        test(*args)
+
+
+@pytest.mark.parametrize("tier", steps.PLANE_TIERS)
+def test_fused_kernels_with_global_embeddings(tier, monkeypatch):
+    """Waves of several batches with global vectors through the fused score + loss kernel and the dual gradient."""
+    monkeypatch.setenv("PBG_CHUNK", "0")
+    monkeypatch.setenv("PBG_FUSED", "1")
+    with steps._tier_tolerance(tier):
+        steps.test_wave_with_global_embeddings_matches_oracle(tier)
