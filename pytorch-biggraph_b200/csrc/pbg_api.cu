@@ -47,7 +47,8 @@ struct pbg_context {
   void *tcplan = nullptr;       // tensor maps of the tcgen05 contractions
   void *pairplan = nullptr;     // tensor maps of the fused score + loss kernel (standard relations, plane tiers)
   bool fused = false;           // training runs gather -> fused score / loss -> dual gradient product
-  bool chunk = false;           // training and scoring run one kernel from the ids to the gradient rows (pbg_chunk.cu)
+  bool chunk = false;           // training runs one kernel from the ids to the gradient rows (pbg_chunk.cu)
+  bool chunk_score = false;     // scoring runs its forward half
   float *psum = nullptr;        // partial gradient rows of hub rows, indexed by slot position
   long long *hublist = nullptr;
   int *hubcnt = nullptr;        // two sets of counters, used in turn
@@ -219,17 +220,30 @@ static bool fused_pays(const pbg_config &cfg, int npl, long long blocks) {
 //                     30 + 60          0.96 - 1.1          1.0  - 1.15          0.91 - 1.05      0.95 - 1.1
 //                     50 + 50, two     0.85                0.85 - 0.9           0.83 - 0.94      0.83 - 0.96
 //   bf16x3, standard  l2: 1.1 - 1.2, dot and cos: 0.95 - 1.06 (its two-plane products are the shortest there are)
+//   tf32, standard    l2: 1.02 - 1.15; dot and cos, whose products are a single pass (4 / 10 / 20 / 28 blocks, all four dimensions):
+//                     one tile  (10 + 5, 16 + 16)           1.05 - 1.1 / 1.05 - 1.1 / 1.0 - 1.1 / 0.98 - 1.1
+//                     two tiles (32 + 32, 50 + 14)          1.0 - 1.1 / 1.0 - 1.1 / 0.93 - 1.03 / 0.91 - 1.03
+//                     three, four (40 + 56 to 64 + 64)      0.95 - 1.03 / 0.95 - 1.05 / 0.80 - 0.98 / 0.83 - 1.03
+//   tf32, dynamic     two tiles: 1.0 - 1.1, l2 1.07 - 1.19
+// Scores alone (one kernel in place of three; whole calls of 40 to 80 us, 2 to 28 blocks, with and without batch negatives):
+//   fp32              1.02 - 1.1 at dimension 16, 1.1 - 1.4 at 100, 1.1 - 1.6 at 200 and 256; dynamic 1.06 - 1.2
+//   tf32x3, bf16x6    1.06 - 1.18, 1.0 - 1.14; tf32x3 dynamic 1.1 - 1.15
+//   bf16x3 l2, tf32   1.1 - 1.3, 0.97 - 1.1 (below 1 with 64 + 64 columns at dimension 128 only)
 // The fp32 tier's own products are on the CUDA cores too (and equal to these bit for bit), so it gains at every dimension; the
-// others do up to the 128 columns that one float4 a lane holds.
-static bool chunk_pays(const pbg_config &cfg, int Pm, int Mm, long long blocks) {
+// others do up to the 128 columns that one float4 a lane holds.  (From 129 floats the training kernel spills 104 to 116 bytes
+// at the 128 registers that two CTAs an SM leave; the table's figures there are with them.)
+static bool chunk_pays(const pbg_config &cfg, int Pm, int Mm, long long blocks, bool train) {
   const char *env = getenv("PBG_CHUNK");
   if (cfg.op == PBG_OP_LINEAR || cfg.op == PBG_OP_AFFINE || !pbg_chunk_fits(Pm, Mm, cfg.dim) || (env && env[0] == '0')) return false;
   if (env && env[0] == '1') return pbg_chunk_available();
   if (getenv("PBG_FUSED") || blocks > 28 || Pm > 64) return false;
   const int tiles = (Mm + 31) / 32 + (cfg.dynamic_relations ? (Pm + 31) / 32 : 0);
   if (cfg.precision == PBG_PREC_FP32) return tiles <= 4 && pbg_chunk_available();
-  if (cfg.dim > 128 || (cfg.precision == PBG_PREC_BF16X3 && cfg.comparator < PBG_CMP_L2)) return false;
-  return tiles <= (cfg.dynamic_relations ? 2 : 4) && pbg_chunk_available();
+  const bool products = cfg.comparator < PBG_CMP_L2;
+  if (cfg.dim > 128 || (cfg.precision == PBG_PREC_BF16X3 && products)) return false;
+  int most = cfg.dynamic_relations ? 2 : 4;
+  if (train && cfg.precision == PBG_PREC_TF32 && products && !cfg.dynamic_relations) most = blocks <= 12 ? 2 : 1;
+  return tiles <= most && pbg_chunk_available();
 }
 
 extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_context **out) {
@@ -318,7 +332,8 @@ extern "C" int pbg_create(const pbg_config *cfg, int device, void *stream, pbg_c
     const char *envk = getenv("PBG_SPLIT_MIN_K");
     if (envk && atoi(envk) >= 2) c->split_min_k = atoi(envk);
   }
-  c->chunk = chunk_pays(*cfg, c->Pm, c->Mm, (long long)c->kmax * c->Cm);
+  c->chunk = chunk_pays(*cfg, c->Pm, c->Mm, (long long)c->kmax * c->Cm, true);
+  c->chunk_score = chunk_pays(*cfg, c->Pm, c->Mm, (long long)c->kmax * c->Cm, false);
   if (planes) {
     oXB[0] = take(nN * npl * Dpb * 2); oXB[1] = take(nN * npl * Dpb * 2);
     if (dyn) { oXB[2] = take(nQ * npl * Dpb * 2); oXB[3] = take(nQ * npl * Dpb * 2); oTB[0] = take(nQ * npl * Kb * 2); oTB[1] = take(nQ * npl * Kb * 2); }
@@ -905,7 +920,7 @@ extern "C" int pbg_score_batch(pbg_context *c, const pbg_bucket *bk, const int64
   wb.n[0] = count; wb.rel[0] = d.dynamic ? 0 : relidx; wb.wrel[0] = 1.0f;
   d.k = 1; d.nblk = d.Cm; d.nocc = d.spb;
   d.blk0 = 0;
-  if (c->chunk) c->launches += launch_chunk_scores(d, wb, w, lhs_pos, rhs_pos, lhs_neg, rhs_neg, c->stream);
+  if (c->chunk_score) c->launches += launch_chunk_scores(d, wb, w, lhs_pos, rhs_pos, lhs_neg, rhs_neg, c->stream);
   else {
     run_forward(c, d, wb, w, c->stream);
     c->launches += launch_export_scores(d, wb, w, lhs_pos, rhs_pos, lhs_neg, rhs_neg, c->stream);

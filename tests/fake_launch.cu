@@ -7,9 +7,11 @@
 #include "pbg_common.cuh"
 
 static std::map<const void *, std::string> names;
+static std::string launched;                        // the kernels since fake_arm, one after the other
 static int launches, fail_at, behind_failure, unclean;
 static bool failed, bad_ids;
-extern "C" void fake_arm(int at, int ids) { fail_at = at; bad_ids = ids != 0; launches = behind_failure = unclean = 0; failed = false; }
+extern "C" void fake_arm(int at, int ids) { fail_at = at; bad_ids = ids != 0; launches = behind_failure = unclean = 0; failed = false; launched.clear(); }
+extern "C" const char *fake_launched() { return launched.c_str(); }
 extern "C" int fake_launches() { return launches; }
 extern "C" int fake_behind_failure() { return behind_failure; }
 extern "C" int fake_unclean() { return unclean; }
@@ -44,6 +46,7 @@ static void run(const std::string &name, void **args) {
 static cudaError_t launch(const void *func, void **args) {
   if (failed) ++behind_failure;
   if (++launches == fail_at) { failed = true; return cudaErrorLaunchOutOfResources; }
+  launched += names[func] + " ";
   run(names[func], args);
   return cudaSuccess;
 }
