@@ -24,9 +24,10 @@ static __device__ __align__(256) unsigned char pbg_noalloc_scratch[NA_TOTAL_BYTE
 // In host code `pbg_noalloc_scratch` is only a handle: its device address is looked up once per
 // device, with that device current, and that address is what the kernels get.
 static unsigned char *scratch_addr[NOALLOC_MAX_DEVICES];
+static bool cluster_sort[NOALLOC_MAX_DEVICES];         // the device can hold the sort's clusters, for the longest list
 static std::mutex scratch_mutex;
 
-static int scratch_for_current_device(unsigned char **out) {
+static int scratch_for_current_device(unsigned char **out, bool &clusters) {
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess) return PBG_ERR_NO_DEVICE;
   if (dev < 0 || dev >= NOALLOC_MAX_DEVICES) return PBG_ERR_TOO_LARGE;
@@ -36,8 +37,10 @@ static int scratch_for_current_device(unsigned char **out) {
     cudaError_t e = cudaGetSymbolAddress(&p, pbg_noalloc_scratch);
     if (e != cudaSuccess || !p) return PBG_ERR_CUDA;
     scratch_addr[dev] = (unsigned char *)p;
+    cluster_sort[dev] = pbg_cluster_sort_available(NOALLOC_MAX_ROWS);
   }
   *out = scratch_addr[dev];
+  clusters = cluster_sort[dev];
   return PBG_OK;
 }
 
@@ -51,7 +54,8 @@ extern "C" int pbg_row_adagrad_static(float *emb, float *state, int64_t num_rows
   if (dim <= 0 || dim % 4 != 0 || dim > 2048) return PBG_ERR_UNSUPPORTED;
   if (n > NOALLOC_MAX_ROWS) return PBG_ERR_TOO_LARGE;      // the fixed scratch holds 16384 rows
   unsigned char *base = nullptr;
-  int rc = scratch_for_current_device(&base);
+  bool clusters = false;
+  int rc = scratch_for_current_device(&base, clusters);
   if (rc != PBG_OK) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   SortPlan sp;
@@ -67,7 +71,7 @@ extern "C" int pbg_row_adagrad_static(float *emb, float *state, int64_t num_rows
   // the array keeps whatever the previous call left: the error word has to start at zero
   if (cudaMemsetAsync(errflag, 0, sizeof(int), st) != cudaSuccess) return PBG_ERR_CUDA;
   const int bits = bit_len((unsigned long long)num_rows);
-  if (pbg_cluster_sort_fits(n, bits)) {
+  if (clusters && pbg_cluster_sort_fits(n, bits)) {
     launch_sort_rows((const long long *)rows_dev, num_rows, n, bits, sp.keys[0], sp.vals[0], errflag, st);
   } else {
     launch_iota_keys((const long long *)rows_dev, num_rows, n, sp.keys[0], sp.vals[0], errflag, st);

@@ -38,7 +38,31 @@ def test_small_waves_take_one_kernel_where_it_is_shorter(fake):
     F.run_child(__file__, fake)
 
 
-def main(fake_so):
+@pytest.mark.parametrize("clusters", [True, False])
+def test_sorts_go_without_clusters_where_the_device_has_no_room_for_them(fake, clusters):
+    """(with part of a device's SMs there may be none): the radix passes, not a launch that fails."""
+    F.run_child(__file__, fake, "clusters" if clusters else "none", **({} if clusters else {"FAKE_NO_CLUSTERS": "1"}))
+
+
+def sorts(fake_so, room):
+    import numpy as np
+    fake, L, lib = F.load(fake_so)
+    n, rows, D = 300, 400, 32
+    ids, W, G, p = F.dev(n, np.int64), F.dev((rows, D), np.float32), F.dev(rows, np.float32), F.p
+    ctx = F.create(L, lib, dim=D, op=0, comparator=0, loss=2, num_batch_negs=20, num_uniform_negs=10, max_batch_size=n)
+    bk = F.bucket(L, rows, D, False)
+    for call in (lambda: F.train(L, lib, ctx, bk, ids, n, 1), lambda: lib.pbg_row_adagrad(ctx, p(W), p(G), rows, p(ids), p(W), n, 0.1),
+                 lambda: lib.pbg_row_adagrad_static(p(W), p(G), rows, D, p(ids), p(W), n, 0.1, None)):
+        fake.fake_arm(0, 0)
+        assert call() == L.PBG_OK
+        names = fake.fake_launched().decode()
+        assert ("sort_waves_kernel" in names or "sort_rows_kernel" in names) == (room == "clusters"), names
+        assert ("radix_scatter" in names) == (room != "clusters"), names
+
+
+def main(fake_so, room=None):
+    if room:
+        return sorts(fake_so, room)
     import numpy as np
     fake, L, lib = F.load(fake_so)
     for precision, comp, dynamic, D, nb, nu, blocks, train, score in ROUTES:
