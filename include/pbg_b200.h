@@ -302,8 +302,10 @@ int64_t pbg_launch_count(const pbg_context *ctx);
  * enable = 2: the halves are launched one after the other on the context's stream, so that a pair
  * brackets its kernels alone -- the durations to hold against a roofline.
  * Classes: 0 sort keys + radix sort, 1 gather/operator/prepare, 2 score contraction, 3 loss,
- * 4 gradient contractions, 5 optimizer updates (the batches' Stats are summed inside them).  ms_out / launches_out: HOST arrays of
- * PBG_NUM_KERNEL_CLASSES entries. */
+ * 4 gradient contractions, 5 optimizer updates (the pull-back of the gradients among them; the batches' Stats are summed inside).
+ * A kernel that does the work of several classes is booked under one, 2: the fused kernel of the plane tiers with its loss,
+ * and the one kernel of small waves, which goes from the gather to the pulled-back gradients (classes 1 and 4 then stay empty,
+ * and rates by class say nothing about such a context).  ms_out / launches_out: HOST arrays of PBG_NUM_KERNEL_CLASSES entries. */
 #define PBG_NUM_KERNEL_CLASSES 6
 int pbg_set_profiling(pbg_context *ctx, int enable);
 int pbg_kernel_times(pbg_context *ctx, double *ms_out, int64_t *launches_out);

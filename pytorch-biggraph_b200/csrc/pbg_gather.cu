@@ -11,10 +11,18 @@
 
 #define GATHER_WARPS 8
 
-// Resident CTAs per SM, by the float4 a lane holds of a row.  A warp waits for one row after the other, so what counts is warps, as
-// long as registers last (gather class of whole buckets, serial): general kernel, rows of up to 128 floats 5 CTAs (two planes:
-// 0.67 ms at 3, 0.59 at 4, 0.55 at 5), of 256 4 (1.09 at 3, 0.99), of 512 3 (1.87; 2.10 at 4 and 2.15 at 2); plain kernel, rows of
-// up to 256 floats 6 (three planes: 1.57 at 4, 1.43 at 6, 1.44 at 8), of 1024 2 (2.09 at 3 with registers spilled, 1.96, 2.74 at 4).
+// Resident CTAs per SM, by the float4 a lane holds of a row.  A warp waits for one row after the other, so what counts is warps, also
+// where registers spill to memory for them (general kernel: 12 to 400 bytes of stores a thread up to 512 floats, 280 to 672 at 1024,
+// 2,056 to 2,664 at 2048; a CTA less spills only at 2048, 380 to 948).  Gather class of a wave of 14 batches (1000 edges, 100 + 100
+// negatives, one after the other), us, with a CTA less / this / a CTA more:
+//   general kernel             128 floats           256              512                1024              2048
+//     translation, cos         34.4 / 33.7 / 32.0   44.0/40.4/41.6   68.1/58.5/59.3     136 /104 /109     216 / 206
+//       three planes           31.1 / 29.2 / 29.3   43.6/41.1/44.8   84.5/77.9/82.6     203 /164 /178     363 / 394
+//     dynamic, complex, dot    37.3 / 36.8 / 36.1   55.6/49.7/53.1   104 /93.0/91.6     270 /199 /202     532 / 479
+//       three planes           46.8 / 45.7 / 47.6   72.7/71.9/81.4   151 /149 /160      386 /315 /328     825 / 779
+//   plain kernel, three planes, two CTAs less up to 256 floats, one more from 513: 64 floats 21.1 / 19.4, 128 23.4 / 21.8, 256 30.0 /
+//   29.5, 768 83.7 / 79.1, 1024 108 / 99.7 (there the third spilled); without planes the same within 2 %.
+// (One row in which a CTA less would do better: standard relations with planes at 2048 floats.)
 template <int VEC> struct GatherCtas {
   enum { GENERAL = VEC >= 8 ? 2 : VEC == 4 ? 3 : VEC == 2 ? 4 : 5, PLAIN = VEC >= 16 ? 1 : VEC == 8 ? 2 : VEC == 4 ? 4 : 6 };
 };

@@ -243,11 +243,11 @@ tc_gemm_kernel(const __grid_constant__ TcMaps maps, TcGeom g, WaveDims d, WaveBa
             }
           }
         } else {
-          constexpr uint32_t KSBO = KB == 32 ? 1024 : 512, KLAY = KB == 32 ? 2 : 4;     // K-major: 8 rows of ROW_BYTES; 128- / 64-byte swizzle
+          constexpr uint32_t KSBO = 1024, KLAY = 2;             // K-major: 8 rows of 128 bytes, 128-byte swizzle
           constexpr uint32_t a_step = A_MN ? 1024 : 32, b_step = B_MN ? 1024 : 32;
           const uint64_t da0 = A_MN ? smem_desc(aH, BOX_BYTES, 512, 1) : smem_desc(aH, 0, KSBO, KLAY);
           const uint64_t db0 = B_MN ? smem_desc(bH, BOX_BYTES, 512, 1) : smem_desc(bH, 0, KSBO, KLAY);
-if (SPLIT) {
+          if (SPLIT) {
             // the two products with lo parts first: their buffer goes back while hi . hi runs
             const uint32_t lo0 = smem_u32(lo);
             const uint64_t dal0 = A_MN ? smem_desc(lo0, BOX_BYTES, 512, 1) : smem_desc(lo0, 0, KSBO, KLAY);
@@ -555,7 +555,7 @@ static void launch_tc(const TcMaps &maps, const TcGeom &g, int nterms, const Wav
   long long tiles = (long long)((g.N + g.BN - 1) / g.BN) * ((g.M + 127) / 128) * d.nblk * 2;
   const int sms = pbg_sm_count();
   dim3 grid((unsigned)(tiles < sms ? tiles : sms));
-  size_t smem = 4 * (128 * 128 + 256 * 128) + 4 * 2 * 4096 + 1024;   // 2 stages x (hi, lo) or 4 stages x raw; epilogue staging
+  size_t smem = 4 * (128 * 128 + 256 * 128) + 4 * 2 * 4096 + 1024;   // 3 raw stages and one buffer of lo parts, or 4 raw stages; epilogue staging
   // the comparator epilogue of the l2 family exists only in the score kernels (both operands K-major)
   const bool l2 = !A_MN && !B_MN && g.score && g.cmp >= PBG_CMP_L2;
   if constexpr (!A_MN && !B_MN) {
