@@ -117,7 +117,10 @@ static int fail(pbg_context *c, int code, const char *fmt, ...) {
 #define CU(c, call)                                                                          \
   do {                                                                                       \
     cudaError_t e_ = (call);                                                                 \
-    if (e_ != cudaSuccess) return fail(c, PBG_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); \
+    if (e_ != cudaSuccess) {                                                                 \
+      cudaGetLastError();              /* reported here: not once more by the next call */   \
+      return fail(c, PBG_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_));                 \
+    }                                                                                        \
   } while (0)
 
 extern "C" const char *pbg_version(void) { return "pbg_b200 0.1 (sm_100a)"; }

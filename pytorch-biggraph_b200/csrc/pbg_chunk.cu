@@ -312,7 +312,6 @@ static cudaError_t chunk_opt_in() { return pbg_opt_in_smem((const void *)chunk_k
 
 bool pbg_chunk_available() {
   const void *kernel = (const void *)chunk_kernel<2, 8, true>;                     // the one that takes the most registers
-  if (chunk_opt_in<2, 8, true>() != cudaSuccess) return false;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(CHUNK_CTAS); cfg.blockDim = dim3(CHUNK_THREADS); cfg.dynamicSmemBytes = chunk_smem();
   cudaLaunchAttribute at;
@@ -320,7 +319,7 @@ bool pbg_chunk_available() {
   at.val.clusterDim.x = CHUNK_CTAS; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
   cfg.attrs = &at; cfg.numAttrs = 1;
   int n = 0;
-  const bool ok = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n >= 1;
+  const bool ok = chunk_opt_in<2, 8, true>() == cudaSuccess && cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n >= 1;
   if (!ok) pbg_take_launch_error();                   // (an answer, not a failure of the call that asked)
   return ok;
 }

@@ -378,10 +378,9 @@ inline void pbg_note_launch(cudaError_t e = cudaGetLastError()) {
 // counts, sums) for places in memory, and would find another call's there.
 inline bool pbg_launch_failed() { return pbg_launch_error() != cudaSuccess; }
 inline cudaError_t pbg_take_launch_error() {
-  cudaError_t e = pbg_launch_error();
+  const cudaError_t e = pbg_launch_error(), last = cudaGetLastError();      // (the runtime keeps the same error: taken with it)
   pbg_launch_error() = cudaSuccess;
-  if (e == cudaSuccess) e = cudaGetLastError();
-  return e;
+  return e != cudaSuccess ? e : last;
 }
 inline cudaError_t pbg_opt_in_smem(const void *kernel, int bytes) {
   static std::mutex mu;

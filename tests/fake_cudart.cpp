@@ -4,7 +4,16 @@
 #include <stdlib.h>
 #include <string.h>
 
+static cudaError_t last = cudaSuccess;               // kept until cudaGetLastError asks for it
+
 extern "C" {
+const char *fake_kernel_name(const void *);
+cudaError_t fake_refuse(cudaError_t e) { return last = e; }
+cudaError_t cudaGetLastError() { const cudaError_t e = last; last = cudaSuccess; return e; }
+cudaError_t cudaFuncSetAttribute(const void *f, cudaFuncAttribute, int) {
+  const char *name = getenv("FAKE_REFUSED");       // a kernel that the device cannot hold
+  return name && strstr(fake_kernel_name(f), name) ? fake_refuse(cudaErrorInvalidValue) : cudaSuccess;
+}
 void **__cudaRegisterFatBinary(void *) { static void *h; return &h; }
 char __cudaInitModule(void **) { return 1; }
 void __cudaRegisterFatBinaryEnd(void **) {}
@@ -13,7 +22,14 @@ void __cudaRegisterVar(void **, char *, char *, const char *, int, size_t, int, 
 unsigned __cudaPushCallConfiguration(dim3, dim3, size_t, struct CUstream_st *) { return 0; }
 cudaError_t __cudaPopCallConfiguration(dim3 *, dim3 *, size_t *, void *) { return cudaSuccess; }
 
-cudaError_t cudaMalloc(void **p, size_t n) { *p = nullptr; if (posix_memalign(p, 256, n ? n : 1)) return cudaErrorMemoryAllocation; memset(*p, 0xA5, n); return cudaSuccess; }
+static bool no_memory = false;
+void fake_no_memory(int yes) { no_memory = yes != 0; }
+cudaError_t cudaMalloc(void **p, size_t n) {
+  *p = nullptr;
+  if (no_memory || posix_memalign(p, 256, n ? n : 1)) return fake_refuse(cudaErrorMemoryAllocation);
+  memset(*p, 0xA5, n);
+  return cudaSuccess;
+}
 cudaError_t cudaFree(void *p) { free(p); return cudaSuccess; }
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return cudaMalloc(p, n); }
 cudaError_t cudaFreeHost(void *p) { return cudaFree(p); }
@@ -28,9 +44,7 @@ cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int) {
   *v = a == cudaDevAttrComputeCapabilityMajor ? 10 : a == cudaDevAttrMultiProcessorCount ? 148 : 0;
   return cudaSuccess;
 }
-cudaError_t cudaFuncSetAttribute(const void *, cudaFuncAttribute, int) { return cudaSuccess; }
 cudaError_t cudaOccupancyMaxActiveClusters(int *n, const void *, const cudaLaunchConfig_t *) { *n = getenv("FAKE_NO_CLUSTERS") ? 0 : 8; return cudaSuccess; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t) { return "fake"; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { *s = nullptr; return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }

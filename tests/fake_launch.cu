@@ -10,6 +10,7 @@ static std::map<const void *, std::string> names;
 static std::string launched;                        // the kernels since fake_arm, one after the other
 static int launches, fail_at, behind_failure, unclean;
 static bool failed, bad_ids;
+extern "C" cudaError_t fake_refuse(cudaError_t);
 extern "C" void fake_arm(int at, int ids) { fail_at = at; bad_ids = ids != 0; launches = behind_failure = unclean = 0; failed = false; launched.clear(); }
 extern "C" const char *fake_launched() { return launched.c_str(); }
 extern "C" int fake_launches() { return launches; }
@@ -45,7 +46,7 @@ static void run(const std::string &name, void **args) {
 
 static cudaError_t launch(const void *func, void **args) {
   if (failed) ++behind_failure;
-  if (++launches == fail_at) { failed = true; return cudaErrorLaunchOutOfResources; }
+  if (++launches == fail_at) { failed = true; return fake_refuse(cudaErrorLaunchOutOfResources); }
   launched += names[func] + " ";
   run(names[func], args);
   return cudaSuccess;
@@ -54,5 +55,6 @@ static cudaError_t launch(const void *func, void **args) {
 extern "C" {
 cudaError_t cudaLaunchKernel(const void *f, dim3, dim3, void **args, size_t, cudaStream_t) { return launch(f, args); }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *, const void *f, void **args) { return launch(f, args); }
+const char *fake_kernel_name(const void *f) { return names[f].c_str(); }
 void __cudaRegisterFunction(void **, const char *f, char *, const char *name, int, uint3 *, uint3 *, dim3 *, dim3 *, int *) { names[f] = name; }
 }

@@ -21,6 +21,23 @@ def test_a_failed_launch_leaves_nothing_behind(fake, call):
     F.run_child(__file__, fake, call, **({"PBG_CLUSTER_SORT": "0"} if call == "train_radix" else {}))
 
 
+def test_a_failed_allocation_is_the_failure_of_its_own_call(fake):
+    """The runtime keeps an error until it is asked for it: the next call must not find it."""
+    F.run_child(__file__, fake, "no_memory")
+
+
+def no_memory(fake, L, lib):
+    import numpy as np
+    n, rows, D = 300, 400, 32
+    ctx = F.create(L, lib, dim=D, op=2, comparator=0, loss=2, num_batch_negs=20, num_uniform_negs=10, precision=1, max_batch_size=n)
+    ids, bk, p, ev = F.dev(n, np.int64), F.bucket(L, rows, D, False), F.p, L.PbgEvalStats()
+    fake.fake_no_memory(1)                                       # (its scratch is allocated at its first call)
+    assert lib.pbg_eval_batch_all_negs(ctx, C.byref(bk), p(ids), p(ids), None, n, 0, 7, C.byref(ev)) == L.PBG_ERR_CUDA
+    fake.fake_no_memory(0)
+    assert F.train(L, lib, ctx, bk, ids, n, 1) == L.PBG_OK
+    assert lib.pbg_eval_batch_all_negs(ctx, C.byref(bk), p(ids), p(ids), None, n, 0, 7, C.byref(ev)) == L.PBG_OK
+
+
 def _calls(L, lib, name):
     """A function that makes the call once and returns its status."""
     import numpy as np
@@ -53,6 +70,8 @@ def _calls(L, lib, name):
 
 def main(fake_so, name):
     fake, L, lib = F.load(fake_so)
+    if name == "no_memory":
+        return no_memory(fake, L, lib)
     call = _calls(L, lib, name)
     fake.fake_arm(0, 0)
     assert call() == L.PBG_OK and fake.fake_unclean() == 0

@@ -1,4 +1,5 @@
 """Which kernels a context takes for its training and its scores, by size and tier.  On the CPU (fake_cuda_util)."""
+import os
 import sys
 
 import pytest
@@ -44,6 +45,24 @@ def test_sorts_go_without_clusters_where_the_device_has_no_room_for_them(fake, c
     F.run_child(__file__, fake, "clusters" if clusters else "none", **({} if clusters else {"FAKE_NO_CLUSTERS": "1"}))
 
 
+@pytest.mark.parametrize("kernel", ["chunk_kernel", "sort_waves_kernel"])
+def test_a_kernel_the_device_cannot_hold_fails_no_call(fake, kernel):
+    """(its opt-in to shared memory is refused when the context asks): the other kernels, and no error left for the next call."""
+    F.run_child(__file__, fake, "without", FAKE_REFUSED=kernel)
+
+
+def without(fake_so):
+    import numpy as np
+    fake, L, lib = F.load(fake_so)
+    n, D = 300, 32
+    ctx, bk, ids = F.create(L, lib, dim=D, op=0, comparator=0, loss=2, num_batch_negs=20, num_uniform_negs=10, max_batch_size=n), F.bucket(L, 400, D, False), F.dev(n, np.int64)
+    for _ in range(2):
+        fake.fake_arm(0, 0)
+        assert F.train(L, lib, ctx, bk, ids, n, 1) == L.PBG_OK, lib.pbg_last_error(ctx)
+        names = fake.fake_launched().decode()
+        assert os.environ["FAKE_REFUSED"] not in names and "narrow_tile_kernel" in names, names
+
+
 def sorts(fake_so, room):
     import numpy as np
     fake, L, lib = F.load(fake_so)
@@ -62,7 +81,7 @@ def sorts(fake_so, room):
 
 def main(fake_so, room=None):
     if room:
-        return sorts(fake_so, room)
+        return without(fake_so) if room == "without" else sorts(fake_so, room)
     import numpy as np
     fake, L, lib = F.load(fake_so)
     for precision, comp, dynamic, D, nb, nu, blocks, train, score in ROUTES:
