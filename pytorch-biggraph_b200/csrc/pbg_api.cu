@@ -855,10 +855,11 @@ extern "C" int pbg_train_batches_host(pbg_context *c, const pbg_bucket *bk, cons
   if (!c) return PBG_ERR_BAD_ARGUMENT;
   const float *ew = take_edge_weights(c);
   if (num_batches == 0) return PBG_OK;
-  if (!lhs || !rhs || num_edges < 0) return fail(c, PBG_ERR_BAD_ARGUMENT, "null edge arrays");
+  if (!lhs || !rhs || num_edges < 0 || num_batches < 0) return fail(c, PBG_ERR_BAD_ARGUMENT, "null edge arrays or a negative count");
   CU(c, cudaSetDevice(c->device));
   if (num_edges > c->edge_cap) {
     long long cap = num_edges + num_edges / 4 + 1024;
+    c->edge_cap = 0;
     for (int i = 0; i < 3; ++i) { int rc = grow_i64(c, &c->edge_dev[i], cap); if (rc) return rc; }
     c->edge_cap = cap;
   }
@@ -870,6 +871,7 @@ extern "C" int pbg_train_batches_host(pbg_context *c, const pbg_bucket *bk, cons
   if (ul || ur) {
     long long per = (long long)num_batches * c->Cm * c->U;
     if (per > c->uni_cap) {
+      c->uni_cap = 0;
       for (int i = 0; i < 2; ++i) { int rc = grow_i64(c, &c->uni_dev[i], per + 1024); if (rc) return rc; }
       c->uni_cap = per + 1024;
     }
@@ -1126,7 +1128,7 @@ extern "C" int pbg_sub_bucket(pbg_context *c, const int64_t *lhs_in, const int64
   if (!pbg_sub_bucket_inline(R) || nb >= 1024) {
     if (need > c->etab_cap) {
       if (c->etab_dev) cudaFree(c->etab_dev);
-      c->etab_dev = nullptr;
+      c->etab_dev = nullptr; c->etab_cap = 0;
       CU(c, cudaMalloc(&c->etab_dev, (size_t)(need + 64) * sizeof(long long)));
       c->etab_cap = need + 64;
     }

@@ -35,7 +35,11 @@ cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return cudaMalloc(p, n
 cudaError_t cudaFreeHost(void *p) { return cudaFree(p); }
 cudaError_t cudaHostGetDevicePointer(void **d, void *h, unsigned) { *d = h; return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void *p, int v, size_t n, cudaStream_t) { memset(p, v, n); return cudaSuccess; }
-cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) { memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  if (!d || !s) return fake_refuse(cudaErrorInvalidValue);
+  memcpy(d, s, n);
+  return cudaSuccess;
+}
 cudaError_t cudaGetSymbolAddress(void **p, const void *) { static char scratch[1 << 22]; *p = scratch; return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }

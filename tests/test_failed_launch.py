@@ -26,6 +26,34 @@ def test_a_failed_allocation_is_the_failure_of_its_own_call(fake):
     F.run_child(__file__, fake, "no_memory")
 
 
+def test_scratch_that_could_not_grow_grows_at_the_next_call(fake):
+    """Freed to make room for a larger one that the device had no memory for: the next call, of the old size, allocates it again."""
+    F.run_child(__file__, fake, "no_growth")
+
+
+def no_growth(fake, L, lib):
+    import numpy as np
+    n, rows, D = 4000, 400, 32
+    ctx = F.create(L, lib, dim=D, op=2, comparator=0, loss=2, num_batch_negs=20, num_uniform_negs=10, precision=1, max_batch_size=100)
+    ids, bk, p = F.dev(n, np.int64), F.bucket(L, rows, D, False), F.p
+
+    def train_host(k):
+        batches, stats = (L.PbgBatch * k)(*[L.PbgBatch(100 * i, 100, 0) for i in range(k)]), (L.PbgBatchStats * k)()
+        neg = np.zeros((k, 5, 10), np.int64)
+        return lib.pbg_train_batches_host(ctx, C.byref(bk), p(ids), p(ids), p(ids), 100 * k, C.addressof(batches), k, p(neg), p(neg), 7, C.addressof(stats))
+
+    def split(relations):
+        counts, perms, sizes = np.zeros(4, np.int64), (C.c_void_p * relations)(*[F.dev(rows, np.int64).ctypes.data] * relations), (C.c_int64 * relations)(*[rows] * relations)
+        return lib.pbg_sub_bucket(ctx, p(ids), p(ids), p(ids), 300, relations, sizes, perms, sizes, perms, p(ids), p(ids), p(ids), 2, 2, 0,
+                                  counts.ctypes.data_as(C.POINTER(C.c_int64)))
+    for call, small, large in ((train_host, 2, 40), (split, 20, 300)):
+        assert call(small) == L.PBG_OK
+        fake.fake_no_memory(1)
+        assert call(large) == L.PBG_ERR_CUDA
+        fake.fake_no_memory(0)
+        assert call(small) == L.PBG_OK and call(large) == L.PBG_OK
+
+
 def no_memory(fake, L, lib):
     import numpy as np
     n, rows, D = 300, 400, 32
@@ -70,8 +98,8 @@ def _calls(L, lib, name):
 
 def main(fake_so, name):
     fake, L, lib = F.load(fake_so)
-    if name == "no_memory":
-        return no_memory(fake, L, lib)
+    if name in ("no_memory", "no_growth"):
+        return globals()[name](fake, L, lib)
     call = _calls(L, lib, name)
     fake.fake_arm(0, 0)
     assert call() == L.PBG_OK and fake.fake_unclean() == 0
