@@ -4,8 +4,8 @@
 // counted and summed where they lie and never stored.
 //
 // The CUDA-core tiles this replaces ran at 18 TFLOP/s of useful work (1000 edges against 14,951 entities a side,
-// dimension 400: 1.0 ms of a 1.33 ms call).  Bound here by shared-memory bandwidth beside the MMAs (72 KB loaded and
-// 144 KB read per 32 k-values), as in the training contractions.
+// dimension 400: 1.0 ms of a 1.33 ms call; this one takes 123 us of 186).  Not at a limit: 32 k-values of a tile take 2,500 to
+// 2,800 cycles, where the products take 1,540 and shared memory is busy for 1,690 (72 KB loaded, 144 KB read).
 //
 // Persistent CTAs walk the tiles of both sides, the row blocks of the same candidates one after the other: CTAs that run at the
 // same time then ask L2 for the same candidates (188.0 us a call, 189.7 with the candidate blocks first).
