@@ -526,7 +526,8 @@ int launch_update(const WaveDims &d, const WaveBatches &wb, const WaveBufs &w, c
 enum { HUB_REL = 32, HUB_SEAM_TILE = 64, HUB_SEAM_HUB = 96, HUB_SET = 128 };
 inline long long pbg_hublist_entries(long long nocc) { return nocc / 8 + 64; }
 // bigtab: a line for each row with 256 and more slots: where its batches start, and (last) a counter (zero between waves)
-inline size_t pbg_bigtab_bytes(long long nocc) { return (size_t)(nocc / 256 + 2) * (PBG_KMAX + 2) * sizeof(long long); }
+enum { BIGTAB_LINE = PBG_KMAX + 1 };
+inline size_t pbg_bigtab_bytes(long long nocc) { return (size_t)(nocc / 256 + 2) * BIGTAB_LINE * sizeof(long long); }
 // Evaluation of one batch after its scores.  out8 (host or device memory): loss, then pos_rank, mrr, r1, r10, r50 summed over
 // both sides, then the AUC hits per side.  part: 8 doubles for each of the kernel's CTAs; done: a counter, zero at first.
 inline int pbg_eval_auc_ctas(int nblk, int Pm) { return (int)((2ll * nblk * Pm + 255) / 256); }

@@ -161,7 +161,6 @@ __device__ __forceinline__ void param_step(const WaveDims &d, const WaveBatches 
 // ------------------------------------------------------------------------------------------------
 #define TILE 4
 #define SHORT_MAX 24
-#define BIGTAB_LINE (PBG_KMAX + 2)
 #define HUB_BIG 256     // rows with at least this many slots in a wave get their batches summed by separate CTAs
 // hublist holds nocc / 8 + 64 entries; a hub row has more than SHORT_MAX slots, so the rows themselves need fewer than
 // nocc / 16 + 32 of them and the list of big rows (at most nocc / HUB_BIG) lives in the rest.  hubcnt[0] counts hub
@@ -609,20 +608,15 @@ narrow_tile_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long l
       }
     }
     // A slot each, as for most rows of a wave: no loop over batches (update class of the plumbing bucket 3.55 -> 3.48 ms).
-    if (__all_sync(FULL, n <= 1 && !is_hub)) {
-      const float *g = (const float *)__shfl_sync(FULL, (unsigned long long)src, start & 31);
-      if (n == 1) {
+    if (__all_sync(FULL, n == 1 && !is_hub)) {
+      const float *g = (const float *)__shfl_sync(FULL, (unsigned long long)src, start);
 #pragma unroll
-        for (int c = 0; c < NP; ++c) if (ok[c]) acc[c] = acc[c] + ld4(g + c * 64 + l16 * 4);
-      }
-      const float ss = square(acc);
-      if (n == 1) {
-        G += ss * invD;
-        const float stepv = lr / (sqrtf(G) + PBG_ADAGRAD_EPS);
+      for (int c = 0; c < NP; ++c) if (ok[c]) acc[c] = acc[c] + ld4(g + c * 64 + l16 * 4);
+      G += square(acc) * invD;
+      const float stepv = lr / (sqrtf(G) + PBG_ADAGRAD_EPS);
 #pragma unroll
-        for (int c = 0; c < NP; ++c) if (ok[c]) st4(prow + c * 64 + l16 * 4, v[c] - acc[c] * stepv);
-        if (l16 == 0) *pacc = G;
-      }
+      for (int c = 0; c < NP; ++c) if (ok[c]) st4(prow + c * 64 + l16 * 4, v[c] - acc[c] * stepv);
+      if (l16 == 0) *pacc = G;
       continue;
     }
     const int other = __shfl_xor_sync(FULL, n, 16), most = n > other ? n : other;
@@ -845,11 +839,11 @@ hub_kernel(WaveDims d, WaveBatches wb, WaveBufs w, const unsigned long long *__r
       if (threadIdx.x == 0) line[b] = q < eb ? q : -1;
       __threadfence();
       __syncthreads();
-      if (threadIdx.x == 0) closing = atomicAdd((unsigned long long *)&line[PBG_KMAX + 1], 1ull) == (unsigned long long)(d.k - 1);
+      if (threadIdx.x == 0) closing = atomicAdd((unsigned long long *)&line[PBG_KMAX], 1ull) == (unsigned long long)(d.k - 1);
       __syncthreads();
       if (!closing) continue;                                 // another batch of the row is still being summed
       __threadfence();
-      if (threadIdx.x == 0) line[PBG_KMAX + 1] = 0;           // for the next wave
+      if (threadIdx.x == 0) line[PBG_KMAX] = 0;           // for the next wave
     }
     const long long p = head + threadIdx.x;
     const unsigned long long kp = p < (long long)d.nocc ? ld_list<RULE>(keys + p) : ~0ull;
