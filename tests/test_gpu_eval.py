@@ -46,6 +46,26 @@ def test_ranking_evaluator_matches_oracle_scores(name):
     assert abs(st.metrics["auc"] / n - float(np.mean(aucs))) <= 4 * 0.5 / np.sqrt(n)
 
 
+def _mix64(z):
+    """The kernels' hash (splitmix64's finalizer)."""
+    m = 2**64 - 1
+    z = z + 0x9E3779B97F4A7C15 & m
+    z = (z ^ z >> 30) * 0xBF58476D1CE4E5B9 & m
+    z = (z ^ z >> 27) * 0x94D049BB133111EB & m
+    return z ^ z >> 31
+
+
+def _auc_samples(seed, side, count, cols, all_negs=False):
+    """The (positive, edge of the negative, its column) triples that the evaluator draws on one side."""
+    for i in range(count):
+        h = _mix64(seed ^ _mix64((0xA11CE5 if all_negs else 0xA0C0FFEE) + side * 0x10001 + i))
+        e, h = h % count, _mix64(h)
+        if all_negs:
+            yield e, h % count, _mix64(h) % cols
+        else:
+            yield e, h % (count * cols) // cols, h % (count * cols) % cols
+
+
 def _allnegs_rig(z, cfg_o, st_o):
     """Model and evaluator for a recorded all_negs case (tests/golden/allnegs_*.npz)."""
     import torch
@@ -102,6 +122,13 @@ def test_ranking_against_all_entities_matches_the_reference_evaluator(name):
         assert abs(st.metrics[k] - float(z["stat_" + k])) <= ties / 2 + 1e-6
     exact_auc = allnegs_stats(cfg_o, sc)["auc"]
     assert abs(st.metrics["auc"] / n - exact_auc) <= 4 * 0.5 / np.sqrt(n)
+    # ... and sample by sample; of those that tie as above either outcome will do
+    hits = unsure = 0
+    for side, (pos, neg) in enumerate(((sc["lhs_pos"], sc["lhs_neg"]), (sc["rhs_pos"], sc["rhs_neg"]))):
+        for e, er, j in _auc_samples(ev.seed + ev._calls, side, n, neg.shape[1], all_negs=True):
+            hits += pos[e] > neg[er, j]
+            unsure += abs(pos[e] - neg[er, j]) <= 2e-5 * (1 + abs(pos[e]))
+    assert abs(2 * st.metrics["auc"] - hits) <= unsure
 
 
 def test_all_negs_relations_are_not_trained():
@@ -118,13 +145,15 @@ def test_all_negs_relations_are_not_trained():
 
 @pytest.mark.parametrize("loss", ["softmax", "ranking", "logistic"])
 @pytest.mark.parametrize("B,nb,nu", [(1, 1, 3), (23, 7, 3), (130, 130, 390), (513, 513, 0), (515, 128, 2), (70, 0, 35)])
-def test_sampled_ranks_are_the_ranks_of_the_forward_scores(B, nb, nu, loss):
+def test_sampled_ranks_are_the_ranks_of_the_forward_scores(B, nb, nu, loss, monkeypatch):
     """Rows whose own column lies at every place of a group of four, chunks that end inside one, more columns than one pass of a
-    warp takes, no batch negatives: ranks and hits are counts over the scores that the forward call returns for the same
-    candidates (the same kernels, so they are equal), the loss is its formula in double precision over those scores.  The device
+    warp takes, no batch negatives, samples of the AUC that end inside a CTA of 256: ranks, hits and samples are counts over the
+    scores that the forward call returns for the same candidates (PBG_CHUNK=0: by the evaluator's own kernels, so they are equal),
+    the loss is its formula in double precision over those scores.  The device
     adds up to 520 terms in single precision: 520 x 2^-24 = 3.1e-5 relative, and the terms' own rounding (exp, log: a few 2^-24)."""
     import torch
     import torchbiggraph_b200 as T
+    monkeypatch.setenv("PBG_CHUNK", "0")
     g = torch.Generator().manual_seed(B + nb)
     rows, D, margin, chunks = 900, 20, 0.1, -(-B // (nb or nu))
     cfg = T.ConfigSchema(entities={"e": T.EntitySchema()}, relations=[T.RelationSchema("r", "e", "e", operator="none")], dimension=D,
@@ -136,12 +165,14 @@ def test_sampled_ranks_are_the_ranks_of_the_forward_scores(B, nb, nu, loss):
     edges = T.EdgeList(T.EntityList.from_tensor(torch.randint(0, rows, (B,), generator=g)), T.EntityList.from_tensor(torch.randint(0, rows, (B,), generator=g)), torch.tensor(0))
     ul, ur = (torch.randint(0, rows, (chunks, nu), generator=g).cuda() if nu else None for _ in range(2))
     sc = m(edges, ul, ur)
-    st = T.B200RankingEvaluator(T.LOSS_FUNCTIONS.get_class(loss)(margin=margin), [1.0]).process_one_batch(m, edges, ul, ur)
-    want, value = np.zeros(4), 0.0
-    for pos, neg in ((sc.lhs_pos, sc.lhs_neg), (sc.rhs_pos, sc.rhs_neg)):
+    ev = T.B200RankingEvaluator(T.LOSS_FUNCTIONS.get_class(loss)(margin=margin), [1.0])
+    st = ev.process_one_batch(m, edges, ul, ur)
+    want, value = np.zeros(6), 0.0
+    for side, (pos, neg) in enumerate(((sc.lhs_pos, sc.lhs_neg), (sc.rhs_pos, sc.rhs_neg))):
         pos, neg = pos.double().cpu(), neg.double().cpu()
         rk = 1 + (neg >= pos[:, None]).sum(1)
-        want += [float(rk.sum()) / 2] + [float((rk <= k).sum()) / 2 for k in (1, 10, 50)]
+        hits = sum(bool(pos[e] > neg[er, j]) for e, er, j in _auc_samples(ev.seed + ev._calls, side, B, neg.shape[1]))
+        want += [x / 2 for x in (float(rk.sum()), *(float((rk <= k).sum()) for k in (1, 10, 50)), float((1.0 / rk.double()).sum()), hits)]
         if loss == "softmax":
             value += float((torch.logsumexp(torch.cat([pos[:, None], neg], 1), 1) - pos).sum())
         elif loss == "ranking":
@@ -149,5 +180,5 @@ def test_sampled_ranks_are_the_ranks_of_the_forward_scores(B, nb, nu, loss):
         else:
             sp = torch.nn.functional.softplus
             value += float(sp(-pos).sum() + sp(neg).sum() / neg.shape[1])
-    assert [st.metrics[k] for k in ("pos_rank", "r1", "r10", "r50")] == pytest.approx(list(want), abs=1e-9)
+    assert [st.metrics[k] for k in ("pos_rank", "r1", "r10", "r50", "mrr", "auc")] == pytest.approx(list(want), abs=1e-9)
     assert st.metrics["loss"] == pytest.approx(value, rel=4e-5, abs=1e-5)
