@@ -28,6 +28,9 @@ SHAPES = [
     (24, 70, 20, 10, "complex_diagonal", "dot", "softmax", True),
     (200, 70, 30, 40, "diagonal", "l2", "logistic", True),
     (104, 99, 33, 31, "translation", "cos", "ranking", True),           # a second tile of GQ rows
+    (132, 150, 70, 59, "diagonal", "dot", "softmax", False),            # two float4 a lane and a column beyond 128
+    (200, 260, 130, 126, "complex_diagonal", "squared_l2", "logistic", False),   # ... and the most columns
+    (256, 90, 45, 100, "translation", "cos", "softmax", True),
 ]
 
 
