@@ -335,7 +335,7 @@ int launch_chunk_step(const WaveDims &d, const WaveBatches &wb, const WaveBufs &
   for (int p = 0; p < 2; ++p) v.TB[p] = nullptr;      // (coefficients as fp32 only: the tensor cores have no part in this)
   const ChunkOut none = {};
   const int vec = (d.D + 127) / 128;
-  const bool wide = d.Ms > 128;
+  const bool wide = d.Ms > 128;                       // (only where PBG_CHUNK=1 asks for it: by itself the rule stops at 128 columns)
 #define CHUNK(V) (wide ? launch_chunk<V, 8, true>(d, wb, v, none, st) : launch_chunk<V, 4, true>(d, wb, v, none, st))
   if (vec <= 1) CHUNK(1); else CHUNK(2);
 #undef CHUNK
